@@ -107,8 +107,8 @@ SNNTC_API int snntc_cv_backward(const float* grad, const float* x_nhwc, const fl
  * Earliest-spike pooling between conv layers. The reference has no native code for it: SNN_maxpool2d
  * pads with 1e5 and calls -MaxPool2D(-x) in TensorFlow (SNN_TC_Modules.py:216-246). Here: window
  * minimum over the UNPADDED NHWC input with out-of-image taps reading `padvalue`; arg[B,Nh,Nw,C]
- * receives the flat input index of each winner (first minimum in (kh,kw) order, -1 for padding) and
- * drives the backward: every input element sums gy over the windows it won, in window order (a gather --
+ * receives the flat input index of each winner (first minimum in (kh,kw) order, -1 for padding; null: not
+ * wanted) and drives the backward: every input element sums gy over the windows it won, in window order (a gather --
  * no atomics, so overlapping windows give the same bits every run); dx[B,H,W,C] is written in full.
  */
 SNNTC_API int snntc_minpool_forward(const float* x_nhwc, float* y, int* arg, int B, int H, int W, int C,
@@ -148,6 +148,12 @@ SNNTC_API int snntc_cv_infer(const float* x_nhwc, const float* w, const float* p
  *                    sums2[1] += number of samples whose arg-min_j y equals the label (snntc-mnist.py:82); the
  *                    caller zeroes sums2. grad (may be null) receives d(sum_b loss_b)/dy * grad_scale, i.e.
  *                    -(softmax(-y) - onehot) * grad_scale; use loss_scale = grad_scale = 1/B for the mean.
+ * snntc_loss_forward / snntc_loss_backward   the same loss as a pair: *loss and *hits (device floats) are WRITTEN, not
+ *                    accumulated, in a fixed order of summation; the backward forms grad from y, the labels and the
+ *                    incoming gradient *gloss (device).
+ * snntc_weight_costs / snntc_weight_cost_grads   snntc_weight_cost for `count` tensors at once (the pointer, rows and
+ *                    cols arrays are on the host): *cost is written, colsum (sum of cols floats, device) receives the
+ *                    column sums in tensor order; the backward writes gw[k] = *gcost * d cost / d w[k] from them.
  * snntc_weight_cost  MyModel.constraint_cost for one weight tensor w[rows,J] (snntc-mnist.py:55-59):
  *                    cost[0] += K * mean_j max(0, 1 - sum_i w_ij) + K2 * mean(w^2); gw (may be null) +=
  *                    its gradient. workspace: snntc_weight_cost_workspace_bytes(J) bytes.
@@ -160,6 +166,16 @@ SNNTC_API int snntc_cv_infer(const float* x_nhwc, const float* w, const float* p
 SNNTC_API int snntc_encode(const float* p, float* x, size_t n, float scale, int one_minus, void* stream);
 SNNTC_API int snntc_loss_ce(const float* y, const long long* labels, float* grad, float* sums2, int B, int J,
                             float loss_scale, float grad_scale, void* stream);
+SNNTC_API int snntc_loss_forward(const float* y, const long long* labels, float* loss, float* hits, int B, int J,
+                                 float loss_scale, void* stream);
+SNNTC_API int snntc_loss_backward(const float* y, const long long* labels, const float* gloss, float* grad, int B, int J,
+                                  float grad_scale, void* stream);
+SNNTC_API size_t snntc_weight_costs_workspace_bytes(int count, const int* rows, const int* cols);
+SNNTC_API int snntc_weight_costs(int count, const float* const* w, const int* rows, const int* cols, float K, float K2,
+                                 float* colsum, float* cost, void* workspace, size_t workspace_bytes, void* stream);
+SNNTC_API int snntc_weight_cost_grads(int count, const float* const* w, float* const* gw, const int* rows,
+                                      const int* cols, float K, float K2, const float* colsum, const float* gcost,
+                                      void* stream);
 SNNTC_API size_t snntc_weight_cost_workspace_bytes(int J);
 SNNTC_API int snntc_weight_cost(const float* w, float* gw, float* cost, int rows, int J, float K, float K2,
                                 void* workspace, size_t workspace_bytes, void* stream);

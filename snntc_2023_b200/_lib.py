@@ -1,4 +1,4 @@
-"""ctypes binding of libsnntc_b200.so (the C ABI declared in include/snntc_b200.h).
+"""Loads libsnntc_b200.so (the C ABI declared in include/snntc_b200.h, bound with ctypes) and the native host path.
 
 There is no fallback: if the library is missing or a call fails, an exception is raised.
 """
@@ -36,6 +36,11 @@ SYMBOLS = {
     "snntc_cv_infer": (_INT, [_F] * 5 + [_INT] * 10 + [_F, _SZ, _F]),
     "snntc_encode": (_INT, [_F, _F, _SZ, ctypes.c_float, _INT, _F]),
     "snntc_loss_ce": (_INT, [_F, _F, _F, _F, _INT, _INT, ctypes.c_float, ctypes.c_float, _F]),
+    "snntc_loss_forward": (_INT, [_F, _F, _F, _F, _INT, _INT, ctypes.c_float, _F]),
+    "snntc_loss_backward": (_INT, [_F, _F, _F, _F, _INT, _INT, ctypes.c_float, _F]),
+    "snntc_weight_costs_workspace_bytes": (_SZ, [_INT, _F, _F]),
+    "snntc_weight_costs": (_INT, [_INT, _F, _F, _F, ctypes.c_float, ctypes.c_float, _F, _F, _F, _SZ, _F]),
+    "snntc_weight_cost_grads": (_INT, [_INT, _F, _F, _F, _F, ctypes.c_float, ctypes.c_float, _F, _F, _F]),
     "snntc_weight_cost_workspace_bytes": (_SZ, [_INT]),
     "snntc_weight_cost": (_INT, [_F, _F, _F, _INT, _INT, ctypes.c_float, ctypes.c_float, _F, _SZ, _F]),
     "snntc_adam_step": (_INT, [_F, _F, _F, _F, _SZ] + [ctypes.c_float] * 5 + [_F, _F]),
@@ -52,6 +57,7 @@ MEASURE_SYMBOLS = {
 
 _lib = None
 _measure = None
+_native = None
 
 
 class SnntcError(RuntimeError):
@@ -80,6 +86,22 @@ def load():
     if _lib is None:
         _lib = _open(LIB_PATH, SYMBOLS)
     return _lib
+
+
+def native():
+    """The native host path of the operators (csrc/snntc_torch.cpp), loaded once; raises if it has not been built."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise SnntcError("the native extension cannot be loaded (%s) -- build it with `python -m "
+                             "snntc_2023_b200.build`; there is no CPU or framework fallback" % e)
+        from . import ops
+        module.init(SnntcError, ops._params)
+        _native = module
+    return _native
 
 
 def load_measure():

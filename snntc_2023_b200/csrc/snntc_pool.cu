@@ -55,10 +55,10 @@ __global__ void minpool_fwd_kernel(const float* __restrict__ x, float* __restric
     }
     if constexpr (V == 4) {
       reinterpret_cast<float4*>(y)[o] = make_float4(best[0], best[1], best[2], best[3]);
-      reinterpret_cast<int4*>(arg)[o] = make_int4(bi[0], bi[1], bi[2], bi[3]);
+      if (arg != nullptr) reinterpret_cast<int4*>(arg)[o] = make_int4(bi[0], bi[1], bi[2], bi[3]);
     } else {
       y[o] = best[0];
-      arg[o] = bi[0];
+      if (arg != nullptr) arg[o] = bi[0];
     }
   }
 }
@@ -122,7 +122,7 @@ extern "C" {
 
 int snntc_minpool_forward(const float* x, float* y, int* arg, int B, int H, int W, int C, int Kh, int Kw,
                           int Sh, int Sw, int pad_top, int pad_left, int Nh, int Nw, float padvalue, void* stream) {
-  if (!x || !y || !arg) return SNNTC_E_NULL;
+  if (!x || !y) return SNNTC_E_NULL;   // arg: null in an evaluation, which has no backward
   if (B <= 0 || H <= 0 || W <= 0 || C <= 0 || Kh <= 0 || Kw <= 0 || Sh <= 0 || Sw <= 0 || Nh <= 0 || Nw <= 0 ||
       pad_top < 0 || pad_left < 0)
     return SNNTC_E_SHAPE;

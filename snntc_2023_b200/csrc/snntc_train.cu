@@ -9,8 +9,10 @@
 // The reference runs these as TensorFlow graph ops; nothing here has native code in the reference.
 #include "../../include/snntc_b200.h"
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math_constants.h>
+#include <stdint.h>
 
 namespace snntc { void count_launch(int n = 1); }
 
@@ -161,6 +163,280 @@ __global__ void sgdm_kernel(float* __restrict__ w, const float* __restrict__ g, 
   }
 }
 
+// ---- loss of a whole batch in one launch, no zeroed accumulators: one cluster of eight CTAs, G lanes per sample
+// (16 for up to 16 classes, else 32), every CTA's partial sums added over distributed shared memory in rank order, so
+// the loss is the same bits every run. Bound by latency (a few rounds of loads and shuffles per group): against the
+// pair of a zero fill and an atomic accumulation it takes two launches off a step.
+constexpr int kLossThreads = 512;
+constexpr int kLossCluster = 8;
+
+struct RowStats { float zmax, lse; int amin; };   // max of z = -y, sum exp(z - zmax), arg-min of y (lowest index on ties)
+
+template <int G>
+__device__ __forceinline__ RowStats row_stats(const float* __restrict__ row, int J, int gl) {
+  RowStats s;
+  s.zmax = -CUDART_INF_F;
+  s.amin = 0x7fffffff;
+  float ymin = CUDART_INF_F;
+  for (int j = gl; j < J; j += G) {
+    const float v = __ldg(row + j);
+    s.zmax = fmaxf(s.zmax, -v);
+    if (v < ymin) { ymin = v; s.amin = j; }
+  }
+#pragma unroll
+  for (int d = G / 2; d >= 1; d >>= 1) {
+    s.zmax = fmaxf(s.zmax, __shfl_xor_sync(0xffffffffu, s.zmax, d));
+    const float oy = __shfl_xor_sync(0xffffffffu, ymin, d);
+    const int oa = __shfl_xor_sync(0xffffffffu, s.amin, d);
+    if (oy < ymin || (oy == ymin && oa < s.amin)) { ymin = oy; s.amin = oa; }
+  }
+  float se = 0.f;
+  for (int j = gl; j < J; j += G) se += expf(-__ldg(row + j) - s.zmax);
+#pragma unroll
+  for (int d = G / 2; d >= 1; d >>= 1) se += __shfl_xor_sync(0xffffffffu, se, d);
+  s.lse = se;
+  return s;
+}
+
+// Sum of (a, b) over the cluster, valid in thread 0 of CTA 0: lanes, warps and CTAs in a fixed order.
+__device__ __forceinline__ float2 cluster_sum(float a, float b) {
+  namespace cg = cooperative_groups;
+  __shared__ float2 part[33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, d);
+    b += __shfl_xor_sync(0xffffffffu, b, d);
+  }
+  if (lane == 0) part[warp] = make_float2(a, b);
+  __syncthreads();
+  cg::cluster_group cl = cg::this_cluster();
+  if (threadIdx.x == 0) {
+    float2 t = part[0];
+    for (int k = 1; k < warps; ++k) { t.x += part[k].x; t.y += part[k].y; }
+    part[32] = t;
+  }
+  cl.sync();
+  float2 sum = make_float2(0.f, 0.f);
+  if (threadIdx.x == 0 && cl.block_rank() == 0)
+    for (unsigned k = 0; k < cl.num_blocks(); ++k) {
+      const float2 o = *cl.map_shared_rank(&part[32], k);
+      sum.x += o.x;
+      sum.y += o.y;
+    }
+  cl.sync();   // no CTA leaves while its shared memory may still be read
+  return sum;
+}
+
+template <int G>
+__global__ void __cluster_dims__(kLossCluster, 1, 1) __launch_bounds__(kLossThreads)
+loss_fwd_kernel(const float* __restrict__ y, const long long* __restrict__ labels, float* __restrict__ loss,
+                float* __restrict__ hits, int B, int J, float lscale) {
+  const int gl = threadIdx.x % G;
+  const int groups = kLossCluster * kLossThreads / G;
+  float loss_acc = 0.f, hit_acc = 0.f;
+  for (int b0 = 0; b0 < B; b0 += groups) {
+    const int b = b0 + (blockIdx.x * kLossThreads + threadIdx.x) / G;
+    const bool ok = b < B;                       // (shuffles run with all lanes: a group without a sample repeats the last)
+    const float* row = y + (size_t)(ok ? b : B - 1) * J;
+    const RowStats s = row_stats<G>(row, J, gl);
+    if (ok && gl == 0) {
+      const int lab = (int)labels[b];
+      // the loss is log(se) + (zmax - z[label]), never logsumexp itself, which would lose the small term beside a large
+      // |zmax| (all outputs at MAX)
+      const float zl = (lab >= 0 && lab < J) ? -__ldg(row + lab) : s.zmax;
+      loss_acc += (logf(s.lse) + (s.zmax - zl)) * lscale;
+      hit_acc += (s.amin == lab) ? 1.0f : 0.0f;
+    }
+  }
+  const float2 sum = cluster_sum(loss_acc, hit_acc);
+  if (blockIdx.x == 0 && threadIdx.x == 0) { *loss = sum.x; *hits = sum.y; }
+}
+
+// grad_y = -(softmax(-y) - onehot) * gscale * (*gloss): the softmax again from y instead of a gradient kept by the forward
+template <int G>
+__global__ void __launch_bounds__(256)
+loss_bwd_kernel(const float* __restrict__ y, const long long* __restrict__ labels, const float* __restrict__ gloss,
+                float* __restrict__ grad, int B, int J, float gscale) {
+  const int gl = threadIdx.x % G;
+  const int b = (blockIdx.x * 256 + threadIdx.x) / G;
+  const bool ok = b < B;
+  const float* row = y + (size_t)(ok ? b : B - 1) * J;
+  const RowStats s = row_stats<G>(row, J, gl);
+  if (!ok) return;
+  const int lab = (int)labels[b];
+  const float inv = 1.0f / s.lse, up = __ldg(gloss);
+  for (int j = gl; j < J; j += G) {
+    const float sm = expf(-__ldg(row + j) - s.zmax) * inv;
+    grad[(size_t)b * J + j] = -(sm - (j == lab ? 1.0f : 0.0f)) * gscale * up;
+  }
+}
+
+// ---- the weight cost of several tensors at once. A network has one small tensor per layer, and cost and gradient of
+// each used to be two memsets, two kernels and three framework operations; here all tensors share three launches.
+// Column sums go through partial sums of row slices that are added in a fixed order: no atomics, same bits every run.
+constexpr int kCostMax = 16;          // tensors per launch
+constexpr int kCostThreads = 256;
+constexpr int kCostChunk = 4096;      // elements per CTA of the gradient kernel
+
+struct CostTensors {
+  int count;
+  const float* w[kCostMax];
+  float* gw[kCostMax];
+  int rows[kCostMax], cols[kCostMax];
+  int slices[kCostMax];               // row slices of the column-sum pass
+  int first_cta[kCostMax + 1];        // of the column-sum pass: slices * blocks of kCostThreads columns
+  int first_col[kCostMax + 1];        // offset of the tensor's columns in colsum
+  int first_chunk[kCostMax + 1];      // of the gradient pass
+  long long partial[kCostMax];        // offset of the tensor's [slices][cols] partial column sums
+};
+
+__device__ __forceinline__ int tensor_of(const int* first, int count, int at) {
+  int t = 0;
+  while (t + 1 < count && at >= first[t + 1]) ++t;
+  return t;
+}
+
+// CTA = (tensor, block of up to 256 columns, slice of the rows): a thread owns one column and every (256 / columns)-th
+// row of the slice, eight loads in flight; the threads of a column are added through shared memory.
+__global__ void __launch_bounds__(kCostThreads)
+cost_sums_kernel(const __grid_constant__ CostTensors c, float* __restrict__ partial, float* __restrict__ sq) {
+  __shared__ float part[kCostThreads];
+  const int t = tensor_of(c.first_cta, c.count, blockIdx.x);
+  const int local = blockIdx.x - c.first_cta[t];
+  const int rows = c.rows[t], J = c.cols[t], slices = c.slices[t];
+  const int slice = local % slices, j0 = (local / slices) * kCostThreads;
+  const int width = min(kCostThreads, J - j0);
+  const int lines = kCostThreads / width;            // rows in step
+  const int line = threadIdx.x / width, col = threadIdx.x % width;
+  const int per = (rows + slices - 1) / slices;
+  const int r0 = slice * per, r1 = min(rows, r0 + per);
+  const float* w = c.w[t] + j0 + col;
+  float s = 0.f, s2 = 0.f;
+  if (line < lines) {
+    int r = r0 + line;
+    for (; r + 7 * lines < r1; r += 8 * lines) {
+      float v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = __ldg(w + (size_t)(r + q * lines) * J);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) { s += v[q]; s2 = fmaf(v[q], v[q], s2); }
+    }
+    for (; r < r1; r += lines) {
+      const float v = __ldg(w + (size_t)r * J);
+      s += v;
+      s2 = fmaf(v, v, s2);
+    }
+  }
+  part[threadIdx.x] = s;
+  __syncthreads();
+  if (line == 0) {
+    for (int k = 1; k < lines; ++k) s += part[k * width + col];
+    partial[c.partial[t] + (long long)slice * J + j0 + col] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, d);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s2;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < kCostThreads / 32; ++k) s2 += part[k];
+    sq[blockIdx.x] = s2;
+  }
+}
+
+// One cluster: column sums out of the partial ones, and the cost of all tensors (added to *cost when `add` is set).
+__global__ void __cluster_dims__(kLossCluster, 1, 1) __launch_bounds__(kLossThreads)
+cost_total_kernel(const __grid_constant__ CostTensors c, const float* __restrict__ partial, const float* __restrict__ sq,
+                  float* __restrict__ colsum, float* __restrict__ cost, float K, float K2, int add) {
+  const int me = blockIdx.x * kLossThreads + threadIdx.x;
+  constexpr int kAll = kLossCluster * kLossThreads;
+  float total = 0.f;
+  for (int col = me; col < c.first_col[c.count]; col += kAll) {
+    const int t = tensor_of(c.first_col, c.count, col);
+    const int J = c.cols[t];
+    const float* p = partial + c.partial[t] + (col - c.first_col[t]);
+    float s = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < c.slices[t]; ++k) s += __ldg(p + (long long)k * J);
+    colsum[col] = s;
+    total += fmaxf(0.f, 1.0f - s) * (K / (float)J);
+  }
+  for (int k = me; k < c.first_cta[c.count]; k += kAll) {
+    const int t = tensor_of(c.first_cta, c.count, k);
+    total += __ldg(sq + k) * (K2 / ((float)c.rows[t] * (float)c.cols[t]));
+  }
+  const float2 sum = cluster_sum(total, 0.f);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *cost = add ? *cost + sum.x : sum.x;
+}
+
+// gw = gcost * (-K/J [colsum < 1] + 2 K2 / n * w), a CTA per 4096 elements of one tensor
+__global__ void __launch_bounds__(kCostThreads)
+cost_grad_kernel(const __grid_constant__ CostTensors c, const float* __restrict__ colsum, const float* __restrict__ gcost,
+                 float K, float K2) {
+  const int t = tensor_of(c.first_chunk, c.count, blockIdx.x);
+  const int J = c.cols[t];
+  const unsigned n = (unsigned)c.rows[t] * (unsigned)J;
+  const unsigned e0 = (unsigned)(blockIdx.x - c.first_chunk[t]) * kCostChunk;
+  const unsigned e1 = min(n, e0 + kCostChunk);
+  const float up = __ldg(gcost);
+  const float a = -K / (float)J, b2 = 2.0f * K2 / (float)n;
+  const float* cs = colsum + c.first_col[t];
+  const float* w = c.w[t];
+  float* gw = c.gw[t];
+  if ((J & 3) == 0 && (((uintptr_t)w | (uintptr_t)gw) & 15) == 0) {
+    for (unsigned e = e0 + 4 * threadIdx.x; e < e1; e += 4 * kCostThreads) {
+      const unsigned j = e % (unsigned)J;
+      const float4 v = __ldg(reinterpret_cast<const float4*>(w + e));
+      float4 r;
+      r.x = ((1.0f - __ldg(cs + j)) > 0.f ? a : 0.f) + b2 * v.x;
+      r.y = ((1.0f - __ldg(cs + j + 1)) > 0.f ? a : 0.f) + b2 * v.y;
+      r.z = ((1.0f - __ldg(cs + j + 2)) > 0.f ? a : 0.f) + b2 * v.z;
+      r.w = ((1.0f - __ldg(cs + j + 3)) > 0.f ? a : 0.f) + b2 * v.w;
+      *reinterpret_cast<float4*>(gw + e) = make_float4(up * r.x, up * r.y, up * r.z, up * r.w);
+    }
+  } else {
+    for (unsigned e = e0 + threadIdx.x; e < e1; e += kCostThreads)
+      gw[e] = up * (((1.0f - __ldg(cs + e % (unsigned)J)) > 0.f ? a : 0.f) + b2 * __ldg(w + e));
+  }
+}
+
+// Tensors [at, at + 16) of a list; the column sums of the earlier ones take the first `cols_before` floats of colsum.
+// Row slices: about 64 rows each, at most 128, so that a large tensor spreads over the GPU.
+CostTensors cost_tensors(int count, const float* const* w, float* const* gw, const int* rows, const int* cols, int at) {
+  CostTensors c;
+  c.count = count - at < kCostMax ? count - at : kCostMax;
+  int cta = 0, col = 0, chunk = 0;
+  long long partial = 0;
+  for (int k = 0; k < c.count; ++k) {
+    const int r = rows[at + k], J = cols[at + k];
+    c.w[k] = w ? w[at + k] : nullptr;
+    c.gw[k] = gw ? gw[at + k] : nullptr;
+    c.rows[k] = r;
+    c.cols[k] = J;
+    int slices = (r + 63) / 64;
+    if (slices > 128) slices = 128;
+    c.slices[k] = slices;
+    c.first_cta[k] = cta;
+    c.first_col[k] = col;
+    c.first_chunk[k] = chunk;
+    c.partial[k] = partial;
+    cta += slices * ((J + kCostThreads - 1) / kCostThreads);
+    col += J;
+    chunk += (int)(((long long)r * J + kCostChunk - 1) / kCostChunk);
+    partial += (long long)slices * J;
+  }
+  c.first_cta[c.count] = cta;
+  c.first_col[c.count] = col;
+  c.first_chunk[c.count] = chunk;
+  return c;
+}
+size_t cost_partial_floats(const CostTensors& c) {
+  size_t n = 0;
+  for (int k = 0; k < c.count; ++k) n += (size_t)c.slices[k] * c.cols[k];
+  return n;
+}
+
 int done() {
   snntc::count_launch();
   return cudaGetLastError() == cudaSuccess ? SNNTC_OK : SNNTC_E_CUDA;
@@ -184,6 +460,79 @@ int snntc_loss_ce(const float* y, const long long* labels, float* grad, float* s
   loss_ce_kernel<<<grid_for((size_t)B * 32), 256, 0, (cudaStream_t)stream>>>(y, labels, grad, sums2, B, J, loss_scale,
                                                                             grad_scale);
   return done();
+}
+
+int snntc_loss_forward(const float* y, const long long* labels, float* loss, float* hits, int B, int J, float loss_scale,
+                       void* stream) {
+  if (!y || !labels || !loss || !hits) return SNNTC_E_NULL;
+  if (B <= 0 || J <= 0) return SNNTC_E_SHAPE;
+  if (J <= 16) loss_fwd_kernel<16><<<kLossCluster, kLossThreads, 0, (cudaStream_t)stream>>>(y, labels, loss, hits, B, J, loss_scale);
+  else loss_fwd_kernel<32><<<kLossCluster, kLossThreads, 0, (cudaStream_t)stream>>>(y, labels, loss, hits, B, J, loss_scale);
+  return done();
+}
+
+int snntc_loss_backward(const float* y, const long long* labels, const float* gloss, float* grad, int B, int J,
+                        float grad_scale, void* stream) {
+  if (!y || !labels || !gloss || !grad) return SNNTC_E_NULL;
+  if (B <= 0 || J <= 0) return SNNTC_E_SHAPE;
+  const int G = J <= 16 ? 16 : 32;
+  const int grid = (int)(((long long)B * G + 255) / 256);
+  if (G == 16) loss_bwd_kernel<16><<<grid, 256, 0, (cudaStream_t)stream>>>(y, labels, gloss, grad, B, J, grad_scale);
+  else loss_bwd_kernel<32><<<grid, 256, 0, (cudaStream_t)stream>>>(y, labels, gloss, grad, B, J, grad_scale);
+  return done();
+}
+
+size_t snntc_weight_costs_workspace_bytes(int count, const int* rows, const int* cols) {
+  if (count <= 0 || !rows || !cols) return 0;
+  size_t most = 0;
+  for (int at = 0; at < count; at += kCostMax) {
+    const CostTensors c = cost_tensors(count, nullptr, nullptr, rows, cols, at);
+    const size_t n = cost_partial_floats(c) + (size_t)c.first_cta[c.count];
+    if (n > most) most = n;
+  }
+  return most * sizeof(float);
+}
+
+int snntc_weight_costs(int count, const float* const* w, const int* rows, const int* cols, float K, float K2, float* colsum,
+                       float* cost, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!w || !rows || !cols || !colsum || !cost || !workspace) return SNNTC_E_NULL;
+  if (count <= 0) return SNNTC_E_SHAPE;
+  for (int k = 0; k < count; ++k) {
+    if (!w[k]) return SNNTC_E_NULL;
+    if (rows[k] <= 0 || cols[k] <= 0) return SNNTC_E_SHAPE;
+    if ((long long)rows[k] * cols[k] > 0x7fffffffLL) return SNNTC_E_TOO_LARGE;
+  }
+  if (workspace_bytes < snntc_weight_costs_workspace_bytes(count, rows, cols)) return SNNTC_E_WORKSPACE;
+  cudaStream_t s = (cudaStream_t)stream;
+  for (int at = 0; at < count; at += kCostMax) {
+    const CostTensors c = cost_tensors(count, w, nullptr, rows, cols, at);
+    float* partial = static_cast<float*>(workspace);
+    float* sq = partial + cost_partial_floats(c);
+    cost_sums_kernel<<<c.first_cta[c.count], kCostThreads, 0, s>>>(c, partial, sq);
+    if (done() != SNNTC_OK) return SNNTC_E_CUDA;
+    cost_total_kernel<<<kLossCluster, kLossThreads, 0, s>>>(c, partial, sq, colsum, cost, K, K2, at > 0);
+    if (done() != SNNTC_OK) return SNNTC_E_CUDA;
+    colsum += c.first_col[c.count];
+  }
+  return SNNTC_OK;
+}
+
+int snntc_weight_cost_grads(int count, const float* const* w, float* const* gw, const int* rows, const int* cols, float K,
+                            float K2, const float* colsum, const float* gcost, void* stream) {
+  if (!w || !gw || !rows || !cols || !colsum || !gcost) return SNNTC_E_NULL;
+  if (count <= 0) return SNNTC_E_SHAPE;
+  for (int k = 0; k < count; ++k) {
+    if (!w[k] || !gw[k]) return SNNTC_E_NULL;
+    if (rows[k] <= 0 || cols[k] <= 0) return SNNTC_E_SHAPE;
+    if ((long long)rows[k] * cols[k] > 0x7fffffffLL) return SNNTC_E_TOO_LARGE;
+  }
+  for (int at = 0; at < count; at += kCostMax) {
+    const CostTensors c = cost_tensors(count, w, gw, rows, cols, at);
+    cost_grad_kernel<<<c.first_chunk[c.count], kCostThreads, 0, (cudaStream_t)stream>>>(c, colsum, gcost, K, K2);
+    if (done() != SNNTC_OK) return SNNTC_E_CUDA;
+    colsum += c.first_col[c.count];
+  }
+  return SNNTC_OK;
 }
 
 size_t snntc_weight_cost_workspace_bytes(int J) { return ((size_t)J + 1) * sizeof(float); }

@@ -139,7 +139,8 @@ class SnnNet(torch.nn.Module):
         for l in ws:
             l.weight.grad = None
         objective.backward()
+        more = [l for l in ws if l.weight.grad is not None]
+        if more:   # one launch for all layers
+            torch._foreach_add_([l.grad_sink for l in more], [l.weight.grad for l in more])
         for l in ws:
-            if l.weight.grad is not None:
-                l.grad_sink.add_(l.weight.grad)
             l.weight.grad = l.grad_sink

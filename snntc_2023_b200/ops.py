@@ -13,9 +13,13 @@ Names, argument order and packed layouts follow the reference's TensorFlow ops
 the `*_layer` forms, which take the UNPADDED image plus padding amounts and return only the spike
 values, so neither a padded copy nor the packed second half ever goes through autograd.
 
-torch is used for device memory and streams only; all arithmetic is in the CUDA library. There is no
-CPU path: a CPU tensor raises.
+torch is used for device memory, streams and autograd plumbing only; all arithmetic is in the CUDA library. The checks,
+allocations, autograd nodes and C-ABI calls of an operator are one call of the native extension (csrc/snntc_torch.cpp);
+the measurement build, the causal-set histogram and the replay tap are reached through ctypes. There is no CPU path: a
+CPU tensor raises.
 """
+import math
+
 import numpy as np
 import torch
 
@@ -30,12 +34,16 @@ TAP = None
 
 
 # ------------------------------------------------------------------------------------------ helpers
+def _tensor(t, name):
+    if isinstance(t, torch.Tensor):
+        return t
+    if hasattr(t, "__dlpack__"):
+        return torch.from_dlpack(t)
+    raise TypeError("%s must be a torch tensor or a DLPack-capable CUDA array" % name)
+
+
 def _as_cuda_f32(t, name):
-    if not isinstance(t, torch.Tensor):
-        if hasattr(t, "__dlpack__"):
-            t = torch.from_dlpack(t)
-        else:
-            raise TypeError("%s must be a torch tensor or a DLPack-capable CUDA array" % name)
+    t = _tensor(t, name)
     if not t.is_cuda:
         raise _lib.SnntcError("%s is not on a CUDA device: the SNN-TC operators have no CPU implementation" % name)
     if t.dtype != torch.float32:
@@ -76,7 +84,6 @@ def conv_geometry(H, W, Kh, Kw, Sh, Sw, padding):
     """(pad_top, pad_left, Nh, Nw) of SNN_conv: SAME pads with MAX by
     total=(ceil(H/S)-1)*S+K-H, before=total//2; VALID drops trailing rows/columns
     (SNN_TC_Modules.py:147-166)."""
-    import math
     if str(padding).upper() == "SAME":
         th = (math.ceil(H / Sh) - 1) * Sh + Kh - H
         tw = (math.ceil(W / Sw) - 1) * Sw + Kw - W
@@ -92,6 +99,8 @@ def conv_geometry(H, W, Kh, Kw, Sh, Sw, padding):
 # `opts` (an opts8 vector from _lib.options) selects kernels explicitly through the measurement build of the
 # library; `workspace` lets a caller keep the scratch between two calls (lists built by one, walked by the next).
 def snn_fc(inp, weight, params, opts=None, workspace=None, out=None):
+    if opts is None and workspace is None and out is None:
+        return _lib.native().fc_forward(_tensor(inp, "in"), _tensor(weight, "weight"), params, False)
     x = _as_cuda_f32(inp, "in"); w = _as_cuda_f32(weight, "weight"); p = _params(params, 6)
     if x.dim() != 2 or w.dim() != 2:
         raise ValueError("snn_fc expects in[B,I] and weight[rows,J]")
@@ -121,6 +130,8 @@ def fc_forward_workspace(B, I, J, device):
 def snn_fc_infer(inp, weight, params, khist=None):
     """Spike values only, [B,J]: SnnFc without the 1/(sum w - theta) half (snntc_fc_infer). `khist`: an int32
     CUDA tensor of I+2 zeros (I without the bias row) that receives the histogram of causal-set sizes."""
+    if khist is None:
+        return _lib.native().fc_forward(_tensor(inp, "in"), _tensor(weight, "weight"), params, True)
     lib = _lib.load()
     x = _as_cuda_f32(inp, "in"); w = _as_cuda_f32(weight, "weight"); p = _params(params, 6)
     if x.dim() != 2 or w.dim() != 2:
@@ -140,6 +151,9 @@ def snn_fc_infer(inp, weight, params, khist=None):
 
 def snn_fc_grad(grad, inp, weight, params, oldout, need_input_grad=True, grad_weight_out=None, opts=None):
     """grad may be the packed [2B,J] tensor or just its first B rows (only those are read)."""
+    if opts is None:
+        return _lib.native().fc_grad(_tensor(grad, "grad"), _tensor(inp, "in"), _tensor(weight, "weight"), params,
+                                     _tensor(oldout, "oldout"), bool(need_input_grad), grad_weight_out)
     g = _as_cuda_f32(grad, "grad"); x = _as_cuda_f32(inp, "in"); w = _as_cuda_f32(weight, "weight")
     y = _as_cuda_f32(oldout, "oldout"); p = _params(params, 6)
     B, I = x.shape
@@ -148,19 +162,15 @@ def snn_fc_grad(grad, inp, weight, params, oldout, need_input_grad=True, grad_we
         raise ValueError("snn_fc_grad: oldout must be [2B,J]")
     if g.shape[0] not in (B, 2 * B) or g.shape[1] != J:
         raise ValueError("snn_fc_grad: Grad/Oldout batch should be 2 * batch")
-    lib = _lib.load() if opts is None else _lib.load_measure()
+    lib = _lib.load_measure()
     with torch.cuda.device(x.device):
         dx = torch.empty_like(x) if need_input_grad else None
         dw = grad_weight_out if grad_weight_out is not None else torch.empty_like(w)
         dp = torch.empty(6, dtype=torch.float32, device=x.device)
         ws, wsb = _workspace(lib.snntc_fc_backward_workspace_bytes(B, I, rows, J), x.device)
-        if opts is None:
-            rc = lib.snntc_fc_backward(g.data_ptr(), x.data_ptr(), w.data_ptr(), p.ctypes.data, y.data_ptr(),
-                                       _ptr(dx), dw.data_ptr(), dp.data_ptr(), B, I, rows, J, _ptr(ws), wsb, _stream(x))
-        else:
-            rc = lib.snntc_measure_fc_backward(g.data_ptr(), x.data_ptr(), w.data_ptr(), p.ctypes.data, y.data_ptr(),
-                                               _ptr(dx), dw.data_ptr(), dp.data_ptr(), B, I, rows, J, _ptr(ws), wsb,
-                                               _opts_ptr(opts), _stream(x))
+        rc = lib.snntc_measure_fc_backward(g.data_ptr(), x.data_ptr(), w.data_ptr(), p.ctypes.data, y.data_ptr(),
+                                           _ptr(dx), dw.data_ptr(), dp.data_ptr(), B, I, rows, J, _ptr(ws), wsb,
+                                           _opts_ptr(opts), _stream(x))
     _lib.check(rc, "SnnFcGrad")
     return dx, dw, dp
 
@@ -181,6 +191,9 @@ def _cv_dims(x, w, p, pad_top, pad_left, Nh, Nw):
 def snn_cv(inp, weight, params, pad_top=0, pad_left=0, Nh=None, Nw=None, opts=None, workspace=None, out=None):
     """With the default pad arguments this is the reference op: `inp` is the tensor SNN_conv.call has
     already padded with MAX (SAME) or cropped (VALID)."""
+    if opts is None and workspace is None and out is None:
+        return _lib.native().cv_forward(_tensor(inp, "in"), _tensor(weight, "weight"), params, pad_top, pad_left,
+                                        -1 if Nh is None else Nh, -1 if Nh is None else Nw, False)
     x = _as_cuda_f32(inp, "in"); w = _as_cuda_f32(weight, "weight"); p = _params(params, 12)
     B, H, W, C, rows, Kc, Kh, Kw, pt, pl, Nh, Nw = _cv_dims(x, w, p, pad_top, pad_left, Nh, Nw)
     if Nh <= 0 or Nw <= 0:
@@ -212,6 +225,9 @@ def cv_forward_workspace(x, weight, params, Nh, Nw):
 def snn_cv_infer(inp, weight, params, pad_top=0, pad_left=0, Nh=None, Nw=None, khist=None):
     """Spike values only, [B,Nh,Nw,Kc]: SnnCv without the 1/(sum w - theta) half (snntc_cv_infer). `khist`: an
     int32 CUDA tensor of Kh*Kw*C+2 zeros that receives the histogram of causal-set sizes."""
+    if khist is None:
+        return _lib.native().cv_forward(_tensor(inp, "in"), _tensor(weight, "weight"), params, pad_top, pad_left,
+                                        -1 if Nh is None else Nh, -1 if Nh is None else Nw, True)
     lib = _lib.load()
     x = _as_cuda_f32(inp, "in"); w = _as_cuda_f32(weight, "weight"); p = _params(params, 12)
     B, H, W, C, rows, Kc, Kh, Kw, pt, pl, Nh, Nw = _cv_dims(x, w, p, pad_top, pad_left, Nh, Nw)
@@ -230,6 +246,9 @@ def snn_cv_infer(inp, weight, params, pad_top=0, pad_left=0, Nh=None, Nw=None, k
 
 def snn_cv_grad(grad, inp, weight, params, oldout, pad_top=0, pad_left=0, need_input_grad=True,
                 grad_weight_out=None, opts=None):
+    if opts is None:
+        return _lib.native().cv_grad(_tensor(grad, "grad"), _tensor(inp, "in"), _tensor(weight, "weight"), params,
+                                     _tensor(oldout, "oldout"), pad_top, pad_left, bool(need_input_grad), grad_weight_out)
     g = _as_cuda_f32(grad, "grad"); x = _as_cuda_f32(inp, "in"); w = _as_cuda_f32(weight, "weight")
     y = _as_cuda_f32(oldout, "oldout"); p = _params(params, 12)
     if y.dim() != 4:
@@ -239,73 +258,37 @@ def snn_cv_grad(grad, inp, weight, params, oldout, pad_top=0, pad_left=0, need_i
         raise ValueError("snn_cv_grad: oldout must be [2B,Nh,Nw,Kc]")
     if g.shape[0] not in (B, 2 * B) or tuple(g.shape[1:]) != tuple(y.shape[1:]):
         raise ValueError("snn_cv_grad: Grad/Oldout batch should be 2 * batch")
-    lib = _lib.load() if opts is None else _lib.load_measure()
+    lib = _lib.load_measure()
     with torch.cuda.device(x.device):
         dx = torch.empty_like(x) if need_input_grad else None
         dw = grad_weight_out if grad_weight_out is not None else torch.empty_like(w)
         dp = torch.empty(12, dtype=torch.float32, device=x.device)
         ws, wsb = _workspace(lib.snntc_cv_backward_workspace_bytes(B, H, W, C, rows, Kc, Nh, Nw), x.device)
-        if opts is None:
-            rc = lib.snntc_cv_backward(g.data_ptr(), x.data_ptr(), w.data_ptr(), p.ctypes.data, y.data_ptr(),
-                                       _ptr(dx), dw.data_ptr(), dp.data_ptr(), B, H, W, C, rows, Kc, pt, pl, Nh, Nw,
-                                       _ptr(ws), wsb, _stream(x))
-        else:
-            rc = lib.snntc_measure_cv_backward(g.data_ptr(), x.data_ptr(), w.data_ptr(), p.ctypes.data, y.data_ptr(),
-                                               _ptr(dx), dw.data_ptr(), dp.data_ptr(), B, H, W, C, rows, Kc, pt, pl,
-                                               Nh, Nw, _ptr(ws), wsb, _opts_ptr(opts), _stream(x))
+        rc = lib.snntc_measure_cv_backward(g.data_ptr(), x.data_ptr(), w.data_ptr(), p.ctypes.data, y.data_ptr(),
+                                           _ptr(dx), dw.data_ptr(), dp.data_ptr(), B, H, W, C, rows, Kc, pt, pl,
+                                           Nh, Nw, _ptr(ws), wsb, _opts_ptr(opts), _stream(x))
     _lib.check(rc, "SnnCvGrad")
     return dx, dw, dp
 
 
 # ------------------------------------------------------------------------------------------ autograd
-class _SnnFc(torch.autograd.Function):
-    """Differentiable SnnFc with the reference's packed [2B,J] output."""
-
-    @staticmethod
-    def forward(ctx, X, W, params):
-        out = snn_fc(X, W, params)
-        ctx.params = _params(params, 6)
-        ctx.save_for_backward(X, W, out)
-        return out
-
-    @staticmethod
-    def backward(ctx, grad):
-        X, W, out = ctx.saved_tensors
-        dx, dw, _ = snn_fc_grad(grad, X, W, ctx.params, out, need_input_grad=ctx.needs_input_grad[0])
-        return dx, dw, None
-
-
-class _SnnCv(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, X, W, params):
-        out = snn_cv(X, W, params)
-        ctx.params = _params(params, 12)
-        ctx.save_for_backward(X, W, out)
-        return out
-
-    @staticmethod
-    def backward(ctx, grad):
-        X, W, out = ctx.saved_tensors
-        dx, dw, _ = snn_cv_grad(grad, X, W, ctx.params, out, need_input_grad=ctx.needs_input_grad[0])
-        return dx, dw, None
-
-
 def snnfc(X, W, params):
-    return _SnnFc.apply(X, W, params)
+    """Differentiable SnnFc with the reference's packed [2B,J] output."""
+    return _lib.native().fc_op(_tensor(X, "in"), _tensor(W, "weight"), params)
 
 
 def snncv(X, W, params):
-    return _SnnCv.apply(X, W, params)
+    return _lib.native().cv_op(_tensor(X, "in"), _tensor(W, "weight"), params)
 
 
 snnfc_grad = snn_fc_grad
 snncv_grad = snn_cv_grad
 
 
+# The layer forms return the spike values only. `sink` (optional) is where dW is written instead of being handed to
+# autograd -- a slice of the flat gradient bucket that the all-reduce works on. These two Python nodes run while TAP is
+# set; otherwise the native extension's do the same.
 class _SnnFcLayer(torch.autograd.Function):
-    """Layer form: returns y[B,J] only. `sink` (optional) is where dW is written instead of being
-    handed to autograd -- a slice of the flat gradient bucket that the all-reduce works on."""
-
     @staticmethod
     def forward(ctx, X, W, params, sink):
         out = snn_fc(X, W, params)
@@ -351,60 +334,27 @@ class _SnnCvLayer(torch.autograd.Function):
         return dx, (None if ctx.sink is not None else dw), None, None, None
 
 
-def _no_grad_needed(X, W):
-    return not (torch.is_grad_enabled() and (X.requires_grad or W.requires_grad))
-
-
 def snn_fc_layer(X, W, params, grad_sink=None):
-    if _no_grad_needed(X, W):   # evaluation: nothing will read 1/(sum w - theta)
-        return snn_fc_infer(X, W, params)
-    return _SnnFcLayer.apply(X, W, params, grad_sink)
+    """y[B,J] of a dense layer; without the half that only a backward reads when nothing asks for a gradient."""
+    if TAP is not None and torch.is_grad_enabled() and (X.requires_grad or W.requires_grad):
+        return _SnnFcLayer.apply(X, W, params, grad_sink)
+    return _lib.native().fc_layer(_tensor(X, "in"), W, params, grad_sink)
 
 
 def snn_cv_layer(X, W, params, geom, grad_sink=None):
-    if _no_grad_needed(X, W):
-        pt, pl, Nh, Nw = geom
-        return snn_cv_infer(X, W, params, pt, pl, Nh, Nw)
-    return _SnnCvLayer.apply(X, W, params, geom, grad_sink)
+    if TAP is not None and torch.is_grad_enabled() and (X.requires_grad or W.requires_grad):
+        return _SnnCvLayer.apply(X, W, params, geom, grad_sink)
+    return _lib.native().cv_layer(_tensor(X, "in"), W, params, *geom, grad_sink)
 
 
 # ------------------------------------------------------------------------------------------ pooling
-class _MinPool(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, X, Kh, Kw, Sh, Sw, padding, padvalue):
-        lib = _lib.load()
-        x = _as_cuda_f32(X, "input")
-        B, H, W, C = x.shape
-        if str(padding).upper() == "SAME":
-            pt, pl, Nh, Nw = conv_geometry(H, W, Kh, Kw, Sh, Sw, "SAME")
-        else:
-            pt = pl = 0
-            Nh, Nw = (H - Kh) // Sh + 1, (W - Kw) // Sw + 1
-        with torch.cuda.device(x.device):
-            y = torch.empty((B, Nh, Nw, C), dtype=torch.float32, device=x.device)
-            arg = torch.empty((B, Nh, Nw, C), dtype=torch.int32, device=x.device)
-            rc = lib.snntc_minpool_forward(x.data_ptr(), y.data_ptr(), arg.data_ptr(), B, H, W, C, Kh, Kw, Sh, Sw,
-                                           pt, pl, Nh, Nw, float(padvalue), _stream(x))
-        _lib.check(rc, "minpool forward")
-        ctx.save_for_backward(arg)
-        ctx.in_shape = tuple(x.shape)
-        ctx.window = (Kh, Kw, Sh, Sw, pt, pl, Nh, Nw)
-        return y
-
-    @staticmethod
-    def backward(ctx, gy):
-        lib = _lib.load()
-        (arg,) = ctx.saved_tensors
-        gy = gy.contiguous()
-        with torch.cuda.device(gy.device):
-            dx = torch.empty(ctx.in_shape, dtype=torch.float32, device=gy.device)
-            B, H, W, C = ctx.in_shape
-            rc = lib.snntc_minpool_backward(gy.data_ptr(), arg.data_ptr(), dx.data_ptr(), B, H, W, C, *ctx.window,
-                                            _stream(gy))
-        _lib.check(rc, "minpool backward")
-        return dx, None, None, None, None, None, None
-
-
 def snn_minpool(X, Kh, Kw, Sh, Sw, padding="SAME", padvalue=1e5):
     """Window minimum with `padvalue` outside the image (SNN_maxpool2d of the reference)."""
-    return _MinPool.apply(X, Kh, Kw, Sh, Sw, padding, padvalue)
+    X = _tensor(X, "input")
+    _, H, W, _ = X.shape
+    if str(padding).upper() == "SAME":
+        pt, pl, Nh, Nw = conv_geometry(H, W, Kh, Kw, Sh, Sw, "SAME")
+    else:
+        pt = pl = 0
+        Nh, Nw = (H - Kh) // Sh + 1, (W - Kw) // Sw + 1
+    return _lib.native().minpool(X, Kh, Kw, Sh, Sw, pt, pl, Nh, Nw, float(padvalue))
