@@ -14,6 +14,7 @@
 
 #include <math_constants.h>
 #include <math.h>
+#include <algorithm>
 #include <type_traits>
 
 namespace snntc {
@@ -33,8 +34,10 @@ constexpr int kTileI = 128;     // dW output tile: 128 fan-in rows x 64 outputs,
 // snn_dw_kernel): *exact_flag is raised when some value lies outside the range in which scaling by a power
 // of two is exact and (y - x) * scale stays below 1 -- an input below -MAX, a non-zero input or spike value
 // smaller than 2^-60 in magnitude, or a u that is not below 2^100 in magnitude (NaN and inf included).
-// `xin` is the whole input tensor (nx elements). The flag must be zero before the launch.
-template <bool V4>   // V4: n and nx are multiples of 4 and all pointers 16-byte aligned: 16-byte loads and stores
+// `xin` is the whole input tensor (nx elements). The flag must be zero before the launch, unless BLOCK_FLAGS is set: then
+// every block writes a flag of its own (exact_flag[blockIdx.x]) that the consumer combines, which saves the memset in
+// front of the two launches a small dense layer's backward consists of.
+template <bool V4, bool BLOCK_FLAGS>   // V4: n and nx are multiples of 4 and all pointers 16-byte aligned: 16-byte loads and stores
 __global__ void snn_u_kernel(const float* __restrict__ grad, const float* __restrict__ out, float* __restrict__ u,
                              size_t n, float maxcomp, const float* __restrict__ xin, size_t nx, float maxv,
                              int* __restrict__ exact_flag, unsigned* __restrict__ nz_count) {
@@ -72,6 +75,11 @@ __global__ void snn_u_kernel(const float* __restrict__ grad, const float* __rest
   } else {
     for (size_t e = t0; e < n; e += stride) u[e] = one(__ldg(out + e), __ldg(grad + e), __ldg(out + n + e));
     for (size_t e = t0; e < nx; e += stride) scan(__ldg(xin + e));
+  }
+  if constexpr (BLOCK_FLAGS) {
+    const int any = __syncthreads_or(odd);
+    if (threadIdx.x == 0) exact_flag[blockIdx.x] = any;
+    return;
   }
   if (odd) *exact_flag = 1;
   if (nz_count != nullptr) {   // one atomic per warp: *nz_count = number of outputs with a gradient (zero before the launch)
@@ -835,6 +843,7 @@ DwPlan plan_dw(const Geometry& g, const LaunchInfo& li) {
 
 static size_t u_bytes(const Geometry& g) { return (((size_t)g.R * g.J * sizeof(float)) + 255) & ~(size_t)255; }
 constexpr size_t kFlagBytes = 256;
+constexpr int kFlagBlocks = (int)(kFlagBytes / sizeof(int));   // most blocks of the u kernel that write a flag each
 
 // The power of two s with 2*MAX*s <= 1/2 (so that (y - x)*s < 1 whenever y <= MAX and x >= -MAX), or 1 when
 // MAX or the bias input are outside the range in which the scaled inner loop of the dW kernels is exact: with
@@ -851,19 +860,23 @@ static float dw_scale(const Geometry& g) {
   return ldexpf(1.0f, -(e + 2));  // 2*maxv*s < 2^(e+1) * 2^-(e+2) = 1/2
 }
 
-// Where the row-skipping dW kernel is used: conv layers it supports with enough rows and fan-in to fill its tiles.
+// Where the row-skipping dW kernel is used: conv layers it supports with enough fan-in to fill its tiles. From 64 rows
+// on: it is never slower than the dense tile there (within a microsecond at 64 rows of 2305 x 256; 100 against 63 us at
+// 1024 rows), because it skips what carries no gradient and splits the rows finely.
 static bool want_dw_skip(const Geometry& g, const Options& opt) {
   if (opt.dw_kernel == 1) return false;
   if (!g.is_conv || (g.C & 3) != 0 || (g.J & 3) != 0) return false;
   if (opt.dw_kernel >= 2) return true;
-  return g.R >= 2048 && g.I >= 128;
+  return g.R >= 64 && g.I >= 128;
 }
 
 // Where the sparse dX kernel is used: conv layers it supports with enough receptive fields to be worth three launches.
+// The dense tile needs taps * J / 16 rounds of about 2.5 us one after the other however few pixels there are (380 us for
+// 64 fields of 1152 x 256), the lists spread over a warp per pixel (50 us).
 static bool want_dx_sparse(const Geometry& g, const Options& opt) {
   if (opt.dx_kernel == 1 || !dx_sparse_shape_ok(g)) return false;
   if (opt.dx_kernel == 2) return true;
-  return g.R >= 2048 && g.J >= 32;
+  return g.R >= 64 && g.J >= 16;
 }
 
 // workspace = u[R,J] | 256 bytes with the range flag of snn_u_kernel | the partial dW planes (sized for whichever dW
@@ -915,6 +928,21 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
   // 16-byte tile loads need J % 4 == 0 and 16-byte aligned bases (rows then start aligned too)
   const bool vec = (g.J % 4 == 0) && (((uintptr_t)out | (uintptr_t)w | (uintptr_t)uv) & 15) == 0 &&
                    (((size_t)g.R * g.J) % 4 == 0);
+  if (dense_bwd_supported(g) && opt.dx_kernel == 0 && opt.dw_kernel == 0) {
+    // u and one range flag per block of the u kernel (at most 64: a quarter of a megabyte per block at the largest sizes
+    // this path takes is still a few microseconds), then both gradients in one launch
+    const size_t n = (size_t)g.R * g.J, nx = (size_t)g.R * g.I;
+    size_t blocks = (std::max(n, nx) / 4 + 255) / 256;
+    if (blocks > kFlagBlocks) blocks = kFlagBlocks;
+    if (blocks < 1) blocks = 1;
+    const bool v4 = (n % 4 == 0) && (nx % 4 == 0) && (((uintptr_t)grad | (uintptr_t)out | (uintptr_t)uv | (uintptr_t)x) & 15) == 0;
+    if (v4) snn_u_kernel<true, true><<<(int)blocks, 1024, 0, s>>>(grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nullptr);
+    else snn_u_kernel<false, true><<<(int)blocks, 1024, 0, s>>>(grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nullptr);
+    count_launch();
+    if (cudaGetLastError() != cudaSuccess) return E_CUDA;
+    return launch_dense_bwd(g, uv, x, w, out, (parts & 1) ? dx : nullptr, (parts & 2) ? dw : nullptr, dw_scale(g), exact_flag,
+                            (int)blocks, li, s);
+  }
   {
     const size_t n = (size_t)g.R * g.J;
     size_t blocks = (n + 255) / 256;
@@ -923,8 +951,8 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
     const size_t nx = g.is_conv ? (size_t)g.B * g.H * g.W * g.C : (size_t)g.R * g.I;
     const bool v4 = (n % 4 == 0) && (nx % 4 == 0) &&
                     (((uintptr_t)grad | (uintptr_t)out | (uintptr_t)uv | (uintptr_t)x) & 15) == 0;
-    if (v4) snn_u_kernel<true><<<(int)blocks, 256, 0, s>>>(grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nz_count);
-    else snn_u_kernel<false><<<(int)blocks, 256, 0, s>>>(grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nz_count);
+    if (v4) snn_u_kernel<true, false><<<(int)blocks, 256, 0, s>>>(grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nz_count);
+    else snn_u_kernel<false, false><<<(int)blocks, 256, 0, s>>>(grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nz_count);
     count_launch();
     if (cudaGetLastError() != cudaSuccess) return E_CUDA;
   }
@@ -944,7 +972,8 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
     // (DxGate: the list-walking one up to 40 % of the outputs carrying a gradient -- its time grows with that share,
     // the dense tile's does not; they cross near 41 % on the benchmark layers); 1 / 2 name one.
     const bool sparse_ok = want_dx_sparse(g, opt) && dx_sparse_supported(g, x, dx);
-    const bool both = sparse_ok && opt.dx_kernel == 0;
+    // Where the dense tiles are fewer than the SMs they are latency-bound and lose at any share: only the lists then.
+    const bool both = sparse_ok && opt.dx_kernel == 0 && (long)grid.x * grid.y >= li.num_sms;
     DxGate gate = {nullptr, 0u};
     if (both) {
       gate.nz = nz_count;

@@ -112,6 +112,12 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
                     float* dx, float* dw, void* ws, size_t ws_bytes, const LaunchInfo& li, const Options& opt,
                     cudaStream_t s);
 
+// Both gradients of a dense layer in one launch (snntc_bwd_dense.cu); dx or dw may be null. `flags`: the range flags
+// that the u kernel's blocks wrote.
+bool dense_bwd_supported(const Geometry& g);
+int launch_dense_bwd(const Geometry& g, const float* uv, const float* x, const float* w, const float* out, float* dx,
+                     float* dw, float scale, const int* flags, int nflags, const LaunchInfo& li, cudaStream_t s);
+
 // dW by a kernel that skips the (row, output) pairs that did not fire (snntc_dw_skip.cu); conv layers whose
 // channel count is a multiple of 4.
 bool dw_skip_supported(const Geometry& g, const float* x, const float* uv, const float* out);
