@@ -21,13 +21,13 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libsnntc_b200.so")
 LIB_MEASURE = os.path.join(HERE, "libsnntc_b200_measure.so")
-SOURCES = ["snntc_forward.cu", "snntc_lists.cu", "snntc_backward.cu", "snntc_bwd_dense.cu",
+SOURCES = ["snntc_forward.cu", "snntc_walk_ring.cu", "snntc_lists.cu", "snntc_backward.cu", "snntc_bwd_dense.cu",
            "snntc_dw_skip.cu", "snntc_dw_tma.cu", "snntc_dx_sparse.cu", "snntc_pool.cu",
            "snntc_noalloc.cu", "snntc_train.cu", "snntc_api.cu"]
 NATIVE = os.path.join(HERE, "_native" + sysconfig.get_config_var("EXT_SUFFIX"))
 NATIVE_SOURCE = os.path.join(CSRC, "snntc_torch.cpp")
 API_SOURCE = "snntc_api.cu"   # the only file that reads SNNTC_MEASURE
-HEADERS = [os.path.join(CSRC, "snntc_common.cuh"), os.path.join(CSRC, "snntc_merge.cuh"),
+HEADERS = [os.path.join(CSRC, "snntc_common.cuh"), os.path.join(CSRC, "snntc_merge.cuh"), os.path.join(CSRC, "snntc_walk.cuh"),
            os.path.join(HERE, "..", "include", "snntc_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]

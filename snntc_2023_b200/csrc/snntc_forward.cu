@@ -20,7 +20,9 @@
 //      lane's outputs: a pair in one 64-bit register (walk_row2, fan-out <= 64), 2 or 4 consecutive outputs read
 //      by one 8/16-byte load, or outputs lane + 32*m (odd fan-out, unaligned weights).
 #include "snntc_common.cuh"
+#include "snntc_walk.cuh"
 
+#include <cooperative_groups.h>
 #include <limits.h>
 #include <math_constants.h>
 
@@ -42,20 +44,6 @@ __device__ __forceinline__ float key_value(u64 e) { return sortable_to_float((ui
 
 // ------------------------------------------------------------------------------------------- walk
 
-// "ysum/wsum > c" without a division, as the reference evaluates it after consuming input c
-// (snntc/snnfc_kernels.cu.cc:53-55)
-__device__ __forceinline__ bool ratio_gt(float ysum, float wsum, float c) {
-  const float wa = fabsf(wsum);
-  const float ya = wsum < 0.f ? -ysum : ysum;
-  return ya > c * wa;
-}
-// "ysum/wsum <= c" (snntc/snnfc_kernels.cu.cc:46-48)
-__device__ __forceinline__ bool ratio_le(float ysum, float wsum, float c) {
-  const float wa = fabsf(wsum);
-  const float ya = wsum < 0.f ? -ysum : ysum;
-  return ya <= c * wa;
-}
-
 // Smallest of three float bit patterns compared as signed integers. For the sign test of the walk that is all
 // that is needed: the result is <= 0 exactly when one of the floats is negative, -0 or +0 (negative floats are
 // negative integers, +0 is 0, positive floats and NaN patterns with a clear sign bit are positive integers).
@@ -76,19 +64,30 @@ __device__ __forceinline__ float walk_tolerance_base(const Geometry& g) {
   return 4.76837158203125e-7f * (fabsf(g.theta) + b) * 1.0001f;   // (a little slack for the rounding of the sums)
 }
 
-// bound[blockIdx.x] = sum over this CTA's weight rows of max_j |w_ij|: summed over the CTAs an upper bound on every
-// column's sum of magnitudes. rows = I + bias row; CTA c takes rows [c * rows_per_cta, (c + 1) * rows_per_cta).
-constexpr int kBoundMaxCtas = 32;
-__global__ void __launch_bounds__(256)
+// bound[cluster] = sum over the weight rows of this cluster's eight CTAs of max_j |w_ij|: summed over the clusters an upper
+// bound on every column's sum of magnitudes. rows = I + bias row; CTA c takes rows [c * rows_per_cta, (c + 1) * rows_per_cta).
+// Bound by memory: up to 256 CTAs, 16 bytes per lane and load (32 CTAs read the 103 MB of a 25 088 x 1024 layer in 300 us).
+constexpr int kBoundClusters = 32;
+constexpr int kBoundCtas = 8 * kBoundClusters;
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256)
 snn_wbound_kernel(const float* __restrict__ w, int rows, int J, int rows_per_cta, float* __restrict__ bound) {
-  __shared__ float part[8];
+  __shared__ float part[9];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r0 = blockIdx.x * rows_per_cta;
+  const bool v4 = (J & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
   float acc = 0.f;                                     // lane 0: sum of the row maxima of this warp's rows
   for (int r = r0 + warp; r < min(rows, r0 + rows_per_cta); r += 8) {
     const float* wr = w + (size_t)r * J;
     float m = 0.f;
-    for (int j = lane; j < J; j += 32) m = fmaxf(m, fabsf(__ldg(wr + j)));
+    if (v4) {
+#pragma unroll 4
+      for (int j = 4 * lane; j < J; j += 128) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(wr + j));
+        m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+      }
+    } else {
+      for (int j = lane; j < J; j += 32) m = fmaxf(m, fabsf(__ldg(wr + j)));
+    }
 #pragma unroll
     for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
     acc += m;
@@ -99,19 +98,17 @@ snn_wbound_kernel(const float* __restrict__ w, int rows, int J, int rows_per_cta
     float t = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) t += part[k];
-    bound[blockIdx.x] = t;
+    part[8] = t;
   }
-}
-
-// Number of list entries whose input value lies strictly below y: the causal-set size of an output that fired
-// at y (every consumed input is below the spike value, every other one is not). Binary search, one thread.
-__device__ __forceinline__ int entries_below(const WalkEntry* __restrict__ ents, int n, float y) {
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (__uint_as_float(__ldcg(ents + mid).x) < y) lo = mid + 1; else hi = mid;
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  cl.sync();
+  if (threadIdx.x == 0 && cl.block_rank() == 0) {
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t += *cl.map_shared_rank(part + 8, k);
+    bound[blockIdx.x / 8] = t;
   }
-  return lo;
+  cl.sync();                                           // no CTA leaves while its sum may still be read
 }
 
 // One warp walks one row for 32*JPT outputs. Let q_k = ysum - x_k*wsum be taken just before input k is
@@ -315,28 +312,6 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* __r
 // ---- two outputs per 64-bit register ---------------------------------------------------------------
 // sm_100 has two-lane FP32 add / sub / fma on 64-bit register pairs: one issue slot, two results, each
 // rounded exactly like the scalar instruction. A pair holds outputs (j, j+1) of one lane.
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ void unpack2i(uint64_t v, int& lo, int& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
 // walk_row with the outputs of a lane held as JP pairs (j, j+1), j = jbase + 2*lane + 64*m: the three
 // FP32 operations of a step (q, the weight sum, the weighted sum) are one packed instruction per pair and
 // a weight-row read is one 8-byte load per pair. The weight sum is carried NEGATED (nws = theta - sum w), so
@@ -1260,12 +1235,19 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   const int istride = key_stride(g);
 
   const int fparts = opt.forward_parts;
-  if (fparts & 2) {   // the walk's bound on the weight sums (see walk_tolerance_base)
+  // The walk that copies its weight rows ahead, up to about 24 items of 32 outputs per SM (8 where the rows have to be copied
+  // 4 bytes at a time): with few warps on an SM latency is what counts, with many the instructions per output. Measured lines:
+  // 784 -> 400 crosses at 3 300 items, 4096 -> 512 behind 4 100, 3x3 convolutions of 128 and 256 channels between 2 000 and 4 100.
+  const long ring_items = (long)g.R * ((g.J + 31) / 32);
+  const bool copies16 = (g.J & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+  const bool ring = (opt.walk_layout & 16) != 0 ||
+                    (opt.walk_layout == 0 && opt.walk_outputs == 0 && ring_items <= (copies16 ? 24L : 8L) * li.num_sms);
+  if ((fparts & 2) && !ring) {   // the walk's bound on the weight sums (see walk_tolerance_base)
     const int rows_w = g.I + g.has_bias;
-    int per = (rows_w + kBoundMaxCtas - 1) / kBoundMaxCtas;
+    int per = (rows_w + kBoundCtas - 1) / kBoundCtas;
     per = (per + 7) & ~7;                                // whole rounds of the CTA's eight warps
-    g.wbound_n = (rows_w + per - 1) / per;
-    snn_wbound_kernel<<<g.wbound_n, 256, 0, s>>>(w, rows_w, g.J, per, wbound);
+    g.wbound_n = (rows_w + 8 * per - 1) / (8 * per);     // clusters
+    snn_wbound_kernel<<<8 * g.wbound_n, 256, 0, s>>>(w, rows_w, g.J, per, wbound);
     count_launch();
     if (cudaGetLastError() != cudaSuccess) return E_CUDA;
   }
@@ -1319,6 +1301,7 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
                      ((opt.walk_layout & 8) != 0 || ((opt.walk_layout & 3) == 0 && g.J == 64 && g.R >= 8192));
   auto walk = [&](cudaStream_t st, int r0, int r1) -> int {
     if (!(fparts & 2)) return OK;
+    if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, st);
     if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage, smemw_bytes, smemw_shift);
     if (variant == 1) {
       // pairs layout: 64 outputs per warp, or (walk_outputs 3) 128 as two pairs per lane
