@@ -245,7 +245,7 @@ SNNTC_API unsigned long long snntc_copy_timeouts(void);
  *             walk_layout     0 auto, 1 output pairs, 2 outputs lane+32m, 3 consecutive outputs per lane; +4: list
  *                             entries straight from global memory instead of staged through shared memory,
  *             walk_outputs    0 auto, 1..4: 1, 2, 4, 8 outputs per lane,
- *             list_builder    0 auto, 1 per-row radix sort, 2 per-pixel sort + merges,
+ *             list_builder    0 auto, 1 per-row bucket sort, 2 per-pixel sort + merges,
  *             backward_parts  bit 0: dX, bit 1: dW (default 3),
  *             dw_kernel       0 auto, 1 dense register tile, 2 row-skipping kernel,
  *             overlap         -1 library setting, 0 one stream, 1 dX beside dW,

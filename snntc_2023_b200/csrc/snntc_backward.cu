@@ -940,8 +940,9 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
     else snn_u_kernel<false, true><<<(int)blocks, 1024, 0, s>>>(grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nullptr);
     count_launch();
     if (cudaGetLastError() != cudaSuccess) return E_CUDA;
-    return launch_dense_bwd(g, uv, x, w, out, (parts & 1) ? dx : nullptr, (parts & 2) ? dw : nullptr, dw_scale(g), exact_flag,
-                            (int)blocks, li, s);
+    const DwPlan p = plan_dw(g, li);
+    return launch_dense_bwd(g, uv, x, w, out, (parts & 1) ? dx : nullptr, (parts & 2) ? dw : nullptr, p.splits,
+                            p.rows_per_split, dw_scale(g), exact_flag, (int)blocks, li, s);
   }
   {
     const size_t n = (size_t)g.R * g.J;

@@ -6,10 +6,11 @@
 //
 // What bounds a dense layer at these sizes is not arithmetic but how little of the GPU a call reaches: 256 samples of a
 // 784 -> 400 layer are 52 tiles of 64 x 64 for dX, each reducing 400 outputs one after the other. Here
-//   - the unit of work is a 32 x 32 tile of dX or dW per WARP, 32 sums per lane, and the warps of a cluster of up to eight
-//     CTAs (four warps each) share out tiles AND the reduction: `split` warps take a part each of one tile's reduction
-//     and are added in a fixed order through distributed shared memory, so that a layer with few tiles still gives every
-//     SM work (32 samples of that layer are 25 tiles: with all of a tile's warps in one CTA, 25 SMs worked for 12 us);
+//   - the unit of work is a small tile per WARP. dX: 32 x 32 down to 8 x 8 (rows x inputs), the largest that still gives every
+//     SM six warps; the reduction over the outputs is one running sum per element, ascending, as in the other dX kernels.
+//     dW: 32 x 32, its rows cut into the slices that plan_dw (snntc_backward.cu) gives the register-tile kernel, a warp per
+//     slice, and the slices added through the distributed shared memory of a cluster in the order snn_dw_reduce_kernel adds
+//     planes. So the sums are the register-tile kernels' bit for bit;
 //   - every warp brings its own chunks of 16 reduction steps in with 16-byte asynchronous copies, two buffers deep, as they
 //     lie in memory, with no CTA barrier in the loop. dX reads four steps of a row at once (16 bytes), so nothing has to be
 //     transposed; rows of 20 floats and a lane's rows 8 apart keep these reads free of bank conflicts. (4-byte copies that
@@ -17,8 +18,8 @@
 //   - dX and dW tiles are blocks of one grid: they run side by side without an auxiliary stream.
 // Per element dX is a compare and a predicated FMA (bound by the half-rate compare pipe), dW a saturating FMA and half a
 // two-lane FMA (the scaled form of relu(y - x), snntc_backward.cu).
-// Measured (B200, batch 256, 784 -> 400, every output with a gradient): dX 67 us, dW 22 us and 9 us around them before,
-// DENSE_BOTH_US us now.
+// Measured (B200, dX + dW with the u kernel, before -> now): 784 -> 400 at 32 samples 85 -> 16 us, at 256: 98 -> 35, at 1024: 142 -> 99;
+// 4096 -> 512 at 256: 185 -> 123; 25 088 -> 1024 at 64: 550 -> 330.
 #include "snntc_common.cuh"
 
 #include <cooperative_groups.h>
@@ -78,9 +79,10 @@ template <int N>
 __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 struct DensePlan {
-  int cluster;                             // CTAs per cluster; a cluster's warps take (its warps / split) neighbouring tiles
-  int dx_clusters, dx_split, dx_tiles_n;   // dX: tiles of [rows][inputs], neighbours along the inputs
-  int dw_clusters, dw_split, dw_tiles_m;   // dW: tiles of [weight rows][outputs], neighbours along the weight rows
+  int cluster;                             // CTAs per cluster
+  int dx_clusters, dx_tiles_n;             // dX: tiles of [rows][inputs], a warp each, neighbours along the inputs
+  int dw_clusters, dw_tiles_m;             // dW: tiles of [weight rows][outputs], neighbours along the weight rows
+  int dw_splits, dw_rows;                  // slices of the rows (at most 32, a warp each) and rows per slice (a multiple of 16)
 };
 
 struct DenseArgs {
@@ -96,42 +98,20 @@ struct DenseArgs {
   float biasvolt, scale;   // scale: the power of two of the scaled dW loop, 1 = not usable
 };
 
-// The sums of a warp's tile (lane -> rows m + MS*k, k < ML, columns n + NS*b, b < NL) are added over the `split` warps of the
-// tile in warp order, and the tile goes out in whole rows of 32 columns.
-template <int ML, int NL, int MS, int NS>
-__device__ __forceinline__ void write_tile(const float (&acc)[ML][NL], float* smem, int gw, int lane, int m, int n, int split,
-                                           float* __restrict__ dst, int m0, int M, int n0, int N) {
-  cg::cluster_group cl = cg::this_cluster();
-  float* mine = smem + (gw % kWarps) * kWarpFloats;    // (this warp's own staging buffers: every copy into them has been waited for)
-  __syncwarp();
-#pragma unroll
-  for (int k = 0; k < ML; ++k)
-#pragma unroll
-    for (int b = 0; b < NL; ++b) mine[(m + MS * k) * kPad + n + NS * b] = acc[k][b];
-  const int part = gw % split, first = gw - part;      // the tile's warps in the cluster: first .. first + split - 1
-  if (split == 1) {
-    __syncwarp();
-    if (n0 + lane < N)
-      for (int row = 0; row < kT && m0 + row < M; ++row) dst[(size_t)(m0 + row) * N + n0 + lane] = mine[row * kPad + lane];
-    return;
+// A warp's tile of MR x NC sums in shared memory goes out in whole rows.
+template <int MR, int NC>
+__device__ __forceinline__ void store_tile(const float* tile, int lane, float* __restrict__ dst, int m0, int M, int n0, int N) {
+#pragma unroll 4
+  for (int e = lane; e < MR * NC; e += 32) {
+    const int row = e / NC, col = e % NC;
+    if (m0 + row < M && n0 + col < N) dst[(size_t)(m0 + row) * N + n0 + col] = tile[row * kPad + col];
   }
-  cl.sync();
-  if (n0 + lane < N) {
-    for (int row = part; row < kT && m0 + row < M; row += split) {
-      float s = 0.f;
-      for (int k = 0; k < split; ++k) {
-        const float* tile = cl.map_shared_rank(smem, (first + k) / kWarps) + ((first + k) % kWarps) * kWarpFloats;
-        s += tile[row * kPad + lane];
-      }
-      dst[(size_t)(m0 + row) * N + n0 + lane] = s;
-    }
-  }
-  cl.sync();                                           // no CTA leaves while its tiles may still be read
 }
 
 // VX: I is a multiple of 4 and x 16-byte aligned; VJ: J is a multiple of 4 and u, y and w 16-byte aligned. Then every copy
 // moves 16 bytes, else 4.
-template <bool VX, bool VJ>
+// ML, NL: rows and inputs of a dX tile per lane (the tile is 8*ML x 4*NL).
+template <bool VX, bool VJ, int ML, int NL>
 __global__ void __launch_bounds__(kThreads, 3)
 snn_dense_bwd_kernel(const DenseArgs a, const DensePlan p) {
   extern __shared__ __align__(16) float smem[];
@@ -145,11 +125,11 @@ snn_dense_bwd_kernel(const DenseArgs a, const DensePlan p) {
 
   if (cluster < p.dx_clusters) {
     // ---------------------------------------------------------------- dX tile: rows r, columns i, reduced over j
-    const int tile = cluster * (cluster_warps / p.dx_split) + gw / p.dx_split;     // (a tile behind the last one has r0 >= R)
-    const int r0 = tile / p.dx_tiles_n * kT, i0 = tile % p.dx_tiles_n * kT;
-    const int part = gw % p.dx_split;
+    constexpr int MR = 8 * ML, NC = 4 * NL;
+    const int tile = cluster * cluster_warps + gw;
+    const int r0 = tile / p.dx_tiles_n * MR, i0 = tile % p.dx_tiles_n * NC;
+    if (r0 >= R) return;                        // (no barrier of the CTA or cluster in this branch)
     const int chunks = (J + kStep - 1) / kStep;
-    const int c0 = chunks * part / p.dx_split, c1 = r0 < R ? chunks * (part + 1) / p.dx_split : c0;
     auto issue = [&](int c, int buf) {
       const unsigned at = mine_at + 4u * (unsigned)(buf * 3 * kTile);
       if constexpr (VJ) {
@@ -161,80 +141,94 @@ snn_dense_bwd_kernel(const DenseArgs a, const DensePlan p) {
         const float* gw = a.w + (size_t)(i0 + row) * J + j;
         const unsigned to = at + 4u * (unsigned)(row * kRow + 4 * (lane & 3));
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const bool rok = jok && r0 + row + 8 * q < R, iok = jok && i0 + row + 8 * q < I;
+        for (int q = 0; q < ML; ++q) {
+          const bool rok = jok && r0 + row + 8 * q < R;
           copy16(to + 4u * (8 * q * kRow), rok ? gy + (size_t)(8 * q) * J : a.y, rok);
           copy16(to + 4u * (8 * q * kRow + kTile), rok ? gu + (size_t)(8 * q) * J : a.u, rok);
+        }
+#pragma unroll
+        for (int q = 0; q < (NL + 1) / 2; ++q) {
+          const bool iok = jok && i0 + row + 8 * q < I && row + 8 * q < NC;
           copy16(to + 4u * (8 * q * kRow + 2 * kTile), iok ? gw + (size_t)(8 * q) * J : a.w, iok);
         }
       } else {
         const int j = c * kStep + (lane & 15), row = lane >> 4;
         const bool jok = j < J;
+        const unsigned to = at + 4u * (unsigned)(row * kRow + (lane & 15));
 #pragma unroll 4
-        for (int q = 0; q < 16; ++q) {
-          const int k = row + 2 * q;
-          const unsigned to = at + 4u * (unsigned)(k * kRow + (lane & 15));
-          const bool rok = jok && r0 + k < R, iok = jok && i0 + k < I;
-          copy4(to, rok ? a.y + (size_t)(r0 + k) * J + j : a.y, rok);
-          copy4(to + 4u * kTile, rok ? a.u + (size_t)(r0 + k) * J + j : a.u, rok);
-          copy4(to + 8u * kTile, iok ? a.w + (size_t)(i0 + k) * J + j : a.w, iok);
+        for (int k = 0; k < MR; k += 2) {
+          const bool rok = jok && r0 + row + k < R;
+          const size_t o = rok ? (size_t)(r0 + row + k) * J + j : 0;
+          copy4(to + 4u * (k * kRow), a.y + o, rok);
+          copy4(to + 4u * (k * kRow + kTile), a.u + o, rok);
+        }
+#pragma unroll 4
+        for (int k = 0; k < NC; k += 2) {
+          const bool iok = jok && i0 + row + k < I;
+          copy4(to + 4u * (k * kRow + 2 * kTile), iok ? a.w + (size_t)(i0 + row + k) * J + j : a.w, iok);
         }
       }
       copies_commit();
     };
-    if (c0 < c1) issue(c0, 0);
-    if (c0 + 1 < c1) issue(c0 + 1, 1);
+    issue(0, 0);
+    if (chunks > 1) issue(1, 1);
     const int m = lane >> 2, n = lane & 3;      // this lane's rows m + 8k and inputs n + 4b
-    float xr[4][8], acc[4][8];
+    float xr[ML][NL], acc[ML][NL];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < ML; ++k) {
       const float* gx = a.x + (size_t)(r0 + m + 8 * k) * I + i0 + n;
       const bool rok = r0 + m + 8 * k < R;
 #pragma unroll
-      for (int b = 0; b < 8; ++b) {
+      for (int b = 0; b < NL; ++b) {
         xr[k][b] = (rok && i0 + n + 4 * b < I) ? __ldg(gx + 4 * b) : CUDART_INF_F;
         acc[k][b] = 0.f;
       }
     }
-    for (int c = c0; c < c1; ++c) {
-      const int buf = (c - c0) & 1;
-      if (c + 1 < c1) copies_wait<1>(); else copies_wait<0>();
+    for (int c = 0; c < chunks; ++c) {
+      const int buf = c & 1;
+      if (c + 1 < chunks) copies_wait<1>(); else copies_wait<0>();
       __syncwarp();
       const float* Y = mine + buf * 3 * kTile + m * kRow;
       const float* W = mine + buf * 3 * kTile + 2 * kTile + n * kRow;
 #pragma unroll
       for (int s = 0; s < kStep; s += 4) {
-        float w[8][4];
+        float w[NL][4];
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
+        for (int b = 0; b < NL; ++b) {
           const float4 w4 = *reinterpret_cast<const float4*>(W + 4 * b * kRow + s);
           w[b][0] = w4.x; w[b][1] = w4.y; w[b][2] = w4.z; w[b][3] = w4.w;
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < ML; ++k) {
           const float4 y4 = *reinterpret_cast<const float4*>(Y + 8 * k * kRow + s);
           const float4 u4 = *reinterpret_cast<const float4*>(Y + kTile + 8 * k * kRow + s);
           const float y[4] = {y4.x, y4.y, y4.z, y4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
 #pragma unroll
           for (int t = 0; t < 4; ++t)
 #pragma unroll
-            for (int b = 0; b < 8; ++b) masked_fma(acc[k][b], xr[k][b], y[t], u[t], w[b][t]);
+            for (int b = 0; b < NL; ++b) masked_fma(acc[k][b], xr[k][b], y[t], u[t], w[b][t]);
         }
       }
       __syncwarp();
-      if (c + 2 < c1) issue(c + 2, buf);
+      if (c + 2 < chunks) issue(c + 2, buf);
     }
-    write_tile<4, 8, 8, 4>(acc, smem, gw, lane, m, n, p.dx_split, a.dx, r0, R, i0, I);
+#pragma unroll
+    for (int k = 0; k < ML; ++k)
+#pragma unroll
+      for (int b = 0; b < NL; ++b) mine[(m + 8 * k) * kPad + n + 4 * b] = acc[k][b];
+    __syncwarp();
+    store_tile<MR, NC>(mine, lane, a.dx, r0, R, i0, I);
     return;
   }
 
   // ------------------------------------------------------------------ dW tile: rows i (bias row last), columns j, reduced over r
   const int Itot = I + a.has_bias;
-  const int tile = (cluster - p.dx_clusters) * (cluster_warps / p.dw_split) + gw / p.dw_split;
-  const int i0 = tile % p.dw_tiles_m * kT, j0 = tile / p.dw_tiles_m * kT;          // (a tile behind the last one has j0 >= J)
-  const int part = gw % p.dw_split;
-  const int chunks = (R + kStep - 1) / kStep;
-  const int c0 = chunks * part / p.dw_split, c1 = j0 < J ? chunks * (part + 1) / p.dw_split : c0;
+  const int per = cluster_warps / p.dw_splits;                                      // tiles per cluster
+  const int mine_tile = gw / p.dw_splits, part = gw % p.dw_splits;
+  const int tile = (cluster - p.dx_clusters) * per + mine_tile;
+  const int i0 = tile % p.dw_tiles_m * kT, j0 = tile / p.dw_tiles_m * kT;           // (a tile behind the last one has j0 >= J)
+  const int r_begin = part * p.dw_rows, r_end = min(R, r_begin + p.dw_rows);
+  const int c0 = r_begin / kStep, c1 = mine_tile < per && j0 < J ? (r_end + kStep - 1) / kStep : c0;
   const int ls = lane >> 3, lc = 4 * (lane & 7);    // 16-byte copies: row ls + 4q of the chunk, columns lc .. lc+3
   auto issue = [&](int c, int buf) {
     const unsigned at = mine_at + 4u * (unsigned)(buf * 3 * kTile);
@@ -323,32 +317,49 @@ snn_dense_bwd_kernel(const DenseArgs a, const DensePlan p) {
     __syncwarp();
     if (c + 2 < c1) issue(c + 2, buf);
   }
-  float acc[8][4];
+  copies_wait<0>();
+  __syncwarp();
 #pragma unroll
-  for (int k = 0; k < 8; ++k)
-#pragma unroll
-    for (int b = 0; b < 2; ++b) unpack2(acc2[k][b], acc[k][2 * b], acc[k][2 * b + 1]);
-  write_tile<8, 4, 1, 1>(acc, smem, gw, lane, m, n, p.dw_split, a.dw, i0, Itot, j0, J);
-}
-
-// How many warps share one tile's reduction of length L: a power of two up to the 32 warps of the largest cluster that
-// minimises (waves of 12 warps per SM) x (steps of a warp + about 20 steps' worth of prologue, pipeline fill and adding up),
-// with at least one chunk of 16 steps per warp.
-int pick_split(long tiles, int L, const LaunchInfo& li) {
-  const long wave = 12L * li.num_sms;
-  int best = 1;
-  long best_cost = 0;
-  for (int s = 1; s <= kMaxCluster * kWarps && (s == 1 || L >= kStep * s); s *= 2) {
-    const long waves = (tiles * s + wave - 1) / wave;
-    const long cost = waves * ((L + s - 1) / s + 20);
-    if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
+  for (int k = 0; k < 8; ++k) {
+    float lo[2], hi[2];
+    unpack2(acc2[k][0], lo[0], hi[0]);
+    unpack2(acc2[k][1], lo[1], hi[1]);
+    *reinterpret_cast<float4*>(mine + (m + k) * kPad + n) = make_float4(lo[0], hi[0], lo[1], hi[1]);
   }
-  return best;
+  if (p.dw_splits == 1) {
+    __syncwarp();
+    if (c0 < c1) store_tile<kT, kT>(mine, lane, a.dw, i0, Itot, j0, J);
+    return;
+  }
+  // the slices of a tile, added as snn_dw_reduce_kernel adds planes: four interleaved sums, then their sum
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  if (mine_tile < per && j0 + lane < J) {
+    const int first = gw - part;
+    auto slice = [&](int k, int row) {
+      const int wk = first + k;
+      return cl.map_shared_rank(smem, wk / kWarps)[(wk % kWarps) * kWarpFloats + row * kPad + lane];
+    };
+    for (int row = part; row < kT && i0 + row < Itot; row += p.dw_splits) {
+      float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+      int k = 0;
+      for (; k + 8 <= p.dw_splits; k += 8) {
+        float v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = slice(k + q, row);
+        s0 += v[0]; s1 += v[1]; s2 += v[2]; s3 += v[3];
+        s0 += v[4]; s1 += v[5]; s2 += v[6]; s3 += v[7];
+      }
+      for (; k < p.dw_splits; ++k) s0 += slice(k, row);
+      a.dw[(size_t)(i0 + row) * J + j0 + lane] = (s0 + s1) + (s2 + s3);
+    }
+  }
+  cl.sync();                                           // no CTA leaves while its tiles may still be read
 }
 
-template <bool VX, bool VJ>
+template <bool VX, bool VJ, int ML, int NL>
 int launch(const DenseArgs& a, const DensePlan& p, cudaStream_t s) {
-  if (cudaFuncSetAttribute(snn_dense_bwd_kernel<VX, VJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) != cudaSuccess)
+  if (cudaFuncSetAttribute(snn_dense_bwd_kernel<VX, VJ, ML, NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) != cudaSuccess)
     return E_CUDA;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((p.dx_clusters + p.dw_clusters) * p.cluster));
@@ -361,37 +372,52 @@ int launch(const DenseArgs& a, const DensePlan& p, cudaStream_t s) {
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, snn_dense_bwd_kernel<VX, VJ>, a, p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, snn_dense_bwd_kernel<VX, VJ, ML, NL>, a, p);
   count_launch();
   return e == cudaSuccess ? OK : E_CUDA;
 }
 
+template <int ML, int NL>
+int launch_tile(DenseArgs a, DensePlan p, bool vx, bool vj, cudaStream_t s) {
+  if (a.dx) {
+    const long m = (a.R + 8 * ML - 1) / (8 * ML), n = (a.I + 4 * NL - 1) / (4 * NL);
+    p.dx_tiles_n = (int)n;
+    p.dx_clusters = (int)((m * n + p.cluster * kWarps - 1) / (p.cluster * kWarps));
+  }
+  if (p.dx_clusters + p.dw_clusters == 0) return OK;
+  if (vx) return vj ? launch<true, true, ML, NL>(a, p, s) : launch<true, false, ML, NL>(a, p, s);
+  return vj ? launch<false, true, ML, NL>(a, p, s) : launch<false, false, ML, NL>(a, p, s);
+}
+
 }  // namespace
 
-// Up to 4096 samples: beyond, the row loop of a dW tile is long enough that the row-split register tiles of
-// snntc_backward.cu keep the GPU as busy.
-bool dense_bwd_supported(const Geometry& g) { return !g.is_conv && g.R <= 4096; }
+// Up to 2048 samples, which plan_dw cuts into at most 32 slices: one per warp of the largest cluster. Beyond, the row loop of a
+// dW tile is long enough that the register-tile kernels keep the GPU as busy.
+bool dense_bwd_supported(const Geometry& g) { return !g.is_conv && g.R <= 2048; }
 
 int launch_dense_bwd(const Geometry& g, const float* uv, const float* x, const float* w, const float* out, float* dx,
-                     float* dw, float scale, const int* flags, int nflags, const LaunchInfo& li, cudaStream_t s) {
-  DenseArgs a = {uv, x, w, out, dx, dw, flags, nflags, g.R, g.I, g.J, g.has_bias, g.biasvolt, scale};
+                     float* dw, int dw_splits, int dw_rows, float scale, const int* flags, int nflags, const LaunchInfo& li,
+                     cudaStream_t s) {
+  const DenseArgs a = {uv, x, w, out, dx, dw, flags, nflags, g.R, g.I, g.J, g.has_bias, g.biasvolt, scale};
   DensePlan p = {};
-  const long rt = (g.R + kT - 1) / kT, it = (g.I + kT - 1) / kT;                                // dX tiles
-  const long wt = (g.I + g.has_bias + kT - 1) / kT, jt = (g.J + kT - 1) / kT;                   // dW tiles
-  p.dx_split = dx ? pick_split(rt * it, g.J, li) : 1;
-  p.dw_split = dw ? pick_split(wt * jt, g.R, li) : 1;
-  const int most = p.dx_split > p.dw_split ? p.dx_split : p.dw_split;
-  p.cluster = most <= kWarps ? 1 : most / kWarps;
-  const long warps = (long)p.cluster * kWarps;
-  p.dx_tiles_n = (int)it;
-  p.dw_tiles_m = (int)wt;
-  if (dx) p.dx_clusters = (int)((rt * it + warps / p.dx_split - 1) / (warps / p.dx_split));
-  if (dw) p.dw_clusters = (int)((jt * wt + warps / p.dw_split - 1) / (warps / p.dw_split));
-  if (p.dx_clusters + p.dw_clusters == 0) return OK;
+  p.dw_splits = dw ? dw_splits : 1;
+  p.dw_rows = dw_rows;
+  p.cluster = (p.dw_splits + kWarps - 1) / kWarps;
+  if (p.cluster > kMaxCluster) return E_UNSUPPORTED;
+  if (dw) {
+    const long m = (g.I + g.has_bias + kT - 1) / kT, n = (g.J + kT - 1) / kT, per = p.cluster * kWarps / p.dw_splits;
+    p.dw_tiles_m = (int)m;
+    p.dw_clusters = (int)((m * n + per - 1) / per);
+  }
   const bool vx = (g.I & 3) == 0 && ((uintptr_t)x & 15) == 0;
   const bool vj = (g.J & 3) == 0 && (((uintptr_t)uv | (uintptr_t)out | (uintptr_t)w) & 15) == 0;
-  if (vx) return vj ? launch<true, true>(a, p, s) : launch<true, false>(a, p, s);
-  return vj ? launch<false, true>(a, p, s) : launch<false, false>(a, p, s);
+  // the largest dX tile that leaves every SM six warps: a large one reads less per product, with few warps latency counts
+  auto tiles = [&](int m, int n) { return (long)((g.R + m - 1) / m) * ((g.I + n - 1) / n); };
+  const long enough = 6L * li.num_sms;
+  if (!dx || tiles(32, 32) >= enough) return launch_tile<4, 8>(a, p, vx, vj, s);
+  if (tiles(16, 32) >= enough) return launch_tile<2, 8>(a, p, vx, vj, s);
+  if (tiles(16, 16) >= enough) return launch_tile<2, 4>(a, p, vx, vj, s);
+  return launch_tile<1, 4>(a, p, vx, vj, s);
 }
 
 }  // namespace snntc

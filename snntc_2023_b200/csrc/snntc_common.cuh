@@ -45,7 +45,7 @@ struct Options {
                             // +8: output pairs with the weights staged in shared memory (where they fit)
                             // 16: one output per lane, the warp's weight rows copied ahead into shared memory
   int walk_outputs = 0;     // 0 auto, 1..4: 1, 2, 4, 8 outputs per lane (pairs layout: 2 only)
-  int list_builder = 0;     // 0 auto, 1 per-row radix sort, 2 per-pixel sort + merges (3x3 stride-1 conv only),
+  int list_builder = 0;     // 0 auto, 1 per-row bucket sort, 2 per-pixel sort + merges (3x3 stride-1 conv only),
                             // 3 per-row sorting network in registers (rows of at most 256 inputs);
                             // + 4*(k+1): the merges are cut into 2^k pieces each (k = 0 .. 5) instead of auto
   int backward_parts = 3;   // bit 0: dX, bit 1: dW
@@ -106,6 +106,10 @@ int launch_merge_lists(const Geometry& g, const float* x, WalkEntry* lists, int*
 int launch_walk_ring(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
                      cudaStream_t s);
 
+// Sorted lists of everything else by a bucket sort per row (snntc_sort.cu).
+int launch_row_sort(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride, const LaunchInfo& li,
+                    cudaStream_t s);
+
 // Sorted lists of rows of at most 256 inputs by a sorting network in registers, one warp per row (snntc_lists.cu).
 bool small_rows_supported(const Geometry& g);
 int launch_small_rows(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride,
@@ -117,11 +121,13 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
                     float* dx, float* dw, void* ws, size_t ws_bytes, const LaunchInfo& li, const Options& opt,
                     cudaStream_t s);
 
-// Both gradients of a dense layer in one launch (snntc_bwd_dense.cu); dx or dw may be null. `flags`: the range flags
-// that the u kernel's blocks wrote.
+// Both gradients of a dense layer in one launch (snntc_bwd_dense.cu); dx or dw may be null. dw_splits, dw_rows: the slices of
+// the rows, as the register-tile dW kernel takes them (the same bits). `flags`: the range flags that the u kernel's blocks
+// wrote.
 bool dense_bwd_supported(const Geometry& g);
 int launch_dense_bwd(const Geometry& g, const float* uv, const float* x, const float* w, const float* out, float* dx,
-                     float* dw, float scale, const int* flags, int nflags, const LaunchInfo& li, cudaStream_t s);
+                     float* dw, int dw_splits, int dw_rows, float scale, const int* flags, int nflags, const LaunchInfo& li,
+                     cudaStream_t s);
 
 // dW by a kernel that skips the (row, output) pairs that did not fire (snntc_dw_skip.cu); conv layers whose
 // channel count is a multiple of 4.

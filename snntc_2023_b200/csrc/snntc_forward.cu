@@ -5,12 +5,7 @@
 // (value, element offset of the weight row), ascending -- joins two stages:
 //   1. the lists. Stride-1 convolutions up to 3x3 on 16 to 512 channels: per-pixel sort and two levels of
 //      merging (snntc_lists.cu). Rows of at most 256 inputs: a sorting network in registers, one warp per row
-//      (snntc_lists.cu). Everything else, here: one warp per row gathers the row into shared memory as 32-bit
-//      sortable value bits plus a 16-bit source index (conv rows find their taps through a per-CTA table, with
-//      predicated loads and no divergent branch), rebases the keys to the row's smallest, counts the 8-bit digits
-//      that the row's range needs and runs a stable least-significant-digit radix sort over those digits only (a
-//      last digit of one or two bits is a ballot split); rows too long for two shared-memory buffers fall back
-//      to a CTA-wide in-place bitonic network;
+//      (snntc_lists.cu). Everything else: a bucket sort per row (snntc_sort.cu);
 //   2. the walk (walk kernels): every warp takes (row, block of outputs) items and walks the row's list, which it
 //      stages through shared memory 32 entries at a time. The running sum(w)-theta and sum(w*x) stay in
 //      registers, in sorted order, bias first, with the arithmetic of the reference kernel
@@ -39,8 +34,6 @@ typedef unsigned long long u64;
 // a shuffle from a fixed lane lets the compiler treat everything derived from it (row numbers, list lengths,
 // loop bounds) as warp-uniform, and with that it drops the divergence check in front of every warp vote.
 __device__ __forceinline__ int uniform_warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
-
-__device__ __forceinline__ float key_value(u64 e) { return sortable_to_float((uint32_t)(e >> 32)); }
 
 // ------------------------------------------------------------------------------------------- walk
 
@@ -515,473 +508,7 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* __
   }
 }
 
-// ------------------------------------------------------------------------------------------- gather
-// Where element i = lane + 32*n of a conv row sits in the receptive field, kept incrementally so that
-// the per-element work has no integer division (the lane -> (kh, kw, c) map is the same for every row).
-struct TapCursor {
-  int kh, kw, c;
-  __device__ __forceinline__ void init(const Geometry& g, int lane) {
-    const int tap = lane / g.C;
-    c = lane - tap * g.C;
-    kh = tap / g.Kw;
-    kw = tap - kh * g.Kw;
-  }
-  __device__ __forceinline__ void advance32(const Geometry& g) {
-    c += 32;
-    while (c >= g.C) {
-      c -= g.C;
-      if (++kw == g.Kw) { kw = 0; ++kh; }
-    }
-  }
-};
-
-// Loads one row, drops inputs above MAX-0.1, writes packed keys to dst[0..n) in index order and
-// (if hist != nullptr) counts the four 8-bit digits of every kept key. Returns n. One warp.
-// `start` is the cursor of element `lane` (conv only).
-__device__ __forceinline__ int gather_row(const Geometry& g, const float* __restrict__ x, int r, int lane,
-                                          u64* __restrict__ dst, unsigned* __restrict__ hist, const TapCursor& start) {
-  const int I = g.I;
-  const float maxcomp = g.maxv - 0.1f;
-  int n = 0;
-  int h0 = 0, w0 = 0;
-  const float* xr = x + (size_t)r * I;
-  TapCursor cur = start;
-  if (g.is_conv) {
-    const int nw = r % g.Nw;
-    const int t = r / g.Nw;
-    const int nh = t % g.Nh;
-    const int b = t / g.Nh;
-    h0 = nh * g.Sh - g.pad_top;
-    w0 = nw * g.Sw - g.pad_left;
-    xr = x + (size_t)b * g.H * g.W * g.C;
-  }
-  // four loads in flight per lane before anything depends on them: the loop is otherwise one global
-  // load latency per 32 elements
-  constexpr int kBatch = 4;
-  for (int i0 = 0; i0 < I; i0 += 32 * kBatch) {
-    float v[kBatch];
-#pragma unroll
-    for (int q = 0; q < kBatch; ++q) {
-      const int i = i0 + 32 * q + lane;
-      v[q] = g.maxv;
-      if (i < I) {
-        if (!g.is_conv) {
-          v[q] = __ldg(xr + i);
-        } else {
-          const int h = h0 + cur.kh, ww = w0 + cur.kw;
-          if (h >= 0 && h < g.H && ww >= 0 && ww < g.W) v[q] = __ldg(xr + ((size_t)h * g.W + ww) * g.C + cur.c);
-        }
-      }
-      if (g.is_conv) cur.advance32(g);
-    }
-#pragma unroll
-    for (int q = 0; q < kBatch; ++q) {
-      const int i = i0 + 32 * q + lane;
-      const bool keep = (i < I) && !(v[q] > maxcomp);
-      const unsigned mask = __ballot_sync(0xffffffffu, keep);
-      if (keep) {
-        const uint32_t key = float_to_sortable(v[q]);
-        dst[n + __popc(mask & ((1u << lane) - 1u))] = ((u64)key << 32) | (uint32_t)i;
-        if (hist) {
-          atomicAdd(&hist[key & 255u], 1u);
-          atomicAdd(&hist[256 + ((key >> 8) & 255u)], 1u);
-          atomicAdd(&hist[512 + ((key >> 16) & 255u)], 1u);
-          atomicAdd(&hist[768 + (key >> 24)], 1u);
-        }
-      }
-      n += __popc(mask);
-    }
-  }
-  return n;
-}
-
-// ------------------------------------------------------------------------------------------- sorts
-// In-place bitonic network for rows too long for two buffers; all threads of the CTA, one row.
-// Every compare-exchange moves the smaller key to the lower index, so the virtual +inf elements at
-// positions >= n never move and need no storage.
-__device__ __forceinline__ void bitonic_sort_cta(u64* keys, int n, int tid) {
-  int npad = 2;
-  while (npad < n) npad <<= 1;
-  const int half = npad >> 1;
-  for (int k = 2; k <= npad; k <<= 1) {
-    const int hk = k >> 1;
-    for (int q = tid; q < half; q += kFwdThreads) {
-      const int o = q & (hk - 1);
-      const int base = (q - o) << 1;
-      const int i = base + o, p = base + k - 1 - o;
-      if (p < n) { const u64 va = keys[i], vb = keys[p]; if (va > vb) { keys[i] = vb; keys[p] = va; } }
-    }
-    __syncthreads();
-    for (int j = hk >> 1; j >= 1; j >>= 1) {
-      for (int q = tid; q < half; q += kFwdThreads) {
-        const int o = q & (j - 1);
-        const int i = ((q - o) << 1) + o, p = i + j;
-        if (p < n) { const u64 va = keys[i], vb = keys[p]; if (va > vb) { keys[i] = vb; keys[p] = va; } }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-// ------------------------------------------------------------------------------------------- compact warp sort
-// The warp sort of snn_sort_kernel keeps keys (32-bit sortable value bits) and source indices (16 bit)
-// in separate arrays and packs the four digit histograms two to a word: 12 bytes per input and 2 KB per
-// warp instead of 16 bytes and 4 KB, which lets a third CTA (24 instead of 16 rows) be resident per SM
-// at fan-in 577 -- the kernel is bound by shared-memory latency, so resident rows are what it needs.
-struct SortBuffers {
-  uint32_t* key;         // buffer b at key + b*I
-  unsigned short* idx;   // buffer b at idx + b*I
-  unsigned* hist;        // [0,256): digit 0 in bits 0..15, digit 1 in bits 16..31; [256,512): digits 2 and 3
-  int I;
-  // (the two buffers are addressed by offset, not through an array of pointers: a pointer picked at run time
-  // out of an array loses its address space and every access through it becomes a generic load or store)
-  __device__ __forceinline__ uint32_t* keys(int b) const { return key + b * I; }
-  __device__ __forceinline__ unsigned short* idxs(int b) const { return idx + b * I; }
-};
-__host__ __device__ __forceinline__ size_t sort_bytes_per_warp(int I) {
-  return (((size_t)12 * I + 15) & ~(size_t)15) + 2048;
-}
-__device__ __forceinline__ SortBuffers sort_buffers(unsigned char* base, int I) {
-  SortBuffers b;
-  b.key = reinterpret_cast<uint32_t*>(base);
-  b.idx = reinterpret_cast<unsigned short*>(b.key + 2 * I);
-  b.hist = reinterpret_cast<unsigned*>(base + (((size_t)12 * I + 15) & ~(size_t)15));
-  b.I = I;
-  return b;
-}
-
-// Where the taps of a conv row sit, relative to the row's top-left input pixel: built once per CTA, the same
-// for every row. off[i] = ((kh*W + kw)*C + c) in elements, khw[i] = kh << 8 | kw (Kh, Kw <= 255). Both arrays
-// are padded to a multiple of 128 entries so that a whole batch of loads may index them.
-struct TapTable {
-  const int* off;
-  const unsigned short* khw;
-};
-__host__ __device__ __forceinline__ int tap_entries(int I) { return (I + 127) & ~127; }
-__host__ __device__ __forceinline__ size_t tap_table_bytes(int I) { return (size_t)tap_entries(I) * 6; }
-
-// Loads one row, drops inputs above MAX-0.1 and writes (sortable key, source index) of the rest to buffer 0
-// in index order; returns their number and the smallest / largest key. One warp, no divergent branch: a tap
-// outside the image (or past the end of the row) is a predicated-off load that reads as MAX and is dropped.
-__device__ __forceinline__ int gather_row_compact(const Geometry& g, const float* __restrict__ x, int r, int lane,
-                                                  const SortBuffers& sb, const TapTable& tt,
-                                                  uint32_t& kmin, uint32_t& kmax) {
-  const int I = g.I;
-  const float maxcomp = g.maxv - 0.1f;
-  int n = 0;
-  int h0 = 0, w0 = 0;
-  const float* xr = x + (size_t)r * I;
-  if (g.is_conv) {
-    const int nw = r % g.Nw;
-    const int t = r / g.Nw;
-    const int nh = t % g.Nh;
-    const int b = t / g.Nh;
-    h0 = nh * g.Sh - g.pad_top;
-    w0 = nw * g.Sw - g.pad_left;
-    // the row's top-left input pixel; may lie outside the image, in which case it is never dereferenced
-    xr = x + ((ptrdiff_t)b * g.H * g.W + (ptrdiff_t)h0 * g.W + w0) * g.C;
-  }
-  uint32_t lmin = 0xFFFFFFFFu, lmax = 0u;
-  const unsigned lt = (1u << lane) - 1u;
-  constexpr int kBatch = 4;   // loads in flight per lane before anything depends on them
-  for (int i0 = 0; i0 < I; i0 += 32 * kBatch) {
-    float v[kBatch];
-#pragma unroll
-    for (int q = 0; q < kBatch; ++q) {
-      const int i = i0 + 32 * q + lane;
-      bool ok = i < I;
-      ptrdiff_t o = i;
-      if (g.is_conv) {
-        const unsigned khw = tt.khw[i];
-        o = tt.off[i];
-        ok = ok && (unsigned)(h0 + (int)(khw >> 8)) < (unsigned)g.H && (unsigned)(w0 + (int)(khw & 255u)) < (unsigned)g.W;
-      }
-      v[q] = g.maxv;
-      if (ok) v[q] = __ldg(xr + o);
-    }
-#pragma unroll
-    for (int q = 0; q < kBatch; ++q) {
-      const int i = i0 + 32 * q + lane;
-      const bool keep = !(v[q] > maxcomp);   // a predicated-off load holds MAX
-      const unsigned mask = __ballot_sync(0xffffffffu, keep);
-      if (keep) {
-        const uint32_t key = float_to_sortable(v[q]);
-        const int pos = n + __popc(mask & lt);
-        sb.key[pos] = key;
-        sb.idx[pos] = (unsigned short)i;
-        lmin = min(lmin, key);
-        lmax = max(lmax, key);
-      }
-      n += __popc(mask);
-    }
-  }
-#pragma unroll
-  for (int d = 16; d >= 1; d >>= 1) {
-    lmin = min(lmin, __shfl_xor_sync(0xffffffffu, lmin, d));
-    lmax = max(lmax, __shfl_xor_sync(0xffffffffu, lmax, d));
-  }
-  kmin = lmin;
-  kmax = lmax;
-  return n;
-}
-
-// Rebase the keys of buffer 0 to key - kmin (order is kept, and the digits above the range of the row become
-// zero, so their passes are not needed at all) and count the lowest `passes` 8-bit digits. One warp.
-__device__ __forceinline__ void rebase_and_count(const SortBuffers& sb, int n, int lane, uint32_t kmin, int passes) {
-  for (int i0 = 0; i0 < n; i0 += 128) {
-    uint32_t k[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = i0 + 32 * q + lane;
-      k[q] = i < n ? sb.key[i] - kmin : 0u;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = i0 + 32 * q + lane;
-      if (i < n) {
-        sb.key[i] = k[q];
-        atomicAdd(&sb.hist[k[q] & 255u], 1u);
-        if (passes > 1) atomicAdd(&sb.hist[(k[q] >> 8) & 255u], 1u << 16);
-        if (passes > 2) atomicAdd(&sb.hist[256 + ((k[q] >> 16) & 255u)], 1u);
-        if (passes > 3) atomicAdd(&sb.hist[256 + (k[q] >> 24)], 1u << 16);
-      }
-    }
-  }
-}
-
-// n <= 32: rank every (key, index) against the others with shuffles. buffers 0 -> 1, one warp.
-__device__ __forceinline__ void sort_small_compact(const SortBuffers& sb, int n, int lane) {
-  const u64 e = lane < n ? (((u64)sb.key[lane] << 32) | sb.idx[lane]) : ~0ull;
-  int rank = 0;
-  for (int j = 0; j < n; ++j) {
-    const u64 o = __shfl_sync(0xffffffffu, e, j);
-    rank += o < e;
-  }
-  if (lane < n) { sb.keys(1)[rank] = (uint32_t)(e >> 32); sb.idxs(1)[rank] = (unsigned short)e; }
-}
-
-// Lanes of the warp whose 8-bit digit equals this lane's: eight ballots, one per bit (lanes without a key carry
-// a digit >= 256 that is unique to them and are masked out by `actmask`). The match instruction gives the
-// same mask in one go but runs on the SM's single address-divergence unit (about 55 cycles each), which bounds
-// the kernel when every batch uses it; the ballots cost some 40 ALU instructions on the issuing scheduler's own
-// pipe. The sort alternates between the two so that neither unit is the bottleneck.
-__device__ __forceinline__ unsigned digit_peers(unsigned d, unsigned actmask) {
-  unsigned same1 = actmask, any0 = 0u;   // AND of the ballots of this lane's set bits, OR of those of its clear bits
-#pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    const bool bit = (d >> b) & 1u;
-    const unsigned m = __ballot_sync(0xffffffffu, bit);
-    if (bit) same1 &= m; else any0 |= m;
-  }
-  return same1 & ~any0;
-}
-
-// Stable LSD radix sort, 8 bits per pass, one warp; returns which buffer (0/1) holds the result.
-// `top_bits` = significant bits of the last digit (the keys are rebased, so the last digit of a row whose values
-// span a few binades holds one or two bits): with at most two, that pass is a stable four-way split by two
-// ballots per batch, with the class bases read from the digit's histogram -- no ranking, no histogram updates.
-__device__ __forceinline__ int radix_sort_row_compact(const SortBuffers& sb, int n, int lane, int passes, int top_bits) {
-  int cur = 0;
-  const unsigned lt = (1u << lane) - 1u;
-#pragma unroll 1
-  for (int p = 0; p < passes; ++p) {
-    unsigned* h = sb.hist + ((p >> 1) << 8);
-    const int fs = (p & 1) << 4;   // this digit's 16-bit field inside the packed word
-    if (p == passes - 1 && top_bits <= 2) {
-      const unsigned c0 = (h[0] >> fs) & 0xFFFFu, c1 = (h[1] >> fs) & 0xFFFFu, c2 = (h[2] >> fs) & 0xFFFFu;
-      if (c0 == (unsigned)n) continue;   // (cannot happen for a rebased top digit with range > 0; kept for safety)
-      unsigned pos0 = 0u, pos1 = c0, pos2 = c0 + c1, pos3 = c0 + c1 + c2;   // next free slot of each class
-      const uint32_t* srcK = sb.keys(cur);
-      const unsigned short* srcI = sb.idxs(cur);
-      uint32_t* dstK = sb.keys(cur ^ 1);
-      unsigned short* dstI = sb.idxs(cur ^ 1);
-      const int shift = 8 * p;
-      for (int i0 = 0; i0 < n; i0 += 32) {
-        const int i = i0 + lane;
-        const bool act = i < n;
-        const uint32_t k = act ? srcK[i] : 0u;
-        const unsigned short ix = act ? srcI[i] : (unsigned short)0;
-        const unsigned cls = (k >> shift) & 3u;
-        const unsigned am = __ballot_sync(0xffffffffu, act);
-        const unsigned b0 = __ballot_sync(0xffffffffu, act && (cls & 1u));
-        const unsigned b1 = __ballot_sync(0xffffffffu, act && (cls & 2u));
-        const unsigned m0 = am & ~b0 & ~b1, m1 = b0 & ~b1, m2 = b1 & ~b0, m3 = b0 & b1;
-        const unsigned mine = cls == 0u ? m0 : (cls == 1u ? m1 : (cls == 2u ? m2 : m3));
-        const unsigned at = cls == 0u ? pos0 : (cls == 1u ? pos1 : (cls == 2u ? pos2 : pos3));
-        if (act) {
-          const unsigned pos = at + __popc(mine & lt);
-          dstK[pos] = k;
-          dstI[pos] = ix;
-        }
-        pos0 += __popc(m0); pos1 += __popc(m1); pos2 += __popc(m2); pos3 += __popc(m3);
-      }
-      __syncwarp();
-      cur ^= 1;
-      continue;
-    }
-    unsigned wds[8], c[8], s = 0;
-    bool single = false;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      wds[q] = h[lane * 8 + q];
-      c[q] = (wds[q] >> fs) & 0xFFFFu;
-      single |= (c[q] == (unsigned)n);
-      s += c[q];
-    }
-    if (__any_sync(0xffffffffu, single)) continue;   // every key has the same digit here: nothing to do
-    unsigned incl = s;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const unsigned o = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += o;
-    }
-    unsigned run = incl - s;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {   // the field now holds the bin's running offset (<= n < 65536)
-      h[lane * 8 + q] = (wds[q] & ~(0xFFFFu << fs)) | (run << fs);
-      run += c[q];
-    }
-    __syncwarp();
-    const uint32_t* srcK = sb.keys(cur);
-    const unsigned short* srcI = sb.idxs(cur);
-    uint32_t* dstK = sb.keys(cur ^ 1);
-    unsigned short* dstI = sb.idxs(cur ^ 1);
-    const int shift = 8 * p;
-    constexpr int kSB = 4;   // batches of 32 keys whose loads and digit matches go ahead of the serial part
-    for (int i0 = 0; i0 < n; i0 += 32 * kSB) {
-      uint32_t k[kSB];
-      unsigned short ix[kSB];
-      unsigned d[kSB], peers[kSB];
-      bool act[kSB];
-#pragma unroll
-      for (int q = 0; q < kSB; ++q) {
-        const int i = i0 + 32 * q + lane;
-        act[q] = i < n;
-        k[q] = act[q] ? srcK[i] : 0u;
-        ix[q] = act[q] ? srcI[i] : (unsigned short)0;
-        d[q] = act[q] ? (k[q] >> shift) & 255u : 256u + (unsigned)lane;
-      }
-#pragma unroll
-      for (int q = 0; q < kSB; ++q)
-        peers[q] = (q & 1) ? digit_peers(d[q], __ballot_sync(0xffffffffu, act[q])) : __match_any_sync(0xffffffffu, d[q]);
-#pragma unroll
-      for (int q = 0; q < kSB; ++q) {
-        // (a batch past the end of the row has no active lane and does nothing here: no branch around the
-        // warp barriers, so that the compiler sees them in converged code)
-        const unsigned before = peers[q] & lt;
-        unsigned word = 0;
-        if (act[q]) word = h[d[q]];
-        __syncwarp();
-        if (act[q] && before == 0) h[d[q]] = word + ((unsigned)__popc(peers[q]) << fs);
-        __syncwarp();
-        if (act[q]) {
-          const unsigned pos = ((word >> fs) & 0xFFFFu) + __popc(before);
-          dstK[pos] = k[q];
-          dstI[pos] = ix[q];
-        }
-      }
-    }
-    __syncwarp();
-    cur ^= 1;
-  }
-  return cur;
-}
-
 // ------------------------------------------------------------------------------------------- kernels
-// Sort kernel: one warp per row. Shared memory per warp: two key buffers of I entries and the four
-// digit histograms. Sorted keys go to keys_g[r*istride ..], their count to nvalid_g[r].
-__global__ void __launch_bounds__(kFwdThreads)
-snn_sort_kernel(const Geometry g, const float* __restrict__ x, WalkEntry* __restrict__ keys_g, int* __restrict__ nvalid_g,
-                int istride, int row_begin, int row_end) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int I = g.I;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpc = blockDim.x >> 5;
-  // conv: the tap table of the CTA comes first, then the warps' buffers
-  TapTable tt = {nullptr, nullptr};
-  unsigned char* warp_base = smem_raw;
-  if (g.is_conv) {
-    int* off = reinterpret_cast<int*>(smem_raw);
-    unsigned short* khw = reinterpret_cast<unsigned short*>(off + tap_entries(I));
-    for (int i = threadIdx.x; i < tap_entries(I); i += blockDim.x) {
-      int o = 0;
-      unsigned kk = 0;
-      if (i < I) {
-        const int tap = i / g.C, c = i - tap * g.C;
-        const int kh = tap / g.Kw, kw = tap - kh * g.Kw;
-        o = (kh * g.W + kw) * g.C + c;
-        kk = (unsigned)(kh << 8 | kw);
-      }
-      off[i] = o;
-      khw[i] = (unsigned short)kk;
-    }
-    tt.off = off;
-    tt.khw = khw;
-    warp_base += (tap_table_bytes(I) + 15) & ~(size_t)15;
-    __syncthreads();
-  }
-  const SortBuffers sb = sort_buffers(warp_base + (size_t)warp * sort_bytes_per_warp(I), I);
-  for (int r = row_begin + blockIdx.x * wpc + warp; r < row_end; r += gridDim.x * wpc) {
-    uint32_t kmin, kmax;
-    const int n = gather_row_compact(g, x, r, lane, sb, tt, kmin, kmax);
-    __syncwarp();
-    int res = 0;
-    uint32_t base = 0u;   // added back to the keys on the way out
-    if (n > 32) {
-      const uint32_t range = kmax - kmin;
-      const int bits = 32 - __clz(range | 1u);
-      const int passes = (bits + 7) >> 3;   // 8-bit digits that cover the range (1 when range < 256)
-      const int top_bits = bits - 8 * (passes - 1);
-      if (range != 0u) {
-        for (int q = lane; q < 512; q += 32) sb.hist[q] = 0u;
-        __syncwarp();
-        rebase_and_count(sb, n, lane, kmin, passes);
-        __syncwarp();
-        res = radix_sort_row_compact(sb, n, lane, passes, top_bits);
-        base = kmin;
-      }   // else: every key is the same, index order is the sorted order
-    } else {
-      sort_small_compact(sb, n, lane);
-      res = 1;
-    }
-    __syncwarp();
-    WalkEntry* dst = keys_g + (size_t)r * istride;
-    const uint32_t* rk = sb.keys(res);
-    const unsigned short* ri = sb.idxs(res);
-    for (int i = lane; i < n; i += 32)
-      dst[i] = make_uint2(__float_as_uint(sortable_to_float(rk[i] + base)), (uint32_t)ri[i] * (uint32_t)g.J);
-    if (lane == 0) nvalid_g[r] = n;
-    __syncwarp();
-  }
-}
-
-// Rows too long for two buffers per warp: one row per CTA at a time, in-place bitonic network.
-__global__ void __launch_bounds__(kFwdThreads)
-snn_sort_long_kernel(const Geometry g, const float* __restrict__ x, WalkEntry* __restrict__ keys_g,
-                     int* __restrict__ nvalid_g, int istride) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  u64* keys = reinterpret_cast<u64*>(smem_raw);
-  __shared__ int s_n;
-  const int tid = threadIdx.x;
-  for (int r = blockIdx.x; r < g.R; r += gridDim.x) {
-    if (tid < 32) {
-      TapCursor start = {0, 0, 0};
-      if (g.is_conv) start.init(g, tid);
-      const int n = gather_row(g, x, r, tid, keys, nullptr, start);
-      if (tid == 0) s_n = n;
-    }
-    __syncthreads();
-    const int n = s_n;
-    bitonic_sort_cta(keys, n, tid);
-    WalkEntry* dst = keys_g + (size_t)r * istride;
-    for (int i = tid; i < n; i += kFwdThreads) {
-      const u64 e = keys[i];
-      dst[i] = make_uint2(__float_as_uint(key_value(e)), (uint32_t)e * (uint32_t)g.J);
-    }
-    if (tid == 0) nvalid_g[r] = n;
-    __syncthreads();
-  }
-}
-
 // Walk kernel: every warp takes (row, block of 32*JPT outputs) items, adjacent warps share a row.
 template <int JPT, bool VECW, bool STAGE>
 __global__ void __launch_bounds__(kFwdThreads, JPT <= 4 ? 4 : 1)   // up to four outputs per lane: 64 registers, 32 warps per SM
@@ -1195,12 +722,16 @@ int launch_walk2_smemw(const Geometry& g, const WalkEntry* keys_g, const int* nv
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
 
-// Lists of a conv layer are built by per-pixel sorting and merging when the geometry allows it and the row
-// sort would sort every input pixel several times over (3x3 stride 1: nine times).
-bool use_merge_lists(const Geometry& g, const Options& opt) {
+// Lists of a conv layer are built by per-pixel sorting and merging when the geometry allows it and there is enough to do:
+// the bucket sort sorts every input pixel of a 3x3 stride-1 convolution nine times over, but spreads a small layer over the
+// GPU, where the merges are three launches of long serial threads (64 fields of 2304 inputs: 46 against 7 us). The two cross at
+// 4.7 M inputs over all fields for up to 128 channels, at 7 M for 256 and 13 M for 512.
+bool use_merge_lists(const Geometry& g, const Options& opt, const LaunchInfo& li) {
   const int want = opt.list_builder & 3;
   if (want == 1 || want == 3 || !merge_lists_supported(g)) return false;
-  return true;
+  if (want == 2) return true;
+  const double line = 30000.0 * li.num_sms * (g.C > 170 ? g.C / 170.0 : 1.0);
+  return (double)g.R * g.I > line;
 }
 
 // Short rows (a first layer on a few image channels) are sorted by a network in registers.
@@ -1318,7 +849,7 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     return launch_walk<4, false>(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage);
   };
 
-  if (use_merge_lists(g, opt)) {
+  if (use_merge_lists(g, opt, li)) {
     if (fparts & 1) {
       const int rc = launch_merge_lists(g, x, keys_g, nvalid_g, istride, merge_scratch, (opt.list_builder >> 2) - 1, li, s);
       if (rc != OK) return rc;
@@ -1333,53 +864,10 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     return walk(s, 0, g.R);
   }
 
-  const size_t budget = (size_t)li.max_smem_optin - 1024;
-  const size_t per_warp = sort_bytes_per_warp(g.I);
-  const size_t table_min = g.is_conv ? ((tap_table_bytes(g.I) + 15) & ~(size_t)15) : 0;
-  if (table_min + per_warp > budget || g.I > 65535 || (g.is_conv && (g.Kh > 255 || g.Kw > 255))) {
-    // rows too long for the warp sort: one CTA-wide bitonic sort per row, then the walk
-    const size_t smem = (size_t)g.I * sizeof(u64);
-    if (smem > budget) return E_UNSUPPORTED;
-    if (cudaFuncSetAttribute(snn_sort_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget) != cudaSuccess)
-      return E_CUDA;
-    int grid = g.R < li.num_sms ? g.R : li.num_sms;
-    if (fparts & 1) {
-      snn_sort_long_kernel<<<grid, kFwdThreads, smem, s>>>(g, x, keys_g, nvalid_g, istride);
-      count_launch();
-      if (cudaGetLastError() != cudaSuccess) return E_CUDA;
-    }
-    return walk(s, 0, g.R);
+  if (fparts & 1) {
+    const int rc = launch_row_sort(g, x, keys_g, nvalid_g, istride, li, s);
+    if (rc != OK) return rc;
   }
-
-  // warps per CTA and CTAs per SM: the combination that keeps the most rows (warps) resident per SM
-  const size_t table = g.is_conv ? ((tap_table_bytes(g.I) + 15) & ~(size_t)15) : 0;
-  int wpc = 1, ctas_per_sm = 1;
-  {
-    int best = 0;
-    for (int cand = kFwdWarps; cand >= 1; --cand) {
-      if (table + per_warp * cand > budget) continue;
-      int c = (int)(((size_t)li.max_smem_optin) / (table + per_warp * cand + 1024));
-      if (c > 4) c = 4;
-      if (c < 1) c = 1;
-      if (cand * c > best) { best = cand * c; wpc = cand; ctas_per_sm = c; }
-    }
-  }
-  const size_t smem = table + per_warp * wpc;
-  if (cudaFuncSetAttribute(snn_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget) != cudaSuccess)
-    return E_CUDA;
-  auto sort = [&](cudaStream_t st, int r0, int r1) -> int {
-    long grid = ((long)(r1 - r0) + wpc - 1) / wpc;
-    const long cap = (long)li.num_sms * ctas_per_sm;
-    if (grid > cap) grid = cap;
-    snn_sort_kernel<<<(int)grid, wpc * 32, smem, st>>>(g, x, keys_g, nvalid_g, istride, r0, r1);
-    count_launch();
-    return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
-  };
-
-  // Sort, then walk, on the caller's stream. (Running the next block's sort beside the current block's walk
-  // on a second stream was measured and gains nothing: both kernels fill the SMs on their own.)
-  int rc = (fparts & 1) ? sort(s, 0, g.R) : OK;
-  if (rc != OK) return rc;
   return walk(s, 0, g.R);
 }
 

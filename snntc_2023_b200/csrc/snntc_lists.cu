@@ -13,7 +13,7 @@
 // Where a layer has too few row segments or fields to fill the GPU with one thread each (deep layers: small
 // images, many channels), 2 to 16 neighbouring threads share a merge, cut into pieces by value.
 // A sequential two- or three-way merge costs a few dozen instructions per entry and thread and needs no
-// cooperation between threads; the per-field radix sort it replaces spends about five hundred per entry.
+// cooperation between threads; a sort per field spends a few hundred per entry.
 // Each thread streams through its own runs, so what bounds these kernels is the number of memory transactions:
 // the merges read and write 32 bytes (four entries) at a time.
 // The order among equal input values differs from a per-field sort's; no output can spike between two equal
