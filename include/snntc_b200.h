@@ -153,7 +153,8 @@ SNNTC_API int snntc_cv_infer(const float* x_nhwc, const float* w, const float* p
  *                    incoming gradient *gloss (device).
  * snntc_weight_costs / snntc_weight_cost_grads   snntc_weight_cost for `count` tensors at once (the pointer, rows and
  *                    cols arrays are on the host): *cost is written, colsum (sum of cols floats, device) receives the
- *                    column sums in tensor order; the backward writes gw[k] = *gcost * d cost / d w[k] from them.
+ *                    column sums in tensor order; the backward writes gw[k] = *gcost * d cost / d w[k] from them, or adds it to
+ *                    gw[k] when `add` is not 0.
  * snntc_weight_cost  MyModel.constraint_cost for one weight tensor w[rows,J] (snntc-mnist.py:55-59):
  *                    cost[0] += K * mean_j max(0, 1 - sum_i w_ij) + K2 * mean(w^2); gw (may be null) +=
  *                    its gradient. workspace: snntc_weight_cost_workspace_bytes(J) bytes.
@@ -175,7 +176,7 @@ SNNTC_API int snntc_weight_costs(int count, const float* const* w, const int* ro
                                  float* colsum, float* cost, void* workspace, size_t workspace_bytes, void* stream);
 SNNTC_API int snntc_weight_cost_grads(int count, const float* const* w, float* const* gw, const int* rows,
                                       const int* cols, float K, float K2, const float* colsum, const float* gcost,
-                                      void* stream);
+                                      int add, void* stream);
 SNNTC_API size_t snntc_weight_cost_workspace_bytes(int J);
 SNNTC_API int snntc_weight_cost(const float* w, float* gw, float* cost, int rows, int J, float K, float K2,
                                 void* workspace, size_t workspace_bytes, void* stream);

@@ -40,7 +40,7 @@ SYMBOLS = {
     "snntc_loss_backward": (_INT, [_F, _F, _F, _F, _INT, _INT, ctypes.c_float, _F]),
     "snntc_weight_costs_workspace_bytes": (_SZ, [_INT, _F, _F]),
     "snntc_weight_costs": (_INT, [_INT, _F, _F, _F, ctypes.c_float, ctypes.c_float, _F, _F, _F, _SZ, _F]),
-    "snntc_weight_cost_grads": (_INT, [_INT, _F, _F, _F, _F, ctypes.c_float, ctypes.c_float, _F, _F, _F]),
+    "snntc_weight_cost_grads": (_INT, [_INT, _F, _F, _F, _F, ctypes.c_float, ctypes.c_float, _F, _F, _INT, _F]),
     "snntc_weight_cost_workspace_bytes": (_SZ, [_INT]),
     "snntc_weight_cost": (_INT, [_F, _F, _F, _INT, _INT, ctypes.c_float, ctypes.c_float, _F, _SZ, _F]),
     "snntc_adam_step": (_INT, [_F, _F, _F, _F, _SZ] + [ctypes.c_float] * 5 + [_F, _F]),

@@ -104,7 +104,7 @@ int launch_merge_lists(const Geometry& g, const float* x, WalkEntry* lists, int*
 
 // The walk with one output per lane and weight rows copied ahead into shared memory (snntc_walk_ring.cu); any shape.
 int launch_walk_ring(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
-                     cudaStream_t s);
+                     const LaunchInfo& li, cudaStream_t s);
 
 // Sorted lists of everything else by a bucket sort per row (snntc_sort.cu).
 int launch_row_sort(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride, const LaunchInfo& li,

@@ -832,7 +832,7 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
                      ((opt.walk_layout & 8) != 0 || ((opt.walk_layout & 3) == 0 && g.J == 64 && g.R >= 8192));
   auto walk = [&](cudaStream_t st, int r0, int r1) -> int {
     if (!(fparts & 2)) return OK;
-    if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, st);
+    if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, li, st);
     if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage, smemw_bytes, smemw_shift);
     if (variant == 1) {
       // pairs layout: 64 outputs per warp, or (walk_outputs 3) 128 as two pairs per lane

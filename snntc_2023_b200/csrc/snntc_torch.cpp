@@ -10,7 +10,9 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <algorithm>
 #include <cstring>
+#include <mutex>
 
 #include "../../include/snntc_b200.h"
 
@@ -402,6 +404,50 @@ struct WeightList {
   }
 };
 
+void cost_grads(const variable_list& ws, const variable_list& gw, const CostState& s, const Tensor& g, bool add) {
+  const c10::cuda::CUDAGuard guard(g.device());
+  WeightList l;
+  std::vector<float*> to;
+  for (const Tensor& t : ws) l.add(t);
+  for (const Tensor& t : gw) to.push_back(ptr(t));
+  check(snntc_weight_cost_grads((int)ws.size(), l.w.data(), to.data(), l.rows.data(), l.cols.data(), s.K, s.K2, ptr(s.colsum),
+                                ptr(g), add ? 1 : 0, stream_of(g)), "constraint_cost");
+}
+
+// A backward pass in which the gradient of a network's constraint cost is added straight to the flat gradient bucket that the
+// layers' dW kernels write (SnnNet.backward), instead of going through one gradient tensor per weight, an accumulation each
+// and an addition: the cost's node leaves what it would have computed here, and it is computed once autograd is through --
+// the dW kernels write their slices, in whatever order autograd visits the nodes.
+struct Fold {
+  struct Pending { variable_list weights; c10::intrusive_ptr<CostState> state; Tensor grad; };
+  std::vector<const void*> weights;
+  variable_list sinks;
+  std::vector<Pending> pending;
+  const Tensor* sink_of(const Tensor& w) const {
+    for (size_t k = 0; k < weights.size(); ++k)
+      if (weights[k] == w.data_ptr()) return &sinks[k];
+    return nullptr;
+  }
+};
+std::mutex g_fold_mutex;
+std::vector<Fold*> g_folds;      // the backward passes of this kind under way, one per calling thread
+
+// true: some pass under way takes the cost's gradient itself (exactly one does, and it knows every weight)
+bool fold_cost(const variable_list& ws, const c10::intrusive_ptr<CostState>& s, const Tensor& g) {
+  const std::lock_guard<std::mutex> lock(g_fold_mutex);
+  Fold* owner = nullptr;
+  for (Fold* f : g_folds) {
+    size_t known = 0;
+    for (const Tensor& w : ws) known += f->sink_of(w) != nullptr;
+    if (known == 0) continue;
+    if (known < ws.size() || owner != nullptr) return false;
+    owner = f;
+  }
+  if (owner == nullptr) return false;
+  owner->pending.push_back({ws, s, g});
+  return true;
+}
+
 struct CostFunction : torch::autograd::Function<CostFunction> {
   static Tensor forward(AutogradContext* ctx, at::TensorList weights, c10::intrusive_ptr<CostState> s) {
     variable_list ws;
@@ -423,21 +469,38 @@ struct CostFunction : torch::autograd::Function<CostFunction> {
     const auto ws = ctx->get_saved_variables();
     const auto s = c10::static_intrusive_pointer_cast<CostState>(ctx->saved_data["call"].toCapsule());
     const Tensor g = as_cuda_f32(grads[0], "gradient of the cost");
-    const c10::cuda::CUDAGuard guard(g.device());
-    WeightList l;
+    if (fold_cost(ws, s, g)) return variable_list(ws.size() + 1);
     variable_list out;
-    std::vector<float*> gw;
-    for (const Tensor& t : ws) {
-      l.add(t);
-      out.push_back(at::empty_like(t));
-      gw.push_back(ptr(out.back()));
-    }
-    check(snntc_weight_cost_grads((int)ws.size(), l.w.data(), gw.data(), l.rows.data(), l.cols.data(), s->K, s->K2, ptr(s->colsum),
-                                  ptr(g), stream_of(g)), "constraint_cost");
+    for (const Tensor& t : ws) out.push_back(at::empty_like(t));
+    cost_grads(ws, out, *s, g, false);
     out.push_back(Tensor());
     return out;
   }
 };
+
+// objective.backward() with the upstream gradient `one`; constraint costs of `weights` go into `sinks` (see Fold)
+void backward(const Tensor& objective, const Tensor& one, const std::vector<Tensor>& weights, const std::vector<Tensor>& sinks) {
+  Fold f;
+  for (const Tensor& w : weights) f.weights.push_back(w.data_ptr());
+  f.sinks = sinks;
+  struct Enter {
+    Fold* f;
+    explicit Enter(Fold* p) : f(p) { const std::lock_guard<std::mutex> lock(g_fold_mutex); g_folds.push_back(f); }
+    ~Enter() {
+      const std::lock_guard<std::mutex> lock(g_fold_mutex);
+      g_folds.erase(std::find(g_folds.begin(), g_folds.end(), f));
+    }
+  };
+  {
+    const Enter entered(&f);
+    torch::autograd::backward({objective}, {one});
+  }
+  for (const Fold::Pending& p : f.pending) {
+    variable_list to;
+    for (const Tensor& w : p.weights) to.push_back(*f.sink_of(w));
+    cost_grads(p.weights, to, *p.state, p.grad, true);
+  }
+}
 
 Tensor constraint_cost(const std::vector<Tensor>& weights, double K, double K2) {
   TORCH_CHECK_VALUE(!weights.empty(), "constraint_cost needs at least one weight");
@@ -481,5 +544,6 @@ PYBIND11_MODULE(_native, m) {
   m.def("encode", &encode, py::call_guard<py::gil_scoped_release>());
   m.def("loss", &loss, py::call_guard<py::gil_scoped_release>());
   m.def("constraint_cost", &constraint_cost, py::call_guard<py::gil_scoped_release>());
+  m.def("backward", &backward, py::call_guard<py::gil_scoped_release>());
   m.def("adam_step", &adam_step, py::call_guard<py::gil_scoped_release>());
 }

@@ -370,7 +370,8 @@ cost_total_kernel(const __grid_constant__ CostTensors c, const float* __restrict
   if (blockIdx.x == 0 && threadIdx.x == 0) *cost = add ? *cost + sum.x : sum.x;
 }
 
-// gw = gcost * (-K/J [colsum < 1] + 2 K2 / n * w), a CTA per 4096 elements of one tensor
+// gw = gcost * (-K/J [colsum < 1] + 2 K2 / n * w), or gw += it, a CTA per 4096 elements of one tensor
+template <bool ADD>
 __global__ void __launch_bounds__(kCostThreads)
 cost_grad_kernel(const __grid_constant__ CostTensors c, const float* __restrict__ colsum, const float* __restrict__ gcost,
                  float K, float K2) {
@@ -393,11 +394,19 @@ cost_grad_kernel(const __grid_constant__ CostTensors c, const float* __restrict_
       r.y = ((1.0f - __ldg(cs + j + 1)) > 0.f ? a : 0.f) + b2 * v.y;
       r.z = ((1.0f - __ldg(cs + j + 2)) > 0.f ? a : 0.f) + b2 * v.z;
       r.w = ((1.0f - __ldg(cs + j + 3)) > 0.f ? a : 0.f) + b2 * v.w;
-      *reinterpret_cast<float4*>(gw + e) = make_float4(up * r.x, up * r.y, up * r.z, up * r.w);
+      // (the product is rounded before it is added, as when a gradient tensor of its own is added to the bucket)
+      float4 o = make_float4(__fmul_rn(up, r.x), __fmul_rn(up, r.y), __fmul_rn(up, r.z), __fmul_rn(up, r.w));
+      if (ADD) {
+        const float4 have = *reinterpret_cast<const float4*>(gw + e);
+        o = make_float4(have.x + o.x, have.y + o.y, have.z + o.z, have.w + o.w);
+      }
+      *reinterpret_cast<float4*>(gw + e) = o;
     }
   } else {
-    for (unsigned e = e0 + threadIdx.x; e < e1; e += kCostThreads)
-      gw[e] = up * (((1.0f - __ldg(cs + e % (unsigned)J)) > 0.f ? a : 0.f) + b2 * __ldg(w + e));
+    for (unsigned e = e0 + threadIdx.x; e < e1; e += kCostThreads) {
+      const float r = __fmul_rn(up, ((1.0f - __ldg(cs + e % (unsigned)J)) > 0.f ? a : 0.f) + b2 * __ldg(w + e));
+      gw[e] = ADD ? gw[e] + r : r;
+    }
   }
 }
 
@@ -518,7 +527,7 @@ int snntc_weight_costs(int count, const float* const* w, const int* rows, const 
 }
 
 int snntc_weight_cost_grads(int count, const float* const* w, float* const* gw, const int* rows, const int* cols, float K,
-                            float K2, const float* colsum, const float* gcost, void* stream) {
+                            float K2, const float* colsum, const float* gcost, int add, void* stream) {
   if (!w || !gw || !rows || !cols || !colsum || !gcost) return SNNTC_E_NULL;
   if (count <= 0) return SNNTC_E_SHAPE;
   for (int k = 0; k < count; ++k) {
@@ -528,7 +537,8 @@ int snntc_weight_cost_grads(int count, const float* const* w, float* const* gw, 
   }
   for (int at = 0; at < count; at += kCostMax) {
     const CostTensors c = cost_tensors(count, w, gw, rows, cols, at);
-    cost_grad_kernel<<<c.first_chunk[c.count], kCostThreads, 0, (cudaStream_t)stream>>>(c, colsum, gcost, K, K2);
+    if (add) cost_grad_kernel<true><<<c.first_chunk[c.count], kCostThreads, 0, (cudaStream_t)stream>>>(c, colsum, gcost, K, K2);
+    else cost_grad_kernel<false><<<c.first_chunk[c.count], kCostThreads, 0, (cudaStream_t)stream>>>(c, colsum, gcost, K, K2);
     if (done() != SNNTC_OK) return SNNTC_E_CUDA;
     colsum += c.first_col[c.count];
   }

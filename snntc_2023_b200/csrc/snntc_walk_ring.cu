@@ -3,7 +3,7 @@
 //
 // With few warps on an SM a walk is bound by latency: the walk from global memory (snntc_forward.cu) waits an L2 round trip for
 // every four to eight weight rows and a vote with its branch at every step, 75 to 130 cycles a step. Here
-//   - weight rows arrive by asynchronous copies, 32 entries to a block, two blocks ahead of the one that is consumed;
+//   - weight rows arrive by asynchronous copies, 32 (or 16) entries to a block, two blocks ahead of the one that is consumed;
 //   - the sums and sign tests of eight steps are formed before one vote, from operands that were read a group ahead. The sums in front of every step of the group stay in
 //     registers, so where the vote finds an output at or near zero, only the steps concerned are taken through the
 //     reference's own comparisons (snntc/snnfc_kernels.cu.cc:46-55) and nothing is replayed (groups of four without the read
@@ -27,11 +27,11 @@ namespace snntc {
 namespace {
 
 constexpr int kWarps = 2;                          // per CTA, each on an item of its own
-constexpr int kBlock = 32;                         // list entries per block
 constexpr int kRing = 3;                           // weight blocks per warp: one consumed, two on their way
 constexpr int kListRing = 4;                       // list blocks per warp
 constexpr int kGroup = 8;                          // steps per vote
 
+template <int kBlock>
 struct RingWarp {
   float w[kRing][kBlock][32];
   float x[kListRing][kBlock];
@@ -87,14 +87,15 @@ struct Walk {
   }
 };
 
-// VEC: J is a multiple of 4 and w 16-byte aligned: 16-byte weight copies, else 4-byte ones.
-template <bool VEC>
+// VEC: J is a multiple of 4 and w 16-byte aligned: 16-byte weight copies, else 4-byte ones. kBlock: list entries per block, 32,
+// or 16 where there are warps to fill the SMs (half the shared memory per warp: 58 against 68 us for 784 -> 400 at 256 samples).
+template <bool VEC, int kBlock>
 __global__ void __launch_bounds__(32 * kWarps)
 snn_walk_ring_kernel(const Geometry g, const WalkEntry* __restrict__ lists, const int* __restrict__ nvalid, int istride,
                      const float* __restrict__ w, float* __restrict__ out, int slices) {
-  __shared__ __align__(16) RingWarp ring[kWarps];
+  __shared__ __align__(16) RingWarp<kBlock> ring[kWarps];
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
-  RingWarp& sm = ring[warp];
+  RingWarp<kBlock>& sm = ring[warp];
   const int J = g.J;
   // neighbouring items are rows of the same output slice: the slice's weights stay in L2 while they run
   const long item = (long)blockIdx.x * kWarps + warp;
@@ -109,11 +110,13 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
   WalkEntry pre = make_uint2(0u, 0u);
   auto read_list = [&](int b) {
     pre = make_uint2(0u, 0u);
-    if (b * kBlock + lane < n) pre = __ldcg(ents + b * kBlock + lane);
+    if ((kBlock == 32 || lane < kBlock) && b * kBlock + lane < n) pre = __ldcg(ents + b * kBlock + lane);
   };
   auto put_list = [&](int b) {
-    sm.x[b % kListRing][lane] = __uint_as_float(pre.x);
-    sm.off[b % kListRing][lane] = pre.y;
+    if (kBlock == 32 || lane < kBlock) {
+      sm.x[b % kListRing][lane] = __uint_as_float(pre.x);
+      sm.off[b % kListRing][lane] = pre.y;
+    }
   };
   // weight block b. VEC: a copy brings four rows of 32 outputs, 16 bytes per lane (columns outside the row: column 0 again)
   // Else 4 bytes per lane, 32 / columns rows at a time.
@@ -224,14 +227,15 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
 }  // namespace
 
 int launch_walk_ring(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
-                     cudaStream_t s) {
+                     const LaunchInfo& li, cudaStream_t s) {
   const int slices = (g.J + 31) / 32;
   const long grid = ((long)g.R * slices + kWarps - 1) / kWarps;
   if (grid > 0x7fffffffL) return E_UNSUPPORTED;
-  if ((g.J & 3) == 0 && ((uintptr_t)w & 15) == 0)
-    snn_walk_ring_kernel<true><<<(unsigned)grid, 32 * kWarps, 0, s>>>(g, lists, nvalid, istride, w, out, slices);
-  else
-    snn_walk_ring_kernel<false><<<(unsigned)grid, 32 * kWarps, 0, s>>>(g, lists, nvalid, istride, w, out, slices);
+  const bool vec = (g.J & 3) == 0 && ((uintptr_t)w & 15) == 0;
+  const bool small = grid * kWarps > 8L * li.num_sms;
+  auto go = [&](auto kernel) { kernel<<<(unsigned)grid, 32 * kWarps, 0, s>>>(g, lists, nvalid, istride, w, out, slices); };
+  if (vec) small ? go(snn_walk_ring_kernel<true, 16>) : go(snn_walk_ring_kernel<true, 32>);
+  else small ? go(snn_walk_ring_kernel<false, 16>) : go(snn_walk_ring_kernel<false, 32>);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }

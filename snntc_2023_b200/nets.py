@@ -11,6 +11,7 @@ A network is described by a list of layer specs:
 import numpy as np
 import torch
 
+from . import _lib
 from .SNN_TC_Modules import SNN_conv, SNN_dense, SNN_maxpool2d, init_weight, loss_func
 
 MNIST_MLP = [("dense", 784, 400), ("dense", 400, 400), ("dense", 400, 10)]
@@ -81,6 +82,7 @@ class SnnNet(torch.nn.Module):
     def __init__(self, specs, weights=None, biasvolt=1.0, device="cuda"):
         super().__init__()
         self.specs = list(specs)
+        self._one = None
         layers = []
         wi = 0
         for s in self.specs:
@@ -136,11 +138,19 @@ class SnnNet(torch.nn.Module):
         by the kernels) plus whatever autograd accumulated in a weight's .grad for the other terms. The .grad
         of every weight is left pointing at its slice of flat_grad, for optimisers that read .grad."""
         ws = self.weighted_layers()
-        for l in ws:
-            l.weight.grad = None
-        objective.backward()
-        more = [l for l in ws if l.weight.grad is not None]
-        if more:   # one launch for all layers
-            torch._foreach_add_([l.grad_sink for l in more], [l.weight.grad for l in more])
-        for l in ws:
-            l.weight.grad = l.grad_sink
+        weights, sinks = [l.weight for l in ws], [l.grad_sink for l in ws]
+        for w in weights:
+            w.grad = None
+        # (a hook on a weight is to see the cost's gradient: autograd's own way then)
+        if (objective.dim() == 0 and objective.is_cuda and objective.dtype == torch.float32 and
+                not any(w._backward_hooks for w in weights)):
+            if self._one is None or self._one.device != objective.device:
+                self._one = torch.ones((), device=objective.device)
+            _lib.native().backward(objective, self._one, weights, sinks)   # adds a constraint cost's gradient to flat_grad itself
+        else:
+            objective.backward()
+        more = [k for k, w in enumerate(weights) if w.grad is not None]
+        if more:   # any other term: one launch for all layers
+            torch._foreach_add_([sinks[k] for k in more], [weights[k].grad for k in more])
+        for w, sink in zip(weights, sinks):
+            w.grad = sink
