@@ -24,7 +24,8 @@ def init_weight(in_size=1, out_size=1, bias_volt=1.0, init_param=15.0):
 
 def _to_weight(weight):
     if isinstance(weight, torch.Tensor):
-        return weight.detach().to(torch.float32).cpu().clone()
+        w = weight.detach().to(torch.float32)
+        return w.cpu() if w.is_cuda else w.clone()   # one copy of one's own: a second one wakes every thread of the CPU pool
     return torch.from_numpy(np.array(weight).astype(np.float32))
 
 

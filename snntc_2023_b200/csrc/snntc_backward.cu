@@ -41,6 +41,8 @@ template <bool V4, bool BLOCK_FLAGS>   // V4: n and nx are multiples of 4 and al
 __global__ void snn_u_kernel(const float* __restrict__ grad, const float* __restrict__ out, float* __restrict__ u,
                              size_t n, float maxcomp, const float* __restrict__ xin, size_t nx, float maxv,
                              int* __restrict__ exact_flag, unsigned* __restrict__ nz_count) {
+  chain_wait();
+  chain_next();
   const float tiny = 8.67361737988e-19f;   // 2^-60
   const float big = 1.26765060023e30f;     // 2^100
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -119,6 +121,8 @@ template <bool VEC>   // VEC: J % 4 == 0, tiles are fetched with 16-byte loads
 __global__ void __launch_bounds__(kBwdThreads)
 snn_dx_kernel(const DxGate gate, const Geometry g, const float* __restrict__ uv, const float* __restrict__ x,
               const float* __restrict__ w, const float* __restrict__ out, float* __restrict__ dx) {
+  chain_wait();
+  chain_next();
   if (gate.nz != nullptr && __ldg(gate.nz) <= gate.threshold) return;   // the list-walking kernel takes this call
   __shared__ __align__(16) float Ys[2][kTile * kJTP];
   __shared__ __align__(16) float Us[2][kTile * kJTP];
@@ -301,6 +305,8 @@ constexpr int kWStride = kTile + 4;
 __global__ void __launch_bounds__(kBwdThreads)
 snn_dx_wide_kernel(const DxGate gate, const Geometry g, const float* __restrict__ uv, const float* __restrict__ x,
                    const float* __restrict__ w, const float* __restrict__ out, float* __restrict__ dx) {
+  chain_wait();
+  chain_next();
   if (gate.nz != nullptr && __ldg(gate.nz) <= gate.threshold) return;   // the list-walking kernel takes this call
   __shared__ __align__(16) float Ys[2][kJT * kYStride];
   __shared__ __align__(16) float Us[2][kJT * kYStride];
@@ -468,6 +474,8 @@ __global__ void __launch_bounds__(kBwdThreads, 3)
 snn_dw_kernel(const Geometry g, const float* __restrict__ uv, const float* __restrict__ x,
               const float* __restrict__ out, float* __restrict__ partial, int rows_per_split,
               float scale, const int* __restrict__ exact_flag) {
+  chain_wait();
+  chain_next();
   // -x*s, y*s and -u/s as plain tiles. A two-lane FMA covers two neighbouring output columns of one fan-in row,
   // so its 64-bit operands are pairs of neighbouring columns straight out of a 16-byte read of the u tile.
   __shared__ __align__(16) float Xs[2][kRT * kTileI];
@@ -671,6 +679,8 @@ __global__ void __launch_bounds__(kBwdThreads)
 snn_dw_small_kernel(const Geometry g, const float* __restrict__ uv, const float* __restrict__ x,
                     const float* __restrict__ out, float* __restrict__ partial, int rows_per_split,
                     float scale, const int* __restrict__ exact_flag) {
+  chain_wait();
+  chain_next();
   constexpr int JJ = 8 * JB;              // fan-out
   constexpr int RS = 4096 / JJ < 64 ? 4096 / JJ : 64;   // rows r per stage: the u and y tiles are at most 16 KB each
   __shared__ __align__(16) float Us[RS * JJ];
@@ -805,6 +815,8 @@ static int dw_small_splits(const Geometry& g, const LaunchInfo& li, int* rows_pe
 // same bits every run, and eight independent loads in flight per thread -- a kernel with a few ten thousand
 // threads and hundreds of planes is bound by load latency otherwise.
 __global__ void snn_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, size_t n, int splits) {
+  chain_wait();
+  chain_next();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
     float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
@@ -932,12 +944,12 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
     // u and one range flag per block of the u kernel (at most 64: a quarter of a megabyte per block at the largest sizes
     // this path takes is still a few microseconds), then both gradients in one launch
     const size_t n = (size_t)g.R * g.J, nx = (size_t)g.R * g.I;
-    size_t blocks = (std::max(n, nx) / 4 + 255) / 256;
+    size_t blocks = (std::max(n, nx) / 4 + 1023) / 1024;
     if (blocks > kFlagBlocks) blocks = kFlagBlocks;
     if (blocks < 1) blocks = 1;
     const bool v4 = (n % 4 == 0) && (nx % 4 == 0) && (((uintptr_t)grad | (uintptr_t)out | (uintptr_t)uv | (uintptr_t)x) & 15) == 0;
-    if (v4) snn_u_kernel<true, true><<<(int)blocks, 1024, 0, s>>>(grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nullptr);
-    else snn_u_kernel<false, true><<<(int)blocks, 1024, 0, s>>>(grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nullptr);
+    if (v4) (void)launch_chained(snn_u_kernel<true, true>, (int)blocks, 1024, 0, s, 0, grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nullptr);
+    else (void)launch_chained(snn_u_kernel<false, true>, (int)blocks, 1024, 0, s, 0, grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nullptr);
     count_launch();
     if (cudaGetLastError() != cudaSuccess) return E_CUDA;
     const DwPlan p = plan_dw(g, li);
@@ -952,8 +964,8 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
     const size_t nx = g.is_conv ? (size_t)g.B * g.H * g.W * g.C : (size_t)g.R * g.I;
     const bool v4 = (n % 4 == 0) && (nx % 4 == 0) &&
                     (((uintptr_t)grad | (uintptr_t)out | (uintptr_t)uv | (uintptr_t)x) & 15) == 0;
-    if (v4) snn_u_kernel<true, false><<<(int)blocks, 256, 0, s>>>(grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nz_count);
-    else snn_u_kernel<false, false><<<(int)blocks, 256, 0, s>>>(grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nz_count);
+    if (v4) (void)launch_chained(snn_u_kernel<true, false>, (int)blocks, 256, 0, s, 0, grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nz_count);
+    else (void)launch_chained(snn_u_kernel<false, false>, (int)blocks, 256, 0, s, 0, grad, out, uv, n, g.maxv - 0.1f, x, nx, g.maxv, exact_flag, nz_count);
     count_launch();
     if (cudaGetLastError() != cudaSuccess) return E_CUDA;
   }
@@ -984,11 +996,11 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
     if (rc == OK && (!sparse_ok || both)) {
       if (vec && P >= 64 * kWideP && (reinterpret_cast<uintptr_t>(dx) & 15) == 0) {   // it stores dx 16 bytes at a time
         dim3 gridw((unsigned)((P + kWideP - 1) / kWideP), (CH + kTile - 1) / kTile);
-        snn_dx_wide_kernel<<<gridw, kBwdThreads, 0, sdx>>>(gate, g, uv, x, w, out, dx);
+        (void)launch_chained(snn_dx_wide_kernel, gridw, kBwdThreads, 0, sdx, 0, gate, g, uv, x, w, out, dx);
       } else if (vec) {
-        snn_dx_kernel<true><<<grid, kBwdThreads, 0, sdx>>>(gate, g, uv, x, w, out, dx);
+        (void)launch_chained(snn_dx_kernel<true>, grid, kBwdThreads, 0, sdx, 0, gate, g, uv, x, w, out, dx);
       } else {
-        snn_dx_kernel<false><<<grid, kBwdThreads, 0, sdx>>>(gate, g, uv, x, w, out, dx);
+        (void)launch_chained(snn_dx_kernel<false>, grid, kBwdThreads, 0, sdx, 0, gate, g, uv, x, w, out, dx);
       }
       count_launch();
       if (cudaGetLastError() != cudaSuccess) rc = E_CUDA;
@@ -1014,7 +1026,7 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
       if (rc == OK) {
         int blocks = (int)((n + 255) / 256);
         if (blocks > 4 * li.num_sms) blocks = 4 * li.num_sms;
-        snn_dw_reduce_kernel<<<blocks, 256, 0, s>>>(partial, dw, n, splits);
+        (void)launch_chained(snn_dw_reduce_kernel, blocks, 256, 0, s, 0, partial, dw, n, splits);
         count_launch();
         if (cudaGetLastError() != cudaSuccess) rc = E_CUDA;
       }
@@ -1023,16 +1035,16 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
       splits = dw_small_splits(g, li, &rps);
       partial = planes;
       dim3 grid(1, 1, splits);
-      if (g.J == 32) snn_dw_small_kernel<4><<<grid, kBwdThreads, 0, s>>>(g, uv, x, out, partial, rps, scale, exact_flag);
-      else if (g.J == 64) snn_dw_small_kernel<8><<<grid, kBwdThreads, 0, s>>>(g, uv, x, out, partial, rps, scale, exact_flag);
-      else if (g.J == 128) snn_dw_small_kernel<16><<<grid, kBwdThreads, 0, s>>>(g, uv, x, out, partial, rps, scale, exact_flag);
-      else snn_dw_small_kernel<32><<<grid, kBwdThreads, 0, s>>>(g, uv, x, out, partial, rps, scale, exact_flag);
+      if (g.J == 32) (void)launch_chained(snn_dw_small_kernel<4>, grid, kBwdThreads, 0, s, 0, g, uv, x, out, partial, rps, scale, exact_flag);
+      else if (g.J == 64) (void)launch_chained(snn_dw_small_kernel<8>, grid, kBwdThreads, 0, s, 0, g, uv, x, out, partial, rps, scale, exact_flag);
+      else if (g.J == 128) (void)launch_chained(snn_dw_small_kernel<16>, grid, kBwdThreads, 0, s, 0, g, uv, x, out, partial, rps, scale, exact_flag);
+      else (void)launch_chained(snn_dw_small_kernel<32>, grid, kBwdThreads, 0, s, 0, g, uv, x, out, partial, rps, scale, exact_flag);
       count_launch();
       if (cudaGetLastError() != cudaSuccess) rc = E_CUDA;
       if (rc == OK) {
         int blocks = (int)((n + 255) / 256);
         if (blocks > 4 * li.num_sms) blocks = 4 * li.num_sms;
-        snn_dw_reduce_kernel<<<blocks, 256, 0, s>>>(partial, dw, n, splits);
+        (void)launch_chained(snn_dw_reduce_kernel, blocks, 256, 0, s, 0, partial, dw, n, splits);
         count_launch();
         if (cudaGetLastError() != cudaSuccess) rc = E_CUDA;
       }
@@ -1040,14 +1052,14 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
       const DwPlan p = plan_dw(g, li);
       if (p.splits > 1) partial = planes;
       dim3 grid((g.J + kTile - 1) / kTile, (Itot + kTileI - 1) / kTileI, p.splits);
-      if (vec) snn_dw_kernel<true><<<grid, kBwdThreads, 0, s>>>(g, uv, x, out, partial, p.rows_per_split, scale, exact_flag);
-      else snn_dw_kernel<false><<<grid, kBwdThreads, 0, s>>>(g, uv, x, out, partial, p.rows_per_split, scale, exact_flag);
+      if (vec) (void)launch_chained(snn_dw_kernel<true>, grid, kBwdThreads, 0, s, 0, g, uv, x, out, partial, p.rows_per_split, scale, exact_flag);
+      else (void)launch_chained(snn_dw_kernel<false>, grid, kBwdThreads, 0, s, 0, g, uv, x, out, partial, p.rows_per_split, scale, exact_flag);
       count_launch();
       if (cudaGetLastError() != cudaSuccess) rc = E_CUDA;
       if (rc == OK && p.splits > 1) {
         int blocks = (int)((n + 255) / 256);
         if (blocks > 4 * li.num_sms) blocks = 4 * li.num_sms;
-        snn_dw_reduce_kernel<<<blocks, 256, 0, s>>>(partial, dw, n, p.splits);
+        (void)launch_chained(snn_dw_reduce_kernel, blocks, 256, 0, s, 0, partial, dw, n, p.splits);
         count_launch();
         if (cudaGetLastError() != cudaSuccess) rc = E_CUDA;
       }

@@ -114,6 +114,8 @@ __device__ __forceinline__ void store_tile(const float* tile, int lane, float* _
 template <bool VX, bool VJ, int ML, int NL>
 __global__ void __launch_bounds__(kThreads, 3)
 snn_dense_bwd_kernel(const DenseArgs a, const DensePlan p) {
+  chain_wait();
+  chain_next();
   extern __shared__ __align__(16) float smem[];
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   float* mine = smem + warp * kWarpFloats;
@@ -359,20 +361,9 @@ snn_dense_bwd_kernel(const DenseArgs a, const DensePlan p) {
 
 template <bool VX, bool VJ, int ML, int NL>
 int launch(const DenseArgs& a, const DensePlan& p, cudaStream_t s) {
-  if (cudaFuncSetAttribute(snn_dense_bwd_kernel<VX, VJ, ML, NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) != cudaSuccess)
-    return E_CUDA;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((p.dx_clusters + p.dw_clusters) * p.cluster));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmemBytes;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)p.cluster;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, snn_dense_bwd_kernel<VX, VJ, ML, NL>, a, p);
+  if (allow_smem<snn_dense_bwd_kernel<VX, VJ, ML, NL>>(kSmemBytes) != cudaSuccess) return E_CUDA;
+  const cudaError_t e = launch_chained(snn_dense_bwd_kernel<VX, VJ, ML, NL>, dim3((unsigned)((p.dx_clusters + p.dw_clusters) * p.cluster)),
+                                       dim3(kThreads), kSmemBytes, s, (unsigned)p.cluster, a, p);
   count_launch();
   return e == cudaSuccess ? OK : E_CUDA;
 }

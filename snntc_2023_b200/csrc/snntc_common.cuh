@@ -1,5 +1,7 @@
 // Shared definitions for the SNN-TC sm_100a kernels.
 #pragma once
+#include "snntc_launch.cuh"
+
 #include <cuda_runtime.h>
 #include <stdint.h>
 

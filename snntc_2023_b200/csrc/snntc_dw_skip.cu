@@ -60,6 +60,8 @@ __global__ void __launch_bounds__(kThreads, 2)
 snn_dw_skip_kernel(const Geometry g, const float* __restrict__ uv, const float* __restrict__ x,
                    const float* __restrict__ out, float* __restrict__ partial, int rows_per_split,
                    float scale, const int* __restrict__ exact_flag) {
+  chain_wait();
+  chain_next();
   constexpr int kTI = 128 * QL;        // fan-in rows per CTA
   constexpr int kCh = 32 * QL;         // 16-byte chunks per row of the x tile
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -251,9 +253,9 @@ template <int QL>
 int launch_ql(const Geometry& g, const float* uv, const float* x, const float* out, float* partial, dim3 grid,
               int rows_per_split, float scale, const int* exact_flag, cudaStream_t s) {
   const size_t smem = smem_bytes(QL);
-  if (cudaFuncSetAttribute(snn_dw_skip_kernel<QL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (allow_smem<snn_dw_skip_kernel<QL>>(smem) != cudaSuccess)
     return E_CUDA;
-  snn_dw_skip_kernel<QL><<<grid, kThreads, smem, s>>>(g, uv, x, out, partial, rows_per_split, scale, exact_flag);
+  (void)launch_chained(snn_dw_skip_kernel<QL>, grid, kThreads, smem, s, 0, g, uv, x, out, partial, rows_per_split, scale, exact_flag);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }

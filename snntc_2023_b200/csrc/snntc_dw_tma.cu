@@ -75,6 +75,8 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                   const __grid_constant__ CUtensorMap map_u, const Geometry g, float* __restrict__ partial,
                   int stages_per_split, float scale, const int* __restrict__ exact_flag, int taps_per_tile,
                   int wseg_log2) {
+  chain_wait();
+  chain_next();
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long bars[2];
   unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);   // boxes land on 128-byte boundaries
@@ -312,9 +314,9 @@ long stage_count(const Geometry& g) {
 template <int QL, bool C256>
 int launch_ql(const CUtensorMap& mx, const CUtensorMap& my, const CUtensorMap& mu, const Geometry& g, float* partial,
               dim3 grid, int stages_per_split, float scale, const int* exact_flag, const TmaPlan& p, cudaStream_t s) {
-  if (cudaFuncSetAttribute(snn_dw_tma_kernel<QL, C256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess)
+  if (allow_smem<snn_dw_tma_kernel<QL, C256>>(p.smem) != cudaSuccess)
     return E_CUDA;
-  snn_dw_tma_kernel<QL, C256><<<grid, kThreads, p.smem, s>>>(mx, my, mu, g, partial, stages_per_split, scale, exact_flag,
+  (void)launch_chained(snn_dw_tma_kernel<QL, C256>, grid, kThreads, p.smem, s, 0, mx, my, mu, g, partial, stages_per_split, scale, exact_flag,
                                                              p.taps_per_tile, stage_wseg_log2(g));
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;

@@ -32,6 +32,8 @@ constexpr int kThreads = 256;
 __global__ void __launch_bounds__(kThreads)
 snn_act_lists_kernel(const float* __restrict__ out, const float* __restrict__ uv, int R, int J,
                      uint4* __restrict__ list, int* __restrict__ count, const DxGate gate) {
+  chain_wait();
+  chain_next();
   if (gate.nz != nullptr && __ldg(gate.nz) > gate.threshold) return;   // the dense kernel takes this call
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -56,6 +58,8 @@ snn_act_lists_kernel(const float* __restrict__ out, const float* __restrict__ uv
 // Wt[(tap*J + j)*C + c] = W[(tap*C + c)*J + j]  (the bias row is not part of dX)
 __global__ void snn_weight_transpose_kernel(const float* __restrict__ w, float* __restrict__ wt, int taps, int C, int J,
                                             const DxGate gate) {
+  chain_wait();
+  chain_next();
   if (gate.nz != nullptr && __ldg(gate.nz) > gate.threshold) return;
   const size_t n = (size_t)taps * C * J;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -89,6 +93,8 @@ __global__ void __launch_bounds__(kThreads)
 snn_dx_sparse_kernel(const Geometry g, const float* __restrict__ x, const float* __restrict__ wt,
                      const uint4* __restrict__ list, const int* __restrict__ count, float* __restrict__ dx,
                      const DxGate gate) {
+  chain_wait();
+  chain_next();
   if (gate.nz != nullptr && __ldg(gate.nz) > gate.threshold) return;
   constexpr int PPW = 32 / LPP;                       // pixels per warp
   constexpr int SB = kStage / PPW;                    // staged entries per pixel and round
@@ -216,7 +222,7 @@ int launch_one(const Geometry& g, const float* x, const float* wt, const uint4* 
   long grid = (warps + (kThreads / 32) - 1) / (kThreads / 32);
   const long cap = (long)li.num_sms * 16;
   if (grid > cap) grid = cap;
-  snn_dx_sparse_kernel<CPL, LPP><<<(int)grid, kThreads, 0, s>>>(g, x, wt, list, count, dx, gate);
+  (void)launch_chained(snn_dx_sparse_kernel<CPL, LPP>, (int)grid, kThreads, 0, s, 0, g, x, wt, list, count, dx, gate);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -248,13 +254,13 @@ int launch_dx_sparse(const Geometry& g, const float* uv, const float* x, const f
 
   long grid = ((long)g.R + (kThreads / 32) - 1) / (kThreads / 32);
   if (grid > (long)li.num_sms * 16) grid = (long)li.num_sms * 16;
-  snn_act_lists_kernel<<<(int)grid, kThreads, 0, s>>>(out, uv, g.R, g.J, list, count, gate);
+  (void)launch_chained(snn_act_lists_kernel, (int)grid, kThreads, 0, s, 0, out, uv, g.R, g.J, list, count, gate);
   count_launch();
   if (cudaGetLastError() != cudaSuccess) return E_CUDA;
   const size_t nw = (size_t)g.Kh * g.Kw * g.C * g.J;
   long tg = (long)((nw + 255) / 256);
   if (tg > (long)li.num_sms * 8) tg = (long)li.num_sms * 8;
-  snn_weight_transpose_kernel<<<(int)tg, 256, 0, s>>>(w, wt, g.Kh * g.Kw, g.C, g.J, gate);
+  (void)launch_chained(snn_weight_transpose_kernel, (int)tg, 256, 0, s, 0, w, wt, g.Kh * g.Kw, g.C, g.J, gate);
   count_launch();
   if (cudaGetLastError() != cudaSuccess) return E_CUDA;
 

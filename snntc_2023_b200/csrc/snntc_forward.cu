@@ -64,6 +64,8 @@ constexpr int kBoundClusters = 32;
 constexpr int kBoundCtas = 8 * kBoundClusters;
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256)
 snn_wbound_kernel(const float* __restrict__ w, int rows, int J, int rows_per_cta, float* __restrict__ bound) {
+  chain_wait();
+  chain_next();
   __shared__ float part[9];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r0 = blockIdx.x * rows_per_cta;
@@ -514,6 +516,8 @@ template <int JPT, bool VECW, bool STAGE>
 __global__ void __launch_bounds__(kFwdThreads, JPT <= 4 ? 4 : 1)   // up to four outputs per lane: 64 registers, 32 warps per SM
 snn_walk_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const int* __restrict__ nvalid_g, int istride,
                 const float* __restrict__ w, float* __restrict__ out, int row_begin, int row_end) {
+  chain_wait();
+  chain_next();
   __shared__ __align__(16) WalkEntry stage[STAGE ? kFwdWarps * 64 : 1];   // two blocks of 32 list entries per warp
   WalkEntry* sbuf = stage + (STAGE ? (threadIdx.x >> 5) * 64 : 0);
   const int J = g.J, R = g.R;
@@ -543,6 +547,8 @@ template <int JP, bool STAGE>
 __global__ void __launch_bounds__(kFwdThreads)
 snn_walk2_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const int* __restrict__ nvalid_g, int istride,
                  const float* __restrict__ w, float* __restrict__ out, int row_begin, int row_end) {
+  chain_wait();
+  chain_next();
   __shared__ __align__(16) WalkEntry stage[STAGE ? kFwdWarps * 64 : 1];   // two blocks of 32 list entries per warp
   WalkEntry* sbuf = stage + (STAGE ? (threadIdx.x >> 5) * 64 : 0);
   const int J = g.J, R = g.R;
@@ -584,6 +590,8 @@ __global__ void __launch_bounds__(kSmemwThreads, 1)
 snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const int* __restrict__ nvalid_g,
                        int istride, const float* __restrict__ w, float* __restrict__ out, int row_begin, int row_end,
                        unsigned wmul) {
+  chain_wait();
+  chain_next();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long copy_done;
   const int J = g.J, R = g.R;
@@ -666,8 +674,8 @@ int launch_walk(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g,
   long grid = (items + kFwdWarps - 1) / kFwdWarps;
   const long cap = (long)li.num_sms * 8;
   if (grid > cap) grid = cap;
-  if (stage) snn_walk_kernel<JPT, VECW, true><<<(int)grid, kFwdThreads, 0, s>>>(g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
-  else snn_walk_kernel<JPT, VECW, false><<<(int)grid, kFwdThreads, 0, s>>>(g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
+  if (stage) (void)launch_chained(snn_walk_kernel<JPT, VECW, true>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
+  else (void)launch_chained(snn_walk_kernel<JPT, VECW, false>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -680,8 +688,8 @@ int launch_walk2(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g
   long grid = (items + kFwdWarps - 1) / kFwdWarps;
   const long cap = (long)li.num_sms * 8;
   if (grid > cap) grid = cap;
-  if (stage) snn_walk2_kernel<JP, true><<<(int)grid, kFwdThreads, 0, s>>>(g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
-  else snn_walk2_kernel<JP, false><<<(int)grid, kFwdThreads, 0, s>>>(g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
+  if (stage) (void)launch_chained(snn_walk2_kernel<JP, true>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
+  else (void)launch_chained(snn_walk2_kernel<JP, false>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -710,13 +718,13 @@ int launch_walk2_smemw(const Geometry& g, const WalkEntry* keys_g, const int* nv
   if (per_slice < 1) per_slice = 1;
   const int grid = (int)(per_slice * slices);
   if (stage) {
-    if (cudaFuncSetAttribute(snn_walk2_smemw_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (allow_smem<snn_walk2_smemw_kernel<true>>(smem) != cudaSuccess)
       return E_CUDA;
-    snn_walk2_smemw_kernel<true><<<grid, kSmemwThreads, smem, s>>>(g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end, (unsigned)wmul);
+    (void)launch_chained(snn_walk2_smemw_kernel<true>, grid, kSmemwThreads, smem, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end, (unsigned)wmul);
   } else {
-    if (cudaFuncSetAttribute(snn_walk2_smemw_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (allow_smem<snn_walk2_smemw_kernel<false>>(smem) != cudaSuccess)
       return E_CUDA;
-    snn_walk2_smemw_kernel<false><<<grid, kSmemwThreads, smem, s>>>(g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end, (unsigned)wmul);
+    (void)launch_chained(snn_walk2_smemw_kernel<false>, grid, kSmemwThreads, smem, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end, (unsigned)wmul);
   }
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
@@ -778,7 +786,7 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     int per = (rows_w + kBoundCtas - 1) / kBoundCtas;
     per = (per + 7) & ~7;                                // whole rounds of the CTA's eight warps
     g.wbound_n = (rows_w + 8 * per - 1) / (8 * per);     // clusters
-    snn_wbound_kernel<<<8 * g.wbound_n, 256, 0, s>>>(w, rows_w, g.J, per, wbound);
+    (void)launch_chained(snn_wbound_kernel, 8 * g.wbound_n, 256, 0, s, 0, w, rows_w, g.J, per, wbound);
     count_launch();
     if (cudaGetLastError() != cudaSuccess) return E_CUDA;
   }

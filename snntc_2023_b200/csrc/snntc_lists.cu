@@ -156,6 +156,8 @@ template <int EPL>
 __global__ void __launch_bounds__(kPixelWarps * 32)
 snn_pixel_runs_kernel(const float* __restrict__ x, int npix, int C, int J, float maxcomp,
                       WalkEntry* __restrict__ runs, int* __restrict__ counts, int stride) {
+  chain_wait();
+  chain_next();
   __shared__ u64 compact[kPixelWarps][EPL >= 2 ? 16 * EPL : 1];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -189,6 +191,8 @@ template <int EPL>
 __global__ void __launch_bounds__(kPixelWarps * 32)
 snn_small_rows_kernel(const Geometry g, const float* __restrict__ x, WalkEntry* __restrict__ lists,
                       int* __restrict__ nvalid, int istride) {
+  chain_wait();
+  chain_next();
   __shared__ int tap_off[32 * EPL];
   __shared__ unsigned short tap_khw[32 * EPL];
   const int I = g.I;
@@ -303,6 +307,8 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(kListThreads)
 snn_row_runs_kernel(const Geometry g, const WalkEntry* __restrict__ pix, const int* __restrict__ pix_n, int pix_stride,
                     WalkEntry* __restrict__ rows, int* __restrict__ rows_n, int row_stride, int parts_log2) {
+  chain_wait();
+  chain_next();
   __shared__ uint2 windows[3 * 4 * kListThreads];
   BlockedMem mem = {windows + threadIdx.x};
   const int items = g.B * g.H * g.Nw;
@@ -348,6 +354,8 @@ __global__ void __launch_bounds__(kListThreads)
 snn_field_lists_kernel(const Geometry g, const WalkEntry* __restrict__ rows, const int* __restrict__ rows_n,
                        int row_stride, WalkEntry* __restrict__ lists, int* __restrict__ nvalid, int istride,
                        int parts_log2) {
+  chain_wait();
+  chain_next();
   __shared__ uint2 windows[3 * 4 * kListThreads];
   BlockedMem mem = {windows + threadIdx.x};
   const int thread = blockIdx.x * blockDim.x + threadIdx.x;
@@ -444,11 +452,11 @@ int launch_merge_lists(const Geometry& g, const float* x, WalkEntry* lists, int*
   const long cap = (long)li.num_sms * 8;
   if (grid > cap) grid = cap;
   const int epl = (g.C + 31) / 32;
-  if (epl <= 1) snn_pixel_runs_kernel<1><<<(int)grid, kPixelWarps * 32, 0, s>>>(x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
-  else if (epl <= 2) snn_pixel_runs_kernel<2><<<(int)grid, kPixelWarps * 32, 0, s>>>(x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
-  else if (epl <= 4) snn_pixel_runs_kernel<4><<<(int)grid, kPixelWarps * 32, 0, s>>>(x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
-  else if (epl <= 8) snn_pixel_runs_kernel<8><<<(int)grid, kPixelWarps * 32, 0, s>>>(x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
-  else snn_pixel_runs_kernel<16><<<(int)grid, kPixelWarps * 32, 0, s>>>(x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
+  if (epl <= 1) (void)launch_chained(snn_pixel_runs_kernel<1>, (int)grid, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
+  else if (epl <= 2) (void)launch_chained(snn_pixel_runs_kernel<2>, (int)grid, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
+  else if (epl <= 4) (void)launch_chained(snn_pixel_runs_kernel<4>, (int)grid, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
+  else if (epl <= 8) (void)launch_chained(snn_pixel_runs_kernel<8>, (int)grid, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
+  else (void)launch_chained(snn_pixel_runs_kernel<16>, (int)grid, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
   count_launch();
   if (cudaGetLastError() != cudaSuccess) return E_CUDA;
 
@@ -456,18 +464,18 @@ int launch_merge_lists(const Geometry& g, const float* x, WalkEntry* lists, int*
   int lg = split_log2 >= 0 ? (split_log2 > 5 ? 5 : split_log2) : merge_split_log2(nrow, li);
   if (((long)nrow << lg) > 0x7fffffffL - kListThreads) lg = 0;
   if (lg == 0)
-    snn_row_runs_kernel<false><<<(nrow + kListThreads - 1) / kListThreads, kListThreads, 0, s>>>(g, pix, pix_n, ps, rows, rows_n, rs, 0);
+    (void)launch_chained(snn_row_runs_kernel<false>, (nrow + kListThreads - 1) / kListThreads, kListThreads, 0, s, 0, g, pix, pix_n, ps, rows, rows_n, rs, 0);
   else
-    snn_row_runs_kernel<true><<<(int)((((long)nrow << lg) + kListThreads - 1) / kListThreads), kListThreads, 0, s>>>(g, pix, pix_n, ps, rows, rows_n, rs, lg);
+    (void)launch_chained(snn_row_runs_kernel<true>, (int)((((long)nrow << lg) + kListThreads - 1) / kListThreads), kListThreads, 0, s, 0, g, pix, pix_n, ps, rows, rows_n, rs, lg);
   count_launch();
   if (cudaGetLastError() != cudaSuccess) return E_CUDA;
 
   lg = split_log2 >= 0 ? (split_log2 > 5 ? 5 : split_log2) : merge_split_log2(g.R, li);
   if (((long)g.R << lg) > 0x7fffffffL - kListThreads) lg = 0;
   if (lg == 0)
-    snn_field_lists_kernel<false><<<(g.R + kListThreads - 1) / kListThreads, kListThreads, 0, s>>>(g, rows, rows_n, rs, lists, nvalid, istride, 0);
+    (void)launch_chained(snn_field_lists_kernel<false>, (g.R + kListThreads - 1) / kListThreads, kListThreads, 0, s, 0, g, rows, rows_n, rs, lists, nvalid, istride, 0);
   else
-    snn_field_lists_kernel<true><<<(int)((((long)g.R << lg) + kListThreads - 1) / kListThreads), kListThreads, 0, s>>>(g, rows, rows_n, rs, lists, nvalid, istride, lg);
+    (void)launch_chained(snn_field_lists_kernel<true>, (int)((((long)g.R << lg) + kListThreads - 1) / kListThreads), kListThreads, 0, s, 0, g, rows, rows_n, rs, lists, nvalid, istride, lg);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -485,14 +493,14 @@ int launch_small_rows(const Geometry& g, const float* x, WalkEntry* lists, int* 
   if (grid > cap) grid = cap;
   const int epl = (g.I + 31) / 32;
   switch (epl) {   // 3, 5, 6, 7 keys per lane: the block network (a bitonic one would round them up to 4 and 8)
-    case 1: snn_small_rows_kernel<1><<<(int)grid, kPixelWarps * 32, 0, s>>>(g, x, lists, nvalid, istride); break;
-    case 2: snn_small_rows_kernel<2><<<(int)grid, kPixelWarps * 32, 0, s>>>(g, x, lists, nvalid, istride); break;
-    case 3: snn_small_rows_kernel<3><<<(int)grid, kPixelWarps * 32, 0, s>>>(g, x, lists, nvalid, istride); break;
-    case 4: snn_small_rows_kernel<4><<<(int)grid, kPixelWarps * 32, 0, s>>>(g, x, lists, nvalid, istride); break;
-    case 5: snn_small_rows_kernel<5><<<(int)grid, kPixelWarps * 32, 0, s>>>(g, x, lists, nvalid, istride); break;
-    case 6: snn_small_rows_kernel<6><<<(int)grid, kPixelWarps * 32, 0, s>>>(g, x, lists, nvalid, istride); break;
-    case 7: snn_small_rows_kernel<7><<<(int)grid, kPixelWarps * 32, 0, s>>>(g, x, lists, nvalid, istride); break;
-    default: snn_small_rows_kernel<8><<<(int)grid, kPixelWarps * 32, 0, s>>>(g, x, lists, nvalid, istride); break;
+    case 1: (void)launch_chained(snn_small_rows_kernel<1>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
+    case 2: (void)launch_chained(snn_small_rows_kernel<2>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
+    case 3: (void)launch_chained(snn_small_rows_kernel<3>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
+    case 4: (void)launch_chained(snn_small_rows_kernel<4>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
+    case 5: (void)launch_chained(snn_small_rows_kernel<5>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
+    case 6: (void)launch_chained(snn_small_rows_kernel<6>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
+    case 7: (void)launch_chained(snn_small_rows_kernel<7>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
+    default: (void)launch_chained(snn_small_rows_kernel<8>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
   }
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;

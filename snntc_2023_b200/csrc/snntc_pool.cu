@@ -2,6 +2,7 @@
 // The reference does this with TensorFlow glue, -MaxPool2D(-x) after tf.pad with 1e5
 // (SNN_TC_Modules.py:216-246); here it is one kernel that also records the winner for the backward.
 #include "../../include/snntc_b200.h"
+#include "snntc_launch.cuh"
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -10,12 +11,18 @@ namespace snntc { void count_launch(int n = 1); }
 
 namespace {
 
+using snntc::chain_next;
+using snntc::chain_wait;
+using snntc::launch_chained;
+
 // One thread per V consecutive channels of one output (V = 4 when C % 4 == 0: 16-byte accesses; else 1).
 // All indices fit 32 bits (checked by the callers).
 template <int V>
 __global__ void minpool_fwd_kernel(const float* __restrict__ x, float* __restrict__ y, int* __restrict__ arg,
                                    int B, int H, int W, int C, int Kh, int Kw, int Sh, int Sw, int pt, int pl,
                                    int Nh, int Nw, float padvalue) {
+  chain_wait();
+  chain_next();
   const unsigned CV = (unsigned)C / V;
   const unsigned n = (unsigned)B * Nh * Nw * CV;
   const unsigned stride = gridDim.x * blockDim.x;
@@ -70,6 +77,8 @@ template <int V>
 __global__ void minpool_bwd_kernel(const float* __restrict__ gy, const int* __restrict__ arg, float* __restrict__ dx,
                                    int B, int H, int W, int C, int Kh, int Kw, int Sh, int Sw, int pt, int pl,
                                    int Nh, int Nw) {
+  chain_wait();
+  chain_next();
   const unsigned CV = (unsigned)C / V;
   const unsigned n = (unsigned)B * H * W * CV;
   const unsigned stride = gridDim.x * blockDim.x;
@@ -130,10 +139,10 @@ int snntc_minpool_forward(const float* x, float* y, int* arg, int B, int H, int 
   const size_t n = (size_t)B * Nh * Nw * C;
   const bool v4 = (C % 4) == 0 && (((uintptr_t)x | (uintptr_t)y | (uintptr_t)arg) & 15) == 0;
   if (v4)
-    minpool_fwd_kernel<4><<<grid_for(n / 4), 256, 0, (cudaStream_t)stream>>>(x, y, arg, B, H, W, C, Kh, Kw, Sh, Sw, pad_top,
+    (void)launch_chained(minpool_fwd_kernel<4>, grid_for(n / 4), 256, 0, (cudaStream_t)stream, 0, x, y, arg, B, H, W, C, Kh, Kw, Sh, Sw, pad_top,
                                                                            pad_left, Nh, Nw, padvalue);
   else
-    minpool_fwd_kernel<1><<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(x, y, arg, B, H, W, C, Kh, Kw, Sh, Sw, pad_top,
+    (void)launch_chained(minpool_fwd_kernel<1>, grid_for(n), 256, 0, (cudaStream_t)stream, 0, x, y, arg, B, H, W, C, Kh, Kw, Sh, Sw, pad_top,
                                                                      pad_left, Nh, Nw, padvalue);
   snntc::count_launch();
   return cudaGetLastError() == cudaSuccess ? SNNTC_OK : SNNTC_E_CUDA;
@@ -149,10 +158,10 @@ int snntc_minpool_backward(const float* gy, const int* arg, float* dx, int B, in
   const size_t n = (size_t)B * H * W * C;
   const bool v4 = (C % 4) == 0 && (((uintptr_t)gy | (uintptr_t)arg | (uintptr_t)dx) & 15) == 0;
   if (v4)
-    minpool_bwd_kernel<4><<<grid_for(n / 4), 256, 0, (cudaStream_t)stream>>>(gy, arg, dx, B, H, W, C, Kh, Kw, Sh, Sw, pad_top,
+    (void)launch_chained(minpool_bwd_kernel<4>, grid_for(n / 4), 256, 0, (cudaStream_t)stream, 0, gy, arg, dx, B, H, W, C, Kh, Kw, Sh, Sw, pad_top,
                                                                            pad_left, Nh, Nw);
   else
-    minpool_bwd_kernel<1><<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(gy, arg, dx, B, H, W, C, Kh, Kw, Sh, Sw, pad_top,
+    (void)launch_chained(minpool_bwd_kernel<1>, grid_for(n), 256, 0, (cudaStream_t)stream, 0, gy, arg, dx, B, H, W, C, Kh, Kw, Sh, Sw, pad_top,
                                                                          pad_left, Nh, Nw);
   snntc::count_launch();
   return cudaGetLastError() == cudaSuccess ? SNNTC_OK : SNNTC_E_CUDA;

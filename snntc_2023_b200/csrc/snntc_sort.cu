@@ -105,6 +105,8 @@ template <int TPR, int EPT>
 __global__ void __launch_bounds__(TPR == 32 ? 256 : TPR)
 snn_bucket_sort_kernel(const Geometry g, const float* __restrict__ x, WalkEntry* __restrict__ lists, int* __restrict__ nvalid,
                        int istride, int nb_log2, int table) {
+  chain_wait();
+  chain_next();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned tmp[33];
   constexpr int kMostBig = TPR == 32 ? 8 : 256;      // at most I / 129 buckets hold more than 128 keys
@@ -298,14 +300,14 @@ int launch(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int
   }
   const size_t smem = table + rows_per_cta * row;
   if (smem > budget) return E_UNSUPPORTED;
-  if (cudaFuncSetAttribute(snn_bucket_sort_kernel<TPR, EPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return E_CUDA;
+  if (allow_smem<snn_bucket_sort_kernel<TPR, EPT>>(smem) != cudaSuccess) return E_CUDA;
   const int threads = TPR == 32 ? 32 * rows_per_cta : TPR;
   long resident = (long)(budget / (smem + 10 * 1024));
   if (resident > 2048 / threads) resident = 2048 / threads;
   if (resident < 1) resident = 1;
   long grid = ((long)g.R + rows_per_cta - 1) / rows_per_cta;
   if (grid > resident * li.num_sms) grid = resident * li.num_sms;
-  snn_bucket_sort_kernel<TPR, EPT><<<(int)grid, threads, smem, s>>>(g, x, lists, nvalid, istride, nb_log2, table > 0);
+  (void)launch_chained(snn_bucket_sort_kernel<TPR, EPT>, (int)grid, threads, smem, s, 0, g, x, lists, nvalid, istride, nb_log2, table > 0);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }

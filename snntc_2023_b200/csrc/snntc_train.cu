@@ -8,6 +8,7 @@
 //                         gradient bucket in place                                  (snntc-mnist.py:70, snntc-imagenet.py:238)
 // The reference runs these as TensorFlow graph ops; nothing here has native code in the reference.
 #include "../../include/snntc_b200.h"
+#include "snntc_launch.cuh"
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -18,6 +19,10 @@ namespace snntc { void count_launch(int n = 1); }
 
 namespace {
 
+using snntc::chain_next;
+using snntc::chain_wait;
+using snntc::launch_chained;
+
 int grid_for(size_t n, int per_block = 256) {
   size_t b = (n + per_block - 1) / per_block;
   if (b > 148 * 16) b = 148 * 16;
@@ -26,6 +31,8 @@ int grid_for(size_t n, int per_block = 256) {
 }
 
 __global__ void encode_kernel(const float* __restrict__ p, float* __restrict__ x, size_t n, float scale, int one_minus) {
+  chain_wait();
+  chain_next();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
     const float v = __ldg(p + e);
@@ -137,6 +144,8 @@ __global__ void wcost_apply_kernel(const float* __restrict__ w, const float* __r
 __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
                             size_t n, float lr, float b1, float b2, float eps, float gscale,
                             const int* __restrict__ step) {
+  chain_wait();
+  chain_next();
   const int t = __ldg(step) + 1;
   const float c1 = 1.0f - powf(b1, (float)t), c2 = 1.0f - powf(b2, (float)t);
   const float lrt = lr * sqrtf(c2) / c1;
@@ -150,7 +159,7 @@ __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, 
     w[e] -= lrt * me / (sqrtf(ve) + eps);
   }
 }
-__global__ void step_inc_kernel(int* step) { *step += 1; }
+__global__ void step_inc_kernel(int* step) { chain_wait(); chain_next(); *step += 1; }
 
 // Keras SGD with momentum: vel = momentum * vel - lr * g; w += vel
 __global__ void sgdm_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ vel, size_t n,
@@ -232,6 +241,8 @@ template <int G>
 __global__ void __cluster_dims__(kLossCluster, 1, 1) __launch_bounds__(kLossThreads)
 loss_fwd_kernel(const float* __restrict__ y, const long long* __restrict__ labels, float* __restrict__ loss,
                 float* __restrict__ hits, int B, int J, float lscale) {
+  chain_wait();
+  chain_next();
   const int gl = threadIdx.x % G;
   const int groups = kLossCluster * kLossThreads / G;
   float loss_acc = 0.f, hit_acc = 0.f;
@@ -258,6 +269,8 @@ template <int G>
 __global__ void __launch_bounds__(256)
 loss_bwd_kernel(const float* __restrict__ y, const long long* __restrict__ labels, const float* __restrict__ gloss,
                 float* __restrict__ grad, int B, int J, float gscale) {
+  chain_wait();
+  chain_next();
   const int gl = threadIdx.x % G;
   const int b = (blockIdx.x * 256 + threadIdx.x) / G;
   const bool ok = b < B;
@@ -301,6 +314,8 @@ __device__ __forceinline__ int tensor_of(const int* first, int count, int at) {
 // row of the slice, eight loads in flight; the threads of a column are added through shared memory.
 __global__ void __launch_bounds__(kCostThreads)
 cost_sums_kernel(const __grid_constant__ CostTensors c, float* __restrict__ partial, float* __restrict__ sq) {
+  chain_wait();
+  chain_next();
   __shared__ float part[kCostThreads];
   const int t = tensor_of(c.first_cta, c.count, blockIdx.x);
   const int local = blockIdx.x - c.first_cta[t];
@@ -349,6 +364,8 @@ cost_sums_kernel(const __grid_constant__ CostTensors c, float* __restrict__ part
 __global__ void __cluster_dims__(kLossCluster, 1, 1) __launch_bounds__(kLossThreads)
 cost_total_kernel(const __grid_constant__ CostTensors c, const float* __restrict__ partial, const float* __restrict__ sq,
                   float* __restrict__ colsum, float* __restrict__ cost, float K, float K2, int add) {
+  chain_wait();
+  chain_next();
   const int me = blockIdx.x * kLossThreads + threadIdx.x;
   constexpr int kAll = kLossCluster * kLossThreads;
   float total = 0.f;
@@ -375,6 +392,8 @@ template <bool ADD>
 __global__ void __launch_bounds__(kCostThreads)
 cost_grad_kernel(const __grid_constant__ CostTensors c, const float* __restrict__ colsum, const float* __restrict__ gcost,
                  float K, float K2) {
+  chain_wait();
+  chain_next();
   const int t = tensor_of(c.first_chunk, c.count, blockIdx.x);
   const int J = c.cols[t];
   const unsigned n = (unsigned)c.rows[t] * (unsigned)J;
@@ -458,7 +477,7 @@ extern "C" {
 int snntc_encode(const float* p, float* x, size_t n, float scale, int one_minus, void* stream) {
   if (!p || !x) return SNNTC_E_NULL;
   if (n == 0) return SNNTC_OK;
-  encode_kernel<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(p, x, n, scale, one_minus);
+  (void)launch_chained(encode_kernel, grid_for(n), 256, 0, (cudaStream_t)stream, 0, p, x, n, scale, one_minus);
   return done();
 }
 
@@ -475,8 +494,8 @@ int snntc_loss_forward(const float* y, const long long* labels, float* loss, flo
                        void* stream) {
   if (!y || !labels || !loss || !hits) return SNNTC_E_NULL;
   if (B <= 0 || J <= 0) return SNNTC_E_SHAPE;
-  if (J <= 16) loss_fwd_kernel<16><<<kLossCluster, kLossThreads, 0, (cudaStream_t)stream>>>(y, labels, loss, hits, B, J, loss_scale);
-  else loss_fwd_kernel<32><<<kLossCluster, kLossThreads, 0, (cudaStream_t)stream>>>(y, labels, loss, hits, B, J, loss_scale);
+  if (J <= 16) (void)launch_chained(loss_fwd_kernel<16>, kLossCluster, kLossThreads, 0, (cudaStream_t)stream, 0, y, labels, loss, hits, B, J, loss_scale);
+  else (void)launch_chained(loss_fwd_kernel<32>, kLossCluster, kLossThreads, 0, (cudaStream_t)stream, 0, y, labels, loss, hits, B, J, loss_scale);
   return done();
 }
 
@@ -486,8 +505,8 @@ int snntc_loss_backward(const float* y, const long long* labels, const float* gl
   if (B <= 0 || J <= 0) return SNNTC_E_SHAPE;
   const int G = J <= 16 ? 16 : 32;
   const int grid = (int)(((long long)B * G + 255) / 256);
-  if (G == 16) loss_bwd_kernel<16><<<grid, 256, 0, (cudaStream_t)stream>>>(y, labels, gloss, grad, B, J, grad_scale);
-  else loss_bwd_kernel<32><<<grid, 256, 0, (cudaStream_t)stream>>>(y, labels, gloss, grad, B, J, grad_scale);
+  if (G == 16) (void)launch_chained(loss_bwd_kernel<16>, grid, 256, 0, (cudaStream_t)stream, 0, y, labels, gloss, grad, B, J, grad_scale);
+  else (void)launch_chained(loss_bwd_kernel<32>, grid, 256, 0, (cudaStream_t)stream, 0, y, labels, gloss, grad, B, J, grad_scale);
   return done();
 }
 
@@ -517,9 +536,9 @@ int snntc_weight_costs(int count, const float* const* w, const int* rows, const 
     const CostTensors c = cost_tensors(count, w, nullptr, rows, cols, at);
     float* partial = static_cast<float*>(workspace);
     float* sq = partial + cost_partial_floats(c);
-    cost_sums_kernel<<<c.first_cta[c.count], kCostThreads, 0, s>>>(c, partial, sq);
+    (void)launch_chained(cost_sums_kernel, c.first_cta[c.count], kCostThreads, 0, s, 0, c, partial, sq);
     if (done() != SNNTC_OK) return SNNTC_E_CUDA;
-    cost_total_kernel<<<kLossCluster, kLossThreads, 0, s>>>(c, partial, sq, colsum, cost, K, K2, at > 0);
+    (void)launch_chained(cost_total_kernel, kLossCluster, kLossThreads, 0, s, 0, c, partial, sq, colsum, cost, K, K2, at > 0);
     if (done() != SNNTC_OK) return SNNTC_E_CUDA;
     colsum += c.first_col[c.count];
   }
@@ -537,8 +556,8 @@ int snntc_weight_cost_grads(int count, const float* const* w, float* const* gw, 
   }
   for (int at = 0; at < count; at += kCostMax) {
     const CostTensors c = cost_tensors(count, w, gw, rows, cols, at);
-    if (add) cost_grad_kernel<true><<<c.first_chunk[c.count], kCostThreads, 0, (cudaStream_t)stream>>>(c, colsum, gcost, K, K2);
-    else cost_grad_kernel<false><<<c.first_chunk[c.count], kCostThreads, 0, (cudaStream_t)stream>>>(c, colsum, gcost, K, K2);
+    if (add) (void)launch_chained(cost_grad_kernel<true>, c.first_chunk[c.count], kCostThreads, 0, (cudaStream_t)stream, 0, c, colsum, gcost, K, K2);
+    else (void)launch_chained(cost_grad_kernel<false>, c.first_chunk[c.count], kCostThreads, 0, (cudaStream_t)stream, 0, c, colsum, gcost, K, K2);
     if (done() != SNNTC_OK) return SNNTC_E_CUDA;
     colsum += c.first_col[c.count];
   }
@@ -568,9 +587,9 @@ int snntc_adam_step(float* w, const float* g, float* m, float* v, size_t n, floa
                     float eps, float grad_scale, int* step, void* stream) {
   if (!w || !g || !m || !v || !step) return SNNTC_E_NULL;
   if (n == 0) return SNNTC_OK;
-  adam_kernel<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(w, g, m, v, n, lr, beta1, beta2, eps, grad_scale, step);
+  (void)launch_chained(adam_kernel, grid_for(n), 256, 0, (cudaStream_t)stream, 0, w, g, m, v, n, lr, beta1, beta2, eps, grad_scale, step);
   if (done() != SNNTC_OK) return SNNTC_E_CUDA;
-  step_inc_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(step);
+  (void)launch_chained(step_inc_kernel, 1, 1, 0, (cudaStream_t)stream, 0, step);
   return done();
 }
 

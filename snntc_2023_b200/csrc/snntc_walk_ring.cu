@@ -93,6 +93,8 @@ template <bool VEC, int kBlock>
 __global__ void __launch_bounds__(32 * kWarps)
 snn_walk_ring_kernel(const Geometry g, const WalkEntry* __restrict__ lists, const int* __restrict__ nvalid, int istride,
                      const float* __restrict__ w, float* __restrict__ out, int slices) {
+  chain_wait();
+  chain_next();
   __shared__ __align__(16) RingWarp<kBlock> ring[kWarps];
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   RingWarp<kBlock>& sm = ring[warp];
@@ -233,7 +235,7 @@ int launch_walk_ring(const Geometry& g, const WalkEntry* lists, const int* nvali
   if (grid > 0x7fffffffL) return E_UNSUPPORTED;
   const bool vec = (g.J & 3) == 0 && ((uintptr_t)w & 15) == 0;
   const bool small = grid * kWarps > 8L * li.num_sms;
-  auto go = [&](auto kernel) { kernel<<<(unsigned)grid, 32 * kWarps, 0, s>>>(g, lists, nvalid, istride, w, out, slices); };
+  auto go = [&](auto kernel) { (void)launch_chained(kernel, (unsigned)grid, 32 * kWarps, 0, s, 0, g, lists, nvalid, istride, w, out, slices); };
   if (vec) small ? go(snn_walk_ring_kernel<true, 16>) : go(snn_walk_ring_kernel<true, 32>);
   else small ? go(snn_walk_ring_kernel<false, 16>) : go(snn_walk_ring_kernel<false, 32>);
   count_launch();
