@@ -308,24 +308,24 @@ std::pair<Tensor, Tensor> minpool_call(const Tensor& X, const PoolGeom& q, float
 struct PoolState : torch::CustomClassHolder {
   PoolGeom q;
   std::vector<int64_t> shape;
-  Tensor arg;
 };
 
 struct PoolFunction : torch::autograd::Function<PoolFunction> {
   static Tensor forward(AutogradContext* ctx, const Tensor& X, c10::intrusive_ptr<PoolState> s, double padvalue) {
     auto r = minpool_call(X, s->q, (float)padvalue, true);
     s->shape = X.sizes().vec();
-    s->arg = r.second;
+    ctx->save_for_backward({r.second});
     ctx->saved_data["call"] = c10::IValue::make_capsule(s);
     return r.first;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = c10::static_intrusive_pointer_cast<PoolState>(ctx->saved_data["call"].toCapsule());
+    const Tensor arg = ctx->get_saved_variables()[0];
     const Tensor gy = as_cuda_f32(grads[0], "grad");
     const c10::cuda::CUDAGuard guard(gy.device());
     const Tensor dx = empty_like_dev(s->shape, gy);
     const PoolGeom& q = s->q;
-    check(snntc_minpool_backward(ptr(gy), s->arg.data_ptr<int>(), ptr(dx), (int)s->shape[0], (int)s->shape[1], (int)s->shape[2],
+    check(snntc_minpool_backward(ptr(gy), arg.data_ptr<int>(), ptr(dx), (int)s->shape[0], (int)s->shape[1], (int)s->shape[2],
                                  (int)s->shape[3], q.Kh, q.Kw, q.Sh, q.Sw, q.pt, q.pl, q.Nh, q.Nw, stream_of(gy)),
           "minpool backward");
     return {dx, Tensor(), Tensor()};
