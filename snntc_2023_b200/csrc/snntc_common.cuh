@@ -48,7 +48,7 @@ struct Options {
                             // 16: one output per lane, the warp's weight rows copied ahead into shared memory
   int walk_outputs = 0;     // 0 auto, 1..4: 1, 2, 4, 8 outputs per lane (pairs layout: 2 only)
   int list_builder = 0;     // 0 auto, 1 per-row bucket sort, 2 per-pixel sort + merges (3x3 stride-1 conv only),
-                            // 3 per-row sorting network in registers (rows of at most 256 inputs);
+                            // 3 per-row sorting network in registers (rows of at most 64 inputs);
                             // + 4*(k+1): the merges are cut into 2^k pieces each (k = 0 .. 5) instead of auto
   int backward_parts = 3;   // bit 0: dX, bit 1: dW
   int dw_kernel = 0;        // 0 auto, 1 dense register tile, 2 row-skipping kernel (conv, C % 4 == 0) with per-thread
@@ -112,7 +112,7 @@ int launch_walk_ring(const Geometry& g, const WalkEntry* lists, const int* nvali
 int launch_row_sort(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride, const LaunchInfo& li,
                     cudaStream_t s);
 
-// Sorted lists of rows of at most 256 inputs by a sorting network in registers, one warp per row (snntc_lists.cu).
+// Sorted lists of rows of at most 64 inputs by a sorting network in registers, one warp per row (snntc_lists.cu).
 bool small_rows_supported(const Geometry& g);
 int launch_small_rows(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride,
                       const LaunchInfo& li, cudaStream_t s);

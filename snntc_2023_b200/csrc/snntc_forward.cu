@@ -4,7 +4,7 @@
 // outside it). A scratch buffer of sorted lists in global memory -- per row the inputs at or below MAX-0.1 as
 // (value, element offset of the weight row), ascending -- joins two stages:
 //   1. the lists. Stride-1 convolutions up to 3x3 on 16 to 512 channels: per-pixel sort and two levels of
-//      merging (snntc_lists.cu). Rows of at most 256 inputs: a sorting network in registers, one warp per row
+//      merging (snntc_lists.cu). Rows of at most 64 inputs: a sorting network in registers, one warp per row
 //      (snntc_lists.cu). Everything else: a bucket sort per row (snntc_sort.cu);
 //   2. the walk (walk kernels): every warp takes (row, block of outputs) items and walks the row's list, which it
 //      stages through shared memory 32 entries at a time. The running sum(w)-theta and sum(w*x) stay in

@@ -68,52 +68,6 @@ __device__ __forceinline__ void warp_bitonic_sort(u64 (&v)[EPL], int lane) {
   }
 }
 
-// Sort of 32*EPL keys for an EPL that is no power of two (the bitonic network above would round it up: 160 keys
-// would be sorted as 256). Every lane sorts its own EPL keys; the lanes then run the bitonic network over their
-// BLOCKS, a compare-exchange being a merge-split: against the partner's block in reverse, min(mine[i], theirs[EPL-1-i])
-// over i are the EPL smallest keys of both blocks, the maxima the EPL largest; what a lane keeps is sorted again
-// (odd-even transposition: EPL (EPL - 1) / 2 exchanges). Same result layout: element lane*EPL + m has rank lane*EPL + m.
-template <int EPL>
-__device__ __forceinline__ void lane_sort(u64 (&v)[EPL]) {
-#pragma unroll
-  for (int round = 0; round < EPL; ++round) {
-#pragma unroll
-    for (int i = round & 1; i + 1 < EPL; i += 2) {
-      const u64 a = v[i], b = v[i + 1];
-      const bool sw = a > b;
-      v[i] = sw ? b : a;
-      v[i + 1] = sw ? a : b;
-    }
-  }
-}
-template <int EPL>
-__device__ __forceinline__ void warp_block_sort(u64 (&v)[EPL], int lane) {
-  lane_sort<EPL>(v);
-#pragma unroll
-  for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j >= 1; j >>= 1) {
-      const bool lower = (lane & j) == 0;
-      const bool asc = (lane & k) == 0 || k == 32;
-      const bool keep_low = asc == lower;
-      u64 o[EPL];
-#pragma unroll
-      for (int i = 0; i < EPL; ++i) o[i] = __shfl_xor_sync(0xffffffffu, v[EPL - 1 - i], j);
-#pragma unroll
-      for (int i = 0; i < EPL; ++i) {
-        const bool o_less = o[i] < v[i];
-        v[i] = (keep_low == o_less) ? o[i] : v[i];
-      }
-      lane_sort<EPL>(v);
-    }
-  }
-}
-template <int EPL>
-__device__ __forceinline__ void warp_sort(u64 (&v)[EPL], int lane) {
-  if constexpr ((EPL & (EPL - 1)) == 0) warp_bitonic_sort<EPL>(v, lane);
-  else warp_block_sort<EPL>(v, lane);
-}
-
 // Sorts the n <= 32*EPL real keys of v (the other slots hold ~0) and writes them as a run. A pixel that has at most
 // half its slots filled -- most pixels of a hidden layer: about half of a layer's inputs never spike -- is first
 // compacted through `buf` (16*EPL keys of shared memory per warp) into half the slots, again and again if it can
@@ -141,7 +95,7 @@ __device__ __forceinline__ void sort_and_write_run(u64 (&v)[EPL], int n, int lan
       return;
     }
   }
-  warp_sort<EPL>(v, lane);
+  warp_bitonic_sort<EPL>(v, lane);
 #pragma unroll
   for (int m = 0; m < EPL; ++m) {
     const int rank = lane * EPL + m;
@@ -183,7 +137,7 @@ snn_pixel_runs_kernel(const float* __restrict__ x, int npix, int C, int J, float
   }
 }
 
-// Rows of at most 256 inputs (the first layer of a network: a few channels under a small kernel), one warp per
+// Rows of at most 64 inputs (the first layer of a network: a few channels under a small kernel), one warp per
 // row: the inputs that can spike, gathered tap by tap through a table in shared memory, sorted by the same
 // register network on (value, source index) -- ties in index order, like a stable sort -- and written straight
 // as the list the walk reads. A dense row is its own table.
@@ -245,7 +199,7 @@ snn_small_rows_kernel(const Geometry g, const float* __restrict__ x, WalkEntry* 
       v[m] = keep ? (((u64)float_to_sortable(val) << 32) | (unsigned)i) : ~0ull;
       n += __popc(__ballot_sync(0xffffffffu, keep));
     }
-    warp_sort<EPL>(v, lane);
+    warp_bitonic_sort<EPL>(v, lane);
     WalkEntry* dst = lists + (size_t)r * istride;
 #pragma unroll
     for (int m = 0; m < EPL; ++m) {
@@ -481,7 +435,9 @@ int launch_merge_lists(const Geometry& g, const float* x, WalkEntry* lists, int*
 }
 
 bool small_rows_supported(const Geometry& g) {
-  if (g.I < 1 || g.I > 256) return false;
+  // (longer rows: the bucket sort is the faster one -- 75 inputs x 65 536 rows 55 against 88 us, 147 x 50 176 59 against 164,
+  // but 54 x 65 536 48 against 45)
+  if (g.I < 1 || g.I > 64) return false;
   if (g.is_conv && (g.Kh > 255 || g.Kw > 255)) return false;
   return true;
 }
@@ -491,17 +447,8 @@ int launch_small_rows(const Geometry& g, const float* x, WalkEntry* lists, int* 
   long grid = ((long)g.R + kPixelWarps - 1) / kPixelWarps;
   const long cap = (long)li.num_sms * 8;
   if (grid > cap) grid = cap;
-  const int epl = (g.I + 31) / 32;
-  switch (epl) {   // 3, 5, 6, 7 keys per lane: the block network (a bitonic one would round them up to 4 and 8)
-    case 1: (void)launch_chained(snn_small_rows_kernel<1>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
-    case 2: (void)launch_chained(snn_small_rows_kernel<2>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
-    case 3: (void)launch_chained(snn_small_rows_kernel<3>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
-    case 4: (void)launch_chained(snn_small_rows_kernel<4>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
-    case 5: (void)launch_chained(snn_small_rows_kernel<5>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
-    case 6: (void)launch_chained(snn_small_rows_kernel<6>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
-    case 7: (void)launch_chained(snn_small_rows_kernel<7>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
-    default: (void)launch_chained(snn_small_rows_kernel<8>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride); break;
-  }
+  if (g.I <= 32) (void)launch_chained(snn_small_rows_kernel<1>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride);
+  else (void)launch_chained(snn_small_rows_kernel<2>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }

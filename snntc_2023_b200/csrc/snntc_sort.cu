@@ -1,5 +1,5 @@
-// Sorted lists of rows that neither the merging builder nor the register network (snntc_lists.cu) covers: dense rows of more
-// than 256 inputs, receptive fields of strided or larger convolutions. One bucket pass, then every bucket ranked in place.
+// Sorted lists of rows that neither the merging builder nor the register network (snntc_lists.cu) covers: rows of more than 64
+// inputs, dense or receptive fields of strided, larger or small convolutions. One bucket pass, then every bucket ranked in place.
 //
 // A list holds the row's inputs at or below MAX - 0.1, ascending in (value, source index). Per row:
 //   1. the keys (values as sortable 32-bit integers) of the inputs that can spike, their smallest and largest;
