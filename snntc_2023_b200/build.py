@@ -21,7 +21,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libsnntc_b200.so")
 LIB_MEASURE = os.path.join(HERE, "libsnntc_b200_measure.so")
-SOURCES = ["snntc_forward.cu", "snntc_sort.cu", "snntc_walk_ring.cu", "snntc_lists.cu", "snntc_backward.cu", "snntc_bwd_dense.cu",
+SOURCES = ["snntc_forward.cu", "snntc_sort.cu", "snntc_walk_ring.cu", "snntc_walk_rows.cu",
+           "snntc_lists.cu", "snntc_backward.cu", "snntc_bwd_dense.cu",
            "snntc_dw_skip.cu", "snntc_dw_tma.cu", "snntc_dx_sparse.cu", "snntc_pool.cu",
            "snntc_noalloc.cu", "snntc_train.cu", "snntc_api.cu"]
 NATIVE = os.path.join(HERE, "_native" + sysconfig.get_config_var("EXT_SUFFIX"))

@@ -22,6 +22,9 @@ struct Geometry {
   int B, H, W, C, Kh, Kw, Sh, Sw, pad_top, pad_left, Nh, Nw;
   // forward only: 1 = inference (the output is [R,J] spike values; 1/(sum w - theta) is not written)
   int infer;
+  // forward only, set by launch_forward: outputs per row of `out`. J itself is the row stride of the weights that the lists and
+  // walks use, which is jout rounded up to a multiple of four where the weights were copied with that padding.
+  int jout;
   // inference only, may be null: I+2 counters. khist[k] += 1 for every output that fired after consuming k inputs
   // (the bias input is not counted), khist[I+1] += 1 for every output that did not fire.
   int* khist;
@@ -46,6 +49,8 @@ struct Options {
                             // +4: read list entries straight from global memory instead of through shared memory
                             // +8: output pairs with the weights staged in shared memory (where they fit)
                             // 16: one output per lane, the warp's weight rows copied ahead into shared memory
+                            // 32, 64: several rows per warp (fan-out <= 64, a multiple of 4), weights from global memory /
+                            // in shared memory where they fit
   int walk_outputs = 0;     // 0 auto, 1..4: 1, 2, 4, 8 outputs per lane (pairs layout: 2 only)
   int list_builder = 0;     // 0 auto, 1 per-row bucket sort, 2 per-pixel sort + merges (3x3 stride-1 conv only),
                             // 3 per-row sorting network in registers (rows of at most 64 inputs);
@@ -107,6 +112,12 @@ int launch_merge_lists(const Geometry& g, const float* x, WalkEntry* lists, int*
 // The walk with one output per lane and weight rows copied ahead into shared memory (snntc_walk_ring.cu); any shape.
 int launch_walk_ring(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
                      const LaunchInfo& li, cudaStream_t s);
+
+// The walk with several rows per warp (snntc_walk_rows.cu): fan-out up to 64 and a multiple of four, weights 16-byte aligned;
+// reads g.wbound. resident: weights in shared memory where they fit.
+bool walk_rows_ok(const Geometry& g, const float* w);
+int launch_walk_rows(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
+                     bool resident, const LaunchInfo& li, cudaStream_t s);
 
 // Sorted lists of everything else by a bucket sort per row (snntc_sort.cu).
 int launch_row_sort(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride, const LaunchInfo& li,

@@ -59,17 +59,19 @@ __device__ __forceinline__ float walk_tolerance_base(const Geometry& g) {
 
 // bound[cluster] = sum over the weight rows of this cluster's eight CTAs of max_j |w_ij|: summed over the clusters an upper
 // bound on every column's sum of magnitudes. rows = I + bias row; CTA c takes rows [c * rows_per_cta, (c + 1) * rows_per_cta).
+// `padded` (may be null): receives the weights with rows of Jp >= J floats, zeros behind column J.
 // Bound by memory: up to 256 CTAs, 16 bytes per lane and load (32 CTAs read the 103 MB of a 25 088 x 1024 layer in 300 us).
 constexpr int kBoundClusters = 32;
 constexpr int kBoundCtas = 8 * kBoundClusters;
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256)
-snn_wbound_kernel(const float* __restrict__ w, int rows, int J, int rows_per_cta, float* __restrict__ bound) {
+snn_wbound_kernel(const float* __restrict__ w, int rows, int J, int rows_per_cta, float* __restrict__ bound,
+                  float* __restrict__ padded, int Jp) {
   chain_wait();
   chain_next();
   __shared__ float part[9];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r0 = blockIdx.x * rows_per_cta;
-  const bool v4 = (J & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+  const bool v4 = padded == nullptr && (J & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
   float acc = 0.f;                                     // lane 0: sum of the row maxima of this warp's rows
   for (int r = r0 + warp; r < min(rows, r0 + rows_per_cta); r += 8) {
     const float* wr = w + (size_t)r * J;
@@ -81,7 +83,11 @@ snn_wbound_kernel(const float* __restrict__ w, int rows, int J, int rows_per_cta
         m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
       }
     } else {
-      for (int j = lane; j < J; j += 32) m = fmaxf(m, fabsf(__ldg(wr + j)));
+      for (int j = lane; j < Jp; j += 32) {
+        const float v = j < J ? __ldg(wr + j) : 0.f;
+        m = fmaxf(m, fabsf(v));
+        if (padded != nullptr) padded[(size_t)r * Jp + j] = v;
+      }
     }
 #pragma unroll
     for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
@@ -133,8 +139,8 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* __r
     // VECW: a lane owns JPT consecutive outputs and reads them with 8- or 16-byte loads (J % JPT == 0,
     // so a lane is wholly inside or wholly outside the row); otherwise outputs lane + 32*m, 4-byte loads
     const int j = VECW ? jbase + JPT * lane + m : jbase + lane + 32 * m;
-    jok[m] = FULL || j < J;
-    jl[m] = jok[m] ? j : (VECW ? J - JPT + m : J - 1);
+    jok[m] = FULL || j < g.jout;
+    jl[m] = jok[m] ? j : (VECW ? J - JPT + m : J - 1);   // (padding behind jout: weights of zero, never stored)
     wsum[m] = -g.theta;
     ysum[m] = 0.f;
     if (g.has_bias) {  // the bias input (value biasvolt, weight row I) is always consumed first
@@ -333,7 +339,7 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* __
 #pragma unroll
   for (int m = 0; m < JP; ++m) {
     const int j = jbase + 2 * lane + 64 * m;
-    jok[m] = FULL || j < J;
+    jok[m] = FULL || j < g.jout;
     jl[m] = jok[m] ? j : J - 2;
     float n0 = g.theta, n1 = g.theta, y0 = 0.f, y1 = 0.f;
     if (g.has_bias) {  // the bias input (value biasvolt, weight row I) is always consumed first
@@ -500,8 +506,8 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* __
         yv = yy * iv;
         if (yv >= g.maxv) { yv = g.maxv; iv = 0.f; }
       }
-      if (jok[m]) {
-        const int j = jbase + 2 * lane + 64 * m + h;
+      const int j = jbase + 2 * lane + 64 * m + h;
+      if (FULL || j < g.jout) {
         y_row[j] = yv;
         if (inv_row != nullptr) inv_row[j] = iv;
         if (g.khist != nullptr) atomicAdd(g.khist + (yv < g.maxv ? entries_below(ents, nvalid, yv) : g.I + 1), 1);
@@ -520,12 +526,12 @@ snn_walk_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const in
   chain_next();
   __shared__ __align__(16) WalkEntry stage[STAGE ? kFwdWarps * 64 : 1];   // two blocks of 32 list entries per warp
   WalkEntry* sbuf = stage + (STAGE ? (threadIdx.x >> 5) * 64 : 0);
-  const int J = g.J, R = g.R;
+  const int R = g.R;
   const int lane = threadIdx.x & 31;
-  const int jchunks = (J + 32 * JPT - 1) / (32 * JPT);
-  const bool full_j = (J % (32 * JPT)) == 0;
+  const int jchunks = (g.jout + 32 * JPT - 1) / (32 * JPT);
+  const bool full_j = (g.jout % (32 * JPT)) == 0;
   float* __restrict__ y_out = out;
-  float* __restrict__ inv_out = g.infer ? nullptr : out + (size_t)R * J;
+  float* __restrict__ inv_out = g.infer ? nullptr : out + (size_t)R * g.jout;
   const long items = (long)(row_end - row_begin) * jchunks;
   const long wstride = (long)gridDim.x * kFwdWarps;
   constexpr int CH = JPT >= 8 ? 2 : (JPT >= 4 ? 4 : 8);
@@ -535,9 +541,9 @@ snn_walk_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const in
     const WalkEntry* krow = keys_g + (size_t)r * istride;
     const int n = __shfl_sync(0xffffffffu, __ldg(nvalid_g + r), 0);
     if (full_j)
-      walk_row<JPT, CH, true, VECW, STAGE>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * J, (inv_out ? inv_out + (size_t)r * J : nullptr), sbuf);
+      walk_row<JPT, CH, true, VECW, STAGE>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * g.jout, (inv_out ? inv_out + (size_t)r * g.jout : nullptr), sbuf);
     else
-      walk_row<JPT, CH, false, VECW, STAGE>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * J, (inv_out ? inv_out + (size_t)r * J : nullptr), sbuf);
+      walk_row<JPT, CH, false, VECW, STAGE>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * g.jout, (inv_out ? inv_out + (size_t)r * g.jout : nullptr), sbuf);
     if (STAGE) __syncwarp();   // the next row's first block goes into the buffer this row may have read last
   }
 }
@@ -551,7 +557,7 @@ snn_walk2_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const i
   chain_next();
   __shared__ __align__(16) WalkEntry stage[STAGE ? kFwdWarps * 64 : 1];   // two blocks of 32 list entries per warp
   WalkEntry* sbuf = stage + (STAGE ? (threadIdx.x >> 5) * 64 : 0);
-  const int J = g.J, R = g.R;
+  const int J = g.jout, R = g.R;
   const int lane = threadIdx.x & 31;
   const int jchunks = (J + 64 * JP - 1) / (64 * JP);
   const bool full_j = (J % (64 * JP)) == 0;
@@ -669,7 +675,7 @@ size_t nvalid_bytes(const Geometry& g) { return nvalid_only_bytes(g) + 256; }
 template <int JPT, bool VECW>
 int launch_walk(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g, const float* w, float* out,
                 const LaunchInfo& li, cudaStream_t s, int row_begin, int row_end, bool stage) {
-  const int jchunks = (g.J + 32 * JPT - 1) / (32 * JPT);
+  const int jchunks = (g.jout + 32 * JPT - 1) / (32 * JPT);
   const long items = (long)(row_end - row_begin) * jchunks;
   long grid = (items + kFwdWarps - 1) / kFwdWarps;
   const long cap = (long)li.num_sms * 8;
@@ -757,9 +763,17 @@ unsigned long long walk_copy_timeouts() {
   return n;
 }
 
+// Where the padded copy of the weights lies in the workspace (fan-out no multiple of four), behind the sorted lists, their
+// lengths and (conv layers that qualify) the scratch of the merging list builder.
+static size_t padded_weights_at(const Geometry& g) {
+  return (keys_bytes(g) + nvalid_bytes(g) + (merge_lists_shape_ok(g) ? merge_lists_bytes(g) : 0) + 255) & ~(size_t)255;
+}
+static size_t padded_weights_bytes(const Geometry& g) {
+  return (g.J & 3) == 0 ? 0 : (size_t)(g.I + 1) * ((g.J + 3) & ~3) * sizeof(float);
+}
+
 size_t forward_workspace_bytes(const Geometry& g) {
-  // sorted lists, their lengths, and (conv layers that qualify) the scratch of the merging list builder
-  return keys_bytes(g) + nvalid_bytes(g) + (merge_lists_shape_ok(g) ? merge_lists_bytes(g) : 0);
+  return padded_weights_at(g) + padded_weights_bytes(g);
 }
 
 int launch_forward(const Geometry& g_in, const float* x, const float* w, float* out, void* ws, size_t ws_bytes,
@@ -777,16 +791,28 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   // The walk that copies its weight rows ahead, up to about 24 items of 32 outputs per SM (8 where the rows have to be copied
   // 4 bytes at a time): with few warps on an SM latency is what counts, with many the instructions per output. Measured lines:
   // 784 -> 400 crosses at 3 300 items, 4096 -> 512 behind 4 100, 3x3 convolutions of 128 and 256 channels between 2 000 and 4 100.
+  g.jout = g.J;
+  const bool own = opt.walk_layout == 0 && opt.walk_outputs == 0;    // the library's own choice
   const long ring_items = (long)g.R * ((g.J + 31) / 32);
+  // A fan-out that is no multiple of four: with more than a few items the weights are copied with padded rows (by the kernel that
+  // reads them for the bound), so that every walk reads them 16 bytes at a time.
+  const int jp = (g.J + 3) & ~3;
+  const bool pad = own && jp != g.J && ring_items > 8L * li.num_sms && (long long)(g.I + 1) * jp <= INT_MAX;
+  const float* const w_in = w;
+  float* const w_padded = reinterpret_cast<float*>(static_cast<unsigned char*>(ws) + padded_weights_at(g_in));
+  if (pad) {
+    w = w_padded;
+    g.J = jp;
+  }
   const bool copies16 = (g.J & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
-  const bool ring = (opt.walk_layout & 16) != 0 ||
-                    (opt.walk_layout == 0 && opt.walk_outputs == 0 && ring_items <= (copies16 ? 24L : 8L) * li.num_sms);
-  if ((fparts & 2) && !ring) {   // the walk's bound on the weight sums (see walk_tolerance_base)
+  const bool ring = (opt.walk_layout & 16) != 0 || (own && ring_items <= (copies16 ? 24L : 8L) * li.num_sms);
+  const bool rows = !ring && walk_rows_ok(g, w) && (own || (opt.walk_layout & 96) != 0);
+  if ((fparts & 2) && (!ring || pad)) {   // the walk's bound on the weight sums (see walk_tolerance_base)
     const int rows_w = g.I + g.has_bias;
     int per = (rows_w + kBoundCtas - 1) / kBoundCtas;
     per = (per + 7) & ~7;                                // whole rounds of the CTA's eight warps
     g.wbound_n = (rows_w + 8 * per - 1) / (8 * per);     // clusters
-    (void)launch_chained(snn_wbound_kernel, 8 * g.wbound_n, 256, 0, s, 0, w, rows_w, g.J, per, wbound);
+    (void)launch_chained(snn_wbound_kernel, 8 * g.wbound_n, 256, 0, s, 0, w_in, rows_w, g.jout, per, wbound, pad ? w_padded : nullptr, g.J);
     count_launch();
     if (cudaGetLastError() != cudaSuccess) return E_CUDA;
   }
@@ -841,6 +867,7 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   auto walk = [&](cudaStream_t st, int r0, int r1) -> int {
     if (!(fparts & 2)) return OK;
     if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, li, st);
+    if (rows) return launch_walk_rows(g, keys_g, nvalid_g, key_stride(g), w, out, own ? g.R >= 8192 : (opt.walk_layout & 64) != 0, li, st);
     if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage, smemw_bytes, smemw_shift);
     if (variant == 1) {
       // pairs layout: 64 outputs per warp, or (walk_outputs 3) 128 as two pairs per lane

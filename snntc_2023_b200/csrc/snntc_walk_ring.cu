@@ -139,7 +139,7 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
   };
 
   const int j = j0 + lane;
-  const bool ok = j < J;
+  const bool ok = j < g.jout;
 #pragma unroll
   for (int b = 0; b < kRing - 1; ++b) {
     read_list(b);
@@ -220,8 +220,8 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
     if (yv >= g.maxv) { yv = g.maxv; iv = 0.f; }
   }
   if (ok) {
-    out[(size_t)r * J + j] = yv;
-    if (!g.infer) out[(size_t)(g.R + r) * J + j] = iv;
+    out[(size_t)r * g.jout + j] = yv;
+    if (!g.infer) out[(size_t)(g.R + r) * g.jout + j] = iv;
     if (g.khist != nullptr) atomicAdd(g.khist + (yv < g.maxv ? entries_below(ents, n, yv) : g.I + 1), 1);
   }
 }

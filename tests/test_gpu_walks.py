@@ -1,0 +1,64 @@
+"""The walk that copies its weight rows ahead into shared memory (csrc/snntc_walk_ring.cu) and the one with several rows per warp
+(csrc/snntc_walk_rows.cu), against the oracle's protocol and bit for bit against the walk from global memory: fan-in around the
+edges of groups (4, 8 entries), blocks (16, 32) and the ring of weight blocks, ragged fan-out, rows of unequal length, ties,
+inputs below the bias input, rows whose every output fires early. And fan-outs whose weights are copied with padded rows."""
+import numpy as np
+import pytest
+
+import oracle as O
+from tests import parity as P
+
+pytestmark = pytest.mark.gpu
+
+LAYOUTS = (16, 32, 64)   # walk_layout of the measurement build: copied ahead; rows per warp, weights global / in shared memory
+
+
+def _checked(x, w, params):
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    a = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=1 if w.shape[1] % 2 == 0 else 2))
+    for layout in LAYOUTS:   # (the last two need a fan-out up to 64 that is a multiple of four)
+        b = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=layout))
+        assert torch.equal(a, b), "layout %d" % layout
+    return b
+
+
+@pytest.mark.parametrize("I", [1, 7, 8, 9, 63, 64, 65, 127, 129, 257, 384, 385, 784, 1500])
+@pytest.mark.parametrize("J", [1, 4, 10, 20, 36, 63, 64, 100, 130])
+def test_walks_agree_with_the_walk_from_global_memory(I, J):
+    bv = 1.0 if (I + J) % 3 else 0.0
+    x, w = P.make_inputs(1000 * I + J, (5, I), (I + (bv > 0), J), "ref" if I > 8 else "test", bias=bv > 0)
+    params = O.fc_params(biasvolt=bv)
+    bc = _checked(x, w, params).cpu().numpy()
+    P.check_forward(bc[:5], bc[5:], O.fc_forward(x, w, params, "f32"), O.fc_forward(x, w, params, "f64"), rows=x,
+                    what="ring walk I=%d J=%d" % (I, J), max_flagged=0.2)
+
+
+@pytest.mark.parametrize("bv", [0.0, 1.0])
+@pytest.mark.parametrize("lo,hi", [(4, 40), (1, 12), (-8, 12)])
+def test_walks_on_exact_ties_and_inputs_below_the_bias_input(bv, lo, hi):
+    rng = np.random.default_rng(10 * abs(lo) + hi)
+    x = (rng.integers(lo, hi, size=(9, 300)) / 4.0).astype(np.float32)
+    x[::2, ::3] = 1e5
+    w = (rng.integers(-12, 13, size=(300 + (bv > 0), 96)) / 4.0).astype(np.float32)
+    _checked(x, w, O.fc_params(biasvolt=bv))
+
+
+def test_walks_stop_when_every_output_has_fired():
+    rng = np.random.default_rng(3)
+    x = np.exp(rng.random((4, 2000))).astype(np.float32)
+    w = np.abs(rng.standard_normal((2001, 70))).astype(np.float32)     # positive weights: everything fires within a few entries
+    assert float(_checked(x, w, O.fc_params(biasvolt=1.0))[:4].max()) < 1e5
+
+
+@pytest.mark.parametrize("R,I,J", [(1300, 40, 3), (1300, 90, 10), (2500, 70, 33), (700, 130, 77), (300, 257, 215)])
+def test_padded_weight_rows(R, I, J):
+    """Enough items that a fan-out that is no multiple of four gets padded weights: the same bits as without (layout 2)."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    x, w = P.make_inputs(R + I + J, (R, I), (I + 1, J), "ref", bias=True)
+    params = O.fc_params(biasvolt=1.0)
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    assert torch.equal(ops.snn_fc(xd, wd, params), ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2)))
+    assert torch.equal(ops.snn_fc_infer(xd, wd, params), ops.snn_fc(xd, wd, params)[:R])
