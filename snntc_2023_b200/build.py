@@ -23,7 +23,8 @@ LIB = os.path.join(HERE, "libsnntc_b200.so")
 LIB_MEASURE = os.path.join(HERE, "libsnntc_b200_measure.so")
 SOURCES = ["snntc_forward.cu", "snntc_sort.cu", "snntc_walk_ring.cu", "snntc_walk_rows.cu",
            "snntc_lists.cu", "snntc_backward.cu", "snntc_bwd_dense.cu",
-           "snntc_dw_skip.cu", "snntc_dw_tma.cu", "snntc_dx_sparse.cu", "snntc_pool.cu",
+           "snntc_dw_skip.cu", "snntc_dw_tma.cu", "snntc_dx_sparse.cu", "snntc_dx_few.cu",
+           "snntc_pool.cu",
            "snntc_noalloc.cu", "snntc_train.cu", "snntc_api.cu"]
 NATIVE = os.path.join(HERE, "_native" + sysconfig.get_config_var("EXT_SUFFIX"))
 NATIVE_SOURCE = os.path.join(CSRC, "snntc_torch.cpp")

@@ -1039,8 +1039,11 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
       gate.nz = nz_count;
       gate.threshold = (unsigned)(((size_t)g.R * g.J) / 5 * 2);
     }
-    if (sparse_ok) rc = launch_dx_sparse(g, uv, x, w, out, dx, dx_scratch, gate, li, sdx);
-    if (rc == OK && (!sparse_ok || both)) {
+    // Few channels (or a count the list-walking kernel does not take): the lanes over the outputs.
+    const bool few = dx_few_supported(g) && (opt.dx_kernel == 3 || (opt.dx_kernel == 0 && !sparse_ok && g.C < 16));
+    if (few) rc = launch_dx_few(g, uv, x, w, out, dx, li, sdx);
+    else if (sparse_ok) rc = launch_dx_sparse(g, uv, x, w, out, dx, dx_scratch, gate, li, sdx);
+    if (rc == OK && !few && (!sparse_ok || both)) {
       if (vec && P >= 64 * kWideP && (reinterpret_cast<uintptr_t>(dx) & 15) == 0) {   // it stores dx 16 bytes at a time
         dim3 gridw((unsigned)((P + kWideP - 1) / kWideP), (CH + kTile - 1) / kTile);
         (void)launch_chained(snn_dx_wide_kernel, gridw, kBwdThreads, 0, sdx, 0, gate, g, uv, x, w, out, dx);

@@ -59,7 +59,8 @@ struct Options {
   int dw_kernel = 0;        // 0 auto, 1 dense register tile, 2 row-skipping kernel (conv, C % 4 == 0) with per-thread
                             // copies, 4 the row-skipping kernel fed through tensor maps (where the shape allows)
   int dx_kernel = 0;        // 0 auto (conv layers the list-walking kernel supports: both queued, the device picks by
-                            // the share of outputs with a gradient), 1 dense register tile, 2 list-walking kernel
+                            // the share of outputs with a gradient), 1 dense register tile, 2 list-walking kernel,
+                            // 3 lanes over the outputs (conv)
   int overlap = -1;         // -1 library setting (snntc_set_overlap), 0 one stream, 1 dX beside dW
 };
 
@@ -168,6 +169,11 @@ struct DxGate {
   const unsigned* nz;
   unsigned threshold;
 };
+
+// dX of a convolution with the lanes over the outputs (snntc_dx_few.cu).
+bool dx_few_supported(const Geometry& g);
+int launch_dx_few(const Geometry& g, const float* uv, const float* x, const float* w, const float* y, float* dx,
+                  const LaunchInfo& li, cudaStream_t s);
 
 // dX by a kernel that walks, per input pixel, the lists of outputs with a non-zero gradient factor
 // (snntc_dx_sparse.cu). dx_sparse_bytes is its scratch (lists, their lengths, transposed weights).

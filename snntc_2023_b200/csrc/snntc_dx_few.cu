@@ -1,0 +1,96 @@
+// Input gradient of a convolution on few channels (SnnCvGrad, snntc/snncvgrad_kernels.cu.cc:15-84), up to 15 of them.
+//
+//   dX[p,c] = sum over receptive fields o that contain pixel p, outputs j of  [x_pc <= y_oj] u_oj W[(tap,c),j]
+//
+// The register-tile kernel (snn_dx_wide_kernel) works on 64 channels at a time and on every tap whatever the stride: with 3
+// channels and a 7x7 window at stride 2 that is 85 products formed for each one wanted, and a small image leaves most of the GPU
+// idle besides. Here a warp takes one pixel, its lanes the outputs j (coalesced reads of y, u and of the weight rows), and the
+// channels' sums sit in registers: per receptive field and 32 outputs two loads, then a load, a compare and a predicated FMA
+// per channel. Only the fields that really contain the pixel are visited. The lanes' sums are added by shuffles at the end, in a
+// fixed order: the same bits every run.
+// What bounds it: instruction issue and the L1 reads of the weights; 30 184 pixels x 3 channels, 7x7 stride 2, 128 outputs:
+// FEW_BEFORE -> FEW_NOW us.
+#include "snntc_common.cuh"
+
+namespace snntc {
+
+namespace {
+
+constexpr int kThreads = 256;
+
+// acc += [x <= y] * u * w as one compare and one predicated FMA
+__device__ __forceinline__ void masked_fma(float& acc, float x, float y, float u, float w) {
+  asm("{\n\t.reg .pred p;\n\tsetp.le.f32 p, %1, %2;\n\t@p fma.rn.f32 %0, %3, %4, %0;\n\t}"
+      : "+f"(acc) : "f"(x), "f"(y), "f"(u), "f"(w));
+}
+
+template <int CT>   // channels held per lane, >= C
+__global__ void __launch_bounds__(kThreads)
+snn_dx_few_kernel(const Geometry g, const float* __restrict__ uv, const float* __restrict__ x, const float* __restrict__ w,
+                  const float* __restrict__ y, float* __restrict__ dx) {
+  chain_wait();
+  chain_next();
+  const int lane = threadIdx.x & 31;
+  const int C = g.C, J = g.J;
+  const int c0 = blockIdx.y * CT;                // this block's channels c0 .. c0 + CT - 1
+  const int P = g.B * g.H * g.W;
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < P; p += warps) {
+    const int pw = p % g.W, t = p / g.W;
+    const int ph = t % g.H + g.pad_top, b = t / g.H, pl = pw + g.pad_left;
+    float xr[CT], acc[CT];
+#pragma unroll
+    for (int c = 0; c < CT; ++c) {
+      xr[c] = c0 + c < C ? __ldg(x + (size_t)p * C + c0 + c) : 0.f;
+      acc[c] = 0.f;
+    }
+    // fields nh with nh*Sh <= ph <= nh*Sh + Kh - 1
+    const int nh1 = min(ph / g.Sh, g.Nh - 1), nw1 = min(pl / g.Sw, g.Nw - 1);
+    const int nh0 = ph < g.Kh ? 0 : (ph - g.Kh) / g.Sh + 1, nw0 = pl < g.Kw ? 0 : (pl - g.Kw) / g.Sw + 1;
+    for (int nh = nh0; nh <= nh1; ++nh) {
+      for (int nw = nw0; nw <= nw1; ++nw) {
+        const int kh = ph - nh * g.Sh, kw = pl - nw * g.Sw;
+        const size_t o = ((size_t)(b * g.Nh + nh) * g.Nw + nw) * J;
+        const float* wt = w + ((size_t)(kh * g.Kw + kw) * C + c0) * J;
+#pragma unroll 2
+        for (int j = lane; j < J; j += 32) {
+          const float yy = __ldg(y + o + j), u = __ldg(uv + o + j);
+#pragma unroll
+          for (int c = 0; c < CT; ++c)
+            if (c0 + c < C) masked_fma(acc[c], xr[c], yy, u, __ldg(wt + (size_t)c * J + j));
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < CT; ++c) {
+#pragma unroll
+      for (int d = 16; d >= 1; d >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], d);
+      if (c0 + c < C && lane == c) dx[(size_t)p * C + c0 + c] = acc[c];
+    }
+  }
+}
+
+template <int CT>
+int launch(const Geometry& g, const float* uv, const float* x, const float* w, const float* y, float* dx, const LaunchInfo& li,
+           cudaStream_t s) {
+  const long P = (long)g.B * g.H * g.W;
+  long grid = (P + kThreads / 32 - 1) / (kThreads / 32);
+  if (grid > 16L * li.num_sms) grid = 16L * li.num_sms;
+  const cudaError_t e = launch_chained(snn_dx_few_kernel<CT>, dim3((unsigned)grid, (g.C + CT - 1) / CT), kThreads, 0, s, 0, g, uv, x, w, y, dx);
+  count_launch();
+  return e == cudaSuccess ? OK : E_CUDA;
+}
+
+}  // namespace
+
+bool dx_few_supported(const Geometry& g) { return g.is_conv; }
+
+int launch_dx_few(const Geometry& g, const float* uv, const float* x, const float* w, const float* y, float* dx,
+                  const LaunchInfo& li, cudaStream_t s) {
+  if (g.C == 1) return launch<1>(g, uv, x, w, y, dx, li, s);
+  if (g.C <= 4) return launch<4>(g, uv, x, w, y, dx, li, s);
+  if (g.C <= 8) return launch<8>(g, uv, x, w, y, dx, li, s);
+  return launch<16>(g, uv, x, w, y, dx, li, s);
+}
+
+}  // namespace snntc

@@ -806,7 +806,18 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   }
   const bool copies16 = (g.J & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
   const bool ring = (opt.walk_layout & 16) != 0 || (own && ring_items <= (copies16 ? 24L : 8L) * li.num_sms);
-  const bool rows = !ring && walk_rows_ok(g, w) && (own || (opt.walk_layout & 96) != 0);
+  // Several rows per warp for fan-out up to 64, where that leaves enough warps: 6 per SM at eight rows to a warp (fan-out 16;
+  // 10 where the weights miss the L1 cache), 14 at four (32), 48 at two (64). With fewer the pairs walk, a warp per row, hides
+  // its latencies better (5 880 rows of 6400 x 16: 540 against 770 us; 8 064 of 576 x 16: 107 against 61).
+  bool rows = !ring && walk_rows_ok(g, w) && (own || (opt.walk_layout & 96) != 0);
+  if (rows && own) {
+    const int lanes = g.J > 32 ? 16 : (g.J > 16 ? 8 : 4);
+    const long warps_per_sm = (long)g.R * lanes / 32 / li.num_sms;
+    const bool in_l1 = (size_t)(g.I + 1) * g.J * sizeof(float) <= (size_t)128 << 10;
+    rows = warps_per_sm >= (lanes == 16 ? 48 : (lanes == 8 ? 14 : (in_l1 ? 6 : 10)));
+    // (65 536 rows of 576 x 64: 364 us with the pairs walk and its weights in shared memory, 380 so; 262 144 of 27 x 64: 222, 208)
+    if (g.jout == 64 && g.I >= 128 && g.R >= 8192) rows = false;
+  }
   if ((fparts & 2) && (!ring || pad)) {   // the walk's bound on the weight sums (see walk_tolerance_base)
     const int rows_w = g.I + g.has_bias;
     int per = (rows_w + kBoundCtas - 1) / kBoundCtas;
@@ -867,7 +878,7 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   auto walk = [&](cudaStream_t st, int r0, int r1) -> int {
     if (!(fparts & 2)) return OK;
     if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, li, st);
-    if (rows) return launch_walk_rows(g, keys_g, nvalid_g, key_stride(g), w, out, own ? g.R >= 8192 : (opt.walk_layout & 64) != 0, li, st);
+    if (rows) return launch_walk_rows(g, keys_g, nvalid_g, key_stride(g), w, out, own ? g.J > 32 && g.R >= 32768 : (opt.walk_layout & 64) != 0, li, st);
     if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage, smemw_bytes, smemw_shift);
     if (variant == 1) {
       // pairs layout: 64 outputs per warp, or (walk_outputs 3) 128 as two pairs per lane
