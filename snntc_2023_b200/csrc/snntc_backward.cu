@@ -1039,8 +1039,12 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
       gate.nz = nz_count;
       gate.threshold = (unsigned)(((size_t)g.R * g.J) / 5 * 2);
     }
-    // Few channels (or a count the list-walking kernel does not take): the lanes over the outputs.
-    const bool few = dx_few_supported(g) && (opt.dx_kernel == 3 || (opt.dx_kernel == 0 && !sparse_ok && g.C < 16));
+    // Few channels: the lanes over the outputs. Up to eight channels always (8 at stride 1, every output with a gradient: 291 ->
+    // 190 us); up to 15 where the dense tile forms products for taps that a stride leaves out, or has fewer tiles than SMs (15
+    // channels at stride 1 on a full GPU: 291 us by the dense tile, 596 so; wider ones lose as well).
+    const bool wasteful = g.Sh * g.Sw >= 2 || (long)grid.x * grid.y < li.num_sms;
+    const bool few = dx_few_supported(g) &&
+                     (opt.dx_kernel == 3 || (opt.dx_kernel == 0 && !sparse_ok && (g.C <= 8 || (g.C < 16 && wasteful))));
     if (few) rc = launch_dx_few(g, uv, x, w, out, dx, li, sdx);
     else if (sparse_ok) rc = launch_dx_sparse(g, uv, x, w, out, dx, dx_scratch, gate, li, sdx);
     if (rc == OK && !few && (!sparse_ok || both)) {

@@ -815,8 +815,9 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     const long warps_per_sm = (long)g.R * lanes / 32 / li.num_sms;
     const bool in_l1 = (size_t)(g.I + 1) * g.J * sizeof(float) <= (size_t)128 << 10;
     rows = warps_per_sm >= (lanes == 16 ? 48 : (lanes == 8 ? 14 : (in_l1 ? 6 : 10)));
-    // (65 536 rows of 576 x 64: 364 us with the pairs walk and its weights in shared memory, 380 so; 262 144 of 27 x 64: 222, 208)
-    if (g.jout == 64 && g.I >= 128 && g.R >= 8192) rows = false;
+    // (65 536 rows of 576 x 64: 364 us with the pairs walk and its weights in shared memory, 380 so, but 16 384 rows 130 and 113;
+    // 262 144 of 27 x 64: 222, 208)
+    if (g.jout == 64 && g.I >= 128 && g.R >= 32768) rows = false;
   }
   if ((fparts & 2) && (!ring || pad)) {   // the walk's bound on the weight sums (see walk_tolerance_base)
     const int rows_w = g.I + g.has_bias;
@@ -874,7 +875,7 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   // from global memory are 5 % faster than two staged slices); walk_layout 8 asks for it wherever it fits, a named
   // layout switches it off
   const bool smemw = walk_smemw_ok(g, w, li, &smemw_bytes, &smemw_shift) &&
-                     ((opt.walk_layout & 8) != 0 || ((opt.walk_layout & 3) == 0 && g.J == 64 && g.R >= 8192));
+                     ((opt.walk_layout & 8) != 0 || ((opt.walk_layout & 3) == 0 && g.J == 64 && g.R >= 32768));
   auto walk = [&](cudaStream_t st, int r0, int r1) -> int {
     if (!(fparts & 2)) return OK;
     if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, li, st);
