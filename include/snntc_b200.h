@@ -244,13 +244,16 @@ SNNTC_API unsigned long long snntc_copy_timeouts(void);
  *   opts8 = { forward_parts   bit 0: build the sorted lists, bit 1: walk them (default 3; without bit 1 the
  *                             output is not written),
  *             walk_layout     0 auto, 1 output pairs, 2 outputs lane+32m, 3 consecutive outputs per lane; +4: list
- *                             entries straight from global memory instead of staged through shared memory,
+ *                             entries straight from global memory instead of staged through shared memory;
+ *                             +8 weights in shared memory, +16 weight rows copied ahead, +32 / +64 several rows per warp
+ *                             (+64: weights in shared memory),
  *             walk_outputs    0 auto, 1..4: 1, 2, 4, 8 outputs per lane,
  *             list_builder    0 auto, 1 per-row bucket sort, 2 per-pixel sort + merges,
  *             backward_parts  bit 0: dX, bit 1: dW (default 3),
- *             dw_kernel       0 auto, 1 dense register tile, 2 row-skipping kernel,
+ *             dw_kernel       0 auto, 1 dense register tile, 2 row-skipping kernel, 4 the same through tensor maps where
+ *                             the shape allows,
  *             overlap         -1 library setting, 0 one stream, 1 dX beside dW,
- *             dx_kernel       0 auto, 1 dense register tile, 2 list-walking kernel }
+ *             dx_kernel       0 auto, 1 dense register tile, 2 list-walking kernel, 3 lanes over the outputs }
  * A null opts8 means the defaults. All variants of a kernel give the same values (the walk variants the same
  * bits). snntc_fp32_probe queues `ctas` CTAs of 256 threads running `iters` rounds of 8 independent FMAs each
  * and reports the flop count: timed by the caller, it gives the FP32 issue ceiling the kernels are judged against.

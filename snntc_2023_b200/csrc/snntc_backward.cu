@@ -919,14 +919,18 @@ static float dw_scale(const Geometry& g) {
   return ldexpf(1.0f, -(e + 2));  // 2*maxv*s < 2^(e+1) * 2^-(e+2) = 1/2
 }
 
-// Where the row-skipping dW kernel is used: conv layers it supports with enough fan-in to fill its tiles. From 64 rows
-// on: it is never slower than the dense tile there (within a microsecond at 64 rows of 2305 x 256; 100 against 63 us at
-// 1024 rows), because it skips what carries no gradient and splits the rows finely.
-static bool want_dw_skip(const Geometry& g, const Options& opt) {
-  if (opt.dw_kernel == 1) return false;
-  if (!g.is_conv || (g.C & 3) != 0 || (g.J & 3) != 0) return false;
+// Where the row-skipping dW kernel is used: conv layers with enough fan-in to fill its tiles. From 64 rows on: it is never
+// slower than the dense tile there (within two microseconds at 64 rows of 2305 x 256; 95 -> 39 us at 1024 rows), because it skips
+// what carries no gradient and splits the rows finely. Channels or outputs that are no multiple of four are copied float by
+// float: from 4096 rows on (16 384 rows of 820 x 128: 266 us by the dense tile, 222 so, 130 with 12 % of the gradients; 256 rows:
+// 25 and 41), and for small windows of up to 128 outputs, which the kernel for small fan-in does not take, from 256 rows on (400 rows
+// of 26 x 16: 22 and 12).
+static bool want_dw_skip(const Geometry& g, const Options& opt, bool small_ok) {
+  if (opt.dw_kernel == 1 || !g.is_conv) return false;
   if (opt.dw_kernel >= 2) return true;
-  return g.R >= 64 && g.I >= 128;
+  if (((g.C | g.J) & 3) == 0) return g.R >= 64 && g.I >= 128;
+  if (g.I >= 128) return g.R >= 4096;
+  return g.R >= 256 && g.J <= 128 && !small_ok;
 }
 
 // Where the sparse dX kernel is used: conv layers it supports with enough receptive fields to be worth three launches.
@@ -948,7 +952,7 @@ static BackwardLayout backward_layout(const Geometry& g, const LaunchInfo& li) {
   Options any;
   any.dw_kernel = 2;
   any.dx_kernel = 2;
-  if (want_dw_skip(g, any)) {   // which dW kernel runs also depends on pointer alignment: sized for either
+  if (want_dw_skip(g, any, false)) {   // which dW kernel runs also depends on pointer alignment: sized for either
     int rps = 0;
     const size_t skip = (size_t)dw_skip_splits(g, li, &rps) * plane;
     if (skip > part) part = skip;
@@ -1065,7 +1069,7 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
     const size_t n = (size_t)Itot * g.J;
     int splits = 1;
     float* partial = dw;
-    if (want_dw_skip(g, opt) && dw_skip_supported(g, x, uv, out)) {
+    if (want_dw_skip(g, opt, dw_small_ok(g, uv, out)) && dw_skip_supported(g, x, uv, out)) {
       int rps = 0;
       partial = planes;   // always reduced from the workspace: its tiles are stored 16 bytes at a time
       // tiles through tensor maps where the shape allows (dw_kernel 2: per-thread copies whatever the shape)

@@ -11,23 +11,33 @@
 // saturating FMA (the clamp [x<=y](y-x) as the saturation of (y-x)*s, s a power of two, see snn_dw_kernel)
 // and half a two-lane FMA.
 //
-// CTA: 256 threads = 8 warps = 32 output channels; 128*QL fan-in rows; blockIdx.z takes a slice of the rows r.
-// The x tile (16 rows of r at a time, double buffered) is gathered straight from the NHWC image with 16-byte
+// CTA: 16 warps = 64 output channels (or 8 = 32); 128*QL fan-in rows; blockIdx.z takes a slice of the rows r.
+// The x tile (16 rows of r at a time, four or two stages in flight) is gathered straight from the NHWC image with 16-byte
 // asynchronous copies (four channels of one tap are contiguous), never passing through registers; taps outside
 // the image, rows past the slice and the bias row are plain 16-byte stores of constants (NOT copies from a
 // constant in global memory: every CTA fetching the same 16 bytes makes one L2 line the bottleneck of the kernel).
+//
+// Channel counts or fan-outs that are no multiple of four (VEC = false: the first layer of an image network, mostly) have no
+// aligned groups of four to copy: there every thread owns single columns of the x tile, copied 4 bytes at a time, y and u likewise,
+// and a lane holds pairs of fan-in rows instead of quadruples, so that the tile comes in steps of 64 and a narrow window does not
+// pay for 128.
+//
+// What bounds it: the copies and the shared memory reads of x where few outputs carry a gradient, then issue. 64 outputs per CTA
+// (each input copied once for twice the outputs), stages queued three ahead, one barrier a stage and one wave of CTAs against 32
+// outputs, two stages, two barriers and eight waves, dW of 131 072 rows of 829 x 128: all outputs that fired 1445 -> 1213 us, 12 %
+// of them 731 -> 506; 65 536 of 325 x 64 at stride 2: 201 -> 146, 135 -> 82. Without VEC, 131 072 of 820 x 128 against the dense
+// tile: 2012 -> 1469, 1998 -> 734.
 #include "snntc_common.cuh"
 
 #include <math_constants.h>
+#include <algorithm>
 #include <type_traits>
 
 namespace snntc {
 
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int kRS = 16;          // rows r per stage
-constexpr int kJT = 32;          // output channels per CTA (4 per warp)
 
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
   uint64_t r;
@@ -52,23 +62,31 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem_src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(gmem_src) : "memory");
+}
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <int QL>
-__global__ void __launch_bounds__(kThreads, 2)
+// VEC: C and J multiples of four, 16-byte aligned tensors; a lane holds QL quadruples of fan-in rows, else QL pairs
+template <int QL, bool VEC, int NW>
+__global__ void __launch_bounds__(32 * NW, 16 / NW)
 snn_dw_skip_kernel(const Geometry g, const float* __restrict__ uv, const float* __restrict__ x,
                    const float* __restrict__ out, float* __restrict__ partial, int rows_per_split,
                    float scale, const int* __restrict__ exact_flag) {
   chain_wait();
   chain_next();
-  constexpr int kTI = 128 * QL;        // fan-in rows per CTA
-  constexpr int kCh = 32 * QL;         // 16-byte chunks per row of the x tile
+  constexpr int kThreads = 32 * NW, kJT = 4 * NW;   // output channels per CTA, 4 per warp
+  constexpr int kDepth = NW == 16 ? 4 : 2;          // stages in shared memory
+  constexpr int CW = VEC ? 4 : 2;      // neighbouring fan-in rows of a lane
+  constexpr int kTI = 32 * CW * QL;    // fan-in rows per CTA
+  constexpr int kCh = 32 * QL;         // chunks of CW per row of the x tile
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* Xs = reinterpret_cast<float*>(smem_raw);                 // [2][kRS][kTI]
-  float* Ys = Xs + 2 * kRS * kTI;                                 // [2][kRS][kJT]
-  float* Us = Ys + 2 * kRS * kJT;                                 // [2][kRS][kJT]
-  int4* rowinfo = reinterpret_cast<int4*>(Us + 2 * kRS * kJT);    // [2][kRS]: .x element offset of the top-left pixel, .y its h, .z its w, .w row valid
+  float* Xs = reinterpret_cast<float*>(smem_raw);                 // [kDepth][kRS][kTI]
+  float* Ys = Xs + kDepth * kRS * kTI;                            // [kDepth][kRS][kJT]
+  float* Us = Ys + kDepth * kRS * kJT;                            // [kDepth][kRS][kJT]
+  int4* rowinfo = reinterpret_cast<int4*>(Us + kDepth * kRS * kJT);    // [2][kRS]: .x element offset of the top-left pixel, .y its h, .z its w, .w row valid
 
   const int J = g.J, I = g.I, R = g.R;
   const int Itot = I + g.has_bias;
@@ -88,8 +106,11 @@ snn_dw_skip_kernel(const Geometry g, const float* __restrict__ uv, const float* 
   // this thread's column chunk of the x tile (threads below kCh): .x element offset of its tap from a row's top-left
   // pixel, .y kh, .z kw, .w 1 = image tap, 2 = bias chunk, 0 = padding behind the last weight row
   int4 tapinfo_reg = make_int4(0, 0, 0, 0);
-  if (tid < kCh) {
-    const int i = i0 + 4 * tid;
+  // (with more threads, kXG of them own a chunk, each every kXG-th row)
+  constexpr int kXG = !VEC || kCh * 2 + 64 > kThreads ? 1 : (kCh * 4 + 64 > kThreads ? 2 : 4);
+  const int chunk = tid % kCh, xgroup = tid / kCh;
+  if (VEC && tid < kCh * kXG) {
+    const int i = i0 + 4 * chunk;
     if (i < I) {
       const int tap = i / g.C, c = i - tap * g.C;
       const int kh = tap / g.Kw, kw = tap - kh * g.Kw;
@@ -98,7 +119,7 @@ snn_dw_skip_kernel(const Geometry g, const float* __restrict__ uv, const float* 
       tapinfo_reg.w = 2;
     }
   }
-  auto fill_rowinfo = [&](int buf, int rb) {
+  auto fill_rowinfo = [&](int slot, int rb) {
     if (tid < kRS) {
       const int r = rb + tid;
       int4 ri = make_int4(0, 0, 0, 0);
@@ -112,27 +133,69 @@ snn_dw_skip_kernel(const Geometry g, const float* __restrict__ uv, const float* 
         ri.x = ((b * g.H + ri.y) * g.W + ri.z) * g.C;
         ri.w = 1;
       }
-      rowinfo[buf * kRS + tid] = ri;
+      rowinfo[slot * kRS + tid] = ri;
     }
   };
-  // Queues the asynchronous copies of the 16 rows starting at rb into buffer `buf` (rowinfo[buf] describes them).
-  // Thread t < kCh owns column chunk t of the x tile -- its tap is the same for every row and stays in registers --
-  // and walks the 16 rows; the other threads fetch the y and u tiles (16 rows x 8 chunks each).
-  static_assert(kCh < kThreads, "some threads must be left for the y and u tiles");
+  // Queues the asynchronous copies of the 16 rows starting at rb into buffer `buf` (rowinfo[slot] describes them). A thread
+  // t < kCh * kXG owns a column chunk of the x tile -- its tap is the same for every row and stays in registers -- and walks the
+  // rows; the other threads fetch the y and u tiles (16 rows x kJT / 4 chunks each).
+  static_assert(!VEC || kCh * kXG < kThreads, "some threads must be left for the y and u tiles");
   const int4 my_tap = tapinfo_reg;
-  auto issue = [&](int buf, int rb) {
-    if (tid < kCh) {
-      float* dst = Xs + buf * kRS * kTI + 4 * tid;
+  // Without VEC: this thread's columns col + kThreads*k (narrow tiles: one column, every kGroups-th row), their offsets
+  // and taps; tap -1: the bias row, -2: padding
+  constexpr int kCols = (kTI + kThreads - 1) / kThreads;
+  constexpr int kGroups = kTI <= kThreads / 2 ? kThreads / kTI : 1;
+  const int col = kGroups > 1 ? tid % kTI : tid, group = kGroups > 1 ? tid / kTI : 0;
+  int col_off[kCols], col_tap[kCols];
+  if constexpr (!VEC) {
 #pragma unroll
-      for (int rl = 0; rl < kRS; ++rl) {
-        const int4 ri = rowinfo[buf * kRS + rl];   // the same word for the whole warp: a broadcast
+    for (int k = 0; k < kCols; ++k) {
+      const int i = i0 + col + k * kThreads;
+      col_off[k] = 0;
+      col_tap[k] = i == I && g.has_bias ? -1 : -2;
+      if (i < I) {
+        const int tap = i / g.C, c = i - tap * g.C;
+        const int kh = tap / g.Kw, kw = tap - kh * g.Kw;
+        col_off[k] = (kh * g.W + kw) * g.C + c;
+        col_tap[k] = kh << 16 | kw;
+      }
+    }
+  }
+  auto issue = [&](int buf, int slot, int rb) {
+    if constexpr (!VEC) {
+#pragma unroll 4
+      for (int rl = group < kGroups ? group : kRS; rl < kRS; rl += kGroups) {
+        const int4 ri = rowinfo[slot * kRS + rl];
+#pragma unroll
+        for (int k = 0; k < kCols; ++k) {
+          if (col + k * kThreads >= kTI) break;
+          float* dst = Xs + (buf * kRS + rl) * kTI + col + k * kThreads;
+          const bool in_image = ri.w != 0 && col_tap[k] >= 0 && (unsigned)(ri.y + (col_tap[k] >> 16)) < (unsigned)g.H &&
+                                (unsigned)(ri.z + (col_tap[k] & 0xffff)) < (unsigned)g.W;
+          if (in_image) cp_async4(dst, x + ((ptrdiff_t)ri.x + col_off[k]));
+          else *dst = ri.w != 0 && col_tap[k] == -1 ? g.biasvolt : g.maxv;
+        }
+      }
+#pragma unroll
+      for (int e = tid; e < 2 * kRS * kJT; e += kThreads) {
+        const int which = e / (kRS * kJT), rl = e / kJT % kRS, jl = e % kJT;
+        float* dst = (which == 0 ? Ys : Us) + (buf * kRS + rl) * kJT + jl;
+        if (rb + rl < r_end && j0 + jl < J) cp_async4(dst, (which == 0 ? out : uv) + (size_t)(rb + rl) * J + j0 + jl);
+        else *dst = 0.f;
+      }
+    } else if (tid < kCh * kXG) {
+      float* dst = Xs + buf * kRS * kTI + 4 * chunk;
+#pragma unroll
+      for (int rk = 0; rk < kRS / kXG; ++rk) {
+        const int rl = rk * kXG + xgroup;
+        const int4 ri = rowinfo[slot * kRS + rl];   // the same word for the whole warp: a broadcast
         const bool in_image = ri.w != 0 && my_tap.w == 1 && (unsigned)(ri.y + my_tap.y) < (unsigned)g.H &&
                               (unsigned)(ri.z + my_tap.z) < (unsigned)g.W;
         if (in_image) cp_async16(dst + rl * kTI, x + ((ptrdiff_t)ri.x + my_tap.x));
         else *reinterpret_cast<float4*>(dst + rl * kTI) = (ri.w != 0 && my_tap.w == 2) ? v_bias : v_never;
       }
     } else {
-      for (int e = tid - kCh; e < 2 * kRS * (kJT / 4); e += kThreads - kCh) {
+      for (int e = tid - kCh * kXG; e < 2 * kRS * (kJT / 4); e += kThreads - kCh * kXG) {
         const int which = e / (kRS * (kJT / 4));            // 0: y, 1: u
         const int h = e - which * (kRS * (kJT / 4));
         const int rl = h / (kJT / 4), cq = h - rl * (kJT / 4);
@@ -146,12 +209,14 @@ snn_dw_skip_kernel(const Geometry g, const float* __restrict__ uv, const float* 
     cp_async_commit();
   };
 
-  // acc[c][jj][h]: fan-in rows i0 + 4*(lane + 32c) + 2h, +1 (one 64-bit pair), output channel j0 + 4*warp + jj
-  uint64_t acc[QL][4][2];
+  // acc[c][jj][h]: fan-in rows i0 + CW*(lane + 32c) + 2h, +1 (one 64-bit pair), output channel j0 + 4*warp + jj
+  uint64_t acc[QL][4][CW / 2];
 #pragma unroll
   for (int c = 0; c < QL; ++c)
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) acc[c][jj][0] = acc[c][jj][1] = pack2(0.f, 0.f);
+    for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+      for (int h = 0; h < CW / 2; ++h) acc[c][jj][h] = pack2(0.f, 0.f);
 
   auto reduce_stage = [&](int buf, auto fast_c) {
     constexpr bool FAST = decltype(fast_c)::value;
@@ -168,11 +233,16 @@ snn_dw_skip_kernel(const Geometry g, const float* __restrict__ uv, const float* 
       todo &= todo - 1u;
       const float4 y4 = *reinterpret_cast<const float4*>(Ys + (buf * kRS + rl) * kJT + 4 * warp);
       const float4 u4 = *reinterpret_cast<const float4*>(Us + (buf * kRS + rl) * kJT + 4 * warp);
-      float xr[QL][4];
+      float xr[QL][CW];
 #pragma unroll
       for (int c = 0; c < QL; ++c) {
-        const float4 v = *reinterpret_cast<const float4*>(xs + rl * kTI + 4 * (lane + 32 * c));
-        xr[c][0] = v.x; xr[c][1] = v.y; xr[c][2] = v.z; xr[c][3] = v.w;
+        if constexpr (VEC) {
+          const float4 v = *reinterpret_cast<const float4*>(xs + rl * kTI + 4 * (lane + 32 * c));
+          xr[c][0] = v.x; xr[c][1] = v.y; xr[c][2] = v.z; xr[c][3] = v.w;
+        } else {
+          const float2 v = *reinterpret_cast<const float2*>(xs + rl * kTI + 2 * (lane + 32 * c));
+          xr[c][0] = v.x; xr[c][1] = v.y;
+        }
       }
       const float yv[4] = {y4.x, y4.y, y4.z, y4.w};
       const float uu[4] = {u4.x, u4.y, u4.z, u4.w};
@@ -184,34 +254,34 @@ snn_dw_skip_kernel(const Geometry g, const float* __restrict__ uv, const float* 
         const uint64_t nu2 = pack2(nu, nu);
 #pragma unroll
         for (int c = 0; c < QL; ++c) {
-          float t[4];
+          float t[CW];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) t[k] = FAST ? fma_sat(xr[c][k], nsc, ys) : fmaxf(ys - xr[c][k], 0.f);
-          acc[c][jj][0] = fma2(pack2(t[0], t[1]), nu2, acc[c][jj][0]);
-          acc[c][jj][1] = fma2(pack2(t[2], t[3]), nu2, acc[c][jj][1]);
+          for (int k = 0; k < CW; ++k) t[k] = FAST ? fma_sat(xr[c][k], nsc, ys) : fmaxf(ys - xr[c][k], 0.f);
+#pragma unroll
+          for (int h = 0; h < CW / 2; ++h) acc[c][jj][h] = fma2(pack2(t[2 * h], t[2 * h + 1]), nu2, acc[c][jj][h]);
         }
       }
     }
   };
 
-  fill_rowinfo(0, r_begin);
-  fill_rowinfo(1, r_begin + kRS);
-  __syncthreads();
-  if (r_begin < r_end) issue(0, r_begin);
-  __syncthreads();   // rowinfo[0] is rewritten inside the loop: every thread must have queued its copies first
-
+  // Stage `it` + kDepth - 1 is queued while stage `it` is worked on; one barrier per stage, behind which that stage's copies are
+  // there for everyone and everyone is through with the buffer that is refilled.
+  for (int d = 0; d < kDepth - 1; ++d) {
+    fill_rowinfo(d & 1, r_begin + d * kRS);
+    __syncthreads();
+    issue(d, d & 1, r_begin + d * kRS);        // (rows from r_end on: an empty stage)
+  }
+  fill_rowinfo((kDepth - 1) & 1, r_begin + (kDepth - 1) * kRS);
   int it = 0;
   for (int rb = r_begin; rb < r_end; rb += kRS, ++it) {
-    const int buf = it & 1;
-    const bool more = rb + kRS < r_end;
-    if (more) issue(buf ^ 1, rb + kRS);
-    fill_rowinfo(buf, rb + 2 * kRS);   // this stage's entries were last read when its copies were queued
-    if (more) cp_async_wait<1>(); else cp_async_wait<0>();
+    cp_async_wait<kDepth - 2>();
     __syncthreads();
-    if (fast) reduce_stage(buf, std::true_type{});
-    else reduce_stage(buf, std::false_type{});
-    __syncthreads();
+    issue((it + kDepth - 1) % kDepth, (it + kDepth - 1) & 1, rb + (kDepth - 1) * kRS);
+    fill_rowinfo((it + kDepth) & 1, rb + kDepth * kRS);
+    if (fast) reduce_stage(it % kDepth, std::true_type{});
+    else reduce_stage(it % kDepth, std::false_type{});
   }
+  cp_async_wait<0>();
 
   float* __restrict__ dst = partial + (size_t)blockIdx.z * Itot * J;
   const int j = j0 + 4 * warp;
@@ -219,43 +289,53 @@ snn_dw_skip_kernel(const Geometry g, const float* __restrict__ uv, const float* 
 #pragma unroll
     for (int c = 0; c < QL; ++c)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
+      for (int h = 0; h < CW / 2; ++h) {
         float v[2][4];
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) unpack2(acc[c][jj][h], v[0][jj], v[1][jj]);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int i = i0 + 4 * (lane + 32 * c) + 2 * h + e;
-          if (i < Itot)
+          const int i = i0 + CW * (lane + 32 * c) + 2 * h + e;
+          if (i >= Itot) continue;
+          if (VEC || (J & 3) == 0) {
             *reinterpret_cast<float4*>(dst + (size_t)i * J + j) = make_float4(v[e][0], v[e][1], v[e][2], v[e][3]);
+          } else {
+#pragma unroll
+            for (int jj = 0; jj < 4; ++jj)
+              if (j + jj < J) dst[(size_t)i * J + j + jj] = v[e][jj];
+          }
         }
       }
   }
 }
 
-size_t smem_bytes(int QL) {
-  const size_t kTI = 128 * (size_t)QL;
-  return (2 * kRS * kTI + 4 * kRS * kJT) * sizeof(float) + 2 * kRS * sizeof(int4);
-}
+// Fan-in rows of a tile come in units of 128 (VEC) or 64.
+int tile_unit(bool vec) { return vec ? 128 : 64; }
+bool vec_shape(const Geometry& g) { return (g.C & 3) == 0 && (g.J & 3) == 0; }
 
 // fan-in tiles: as few as possible with at most 640 rows each, then the narrowest tile that covers the share
-void plan_tiles(int Itot, int* ntiles, int* ql) {
-  int n = (Itot + 639) / 640;
-  int per = (Itot + n - 1) / n;
-  int q = (per + 127) / 128;
-  if (q < 1) q = 1;
-  if (q > 5) q = 5;
+void plan_tiles(int Itot, bool vec, int* ntiles, int* ql) {
+  const int unit = tile_unit(vec);
+  const int n = (Itot + 639) / 640;
+  const int per = (Itot + n - 1) / n;
+  int q = (per + unit - 1) / unit;
+  if (!vec && q > 4) q = (q + 1) & ~1;   // widths that are compiled: 1 to 4, 6, 8 and 10 units of 64
   *ql = q;
-  *ntiles = (Itot + 128 * q - 1) / (128 * q);
+  *ntiles = (Itot + unit * q - 1) / (unit * q);
 }
 
-template <int QL>
+// 64 outputs per CTA halve the copies (which bound the kernel where few outputs carry a gradient) and leave room for four
+// stages; where that would leave half of a last CTA without outputs, 32 and two CTAs per SM.
+int plan_warps(const Geometry& g) { return (g.J & 63) == 0 || (g.J & 63) > 32 ? 16 : 8; }
+
+template <int QL, bool VEC, int NW>
 int launch_ql(const Geometry& g, const float* uv, const float* x, const float* out, float* partial, dim3 grid,
               int rows_per_split, float scale, const int* exact_flag, cudaStream_t s) {
-  const size_t smem = smem_bytes(QL);
-  if (allow_smem<snn_dw_skip_kernel<QL>>(smem) != cudaSuccess)
+  const size_t tile = (size_t)tile_unit(VEC) * QL;
+  const size_t smem = (NW == 16 ? 4 : 2) * kRS * (tile + 8 * NW) * sizeof(float) + 2 * kRS * sizeof(int4);
+  if (allow_smem<snn_dw_skip_kernel<QL, VEC, NW>>(smem) != cudaSuccess)
     return E_CUDA;
-  (void)launch_chained(snn_dw_skip_kernel<QL>, grid, kThreads, smem, s, 0, g, uv, x, out, partial, rows_per_split, scale, exact_flag);
+  (void)launch_chained(snn_dw_skip_kernel<QL, VEC, NW>, grid, 32 * NW, smem, s, 0, g, uv, x, out, partial, rows_per_split, scale, exact_flag);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -263,19 +343,19 @@ int launch_ql(const Geometry& g, const float* uv, const float* x, const float* o
 }  // namespace
 
 bool dw_skip_supported(const Geometry& g, const float* x, const float* uv, const float* out) {
-  if (!g.is_conv || (g.C & 3) != 0 || (g.J & 3) != 0) return false;
-  if (((uintptr_t)x | (uintptr_t)uv | (uintptr_t)out) & 15) return false;
+  if (!g.is_conv) return false;
+  if (vec_shape(g) && (((uintptr_t)x | (uintptr_t)uv | (uintptr_t)out) & 15)) return false;
   if ((long long)g.B * g.H * g.W * g.C > 0x7fffffffLL) return false;   // element offsets are 32-bit
-  return true;
+  return g.Kh < 32768 && g.Kw < 65536;
 }
 
 int dw_skip_splits(const Geometry& g, const LaunchInfo& li, int* rows_per_split) {
   int ntiles = 1, ql = 1;
-  plan_tiles(g.I + g.has_bias, &ntiles, &ql);
-  const long tiles = (long)ntiles * ((g.J + kJT - 1) / kJT);
-  // several waves of CTAs: the work of a CTA depends on how often ITS channels fired, small slices even that out
-  long want = (8L * li.num_sms + tiles - 1) / tiles;
-  const long max_splits = ((long)g.R + 4 * kRS - 1) / (4 * kRS);
+  plan_tiles(g.I + g.has_bias, vec_shape(g), &ntiles, &ql);
+  const int nw = plan_warps(g);
+  const long tiles = (long)ntiles * ((g.J + 4 * nw - 1) / (4 * nw));
+  long want = std::max(1L, 16L / nw * li.num_sms / tiles);   // one wave of CTAs, 512 threads per SM
+  const long max_splits = ((long)g.R + kRS - 1) / kRS;
   if (want > max_splits) want = max_splits;
   if (want > 1024) want = 1024;
   if (want < 1) want = 1;
@@ -290,15 +370,32 @@ int launch_dw_skip(const Geometry& g, const float* uv, const float* x, const flo
                    const LaunchInfo& li, cudaStream_t s) {
   (void)li;
   int ntiles = 1, ql = 1;
-  plan_tiles(g.I + g.has_bias, &ntiles, &ql);
-  dim3 grid((g.J + kJT - 1) / kJT, ntiles, splits);
-  switch (ql) {
-    case 1: return launch_ql<1>(g, uv, x, out, partial, grid, rows_per_split, scale, exact_flag, s);
-    case 2: return launch_ql<2>(g, uv, x, out, partial, grid, rows_per_split, scale, exact_flag, s);
-    case 3: return launch_ql<3>(g, uv, x, out, partial, grid, rows_per_split, scale, exact_flag, s);
-    case 4: return launch_ql<4>(g, uv, x, out, partial, grid, rows_per_split, scale, exact_flag, s);
-    default: return launch_ql<5>(g, uv, x, out, partial, grid, rows_per_split, scale, exact_flag, s);
-  }
+  plan_tiles(g.I + g.has_bias, vec_shape(g), &ntiles, &ql);
+  const int nw = plan_warps(g), jt = 4 * nw;
+  dim3 grid((g.J + jt - 1) / jt, ntiles, splits);
+  auto run = [&](auto launch) { return launch(g, uv, x, out, partial, grid, rows_per_split, scale, exact_flag, s); };
+  auto pick = [&](auto nw_c) {
+    constexpr int NW = decltype(nw_c)::value;
+    if (!vec_shape(g)) {
+      switch (ql) {
+        case 1: return run(launch_ql<1, false, NW>);
+        case 2: return run(launch_ql<2, false, NW>);
+        case 3: return run(launch_ql<3, false, NW>);
+        case 4: return run(launch_ql<4, false, NW>);
+        case 6: return run(launch_ql<6, false, NW>);
+        case 8: return run(launch_ql<8, false, NW>);
+        default: return run(launch_ql<10, false, NW>);
+      }
+    }
+    switch (ql) {
+      case 1: return run(launch_ql<1, true, NW>);
+      case 2: return run(launch_ql<2, true, NW>);
+      case 3: return run(launch_ql<3, true, NW>);
+      case 4: return run(launch_ql<4, true, NW>);
+      default: return run(launch_ql<5, true, NW>);
+    }
+  };
+  return nw == 16 ? pick(std::integral_constant<int, 16>{}) : pick(std::integral_constant<int, 8>{});
 }
 
 }  // namespace snntc

@@ -17,8 +17,14 @@
 // inner loop flushes a NaN to +0 (PTX .sat), and fmaxf(NaN, 0) of the unscaled loop is 0. The y and u tiles are two
 // more boxes, of the outputs seen as [image][row][column][channel]; where the map's width or height is no multiple
 // of the block, the fields past its edge read as u = 0 (zero fill) and are skipped like any field without a
-// gradient. Every copy completes on the mbarrier of its buffer; the warps wait for it (with a time limit) and meet
-// once per stage, after the arithmetic, before the buffer is refilled.
+// gradient. Every copy completes on the `full` mbarrier of its buffer; a warp waits for that (with a time limit),
+// does its arithmetic and arrives on the buffer's `empty` barrier, which whoever refills the buffer waits for. Nothing
+// holds the warps together stage by stage: how much a warp has to do depends on how many of its four channels carry
+// gradients, and with a barrier per stage every warp took the time of the busiest (the largest stall of the kernel).
+//
+// What bounds it: shared memory reads of x (about as many cycles as the arithmetic where few outputs carry a
+// gradient), then issue. With dW of 262 144 rows of 577 x 64, 12 % of the outputs carrying a gradient, 353 -> 256 us
+// against two stages, a CTA barrier per stage, 32 outputs per CTA and eight waves of CTAs; 200 704 x 1153 x 128 790 -> 658 us.
 //
 // The x tile of a stage is laid out [tap][row][channel] (one box after the other), so a fan-in tile is made of
 // whole taps, taps_per_tile = 640 / C of them; the bias row (x = biasvolt for every r) is a sum per output channel
@@ -27,6 +33,7 @@
 
 #include <cuda.h>
 #include <math_constants.h>
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -34,10 +41,9 @@ namespace snntc {
 
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int kRS = 16;          // rows r per stage
-constexpr int kJT = 32;          // output channels per CTA (4 per warp)
 constexpr int kMaxTileFloats = 640;
+constexpr int kMaxDepth = 8;     // stages in flight at most
 constexpr long long kWaitClocks = 2000000000LL;   // SM clocks a thread waits for a stage's copies (about a second)
 __device__ unsigned g_dw_copy_timeouts = 0u;        // CTAs that gave up waiting since the library was loaded
 
@@ -69,16 +75,19 @@ __device__ __forceinline__ void tma_load_4d(unsigned dst, const CUtensorMap* map
 // (the y / u boxes use the same instruction: coordinates (output channel, column, row, image), the channel
 // coordinate a multiple of 32)
 
-template <int QL, bool C256>   // C256: 256 channels (a chunk column is half a tap), else a power of two up to 128
-__global__ void __launch_bounds__(kThreads, 2)
+// C256: 256 channels (a chunk column is half a tap), else a power of two up to 128; NW warps
+template <int QL, bool C256, int NW>
+__global__ void __launch_bounds__(32 * NW, 16 / NW)
 snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                   const __grid_constant__ CUtensorMap map_u, const Geometry g, float* __restrict__ partial,
                   int stages_per_split, float scale, const int* __restrict__ exact_flag, int taps_per_tile,
-                  int wseg_log2) {
+                  int wseg_log2, int depth) {
+  constexpr int kJT = 4 * NW;                                      // output channels per CTA, 4 per warp
   chain_wait();
   chain_next();
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) unsigned long long bars[2];
+  __shared__ __align__(8) unsigned long long full[kMaxDepth], empty[kMaxDepth];
+  __shared__ int gave_up;
   unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);   // boxes land on 128-byte boundaries
   const int C = g.C, J = g.J, I = g.I;
   const int Itot = I + g.has_bias;
@@ -87,9 +96,9 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   const int ntap = max(0, min(taps_per_tile, taps - tap0));
   const bool bias_here = g.has_bias && blockIdx.y == gridDim.y - 1;
   const int xfloats = taps_per_tile * kRS * C;                     // floats of one x buffer
-  float* Xs = reinterpret_cast<float*>(base);                      // [2][taps_per_tile][kRS][C]
-  float* Ys = Xs + 2 * xfloats;                                    // [2][kRS][kJT]
-  float* Us = Ys + 2 * kRS * kJT;                                  // [2][kRS][kJT]
+  float* Xs = reinterpret_cast<float*>(base);                      // [depth][taps_per_tile][kRS][C]
+  float* Ys = Xs + depth * xfloats;                                // [depth][kRS][kJT]
+  float* Us = Ys + depth * kRS * kJT;                              // [depth][kRS][kJT]
 
   const bool fast = scale != 1.0f && __ldg(exact_flag) == 0;
   const float sc = fast ? scale : 1.0f;                 // s
@@ -106,36 +115,47 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   const int nstages = max(0, min(total_stages, s_begin + stages_per_split) - s_begin);
 
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bars[0])) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bars[1])) : "memory");
+    for (int d = 0; d < depth; ++d) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full[d])) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&empty[d])), "r"(NW) : "memory");
+    }
+    gave_up = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
 
-  // Thread 0 queues the copies of stage `st` into buffer `buf`: one box per tap, the y box and the u box.
+  // The calling warp queues the copies of stage `st` into buffer `buf`, a box per lane: the taps, then the y box and the u box.
   auto issue = [&](int st, int buf) {
     const int sg = s_begin + st;
     const int nw0 = (sg % WB) << wseg_log2;
     const int t = sg / WB;
     const int nh0 = (t % HB) * hseg;
     const int b = t / HB;
-    const unsigned bar = smem_u32(&bars[buf]);
-    const unsigned bytes = (unsigned)(ntap * kRS * C + 2 * kRS * kJT) * 4u;
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-    for (int tl = 0; tl < ntap; ++tl) {
-      const int tap = tap0 + tl;
-      const int kh = tap / g.Kw, kw = tap - kh * g.Kw;
-      tma_load_4d(smem_u32(Xs + buf * xfloats + tl * kRS * C), &map_x, bar, 0, nw0 - g.pad_left + kw,
-                  nh0 - g.pad_top + kh, b);
+    const unsigned bar = smem_u32(&full[buf]);
+    if (lane == 0) {
+      const unsigned bytes = (unsigned)(ntap * kRS * C + 2 * kRS * kJT) * 4u;
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
     }
-    tma_load_4d(smem_u32(Ys + buf * kRS * kJT), &map_y, bar, j0, nw0, nh0, b);
-    tma_load_4d(smem_u32(Us + buf * kRS * kJT), &map_u, bar, j0, nw0, nh0, b);
+    __syncwarp();
+    for (int tl = lane; tl < ntap + 2; tl += 32) {
+      if (tl < ntap) {
+        const int tap = tap0 + tl;
+        const int kh = tap / g.Kw, kw = tap - kh * g.Kw;
+        tma_load_4d(smem_u32(Xs + buf * xfloats + tl * kRS * C), &map_x, bar, 0, nw0 - g.pad_left + kw,
+                    nh0 - g.pad_top + kh, b);
+      } else if (tl == ntap) {
+        tma_load_4d(smem_u32(Ys + buf * kRS * kJT), &map_y, bar, j0, nw0, nh0, b);
+      } else {
+        tma_load_4d(smem_u32(Us + buf * kRS * kJT), &map_u, bar, j0, nw0, nh0, b);
+      }
+    }
+    __syncwarp();
   };
   // try_wait suspends the thread until the phase completes or a hardware time limit passes, so a waiting warp does
   // not take issue slots from the SM's other CTA; the clock bounds the number of attempts
-  auto copies_arrived = [&](int buf, unsigned parity) {
-    const unsigned bar = smem_u32(&bars[buf]);
+  auto passed = [&](const unsigned long long* barrier, unsigned parity) {
+    const unsigned bar = smem_u32(barrier);
     auto attempt = [&]() {
       unsigned ok;
       asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -147,7 +167,7 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       const long long t0 = clock64();
       do arrived = attempt(); while (!arrived && clock64() - t0 < kWaitClocks);
     }
-    return arrived;
+    return __all_sync(0xffffffffu, arrived) != 0;
   };
 
   // This lane's 16-byte chunks of the fan-in tile: chunk q = lane + 32c holds fan-in floats f = 4*lane + 128c of the
@@ -217,23 +237,32 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
   };
 
-  if (tid == 0) {
-    if (nstages > 0) issue(0, 0);
-    if (nstages > 1) issue(1, 1);
-  }
+  // The warps are not held together by a barrier per stage: a warp that is through with a stage says so on the buffer's `empty`
+  // barrier and goes on, ahead of the slowest by what is in flight. In turn, warp k mod NW when it comes to stage k, they wait
+  // until everyone is through with stage k - lag and queue stage k - lag + depth in its place.
+  for (int st = warp; st < min(depth, nstages); st += NW) issue(st, st);
+  const int lag = min(2, depth - 1);
   bool failed = false;
+  int buf = 0, rbuf = depth - lag;        // buffers of stages it and it - lag
+  unsigned phase = 0u, rphase = 1u;       // and the parities of their phases
   for (int it = 0; it < nstages; ++it) {
-    const int buf = it & 1;
-    if (!failed) failed = !copies_arrived(buf, (unsigned)(it >> 1) & 1u);
-    if (!failed) {
-      if (fast) reduce_stage(buf, std::true_type{});
-      else reduce_stage(buf, std::false_type{});
+    if (it >= lag && it % NW == warp && it - lag + depth < nstages) {
+      failed = !passed(&empty[rbuf], rphase);
+      if (failed) break;
+      issue(it - lag + depth, rbuf);
     }
-    // everyone is through with this buffer (or some thread's copies never came: the CTA stops)
-    if (__syncthreads_or(failed)) { failed = true; break; }
-    if (tid == 0 && it + 2 < nstages) issue(it + 2, buf);
+    failed = !passed(&full[buf], phase);
+    if (failed) break;
+    if (fast) reduce_stage(buf, std::true_type{});
+    else reduce_stage(buf, std::false_type{});
+    __syncwarp();
+    if (lane == 0) asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty[buf])) : "memory");
+    if (++buf == depth) { buf = 0; phase ^= 1u; }
+    if (++rbuf == depth) { rbuf = 0; rphase ^= 1u; }
   }
-  if (failed) {
+  if (failed) gave_up = 1;
+  __syncthreads();
+  if (gave_up != 0) {
     // give the copies that may still be in flight the same time once more before the shared memory is handed on
     if (tid == 0) atomicAdd(&g_dw_copy_timeouts, 1u);
     const long long t0 = clock64();
@@ -264,7 +293,7 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   }
 }
 
-struct TmaPlan { int taps_per_tile, ntiles, ql; size_t smem; };
+struct TmaPlan { int taps_per_tile, ntiles, ql, nw, depth; size_t smem; };
 
 TmaPlan plan(const Geometry& g) {
   TmaPlan p;
@@ -275,7 +304,13 @@ TmaPlan plan(const Geometry& g) {
   p.taps_per_tile = tpt;
   p.ntiles = (taps + tpt - 1) / tpt;                   // the bias row rides in the last tile
   p.ql = (tpt * g.C + 127) / 128;
-  p.smem = (size_t)2 * tpt * kRS * g.C * sizeof(float) + (size_t)4 * kRS * kJT * sizeof(float) + 128;
+  // 64 outputs per CTA read every input once for twice the outputs and leave room for four stages in flight; where that would
+  // leave half of a last CTA without outputs, 32 and two CTAs per SM (96 outputs: 54 against 58 us)
+  p.nw = (g.J & 63) == 0 || (g.J & 63) > 32 ? 16 : 8;
+  const size_t stage = (size_t)kRS * (tpt * g.C + 8 * p.nw) * sizeof(float);
+  const size_t room = (p.nw == 16 ? 224 : 111) * 1024;
+  p.depth = (int)std::min<size_t>(kMaxDepth, room / stage);
+  p.smem = p.depth * stage + 128;
   return p;
 }
 
@@ -302,7 +337,7 @@ EncodeTiledFn encode_tiled() {
 // how the 16 fields of a stage are laid over the output map: wseg columns (a power of two, at most 16) x 16/wseg rows
 int stage_wseg_log2(const Geometry& g) {
   int lg = 0;
-  while (lg < 4 && (1 << lg) < g.Nw) ++lg;
+  while ((1 << lg) < kRS && (1 << lg) < g.Nw) ++lg;
   return lg;
 }
 long stage_count(const Geometry& g) {
@@ -311,13 +346,13 @@ long stage_count(const Geometry& g) {
   return (long)g.B * ((g.Nh + hseg - 1) / hseg) * ((g.Nw + wseg - 1) / wseg);
 }
 
-template <int QL, bool C256>
+template <int QL, bool C256, int NW>
 int launch_ql(const CUtensorMap& mx, const CUtensorMap& my, const CUtensorMap& mu, const Geometry& g, float* partial,
               dim3 grid, int stages_per_split, float scale, const int* exact_flag, const TmaPlan& p, cudaStream_t s) {
-  if (allow_smem<snn_dw_tma_kernel<QL, C256>>(p.smem) != cudaSuccess)
+  if (allow_smem<snn_dw_tma_kernel<QL, C256, NW>>(p.smem) != cudaSuccess)
     return E_CUDA;
-  (void)launch_chained(snn_dw_tma_kernel<QL, C256>, grid, kThreads, p.smem, s, 0, mx, my, mu, g, partial, stages_per_split, scale, exact_flag,
-                                                             p.taps_per_tile, stage_wseg_log2(g));
+  (void)launch_chained(snn_dw_tma_kernel<QL, C256, NW>, grid, 32 * NW, p.smem, s, 0, mx, my, mu, g, partial, stages_per_split, scale, exact_flag,
+                       p.taps_per_tile, stage_wseg_log2(g), p.depth);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -342,12 +377,12 @@ bool dw_tma_supported(const Geometry& g, const float* x, const float* uv, const 
 // The stages are cut into `return value` slices of *stages_per_split stages each (blockIdx.z).
 int dw_tma_splits(const Geometry& g, const LaunchInfo& li, int* stages_per_split) {
   const TmaPlan p = plan(g);
-  const long tiles = (long)p.ntiles * ((g.J + kJT - 1) / kJT);
+  const long tiles = (long)p.ntiles * ((g.J + 4 * p.nw - 1) / (4 * p.nw));
   const long stages = stage_count(g);
-  // several waves of CTAs: the work of a CTA depends on how often ITS channels carry a gradient
-  long want = (8L * li.num_sms + tiles - 1) / tiles;
-  const long max_splits = (stages + 3) / 4;
-  if (want > max_splits) want = max_splits;
+  // one wave of CTAs (512 threads per SM): what a second one evens out is less than what its start and its planes cost (15 layers,
+  // sum of the times with 1, 2, 4 and 8 waves: 4829, 4968, 5107, 5511 us)
+  long want = std::max(1L, 16L / p.nw * li.num_sms / tiles);
+  if (want > stages) want = stages;
   if (want > 1024) want = 1024;
   if (want < 1) want = 1;
   const long sps = (stages + want - 1) / want;
@@ -363,6 +398,7 @@ int launch_dw_tma(const Geometry& g, const float* uv, const float* x, const floa
   const TmaPlan p = plan(g);
   const int lg = stage_wseg_log2(g);
   const cuuint32_t wseg = 1u << lg, hseg = (cuuint32_t)kRS >> lg;
+  const cuuint32_t jt = 4u * p.nw;
   const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
   CUtensorMap mx, my, mu;
   {
@@ -378,7 +414,7 @@ int launch_dw_tma(const Geometry& g, const float* uv, const float* x, const floa
     // the outputs as [image][row][column][channel]: fields past the edge of the map read as zero
     const cuuint64_t dims[4] = {(cuuint64_t)g.J, (cuuint64_t)g.Nw, (cuuint64_t)g.Nh, (cuuint64_t)g.B};
     const cuuint64_t strides[3] = {(cuuint64_t)g.J * 4, (cuuint64_t)g.Nw * g.J * 4, (cuuint64_t)g.Nh * g.Nw * g.J * 4};
-    const cuuint32_t box[4] = {(cuuint32_t)kJT, wseg, hseg, 1u};
+    const cuuint32_t box[4] = {jt, wseg, hseg, 1u};
     if (enc(&my, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(out), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
@@ -388,18 +424,21 @@ int launch_dw_tma(const Geometry& g, const float* uv, const float* x, const floa
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return E_UNSUPPORTED;
   }
-  dim3 grid((g.J + kJT - 1) / kJT, p.ntiles, splits);
-  if (g.C == 256) {   // tiles of one or two taps: 2 or 4 chunk columns
-    if (p.ql <= 2) return launch_ql<2, true>(mx, my, mu, g, partial, grid, stages_per_split, scale, exact_flag, p, s);
-    return launch_ql<4, true>(mx, my, mu, g, partial, grid, stages_per_split, scale, exact_flag, p, s);
-  }
-  switch (p.ql) {
-    case 1: return launch_ql<1, false>(mx, my, mu, g, partial, grid, stages_per_split, scale, exact_flag, p, s);
-    case 2: return launch_ql<2, false>(mx, my, mu, g, partial, grid, stages_per_split, scale, exact_flag, p, s);
-    case 3: return launch_ql<3, false>(mx, my, mu, g, partial, grid, stages_per_split, scale, exact_flag, p, s);
-    case 4: return launch_ql<4, false>(mx, my, mu, g, partial, grid, stages_per_split, scale, exact_flag, p, s);
-    default: return launch_ql<5, false>(mx, my, mu, g, partial, grid, stages_per_split, scale, exact_flag, p, s);
-  }
+  dim3 grid((g.J + jt - 1) / jt, p.ntiles, splits);
+  auto run = [&](auto launch) { return launch(mx, my, mu, g, partial, grid, stages_per_split, scale, exact_flag, p, s); };
+  auto pick = [&](auto nw) {
+    constexpr int NW = decltype(nw)::value;
+    if (g.C == 256)   // tiles of one or two taps: 2 or 4 chunk columns
+      return p.ql <= 2 ? run(launch_ql<2, true, NW>) : run(launch_ql<4, true, NW>);
+    switch (p.ql) {
+      case 1: return run(launch_ql<1, false, NW>);
+      case 2: return run(launch_ql<2, false, NW>);
+      case 3: return run(launch_ql<3, false, NW>);
+      case 4: return run(launch_ql<4, false, NW>);
+      default: return run(launch_ql<5, false, NW>);
+    }
+  };
+  return p.nw == 16 ? pick(std::integral_constant<int, 16>{}) : pick(std::integral_constant<int, 8>{});
 }
 
 unsigned long long dw_copy_timeouts() {
