@@ -4,10 +4,10 @@
 // With few warps on an SM a walk is bound by latency: the walk from global memory (snntc_forward.cu) waits an L2 round trip for
 // every four to eight weight rows and a vote with its branch at every step, 75 to 130 cycles a step. Here
 //   - weight rows arrive by asynchronous copies, 32 (or 16) entries to a block, two blocks ahead of the one that is consumed;
-//   - the sums and sign tests of eight steps are formed before one vote, from operands that were read a group ahead. The sums in front of every step of the group stay in
-//     registers, so where the vote finds an output at or near zero, only the steps concerned are taken through the
-//     reference's own comparisons (snntc/snnfc_kernels.cu.cc:46-55) and nothing is replayed (groups of four without the read
-//     ahead: 30 % slower at one row of 25 088 inputs);
+//   - the sums and sign tests of 16 (or 8) steps are formed before one vote, from operands that were read a group ahead. The
+//     sums in front of every step of the group stay in registers, so where the vote finds an output at or near zero, only the
+//     steps concerned are taken through the reference's own comparisons (snntc/snnfc_kernels.cu.cc:46-55) and nothing is
+//     replayed (groups of four without the read ahead: 30 % slower at one row of 25 088 inputs);
 //   - one output per lane: with a warp per scheduler every instruction of the dependent chain costs its latency, so the fewest
 //     instructions per step win (two outputs per lane, as pairs in 64-bit registers, took 82 cycles a step).
 // Arithmetic, order and decisions are those of walk_row: the same bits. The margin of a sign test is 2^-22 |x * sum w|, formed
@@ -29,7 +29,6 @@ namespace {
 constexpr int kWarps = 2;                          // per CTA, each on an item of its own
 constexpr int kRing = 3;                           // weight blocks per warp: one consumed, two on their way
 constexpr int kListRing = 4;                       // list blocks per warp
-constexpr int kGroup = 8;                          // steps per vote
 
 template <int kBlock>
 struct RingWarp {
@@ -56,7 +55,7 @@ struct Walk {
   int sticky;             // INT_MIN: the output was at or near zero at the last entry without firing, else INT_MAX
   float xprev;
 
-  template <int G>
+  template <bool FIRST, int G>
   __device__ __forceinline__ void steps(const float (&x)[G], const float (&w)[G]) {
     float sw[G], sy[G];
     int p[G];
@@ -71,6 +70,29 @@ struct Walk {
       ysum = fmaf(x[u], w[u], ysum);
     }
     if (__builtin_expect(__any_sync(0xffffffffu, m <= 0), 0)) {
+      // FIRST: every lane takes its own first step at or near zero through the comparisons, all lanes at once. Nearly always
+      // that step fires; where one does not, or was waited for from the group before, the steps are gone through one by one.
+      // (784 -> 400 at 32 samples with its sort 19.9 -> 17.3 us; where bandwidth counts the one by one code is the better one:
+      // 25 088 -> 1024 at 64 samples 819 us, 882 with FIRST)
+      if constexpr (FIRST) {
+        float tw = 0.f, ty = 0.f, tx = 0.f, txp = 0.f;
+        bool at = false;
+#pragma unroll
+        for (int u = G - 1; u >= 0; --u) {
+          if (p[u] <= 0) { tw = sw[u]; ty = sy[u]; tx = x[u]; txp = u == 0 ? xprev : x[u > 0 ? u - 1 : 0]; at = true; }
+        }
+        at &= live;
+        const bool hit = at & ratio_gt(ty, tw, txp) & ratio_le(ty, tw, tx);
+        if (!__any_sync(0xffffffffu, (at & !hit) | (sticky < 0))) {
+          if (hit) {
+            fin = make_float2(tw, ty);
+            wsum = -CUDART_INF_F;
+            live = false;
+          }
+          xprev = x[G - 1];
+          return;
+        }
+      }
 #pragma unroll
       for (int u = 0; u < G; ++u) {
         const bool near = live & (p[u] <= 0);
@@ -172,6 +194,7 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
     __syncwarp();
     const float* xb = sm.x[b % kListRing];
     const float* wb = &sm.w[b % kRing][0][lane];
+    constexpr int kGroup = kBlock / 2;             // steps per vote
     const int nb = min(kBlock, n - b * kBlock);
     int k = 0;
     // the next group's operands are read while this one's vote is on its way
@@ -189,18 +212,25 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
 #pragma unroll 1
     for (; k + 2 * kGroup <= nb; k += 2 * kGroup) {
       read(k + kGroup, x[1], wv[1]);
-      wk.steps<kGroup>(x[0], wv[0]);
+      wk.steps<kBlock == 32, kGroup>(x[0], wv[0]);
       read(k + 2 * kGroup < kBlock ? k + 2 * kGroup : 0, x[0], wv[0]);
-      wk.steps<kGroup>(x[1], wv[1]);
+      wk.steps<kBlock == 32, kGroup>(x[1], wv[1]);
     }
     if (k + kGroup <= nb) {
-      wk.steps<kGroup>(x[0], wv[0]);
+      wk.steps<kBlock == 32, kGroup>(x[0], wv[0]);
       k += kGroup;
+    }
+    if (kGroup > 8 && k + 8 <= nb) {
+      float x8[8], w8[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) { x8[u] = xb[k + u]; w8[u] = wb[(k + u) * 32]; }
+      wk.steps<kBlock == 32, 8>(x8, w8);
+      k += 8;
     }
 #pragma unroll 1
     for (; k < nb; ++k) {
       const float x1[1] = {xb[k]}, w1[1] = {wb[k * 32]};
-      wk.steps<1>(x1, w1);
+      wk.steps<false, 1>(x1, w1);
     }
     if (!__any_sync(0xffffffffu, wk.live)) break;  // every output has fired
   }
