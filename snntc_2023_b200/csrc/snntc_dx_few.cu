@@ -8,8 +8,11 @@
 // channels' sums sit in registers: per receptive field and 32 outputs two loads, then a load, a compare and a predicated FMA
 // per channel. Only the fields that really contain the pixel are visited. The lanes' sums are added by shuffles at the end, in a
 // fixed order: the same bits every run.
-// What bounds it: instruction issue and the L1 reads of the weights; 30 184 pixels x 3 channels, 7x7 stride 2, 128 outputs:
-// 1519 -> 90 us.
+// Where the fan-out is a multiple of four a lane takes four outputs at a time, 16 bytes to a load, and narrow fan-outs leave room
+// for several fields at once: a quarter of the load instructions, which bound the version with one output per lane and load.
+// What bounds it: instruction issue and the L1 reads of the weights; 30 184 pixels x 3 channels, 7x7 stride 2, 128 outputs: 1517 us
+// by the register tiles, 89 with one output per load, 62 with four; 200 704 pixels, 64 outputs: 3914, 439, 234; 65 536 x 8
+// channels, 3x3, 64 outputs: 291, 187, 140.
 #include "snntc_common.cuh"
 
 namespace snntc {
@@ -24,10 +27,12 @@ __device__ __forceinline__ void masked_fma(float& acc, float x, float y, float u
       : "+f"(acc) : "f"(x), "f"(y), "f"(u), "f"(w));
 }
 
-template <int CT>   // channels held per lane, >= C
+// CT: channels held per lane. V4: a lane takes four outputs at a time by 16-byte loads (J a multiple of 4, y, u and w aligned);
+// `lanes` = 4, 8, 16 or 32 of them take a field, 32 / lanes fields at once.
+template <int CT, bool V4>
 __global__ void __launch_bounds__(kThreads)
 snn_dx_few_kernel(const Geometry g, const float* __restrict__ uv, const float* __restrict__ x, const float* __restrict__ w,
-                  const float* __restrict__ y, float* __restrict__ dx) {
+                  const float* __restrict__ y, float* __restrict__ dx, int lanes) {
   chain_wait();
   chain_next();
   const int lane = threadIdx.x & 31;
@@ -47,17 +52,44 @@ snn_dx_few_kernel(const Geometry g, const float* __restrict__ uv, const float* _
     // fields nh with nh*Sh <= ph <= nh*Sh + Kh - 1
     const int nh1 = min(ph / g.Sh, g.Nh - 1), nw1 = min(pl / g.Sw, g.Nw - 1);
     const int nh0 = ph < g.Kh ? 0 : (ph - g.Kh) / g.Sh + 1, nw0 = pl < g.Kw ? 0 : (pl - g.Kw) / g.Sw + 1;
-    for (int nh = nh0; nh <= nh1; ++nh) {
-      for (int nw = nw0; nw <= nw1; ++nw) {
+    if constexpr (V4) {
+      const int cols = nw1 - nw0 + 1, fields = max(0, nh1 - nh0 + 1) * max(0, cols);
+      const int step = 32 / lanes;
+      int nh = nh0, nw = nw0 + lane / lanes;
+      for (int f = lane / lanes; f < fields; f += step, nw += step) {
+        while (nw > nw1) { nw -= cols; ++nh; }
         const int kh = ph - nh * g.Sh, kw = pl - nw * g.Sw;
         const size_t o = ((size_t)(b * g.Nh + nh) * g.Nw + nw) * J;
         const float* wt = w + ((size_t)(kh * g.Kw + kw) * C + c0) * J;
 #pragma unroll 2
-        for (int j = lane; j < J; j += 32) {
-          const float yy = __ldg(y + o + j), u = __ldg(uv + o + j);
+        for (int j = 4 * (lane & (lanes - 1)); j < J; j += 4 * lanes) {
+          const float4 yy = __ldg(reinterpret_cast<const float4*>(y + o + j));
+          const float4 u = __ldg(reinterpret_cast<const float4*>(uv + o + j));
 #pragma unroll
-          for (int c = 0; c < CT; ++c)
-            if (c0 + c < C) masked_fma(acc[c], xr[c], yy, u, __ldg(wt + (size_t)c * J + j));
+          for (int c = 0; c < CT; ++c) {
+            if (c0 + c >= C) break;
+            const float4 wv = __ldg(reinterpret_cast<const float4*>(wt + (size_t)c * J + j));
+            masked_fma(acc[c], xr[c], yy.x, u.x, wv.x);
+            masked_fma(acc[c], xr[c], yy.y, u.y, wv.y);
+            masked_fma(acc[c], xr[c], yy.z, u.z, wv.z);
+            masked_fma(acc[c], xr[c], yy.w, u.w, wv.w);
+          }
+        }
+      }
+      __syncwarp();
+    } else {
+      for (int nh = nh0; nh <= nh1; ++nh) {
+        for (int nw = nw0; nw <= nw1; ++nw) {
+          const int kh = ph - nh * g.Sh, kw = pl - nw * g.Sw;
+          const size_t o = ((size_t)(b * g.Nh + nh) * g.Nw + nw) * J;
+          const float* wt = w + ((size_t)(kh * g.Kw + kw) * C + c0) * J;
+#pragma unroll 2
+          for (int j = lane; j < J; j += 32) {
+            const float yy = __ldg(y + o + j), u = __ldg(uv + o + j);
+#pragma unroll
+            for (int c = 0; c < CT; ++c)
+              if (c0 + c < C) masked_fma(acc[c], xr[c], yy, u, __ldg(wt + (size_t)c * J + j));
+          }
         }
       }
     }
@@ -76,7 +108,11 @@ int launch(const Geometry& g, const float* uv, const float* x, const float* w, c
   const long P = (long)g.B * g.H * g.W;
   long grid = (P + kThreads / 32 - 1) / (kThreads / 32);
   if (grid > 16L * li.num_sms) grid = 16L * li.num_sms;
-  const cudaError_t e = launch_chained(snn_dx_few_kernel<CT>, dim3((unsigned)grid, (g.C + CT - 1) / CT), kThreads, 0, s, 0, g, uv, x, w, y, dx);
+  const bool v4 = (g.J & 3) == 0 && (((uintptr_t)uv | (uintptr_t)w | (uintptr_t)y) & 15) == 0;
+  const int lanes = g.J > 64 ? 32 : (g.J > 32 ? 16 : (g.J > 16 ? 8 : 4));
+  const dim3 grid2((unsigned)grid, (g.C + CT - 1) / CT);
+  const cudaError_t e = v4 ? launch_chained(snn_dx_few_kernel<CT, true>, grid2, kThreads, 0, s, 0, g, uv, x, w, y, dx, lanes)
+                           : launch_chained(snn_dx_few_kernel<CT, false>, grid2, kThreads, 0, s, 0, g, uv, x, w, y, dx, lanes);
   count_launch();
   return e == cudaSuccess ? OK : E_CUDA;
 }
@@ -88,9 +124,9 @@ bool dx_few_supported(const Geometry& g) { return g.is_conv; }
 int launch_dx_few(const Geometry& g, const float* uv, const float* x, const float* w, const float* y, float* dx,
                   const LaunchInfo& li, cudaStream_t s) {
   if (g.C == 1) return launch<1>(g, uv, x, w, y, dx, li, s);
+  if (g.C == 3) return launch<3>(g, uv, x, w, y, dx, li, s);
   if (g.C <= 4) return launch<4>(g, uv, x, w, y, dx, li, s);
-  if (g.C <= 8) return launch<8>(g, uv, x, w, y, dx, li, s);
-  return launch<16>(g, uv, x, w, y, dx, li, s);
+  return launch<8>(g, uv, x, w, y, dx, li, s);          // (more than eight channels: blocks of eight)
 }
 
 }  // namespace snntc
