@@ -942,6 +942,16 @@ static bool want_dx_sparse(const Geometry& g, const Options& opt) {
   return g.R >= 64 && g.J >= 16;
 }
 
+// Where the lanes-over-the-outputs dX kernel takes 16 channels or more that the lists do not take (no multiple of four): where the
+// dense tiles are fewer than the SMs, so that their rounds, 16 outputs of a tap each, follow one another (about 2.5 us a round; the
+// line is drawn at 0.15 us per tap and output). Its own time in microseconds is fitted to layers of 64 to 2900 pixels. (Where the
+// lists apply the choice stays between the two kernels whose sums have the same order.)
+static bool few_pixels(const Geometry& g, long P) {
+  if (g.J < 64 || (g.J & 3) != 0) return false;
+  const double taps = (double)g.Kh * g.Kw;
+  return 14.0 + 0.45e-6 * P * taps / ((double)g.Sh * g.Sw) * g.C * g.J < 0.15 * taps * g.J;
+}
+
 // workspace = u[R,J] | 256 bytes with the range flag of snn_u_kernel | the partial dW planes (sized for whichever dW
 // kernel needs more; none when neither splits the rows) | the scratch of the sparse dX kernel (conv layers it supports)
 struct BackwardLayout { size_t flag, planes, dx_scratch, total; };
@@ -1046,9 +1056,11 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
     // Few channels: the lanes over the outputs. Up to eight channels always (8 at stride 1, every output with a gradient: 291 ->
     // 190 us); up to 15 where the dense tile forms products for taps that a stride leaves out, or has fewer tiles than SMs (15
     // channels at stride 1 on a full GPU: 291 us by the dense tile, 596 so; wider ones lose as well).
-    const bool wasteful = g.Sh * g.Sw >= 2 || (long)grid.x * grid.y < li.num_sms;
+    const bool idle = (long)grid.x * grid.y < li.num_sms;
+    const bool wasteful = g.Sh * g.Sw >= 2 || idle;
     const bool few = dx_few_supported(g) &&
-                     (opt.dx_kernel == 3 || (opt.dx_kernel == 0 && !sparse_ok && (g.C <= 8 || (g.C < 16 && wasteful))));
+                     (opt.dx_kernel == 3 || (opt.dx_kernel == 0 && !sparse_ok &&
+                                             (g.C <= 8 || (g.C < 16 && wasteful) || (idle && vec && few_pixels(g, P)))));
     if (few) rc = launch_dx_few(g, uv, x, w, out, dx, li, sdx);
     else if (sparse_ok) rc = launch_dx_sparse(g, uv, x, w, out, dx, dx_scratch, gate, li, sdx);
     if (rc == OK && !few && (!sparse_ok || both)) {

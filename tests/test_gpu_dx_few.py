@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("B,H,W,C,Kh,Kw,Sh,Sw,Kc,padding", [
     (1, 5, 7, 1, 1, 1, 1, 1, 1, "SAME"), (2, 9, 8, 1, 5, 5, 2, 2, 40, "SAME"), (3, 12, 11, 3, 7, 7, 2, 2, 64, "SAME"),
     (2, 10, 13, 4, 3, 3, 1, 1, 33, "VALID"), (1, 11, 10, 5, 2, 3, 3, 1, 31, "VALID"), (2, 8, 9, 9, 3, 3, 2, 1, 100, "SAME"),
-    (1, 9, 9, 15, 5, 3, 1, 2, 8, "SAME"), (1, 8, 8, 18, 3, 3, 1, 1, 24, "SAME"), (2, 7, 7, 37, 3, 3, 2, 2, 36, "VALID")])
+    (1, 9, 9, 15, 5, 3, 1, 2, 8, "SAME"), (2, 6, 6, 17, 5, 5, 1, 1, 128, "SAME"), (1, 8, 8, 18, 3, 3, 1, 1, 24, "SAME"), (2, 7, 7, 37, 3, 3, 2, 2, 36, "VALID")])
 def test_conv_dx_with_lanes_over_the_outputs(B, H, W, C, Kh, Kw, Sh, Sw, Kc, padding):
     import torch
     from snntc_2023_b200 import _lib, ops
