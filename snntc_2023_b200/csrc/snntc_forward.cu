@@ -25,7 +25,11 @@ namespace snntc {
 
 namespace {
 
-constexpr int kFwdThreads = 256;
+// A CTA of the walks from global memory is two warps with one item each: the rows differ in length and in when their outputs have
+// fired, and small CTAs leave it to the hardware to give a free place the next item (eight warps that took every grid-th
+// item, 8 CTAs per SM: 2570 us for 131 072 rows of 576 x 128, 2370 so; 4096 of 1152 x 128: 135, 120; one item per warp but eight
+// warps: 2387, 135).
+constexpr int kFwdThreads = 64;
 constexpr int kFwdWarps = kFwdThreads / 32;
 
 typedef unsigned long long u64;
@@ -519,7 +523,7 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* __
 // ------------------------------------------------------------------------------------------- kernels
 // Walk kernel: every warp takes (row, block of 32*JPT outputs) items, adjacent warps share a row.
 template <int JPT, bool VECW, bool STAGE>
-__global__ void __launch_bounds__(kFwdThreads, JPT <= 4 ? 4 : 1)   // up to four outputs per lane: 64 registers, 32 warps per SM
+__global__ void __launch_bounds__(kFwdThreads, JPT <= 4 ? 1024 / kFwdThreads : 1)   // up to four outputs per lane: 64 registers, 32 warps per SM
 snn_walk_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const int* __restrict__ nvalid_g, int istride,
                 const float* __restrict__ w, float* __restrict__ out, int row_begin, int row_end) {
   chain_wait();
@@ -550,7 +554,7 @@ snn_walk_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const in
 
 // The same items with the outputs of a lane held in pairs (walk_row2): a warp covers 64*JP outputs.
 template <int JP, bool STAGE>
-__global__ void __launch_bounds__(kFwdThreads)
+__global__ void __launch_bounds__(kFwdThreads, 1024 / kFwdThreads)
 snn_walk2_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const int* __restrict__ nvalid_g, int istride,
                  const float* __restrict__ w, float* __restrict__ out, int row_begin, int row_end) {
   chain_wait();
@@ -678,8 +682,7 @@ int launch_walk(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g,
   const int jchunks = (g.jout + 32 * JPT - 1) / (32 * JPT);
   const long items = (long)(row_end - row_begin) * jchunks;
   long grid = (items + kFwdWarps - 1) / kFwdWarps;
-  const long cap = (long)li.num_sms * 8;
-  if (grid > cap) grid = cap;
+  if (grid > 0x7fffffffL) grid = 0x7fffffffL;      // (a warp goes on to item + warps of the grid)
   if (stage) (void)launch_chained(snn_walk_kernel<JPT, VECW, true>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
   else (void)launch_chained(snn_walk_kernel<JPT, VECW, false>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
   count_launch();
@@ -692,8 +695,7 @@ int launch_walk2(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g
   const int jchunks = (g.J + 64 * JP - 1) / (64 * JP);
   const long items = (long)(row_end - row_begin) * jchunks;
   long grid = (items + kFwdWarps - 1) / kFwdWarps;
-  const long cap = (long)li.num_sms * 8;
-  if (grid > cap) grid = cap;
+  if (grid > 0x7fffffffL) grid = 0x7fffffffL;      // (a warp goes on to item + warps of the grid)
   if (stage) (void)launch_chained(snn_walk2_kernel<JP, true>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
   else (void)launch_chained(snn_walk2_kernel<JP, false>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
   count_launch();
@@ -832,17 +834,17 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   }
   // Outputs per lane: more of them amortise the per-step cost (list entry, address, vote) over more
   // outputs, fewer give more (row, output block) items to spread over the SMs. `cost` is the measured number
-  // of instructions per warp-step, `ctas` how many CTAs fit per SM; with few items pick the smallest
+  // of instructions per warp-step, `warps` how many fit on an SM; with few items pick the smallest
   // estimate of (waves of items) x (cost of a step).
-  auto pick = [&](int unit, const double (&cost)[4], const int (&ctas)[4], int top) {
+  auto pick = [&](int unit, const double (&cost)[4], const int (&warps)[4], int top) {
     int best_c = top;
     const double items_top = (double)g.R * ((g.J + unit * (1 << top) - 1) / (unit * (1 << top)));
-    if (items_top < 4.0 * li.num_sms * ctas[top] * kFwdWarps) {
+    if (items_top < 4.0 * li.num_sms * warps[top]) {
       double best = 0;
       for (int c = 0; c <= top; ++c) {
         const int per = unit * (1 << c);
         const double items = (double)g.R * ((g.J + per - 1) / per);
-        const double slots = (double)li.num_sms * ctas[c] * kFwdWarps;
+        const double slots = (double)li.num_sms * warps[c];
         const double est = (double)(long)(items / slots + 0.999) * cost[c];
         if (c == 0 || est < best) { best = est; best_c = c; }
       }
@@ -856,10 +858,10 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   const bool al16 = (g.J % 4 == 0) && (reinterpret_cast<uintptr_t>(w) % 16 == 0);
   const bool al32 = al16 && (g.J % 8 == 0);
   const double cost[4] = {19.0, 24.0, 39.0, 62.0};
-  const int ctas[4] = {6, 4, 4, 2};
+  const int warps[4] = {48, 32, 32, 16};
   // (eight outputs per lane exist as a variant but were measured slower than four on every layer of the benchmark
   // networks -- 1.91 against 1.32 ms on the 2305 x 256 layer: 98 registers, two CTAs per SM -- and are never picked)
-  int jsel = pick(32, cost, ctas, g.J <= 32 ? 0 : (g.J <= 64 ? 1 : 2));
+  int jsel = pick(32, cost, warps, g.J <= 32 ? 0 : (g.J <= 64 ? 1 : 2));
   int variant = 2;
   if (al8) variant = (g.J <= 64 || jsel < 2) ? 1 : 3;
   if ((opt.walk_layout & 3) != 0) {
