@@ -1053,14 +1053,17 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
       gate.nz = nz_count;
       gate.threshold = (unsigned)(((size_t)g.R * g.J) / 5 * 2);
     }
-    // Few channels: the lanes over the outputs. Up to eight channels always (8 at stride 1, every output with a gradient: 291 ->
-    // 190 us); up to 15 where the dense tile forms products for taps that a stride leaves out, or has fewer tiles than SMs (15
-    // channels at stride 1 on a full GPU: 291 us by the dense tile, 596 so; wider ones lose as well).
+    // Few channels: the lanes over the outputs. Its cost per pixel and channel (the sums over the lanes) wants some taps and outputs
+    // to set against: with up to eight channels always but for small 1x1 windows (65 536 pixels, 1x1, 8 -> 64: 53 us by the dense
+    // tile, 67 so; 3x3, 3 -> 16: 80 and 53); up to 15 where there are 400 of them read 16 bytes at a time (3x3, 12 -> 128: 568 and 322; 15 ->
+    // 64: 292 and 252; but 12 -> 32: 156 and 164), where the dense tile forms products for taps that a stride leaves out, or where
+    // it has fewer tiles than SMs.
     const bool idle = (long)grid.x * grid.y < li.num_sms;
-    const bool wasteful = g.Sh * g.Sw >= 2 || idle;
-    const bool few = dx_few_supported(g) &&
-                     (opt.dx_kernel == 3 || (opt.dx_kernel == 0 && !sparse_ok &&
-                                             (g.C <= 8 || (g.C < 16 && wasteful) || (idle && vec && few_pixels(g, P)))));
+    const long taps_outputs = (long)g.Kh * g.Kw * g.J;
+    const bool few_wins = g.C <= 8 ? idle || taps_outputs > 15 + 9 * g.C
+                          : g.C < 16 ? idle || g.Sh * g.Sw >= 2 || (vec && taps_outputs >= 400)
+                                     : idle && vec && few_pixels(g, P);
+    const bool few = dx_few_supported(g) && (opt.dx_kernel == 3 || (opt.dx_kernel == 0 && !sparse_ok && few_wins));
     if (few) rc = launch_dx_few(g, uv, x, w, out, dx, li, sdx);
     else if (sparse_ok) rc = launch_dx_sparse(g, uv, x, w, out, dx, dx_scratch, gate, li, sdx);
     if (rc == OK && !few && (!sparse_ok || both)) {

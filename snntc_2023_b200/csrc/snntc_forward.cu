@@ -820,8 +820,8 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     const bool in_l1 = (size_t)(g.I + 1) * g.J * sizeof(float) <= (size_t)128 << 10;
     rows = warps_per_sm >= (lanes == 16 ? 48 : (lanes == 8 ? 14 : (in_l1 ? 6 : 10)));
     // (65 536 rows of 576 x 64: 364 us with the pairs walk and its weights in shared memory, 380 so, but 16 384 rows 130 and 113;
-    // 262 144 of 27 x 64: 222, 208)
-    if (g.jout == 64 && g.I >= 128 && g.R >= 32768) rows = false;
+    // 262 144 of 27 x 64: 222, 208, but 59 400 of 64 x 64 75, 83)
+    if (g.jout == 64 && g.I >= 64 && g.R >= 32768) rows = false;
   }
   if ((fparts & 2) && (!ring || pad)) {   // the walk's bound on the weight sums (see walk_tolerance_base)
     const int rows_w = g.I + g.has_bias;
