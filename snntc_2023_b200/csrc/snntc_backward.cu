@@ -38,8 +38,8 @@ constexpr int kTileI = 128;     // dW output tile: 128 fan-in rows x 64 outputs,
 // every block writes a flag of its own (exact_flag[blockIdx.x]) that the consumer combines, which saves the memset in
 // front of the two launches a small dense layer's backward consists of.
 template <bool V4, bool BLOCK_FLAGS>   // V4: n and nx are multiples of 4 and all pointers 16-byte aligned: 16-byte loads and stores
-__global__ void snn_u_kernel(const float* __restrict__ grad, const float* __restrict__ out, float* __restrict__ u,
-                             size_t n, float maxcomp, const float* __restrict__ xin, size_t nx, float maxv,
+__global__ void snn_u_kernel(const float* grad, const float* out, float* __restrict__ u,
+                             size_t n, float maxcomp, const float* xin, size_t nx, float maxv,
                              int* __restrict__ exact_flag, unsigned* __restrict__ nz_count) {
   chain_wait();
   chain_next();
@@ -66,17 +66,17 @@ __global__ void snn_u_kernel(const float* __restrict__ grad, const float* __rest
     const float4* g4 = reinterpret_cast<const float4*>(grad);
     float4* u4 = reinterpret_cast<float4*>(u);
     for (size_t e = t0; e < n / 4; e += stride) {
-      const float4 y = __ldg(y4 + e), g = __ldg(g4 + e), iv = __ldg(i4 + e);
+      const float4 y = ld_plain(y4 + e), g = ld_plain(g4 + e), iv = ld_plain(i4 + e);
       u4[e] = make_float4(one(y.x, g.x, iv.x), one(y.y, g.y, iv.y), one(y.z, g.z, iv.z), one(y.w, g.w, iv.w));
     }
     const float4* x4 = reinterpret_cast<const float4*>(xin);
     for (size_t e = t0; e < nx / 4; e += stride) {
-      const float4 xv = __ldg(x4 + e);
+      const float4 xv = ld_plain(x4 + e);
       scan(xv.x); scan(xv.y); scan(xv.z); scan(xv.w);
     }
   } else {
-    for (size_t e = t0; e < n; e += stride) u[e] = one(__ldg(out + e), __ldg(grad + e), __ldg(out + n + e));
-    for (size_t e = t0; e < nx; e += stride) scan(__ldg(xin + e));
+    for (size_t e = t0; e < n; e += stride) u[e] = one(ld_plain(out + e), ld_plain(grad + e), ld_plain(out + n + e));
+    for (size_t e = t0; e < nx; e += stride) scan(ld_plain(xin + e));
   }
   if constexpr (BLOCK_FLAGS) {
     const int any = __syncthreads_or(odd);
@@ -119,11 +119,11 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 // the arithmetic of tile t and parked in registers, shared memory is double buffered.
 template <bool VEC>   // VEC: J % 4 == 0, tiles are fetched with 16-byte loads
 __global__ void __launch_bounds__(kBwdThreads)
-snn_dx_kernel(const DxGate gate, const Geometry g, const float* __restrict__ uv, const float* __restrict__ x,
-              const float* __restrict__ w, const float* __restrict__ out, float* __restrict__ dx) {
+snn_dx_kernel(const DxGate gate, const Geometry g, const float* uv, const float* x,
+              const float* w, const float* out, float* __restrict__ dx) {
   chain_wait();
   chain_next();
-  if (gate.nz != nullptr && __ldg(gate.nz) <= gate.threshold) return;   // the list-walking kernel takes this call
+  if (gate.nz != nullptr && ld_plain(gate.nz) <= gate.threshold) return;   // the list-walking kernel takes this call
   __shared__ __align__(16) float Ys[2][kTile * kJTP];
   __shared__ __align__(16) float Us[2][kTile * kJTP];
   __shared__ __align__(16) float Ws[2][kTile * kJTP];
@@ -135,7 +135,7 @@ snn_dx_kernel(const DxGate gate, const Geometry g, const float* __restrict__ uv,
   const int taps = g.is_conv ? g.Kh * g.Kw : 1;
   const int njt = (J + kJT - 1) / kJT;
   const int ntiles = taps * njt;
-  const float* __restrict__ yv = out;
+  const float* yv = out;
 
   const int tid = threadIdx.x;
   const int tr = tid >> 4, ti = tid & 15;
@@ -164,7 +164,7 @@ snn_dx_kernel(const DxGate gate, const Geometry g, const float* __restrict__ uv,
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int p = p0 + tr + 16 * a, c = c0 + ti + 16 * b;
-      xr[a][b] = (p < P && c < CH) ? __ldg(x + (size_t)p * CH + c) : CUDART_INF_F;
+      xr[a][b] = (p < P && c < CH) ? ld_plain(x + (size_t)p * CH + c) : CUDART_INF_F;
       acc[a][b] = 0.f;
     }
   __syncthreads();
@@ -202,11 +202,11 @@ snn_dx_kernel(const DxGate gate, const Geometry g, const float* __restrict__ uv,
       float4 u4 = make_float4(0.f, 0.f, 0.f, 0.f), w4 = u4;
       if (orow >= 0 && j < J) {
         const size_t o = (size_t)orow * J + j;
-        y4 = __ldg(reinterpret_cast<const float4*>(yv + o));
-        u4 = __ldg(reinterpret_cast<const float4*>(uv + o));
+        y4 = ld_plain(reinterpret_cast<const float4*>(yv + o));
+        u4 = ld_plain(reinterpret_cast<const float4*>(uv + o));
       }
       const int c = c0 + ld_row;
-      if (c < CH && j < J) w4 = __ldg(reinterpret_cast<const float4*>(w + ((size_t)tap * CH + c) * J + j));
+      if (c < CH && j < J) w4 = ld_plain(reinterpret_cast<const float4*>(w + ((size_t)tap * CH + c) * J + j));
       py[0] = y4.x; py[1] = y4.y; py[2] = y4.z; py[3] = y4.w;
       pu[0] = u4.x; pu[1] = u4.y; pu[2] = u4.z; pu[3] = u4.w;
       pwv[0] = w4.x; pwv[1] = w4.y; pwv[2] = w4.z; pwv[3] = w4.w;
@@ -218,11 +218,11 @@ snn_dx_kernel(const DxGate gate, const Geometry g, const float* __restrict__ uv,
         float y = -CUDART_INF_F, u = 0.f, wv = 0.f;
         if (orow >= 0 && j < J) {
           const size_t o = (size_t)orow * J + j;
-          y = __ldg(yv + o);
-          u = __ldg(uv + o);
+          y = ld_plain(yv + o);
+          u = ld_plain(uv + o);
         }
         const int c = c0 + row;
-        if (c < CH && j < J) wv = __ldg(w + ((size_t)tap * CH + c) * J + j);
+        if (c < CH && j < J) wv = ld_plain(w + ((size_t)tap * CH + c) * J + j);
         py[q] = y; pu[q] = u; pwv[q] = wv;
       }
     }
@@ -303,11 +303,11 @@ constexpr int kYStride = kWideP + 4;
 constexpr int kWStride = kTile + 4;
 
 __global__ void __launch_bounds__(kBwdThreads)
-snn_dx_wide_kernel(const DxGate gate, const Geometry g, const float* __restrict__ uv, const float* __restrict__ x,
-                   const float* __restrict__ w, const float* __restrict__ out, float* __restrict__ dx) {
+snn_dx_wide_kernel(const DxGate gate, const Geometry g, const float* uv, const float* x,
+                   const float* w, const float* out, float* __restrict__ dx) {
   chain_wait();
   chain_next();
-  if (gate.nz != nullptr && __ldg(gate.nz) <= gate.threshold) return;   // the list-walking kernel takes this call
+  if (gate.nz != nullptr && ld_plain(gate.nz) <= gate.threshold) return;   // the list-walking kernel takes this call
   __shared__ __align__(16) float Ys[2][kJT * kYStride];
   __shared__ __align__(16) float Us[2][kJT * kYStride];
   __shared__ __align__(16) float Ws[2][kJT * kWStride];
@@ -319,7 +319,7 @@ snn_dx_wide_kernel(const DxGate gate, const Geometry g, const float* __restrict_
   const int taps = g.is_conv ? g.Kh * g.Kw : 1;
   const int njt = (J + kJT - 1) / kJT;
   const int ntiles = taps * njt;
-  const float* __restrict__ yv = out;
+  const float* yv = out;
 
   const int tid = threadIdx.x;
   const int tp = tid >> 4, tc = tid & 15;
@@ -348,7 +348,7 @@ snn_dx_wide_kernel(const DxGate gate, const Geometry g, const float* __restrict_
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int p = p0 + 8 * tp + a, c = c0 + 4 * tc + b;
-      xr[a][b] = (p < P && c < CH) ? __ldg(x + (size_t)p * CH + c) : CUDART_INF_F;
+      xr[a][b] = (p < P && c < CH) ? ld_plain(x + (size_t)p * CH + c) : CUDART_INF_F;
       acc[a][b] = 0.f;
     }
   __syncthreads();
@@ -384,13 +384,13 @@ snn_dx_wide_kernel(const DxGate gate, const Geometry g, const float* __restrict_
       pu[q] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (orow >= 0 && j < J) {
         const size_t o = (size_t)orow * J + j;
-        py[q] = __ldg(reinterpret_cast<const float4*>(yv + o));
-        pu[q] = __ldg(reinterpret_cast<const float4*>(uv + o));
+        py[q] = ld_plain(reinterpret_cast<const float4*>(yv + o));
+        pu[q] = ld_plain(reinterpret_cast<const float4*>(uv + o));
       }
     }
     pwv = make_float4(0.f, 0.f, 0.f, 0.f);
     const int c = c0 + ld_row;
-    if (c < CH && j < J) pwv = __ldg(reinterpret_cast<const float4*>(w + ((size_t)tap * CH + c) * J + j));
+    if (c < CH && j < J) pwv = ld_plain(reinterpret_cast<const float4*>(w + ((size_t)tap * CH + c) * J + j));
   };
   auto park = [&](int buf) {
 #pragma unroll
@@ -471,9 +471,9 @@ __device__ __forceinline__ float add_sat(float a, float b) {
 
 template <bool VEC>   // VEC: J % 4 == 0, the y/u tiles are fetched with 16-byte loads
 __global__ void __launch_bounds__(kBwdThreads, 3)
-snn_dw_kernel(const Geometry g, const float* __restrict__ uv, const float* __restrict__ x,
-              const float* __restrict__ out, float* __restrict__ partial, int rows_per_split,
-              float scale, const int* __restrict__ exact_flag) {
+snn_dw_kernel(const Geometry g, const float* uv, const float* x,
+              const float* out, float* __restrict__ partial, int rows_per_split,
+              float scale, const int* exact_flag) {
   chain_wait();
   chain_next();
   // -x*s, y*s and -u/s as plain tiles. A two-lane FMA covers two neighbouring output columns of one fan-in row,
@@ -484,8 +484,8 @@ snn_dw_kernel(const Geometry g, const float* __restrict__ uv, const float* __res
 
   const int J = g.J, I = g.I, R = g.R;
   const int Itot = I + g.has_bias;
-  const float* __restrict__ yv = out;
-  const bool fast = scale != 1.0f && __ldg(exact_flag) == 0;
+  const float* yv = out;
+  const bool fast = scale != 1.0f && ld_plain(exact_flag) == 0;
   const float sc = fast ? scale : 1.0f;     // s
   const float nsc = -sc;                    // -s
   const float nusc = fast ? -1.0f / scale : -1.0f;   // -1/s, exact: s is a power of two
@@ -541,11 +541,11 @@ snn_dw_kernel(const Geometry g, const float* __restrict__ uv, const float* __res
       // The loaded value must not be touched here (not even by a select): it is still in flight.
       float xv = (li == I && g.has_bias && r < r_end) ? g.biasvolt : CUDART_INF_F;
       if (!g.is_conv) {
-        if (r < r_end && li < I) xv = __ldg(x + (size_t)r * I + li);
+        if (r < r_end && li < I) xv = ld_plain(x + (size_t)r * I + li);
       } else {
         const int4 ri = rowinfo[ibuf][rl];
         const bool ok = li < I && (unsigned)(ri.y + l_kh) < (unsigned)g.H && (unsigned)(ri.z + l_kw) < (unsigned)g.W;
-        if (ok) xv = __ldg(x + (ptrdiff_t)ri.x + l_off);
+        if (ok) xv = ld_plain(x + (ptrdiff_t)ri.x + l_off);
       }
       px[q] = xv;
     }
@@ -554,8 +554,8 @@ snn_dw_kernel(const Geometry g, const float* __restrict__ uv, const float* __res
       float4 y4 = make_float4(0.f, 0.f, 0.f, 0.f), u4 = y4;
       if (r < r_end && lj < J) {
         const size_t o = (size_t)r * J + lj;
-        y4 = __ldg(reinterpret_cast<const float4*>(yv + o));
-        u4 = __ldg(reinterpret_cast<const float4*>(uv + o));
+        y4 = ld_plain(reinterpret_cast<const float4*>(yv + o));
+        u4 = ld_plain(reinterpret_cast<const float4*>(uv + o));
       }
       py[0] = y4.x; py[1] = y4.y; py[2] = y4.z; py[3] = y4.w;
       pu[0] = u4.x; pu[1] = u4.y; pu[2] = u4.z; pu[3] = u4.w;
@@ -566,8 +566,8 @@ snn_dw_kernel(const Geometry g, const float* __restrict__ uv, const float* __res
         float y = 0.f, u = 0.f;
         if (r < r_end && lj < J) {
           const size_t o = (size_t)r * J + lj;
-          y = __ldg(yv + o);
-          u = __ldg(uv + o);
+          y = ld_plain(yv + o);
+          u = ld_plain(uv + o);
         }
         py[q] = y; pu[q] = u;
       }
@@ -676,9 +676,9 @@ __device__ __forceinline__ float fma_sat(float a, float b, float c) {
 
 template <int JB>
 __global__ void __launch_bounds__(kBwdThreads)
-snn_dw_small_kernel(const Geometry g, const float* __restrict__ uv, const float* __restrict__ x,
-                    const float* __restrict__ out, float* __restrict__ partial, int rows_per_split,
-                    float scale, const int* __restrict__ exact_flag) {
+snn_dw_small_kernel(const Geometry g, const float* uv, const float* x,
+                    const float* out, float* __restrict__ partial, int rows_per_split,
+                    float scale, const int* exact_flag) {
   chain_wait();
   chain_next();
   constexpr int JJ = 8 * JB;              // fan-out
@@ -689,7 +689,7 @@ snn_dw_small_kernel(const Geometry g, const float* __restrict__ uv, const float*
   __shared__ int4 rowinfo[RS];            // .x element offset of the row's top-left pixel, .y its h, .z its w, .w row valid
   const int I = g.I, R = g.R;
   const int Itot = I + g.has_bias;
-  const bool fast = scale != 1.0f && __ldg(exact_flag) == 0;
+  const bool fast = scale != 1.0f && ld_plain(exact_flag) == 0;
   const float sc = fast ? scale : 1.0f;
   const float nsc = -sc;
   const float nusc = fast ? -1.0f / scale : -1.0f;
@@ -718,7 +718,7 @@ snn_dw_small_kernel(const Geometry g, const float* __restrict__ uv, const float*
     for (int n = 0; n < (RS * JJ / 4) / kBwdThreads; ++n) {
       const int e = tid + kBwdThreads * n;
       float4 u = make_float4(0.f, 0.f, 0.f, 0.f), y = u;
-      if (e < valid4) { u = __ldg(u4g + e); y = __ldg(y4g + e); }
+      if (e < valid4) { u = ld_plain(u4g + e); y = ld_plain(y4g + e); }
       reinterpret_cast<float4*>(Us)[e] = u;
       reinterpret_cast<float4*>(Ys)[e] = y;
     }
@@ -748,11 +748,11 @@ snn_dw_small_kernel(const Geometry g, const float* __restrict__ uv, const float*
           xv = g.biasvolt;
         } else if (lane < I) {
           if (!g.is_conv) {
-            xv = __ldg(x + (size_t)r * I + lane);
+            xv = ld_plain(x + (size_t)r * I + lane);
           } else {
             const int4 ri = rowinfo[rl];
             if ((unsigned)(ri.y + l_kh) < (unsigned)g.H && (unsigned)(ri.z + l_kw) < (unsigned)g.W)
-              xv = __ldg(x + (ptrdiff_t)ri.x + l_off);
+              xv = ld_plain(x + (ptrdiff_t)ri.x + l_off);
           }
         }
       }
@@ -814,7 +814,7 @@ static int dw_small_splits(const Geometry& g, const LaunchInfo& li, int* rows_pe
 // Adds the partial planes of every element in a fixed order (four interleaved running sums, then their sum): the
 // same bits every run, and eight independent loads in flight per thread -- a kernel with a few ten thousand
 // threads and hundreds of planes is bound by load latency otherwise.
-__global__ void snn_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, size_t n, int splits) {
+__global__ void snn_dw_reduce_kernel(const float* partial, float* __restrict__ dw, size_t n, int splits) {
   chain_wait();
   chain_next();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -824,11 +824,11 @@ __global__ void snn_dw_reduce_kernel(const float* __restrict__ partial, float* _
     for (; k + 8 <= splits; k += 8) {
       float v[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) v[q] = __ldcs(partial + (size_t)(k + q) * n + e);
+      for (int q = 0; q < 8; ++q) v[q] = ld_stream(partial + (size_t)(k + q) * n + e);
       s0 += v[0]; s1 += v[1]; s2 += v[2]; s3 += v[3];
       s0 += v[4]; s1 += v[5]; s2 += v[6]; s3 += v[7];
     }
-    for (; k < splits; ++k) s0 += __ldcs(partial + (size_t)k * n + e);
+    for (; k < splits; ++k) s0 += ld_stream(partial + (size_t)k * n + e);
     dw[e] = (s0 + s1) + (s2 + s3);
   }
 }
@@ -837,7 +837,7 @@ __global__ void snn_dw_reduce_kernel(const float* __restrict__ partial, float* _
 // each (26 052 elements of a 5x5 20 -> 52 layer: dW 54 -> 47 us; from 300 000 elements on it is a little slower). Lanes c, c + 8,
 // c + 16 and c + 24 of a warp hold one element, so a load touches whole 32-byte sectors of four planes.
 __global__ void __launch_bounds__(256)
-snn_dw_reduce_shared_kernel(const float* __restrict__ partial, float* __restrict__ dw, size_t n, int splits) {
+snn_dw_reduce_shared_kernel(const float* partial, float* __restrict__ dw, size_t n, int splits) {
   chain_wait();
   chain_next();
   const int lane = threadIdx.x & 31, chain = lane >> 3;
@@ -852,16 +852,16 @@ snn_dw_reduce_shared_kernel(const float* __restrict__ partial, float* __restrict
       for (; k + 4 <= rounds; k += 4) {
         float v[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = __ldcs(p + (size_t)(8 * k + 4 * q) * n);
+        for (int q = 0; q < 8; ++q) v[q] = ld_stream(p + (size_t)(8 * k + 4 * q) * n);
 #pragma unroll
         for (int q = 0; q < 8; ++q) s += v[q];
       }
       for (; k < rounds; ++k) {
-        s += __ldcs(p + (size_t)(8 * k) * n);
-        s += __ldcs(p + (size_t)(8 * k + 4) * n);
+        s += ld_stream(p + (size_t)(8 * k) * n);
+        s += ld_stream(p + (size_t)(8 * k + 4) * n);
       }
       if (chain == 0)                      // the first one takes the remainder
-        for (int q = 8 * rounds; q < splits; ++q) s += __ldcs(partial + (size_t)q * n + e);
+        for (int q = 8 * rounds; q < splits; ++q) s += ld_stream(partial + (size_t)q * n + e);
     }
     s += __shfl_xor_sync(0xffffffffu, s, 8);      // s0 + s1, s2 + s3
     s += __shfl_xor_sync(0xffffffffu, s, 16);

@@ -182,7 +182,7 @@ snn_dense_bwd_kernel(const DenseArgs a, const DensePlan p) {
       const bool rok = r0 + m + 8 * k < R;
 #pragma unroll
       for (int b = 0; b < NL; ++b) {
-        xr[k][b] = (rok && i0 + n + 4 * b < I) ? __ldg(gx + 4 * b) : CUDART_INF_F;
+        xr[k][b] = (rok && i0 + n + 4 * b < I) ? ld_plain(gx + 4 * b) : CUDART_INF_F;
         acc[k][b] = 0.f;
       }
     }
@@ -273,7 +273,7 @@ snn_dense_bwd_kernel(const DenseArgs a, const DensePlan p) {
   if (c0 < c1) issue(c0, 0);
   if (c0 + 1 < c1) issue(c0 + 1, 1);
   int raised = 0;
-  for (int k = threadIdx.x; k < a.nflags; k += kThreads) raised |= __ldg(a.flags + k);
+  for (int k = threadIdx.x; k < a.nflags; k += kThreads) raised |= ld_plain(a.flags + k);
   const bool fast = !__syncthreads_or(raised) && a.scale != 1.0f;
   const float sc = fast ? a.scale : 1.0f, nsc = -sc, nusc = fast ? -1.0f / a.scale : -1.0f;   // exact: powers of two
   const int m = 8 * (lane >> 3), n = 4 * (lane & 7);

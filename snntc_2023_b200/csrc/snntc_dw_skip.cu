@@ -72,9 +72,9 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // VEC: C and J multiples of four, 16-byte aligned tensors; a lane holds QL quadruples of fan-in rows, else QL pairs
 template <int QL, bool VEC, int NW>
 __global__ void __launch_bounds__(32 * NW, 16 / NW)
-snn_dw_skip_kernel(const Geometry g, const float* __restrict__ uv, const float* __restrict__ x,
-                   const float* __restrict__ out, float* __restrict__ partial, int rows_per_split,
-                   float scale, const int* __restrict__ exact_flag) {
+snn_dw_skip_kernel(const Geometry g, const float* uv, const float* x,
+                   const float* out, float* __restrict__ partial, int rows_per_split,
+                   float scale, const int* exact_flag) {
   chain_wait();
   chain_next();
   constexpr int kThreads = 32 * NW, kJT = 4 * NW;   // output channels per CTA, 4 per warp
@@ -90,7 +90,7 @@ snn_dw_skip_kernel(const Geometry g, const float* __restrict__ uv, const float* 
 
   const int J = g.J, I = g.I, R = g.R;
   const int Itot = I + g.has_bias;
-  const bool fast = scale != 1.0f && __ldg(exact_flag) == 0;
+  const bool fast = scale != 1.0f && ld_plain(exact_flag) == 0;
   const float sc = fast ? scale : 1.0f;                 // s
   const float nsc = -sc;
   const float nusc = fast ? -1.0f / scale : -1.0f;      // -1/s, exact: s is a power of two

@@ -80,7 +80,7 @@ template <int QL, bool C256, int NW>
 __global__ void __launch_bounds__(32 * NW, 16 / NW)
 snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                   const __grid_constant__ CUtensorMap map_u, const Geometry g, float* __restrict__ partial,
-                  int stages_per_split, float scale, const int* __restrict__ exact_flag, int taps_per_tile,
+                  int stages_per_split, float scale, const int* exact_flag, int taps_per_tile,
                   int wseg_log2, int depth) {
   constexpr int kJT = 4 * NW;                                      // output channels per CTA, 4 per warp
   chain_wait();
@@ -100,7 +100,7 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   float* Ys = Xs + depth * xfloats;                                // [depth][kRS][kJT]
   float* Us = Ys + depth * kRS * kJT;                              // [depth][kRS][kJT]
 
-  const bool fast = scale != 1.0f && __ldg(exact_flag) == 0;
+  const bool fast = scale != 1.0f && ld_plain(exact_flag) == 0;
   const float sc = fast ? scale : 1.0f;                 // s
   const float nsc = -sc;
   const float nusc = fast ? -1.0f / scale : -1.0f;      // -1/s, exact: s is a power of two

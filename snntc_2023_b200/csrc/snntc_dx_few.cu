@@ -31,8 +31,8 @@ __device__ __forceinline__ void masked_fma(float& acc, float x, float y, float u
 // `lanes` = 4, 8, 16 or 32 of them take a field, 32 / lanes fields at once.
 template <int CT, bool V4>
 __global__ void __launch_bounds__(kThreads)
-snn_dx_few_kernel(const Geometry g, const float* __restrict__ uv, const float* __restrict__ x, const float* __restrict__ w,
-                  const float* __restrict__ y, float* __restrict__ dx, int lanes) {
+snn_dx_few_kernel(const Geometry g, const float* uv, const float* x, const float* w,
+                  const float* y, float* __restrict__ dx, int lanes) {
   chain_wait();
   chain_next();
   const int lane = threadIdx.x & 31;
@@ -46,7 +46,7 @@ snn_dx_few_kernel(const Geometry g, const float* __restrict__ uv, const float* _
     float xr[CT], acc[CT];
 #pragma unroll
     for (int c = 0; c < CT; ++c) {
-      xr[c] = c0 + c < C ? __ldg(x + (size_t)p * C + c0 + c) : 0.f;
+      xr[c] = c0 + c < C ? ld_plain(x + (size_t)p * C + c0 + c) : 0.f;
       acc[c] = 0.f;
     }
     // fields nh with nh*Sh <= ph <= nh*Sh + Kh - 1
@@ -63,12 +63,12 @@ snn_dx_few_kernel(const Geometry g, const float* __restrict__ uv, const float* _
         const float* wt = w + ((size_t)(kh * g.Kw + kw) * C + c0) * J;
 #pragma unroll 2
         for (int j = 4 * (lane & (lanes - 1)); j < J; j += 4 * lanes) {
-          const float4 yy = __ldg(reinterpret_cast<const float4*>(y + o + j));
-          const float4 u = __ldg(reinterpret_cast<const float4*>(uv + o + j));
+          const float4 yy = ld_plain(reinterpret_cast<const float4*>(y + o + j));
+          const float4 u = ld_plain(reinterpret_cast<const float4*>(uv + o + j));
 #pragma unroll
           for (int c = 0; c < CT; ++c) {
             if (c0 + c >= C) break;
-            const float4 wv = __ldg(reinterpret_cast<const float4*>(wt + (size_t)c * J + j));
+            const float4 wv = ld_plain(reinterpret_cast<const float4*>(wt + (size_t)c * J + j));
             masked_fma(acc[c], xr[c], yy.x, u.x, wv.x);
             masked_fma(acc[c], xr[c], yy.y, u.y, wv.y);
             masked_fma(acc[c], xr[c], yy.z, u.z, wv.z);
@@ -85,10 +85,10 @@ snn_dx_few_kernel(const Geometry g, const float* __restrict__ uv, const float* _
           const float* wt = w + ((size_t)(kh * g.Kw + kw) * C + c0) * J;
 #pragma unroll 2
           for (int j = lane; j < J; j += 32) {
-            const float yy = __ldg(y + o + j), u = __ldg(uv + o + j);
+            const float yy = ld_plain(y + o + j), u = ld_plain(uv + o + j);
 #pragma unroll
             for (int c = 0; c < CT; ++c)
-              if (c0 + c < C) masked_fma(acc[c], xr[c], yy, u, __ldg(wt + (size_t)c * J + j));
+              if (c0 + c < C) masked_fma(acc[c], xr[c], yy, u, ld_plain(wt + (size_t)c * J + j));
           }
         }
       }

@@ -30,11 +30,11 @@ constexpr int kThreads = 256;
 // One warp per receptive field r: list[r*J ..] receives (y bits, u bits, j, 0) for every output with u != 0, in
 // ascending j; count[r] their number.
 __global__ void __launch_bounds__(kThreads)
-snn_act_lists_kernel(const float* __restrict__ out, const float* __restrict__ uv, int R, int J,
+snn_act_lists_kernel(const float* out, const float* uv, int R, int J,
                      uint4* __restrict__ list, int* __restrict__ count, const DxGate gate) {
   chain_wait();
   chain_next();
-  if (gate.nz != nullptr && __ldg(gate.nz) > gate.threshold) return;   // the dense kernel takes this call
+  if (gate.nz != nullptr && ld_plain(gate.nz) > gate.threshold) return;   // the dense kernel takes this call
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < R; r += warps) {
@@ -45,7 +45,7 @@ snn_act_lists_kernel(const float* __restrict__ out, const float* __restrict__ uv
     for (int j0 = 0; j0 < J; j0 += 32) {
       const int j = j0 + lane;
       float y = 0.f, u = 0.f;
-      if (j < J) { y = __ldg(yr + j); u = __ldg(ur + j); }
+      if (j < J) { y = ld_plain(yr + j); u = ld_plain(ur + j); }
       const bool keep = u != 0.f;
       const unsigned m = __ballot_sync(0xffffffffu, keep);
       if (keep) dst[n + __popc(m & ((1u << lane) - 1u))] = make_uint4(__float_as_uint(y), __float_as_uint(u), (unsigned)j, 0u);
@@ -56,11 +56,11 @@ snn_act_lists_kernel(const float* __restrict__ out, const float* __restrict__ uv
 }
 
 // Wt[(tap*J + j)*C + c] = W[(tap*C + c)*J + j]  (the bias row is not part of dX)
-__global__ void snn_weight_transpose_kernel(const float* __restrict__ w, float* __restrict__ wt, int taps, int C, int J,
+__global__ void snn_weight_transpose_kernel(const float* w, float* __restrict__ wt, int taps, int C, int J,
                                             const DxGate gate) {
   chain_wait();
   chain_next();
-  if (gate.nz != nullptr && __ldg(gate.nz) > gate.threshold) return;
+  if (gate.nz != nullptr && ld_plain(gate.nz) > gate.threshold) return;
   const size_t n = (size_t)taps * C * J;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
@@ -68,7 +68,7 @@ __global__ void snn_weight_transpose_kernel(const float* __restrict__ w, float* 
     const size_t tj = e / C;
     const int j = (int)(tj % J);
     const int tap = (int)(tj / J);
-    wt[e] = __ldg(w + ((size_t)tap * C + c) * J + j);
+    wt[e] = ld_plain(w + ((size_t)tap * C + c) * J + j);
   }
 }
 
@@ -90,12 +90,12 @@ constexpr int kStage = 256;   // staged list entries per warp and round
 
 template <int CPL, int LPP>
 __global__ void __launch_bounds__(kThreads)
-snn_dx_sparse_kernel(const Geometry g, const float* __restrict__ x, const float* __restrict__ wt,
-                     const uint4* __restrict__ list, const int* __restrict__ count, float* __restrict__ dx,
+snn_dx_sparse_kernel(const Geometry g, const float* x, const float* wt,
+                     const uint4* list, const int* count, float* __restrict__ dx,
                      const DxGate gate) {
   chain_wait();
   chain_next();
-  if (gate.nz != nullptr && __ldg(gate.nz) > gate.threshold) return;
+  if (gate.nz != nullptr && ld_plain(gate.nz) > gate.threshold) return;
   constexpr int PPW = 32 / LPP;                       // pixels per warp
   constexpr int SB = kStage / PPW;                    // staged entries per pixel and round
   constexpr int UN = CPL <= 4 ? 4 : 2;                // entries whose weight reads are in flight together
@@ -121,7 +121,7 @@ snn_dx_sparse_kernel(const Geometry g, const float* __restrict__ x, const float*
 #pragma unroll
       for (int k4 = 0; k4 < CPL; k4 += 4) {
         if (c0 + k4 < C) {
-          const float4 v = __ldg(reinterpret_cast<const float4*>(x + (size_t)p * C + c0 + k4));
+          const float4 v = ld_plain(reinterpret_cast<const float4*>(x + (size_t)p * C + c0 + k4));
           xr[k4] = v.x; xr[k4 + 1] = v.y; xr[k4 + 2] = v.z; xr[k4 + 3] = v.w;
         }
       }
@@ -153,13 +153,13 @@ snn_dx_sparse_kernel(const Geometry g, const float* __restrict__ x, const float*
         const uint4* src = list;
         if (ok) {
           const int r = (pb * g.Nh + nh) * g.Nw + nw;
-          n = __ldg(count + r);
+          n = ld_plain(count + r);
           src = list + (size_t)r * J;
         }
         const int take = min(n - e0, SB - staged);
         const unsigned tapoff = (unsigned)tap * (unsigned)J;
         for (int e = gl; e < take; e += LPP) {
-          uint4 en = __ldg(src + e0 + e);
+          uint4 en = ld_plain(src + e0 + e);
           en.z = (tapoff + en.z) * (unsigned)C;
           stage[staged + e] = en;
         }
@@ -186,7 +186,7 @@ snn_dx_sparse_kernel(const Geometry g, const float* __restrict__ x, const float*
             const float* wrow = wlane + en[q].z;
 #pragma unroll
             for (int k4 = 0; k4 < CPL; k4 += 4)
-              w4[q][k4 / 4] = (c0 + k4 < C) ? __ldg(reinterpret_cast<const float4*>(wrow + k4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+              w4[q][k4 / 4] = (c0 + k4 < C) ? ld_plain(reinterpret_cast<const float4*>(wrow + k4)) : make_float4(0.f, 0.f, 0.f, 0.f);
           }
 #pragma unroll
           for (int q = 0; q < UN; ++q) {

@@ -55,7 +55,7 @@ __device__ __forceinline__ int imin3(int a, int b, int c) { return min(min(a, b)
 // to be met by chance about once in 10^5 output steps. Compared as integers: tol >= +0, negative q are negative.
 __device__ __forceinline__ float walk_tolerance_base(const Geometry& g) {
   const int lane = threadIdx.x & 31;
-  float b = lane < g.wbound_n ? __ldg(g.wbound + lane) : 0.f;
+  float b = lane < g.wbound_n ? ld_plain(g.wbound + lane) : 0.f;
 #pragma unroll
   for (int d = 16; d >= 1; d >>= 1) b += __shfl_xor_sync(0xffffffffu, b, d);
   return 4.76837158203125e-7f * (fabsf(g.theta) + b) * 1.0001f;   // (a little slack for the rounding of the sums)
@@ -68,7 +68,7 @@ __device__ __forceinline__ float walk_tolerance_base(const Geometry& g) {
 constexpr int kBoundClusters = 32;
 constexpr int kBoundCtas = 8 * kBoundClusters;
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256)
-snn_wbound_kernel(const float* __restrict__ w, int rows, int J, int rows_per_cta, float* __restrict__ bound,
+snn_wbound_kernel(const float* w, int rows, int J, int rows_per_cta, float* __restrict__ bound,
                   float* __restrict__ padded, int Jp) {
   chain_wait();
   chain_next();
@@ -83,12 +83,12 @@ snn_wbound_kernel(const float* __restrict__ w, int rows, int J, int rows_per_cta
     if (v4) {
 #pragma unroll 4
       for (int j = 4 * lane; j < J; j += 128) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(wr + j));
+        const float4 v = ld_plain(reinterpret_cast<const float4*>(wr + j));
         m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
       }
     } else {
       for (int j = lane; j < Jp; j += 32) {
-        const float v = j < J ? __ldg(wr + j) : 0.f;
+        const float v = j < J ? ld_plain(wr + j) : 0.f;
         m = fmaxf(m, fabsf(v));
         if (padded != nullptr) padded[(size_t)r * Jp + j] = v;
       }
@@ -129,8 +129,8 @@ snn_wbound_kernel(const float* __restrict__ w, int rows, int J, int rows_per_cta
 // reference fires on the way back up through zero -- makes the lane "sticky": the exact tests run again at
 // the next step whatever q is, until no live output of the lane is in that state any more.
 template <int JPT, int CH, bool FULL, bool VECW, bool STAGE>
-__device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* __restrict__ ents, int nvalid,
-                                         const float* __restrict__ w, int jbase, int lane,
+__device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ents, int nvalid,
+                                         const float* w, int jbase, int lane,
                                          float* __restrict__ y_row, float* __restrict__ inv_row,
                                          WalkEntry* __restrict__ sbuf) {
   const int J = g.J;
@@ -148,7 +148,7 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* __r
     wsum[m] = -g.theta;
     ysum[m] = 0.f;
     if (g.has_bias) {  // the bias input (value biasvolt, weight row I) is always consumed first
-      const float wb = __ldg(w + (size_t)g.I * J + jl[m]);
+      const float wb = ld_plain(w + (size_t)g.I * J + jl[m]);
       wsum[m] += wb;
       ysum[m] = g.biasvolt * wb;
     }
@@ -172,18 +172,18 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* __r
     const float* wrow = wl + eoff;
     if constexpr (VECW && JPT == 8) {
       const float4* p4 = reinterpret_cast<const float4*>(wbase + (size_t)(eoff + lane_off) * 4u);
-      const float4 v = __ldg(p4), v2 = __ldg(p4 + 1);
+      const float4 v = ld_plain(p4), v2 = ld_plain(p4 + 1);
       wv[0] = v.x; wv[1] = v.y; wv[2] = v.z; wv[3] = v.w;
       wv[4] = v2.x; wv[5] = v2.y; wv[6] = v2.z; wv[7] = v2.w;
     } else if constexpr (VECW && JPT == 4) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(wbase + (size_t)(eoff + lane_off) * 4u));
+      const float4 v = ld_plain(reinterpret_cast<const float4*>(wbase + (size_t)(eoff + lane_off) * 4u));
       wv[0] = v.x; wv[1] = v.y; wv[2] = v.z; wv[3] = v.w;
     } else if constexpr (VECW && JPT == 2) {
-      const float2 v = __ldg(reinterpret_cast<const float2*>(wbase + (size_t)(eoff + lane_off) * 4u));
+      const float2 v = ld_plain(reinterpret_cast<const float2*>(wbase + (size_t)(eoff + lane_off) * 4u));
       wv[0] = v.x; wv[1] = v.y;
     } else {
 #pragma unroll
-      for (int m = 0; m < JPT; ++m) wv[m] = FULL ? __ldg(wrow + 32 * m) : __ldg(wrow + jl[m]);
+      for (int m = 0; m < JPT; ++m) wv[m] = FULL ? ld_plain(wrow + 32 * m) : ld_plain(wrow + jl[m]);
     }
   };
 
@@ -264,12 +264,12 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* __r
     // whole block ahead, instead of one L2 round trip in front of every chunk; a step then reads its entry with
     // one broadcast shared-memory load. Two buffers of 32 entries per warp.
     WalkEntry pre = make_uint2(0u, 0u);
-    if (lane < nvalid) pre = __ldcg(ents + lane);
+    if (lane < nvalid) pre = ld_l2(ents + lane);
     int b = 0;
     for (int base = 0; base < nvalid && !all_done; base += 32, b ^= 32) {
       sbuf[b + lane] = pre;
       __syncwarp();
-      if (base + 32 + lane < nvalid) pre = __ldcg(ents + base + 32 + lane);
+      if (base + 32 + lane < nvalid) pre = ld_l2(ents + base + 32 + lane);
       const int nb = min(32, nvalid - base);
       const WalkEntry* cur = sbuf + b;
       auto fetch2 = [&](int i) { return *reinterpret_cast<const uint4*>(cur + i); };
@@ -283,11 +283,11 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* __r
     int k = 0;
     for (; k + CH <= nvalid && !all_done; k += CH) {
       // list entries bypass L1: it is kept for the weights
-      chunk([&](int i) { return __ldcg(reinterpret_cast<const uint4*>(ents + i)); }, k);
+      chunk([&](int i) { return ld_l2(reinterpret_cast<const uint4*>(ents + i)); }, k);
       check_done();
     }
     if (!all_done)
-      for (; k < nvalid; ++k) single(__ldcg(ents + k));
+      for (; k < nvalid; ++k) single(ld_l2(ents + k));
   }
 
 #pragma unroll
@@ -329,8 +329,8 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* __r
 // list entry's element offset (source index * J) times wmul is the row's byte offset in the slice -- one integer
 // multiply-add on the FMA pipe per weight read. JP == 1 only.
 template <int JP, int CH, bool FULL, bool STAGE, bool WS = false>
-__device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* __restrict__ ents, int nvalid,
-                                          const float* __restrict__ w, int jbase, int lane,
+__device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* ents, int nvalid,
+                                          const float* w, int jbase, int lane,
                                           float* __restrict__ y_row, float* __restrict__ inv_row,
                                           WalkEntry* __restrict__ sbuf, unsigned ws_lane = 0u, unsigned wmul = 0u) {
   static_assert(!WS || JP == 1, "weights in shared memory: one output pair per lane");
@@ -347,7 +347,7 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* __
     jl[m] = jok[m] ? j : J - 2;
     float n0 = g.theta, n1 = g.theta, y0 = 0.f, y1 = 0.f;
     if (g.has_bias) {  // the bias input (value biasvolt, weight row I) is always consumed first
-      const float2 wb = __ldg(reinterpret_cast<const float2*>(w + (size_t)g.I * J + jl[m]));
+      const float2 wb = ld_plain(reinterpret_cast<const float2*>(w + (size_t)g.I * J + jl[m]));
       n0 -= wb.x; n1 -= wb.y;
       y0 = g.biasvolt * wb.x; y1 = g.biasvolt * wb.y;
     }
@@ -408,7 +408,7 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* __
   };
   const unsigned lane_off = (unsigned)jl[0];   // element offset of this lane's first pair within a weight row
   auto load_pair = [&](const float* wrow, int m) -> uint64_t {
-    return __ldg(reinterpret_cast<const unsigned long long*>(FULL ? wrow + 64 * m : wrow + jl[m]));
+    return ld_plain(reinterpret_cast<const unsigned long long*>(FULL ? wrow + 64 * m : wrow + jl[m]));
   };
 
   bool all_done = false;
@@ -418,7 +418,7 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* __
     } else if constexpr (JP == 1) {
       // one pair per lane: a 32-bit element offset from the (uniform) weight base measured faster than a
       // 64-bit per-lane pointer plus the entry's offset
-      wv[0] = __ldg(reinterpret_cast<const unsigned long long*>(
+      wv[0] = ld_plain(reinterpret_cast<const unsigned long long*>(
           reinterpret_cast<const char*>(w) + (size_t)(eoff + lane_off) * 4u));
     } else {
       const float* wrow = wl + eoff;
@@ -464,12 +464,12 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* __
   };
   if constexpr (STAGE) {   // the list through shared memory, 32 entries at a time, read a block ahead (see walk_row)
     WalkEntry pre = make_uint2(0u, 0u);
-    if (lane < nvalid) pre = __ldcg(ents + lane);
+    if (lane < nvalid) pre = ld_l2(ents + lane);
     int b = 0;
     for (int base = 0; base < nvalid && !all_done; base += 32, b ^= 32) {
       sbuf[b + lane] = pre;
       __syncwarp();
-      if (base + 32 + lane < nvalid) pre = __ldcg(ents + base + 32 + lane);
+      if (base + 32 + lane < nvalid) pre = ld_l2(ents + base + 32 + lane);
       const int nb = min(32, nvalid - base);
       const WalkEntry* cur = sbuf + b;
       auto fetch2 = [&](int i) { return *reinterpret_cast<const uint4*>(cur + i); };
@@ -483,11 +483,11 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* __
     int k = 0;
     for (; k + CH <= nvalid && !all_done; k += CH) {
       // list entries bypass L1: it is kept for the weights
-      chunk([&](int i) { return __ldcg(reinterpret_cast<const uint4*>(ents + i)); }, k);
+      chunk([&](int i) { return ld_l2(reinterpret_cast<const uint4*>(ents + i)); }, k);
       check_done();
     }
     if (!all_done)
-      for (; k < nvalid; ++k) single(__ldcg(ents + k));
+      for (; k < nvalid; ++k) single(ld_l2(ents + k));
   }
 
 #pragma unroll
@@ -524,8 +524,8 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* __
 // Walk kernel: every warp takes (row, block of 32*JPT outputs) items, adjacent warps share a row.
 template <int JPT, bool VECW, bool STAGE>
 __global__ void __launch_bounds__(kFwdThreads, JPT <= 4 ? 1024 / kFwdThreads : 1)   // up to four outputs per lane: 64 registers, 32 warps per SM
-snn_walk_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const int* __restrict__ nvalid_g, int istride,
-                const float* __restrict__ w, float* __restrict__ out, int row_begin, int row_end) {
+snn_walk_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, int istride,
+                const float* w, float* __restrict__ out, int row_begin, int row_end) {
   chain_wait();
   chain_next();
   __shared__ __align__(16) WalkEntry stage[STAGE ? kFwdWarps * 64 : 1];   // two blocks of 32 list entries per warp
@@ -543,7 +543,7 @@ snn_walk_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const in
     const int rl = (int)(item / jchunks), jc = (int)(item - (long)rl * jchunks);
     const int r = row_begin + rl;
     const WalkEntry* krow = keys_g + (size_t)r * istride;
-    const int n = __shfl_sync(0xffffffffu, __ldg(nvalid_g + r), 0);
+    const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     if (full_j)
       walk_row<JPT, CH, true, VECW, STAGE>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * g.jout, (inv_out ? inv_out + (size_t)r * g.jout : nullptr), sbuf);
     else
@@ -555,8 +555,8 @@ snn_walk_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const in
 // The same items with the outputs of a lane held in pairs (walk_row2): a warp covers 64*JP outputs.
 template <int JP, bool STAGE>
 __global__ void __launch_bounds__(kFwdThreads, 1024 / kFwdThreads)
-snn_walk2_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const int* __restrict__ nvalid_g, int istride,
-                 const float* __restrict__ w, float* __restrict__ out, int row_begin, int row_end) {
+snn_walk2_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, int istride,
+                 const float* w, float* __restrict__ out, int row_begin, int row_end) {
   chain_wait();
   chain_next();
   __shared__ __align__(16) WalkEntry stage[STAGE ? kFwdWarps * 64 : 1];   // two blocks of 32 list entries per warp
@@ -573,7 +573,7 @@ snn_walk2_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const i
     const int rl = (int)(item / jchunks), jc = (int)(item - (long)rl * jchunks);
     const int r = row_begin + rl;
     const WalkEntry* krow = keys_g + (size_t)r * istride;
-    const int n = __shfl_sync(0xffffffffu, __ldg(nvalid_g + r), 0);
+    const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     if (full_j)
       walk_row2<JP, (JP >= 2 ? 4 : 8), true, STAGE>(g, krow, n, w, jc * 64 * JP, lane, y_out + (size_t)r * J, (inv_out ? inv_out + (size_t)r * J : nullptr), sbuf);
     else
@@ -597,8 +597,8 @@ __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)_
 
 template <bool STAGE>
 __global__ void __launch_bounds__(kSmemwThreads, 1)
-snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, const int* __restrict__ nvalid_g,
-                       int istride, const float* __restrict__ w, float* __restrict__ out, int row_begin, int row_end,
+snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g,
+                       int istride, const float* w, float* __restrict__ out, int row_begin, int row_end,
                        unsigned wmul) {
   chain_wait();
   chain_next();
@@ -656,7 +656,7 @@ snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* __restrict__ keys_g, c
   for (long rl = (long)cta * kSmemwWarps + warp; rl < row_end - row_begin; rl += (long)ctas * kSmemwWarps) {
     const int r = row_begin + (int)rl;
     const WalkEntry* krow = keys_g + (size_t)r * istride;
-    const int n = __shfl_sync(0xffffffffu, __ldg(nvalid_g + r), 0);
+    const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     float* yr = y_out + (size_t)r * J;
     float* ir = inv_out ? inv_out + (size_t)r * J : nullptr;
     if (staged) walk_row2<1, 8, true, STAGE, true>(g, krow, n, w, j0, lane, yr, ir, sbuf, ws_lane, wmul);

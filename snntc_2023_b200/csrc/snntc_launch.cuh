@@ -1,6 +1,7 @@
 // How the kernels are launched: programmatic dependent launch, clusters, and the shared-memory attribute set once.
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 #include <atomic>
 #include <mutex>
@@ -18,6 +19,33 @@ namespace snntc {
 constexpr long kChainThreads = 148L * 128;
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// What a chained kernel reads, the kernel in front of it may still be writing while this one is already on the SMs. Loads through
+// the read-only path (__ldg, or any load through a const __restrict__ kernel parameter, which the compiler turns into one) are
+// defined for memory that nobody writes during the WHOLE life of a kernel: the compiler may move them in front of chain_wait(),
+// and the path need not see the other kernel's stores. So a chained kernel takes none of them: its read pointers carry no
+// __restrict__ (the pointers it writes through do, which is all that overlapping the loads needs), and it reads with
+//   ld_plain    an ordinary load, ordered behind chain_wait() by its memory clobber
+//   ld_l2       past L1: data that is read once and should leave L1 to the weights
+//   ld_stream   evict first: data that nobody reads again
+template <typename T>
+__device__ __forceinline__ T ld_plain(const T* p) { return *p; }
+__device__ __forceinline__ uint2 ld_l2(const uint2* p) {
+  uint2 v;
+  asm volatile("ld.global.cg.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_l2(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+__device__ __forceinline__ float ld_stream(const float* p) {
+  float v;
+  asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
 
 template <typename... Params, typename... Args>
 cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, unsigned cluster,

@@ -108,7 +108,7 @@ __device__ __forceinline__ void sort_and_write_run(u64 (&v)[EPL], int n, int lan
 // as (float bits, c*J) in ascending order followed by a terminator; counts[p] their number.
 template <int EPL>
 __global__ void __launch_bounds__(kPixelWarps * 32)
-snn_pixel_runs_kernel(const float* __restrict__ x, int npix, int C, int J, float maxcomp,
+snn_pixel_runs_kernel(const float* x, int npix, int C, int J, float maxcomp,
                       WalkEntry* __restrict__ runs, int* __restrict__ counts, int stride) {
   chain_wait();
   chain_next();
@@ -123,7 +123,7 @@ snn_pixel_runs_kernel(const float* __restrict__ x, int npix, int C, int J, float
     for (int m = 0; m < EPL; ++m) {
       const int c = m * 32 + lane;                    // coalesced: the network does not care where a key starts
       float val = CUDART_INF_F;
-      if (c < C) val = __ldg(xp + c);
+      if (c < C) val = ld_plain(xp + c);
       const bool keep = val <= maxcomp;               // false for NaN and for inputs that never spike
       v[m] = keep ? (((u64)float_to_sortable(val) << 32) | (unsigned)c) : ~0ull;
       n += __popc(__ballot_sync(0xffffffffu, keep));
@@ -143,7 +143,7 @@ snn_pixel_runs_kernel(const float* __restrict__ x, int npix, int C, int J, float
 // as the list the walk reads. A dense row is its own table.
 template <int EPL>
 __global__ void __launch_bounds__(kPixelWarps * 32)
-snn_small_rows_kernel(const Geometry g, const float* __restrict__ x, WalkEntry* __restrict__ lists,
+snn_small_rows_kernel(const Geometry g, const float* x, WalkEntry* __restrict__ lists,
                       int* __restrict__ nvalid, int istride) {
   chain_wait();
   chain_next();
@@ -194,7 +194,7 @@ snn_small_rows_kernel(const Geometry g, const float* __restrict__ x, WalkEntry* 
         ok = ok && (unsigned)(h0 + (int)(khw >> 8)) < (unsigned)g.H && (unsigned)(w0 + (int)(khw & 255u)) < (unsigned)g.W;
       }
       float val = CUDART_INF_F;
-      if (ok) val = __ldg(xr + o);
+      if (ok) val = ld_plain(xr + o);
       const bool keep = val <= maxcomp;               // false for NaN, padding and inputs that never spike
       v[m] = keep ? (((u64)float_to_sortable(val) << 32) | (unsigned)i) : ~0ull;
       n += __popc(__ballot_sync(0xffffffffu, keep));
@@ -259,7 +259,7 @@ __device__ __forceinline__ void merge_piece(const WalkEntry* const* run, const i
 // (b, h, nw - pad_left + kw), kw < Kw, columns outside the image being empty. Entry offsets gain kw*C*J.
 template <bool SPLIT>
 __global__ void __launch_bounds__(kListThreads)
-snn_row_runs_kernel(const Geometry g, const WalkEntry* __restrict__ pix, const int* __restrict__ pix_n, int pix_stride,
+snn_row_runs_kernel(const Geometry g, const WalkEntry* pix, const int* pix_n, int pix_stride,
                     WalkEntry* __restrict__ rows, int* __restrict__ rows_n, int row_stride, int parts_log2) {
   chain_wait();
   chain_next();
@@ -281,7 +281,7 @@ snn_row_runs_kernel(const Geometry g, const WalkEntry* __restrict__ pix, const i
     if (valid && kw < g.Kw && wc >= 0 && wc < g.W) {
       const int p = bh * g.W + wc;
       run[kw] = pix + (size_t)p * pix_stride;
-      n[kw] = __ldg(pix_n + p);
+      n[kw] = ld_plain(pix_n + p);
     }
     off[kw] = (uint32_t)kw * (uint32_t)g.C * (uint32_t)g.J;
   }
@@ -305,7 +305,7 @@ snn_row_runs_kernel(const Geometry g, const WalkEntry* __restrict__ pix, const i
 // gain kh*Kw*C*J.
 template <bool SPLIT>
 __global__ void __launch_bounds__(kListThreads)
-snn_field_lists_kernel(const Geometry g, const WalkEntry* __restrict__ rows, const int* __restrict__ rows_n,
+snn_field_lists_kernel(const Geometry g, const WalkEntry* rows, const int* rows_n,
                        int row_stride, WalkEntry* __restrict__ lists, int* __restrict__ nvalid, int istride,
                        int parts_log2) {
   chain_wait();
@@ -329,7 +329,7 @@ snn_field_lists_kernel(const Geometry g, const WalkEntry* __restrict__ rows, con
     if (valid && kh < g.Kh && h >= 0 && h < g.H) {
       const int t = (b * g.H + h) * g.Nw + nw;
       run[kh] = rows + (size_t)t * row_stride;
-      n[kh] = __ldg(rows_n + t);
+      n[kh] = ld_plain(rows_n + t);
     }
     off[kh] = (uint32_t)kh * (uint32_t)g.Kw * (uint32_t)g.C * (uint32_t)g.J;
   }

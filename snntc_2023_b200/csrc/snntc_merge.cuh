@@ -34,7 +34,7 @@ constexpr uint32_t kRunEndBits = 0x7f800000u;   // +inf
 // terminator, so that dst is a run itself. Entries are written two at a time (16 bytes) where dst allows it:
 // dst must be 16-byte aligned.
 template <typename Entry, typename Entry2>
-SNNTC_HD void merge3_runs(const Entry* __restrict__ a, const Entry* __restrict__ b, const Entry* __restrict__ c,
+SNNTC_HD void merge3_runs(const Entry* a, const Entry* b, const Entry* c,
                           uint32_t off_a, uint32_t off_b, uint32_t off_c, int total, Entry* __restrict__ dst,
                           bool terminate) {
   Entry ha = a[0], hb = b[0], hc = c[0];
@@ -79,7 +79,7 @@ SNNTC_HD void merge3_runs(const Entry* __restrict__ a, const Entry* __restrict__
 // entries past their terminator (past `total` for dst): the last group is written whole, whatever lies behind
 // `total` in it is unspecified.
 template <typename Entry, typename Mem>
-SNNTC_HD void merge3_runs_blocked(const Entry* __restrict__ a, const Entry* __restrict__ b, const Entry* __restrict__ c,
+SNNTC_HD void merge3_runs_blocked(const Entry* a, const Entry* b, const Entry* c,
                                   uint32_t off_a, uint32_t off_b, uint32_t off_c, int total, Entry* __restrict__ dst,
                                   bool terminate, Mem& mem) {
   mem.load_window(0, a);
@@ -119,7 +119,7 @@ SNNTC_HD void merge3_runs_blocked(const Entry* __restrict__ a, const Entry* __re
 
 // Number of entries of `run` (n real entries, ascending) whose value is < v (or_equal = false) or <= v (true).
 template <typename Entry>
-SNNTC_HD int run_bound(const Entry* __restrict__ run, int n, float v, bool or_equal) {
+SNNTC_HD int run_bound(const Entry* run, int n, float v, bool or_equal) {
   int lo = 0, hi = n;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
@@ -161,8 +161,8 @@ SNNTC_HD void merge3_cut(const Entry* const* run, const int* n, int part, int pa
 // the first and behind the last such group one by one (the rest of those groups belongs to the neighbouring
 // pieces). Additionally needs Mem::store1(dst, e). Writes no terminator.
 template <typename Entry, typename Mem>
-SNNTC_HD void merge3_runs_blocked_range(const Entry* __restrict__ a, const Entry* __restrict__ b,
-                                        const Entry* __restrict__ c, uint32_t off_a, uint32_t off_b, uint32_t off_c,
+SNNTC_HD void merge3_runs_blocked_range(const Entry* a, const Entry* b,
+                                        const Entry* c, uint32_t off_a, uint32_t off_b, uint32_t off_c,
                                         int pa_, int pb_, int pc_, int count, Entry* __restrict__ dst, Mem& mem) {
   uint32_t pa = (uint32_t)pa_, pb = (uint32_t)pb_, pc = (uint32_t)pc_;
   mem.load_window(0, a + (pa & ~3u));

@@ -13,12 +13,13 @@ namespace {
 
 using snntc::chain_next;
 using snntc::chain_wait;
+using snntc::ld_plain;
 using snntc::launch_chained;
 
 // One thread per V consecutive channels of one output (V = 4 when C % 4 == 0: 16-byte accesses; else 1).
 // All indices fit 32 bits (checked by the callers).
 template <int V>
-__global__ void minpool_fwd_kernel(const float* __restrict__ x, float* __restrict__ y, int* __restrict__ arg,
+__global__ void minpool_fwd_kernel(const float* x, float* __restrict__ y, int* __restrict__ arg,
                                    int B, int H, int W, int C, int Kh, int Kw, int Sh, int Sw, int pt, int pl,
                                    int Nh, int Nw, float padvalue) {
   chain_wait();
@@ -48,10 +49,10 @@ __global__ void minpool_fwd_kernel(const float* __restrict__ x, float* __restric
         if (h >= 0 && h < H && w >= 0 && w < W) {
           idx = ((b * H + h) * W + w) * C + (int)cv * V;
           if constexpr (V == 4) {
-            const float4 q = __ldg(reinterpret_cast<const float4*>(x + idx));
+            const float4 q = ld_plain(reinterpret_cast<const float4*>(x + idx));
             v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
           } else {
-            v[0] = __ldg(x + idx);
+            v[0] = ld_plain(x + idx);
           }
         }
 #pragma unroll
@@ -74,7 +75,7 @@ __global__ void minpool_fwd_kernel(const float* __restrict__ x, float* __restric
 // contain it and whose winner it was. No atomics and no zero-fill: the sum of an element that overlapping
 // windows (kernel larger than stride) share is formed in a fixed order, so the result is the same bits every run.
 template <int V>
-__global__ void minpool_bwd_kernel(const float* __restrict__ gy, const int* __restrict__ arg, float* __restrict__ dx,
+__global__ void minpool_bwd_kernel(const float* gy, const int* arg, float* __restrict__ dx,
                                    int B, int H, int W, int C, int Kh, int Kw, int Sh, int Sw, int pt, int pl,
                                    int Nh, int Nw) {
   chain_wait();
@@ -101,16 +102,16 @@ __global__ void minpool_bwd_kernel(const float* __restrict__ gy, const int* __re
       for (int nw = nw0; nw <= nw1; ++nw) {
         const int o = ((b * Nh + nh) * Nw + nw) * C + (int)cv * V;
         if constexpr (V == 4) {
-          const int4 a = __ldg(reinterpret_cast<const int4*>(arg + o));
+          const int4 a = ld_plain(reinterpret_cast<const int4*>(arg + o));
           if (a.x == e || a.y == e + 1 || a.z == e + 2 || a.w == e + 3) {
-            const float4 g4 = __ldg(reinterpret_cast<const float4*>(gy + o));
+            const float4 g4 = ld_plain(reinterpret_cast<const float4*>(gy + o));
             if (a.x == e) s[0] += g4.x;
             if (a.y == e + 1) s[1] += g4.y;
             if (a.z == e + 2) s[2] += g4.z;
             if (a.w == e + 3) s[3] += g4.w;
           }
         } else {
-          if (__ldg(arg + o) == e) s[0] += __ldg(gy + o);
+          if (ld_plain(arg + o) == e) s[0] += ld_plain(gy + o);
         }
       }
     if constexpr (V == 4) reinterpret_cast<float4*>(dx)[ev] = make_float4(s[0], s[1], s[2], s[3]);

@@ -103,7 +103,7 @@ __host__ __device__ __forceinline__ size_t row_bytes(int I, int nb_log2) {
 // TPR threads per row (32: several rows per CTA, else one), EPT keys per thread in registers (0: in shared memory).
 template <int TPR, int EPT>
 __global__ void __launch_bounds__(TPR == 32 ? 256 : TPR)
-snn_bucket_sort_kernel(const Geometry g, const float* __restrict__ x, WalkEntry* __restrict__ lists, int* __restrict__ nvalid,
+snn_bucket_sort_kernel(const Geometry g, const float* x, WalkEntry* __restrict__ lists, int* __restrict__ nvalid,
                        int istride, int nb_log2, int table) {
   chain_wait();
   chain_next();
@@ -150,13 +150,13 @@ snn_bucket_sort_kernel(const Geometry g, const float* __restrict__ x, WalkEntry*
       if (i < I) {
         if (table) {
           const unsigned khw = tap_khw[i];
-          if ((unsigned)(h0 + (int)(khw >> 8)) < (unsigned)g.H && (unsigned)(w0 + (int)(khw & 255u)) < (unsigned)g.W) v = __ldg(xr + tap_off[i]);
+          if ((unsigned)(h0 + (int)(khw >> 8)) < (unsigned)g.H && (unsigned)(w0 + (int)(khw & 255u)) < (unsigned)g.W) v = ld_plain(xr + tap_off[i]);
         } else if (g.is_conv) {     // a window too large for the table
           const int tap = i / g.C, c = i - tap * g.C;
           const int kh = tap / g.Kw, kw = tap - kh * g.Kw;
-          if ((unsigned)(h0 + kh) < (unsigned)g.H && (unsigned)(w0 + kw) < (unsigned)g.W) v = __ldg(xr + (ptrdiff_t)(kh * g.W + kw) * g.C + c);
+          if ((unsigned)(h0 + kh) < (unsigned)g.H && (unsigned)(w0 + kw) < (unsigned)g.W) v = ld_plain(xr + (ptrdiff_t)(kh * g.W + kw) * g.C + c);
         } else {
-          v = __ldg(xr + i);
+          v = ld_plain(xr + i);
         }
       }
       return v;

@@ -21,6 +21,7 @@ namespace {
 
 using snntc::chain_next;
 using snntc::chain_wait;
+using snntc::ld_plain;
 using snntc::launch_chained;
 
 int grid_for(size_t n, int per_block = 256) {
@@ -30,12 +31,12 @@ int grid_for(size_t n, int per_block = 256) {
   return (int)b;
 }
 
-__global__ void encode_kernel(const float* __restrict__ p, float* __restrict__ x, size_t n, float scale, int one_minus) {
+__global__ void encode_kernel(const float* p, float* __restrict__ x, size_t n, float scale, int one_minus) {
   chain_wait();
   chain_next();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
-    const float v = __ldg(p + e);
+    const float v = ld_plain(p + e);
     x[e] = expf(scale * (one_minus ? 1.0f - v : v));
   }
 }
@@ -141,17 +142,17 @@ __global__ void wcost_apply_kernel(const float* __restrict__ w, const float* __r
 // Keras Adam: lr_t = lr * sqrt(1 - b2^t) / (1 - b1^t); m += (g - m)(1 - b1); v += (g^2 - v)(1 - b2);
 // w -= lr_t * m / (sqrt(v) + eps). The step count t lives on the device (step[0] = steps taken so far), so that
 // a captured CUDA graph replays with the count advancing; a one-thread kernel increments it after the update.
-__global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
+__global__ void adam_kernel(float* __restrict__ w, const float* g, float* __restrict__ m, float* __restrict__ v,
                             size_t n, float lr, float b1, float b2, float eps, float gscale,
-                            const int* __restrict__ step) {
+                            const int* step) {
   chain_wait();
   chain_next();
-  const int t = __ldg(step) + 1;
+  const int t = ld_plain(step) + 1;
   const float c1 = 1.0f - powf(b1, (float)t), c2 = 1.0f - powf(b2, (float)t);
   const float lrt = lr * sqrtf(c2) / c1;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
-    const float ge = __ldg(g + e) * gscale;
+    const float ge = ld_plain(g + e) * gscale;
     const float me = m[e] + (ge - m[e]) * (1.0f - b1);
     const float ve = v[e] + (ge * ge - v[e]) * (1.0f - b2);
     m[e] = me;
@@ -182,13 +183,13 @@ constexpr int kLossCluster = 8;
 struct RowStats { float zmax, lse; int amin; };   // max of z = -y, sum exp(z - zmax), arg-min of y (lowest index on ties)
 
 template <int G>
-__device__ __forceinline__ RowStats row_stats(const float* __restrict__ row, int J, int gl) {
+__device__ __forceinline__ RowStats row_stats(const float* row, int J, int gl) {
   RowStats s;
   s.zmax = -CUDART_INF_F;
   s.amin = 0x7fffffff;
   float ymin = CUDART_INF_F;
   for (int j = gl; j < J; j += G) {
-    const float v = __ldg(row + j);
+    const float v = ld_plain(row + j);
     s.zmax = fmaxf(s.zmax, -v);
     if (v < ymin) { ymin = v; s.amin = j; }
   }
@@ -200,7 +201,7 @@ __device__ __forceinline__ RowStats row_stats(const float* __restrict__ row, int
     if (oy < ymin || (oy == ymin && oa < s.amin)) { ymin = oy; s.amin = oa; }
   }
   float se = 0.f;
-  for (int j = gl; j < J; j += G) se += expf(-__ldg(row + j) - s.zmax);
+  for (int j = gl; j < J; j += G) se += expf(-ld_plain(row + j) - s.zmax);
 #pragma unroll
   for (int d = G / 2; d >= 1; d >>= 1) se += __shfl_xor_sync(0xffffffffu, se, d);
   s.lse = se;
@@ -239,7 +240,7 @@ __device__ __forceinline__ float2 cluster_sum(float a, float b) {
 
 template <int G>
 __global__ void __cluster_dims__(kLossCluster, 1, 1) __launch_bounds__(kLossThreads)
-loss_fwd_kernel(const float* __restrict__ y, const long long* __restrict__ labels, float* __restrict__ loss,
+loss_fwd_kernel(const float* y, const long long* labels, float* __restrict__ loss,
                 float* __restrict__ hits, int B, int J, float lscale) {
   chain_wait();
   chain_next();
@@ -255,7 +256,7 @@ loss_fwd_kernel(const float* __restrict__ y, const long long* __restrict__ label
       const int lab = (int)labels[b];
       // the loss is log(se) + (zmax - z[label]), never logsumexp itself, which would lose the small term beside a large
       // |zmax| (all outputs at MAX)
-      const float zl = (lab >= 0 && lab < J) ? -__ldg(row + lab) : s.zmax;
+      const float zl = (lab >= 0 && lab < J) ? -ld_plain(row + lab) : s.zmax;
       loss_acc += (logf(s.lse) + (s.zmax - zl)) * lscale;
       hit_acc += (s.amin == lab) ? 1.0f : 0.0f;
     }
@@ -267,7 +268,7 @@ loss_fwd_kernel(const float* __restrict__ y, const long long* __restrict__ label
 // grad_y = -(softmax(-y) - onehot) * gscale * (*gloss): the softmax again from y instead of a gradient kept by the forward
 template <int G>
 __global__ void __launch_bounds__(256)
-loss_bwd_kernel(const float* __restrict__ y, const long long* __restrict__ labels, const float* __restrict__ gloss,
+loss_bwd_kernel(const float* y, const long long* labels, const float* gloss,
                 float* __restrict__ grad, int B, int J, float gscale) {
   chain_wait();
   chain_next();
@@ -278,9 +279,9 @@ loss_bwd_kernel(const float* __restrict__ y, const long long* __restrict__ label
   const RowStats s = row_stats<G>(row, J, gl);
   if (!ok) return;
   const int lab = (int)labels[b];
-  const float inv = 1.0f / s.lse, up = __ldg(gloss);
+  const float inv = 1.0f / s.lse, up = ld_plain(gloss);
   for (int j = gl; j < J; j += G) {
-    const float sm = expf(-__ldg(row + j) - s.zmax) * inv;
+    const float sm = expf(-ld_plain(row + j) - s.zmax) * inv;
     grad[(size_t)b * J + j] = -(sm - (j == lab ? 1.0f : 0.0f)) * gscale * up;
   }
 }
@@ -333,12 +334,12 @@ cost_sums_kernel(const __grid_constant__ CostTensors c, float* __restrict__ part
     for (; r + 7 * lines < r1; r += 8 * lines) {
       float v[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) v[q] = __ldg(w + (size_t)(r + q * lines) * J);
+      for (int q = 0; q < 8; ++q) v[q] = ld_plain(w + (size_t)(r + q * lines) * J);
 #pragma unroll
       for (int q = 0; q < 8; ++q) { s += v[q]; s2 = fmaf(v[q], v[q], s2); }
     }
     for (; r < r1; r += lines) {
-      const float v = __ldg(w + (size_t)r * J);
+      const float v = ld_plain(w + (size_t)r * J);
       s += v;
       s2 = fmaf(v, v, s2);
     }
@@ -362,7 +363,7 @@ cost_sums_kernel(const __grid_constant__ CostTensors c, float* __restrict__ part
 
 // One cluster: column sums out of the partial ones, and the cost of all tensors (added to *cost when `add` is set).
 __global__ void __cluster_dims__(kLossCluster, 1, 1) __launch_bounds__(kLossThreads)
-cost_total_kernel(const __grid_constant__ CostTensors c, const float* __restrict__ partial, const float* __restrict__ sq,
+cost_total_kernel(const __grid_constant__ CostTensors c, const float* partial, const float* sq,
                   float* __restrict__ colsum, float* __restrict__ cost, float K, float K2, int add) {
   chain_wait();
   chain_next();
@@ -375,13 +376,13 @@ cost_total_kernel(const __grid_constant__ CostTensors c, const float* __restrict
     const float* p = partial + c.partial[t] + (col - c.first_col[t]);
     float s = 0.f;
 #pragma unroll 8
-    for (int k = 0; k < c.slices[t]; ++k) s += __ldg(p + (long long)k * J);
+    for (int k = 0; k < c.slices[t]; ++k) s += ld_plain(p + (long long)k * J);
     colsum[col] = s;
     total += fmaxf(0.f, 1.0f - s) * (K / (float)J);
   }
   for (int k = me; k < c.first_cta[c.count]; k += kAll) {
     const int t = tensor_of(c.first_cta, c.count, k);
-    total += __ldg(sq + k) * (K2 / ((float)c.rows[t] * (float)c.cols[t]));
+    total += ld_plain(sq + k) * (K2 / ((float)c.rows[t] * (float)c.cols[t]));
   }
   const float2 sum = cluster_sum(total, 0.f);
   if (blockIdx.x == 0 && threadIdx.x == 0) *cost = add ? *cost + sum.x : sum.x;
@@ -390,7 +391,7 @@ cost_total_kernel(const __grid_constant__ CostTensors c, const float* __restrict
 // gw = gcost * (-K/J [colsum < 1] + 2 K2 / n * w), or gw += it, a CTA per 4096 elements of one tensor
 template <bool ADD>
 __global__ void __launch_bounds__(kCostThreads)
-cost_grad_kernel(const __grid_constant__ CostTensors c, const float* __restrict__ colsum, const float* __restrict__ gcost,
+cost_grad_kernel(const __grid_constant__ CostTensors c, const float* colsum, const float* gcost,
                  float K, float K2) {
   chain_wait();
   chain_next();
@@ -399,7 +400,7 @@ cost_grad_kernel(const __grid_constant__ CostTensors c, const float* __restrict_
   const unsigned n = (unsigned)c.rows[t] * (unsigned)J;
   const unsigned e0 = (unsigned)(blockIdx.x - c.first_chunk[t]) * kCostChunk;
   const unsigned e1 = min(n, e0 + kCostChunk);
-  const float up = __ldg(gcost);
+  const float up = ld_plain(gcost);
   const float a = -K / (float)J, b2 = 2.0f * K2 / (float)n;
   const float* cs = colsum + c.first_col[t];
   const float* w = c.w[t];
@@ -407,12 +408,12 @@ cost_grad_kernel(const __grid_constant__ CostTensors c, const float* __restrict_
   if ((J & 3) == 0 && (((uintptr_t)w | (uintptr_t)gw) & 15) == 0) {
     for (unsigned e = e0 + 4 * threadIdx.x; e < e1; e += 4 * kCostThreads) {
       const unsigned j = e % (unsigned)J;
-      const float4 v = __ldg(reinterpret_cast<const float4*>(w + e));
+      const float4 v = ld_plain(reinterpret_cast<const float4*>(w + e));
       float4 r;
-      r.x = ((1.0f - __ldg(cs + j)) > 0.f ? a : 0.f) + b2 * v.x;
-      r.y = ((1.0f - __ldg(cs + j + 1)) > 0.f ? a : 0.f) + b2 * v.y;
-      r.z = ((1.0f - __ldg(cs + j + 2)) > 0.f ? a : 0.f) + b2 * v.z;
-      r.w = ((1.0f - __ldg(cs + j + 3)) > 0.f ? a : 0.f) + b2 * v.w;
+      r.x = ((1.0f - ld_plain(cs + j)) > 0.f ? a : 0.f) + b2 * v.x;
+      r.y = ((1.0f - ld_plain(cs + j + 1)) > 0.f ? a : 0.f) + b2 * v.y;
+      r.z = ((1.0f - ld_plain(cs + j + 2)) > 0.f ? a : 0.f) + b2 * v.z;
+      r.w = ((1.0f - ld_plain(cs + j + 3)) > 0.f ? a : 0.f) + b2 * v.w;
       // (the product is rounded before it is added, as when a gradient tensor of its own is added to the bucket)
       float4 o = make_float4(__fmul_rn(up, r.x), __fmul_rn(up, r.y), __fmul_rn(up, r.z), __fmul_rn(up, r.w));
       if (ADD) {
@@ -423,7 +424,7 @@ cost_grad_kernel(const __grid_constant__ CostTensors c, const float* __restrict_
     }
   } else {
     for (unsigned e = e0 + threadIdx.x; e < e1; e += kCostThreads) {
-      const float r = __fmul_rn(up, ((1.0f - __ldg(cs + e % (unsigned)J)) > 0.f ? a : 0.f) + b2 * __ldg(w + e));
+      const float r = __fmul_rn(up, ((1.0f - ld_plain(cs + e % (unsigned)J)) > 0.f ? a : 0.f) + b2 * ld_plain(w + e));
       gw[e] = ADD ? gw[e] + r : r;
     }
   }

@@ -20,11 +20,11 @@ __device__ __forceinline__ bool ratio_le(float ysum, float wsum, float c) {
 
 // Number of list entries whose input value lies strictly below y: the causal-set size of an output that fired
 // at y (every consumed input is below the spike value, every other one is not). Binary search, one thread.
-__device__ __forceinline__ int entries_below(const WalkEntry* __restrict__ ents, int n, float y) {
+__device__ __forceinline__ int entries_below(const WalkEntry* ents, int n, float y) {
   int lo = 0, hi = n;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
-    if (__uint_as_float(__ldcg(ents + mid).x) < y) lo = mid + 1; else hi = mid;
+    if (__uint_as_float(ld_l2(ents + mid).x) < y) lo = mid + 1; else hi = mid;
   }
   return lo;
 }

@@ -113,8 +113,8 @@ struct Walk {
 // or 16 where there are warps to fill the SMs (half the shared memory per warp: 58 against 68 us for 784 -> 400 at 256 samples).
 template <bool VEC, int kBlock>
 __global__ void __launch_bounds__(32 * kWarps)
-snn_walk_ring_kernel(const Geometry g, const WalkEntry* __restrict__ lists, const int* __restrict__ nvalid, int istride,
-                     const float* __restrict__ w, float* __restrict__ out, int slices) {
+snn_walk_ring_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid, int istride,
+                     const float* w, float* __restrict__ out, int slices) {
   chain_wait();
   chain_next();
   __shared__ __align__(16) RingWarp<kBlock> ring[kWarps];
@@ -125,8 +125,8 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
   const long item = (long)blockIdx.x * kWarps + warp;
   if (item >= (long)g.R * slices) return;
   const int r = (int)(item % g.R), j0 = (int)(item / g.R) * 32;
-  const WalkEntry* __restrict__ ents = lists + (size_t)r * istride;
-  const int n = __shfl_sync(0xffffffffu, __ldg(nvalid + r), 0);
+  const WalkEntry* ents = lists + (size_t)r * istride;
+  const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid + r), 0);
   const int blocks = (n + kBlock - 1) / kBlock;
 
   // list block b: read a block ahead into a register, then put into shared memory. Behind the end of the list: offset 0 (a
@@ -134,7 +134,7 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
   WalkEntry pre = make_uint2(0u, 0u);
   auto read_list = [&](int b) {
     pre = make_uint2(0u, 0u);
-    if ((kBlock == 32 || lane < kBlock) && b * kBlock + lane < n) pre = __ldcg(ents + b * kBlock + lane);
+    if ((kBlock == 32 || lane < kBlock) && b * kBlock + lane < n) pre = ld_l2(ents + b * kBlock + lane);
   };
   auto put_list = [&](int b) {
     if (kBlock == 32 || lane < kBlock) {
@@ -175,7 +175,7 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
   wk.wsum = -g.theta;
   wk.ysum = 0.f;
   if (g.has_bias) {   // the bias input (value biasvolt, weight row I) is always consumed first
-    const float wb = ok ? __ldg(w + (size_t)g.I * J + j) : 0.f;
+    const float wb = ok ? ld_plain(w + (size_t)g.I * J + j) : 0.f;
     wk.wsum += wb;
     wk.ysum = g.biasvolt * wb;
   }

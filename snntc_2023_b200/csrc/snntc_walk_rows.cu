@@ -36,8 +36,8 @@ __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)_
 
 template <int LPR, bool WS>
 __global__ void __launch_bounds__(WS ? 1024 : 256, WS ? 1 : 4)
-snn_walk_rows_kernel(const Geometry g, const WalkEntry* __restrict__ lists, const int* __restrict__ nvalid, int istride,
-                     const float* __restrict__ w, float* __restrict__ out) {
+snn_walk_rows_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid, int istride,
+                     const float* w, float* __restrict__ out) {
   chain_wait();
   chain_next();
   constexpr int RPW = Shape<LPR>::rows, BLK = Shape<LPR>::block, PER = BLK / LPR;
@@ -58,7 +58,7 @@ snn_walk_rows_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
   WalkEntry* stage = stage_all + (size_t)(warp * RPW + sub) * BLK;
   float tolbase;                                  // see walk_tolerance_base in snntc_forward.cu
   {
-    float b = lane < g.wbound_n ? __ldg(g.wbound + lane) : 0.f;
+    float b = lane < g.wbound_n ? ld_plain(g.wbound + lane) : 0.f;
 #pragma unroll
     for (int d = 16; d >= 1; d >>= 1) b += __shfl_xor_sync(0xffffffffu, b, d);
     tolbase = 4.76837158203125e-7f * (fabsf(g.theta) + b) * 1.0001f;
@@ -74,7 +74,7 @@ snn_walk_rows_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
       asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(4u * eoff + ws_lane));
       return v;
     } else {
-      return __ldg(reinterpret_cast<const float4*>(wbytes + (size_t)(eoff + lane_off) * 4u));
+      return ld_plain(reinterpret_cast<const float4*>(wbytes + (size_t)(eoff + lane_off) * 4u));
     }
   };
 
@@ -82,10 +82,10 @@ snn_walk_rows_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
   for (int grp = blockIdx.x * WARPS + warp; grp < groups; grp += gridDim.x * WARPS) {
     const int r = grp * RPW + sub;
     const bool row_ok = r < g.R;
-    const int n = row_ok ? __ldg(nvalid + r) : 0;
+    const int n = row_ok ? ld_plain(nvalid + r) : 0;
     const int nmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)n);
     const int nmin = (int)__reduce_min_sync(0xffffffffu, (unsigned)n);
-    const WalkEntry* __restrict__ ents = lists + (size_t)(row_ok ? r : 0) * istride;
+    const WalkEntry* ents = lists + (size_t)(row_ok ? r : 0) * istride;
     // the bias input (value biasvolt, weight row I) is always consumed first
     float wsum[4] = {-g.theta, -g.theta, -g.theta, -g.theta}, ysum[4] = {0.f, 0.f, 0.f, 0.f};
     if (g.has_bias) {
@@ -167,7 +167,7 @@ snn_walk_rows_kernel(const Geometry g, const WalkEntry* __restrict__ lists, cons
       for (int q = 0; q < PER; ++q) {
         const int k = base + gl + q * LPR;
         pre[q] = make_uint2(0u, 0u);
-        if (k < n) pre[q] = __ldcg(ents + k);
+        if (k < n) pre[q] = ld_l2(ents + k);
       }
     };
     read_block(0);
