@@ -9,6 +9,8 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/graph_task.h>
 
 #include <algorithm>
 #include <cstring>
@@ -420,6 +422,7 @@ void cost_grads(const variable_list& ws, const variable_list& gw, const CostStat
 // the dW kernels write their slices, in whatever order autograd visits the nodes.
 struct Fold {
   struct Pending { variable_list weights; c10::intrusive_ptr<CostState> state; Tensor grad; };
+  int graph_task = -1;             // of the pass: a cost's node that runs in any other pass is none of this one's
   std::vector<const void*> weights;
   variable_list sinks;
   std::vector<Pending> pending;
@@ -430,22 +433,31 @@ struct Fold {
   }
 };
 std::mutex g_fold_mutex;
-std::vector<Fold*> g_folds;      // the backward passes of this kind under way, one per calling thread
+std::vector<Fold*> g_folds;        // the backward passes of this kind under way
 
-// true: some pass under way takes the cost's gradient itself (exactly one does, and it knows every weight)
+// The first node of such a pass (autograd runs it on a thread of its own choice): hands the gradient on, and the pass is known.
+struct FoldRoot : torch::autograd::Node {
+  Fold* fold = nullptr;
+  variable_list apply(variable_list&& grads) override {
+    const std::lock_guard<std::mutex> lock(g_fold_mutex);
+    fold->graph_task = torch::autograd::get_current_graph_task_id();
+    g_folds.push_back(fold);
+    return std::move(grads);
+  }
+};
+
+// true: the pass that the calling node runs in takes the cost's gradient itself (it knows every weight)
 bool fold_cost(const variable_list& ws, const c10::intrusive_ptr<CostState>& s, const Tensor& g) {
   const std::lock_guard<std::mutex> lock(g_fold_mutex);
-  Fold* owner = nullptr;
+  const int task = torch::autograd::get_current_graph_task_id();
   for (Fold* f : g_folds) {
-    size_t known = 0;
-    for (const Tensor& w : ws) known += f->sink_of(w) != nullptr;
-    if (known == 0) continue;
-    if (known < ws.size() || owner != nullptr) return false;
-    owner = f;
+    if (f->graph_task != task) continue;
+    for (const Tensor& w : ws)
+      if (f->sink_of(w) == nullptr) return false;
+    f->pending.push_back({ws, s, g});
+    return true;
   }
-  if (owner == nullptr) return false;
-  owner->pending.push_back({ws, s, g});
-  return true;
+  return false;
 }
 
 struct CostFunction : torch::autograd::Function<CostFunction> {
@@ -483,17 +495,24 @@ void backward(const Tensor& objective, const Tensor& one, const std::vector<Tens
   Fold f;
   for (const Tensor& w : weights) f.weights.push_back(w.data_ptr());
   f.sinks = sinks;
-  struct Enter {
+  struct Leave {
     Fold* f;
-    explicit Enter(Fold* p) : f(p) { const std::lock_guard<std::mutex> lock(g_fold_mutex); g_folds.push_back(f); }
-    ~Enter() {
+    ~Leave() {
       const std::lock_guard<std::mutex> lock(g_fold_mutex);
-      g_folds.erase(std::find(g_folds.begin(), g_folds.end(), f));
+      g_folds.erase(std::remove(g_folds.begin(), g_folds.end(), f), g_folds.end());
     }
   };
   {
-    const Enter entered(&f);
-    torch::autograd::backward({objective}, {one});
+    const Leave leave{&f};
+    Tensor root = objective;
+    if (objective.requires_grad()) {
+      auto node = std::make_shared<FoldRoot>();
+      node->fold = &f;
+      node->add_next_edge(torch::autograd::impl::gradient_edge(objective));
+      root = objective.detach();
+      torch::autograd::set_history(root, node);
+    }
+    torch::autograd::backward({root}, {one});
   }
   for (const Fold::Pending& p : f.pending) {
     variable_list to;
