@@ -9,6 +9,7 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/functions/accumulate_grad.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/graph_task.h>
 
@@ -446,14 +447,22 @@ struct FoldRoot : torch::autograd::Node {
   }
 };
 
-// true: the pass that the calling node runs in takes the cost's gradient itself (it knows every weight)
+// Whether autograd would do no more with the calling node's k-th gradient than add it to a leaf's .grad. Not so for a weight that
+// requires no gradient, which gets none.
+bool only_accumulated(size_t k) {
+  const torch::autograd::Edge& edge = torch::autograd::get_current_node()->next_edge(k);
+  return dynamic_cast<torch::autograd::AccumulateGrad*>(edge.function.get()) != nullptr;
+}
+
+// true: the pass that the calling node runs in takes the cost's gradient itself (it knows every weight, and nothing else is to
+// happen to their gradients)
 bool fold_cost(const variable_list& ws, const c10::intrusive_ptr<CostState>& s, const Tensor& g) {
   const std::lock_guard<std::mutex> lock(g_fold_mutex);
   const int task = torch::autograd::get_current_graph_task_id();
   for (Fold* f : g_folds) {
     if (f->graph_task != task) continue;
-    for (const Tensor& w : ws)
-      if (f->sink_of(w) == nullptr) return false;
+    for (size_t k = 0; k < ws.size(); ++k)
+      if (f->sink_of(ws[k]) == nullptr || !only_accumulated(k)) return false;
     f->pending.push_back({ws, s, g});
     return true;
   }
