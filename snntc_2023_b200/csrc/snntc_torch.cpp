@@ -448,10 +448,12 @@ struct FoldRoot : torch::autograd::Node {
 };
 
 // Whether autograd would do no more with the calling node's k-th gradient than add it to a leaf's .grad. Not so for a weight that
-// requires no gradient, which gets none.
+// requires no gradient, which gets none, nor where a hook of any kind is to see the gradient.
 bool only_accumulated(size_t k) {
   const torch::autograd::Edge& edge = torch::autograd::get_current_node()->next_edge(k);
-  return dynamic_cast<torch::autograd::AccumulateGrad*>(edge.function.get()) != nullptr;
+  auto* leaf = dynamic_cast<torch::autograd::AccumulateGrad*>(edge.function.get());
+  return leaf != nullptr && leaf->tensor_pre_hooks().empty() && leaf->tensor_post_acc_grad_hooks() == nullptr &&
+         leaf->retains_grad_hooks().empty() && leaf->pre_hooks().empty() && leaf->post_hooks().empty();
 }
 
 // true: the pass that the calling node runs in takes the cost's gradient itself (it knows every weight, and nothing else is to

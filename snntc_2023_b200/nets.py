@@ -141,12 +141,10 @@ class SnnNet(torch.nn.Module):
         weights, sinks = [l.weight for l in ws], [l.grad_sink for l in ws]
         for w in weights:
             w.grad = None
-        # (a hook on a weight is to see the cost's gradient: autograd's own way then)
-        if (objective.dim() == 0 and objective.is_cuda and objective.dtype == torch.float32 and
-                not any(w._backward_hooks for w in weights)):
+        if objective.dim() == 0 and objective.is_cuda and objective.dtype == torch.float32:
             if self._one is None or self._one.device != objective.device:
                 self._one = torch.ones((), device=objective.device)
-            _lib.native().backward(objective, self._one, weights, sinks)   # adds a constraint cost's gradient to flat_grad itself
+            _lib.native().backward(objective, self._one, weights, sinks)   # adds a constraint cost's gradient to flat_grad itself (where no hook is to see it)
         else:
             objective.backward()
         more = [k for k, w in enumerate(weights) if w.grad is not None]
