@@ -424,6 +424,7 @@ void cost_grads(const variable_list& ws, const variable_list& gw, const CostStat
 struct Fold {
   struct Pending { variable_list weights; c10::intrusive_ptr<CostState> state; Tensor grad; };
   int graph_task = -1;             // of the pass: a cost's node that runs in any other pass is none of this one's
+  c10::cuda::CUDAStream stream;    // the caller's, on which the gradients are formed in the end
   std::vector<const void*> weights;
   variable_list sinks;
   std::vector<Pending> pending;
@@ -456,13 +457,14 @@ bool only_accumulated(size_t k) {
          leaf->retains_grad_hooks().empty() && leaf->pre_hooks().empty() && leaf->post_hooks().empty();
 }
 
-// true: the pass that the calling node runs in takes the cost's gradient itself (it knows every weight, and nothing else is to
-// happen to their gradients)
+// true: the pass that the calling node runs in takes the cost's gradient itself (it knows every weight, nothing else is to happen
+// to their gradients, and the node runs on the caller's stream, so that nothing has to be waited for)
 bool fold_cost(const variable_list& ws, const c10::intrusive_ptr<CostState>& s, const Tensor& g) {
   const std::lock_guard<std::mutex> lock(g_fold_mutex);
   const int task = torch::autograd::get_current_graph_task_id();
   for (Fold* f : g_folds) {
     if (f->graph_task != task) continue;
+    if (at::cuda::getCurrentCUDAStream(g.get_device()) != f->stream) return false;
     for (size_t k = 0; k < ws.size(); ++k)
       if (f->sink_of(ws[k]) == nullptr || !only_accumulated(k)) return false;
     f->pending.push_back({ws, s, g});
@@ -503,7 +505,7 @@ struct CostFunction : torch::autograd::Function<CostFunction> {
 
 // objective.backward() with the upstream gradient `one`; constraint costs of `weights` go into `sinks` (see Fold)
 void backward(const Tensor& objective, const Tensor& one, const std::vector<Tensor>& weights, const std::vector<Tensor>& sinks) {
-  Fold f;
+  Fold f{.stream = at::cuda::getCurrentCUDAStream(objective.get_device())};
   for (const Tensor& w : weights) f.weights.push_back(w.data_ptr());
   f.sinks = sinks;
   struct Leave {
