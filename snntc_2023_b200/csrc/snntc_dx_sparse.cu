@@ -224,7 +224,9 @@ int launch_one(const Geometry& g, const float* x, const float* wt, const uint4* 
   long grid = (warps + (kThreads / 32) - 1) / (kThreads / 32);
   const long cap = (long)li.num_sms * 16;
   if (grid > cap) grid = cap;
-  (void)launch_chained(snn_dx_sparse_kernel<CPL, LPP>, (int)grid, kThreads, 0, s, 0, g, x, wt, list, count, dx, gate);
+  // (in plain order: the transposed weights are read through the read-only path -- 256 channels: 64 us so, 90 with ordinary loads;
+  // 512: 246 and 268)
+  snn_dx_sparse_kernel<CPL, LPP><<<(int)grid, kThreads, 0, s>>>(g, x, wt, list, count, dx, gate);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -254,17 +256,15 @@ int launch_dx_sparse(const Geometry& g, const float* uv, const float* x, const f
   int* count = reinterpret_cast<int*>(base + align256((size_t)g.R * g.J * sizeof(uint4)));
   float* wt = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(count) + align256((size_t)g.R * sizeof(int)));
 
-  // The transpose first: the kernel that walks the lists reads its result through the read-only path, so that it must not be the
-  // kernel directly in front (256 channels: 64 us so, 90 with ordinary loads; 512: 246 and 268).
+  long grid = ((long)g.R + (kThreads / 32) - 1) / (kThreads / 32);
+  if (grid > (long)li.num_sms * 16) grid = (long)li.num_sms * 16;
+  (void)launch_chained(snn_act_lists_kernel, (int)grid, kThreads, 0, s, 0, out, uv, g.R, g.J, list, count, gate);
+  count_launch();
+  if (cudaGetLastError() != cudaSuccess) return E_CUDA;
   const size_t nw = (size_t)g.Kh * g.Kw * g.C * g.J;
   long tg = (long)((nw + 255) / 256);
   if (tg > (long)li.num_sms * 8) tg = (long)li.num_sms * 8;
   (void)launch_chained(snn_weight_transpose_kernel, (int)tg, 256, 0, s, 0, w, wt, g.Kh * g.Kw, g.C, g.J, gate);
-  count_launch();
-  if (cudaGetLastError() != cudaSuccess) return E_CUDA;
-  long grid = ((long)g.R + (kThreads / 32) - 1) / (kThreads / 32);
-  if (grid > (long)li.num_sms * 16) grid = (long)li.num_sms * 16;
-  (void)launch_chained(snn_act_lists_kernel, (int)grid, kThreads, 0, s, 0, out, uv, g.R, g.J, list, count, gate);
   count_launch();
   if (cudaGetLastError() != cudaSuccess) return E_CUDA;
 

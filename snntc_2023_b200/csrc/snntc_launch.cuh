@@ -28,9 +28,8 @@ __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.laun
 //   ld_plain    an ordinary load, ordered behind chain_wait() by its memory clobber
 //   ld_l2       past L1: data that is read once and should leave L1 to the weights
 //   ld_stream   evict first: data that nobody reads again
-//   ld_readonly the read-only path after all, for what was written at least two launches in front of the reader in its own stream:
-//               every kernel calls chain_next() behind chain_wait(), so when the reader is put on the SMs only the kernel directly
-//               in front can still be running. Used where the compiler's freedom to move such loads was measured to pay.
+//   ld_readonly the read-only path after all, in kernels that are never launched as dependents but in plain stream order. Used
+//               where the compiler's freedom to move such loads was measured to pay.
 template <typename T>
 __device__ __forceinline__ T ld_plain(const T* p) { return *p; }
 template <typename T>

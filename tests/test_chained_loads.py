@@ -51,27 +51,22 @@ def test_no_read_only_loads_in_chained_kernels(source):
     text = _strip_comments(open(os.path.join(CSRC, source)).read())
     if source == "snntc_launch.cuh":          # where ld_readonly is defined: the one exception, held to its rule below
         text = text.replace("return __ldg(p);", "", 1)
-    unchained = set(re.findall(r"\b(\w+_kernel)\s*<<<", text))
+    unchained = set(re.findall(r"\b(\w+_kernel)(?:<[\w, ]+>)?\s*<<<", text))
     for name, body in _kernels(text):
         if name in unchained and "chain_wait" not in body:
             text = text.replace(body, "")     # launched in plain stream order: nothing in front of it is still running
     assert not READ_ONLY.findall(text), [m.group(0) for m in READ_ONLY.finditer(text)]
 
 
-def test_the_read_only_path_serves_older_data_only():
-    """ld_readonly is for what the kernel directly in front of the reader does not write. Its one user reads the transposed
-    weights: the transpose is launched first, then the lists, then the reader, and every kernel lets its successor onto the
-    SMs only behind its own wait."""
-    users = {}
+def test_the_read_only_path_only_where_nothing_is_still_running():
+    """Kernels that read by ld_readonly are launched in plain stream order, never as dependents; every kernel that lets its
+    successor onto the SMs early has waited for its own predecessor first."""
     for f in _sources():
         text = _strip_comments(open(os.path.join(CSRC, f)).read())
+        chained = set(re.findall(r"launch_chained\(\s*(\w+_kernel)", text)) | {"snn_walk_ring_kernel"}
+        plain = set(re.findall(r"\b(\w+_kernel)(?:<[\w, ]+>)?\s*<<<", text))
         for name, body in _kernels(text):
             if "chain_next" in body:
                 assert body.index("chain_wait();") < body.index("chain_next();"), name
             if "ld_readonly" in body:
-                users[name] = (f, re.findall(r"ld_readonly\([^;]*?\(?(\w+)\s*\+", body))
-    assert users == {"snn_dx_sparse_kernel": ("snntc_dx_sparse.cu", ["wrow"])}
-    text = _strip_comments(open(os.path.join(CSRC, "snntc_dx_sparse.cu")).read())
-    body = text[text.index("int launch_dx_sparse("):]
-    order = [body.index(k) for k in ("snn_weight_transpose_kernel", "snn_act_lists_kernel", "launch_one<")]
-    assert order == sorted(order) and text.count("launch_chained(") == 3
+                assert name in plain and name not in chained, name
