@@ -155,6 +155,10 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
     wfin[m] = wsum[m];
     yfin[m] = ysum[m];
     livemask[m] = -1;
+    if (!jok[m]) {   // no output: parked from the start like one that has fired, or the walk would wait for it
+      livemask[m] = 0;
+      wsum[m] = -CUDART_INF_F;
+    }
   }
   // Without bias the sums start at (-theta, 0), for which "ysum/wsum > c" is false for every c >= 0, so the
   // first step needs no special case; with bias the previous input is the bias input itself.
@@ -351,11 +355,15 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* en
       n0 -= wb.x; n1 -= wb.y;
       y0 = g.biasvolt * wb.x; y1 = g.biasvolt * wb.y;
     }
-    nws[m] = pack2(n0, n1);
-    ys[m] = pack2(y0, y1);
     wfin[2 * m] = 0.f - n0; wfin[2 * m + 1] = 0.f - n1;
     yfin[2 * m] = y0; yfin[2 * m + 1] = y1;
     live[2 * m] = live[2 * m + 1] = -1;
+    if (!FULL) {     // no output: parked from the start like one that has fired, or the walk would wait for it
+      if (j >= g.jout) { live[2 * m] = 0; n0 = CUDART_INF_F; }
+      if (j + 1 >= g.jout) { live[2 * m + 1] = 0; n1 = CUDART_INF_F; }
+    }
+    nws[m] = pack2(n0, n1);
+    ys[m] = pack2(y0, y1);
   }
   float xprev = g.has_bias ? g.biasvolt : 0.f;
 

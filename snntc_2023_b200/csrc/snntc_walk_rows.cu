@@ -98,7 +98,7 @@ snn_walk_rows_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
       wfin[m] = 0.f; yfin[m] = 0.f;
-      live[m] = row_ok && in_row ? -1 : 0;
+      live[m] = row_ok && j + m < jout ? -1 : 0;   // (padding behind jout never fires: the walk would wait for it)
       if (live[m] == 0) wsum[m] = -CUDART_INF_F;
     }
     float xprev = g.has_bias ? g.biasvolt : 0.f;
