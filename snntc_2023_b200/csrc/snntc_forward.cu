@@ -19,6 +19,7 @@
 
 #include <cooperative_groups.h>
 #include <limits.h>
+#include <math.h>
 #include <math_constants.h>
 
 namespace snntc {
@@ -714,6 +715,7 @@ int launch_walk2(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g
 // aligned, all (I + bias) rows of a 64-output slice plus the list staging buffers within one CTA's shared memory.
 bool walk_smemw_ok(const Geometry& g, const float* w, const LaunchInfo& li, size_t* smem_bytes, int* wmul) {
   if ((g.J != 64 && g.J != 128 && g.J != 256) || (reinterpret_cast<uintptr_t>(w) & 15) != 0) return false;
+  if (g.jout != g.J) return false;      // J is the kernel's output stride too
   const size_t rows_w = (size_t)g.I + g.has_bias;
   const size_t smem = rows_w * 256 + (size_t)kSmemwWarps * 64 * sizeof(WalkEntry);
   if (smem + 2048 > (size_t)li.max_smem_optin || rows_w * 256 >= (1u << 20)) return false;
@@ -744,6 +746,23 @@ int launch_walk2_smemw(const Geometry& g, const WalkEntry* keys_g, const int* nv
   }
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
+}
+
+// What a walk from global memory takes with n warps to an SM, in microseconds for rows of 500 inputs of which half spike: 32 warps
+// run at once, each full wave of them takes `wave`, the last one first + n * warp. Fitted to 100 to 16 000 rows x fan-outs
+// 68 to 1000 (n = 2 to 3500; within 5 % from n = 8 on). What counts is where two of them cross: at 300 to 4096 inputs, half or all
+// of them spiking, 33 to 70 warps of 64 outputs per SM, pairs against quads were 1.15 times as slow on average (700 rows of
+// 784 -> 512: 128 against 103 us all spiking, 74 against 78 half; 1024 of 784 -> 400: 144 against 126), below 32 the quads
+// (300 rows of 500 -> 400: 29 against 35 us). What the rule cannot know is whether an output never fires, for which a warp walks
+// to the end of its list: with one such output in the layer the pairs lose less of the fan-out to it (2450 of 2305 -> 128: 179
+// against 216 us; with none, or many, 337 against 273).
+struct WalkCost { double wave, first, warp; };
+constexpr WalkCost kCostPairs = {27, 20, 0.6};                                        // 64 outputs per warp
+constexpr WalkCost kCostQuads = {43, 29, 0.8};                                        // 128
+constexpr WalkCost kCostLanes[3] = {{25, 20, 0.37}, {36, 21.5, 0.67}, {69, 30, 1.3}};    // 32, 64, 128 by 4-byte loads
+double walk_cost(double n, const WalkCost& c) {
+  const double waves = n > 32 ? ceil(n / 32) - 1 : 0;
+  return waves * c.wave + c.first + (n - 32 * waves) * c.warp;
 }
 
 // Lists of a conv layer are built by per-pixel sorting and merging when the geometry allows it and there is enough to do:
@@ -840,45 +859,30 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     count_launch();
     if (cudaGetLastError() != cudaSuccess) return E_CUDA;
   }
-  // Outputs per lane: more of them amortise the per-step cost (list entry, address, vote) over more
-  // outputs, fewer give more (row, output block) items to spread over the SMs. `cost` is the measured number
-  // of instructions per warp-step, `warps` how many fit on an SM; with few items pick the smallest
-  // estimate of (waves of items) x (cost of a step).
-  auto pick = [&](int unit, const double (&cost)[4], const int (&warps)[4], int top) {
-    int best_c = top;
-    const double items_top = (double)g.R * ((g.J + unit * (1 << top) - 1) / (unit * (1 << top)));
-    if (items_top < 4.0 * li.num_sms * warps[top]) {
-      double best = 0;
-      for (int c = 0; c <= top; ++c) {
-        const int per = unit * (1 << c);
-        const double items = (double)g.R * ((g.J + per - 1) / per);
-        const double slots = (double)li.num_sms * warps[c];
-        const double est = (double)(long)(items / slots + 0.999) * cost[c];
-        if (c == 0 || est < best) { best = est; best_c = c; }
-      }
-    }
-    return best_c;
-  };
-  // Variants of the walk: 1 = output pairs in 64-bit registers, 64 outputs per warp (fan-out <= 64, or few rows:
-  // more warps); 3 = scalar, 2, 4 or 8 consecutive outputs per lane read by 8/16-byte loads (fan-out > 64);
-  // 2 = scalar with outputs lane + 32*m (odd fan-out or unaligned weights).
+  // Variants of the walk from global memory: 1 = output pairs in 64-bit registers, 64 outputs per warp; 3 = four consecutive outputs
+  // per lane, 128 per warp; 2 = outputs lane + 32*m (odd fan-out, weights that are not even 8-byte aligned). More outputs per warp
+  // share a step's list entry, address and vote, fewer make more warps: priced by walk_cost.
   const bool al8 = (g.J % 2 == 0) && (reinterpret_cast<uintptr_t>(w) % 8 == 0);
   const bool al16 = (g.J % 4 == 0) && (reinterpret_cast<uintptr_t>(w) % 16 == 0);
-  const bool al32 = al16 && (g.J % 8 == 0);
-  const double cost[4] = {19.0, 24.0, 39.0, 62.0};
-  const int warps[4] = {48, 32, 32, 16};
-  // (eight outputs per lane exist as a variant but were measured slower than four on every layer of the benchmark
-  // networks -- 1.91 against 1.32 ms on the 2305 x 256 layer: 98 registers, two CTAs per SM -- and are never picked)
-  int jsel = pick(32, cost, warps, g.J <= 32 ? 0 : (g.J <= 64 ? 1 : 2));
-  int variant = 2;
-  if (al8) variant = (g.J <= 64 || jsel < 2) ? 1 : 3;
+  auto cost = [&](int outputs, const WalkCost& c) {
+    return walk_cost((double)g.R * ((g.J + outputs - 1) / outputs) / li.num_sms, c);
+  };
+  int variant = 2, jsel = 0;                           // jsel: 1, 2, 4 outputs per lane (variants 2 and 3)
+  if (al8) {
+    variant = al16 && g.J > 64 && cost(128, kCostQuads) < cost(64, kCostPairs) ? 3 : 1;
+    jsel = variant == 3 ? 2 : 1;
+  } else {
+    for (int c = 1; c < 3; ++c)
+      if (cost(32 << c, kCostLanes[c]) < cost(32 << jsel, kCostLanes[jsel])) jsel = c;
+  }
   if ((opt.walk_layout & 3) != 0) {
     variant = opt.walk_layout & 3;
     if (variant != 2 && !al8) variant = 2;
+    if (variant == 3) jsel = 2;
   }
   const bool stage = (opt.walk_layout & 4) == 0;   // list entries through shared memory (4: straight from global memory)
   if (opt.walk_outputs != 0) jsel = opt.walk_outputs - 1;
-  if (jsel == 3 && !(variant == 3 && al32)) jsel = 2;   // eight outputs per lane exist only as consecutive outputs
+  if (jsel == 3 && !(variant == 3 && al16 && g.J % 8 == 0)) jsel = 2;   // eight outputs per lane exist only as consecutive outputs
   if (variant == 3 && jsel == 2 && !al16) jsel = 1;
   size_t smemw_bytes = 0;
   int smemw_shift = 0;

@@ -88,3 +88,23 @@ def test_padded_weight_rows_of_every_walk(R, I, J, bv, sentinels, positive):
     assert torch.equal(ops.snn_fc_infer(xd, wd, params), out[:R])
     # (a decision within rounding of a tie can leave an output without a spike: 1 of 243 000 of the fp32 oracle at 9000 x 90 x 27)
     assert not positive or float((out[:R] >= 1e5).float().mean()) < 1e-4
+
+
+@pytest.mark.parametrize("R,I,J", [(1400, 40, 200), (1500, 33, 200), (2600, 30, 128), (4900, 30, 128), (9400, 21, 160), (700, 50, 512),
+                                   (1300, 64, 66), (5000, 20, 68), (2500, 90, 1000)])
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_choice_among_the_walks_from_global_memory(R, I, J, offset):
+    """Both sides of the lines between output pairs and four outputs per lane (33 to 70 warps of 64 outputs per SM and beyond,
+    narrow last blocks), with weights that start on a 16-, 4- or 8-byte boundary: the bits of one output per lane."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    x, w = P.make_inputs(R + I + J, (R, I), (I + 1, J), "ref", bias=True)
+    params = O.fc_params(biasvolt=1.0)
+    xd = torch.from_numpy(x).cuda()
+    flat = torch.zeros(w.size + 4, device="cuda")
+    wd = flat[offset:offset + w.size].view(w.shape).copy_(torch.from_numpy(w))
+    assert wd.data_ptr() % 16 == 4 * offset
+    out = ops.snn_fc(xd, wd, params)
+    ref = ops.snn_fc(xd, torch.from_numpy(w).cuda(), params, opts=_lib.options(walk_layout=2, walk_outputs=1))
+    assert torch.equal(out, ref)
+    assert torch.equal(ops.snn_fc_infer(xd, wd, params), out[:R])
