@@ -150,7 +150,10 @@ SNNTC_API int snntc_cv_infer(const float* x_nhwc, const float* w, const float* p
  *                    -(softmax(-y) - onehot) * grad_scale; use loss_scale = grad_scale = 1/B for the mean.
  * snntc_loss_forward / snntc_loss_backward   the same loss as a pair: *loss and *hits (device floats) are WRITTEN, not
  *                    accumulated, in a fixed order of summation; the backward forms grad from y, the labels and the
- *                    incoming gradient *gloss (device).
+ *                    incoming gradient *gloss (device). snntc_loss_forward works through the batch with eight thread
+ *                    blocks; snntc_loss_forward_ws spreads a large one over the GPU, with a workspace of
+ *                    snntc_loss_forward_workspace_bytes(B, J) bytes, 8-byte aligned (0 bytes, and a null pointer will do,
+ *                    where the eight blocks are the faster way).
  * snntc_weight_costs / snntc_weight_cost_grads   snntc_weight_cost for `count` tensors at once (the pointer, rows and
  *                    cols arrays are on the host): *cost is written, colsum (sum of cols floats, device) receives the
  *                    column sums in tensor order; the backward writes gw[k] = *gcost * d cost / d w[k] from them, or adds it to
@@ -169,6 +172,9 @@ SNNTC_API int snntc_loss_ce(const float* y, const long long* labels, float* grad
                             float loss_scale, float grad_scale, void* stream);
 SNNTC_API int snntc_loss_forward(const float* y, const long long* labels, float* loss, float* hits, int B, int J,
                                  float loss_scale, void* stream);
+SNNTC_API size_t snntc_loss_forward_workspace_bytes(int B, int J);
+SNNTC_API int snntc_loss_forward_ws(const float* y, const long long* labels, float* loss, float* hits, int B, int J,
+                                    float loss_scale, void* workspace, size_t workspace_bytes, void* stream);
 SNNTC_API int snntc_loss_backward(const float* y, const long long* labels, const float* gloss, float* grad, int B, int J,
                                   float grad_scale, void* stream);
 SNNTC_API size_t snntc_weight_costs_workspace_bytes(int count, const int* rows, const int* cols);

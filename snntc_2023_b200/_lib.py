@@ -37,6 +37,8 @@ SYMBOLS = {
     "snntc_encode": (_INT, [_F, _F, _SZ, ctypes.c_float, _INT, _F]),
     "snntc_loss_ce": (_INT, [_F, _F, _F, _F, _INT, _INT, ctypes.c_float, ctypes.c_float, _F]),
     "snntc_loss_forward": (_INT, [_F, _F, _F, _F, _INT, _INT, ctypes.c_float, _F]),
+    "snntc_loss_forward_workspace_bytes": (_SZ, [_INT, _INT]),
+    "snntc_loss_forward_ws": (_INT, [_F, _F, _F, _F, _INT, _INT, ctypes.c_float, _F, _SZ, _F]),
     "snntc_loss_backward": (_INT, [_F, _F, _F, _F, _INT, _INT, ctypes.c_float, _F]),
     "snntc_weight_costs_workspace_bytes": (_SZ, [_INT, _F, _F]),
     "snntc_weight_costs": (_INT, [_INT, _F, _F, _F, ctypes.c_float, ctypes.c_float, _F, _F, _F, _SZ, _F]),

@@ -360,8 +360,10 @@ struct LossFunction : torch::autograd::Function<LossFunction> {
     const int B = to_int(y.size(0), "loss_func"), J = to_int(y.size(1), "loss_func");
     const c10::cuda::CUDAGuard guard(y.device());
     const Tensor loss = empty_like_dev({}, y), hits = empty_like_dev({}, y);
-    check(snntc_loss_forward(ptr(y), (const long long*)label.data_ptr<int64_t>(), ptr(loss), ptr(hits), B, J, 1.0f / B, stream_of(y)),
-          "loss_func");
+    const size_t bytes = snntc_loss_forward_workspace_bytes(B, J);
+    const Tensor ws = bytes ? workspace(bytes, y) : Tensor();
+    check(snntc_loss_forward_ws(ptr(y), (const long long*)label.data_ptr<int64_t>(), ptr(loss), ptr(hits), B, J, 1.0f / B,
+                                bytes ? ws.data_ptr() : nullptr, bytes, stream_of(y)), "loss_func");
     ctx->save_for_backward({y, label});
     ctx->mark_non_differentiable({hits});
     return {loss, hits};

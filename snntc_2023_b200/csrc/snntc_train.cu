@@ -173,10 +173,12 @@ __global__ void sgdm_kernel(float* __restrict__ w, const float* __restrict__ g, 
   }
 }
 
-// ---- loss of a whole batch in one launch, no zeroed accumulators: one cluster of eight CTAs, G lanes per sample
-// (16 for up to 16 classes, else 32), every CTA's partial sums added over distributed shared memory in rank order, so
-// the loss is the same bits every run. Bound by latency (a few rounds of loads and shuffles per group): against the
-// pair of a zero fill and an atomic accumulation it takes two launches off a step.
+// ---- loss of a whole batch, no zeroed accumulators, in a fixed order of summation: the same bits every run. G lanes per sample
+// (16 for up to 16 classes, else 32).
+// Small batches: one launch of one cluster of eight CTAs, whose partial sums are added over distributed shared memory in rank
+// order. Bound by latency (a few rounds of loads and shuffles per group): against the pair of a zero fill and an atomic
+// accumulation it takes a launch off a step.
+// Large ones (loss_in_one_cluster): CTAs over the whole GPU, each leaves its sum in a workspace, and a second launch adds them.
 constexpr int kLossThreads = 512;
 constexpr int kLossCluster = 8;
 
@@ -238,17 +240,13 @@ __device__ __forceinline__ float2 cluster_sum(float a, float b) {
   return sum;
 }
 
+// (loss, hits) of the samples that this thread's group of G lanes takes, `groups` in step: in lane 0 of the group
 template <int G>
-__global__ void __cluster_dims__(kLossCluster, 1, 1) __launch_bounds__(kLossThreads)
-loss_fwd_kernel(const float* y, const long long* labels, float* __restrict__ loss,
-                float* __restrict__ hits, int B, int J, float lscale) {
-  chain_wait();
-  chain_next();
+__device__ __forceinline__ float2 loss_of_samples(const float* y, const long long* labels, int B, int J, float lscale, int groups) {
   const int gl = threadIdx.x % G;
-  const int groups = kLossCluster * kLossThreads / G;
   float loss_acc = 0.f, hit_acc = 0.f;
   for (int b0 = 0; b0 < B; b0 += groups) {
-    const int b = b0 + (blockIdx.x * kLossThreads + threadIdx.x) / G;
+    const int b = b0 + (blockIdx.x * blockDim.x + threadIdx.x) / G;
     const bool ok = b < B;                       // (shuffles run with all lanes: a group without a sample repeats the last)
     const float* row = y + (size_t)(ok ? b : B - 1) * J;
     const RowStats s = row_stats<G>(row, J, gl);
@@ -261,8 +259,45 @@ loss_fwd_kernel(const float* y, const long long* labels, float* __restrict__ los
       hit_acc += (s.amin == lab) ? 1.0f : 0.0f;
     }
   }
-  const float2 sum = cluster_sum(loss_acc, hit_acc);
+  return make_float2(loss_acc, hit_acc);
+}
+
+template <int G>
+__global__ void __cluster_dims__(kLossCluster, 1, 1) __launch_bounds__(kLossThreads)
+loss_fwd_kernel(const float* y, const long long* labels, float* __restrict__ loss, float* __restrict__ hits, int B, int J,
+                float lscale) {
+  chain_wait();
+  chain_next();
+  const float2 mine = loss_of_samples<G>(y, labels, B, J, lscale, kLossCluster * kLossThreads / G);
+  const float2 sum = cluster_sum(mine.x, mine.y);
   if (blockIdx.x == 0 && threadIdx.x == 0) { *loss = sum.x; *hits = sum.y; }
+}
+
+constexpr int kLossWideThreads = 256;
+constexpr int kLossWideCtas = 592;      // four per SM of a B200 at most; fixed, so that the order of summation is
+
+template <int G>
+__global__ void __launch_bounds__(kLossWideThreads)
+loss_partial_kernel(const float* y, const long long* labels, float2* __restrict__ partial, int B, int J, float lscale) {
+  chain_wait();
+  chain_next();
+  const float2 mine = loss_of_samples<G>(y, labels, B, J, lscale, (int)gridDim.x * (kLossWideThreads / G));
+  const float2 sum = cluster_sum(mine.x, mine.y);     // (every CTA is a cluster of its own)
+  if (threadIdx.x == 0) partial[blockIdx.x] = sum;
+}
+
+__global__ void __launch_bounds__(kLossWideThreads)
+loss_total_kernel(const float2* partial, int n, float* __restrict__ loss, float* __restrict__ hits) {
+  chain_wait();
+  chain_next();
+  float2 mine = make_float2(0.f, 0.f);
+  for (int k = threadIdx.x; k < n; k += kLossWideThreads) {
+    const float2 p = ld_plain(partial + k);
+    mine.x += p.x;
+    mine.y += p.y;
+  }
+  const float2 sum = cluster_sum(mine.x, mine.y);
+  if (threadIdx.x == 0) { *loss = sum.x; *hits = sum.y; }
 }
 
 // grad_y = -(softmax(-y) - onehot) * gscale * (*gloss): the softmax again from y instead of a gradient kept by the forward
@@ -466,6 +501,21 @@ size_t cost_partial_floats(const CostTensors& c) {
   return n;
 }
 
+int loss_lanes(int J) { return J <= 16 ? 16 : 32; }
+int loss_wide_ctas(int B, int J) {
+  const long long ctas = ((long long)B * loss_lanes(J) + kLossWideThreads - 1) / kLossWideThreads;
+  return ctas < kLossWideCtas ? (int)ctas : kLossWideCtas;
+}
+// One cluster takes about 0.9 us for a round of its 4096 lanes and 0.1 us for each load of a lane in it, two launches over the whole
+// GPU 6.5 us and up: they cross at 1024 samples of 10 classes (6.2 us in one cluster, 6.5 in two launches; 4096: 17.5 and 7.0), 256 of
+// 300 (6.2, 6.5) and 128 of 1000 (6.6, 7.2; 256: 10.2, 7.6; 1024: 32 and 8.6; 65 536: 2850 and 95).
+bool loss_in_one_cluster(int B, int J) {
+  const int G = loss_lanes(J);
+  constexpr int lanes = kLossCluster * kLossThreads;
+  const long long rounds = ((long long)B * G + lanes - 1) / lanes;
+  return rounds * (9 + (J + G - 1) / G) <= 42;
+}
+
 int done() {
   snntc::count_launch();
   return cudaGetLastError() == cudaSuccess ? SNNTC_OK : SNNTC_E_CUDA;
@@ -497,6 +547,26 @@ int snntc_loss_forward(const float* y, const long long* labels, float* loss, flo
   if (B <= 0 || J <= 0) return SNNTC_E_SHAPE;
   if (J <= 16) (void)launch_chained(loss_fwd_kernel<16>, kLossCluster, kLossThreads, 0, (cudaStream_t)stream, 0, y, labels, loss, hits, B, J, loss_scale);
   else (void)launch_chained(loss_fwd_kernel<32>, kLossCluster, kLossThreads, 0, (cudaStream_t)stream, 0, y, labels, loss, hits, B, J, loss_scale);
+  return done();
+}
+
+size_t snntc_loss_forward_workspace_bytes(int B, int J) {
+  if (B <= 0 || J <= 0 || loss_in_one_cluster(B, J)) return 0;
+  return (size_t)loss_wide_ctas(B, J) * sizeof(float2);
+}
+
+int snntc_loss_forward_ws(const float* y, const long long* labels, float* loss, float* hits, int B, int J, float loss_scale,
+                          void* workspace, size_t workspace_bytes, void* stream) {
+  const size_t need = snntc_loss_forward_workspace_bytes(B, J);
+  if (need == 0) return snntc_loss_forward(y, labels, loss, hits, B, J, loss_scale, stream);
+  if (!y || !labels || !loss || !hits || !workspace) return SNNTC_E_NULL;
+  if (workspace_bytes < need) return SNNTC_E_WORKSPACE;
+  const int ctas = loss_wide_ctas(B, J);
+  float2* partial = static_cast<float2*>(workspace);
+  if (J <= 16) (void)launch_chained(loss_partial_kernel<16>, ctas, kLossWideThreads, 0, (cudaStream_t)stream, 0, y, labels, partial, B, J, loss_scale);
+  else (void)launch_chained(loss_partial_kernel<32>, ctas, kLossWideThreads, 0, (cudaStream_t)stream, 0, y, labels, partial, B, J, loss_scale);
+  if (done() != SNNTC_OK) return SNNTC_E_CUDA;
+  (void)launch_chained(loss_total_kernel, 1, kLossWideThreads, 0, (cudaStream_t)stream, 0, partial, ctas, loss, hits);
   return done();
 }
 

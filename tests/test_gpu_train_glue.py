@@ -44,6 +44,29 @@ def test_loss_matches_cross_entropy_on_negated_logits(B, J):
     assert abs(float(train.loss_func(y, onehot)) - float(ref)) <= 1e-5 * max(1.0, abs(float(ref)))
 
 
+@pytest.mark.parametrize("B,J,launches", [(1024, 10, 1), (1061, 10, 2), (20000, 16, 2), (70001, 2, 2), (384, 33, 1), (1000, 33, 2),
+                                          (128, 1000, 1), (129, 1001, 2), (3000, 1000, 2), (65, 9999, 2)])
+def test_loss_of_large_batches_is_spread_over_the_gpu(B, J, launches):
+    """Both sides of the line between one cluster of CTAs and two launches: the loss in float64, the hits, and the same bits
+    in a second run. 32-bit sums of B positive terms in groups: relative error well below 1e-6 * log2(B)."""
+    import torch
+    import torch.nn.functional as F
+    from snntc_2023_b200 import _lib, train
+    g = torch.Generator("cuda").manual_seed(B + J)
+    y = torch.rand(B, J, device="cuda", generator=g) * 3 + 1
+    y[torch.rand(B, J, device="cuda", generator=g) < 0.3] = 1e5
+    lab = torch.where(torch.rand(B, device="cuda", generator=g) < 0.5, y.argmin(1), torch.randint(0, J, (B,), device="cuda", generator=g))
+    y[torch.arange(B, device="cuda"), lab] = y.gather(1, lab[:, None]).clamp(max=9.0)[:, 0]
+    before = _lib.load().snntc_launch_count()
+    loss, hits = train.loss_func(y, lab, with_hits=True)
+    assert _lib.load().snntc_launch_count() - before == launches
+    ref = F.cross_entropy(-y.double(), lab)
+    assert abs(float(loss) - float(ref)) <= 1e-5 * float(ref)
+    assert int(hits) == int((y.argmin(1) == lab).sum())
+    again = train.loss_func(y, lab, with_hits=True)
+    assert torch.equal(loss, again[0]) and torch.equal(hits, again[1])
+
+
 def test_constraint_cost_matches_reference_formula():
     import torch
     from snntc_2023_b200 import train
