@@ -9,8 +9,8 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/engine.h>
 #include <torch/csrc/autograd/functions/accumulate_grad.h>
-#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/graph_task.h>
 
 #include <algorithm>
@@ -519,15 +519,15 @@ void backward(const Tensor& objective, const Tensor& one, const std::vector<Tens
   };
   {
     const Leave leave{&f};
-    Tensor root = objective;
     if (objective.requires_grad()) {
       auto node = std::make_shared<FoldRoot>();
       node->fold = &f;
+      node->add_input_metadata(objective);
       node->add_next_edge(torch::autograd::impl::gradient_edge(objective));
-      root = objective.detach();
-      torch::autograd::set_history(root, node);
+      torch::autograd::Engine::get_default_engine().execute({torch::autograd::Edge(std::move(node), 0)}, {one}, false, false, true);
+    } else {
+      torch::autograd::backward({objective}, {one});     // raises
     }
-    torch::autograd::backward({root}, {one});
   }
   for (const Fold::Pending& p : f.pending) {
     variable_list to;
