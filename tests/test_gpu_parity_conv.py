@@ -115,15 +115,16 @@ VARIANT_CASES = [c for c in CONV_CASES if c[0] in (44, 48, 51, 82, 84, 86, 92, 9
 
 @pytest.mark.parametrize("case", VARIANT_CASES, ids=_ids)
 def test_conv_list_builders_agree(case):
-    """Sorted lists by per-field radix sort and by per-pixel sort + merges: the same lists up to the order of equal
-    inputs, which can move the last bits of a sum but not a decision on a well-conditioned output."""
+    """Sorted lists by per-field bucket sort and by per-pixel sort + merges: the same lists up to the order of equal
+    inputs, which can move the last bits of a sum but not a decision on a well-conditioned output. (At these sizes the
+    library's own choice is the bucket sort; where it is the merges: test_conv_on_merged_lists_by_default.)"""
     import torch
     from snntc_2023_b200 import _lib, ops
     seed, B, H, W, C, Kh, Kw, Sh, Sw, Kc, bv, padding, dist = case
     x, w, params, xd, wd, out, outc, (pt, pl, Nh, Nw) = _run_conv(*case)
     a = ops.snn_cv(xd, wd, params, pt, pl, Nh, Nw, opts=_lib.options(list_builder=1)).cpu().numpy()
     b = ops.snn_cv(xd, wd, params, pt, pl, Nh, Nw, opts=_lib.options(list_builder=2)).cpu().numpy()
-    assert np.array_equal(outc, b), "the default list builder of a 3x3 stride-1 layer is the merging one"
+    assert np.array_equal(outc, b), "no equal inputs in these cases: both builders, the same lists"
     fa, fb = a[:B] < 1e5 - 0.1, b[:B] < 1e5 - 0.1
     assert (fa != fb).sum() <= 1e-4 * fa.size
     both = fa & fb
@@ -138,13 +139,35 @@ def test_conv_list_builders_agree(case):
         assert np.array_equal(c, b), "pieces per merge: %d" % (1 << k)
 
 
+@pytest.mark.parametrize("B,H,W,C,Kc,bv", [(8, 32, 32, 64, 12, 1.0), (33, 16, 15, 96, 8, 0.0), (20, 14, 14, 256, 8, 1.0), (5, 24, 25, 512, 4, 1.0)])
+def test_conv_on_merged_lists_by_default(B, H, W, C, Kc, bv):
+    """Layers large enough that the library merges pixel runs by itself (from 4.4 M inputs over all fields, more from 170
+    channels on): the bits of the merging builder, the protocol of the oracle."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    case = (B + C, B, H, W, C, 3, 3, 1, 1, Kc, bv, "SAME", "ref")
+    x, w, params, xd, wd, out, outc, (pt, pl, Nh, Nw) = _run_conv(*case)
+    line = 30000 * torch.cuda.get_device_properties(0).multi_processor_count * max(1.0, C / 170)
+    if B * Nh * Nw * 9 * C <= line:
+        pytest.skip("below the line on this GPU")
+    launches = _lib.load().snntc_launch_count()
+    ops.snn_cv(xd, wd, params, pt, pl, Nh, Nw)
+    assert _lib.load().snntc_launch_count() - launches >= 4          # pixel runs, row runs, field lists, walk
+    merged = ops.snn_cv(xd, wd, params, pt, pl, Nh, Nw, opts=_lib.options(list_builder=2))
+    assert torch.equal(out, merged)
+    keep = slice(0, 2)                                               # (the oracle takes two images of the batch)
+    o32, o64 = O.cv_forward(x[keep], w, params, "f32"), O.cv_forward(x[keep], w, params, "f64")
+    P.check_forward(outc[:2], outc[B:B + 2], o32, o64, rows=P.im2col_rows(x[keep], 3, 3, 1, 1, "SAME"), what="merged lists %s" % (case,))
+
+
 SMALL_ROW_CASES = [c for c in CONV_CASES if c[5] * c[6] * c[4] <= 256]
 
 
 @pytest.mark.parametrize("case", SMALL_ROW_CASES, ids=_ids)
 def test_conv_small_row_builder_matches_the_row_sort(case):
-    """Rows of at most 256 inputs sorted by the register network and by the per-row radix sort: both order equal
-    inputs by source index, so the lists and with them every output bit are the same."""
+    """Rows of at most 64 inputs sorted by the register network and by the per-row bucket sort: both order equal
+    inputs by source index, so the lists and with them every output bit are the same. (Longer rows: the bucket sort
+    both times; their lists are checked in test_gpu_row_sort.py.)"""
     from snntc_2023_b200 import _lib, ops
     x, w, params, xd, wd, out, outc, (pt, pl, Nh, Nw) = _run_conv(*case)
     a = ops.snn_cv(xd, wd, params, pt, pl, Nh, Nw, opts=_lib.options(list_builder=1)).cpu().numpy()

@@ -166,9 +166,10 @@ def test_dense_repeatable():
 
 @pytest.mark.parametrize("I", [1, 31, 32, 33, 64, 70, 100, 147, 170, 200, 255, 256])
 def test_dense_short_rows_by_the_register_network_match_the_row_sort(I):
-    """Rows of at most 256 inputs are sorted by a network in registers; the per-row radix sort forced through the
-    measurement build gives the same lists (equal inputs in index order), hence the same bits. Inputs include
-    ties and values that never spike."""
+    """Rows of at most 64 inputs are sorted by a network in registers; the per-row bucket sort forced through the
+    measurement build gives the same lists (equal inputs in index order), hence the same bits. Longer rows go through the
+    bucket sort whichever is named (their lists are checked in test_gpu_row_sort.py). Inputs include ties and values that
+    never spike."""
     import torch
     from snntc_2023_b200 import _lib, ops
     rng = np.random.default_rng(I)

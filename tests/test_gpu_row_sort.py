@@ -79,3 +79,37 @@ def test_receptive_fields(B, H, W, C, K, S):
     ws = ops.cv_forward_workspace(xd, w, params, Nh, Nw)
     ops.snn_cv(xd, w, params, pt, pl, Nh, Nw, opts=_lib.options(forward_parts=1, list_builder=1), workspace=ws)
     _check(ws, P.im2col_rows(x, K, K, S, S, "SAME"), 4, "fields")
+
+
+@pytest.mark.parametrize("R,I", [(7, 65), (5, 70), (3, 147), (6, 200), (9, 256), (2500, 65), (2400, 147), (2400, 256), (2400, 511),
+                                 (5, 1), (2500, 31), (11, 33), (2500, 64)])
+@pytest.mark.parametrize("kind", ["spread", "equal", "few", "outlier"])
+def test_short_dense_rows(R, I, kind):
+    """65 to 256 inputs, a CTA per row and (from 16 rows per SM on) a warp per row; up to 64, the register network, which is the
+    library's own choice there."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    rng = np.random.default_rng(R + I)
+    x = _values(rng, (R, I), kind)
+    w = torch.zeros((I + 1, 4), device="cuda")
+    for builder in (0, 1) if I > 64 else (0, 1, 3):
+        ws = ops.fc_forward_workspace(R, I, 4, "cuda")
+        ops.snn_fc(torch.from_numpy(x).cuda(), w, O.fc_params(biasvolt=1.0), opts=_lib.options(forward_parts=1, list_builder=builder), workspace=ws)
+        _check(ws, x, 4, "short rows %d %s, builder %d" % (I, kind, builder))
+
+
+@pytest.mark.parametrize("B,H,W,C,K,S", [(3, 31, 30, 70, 3, 1), (10, 32, 31, 16, 7, 2), (3, 29, 30, 7, 9, 1)])
+def test_many_receptive_fields(B, H, W, C, K, S):
+    """A warp per row of more than 512 inputs, which only receptive fields get (630, 784 and 567 inputs, at least 2368 rows)."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    rng = np.random.default_rng(C + K)
+    x = _values(rng, (B, H, W, C), "spread")
+    params = O.cv_params(K, K, S, S, "SAME", 1.0)
+    pt, pl, Nh, Nw = ops.conv_geometry(H, W, K, K, S, S, "SAME")
+    assert 512 < K * K * C <= 1024 and B * Nh * Nw >= 2368
+    w = torch.zeros((K * K * C + 1, 4), device="cuda")
+    xd = torch.from_numpy(x).cuda()
+    ws = ops.cv_forward_workspace(xd, w, params, Nh, Nw)
+    ops.snn_cv(xd, w, params, pt, pl, Nh, Nw, opts=_lib.options(forward_parts=1, list_builder=1), workspace=ws)
+    _check(ws, P.im2col_rows(x, K, K, S, S, "SAME"), 4, "fields")
