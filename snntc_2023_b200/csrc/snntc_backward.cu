@@ -11,6 +11,7 @@
 // NHWC image. dW splits the row dimension over CTAs and a second kernel adds the partial tiles in a
 // fixed order, so results are reproducible run to run.
 #include "snntc_common.cuh"
+#include "snntc_ptx.cuh"
 
 #include <math_constants.h>
 #include <math.h>
@@ -89,28 +90,6 @@ __global__ void snn_u_kernel(const float* grad, const float* out, float* __restr
     for (int d = 16; d >= 1; d >>= 1) nz += __shfl_xor_sync(0xffffffffu, nz, d);
     if ((threadIdx.x & 31) == 0 && nz != 0u) atomicAdd(nz_count, nz);
   }
-}
-
-// acc += [x <= y] * u * w as one compare and one predicated FMA
-__device__ __forceinline__ void masked_fma(float& acc, float x, float y, float u, float w) {
-  asm("{\n\t.reg .pred p;\n\tsetp.le.f32 p, %1, %2;\n\t@p fma.rn.f32 %0, %3, %4, %0;\n\t}"
-      : "+f"(acc) : "f"(x), "f"(y), "f"(u), "f"(w));
-}
-
-// Two-lane FP32 arithmetic of sm_100 (one issue slot for two IEEE single-precision results; each lane
-// rounds exactly like the scalar instruction). A pair lives in one 64-bit register: low word = lane 0.
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
 }
 
 // ------------------------------------------------------------------------------------------- dX
@@ -463,11 +442,6 @@ snn_dx_wide_kernel(const DxGate gate, const Geometry g, const float* uv, const f
 // half-rate compare/min pipe. Scaling by s is exact unless it underflows, and the bound on (y-x) needs
 // x >= -MAX; snn_u_kernel checks the ranges of the call's tensors and raises *exact_flag otherwise, in
 // which case the tiles stay unscaled (s = 1) and the clamp is an explicit max(., 0).
-__device__ __forceinline__ float add_sat(float a, float b) {
-  float r;
-  asm("add.rn.sat.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-  return r;
-}
 
 template <bool VEC>   // VEC: J % 4 == 0, the y/u tiles are fetched with 16-byte loads
 __global__ void __launch_bounds__(kBwdThreads, 3)
@@ -668,11 +642,6 @@ snn_dw_kernel(const Geometry g, const float* uv, const float* x,
 // Whether output (r,j) carries a gradient is the same question for all lanes, so rows without one are skipped by
 // a warp-uniform branch. Same arithmetic per element as the other dW kernels (saturating FMA of the scaled difference, FMA with
 // -u/s), same exactness rule.
-__device__ __forceinline__ float fma_sat(float a, float b, float c) {
-  float r;
-  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
 
 template <int JB>
 __global__ void __launch_bounds__(kBwdThreads)

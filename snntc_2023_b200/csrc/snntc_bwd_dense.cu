@@ -21,6 +21,7 @@
 // Measured (B200, dX + dW with the u kernel, before -> now): 784 -> 400 at 32 samples 85 -> 16 us, at 256: 98 -> 35, at 1024: 142 -> 99;
 // 4096 -> 512 at 256: 185 -> 123; 25 088 -> 1024 at 64: 550 -> 330.
 #include "snntc_common.cuh"
+#include "snntc_ptx.cuh"
 
 #include <cooperative_groups.h>
 #include <math_constants.h>
@@ -43,30 +44,6 @@ constexpr int kWarpFloats = 2 * 3 * kTile;                              // two b
 constexpr size_t kSmemBytes = (size_t)kWarps * kWarpFloats * sizeof(float);
 static_assert(kT * kPad <= kWarpFloats, "the reduction tile lies over the warp's own staging buffers");
 
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ float fma_sat(float a, float b, float c) {
-  float r;
-  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-// acc += [x <= y] * u * w as one compare and one predicated FMA
-__device__ __forceinline__ void masked_fma(float& acc, float x, float y, float u, float w) {
-  asm("{\n\t.reg .pred p;\n\tsetp.le.f32 p, %1, %2;\n\t@p fma.rn.f32 %0, %3, %4, %0;\n\t}"
-      : "+f"(acc) : "f"(x), "f"(y), "f"(u), "f"(w));
-}
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 // 4- and 16-byte asynchronous copies; `ok` false writes zeros and reads nothing
 __device__ __forceinline__ void copy4(unsigned dst, const float* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
@@ -74,9 +51,6 @@ __device__ __forceinline__ void copy4(unsigned dst, const float* src, bool ok) {
 __device__ __forceinline__ void copy16(unsigned dst, const float* src, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 struct DensePlan {
   int cluster;                             // CTAs per cluster

@@ -28,6 +28,7 @@
 // of them 731 -> 506; 65 536 of 325 x 64 at stride 2: 201 -> 146, 135 -> 82. Without VEC, 131 072 of 820 x 128 against the dense
 // tile: 2012 -> 1469, 1998 -> 734.
 #include "snntc_common.cuh"
+#include "snntc_ptx.cuh"
 
 #include <math_constants.h>
 #include <algorithm>
@@ -39,35 +40,14 @@ namespace {
 
 constexpr int kRS = 16;          // rows r per stage
 
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ float fma_sat(float a, float b, float c) {
-  float r;
-  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem_src) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(gmem_src) : "memory");
 }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // VEC: C and J multiples of four, 16-byte aligned tensors; a lane holds QL quadruples of fan-in rows, else QL pairs
 template <int QL, bool VEC, int NW>
@@ -206,7 +186,7 @@ snn_dw_skip_kernel(const Geometry g, const float* uv, const float* x,
         else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);   // no spike value, no gradient
       }
     }
-    cp_async_commit();
+    copies_commit();
   };
 
   // acc[c][jj][h]: fan-in rows i0 + CW*(lane + 32c) + 2h, +1 (one 64-bit pair), output channel j0 + 4*warp + jj
@@ -274,14 +254,14 @@ snn_dw_skip_kernel(const Geometry g, const float* uv, const float* x,
   fill_rowinfo((kDepth - 1) & 1, r_begin + (kDepth - 1) * kRS);
   int it = 0;
   for (int rb = r_begin; rb < r_end; rb += kRS, ++it) {
-    cp_async_wait<kDepth - 2>();
+    copies_wait<kDepth - 2>();
     __syncthreads();
     issue((it + kDepth - 1) % kDepth, (it + kDepth - 1) & 1, rb + (kDepth - 1) * kRS);
     fill_rowinfo((it + kDepth) & 1, rb + kDepth * kRS);
     if (fast) reduce_stage(it % kDepth, std::true_type{});
     else reduce_stage(it % kDepth, std::false_type{});
   }
-  cp_async_wait<0>();
+  copies_wait<0>();
 
   float* __restrict__ dst = partial + (size_t)blockIdx.z * Itot * J;
   const int j = j0 + 4 * warp;

@@ -30,6 +30,7 @@
 // whole taps, taps_per_tile = 640 / C of them; the bias row (x = biasvolt for every r) is a sum per output channel
 // that the CTAs of the last fan-in tile keep beside their tile.
 #include "snntc_common.cuh"
+#include "snntc_ptx.cuh"
 
 #include <cuda.h>
 #include <math_constants.h>
@@ -46,26 +47,6 @@ constexpr int kMaxTileFloats = 640;
 constexpr int kMaxDepth = 8;     // stages in flight at most
 constexpr long long kWaitClocks = 2000000000LL;   // SM clocks a thread waits for a stage's copies (about a second)
 __device__ unsigned g_dw_copy_timeouts = 0u;        // CTAs that gave up waiting since the library was loaded
-
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ float fma_sat(float a, float b, float c) {
-  float r;
-  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 // x box: coordinates (channel, column, row, image); the channel coordinate is always 0 (16-byte aligned)
 __device__ __forceinline__ void tma_load_4d(unsigned dst, const CUtensorMap* map, unsigned bar, int c, int w, int h, int b) {

@@ -14,18 +14,13 @@
 // by the register tiles, 89 with one output per load, 62 with four; 200 704 pixels, 64 outputs: 3914, 439, 234; 65 536 x 8
 // channels, 3x3, 64 outputs: 291, 187, 140.
 #include "snntc_common.cuh"
+#include "snntc_ptx.cuh"
 
 namespace snntc {
 
 namespace {
 
 constexpr int kThreads = 256;
-
-// acc += [x <= y] * u * w as one compare and one predicated FMA
-__device__ __forceinline__ void masked_fma(float& acc, float x, float y, float u, float w) {
-  asm("{\n\t.reg .pred p;\n\tsetp.le.f32 p, %1, %2;\n\t@p fma.rn.f32 %0, %3, %4, %0;\n\t}"
-      : "+f"(acc) : "f"(x), "f"(y), "f"(u), "f"(w));
-}
 
 // CT: channels held per lane. V4: a lane takes four outputs at a time by 16-byte loads (J a multiple of 4, y, u and w aligned);
 // `lanes` = 4, 8, 16 or 32 of them take a field, 32 / lanes fields at once.

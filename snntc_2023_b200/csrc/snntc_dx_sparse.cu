@@ -18,6 +18,7 @@
 // The terms of a sum are added in the same order as in the dense kernel (tap-major, j ascending; the skipped ones
 // are +-0), so the two kernels give the same bits.
 #include "snntc_common.cuh"
+#include "snntc_ptx.cuh"
 
 #include <math_constants.h>
 
@@ -72,12 +73,6 @@ __global__ void snn_weight_transpose_kernel(const float* w, float* __restrict__ 
     const int tap = (int)(tj / J);
     wt[e] = ld_plain(w + ((size_t)tap * C + c) * J + j);
   }
-}
-
-// acc += [x <= y] * u * w as one compare and one predicated FMA
-__device__ __forceinline__ void masked_fma(float& acc, float x, float y, float u, float w) {
-  asm("{\n\t.reg .pred p;\n\tsetp.le.f32 p, %1, %2;\n\t@p fma.rn.f32 %0, %3, %4, %0;\n\t}"
-      : "+f"(acc) : "f"(x), "f"(y), "f"(u), "f"(w));
 }
 
 // CPL channels per lane (4, 8 or 16), LPP lanes per pixel (a power of two, LPP * CPL >= C): a warp holds

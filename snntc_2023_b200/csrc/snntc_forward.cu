@@ -42,11 +42,6 @@ __device__ __forceinline__ int uniform_warp_index() { return __shfl_sync(0xfffff
 
 // ------------------------------------------------------------------------------------------- walk
 
-// Smallest of three float bit patterns compared as signed integers. For the sign test of the walk that is all
-// that is needed: the result is <= 0 exactly when one of the floats is negative, -0 or +0 (negative floats are
-// negative integers, +0 is 0, positive floats and NaN patterns with a clear sign bit are positive integers).
-__device__ __forceinline__ int imin3(int a, int b, int c) { return min(min(a, b), c); }
-
 // How close to zero q = ysum - x*wsum may be before the sign of q stops deciding. The reference compares
 // ysum against the ROUNDED product x*wsum (ratio_gt / ratio_le below), so it can see "ysum <= x*wsum" while the
 // exact difference is still positive by up to half an ulp of the product, and the other way round for the test
@@ -601,8 +596,6 @@ constexpr int kSmemwThreads = 1024;
 constexpr int kSmemwWarps = kSmemwThreads / 32;
 constexpr long long kSmemwWaitClocks = 2000000000LL;   // SM clocks a CTA waits for its weight copies (about a second)
 __device__ unsigned g_walk_copy_timeouts = 0u;          // CTAs that gave up waiting since the library was loaded
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 template <bool STAGE>
 __global__ void __launch_bounds__(kSmemwThreads, 1)

@@ -1,0 +1,58 @@
+// The few instructions that the compiler has no spelling for, shared by the kernels: two-lane and saturating FP32 arithmetic, the
+// compare with a predicated FMA, shared-memory addresses, and the groups of asynchronous copies.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace snntc {
+
+// sm_100 has two-lane FP32 add / sub / fma on 64-bit register pairs: one issue slot, two results, each rounded exactly
+// like the scalar instruction. Low word = first lane.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ void unpack2i(uint64_t v, int& lo, int& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// clamped to [0, 1], NaN to 0
+__device__ __forceinline__ float add_sat(float a, float b) {
+  float r;
+  asm("add.rn.sat.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float fma_sat(float a, float b, float c) {
+  float r;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// acc += [x <= y] * u * w as one compare and one predicated FMA
+__device__ __forceinline__ void masked_fma(float& acc, float x, float y, float u, float w) {
+  asm("{\n\t.reg .pred p;\n\tsetp.le.f32 p, %1, %2;\n\t@p fma.rn.f32 %0, %3, %4, %0;\n\t}"
+      : "+f"(acc) : "f"(x), "f"(y), "f"(u), "f"(w));
+}
+
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+// asynchronous copies of a thread (cp.async) in groups
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+}  // namespace snntc

@@ -1,6 +1,7 @@
-// What the walk kernels share: the reference's fire comparisons, the causal-set size, two-lane FP32 arithmetic.
+// What the walk kernels share: the reference's fire comparisons, the causal-set size, the integer minimum of a step's sign test.
 #pragma once
 #include "snntc_common.cuh"
+#include "snntc_ptx.cuh"
 
 namespace snntc {
 
@@ -29,29 +30,9 @@ __device__ __forceinline__ int entries_below(const WalkEntry* ents, int n, float
   return lo;
 }
 
-// sm_100 has two-lane FP32 add / sub / fma on 64-bit register pairs: one issue slot, two results, each rounded exactly
-// like the scalar instruction. Low word = first lane.
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ void unpack2i(uint64_t v, int& lo, int& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
+// Smallest of three float bit patterns compared as signed integers. For the sign test of the walks that is all that is needed:
+// the result is <= 0 exactly when one of the floats is negative, -0 or +0 (negative floats are negative integers, +0 is 0,
+// positive floats and NaN patterns with a clear sign bit are positive integers).
+__device__ __forceinline__ int imin3(int a, int b, int c) { return min(min(a, b), c); }
 
 }  // namespace snntc

@@ -37,14 +37,10 @@ struct RingWarp {
   unsigned off[kListRing][kBlock];                 // element offset of the weight row
 };
 
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 template <int BYTES>
 __device__ __forceinline__ void copy_async(unsigned dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
 }
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // One output of one lane. wsum = sum w - theta and ysum = sum w*x run on; an output that has fired keeps its sums in fin and
 // its running weight sum at -inf, where q stays +inf.

@@ -31,8 +31,6 @@ struct Shape {
   static constexpr int block = LPR >= 16 ? 32 : 16;   // list entries staged per row
 };
 
-__device__ __forceinline__ int imin3(int a, int b, int c) { return min(min(a, b), c); }
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 template <int LPR, bool WS>
 __global__ void __launch_bounds__(WS ? 1024 : 256, WS ? 1 : 4)
