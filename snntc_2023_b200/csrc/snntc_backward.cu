@@ -1032,7 +1032,7 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
     const bool few_wins = g.C <= 8 ? idle || taps_outputs > 15 + 9 * g.C
                           : g.C < 16 ? idle || g.Sh * g.Sw >= 2 || (vec && taps_outputs >= 400)
                                      : idle && vec && few_pixels(g, P);
-    const bool few = dx_few_supported(g) && (opt.dx_kernel == 3 || (opt.dx_kernel == 0 && !sparse_ok && few_wins));
+    const bool few = g.is_conv && (opt.dx_kernel == 3 || (opt.dx_kernel == 0 && !sparse_ok && few_wins));
     if (few) rc = launch_dx_few(g, uv, x, w, out, dx, li, sdx);
     else if (sparse_ok) rc = launch_dx_sparse(g, uv, x, w, out, dx, dx_scratch, gate, li, sdx);
     if (rc == OK && !few && (!sparse_ok || both)) {
@@ -1059,10 +1059,10 @@ int launch_backward(const Geometry& g, const float* grad, const float* x, const 
       // tiles through tensor maps where the shape allows (dw_kernel 2: per-thread copies whatever the shape)
       if (opt.dw_kernel != 2 && dw_tma_supported(g, x, uv, out)) {
         splits = dw_tma_splits(g, li, &rps);
-        rc = launch_dw_tma(g, uv, x, out, partial, splits, rps, scale, exact_flag, li, s);
+        rc = launch_dw_tma(g, uv, x, out, partial, splits, rps, scale, exact_flag, s);
       } else {
         splits = dw_skip_splits(g, li, &rps);
-        rc = launch_dw_skip(g, uv, x, out, partial, splits, rps, scale, exact_flag, li, s);
+        rc = launch_dw_skip(g, uv, x, out, partial, splits, rps, scale, exact_flag, s);
       }
       splits = splits < 1 ? 1 : splits;
       if (rc == OK) {

@@ -149,7 +149,7 @@ bool dw_skip_supported(const Geometry& g, const float* x, const float* uv, const
 int dw_skip_splits(const Geometry& g, const LaunchInfo& li, int* rows_per_split);
 int launch_dw_skip(const Geometry& g, const float* uv, const float* x, const float* out, float* partial,
                    int splits, int rows_per_split, float scale, const int* exact_flag,
-                   const LaunchInfo& li, cudaStream_t s);
+                   cudaStream_t s);
 
 // The same kernel with its tiles brought in by tiled bulk copies through tensor maps (snntc_dw_tma.cu): stride-1
 // convolutions on a power-of-two number of channels (<= 256). Its slices are counted in stages of 16 fields.
@@ -157,7 +157,7 @@ bool dw_tma_shape_ok(const Geometry& g);
 bool dw_tma_supported(const Geometry& g, const float* x, const float* uv, const float* out);
 int dw_tma_splits(const Geometry& g, const LaunchInfo& li, int* stages_per_split);
 int launch_dw_tma(const Geometry& g, const float* uv, const float* x, const float* out, float* partial, int splits,
-                  int stages_per_split, float scale, const int* exact_flag, const LaunchInfo& li, cudaStream_t s);
+                  int stages_per_split, float scale, const int* exact_flag, cudaStream_t s);
 // CTAs of that kernel that gave up waiting for their copies (current device, since the library was loaded)
 unsigned long long dw_copy_timeouts();
 
@@ -171,7 +171,6 @@ struct DxGate {
 };
 
 // dX of a convolution with the lanes over the outputs (snntc_dx_few.cu).
-bool dx_few_supported(const Geometry& g);
 int launch_dx_few(const Geometry& g, const float* uv, const float* x, const float* w, const float* y, float* dx,
                   const LaunchInfo& li, cudaStream_t s);
 

@@ -347,8 +347,7 @@ int dw_skip_splits(const Geometry& g, const LaunchInfo& li, int* rows_per_split)
 
 int launch_dw_skip(const Geometry& g, const float* uv, const float* x, const float* out, float* partial,
                    int splits, int rows_per_split, float scale, const int* exact_flag,
-                   const LaunchInfo& li, cudaStream_t s) {
-  (void)li;
+                   cudaStream_t s) {
   int ntiles = 1, ql = 1;
   plan_tiles(g.I + g.has_bias, vec_shape(g), &ntiles, &ql);
   const int nw = plan_warps(g), jt = 4 * nw;

@@ -372,8 +372,7 @@ int dw_tma_splits(const Geometry& g, const LaunchInfo& li, int* stages_per_split
 }
 
 int launch_dw_tma(const Geometry& g, const float* uv, const float* x, const float* out, float* partial, int splits,
-                  int stages_per_split, float scale, const int* exact_flag, const LaunchInfo& li, cudaStream_t s) {
-  (void)li;
+                  int stages_per_split, float scale, const int* exact_flag, cudaStream_t s) {
   EncodeTiledFn enc = encode_tiled();
   if (!enc) return E_UNSUPPORTED;
   const TmaPlan p = plan(g);

@@ -114,8 +114,6 @@ int launch(const Geometry& g, const float* uv, const float* x, const float* w, c
 
 }  // namespace
 
-bool dx_few_supported(const Geometry& g) { return g.is_conv; }
-
 int launch_dx_few(const Geometry& g, const float* uv, const float* x, const float* w, const float* y, float* dx,
                   const LaunchInfo& li, cudaStream_t s) {
   if (g.C == 1) return launch<1>(g, uv, x, w, y, dx, li, s);

@@ -529,7 +529,7 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* en
 template <int JPT, bool VECW, bool STAGE>
 __global__ void __launch_bounds__(kFwdThreads, JPT <= 4 ? 1024 / kFwdThreads : 1)   // up to four outputs per lane: 64 registers, 32 warps per SM
 snn_walk_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, int istride,
-                const float* w, float* __restrict__ out, int row_begin, int row_end) {
+                const float* w, float* __restrict__ out) {
   chain_wait();
   chain_next();
   __shared__ __align__(16) WalkEntry stage[STAGE ? kFwdWarps * 64 : 1];   // two blocks of 32 list entries per warp
@@ -540,12 +540,11 @@ snn_walk_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, 
   const bool full_j = (g.jout % (32 * JPT)) == 0;
   float* __restrict__ y_out = out;
   float* __restrict__ inv_out = g.infer ? nullptr : out + (size_t)R * g.jout;
-  const long items = (long)(row_end - row_begin) * jchunks;
+  const long items = (long)R * jchunks;
   const long wstride = (long)gridDim.x * kFwdWarps;
   constexpr int CH = JPT >= 8 ? 2 : (JPT >= 4 ? 4 : 8);
   for (long item = (long)blockIdx.x * kFwdWarps + uniform_warp_index(); item < items; item += wstride) {
-    const int rl = (int)(item / jchunks), jc = (int)(item - (long)rl * jchunks);
-    const int r = row_begin + rl;
+    const int r = (int)(item / jchunks), jc = (int)(item - (long)r * jchunks);
     const WalkEntry* krow = keys_g + (size_t)r * istride;
     const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     if (full_j)
@@ -560,7 +559,7 @@ snn_walk_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, 
 template <int JP, bool STAGE>
 __global__ void __launch_bounds__(kFwdThreads, 1024 / kFwdThreads)
 snn_walk2_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, int istride,
-                 const float* w, float* __restrict__ out, int row_begin, int row_end) {
+                 const float* w, float* __restrict__ out) {
   chain_wait();
   chain_next();
   __shared__ __align__(16) WalkEntry stage[STAGE ? kFwdWarps * 64 : 1];   // two blocks of 32 list entries per warp
@@ -571,11 +570,10 @@ snn_walk2_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g,
   const bool full_j = (J % (64 * JP)) == 0;
   float* __restrict__ y_out = out;
   float* __restrict__ inv_out = g.infer ? nullptr : out + (size_t)R * J;
-  const long items = (long)(row_end - row_begin) * jchunks;
+  const long items = (long)R * jchunks;
   const long wstride = (long)gridDim.x * kFwdWarps;
   for (long item = (long)blockIdx.x * kFwdWarps + uniform_warp_index(); item < items; item += wstride) {
-    const int rl = (int)(item / jchunks), jc = (int)(item - (long)rl * jchunks);
-    const int r = row_begin + rl;
+    const int r = (int)(item / jchunks), jc = (int)(item - (long)r * jchunks);
     const WalkEntry* krow = keys_g + (size_t)r * istride;
     const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     if (full_j)
@@ -600,8 +598,7 @@ __device__ unsigned g_walk_copy_timeouts = 0u;          // CTAs that gave up wai
 template <bool STAGE>
 __global__ void __launch_bounds__(kSmemwThreads, 1)
 snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g,
-                       int istride, const float* w, float* __restrict__ out, int row_begin, int row_end,
-                       unsigned wmul) {
+                       int istride, const float* w, float* __restrict__ out, unsigned wmul) {
   chain_wait();
   chain_next();
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -655,8 +652,7 @@ snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nva
   const unsigned ws_lane = smem_u32(ws) + 8u * (unsigned)lane;
   const int ctas = gridDim.x / slices;                 // CTAs that share this slice (the host makes gridDim.x a multiple)
   const int cta = blockIdx.x / slices;
-  for (long rl = (long)cta * kSmemwWarps + warp; rl < row_end - row_begin; rl += (long)ctas * kSmemwWarps) {
-    const int r = row_begin + (int)rl;
+  for (int r = cta * kSmemwWarps + warp; r < R; r += ctas * kSmemwWarps) {
     const WalkEntry* krow = keys_g + (size_t)r * istride;
     const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     float* yr = y_out + (size_t)r * J;
@@ -680,26 +676,26 @@ size_t nvalid_bytes(const Geometry& g) { return nvalid_only_bytes(g) + 256; }
 
 template <int JPT, bool VECW>
 int launch_walk(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g, const float* w, float* out,
-                const LaunchInfo& li, cudaStream_t s, int row_begin, int row_end, bool stage) {
+                cudaStream_t s, bool stage) {
   const int jchunks = (g.jout + 32 * JPT - 1) / (32 * JPT);
-  const long items = (long)(row_end - row_begin) * jchunks;
+  const long items = (long)g.R * jchunks;
   long grid = (items + kFwdWarps - 1) / kFwdWarps;
   if (grid > 0x7fffffffL) grid = 0x7fffffffL;      // (a warp goes on to item + warps of the grid)
-  if (stage) (void)launch_chained(snn_walk_kernel<JPT, VECW, true>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
-  else (void)launch_chained(snn_walk_kernel<JPT, VECW, false>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
+  if (stage) (void)launch_chained(snn_walk_kernel<JPT, VECW, true>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
+  else (void)launch_chained(snn_walk_kernel<JPT, VECW, false>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
 
 template <int JP>
 int launch_walk2(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g, const float* w, float* out,
-                 const LaunchInfo& li, cudaStream_t s, int row_begin, int row_end, bool stage) {
+                 cudaStream_t s, bool stage) {
   const int jchunks = (g.J + 64 * JP - 1) / (64 * JP);
-  const long items = (long)(row_end - row_begin) * jchunks;
+  const long items = (long)g.R * jchunks;
   long grid = (items + kFwdWarps - 1) / kFwdWarps;
   if (grid > 0x7fffffffL) grid = 0x7fffffffL;      // (a warp goes on to item + warps of the grid)
-  if (stage) (void)launch_chained(snn_walk2_kernel<JP, true>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
-  else (void)launch_chained(snn_walk2_kernel<JP, false>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end);
+  if (stage) (void)launch_chained(snn_walk2_kernel<JP, true>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
+  else (void)launch_chained(snn_walk2_kernel<JP, false>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -719,23 +715,21 @@ bool walk_smemw_ok(const Geometry& g, const float* w, const LaunchInfo& li, size
 }
 
 int launch_walk2_smemw(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g, const float* w, float* out,
-                       const LaunchInfo& li, cudaStream_t s, int row_begin, int row_end, bool stage, size_t smem,
-                       int wmul) {
+                       const LaunchInfo& li, cudaStream_t s, bool stage, size_t smem, int wmul) {
   const int slices = g.J >> 6;
-  const long rows = row_end - row_begin;
   long per_slice = li.num_sms / slices;                       // persistent: one CTA per SM
-  const long need = (rows + kSmemwWarps - 1) / kSmemwWarps;
+  const long need = ((long)g.R + kSmemwWarps - 1) / kSmemwWarps;
   if (per_slice > need) per_slice = need;
   if (per_slice < 1) per_slice = 1;
   const int grid = (int)(per_slice * slices);
   if (stage) {
     if (allow_smem<snn_walk2_smemw_kernel<true>>(smem) != cudaSuccess)
       return E_CUDA;
-    (void)launch_chained(snn_walk2_smemw_kernel<true>, grid, kSmemwThreads, smem, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end, (unsigned)wmul);
+    (void)launch_chained(snn_walk2_smemw_kernel<true>, grid, kSmemwThreads, smem, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, (unsigned)wmul);
   } else {
     if (allow_smem<snn_walk2_smemw_kernel<false>>(smem) != cudaSuccess)
       return E_CUDA;
-    (void)launch_chained(snn_walk2_smemw_kernel<false>, grid, kSmemwThreads, smem, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, row_begin, row_end, (unsigned)wmul);
+    (void)launch_chained(snn_walk2_smemw_kernel<false>, grid, kSmemwThreads, smem, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, (unsigned)wmul);
   }
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
@@ -885,24 +879,24 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   // layout switches it off
   const bool smemw = walk_smemw_ok(g, w, li, &smemw_bytes, &smemw_shift) &&
                      ((opt.walk_layout & 8) != 0 || ((opt.walk_layout & 3) == 0 && g.J == 64 && g.R >= 32768));
-  auto walk = [&](cudaStream_t st, int r0, int r1) -> int {
+  auto walk = [&]() -> int {
     if (!(fparts & 2)) return OK;
-    if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, li, st);
-    if (rows) return launch_walk_rows(g, keys_g, nvalid_g, key_stride(g), w, out, own ? g.J > 32 && g.R >= 32768 : (opt.walk_layout & 64) != 0, li, st);
-    if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage, smemw_bytes, smemw_shift);
+    if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, li, s);
+    if (rows) return launch_walk_rows(g, keys_g, nvalid_g, key_stride(g), w, out, own ? g.J > 32 && g.R >= 32768 : (opt.walk_layout & 64) != 0, li, s);
+    if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, s, stage, smemw_bytes, smemw_shift);
     if (variant == 1) {
       // pairs layout: 64 outputs per warp, or (walk_outputs 3) 128 as two pairs per lane
-      if (jsel >= 2) return launch_walk2<2>(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage);
-      return launch_walk2<1>(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage);
+      if (jsel >= 2) return launch_walk2<2>(g, keys_g, nvalid_g, w, out, s, stage);
+      return launch_walk2<1>(g, keys_g, nvalid_g, w, out, s, stage);
     }
-    if (jsel == 0) return launch_walk<1, false>(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage);
+    if (jsel == 0) return launch_walk<1, false>(g, keys_g, nvalid_g, w, out, s, stage);
     if (variant == 3) {
-      if (jsel == 1) return launch_walk<2, true>(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage);
-      if (jsel == 2) return launch_walk<4, true>(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage);
-      return launch_walk<8, true>(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage);
+      if (jsel == 1) return launch_walk<2, true>(g, keys_g, nvalid_g, w, out, s, stage);
+      if (jsel == 2) return launch_walk<4, true>(g, keys_g, nvalid_g, w, out, s, stage);
+      return launch_walk<8, true>(g, keys_g, nvalid_g, w, out, s, stage);
     }
-    if (jsel == 1) return launch_walk<2, false>(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage);
-    return launch_walk<4, false>(g, keys_g, nvalid_g, w, out, li, st, r0, r1, stage);
+    if (jsel == 1) return launch_walk<2, false>(g, keys_g, nvalid_g, w, out, s, stage);
+    return launch_walk<4, false>(g, keys_g, nvalid_g, w, out, s, stage);
   };
 
   if (use_merge_lists(g, opt, li)) {
@@ -910,21 +904,21 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
       const int rc = launch_merge_lists(g, x, keys_g, nvalid_g, istride, merge_scratch, (opt.list_builder >> 2) - 1, li, s);
       if (rc != OK) return rc;
     }
-    return walk(s, 0, g.R);
+    return walk();
   }
   if (use_small_rows(g, opt)) {
     if (fparts & 1) {
       const int rc = launch_small_rows(g, x, keys_g, nvalid_g, istride, li, s);
       if (rc != OK) return rc;
     }
-    return walk(s, 0, g.R);
+    return walk();
   }
 
   if (fparts & 1) {
     const int rc = launch_row_sort(g, x, keys_g, nvalid_g, istride, li, s);
     if (rc != OK) return rc;
   }
-  return walk(s, 0, g.R);
+  return walk();
 }
 
 }  // namespace snntc
