@@ -249,12 +249,12 @@ SNNTC_API unsigned long long snntc_copy_timeouts(void);
  * benchmark can time the kernels of an operator apart and a test can check the variants against each other:
  *   opts8 = { forward_parts   bit 0: build the sorted lists, bit 1: walk them (default 3; without bit 1 the
  *                             output is not written),
- *             walk_layout     0 auto, 1 output pairs, 2 outputs lane+32m, 3 consecutive outputs per lane; +4: list
- *                             entries straight from global memory instead of staged through shared memory;
- *                             +8 weights in shared memory, +16 weight rows copied ahead, +32 / +64 several rows per warp
- *                             (+64: weights in shared memory),
- *             walk_outputs    0 auto, 1..4: 1, 2, 4, 8 outputs per lane,
- *             list_builder    0 auto, 1 per-row bucket sort, 2 per-pixel sort + merges,
+ *             walk_layout     0 auto, 1 output pairs, 2 outputs lane+32m, 3 four consecutive outputs per lane, 8 output
+ *                             pairs with the weights in shared memory, 16 weight rows copied ahead, 32 / 64 several rows
+ *                             per warp (64: weights in shared memory); a layout that the weights do not allow: auto,
+ *             walk_outputs    outputs per lane of layout 2: 0 auto, 1..3: 1, 2, 4,
+ *             list_builder    0 auto, 1 per-row bucket sort, 2 per-pixel sort + merges, 3 register network (up to 64
+ *                             inputs); + 4*(k+1): merges cut into 2^k pieces,
  *             backward_parts  bit 0: dX, bit 1: dW (default 3),
  *             dw_kernel       0 auto, 1 dense register tile, 2 row-skipping kernel, 4 the same through tensor maps where
  *                             the shape allows,

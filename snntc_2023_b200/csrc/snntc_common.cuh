@@ -45,13 +45,12 @@ struct LaunchInfo {
 // and from the tests that check the variants against each other. Nothing here is process-wide state.
 struct Options {
   int forward_parts = 3;    // bit 0: build the sorted lists, bit 1: walk them
-  int walk_layout = 0;      // 0 auto, 1 output pairs, 2 outputs lane+32m, 3 consecutive outputs per lane;
-                            // +4: read list entries straight from global memory instead of through shared memory
-                            // +8: output pairs with the weights staged in shared memory (where they fit)
+  int walk_layout = 0;      // 0 auto, 1 output pairs, 2 outputs lane+32m, 3 four consecutive outputs per lane,
+                            // 8: output pairs with the weights staged in shared memory (where they fit)
                             // 16: one output per lane, the warp's weight rows copied ahead into shared memory
                             // 32, 64: several rows per warp (fan-out <= 64, a multiple of 4), weights from global memory /
-                            // in shared memory where they fit
-  int walk_outputs = 0;     // 0 auto, 1..4: 1, 2, 4, 8 outputs per lane (pairs layout: 2 only)
+                            // in shared memory where they fit. A layout that the weights do not allow: auto
+  int walk_outputs = 0;     // outputs per lane of layout 2: 0 auto, 1..3: 1, 2, 4
   int list_builder = 0;     // 0 auto, 1 per-row bucket sort, 2 per-pixel sort + merges (3x3 stride-1 conv only),
                             // 3 per-row sorting network in registers (rows of at most 64 inputs);
                             // + 4*(k+1): the merges are cut into 2^k pieces each (k = 0 .. 5) instead of auto

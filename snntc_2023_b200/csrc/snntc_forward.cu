@@ -12,8 +12,8 @@
 //      (snntc/snnfc_kernels.cu.cc:33-69); the causality test is the sign of q = ysum - x*wsum per step -- one FMA
 //      per output, the lane's smallest q as an integer, one warp vote -- backed by the reference's exact
 //      division-free comparisons whenever it turns non-positive in any lane (see walk_row). Three layouts of a
-//      lane's outputs: a pair in one 64-bit register (walk_row2, fan-out <= 64), 2 or 4 consecutive outputs read
-//      by one 8/16-byte load, or outputs lane + 32*m (odd fan-out, unaligned weights).
+//      lane's outputs: a pair in one 64-bit register (walk_row2), four consecutive outputs read by one 16-byte load, or
+//      outputs lane + 32*m (odd fan-out, unaligned weights).
 #include "snntc_common.cuh"
 #include "snntc_walk.cuh"
 
@@ -124,7 +124,7 @@ snn_wbound_kernel(const float* w, int rows, int J, int rows_per_cta, float* __re
 // ulp of zero, or a NEGATIVE denominator, which inputs below the bias input can produce and for which the
 // reference fires on the way back up through zero -- makes the lane "sticky": the exact tests run again at
 // the next step whatever q is, until no live output of the lane is in that state any more.
-template <int JPT, int CH, bool FULL, bool VECW, bool STAGE>
+template <int JPT, int CH, bool FULL, bool VECW>
 __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ents, int nvalid,
                                          const float* w, int jbase, int lane,
                                          float* __restrict__ y_row, float* __restrict__ inv_row,
@@ -136,8 +136,8 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
   int livemask[JPT];
 #pragma unroll
   for (int m = 0; m < JPT; ++m) {
-    // VECW: a lane owns JPT consecutive outputs and reads them with 8- or 16-byte loads (J % JPT == 0,
-    // so a lane is wholly inside or wholly outside the row); otherwise outputs lane + 32*m, 4-byte loads
+    // VECW: a lane owns four consecutive outputs and reads them with one 16-byte load (J % 4 == 0, so a lane is wholly
+    // inside or wholly outside the row); otherwise outputs lane + 32*m, 4-byte loads
     const int j = VECW ? jbase + JPT * lane + m : jbase + lane + 32 * m;
     jok[m] = FULL || j < g.jout;
     jl[m] = jok[m] ? j : (VECW ? J - JPT + m : J - 1);   // (padding behind jout: weights of zero, never stored)
@@ -170,17 +170,9 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
   const char* wbase = reinterpret_cast<const char*>(w);
   auto load_weights = [&](unsigned eoff, float (&wv)[JPT]) {
     const float* wrow = wl + eoff;
-    if constexpr (VECW && JPT == 8) {
-      const float4* p4 = reinterpret_cast<const float4*>(wbase + (size_t)(eoff + lane_off) * 4u);
-      const float4 v = ld_plain(p4), v2 = ld_plain(p4 + 1);
-      wv[0] = v.x; wv[1] = v.y; wv[2] = v.z; wv[3] = v.w;
-      wv[4] = v2.x; wv[5] = v2.y; wv[6] = v2.z; wv[7] = v2.w;
-    } else if constexpr (VECW && JPT == 4) {
+    if constexpr (VECW) {
       const float4 v = ld_plain(reinterpret_cast<const float4*>(wbase + (size_t)(eoff + lane_off) * 4u));
       wv[0] = v.x; wv[1] = v.y; wv[2] = v.z; wv[3] = v.w;
-    } else if constexpr (VECW && JPT == 2) {
-      const float2 v = ld_plain(reinterpret_cast<const float2*>(wbase + (size_t)(eoff + lane_off) * 4u));
-      wv[0] = v.x; wv[1] = v.y;
     } else {
 #pragma unroll
       for (int m = 0; m < JPT; ++m) wv[m] = FULL ? ld_plain(wrow + 32 * m) : ld_plain(wrow + jl[m]);
@@ -195,8 +187,7 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
     int qmin;
     if constexpr (JPT == 1) qmin = min(q[0], sticky);
     else if constexpr (JPT == 2) qmin = imin3(q[0], q[1], sticky);
-    else if constexpr (JPT == 4) qmin = imin3(imin3(q[0], q[1], q[2]), q[3], sticky);
-    else qmin = imin3(imin3(q[0], q[1], q[2]), imin3(q[3], q[4], q[5]), imin3(q[6], q[7], sticky));
+    else qmin = imin3(imin3(q[0], q[1], q[2]), q[3], sticky);
     if (__builtin_expect(__any_sync(0xffffffffu, qmin <= qlim), 0)) {
       // rare path: the reference's own rounded comparisons for the live outputs concerned (usually one of the
       // lane's outputs in one lane: skip the others with a warp-uniform test each)
@@ -225,8 +216,6 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
     }
   };
 
-  // One chunk of CH steps: entries, then their weight rows, then the arithmetic. `fetch(i)` returns entry i of
-  // the part of the list at hand.
   bool all_done = false;
   auto check_done = [&]() {
     int any_live = 0;
@@ -234,14 +223,14 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
     for (int m = 0; m < JPT; ++m) any_live |= livemask[m];
     all_done = !__any_sync(0xffffffffu, any_live != 0);
   };
-  // `fetch2(i)` returns entries i and i+1 (i even) of the part of the list at hand as one 16-byte read.
+  // One chunk of CH steps: entries, two by one 16-byte read, then their weight rows, then the arithmetic.
   static_assert(CH % 2 == 0, "entries are fetched two at a time");
-  auto chunk = [&](auto fetch2, int k0) {
+  auto chunk = [&](const WalkEntry* cur) {
     float xs[CH];
     float wv[CH][JPT];
 #pragma unroll
     for (int u = 0; u < CH; u += 2) {
-      const uint4 e2 = fetch2(k0 + u);
+      const uint4 e2 = *reinterpret_cast<const uint4*>(cur + u);
       xs[u] = __uint_as_float(e2.x);
       load_weights(e2.y, wv[u]);
       xs[u + 1] = __uint_as_float(e2.z);
@@ -259,35 +248,23 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
     step(__uint_as_float(e.x), xprev, wv);
     xprev = __uint_as_float(e.x);
   };
-  if constexpr (STAGE) {
-    // The list goes through shared memory 32 entries at a time: one coalesced read per lane and block, issued a
-    // whole block ahead, instead of one L2 round trip in front of every chunk; a step then reads its entry with
-    // one broadcast shared-memory load. Two buffers of 32 entries per warp.
-    WalkEntry pre = make_uint2(0u, 0u);
-    if (lane < nvalid) pre = ld_l2(ents + lane);
-    int b = 0;
-    for (int base = 0; base < nvalid && !all_done; base += 32, b ^= 32) {
-      sbuf[b + lane] = pre;
-      __syncwarp();
-      if (base + 32 + lane < nvalid) pre = ld_l2(ents + base + 32 + lane);
-      const int nb = min(32, nvalid - base);
-      const WalkEntry* cur = sbuf + b;
-      auto fetch2 = [&](int i) { return *reinterpret_cast<const uint4*>(cur + i); };
-      int kk = 0;
+  // The list goes through shared memory 32 entries at a time: one coalesced read per lane and block, issued a
+  // whole block ahead, instead of one L2 round trip in front of every chunk; a step then reads its entry with
+  // one broadcast shared-memory load. Two buffers of 32 entries per warp.
+  WalkEntry pre = make_uint2(0u, 0u);
+  if (lane < nvalid) pre = ld_l2(ents + lane);
+  int b = 0;
+  for (int base = 0; base < nvalid && !all_done; base += 32, b ^= 32) {
+    sbuf[b + lane] = pre;
+    __syncwarp();
+    if (base + 32 + lane < nvalid) pre = ld_l2(ents + base + 32 + lane);
+    const int nb = min(32, nvalid - base);
+    const WalkEntry* cur = sbuf + b;
+    int kk = 0;
 #pragma unroll 1
-      for (; kk + CH <= nb; kk += CH) chunk(fetch2, kk);
-      for (; kk < nb; ++kk) single(cur[kk]);
-      check_done();   // one "has every output fired" vote per block
-    }
-  } else {
-    int k = 0;
-    for (; k + CH <= nvalid && !all_done; k += CH) {
-      // list entries bypass L1: it is kept for the weights
-      chunk([&](int i) { return ld_l2(reinterpret_cast<const uint4*>(ents + i)); }, k);
-      check_done();
-    }
-    if (!all_done)
-      for (; k < nvalid; ++k) single(ld_l2(ents + k));
+    for (; kk + CH <= nb; kk += CH) chunk(cur + kk);
+    for (; kk < nb; ++kk) single(cur[kk]);
+    check_done();   // one "has every output fired" vote per block
   }
 
 #pragma unroll
@@ -317,136 +294,104 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
 // ---- two outputs per 64-bit register ---------------------------------------------------------------
 // sm_100 has two-lane FP32 add / sub / fma on 64-bit register pairs: one issue slot, two results, each
 // rounded exactly like the scalar instruction. A pair holds outputs (j, j+1) of one lane.
-// walk_row with the outputs of a lane held as JP pairs (j, j+1), j = jbase + 2*lane + 64*m: the three
-// FP32 operations of a step (q, the weight sum, the weighted sum) are one packed instruction per pair and
-// a weight-row read is one 8-byte load per pair. The weight sum is carried NEGATED (nws = theta - sum w), so
-// that q = fma(x, nws, ysum) needs no negated copy of x; negation is exact, so every value is bit for bit the
-// scalar walk's -- except the sign of an exactly cancelled sum (+0 on both sides), which is why the sum is
+// walk_row with the outputs of a lane held as one pair (j, j+1), j = jbase + 2*lane: the three FP32 operations of a step (q, the
+// weight sum, the weighted sum) are one packed instruction and a weight-row read is one 8-byte load. The weight sum is carried
+// NEGATED (nws = theta - sum w), so that q = fma(x, nws, ysum) needs no negated copy of x; negation is exact, so every value is
+// bit for bit the scalar walk's -- except the sign of an exactly cancelled sum (+0 on both sides), which is why the sum is
 // read back as 0 - nws: 1/(+0) = +inf clamps to "no spike", 1/(-0) would not. Requires J even and the
 // weights 8-byte aligned.
 // WS: the weights of this warp's 64 outputs sit in shared memory as [fan-in row][64] (see snn_walk2_smemw_kernel);
 // `ws_lane` is the shared-memory byte address of this lane's pair in row 0 and `wmul` = 256 / J (J = 64, 128 or 256): a
 // list entry's element offset (source index * J) times wmul is the row's byte offset in the slice -- one integer
-// multiply-add on the FMA pipe per weight read. JP == 1 only.
-template <int JP, int CH, bool FULL, bool STAGE, bool WS = false>
+// multiply-add on the FMA pipe per weight read.
+template <int CH, bool FULL, bool WS = false>
 __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* ents, int nvalid,
                                           const float* w, int jbase, int lane,
                                           float* __restrict__ y_row, float* __restrict__ inv_row,
                                           WalkEntry* __restrict__ sbuf, unsigned ws_lane = 0u, unsigned wmul = 0u) {
-  static_assert(!WS || JP == 1, "weights in shared memory: one output pair per lane");
   const int J = g.J;
-  int jl[JP];
-  bool jok[JP];
-  uint64_t nws[JP], ys[JP];
-  float wfin[2 * JP], yfin[2 * JP];
-  int live[2 * JP];
-#pragma unroll
-  for (int m = 0; m < JP; ++m) {
-    const int j = jbase + 2 * lane + 64 * m;
-    jok[m] = FULL || j < g.jout;
-    jl[m] = jok[m] ? j : J - 2;
+  const int j0 = jbase + 2 * lane;                        // this lane's outputs: j0, j0 + 1
+  const int jl = FULL || j0 < g.jout ? j0 : J - 2;
+  uint64_t nws, ys;
+  float wfin[2], yfin[2];
+  int live[2] = {-1, -1};
+  {
     float n0 = g.theta, n1 = g.theta, y0 = 0.f, y1 = 0.f;
     if (g.has_bias) {  // the bias input (value biasvolt, weight row I) is always consumed first
-      const float2 wb = ld_plain(reinterpret_cast<const float2*>(w + (size_t)g.I * J + jl[m]));
+      const float2 wb = ld_plain(reinterpret_cast<const float2*>(w + (size_t)g.I * J + jl));
       n0 -= wb.x; n1 -= wb.y;
       y0 = g.biasvolt * wb.x; y1 = g.biasvolt * wb.y;
     }
-    wfin[2 * m] = 0.f - n0; wfin[2 * m + 1] = 0.f - n1;
-    yfin[2 * m] = y0; yfin[2 * m + 1] = y1;
-    live[2 * m] = live[2 * m + 1] = -1;
+    wfin[0] = 0.f - n0; wfin[1] = 0.f - n1;
+    yfin[0] = y0; yfin[1] = y1;
     if (!FULL) {     // no output: parked from the start like one that has fired, or the walk would wait for it
-      if (j >= g.jout) { live[2 * m] = 0; n0 = CUDART_INF_F; }
-      if (j + 1 >= g.jout) { live[2 * m + 1] = 0; n1 = CUDART_INF_F; }
+      if (j0 >= g.jout) { live[0] = 0; n0 = CUDART_INF_F; }
+      if (j0 + 1 >= g.jout) { live[1] = 0; n1 = CUDART_INF_F; }
     }
-    nws[m] = pack2(n0, n1);
-    ys[m] = pack2(y0, y1);
+    nws = pack2(n0, n1);
+    ys = pack2(y0, y1);
   }
   float xprev = g.has_bias ? g.biasvolt : 0.f;
-
-  const float* wl = w + (FULL ? jbase + 2 * lane : 0);
 
   int sticky = INT_MAX;   // INT_MIN while some live output of this lane must be tested exactly at the next step
   const float tolbase = walk_tolerance_base(g);
   int qlim = 0;           // bits of the largest q that still goes to the exact tests (see walk_tolerance_base)
-  auto step = [&](const float x, const float xprev, const uint64_t (&wv)[JP]) {
+  auto step = [&](const float x, const float xprev, const uint64_t wv) {
     const uint64_t x2 = pack2(x, x);
-    int q[2 * JP];
-#pragma unroll
-    for (int m = 0; m < JP; ++m) unpack2i(fma2(x2, nws[m], ys[m]), q[2 * m], q[2 * m + 1]);
-    int qmin;
-    if constexpr (JP == 1) qmin = imin3(q[0], q[1], sticky);
-    else if constexpr (JP == 2) qmin = imin3(imin3(q[0], q[1], q[2]), q[3], sticky);
-    else qmin = imin3(imin3(q[0], q[1], q[2]), imin3(q[3], q[4], q[5]), imin3(q[6], q[7], sticky));
-    if (__builtin_expect(__any_sync(0xffffffffu, qmin <= qlim), 0)) {
+    int q[2];
+    unpack2i(fma2(x2, nws, ys), q[0], q[1]);
+    if (__builtin_expect(__any_sync(0xffffffffu, imin3(q[0], q[1], sticky) <= qlim), 0)) {
       // rare path: the reference's own rounded comparisons for the live outputs (see walk_row)
       bool again = false;
+      float n[2], y[2];
+      unpack2(nws, n[0], n[1]);
+      unpack2(ys, y[0], y[1]);
 #pragma unroll
-      for (int m = 0; m < JP; ++m) {
-        float n[2], y[2];
-        unpack2(nws[m], n[0], n[1]);
-        unpack2(ys[m], y[0], y[1]);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          // usually one output of one lane is concerned: skip the other half with a warp-uniform test
-          if (!__any_sync(0xffffffffu, (q[2 * m + h] <= qlim) | (sticky < 0))) continue;
-          const float wsum = 0.f - n[h];   // not -n: an exactly cancelled sum must read +0 as in the scalar walk
-          const bool lv = live[2 * m + h] != 0;
-          const bool fire = lv & ratio_gt(y[h], wsum, xprev) & ratio_le(y[h], wsum, x);
-          if (fire) {
-            live[2 * m + h] = 0;   // spike lies in (previous input, x]: keep the sums aside ...
-            wfin[2 * m + h] = wsum;
-            yfin[2 * m + h] = y[h];
-            n[h] = CUDART_INF_F;   // ... and park the running weight sum where q stays +inf
-          }
-          again |= lv & !fire & (q[2 * m + h] <= qlim);
+      for (int h = 0; h < 2; ++h) {
+        // usually one output of one lane is concerned: skip the other half with a warp-uniform test
+        if (!__any_sync(0xffffffffu, (q[h] <= qlim) | (sticky < 0))) continue;
+        const float wsum = 0.f - n[h];   // not -n: an exactly cancelled sum must read +0 as in the scalar walk
+        const bool lv = live[h] != 0;
+        const bool fire = lv & ratio_gt(y[h], wsum, xprev) & ratio_le(y[h], wsum, x);
+        if (fire) {
+          live[h] = 0;           // spike lies in (previous input, x]: keep the sums aside ...
+          wfin[h] = wsum;
+          yfin[h] = y[h];
+          n[h] = CUDART_INF_F;   // ... and park the running weight sum where q stays +inf
         }
-        nws[m] = pack2(n[0], n[1]);
+        again |= lv & !fire & (q[h] <= qlim);
       }
+      nws = pack2(n[0], n[1]);
       sticky = again ? INT_MIN : INT_MAX;
     }
-#pragma unroll
-    for (int m = 0; m < JP; ++m) {
-      nws[m] = sub2(nws[m], wv[m]);
-      ys[m] = fma2(x2, wv[m], ys[m]);
-    }
+    nws = sub2(nws, wv);
+    ys = fma2(x2, wv, ys);
   };
-  const unsigned lane_off = (unsigned)jl[0];   // element offset of this lane's first pair within a weight row
-  auto load_pair = [&](const float* wrow, int m) -> uint64_t {
-    return ld_plain(reinterpret_cast<const unsigned long long*>(FULL ? wrow + 64 * m : wrow + jl[m]));
-  };
-
+  const unsigned lane_off = (unsigned)jl;   // element offset of this lane's pair within a weight row
   bool all_done = false;
-  auto load_row = [&](unsigned eoff, uint64_t (&wv)[JP]) {
+  auto load_row = [&](unsigned eoff) -> uint64_t {
     if constexpr (WS) {
-      asm("ld.shared.b64 %0, [%1];" : "=l"(wv[0]) : "r"(eoff * wmul + ws_lane));
-    } else if constexpr (JP == 1) {
-      // one pair per lane: a 32-bit element offset from the (uniform) weight base measured faster than a
-      // 64-bit per-lane pointer plus the entry's offset
-      wv[0] = ld_plain(reinterpret_cast<const unsigned long long*>(
-          reinterpret_cast<const char*>(w) + (size_t)(eoff + lane_off) * 4u));
+      uint64_t v;
+      asm("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(eoff * wmul + ws_lane));
+      return v;
     } else {
-      const float* wrow = wl + eoff;
-#pragma unroll
-      for (int m = 0; m < JP; ++m) wv[m] = load_pair(wrow, m);
+      // a 32-bit element offset from the (uniform) weight base measured faster than a 64-bit per-lane pointer plus the
+      // entry's offset
+      return ld_plain(reinterpret_cast<const unsigned long long*>(
+          reinterpret_cast<const char*>(w) + (size_t)(eoff + lane_off) * 4u));
     }
-  };
-  auto check_done = [&]() {
-    int any_live = 0;
-#pragma unroll
-    for (int m = 0; m < 2 * JP; ++m) any_live |= live[m];
-    all_done = !__any_sync(0xffffffffu, any_live != 0);
   };
   static_assert(CH % 2 == 0, "entries are fetched two at a time");
-  auto chunk = [&](auto fetch2, int k0) {
+  auto chunk = [&](const WalkEntry* cur) {
     float xs[CH];
-    uint64_t wv[CH][JP];
+    uint64_t wv[CH];
 #pragma unroll
     for (int u = 0; u < CH; u += 2) {
-      const uint4 e2 = fetch2(k0 + u);
+      const uint4 e2 = *reinterpret_cast<const uint4*>(cur + u);
       xs[u] = __uint_as_float(e2.x);
-      load_row(e2.y, wv[u]);
+      wv[u] = load_row(e2.y);
       xs[u + 1] = __uint_as_float(e2.z);
-      load_row(e2.w, wv[u + 1]);
+      wv[u + 1] = load_row(e2.w);
     }
     qlim = __float_as_int(tolbase * fmaxf(fabsf(xs[0]), fabsf(xs[CH - 1])));   // inputs ascend: |x| peaks at an end
 #pragma unroll
@@ -454,86 +399,65 @@ __device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* en
     xprev = xs[CH - 1];
   };
   auto single = [&](const WalkEntry e) {
-    uint64_t wv[JP];
-    if constexpr (WS) {
-      load_row(e.y, wv);
-    } else {
-      const float* wrow = wl + e.y;
-#pragma unroll
-      for (int m = 0; m < JP; ++m) wv[m] = load_pair(wrow, m);
-    }
+    const uint64_t wv = load_row(e.y);
     qlim = __float_as_int(tolbase * fabsf(__uint_as_float(e.x)));
     step(__uint_as_float(e.x), xprev, wv);
     xprev = __uint_as_float(e.x);
   };
-  if constexpr (STAGE) {   // the list through shared memory, 32 entries at a time, read a block ahead (see walk_row)
-    WalkEntry pre = make_uint2(0u, 0u);
-    if (lane < nvalid) pre = ld_l2(ents + lane);
-    int b = 0;
-    for (int base = 0; base < nvalid && !all_done; base += 32, b ^= 32) {
-      sbuf[b + lane] = pre;
-      __syncwarp();
-      if (base + 32 + lane < nvalid) pre = ld_l2(ents + base + 32 + lane);
-      const int nb = min(32, nvalid - base);
-      const WalkEntry* cur = sbuf + b;
-      auto fetch2 = [&](int i) { return *reinterpret_cast<const uint4*>(cur + i); };
-      int kk = 0;
+  // the list through shared memory, 32 entries at a time, read a block ahead (see walk_row)
+  WalkEntry pre = make_uint2(0u, 0u);
+  if (lane < nvalid) pre = ld_l2(ents + lane);
+  int b = 0;
+  for (int base = 0; base < nvalid && !all_done; base += 32, b ^= 32) {
+    sbuf[b + lane] = pre;
+    __syncwarp();
+    if (base + 32 + lane < nvalid) pre = ld_l2(ents + base + 32 + lane);
+    const int nb = min(32, nvalid - base);
+    const WalkEntry* cur = sbuf + b;
+    int kk = 0;
 #pragma unroll 1
-      for (; kk + CH <= nb; kk += CH) chunk(fetch2, kk);
-      for (; kk < nb; ++kk) single(cur[kk]);
-      check_done();   // one "has every output fired" vote per block
-    }
-  } else {
-    int k = 0;
-    for (; k + CH <= nvalid && !all_done; k += CH) {
-      // list entries bypass L1: it is kept for the weights
-      chunk([&](int i) { return ld_l2(reinterpret_cast<const uint4*>(ents + i)); }, k);
-      check_done();
-    }
-    if (!all_done)
-      for (; k < nvalid; ++k) single(ld_l2(ents + k));
+    for (; kk + CH <= nb; kk += CH) chunk(cur + kk);
+    for (; kk < nb; ++kk) single(cur[kk]);
+    all_done = !__any_sync(0xffffffffu, (live[0] | live[1]) != 0);   // one "has every output fired" vote per block
   }
 
+  float n[2], y[2];
+  unpack2(nws, n[0], n[1]);
+  unpack2(ys, y[0], y[1]);
 #pragma unroll
-  for (int m = 0; m < JP; ++m) {
-    float n[2], y[2];
-    unpack2(nws[m], n[0], n[1]);
-    unpack2(ys[m], y[0], y[1]);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      // an output that stopped has fired; one that consumed every input fires iff it is armed
-      bool fired = true;
-      float ws = wfin[2 * m + h], yy = yfin[2 * m + h];
-      if (live[2 * m + h]) {
-        ws = 0.f - n[h]; yy = y[h];
-        fired = ratio_gt(yy, ws, xprev);
-      }
-      float yv = g.maxv, iv = 0.f;
-      if (fired) {
-        iv = __fdividef(1.0f, ws);
-        yv = yy * iv;
-        if (yv >= g.maxv) { yv = g.maxv; iv = 0.f; }
-      }
-      const int j = jbase + 2 * lane + 64 * m + h;
-      if (FULL || j < g.jout) {
-        y_row[j] = yv;
-        if (inv_row != nullptr) inv_row[j] = iv;
-        if (g.khist != nullptr) atomicAdd(g.khist + (yv < g.maxv ? entries_below(ents, nvalid, yv) : g.I + 1), 1);
-      }
+  for (int h = 0; h < 2; ++h) {
+    // an output that stopped has fired; one that consumed every input fires iff it is armed
+    bool fired = true;
+    float ws = wfin[h], yy = yfin[h];
+    if (live[h]) {
+      ws = 0.f - n[h]; yy = y[h];
+      fired = ratio_gt(yy, ws, xprev);
+    }
+    float yv = g.maxv, iv = 0.f;
+    if (fired) {
+      iv = __fdividef(1.0f, ws);
+      yv = yy * iv;
+      if (yv >= g.maxv) { yv = g.maxv; iv = 0.f; }
+    }
+    const int j = j0 + h;
+    if (FULL || j < g.jout) {
+      y_row[j] = yv;
+      if (inv_row != nullptr) inv_row[j] = iv;
+      if (g.khist != nullptr) atomicAdd(g.khist + (yv < g.maxv ? entries_below(ents, nvalid, yv) : g.I + 1), 1);
     }
   }
 }
 
 // ------------------------------------------------------------------------------------------- kernels
 // Walk kernel: every warp takes (row, block of 32*JPT outputs) items, adjacent warps share a row.
-template <int JPT, bool VECW, bool STAGE>
-__global__ void __launch_bounds__(kFwdThreads, JPT <= 4 ? 1024 / kFwdThreads : 1)   // up to four outputs per lane: 64 registers, 32 warps per SM
+template <int JPT, bool VECW>
+__global__ void __launch_bounds__(kFwdThreads, 1024 / kFwdThreads)   // 64 registers, 32 warps per SM
 snn_walk_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, int istride,
                 const float* w, float* __restrict__ out) {
   chain_wait();
   chain_next();
-  __shared__ __align__(16) WalkEntry stage[STAGE ? kFwdWarps * 64 : 1];   // two blocks of 32 list entries per warp
-  WalkEntry* sbuf = stage + (STAGE ? (threadIdx.x >> 5) * 64 : 0);
+  __shared__ __align__(16) WalkEntry stage[kFwdWarps * 64];   // two blocks of 32 list entries per warp
+  WalkEntry* sbuf = stage + (threadIdx.x >> 5) * 64;
   const int R = g.R;
   const int lane = threadIdx.x & 31;
   const int jchunks = (g.jout + 32 * JPT - 1) / (32 * JPT);
@@ -542,32 +466,31 @@ snn_walk_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, 
   float* __restrict__ inv_out = g.infer ? nullptr : out + (size_t)R * g.jout;
   const long items = (long)R * jchunks;
   const long wstride = (long)gridDim.x * kFwdWarps;
-  constexpr int CH = JPT >= 8 ? 2 : (JPT >= 4 ? 4 : 8);
+  constexpr int CH = JPT == 4 ? 4 : 8;
   for (long item = (long)blockIdx.x * kFwdWarps + uniform_warp_index(); item < items; item += wstride) {
     const int r = (int)(item / jchunks), jc = (int)(item - (long)r * jchunks);
     const WalkEntry* krow = keys_g + (size_t)r * istride;
     const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     if (full_j)
-      walk_row<JPT, CH, true, VECW, STAGE>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * g.jout, (inv_out ? inv_out + (size_t)r * g.jout : nullptr), sbuf);
+      walk_row<JPT, CH, true, VECW>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * g.jout, (inv_out ? inv_out + (size_t)r * g.jout : nullptr), sbuf);
     else
-      walk_row<JPT, CH, false, VECW, STAGE>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * g.jout, (inv_out ? inv_out + (size_t)r * g.jout : nullptr), sbuf);
-    if (STAGE) __syncwarp();   // the next row's first block goes into the buffer this row may have read last
+      walk_row<JPT, CH, false, VECW>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * g.jout, (inv_out ? inv_out + (size_t)r * g.jout : nullptr), sbuf);
+    __syncwarp();   // the next row's first block goes into the buffer this row may have read last
   }
 }
 
-// The same items with the outputs of a lane held in pairs (walk_row2): a warp covers 64*JP outputs.
-template <int JP, bool STAGE>
+// The same items with the outputs of a lane held as a pair (walk_row2): a warp covers 64 outputs.
 __global__ void __launch_bounds__(kFwdThreads, 1024 / kFwdThreads)
 snn_walk2_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, int istride,
                  const float* w, float* __restrict__ out) {
   chain_wait();
   chain_next();
-  __shared__ __align__(16) WalkEntry stage[STAGE ? kFwdWarps * 64 : 1];   // two blocks of 32 list entries per warp
-  WalkEntry* sbuf = stage + (STAGE ? (threadIdx.x >> 5) * 64 : 0);
+  __shared__ __align__(16) WalkEntry stage[kFwdWarps * 64];   // two blocks of 32 list entries per warp
+  WalkEntry* sbuf = stage + (threadIdx.x >> 5) * 64;
   const int J = g.jout, R = g.R;
   const int lane = threadIdx.x & 31;
-  const int jchunks = (J + 64 * JP - 1) / (64 * JP);
-  const bool full_j = (J % (64 * JP)) == 0;
+  const int jchunks = (J + 63) / 64;
+  const bool full_j = (J % 64) == 0;
   float* __restrict__ y_out = out;
   float* __restrict__ inv_out = g.infer ? nullptr : out + (size_t)R * J;
   const long items = (long)R * jchunks;
@@ -577,10 +500,10 @@ snn_walk2_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g,
     const WalkEntry* krow = keys_g + (size_t)r * istride;
     const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     if (full_j)
-      walk_row2<JP, (JP >= 2 ? 4 : 8), true, STAGE>(g, krow, n, w, jc * 64 * JP, lane, y_out + (size_t)r * J, (inv_out ? inv_out + (size_t)r * J : nullptr), sbuf);
+      walk_row2<8, true>(g, krow, n, w, jc * 64, lane, y_out + (size_t)r * J, (inv_out ? inv_out + (size_t)r * J : nullptr), sbuf);
     else
-      walk_row2<JP, (JP >= 2 ? 4 : 8), false, STAGE>(g, krow, n, w, jc * 64 * JP, lane, y_out + (size_t)r * J, (inv_out ? inv_out + (size_t)r * J : nullptr), sbuf);
-    if (STAGE) __syncwarp();
+      walk_row2<8, false>(g, krow, n, w, jc * 64, lane, y_out + (size_t)r * J, (inv_out ? inv_out + (size_t)r * J : nullptr), sbuf);
+    __syncwarp();
   }
 }
 
@@ -595,7 +518,6 @@ constexpr int kSmemwWarps = kSmemwThreads / 32;
 constexpr long long kSmemwWaitClocks = 2000000000LL;   // SM clocks a CTA waits for its weight copies (about a second)
 __device__ unsigned g_walk_copy_timeouts = 0u;          // CTAs that gave up waiting since the library was loaded
 
-template <bool STAGE>
 __global__ void __launch_bounds__(kSmemwThreads, 1)
 snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g,
                        int istride, const float* w, float* __restrict__ out, unsigned wmul) {
@@ -657,9 +579,9 @@ snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nva
     const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     float* yr = y_out + (size_t)r * J;
     float* ir = inv_out ? inv_out + (size_t)r * J : nullptr;
-    if (staged) walk_row2<1, 8, true, STAGE, true>(g, krow, n, w, j0, lane, yr, ir, sbuf, ws_lane, wmul);
-    else walk_row2<1, 8, true, STAGE, false>(g, krow, n, w, j0, lane, yr, ir, sbuf);
-    if (STAGE) __syncwarp();
+    if (staged) walk_row2<8, true, true>(g, krow, n, w, j0, lane, yr, ir, sbuf, ws_lane, wmul);
+    else walk_row2<8, true, false>(g, krow, n, w, j0, lane, yr, ir, sbuf);
+    __syncwarp();
   }
   if (!staged) {
     __syncthreads();
@@ -676,26 +598,22 @@ size_t nvalid_bytes(const Geometry& g) { return nvalid_only_bytes(g) + 256; }
 
 template <int JPT, bool VECW>
 int launch_walk(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g, const float* w, float* out,
-                cudaStream_t s, bool stage) {
+                cudaStream_t s) {
   const int jchunks = (g.jout + 32 * JPT - 1) / (32 * JPT);
   const long items = (long)g.R * jchunks;
   long grid = (items + kFwdWarps - 1) / kFwdWarps;
   if (grid > 0x7fffffffL) grid = 0x7fffffffL;      // (a warp goes on to item + warps of the grid)
-  if (stage) (void)launch_chained(snn_walk_kernel<JPT, VECW, true>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
-  else (void)launch_chained(snn_walk_kernel<JPT, VECW, false>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
+  (void)launch_chained(snn_walk_kernel<JPT, VECW>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
 
-template <int JP>
-int launch_walk2(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g, const float* w, float* out,
-                 cudaStream_t s, bool stage) {
-  const int jchunks = (g.J + 64 * JP - 1) / (64 * JP);
+int launch_walk2(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g, const float* w, float* out, cudaStream_t s) {
+  const int jchunks = (g.J + 63) / 64;
   const long items = (long)g.R * jchunks;
   long grid = (items + kFwdWarps - 1) / kFwdWarps;
   if (grid > 0x7fffffffL) grid = 0x7fffffffL;      // (a warp goes on to item + warps of the grid)
-  if (stage) (void)launch_chained(snn_walk2_kernel<JP, true>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
-  else (void)launch_chained(snn_walk2_kernel<JP, false>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
+  (void)launch_chained(snn_walk2_kernel, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -715,22 +633,15 @@ bool walk_smemw_ok(const Geometry& g, const float* w, const LaunchInfo& li, size
 }
 
 int launch_walk2_smemw(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g, const float* w, float* out,
-                       const LaunchInfo& li, cudaStream_t s, bool stage, size_t smem, int wmul) {
+                       const LaunchInfo& li, cudaStream_t s, size_t smem, int wmul) {
   const int slices = g.J >> 6;
   long per_slice = li.num_sms / slices;                       // persistent: one CTA per SM
   const long need = ((long)g.R + kSmemwWarps - 1) / kSmemwWarps;
   if (per_slice > need) per_slice = need;
   if (per_slice < 1) per_slice = 1;
   const int grid = (int)(per_slice * slices);
-  if (stage) {
-    if (allow_smem<snn_walk2_smemw_kernel<true>>(smem) != cudaSuccess)
-      return E_CUDA;
-    (void)launch_chained(snn_walk2_smemw_kernel<true>, grid, kSmemwThreads, smem, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, (unsigned)wmul);
-  } else {
-    if (allow_smem<snn_walk2_smemw_kernel<false>>(smem) != cudaSuccess)
-      return E_CUDA;
-    (void)launch_chained(snn_walk2_smemw_kernel<false>, grid, kSmemwThreads, smem, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, (unsigned)wmul);
-  }
+  if (allow_smem<snn_walk2_smemw_kernel>(smem) != cudaSuccess) return E_CUDA;
+  (void)launch_chained(snn_walk2_smemw_kernel, grid, kSmemwThreads, smem, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, (unsigned)wmul);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -854,23 +765,14 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   auto cost = [&](int outputs, const WalkCost& c) {
     return walk_cost((double)g.R * ((g.J + outputs - 1) / outputs) / li.num_sms, c);
   };
-  int variant = 2, jsel = 0;                           // jsel: 1, 2, 4 outputs per lane (variants 2 and 3)
-  if (al8) {
-    variant = al16 && g.J > 64 && cost(128, kCostQuads) < cost(64, kCostPairs) ? 3 : 1;
-    jsel = variant == 3 ? 2 : 1;
-  } else {
-    for (int c = 1; c < 3; ++c)
-      if (cost(32 << c, kCostLanes[c]) < cost(32 << jsel, kCostLanes[jsel])) jsel = c;
-  }
-  if ((opt.walk_layout & 3) != 0) {
-    variant = opt.walk_layout & 3;
-    if (variant != 2 && !al8) variant = 2;
-    if (variant == 3) jsel = 2;
-  }
-  const bool stage = (opt.walk_layout & 4) == 0;   // list entries through shared memory (4: straight from global memory)
-  if (opt.walk_outputs != 0) jsel = opt.walk_outputs - 1;
-  if (jsel == 3 && !(variant == 3 && al16 && g.J % 8 == 0)) jsel = 2;   // eight outputs per lane exist only as consecutive outputs
-  if (variant == 3 && jsel == 2 && !al16) jsel = 1;
+  int variant = 2, lanes = 0;                          // lanes: variant 2 with 1, 2 or 4 outputs per lane
+  for (int c = 1; c < 3; ++c)
+    if (cost(32 << c, kCostLanes[c]) < cost(32 << lanes, kCostLanes[lanes])) lanes = c;
+  if (al8) variant = al16 && g.J > 64 && cost(128, kCostQuads) < cost(64, kCostPairs) ? 3 : 1;
+  // a layout that the call names, where the weights allow it
+  const int named = opt.walk_layout & 3;
+  if (named == 2 || (named == 1 && al8) || (named == 3 && al16)) variant = named;
+  if (opt.walk_outputs >= 1 && opt.walk_outputs <= 3) lanes = opt.walk_outputs - 1;
   size_t smemw_bytes = 0;
   int smemw_shift = 0;
   // weights staged in shared memory: where they fit, for fan-out 64 with enough rows to keep one CTA of 32 warps
@@ -883,20 +785,12 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     if (!(fparts & 2)) return OK;
     if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, li, s);
     if (rows) return launch_walk_rows(g, keys_g, nvalid_g, key_stride(g), w, out, own ? g.J > 32 && g.R >= 32768 : (opt.walk_layout & 64) != 0, li, s);
-    if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, s, stage, smemw_bytes, smemw_shift);
-    if (variant == 1) {
-      // pairs layout: 64 outputs per warp, or (walk_outputs 3) 128 as two pairs per lane
-      if (jsel >= 2) return launch_walk2<2>(g, keys_g, nvalid_g, w, out, s, stage);
-      return launch_walk2<1>(g, keys_g, nvalid_g, w, out, s, stage);
-    }
-    if (jsel == 0) return launch_walk<1, false>(g, keys_g, nvalid_g, w, out, s, stage);
-    if (variant == 3) {
-      if (jsel == 1) return launch_walk<2, true>(g, keys_g, nvalid_g, w, out, s, stage);
-      if (jsel == 2) return launch_walk<4, true>(g, keys_g, nvalid_g, w, out, s, stage);
-      return launch_walk<8, true>(g, keys_g, nvalid_g, w, out, s, stage);
-    }
-    if (jsel == 1) return launch_walk<2, false>(g, keys_g, nvalid_g, w, out, s, stage);
-    return launch_walk<4, false>(g, keys_g, nvalid_g, w, out, s, stage);
+    if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, s, smemw_bytes, smemw_shift);
+    if (variant == 1) return launch_walk2(g, keys_g, nvalid_g, w, out, s);
+    if (variant == 3) return launch_walk<4, true>(g, keys_g, nvalid_g, w, out, s);
+    if (lanes == 0) return launch_walk<1, false>(g, keys_g, nvalid_g, w, out, s);
+    if (lanes == 1) return launch_walk<2, false>(g, keys_g, nvalid_g, w, out, s);
+    return launch_walk<4, false>(g, keys_g, nvalid_g, w, out, s);
   };
 
   if (use_merge_lists(g, opt, li)) {

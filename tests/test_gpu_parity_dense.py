@@ -187,35 +187,34 @@ def test_dense_short_rows_by_the_register_network_match_the_row_sort(I):
 
 
 def test_walk_variants_agree_bit_for_bit():
-    """The library picks among several walk kernels (output pairs, consecutive outputs per lane, strided outputs,
-    1/2/4/8 outputs per lane); forced one by one through the measurement build they must give identical bits."""
+    """The library picks among several walk kernels (output pairs, four consecutive outputs per lane, 1, 2 or 4 strided
+    outputs per lane); forced one by one through the measurement build they must give identical bits."""
     import torch
     from snntc_2023_b200 import _lib, ops
     x, w = P.make_inputs(71, (50, 300), (301, 256), "cfg")
     params = O.fc_params(biasvolt=1.0)
     xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
     ref = ops.snn_fc(xd, wd, params)
-    for layout in (1, 2, 3, 5, 6, 7):      # 5..7: the same layouts reading list entries straight from global memory
-        for outputs in (0, 1, 2, 3, 4):
+    for layout in (1, 2, 3):
+        for outputs in (0, 1, 2, 3):       # (of layout 2)
             out = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=layout, walk_outputs=outputs))
             assert torch.equal(out, ref), "layout %d, outputs-per-lane choice %d" % (layout, outputs)
-    # the pairs walk with the weights of 64 outputs staged in shared memory by asynchronous bulk copies (8, 12: with and
-    # without staged list entries), one and several slices of 64 outputs, with and without bias row, more rows than warps
+    # the pairs walk with the weights of 64 outputs staged in shared memory by asynchronous bulk copies: one and several
+    # slices of 64 outputs, with and without bias row, more rows than warps
     for (B, I, J, bv) in ((50, 300, 256, 1.0), (2100, 37, 64, 1.0), (70, 577, 128, 0.0), (3, 799, 64, 1.0)):
         x, w = P.make_inputs(73 + I, (B, I), (I + (1 if bv else 0), J), "cfg")
         prm = O.fc_params(biasvolt=bv)
         xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
         ref = ops.snn_fc(xd, wd, prm, opts=_lib.options(walk_layout=1))
-        for layout in (8, 12):
-            assert torch.equal(ops.snn_fc(xd, wd, prm, opts=_lib.options(walk_layout=layout)), ref), (B, I, J, bv, layout)
+        assert torch.equal(ops.snn_fc(xd, wd, prm, opts=_lib.options(walk_layout=8)), ref), (B, I, J, bv)
     assert _lib.load_measure().snntc_copy_timeouts() == 0
-    # a fan-out that leaves the last block of eight-per-lane outputs partly empty
+    # a fan-out that leaves the last block of 64 and of 128 outputs partly empty
     x, w = P.make_inputs(72, (20, 100), (101, 1000), "test")
     params = O.fc_params(biasvolt=1.0)
     xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
     ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
-    for outputs in (2, 3, 4):
-        assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=3, walk_outputs=outputs)), ref)
+    for layout, outputs in ((1, 0), (2, 2), (2, 3), (3, 0)):
+        assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=layout, walk_outputs=outputs)), ref)
 
 
 def _small_grid_problem(seed, B, I, J, bv, lo, hi):
