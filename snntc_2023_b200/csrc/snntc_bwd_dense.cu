@@ -1,5 +1,5 @@
 // Both gradients of a dense layer (SnnFcGrad, snntc/snnfcgrad_kernels.cu.cc:15-225) in one launch behind the u kernel, for
-// up to a few thousand samples.
+// up to 2048 samples.
 //
 //   dX[r,i] = sum_j [x_ri <= y_rj] u_rj W[i,j]        dW[i,j] = sum_r [x_ri <= y_rj] (x_ri - y_rj) u_rj
 //   u[r,j]  = y[r,j] fired ? grad[r,j] * inv[r,j] : 0
@@ -19,7 +19,7 @@
 // Per element dX is a compare and a predicated FMA (bound by the half-rate compare pipe), dW a saturating FMA and half a
 // two-lane FMA (the scaled form of relu(y - x), snntc_backward.cu).
 // Measured (B200, dX + dW with the u kernel, before -> now): 784 -> 400 at 32 samples 85 -> 16 us, at 256: 98 -> 35, at 1024: 142 -> 99;
-// 4096 -> 512 at 256: 185 -> 123; 25 088 -> 1024 at 64: 550 -> 330.
+// 4096 -> 512 at 256: 166 -> 126; 25 088 -> 1024 at 64: 501 -> 332.
 #include "snntc_common.cuh"
 #include "snntc_ptx.cuh"
 

@@ -9,7 +9,7 @@
 // carry no gradient are skipped by a warp-uniform branch. What differs is how a stage gets into shared memory. In
 // snn_dw_skip_kernel 160 threads issue sixteen 16-byte copies each per stage, with the tap arithmetic and the
 // image-border tests in front of every copy -- a third of the instructions of the warps that also do the
-// arithmetic. Here one thread issues one tiled bulk copy per tap of the kernel window. A stage is a block of
+// arithmetic. Here one tiled bulk copy per tap of the kernel window, a lane each, does it. A stage is a block of
 // hseg x wseg = 16 receptive fields of one image (16 columns of one row of the output map, or 8 columns of two rows,
 // ... where the map is narrower than 16): through tap (kh, kw) they read a box of [rows][columns][channels] of the
 // NHWC image, which is exactly what a 4-D tensor map describes. Coordinates outside the image are legal for a load
@@ -22,8 +22,9 @@
 // holds the warps together stage by stage: how much a warp has to do depends on how many of its four channels carry
 // gradients, and with a barrier per stage every warp took the time of the busiest (the largest stall of the kernel).
 //
-// What bounds it: shared memory reads of x (about as many cycles as the arithmetic where few outputs carry a
-// gradient), then issue. With dW of 262 144 rows of 577 x 64, 12 % of the outputs carrying a gradient, 353 -> 256 us
+// What bounds it: waiting for a stage's copies (65 536 rows of 577 x 64, 12 % of the gradients, 100 us: of the warps per issue 2.98 wait
+// for copies, 2.13 for fixed latencies, 1.31 for shared memory; L1 and shared memory 53 % busy, issue 40 %): the taps' boxes overlap,
+// so that a stage brings every pixel in up to nine times. With dW of 262 144 rows of 577 x 64, 12 % of the outputs carrying a gradient, 353 -> 256 us
 // against two stages, a CTA barrier per stage, 32 outputs per CTA and eight waves of CTAs; 200 704 x 1153 x 128 790 -> 658 us.
 //
 // The x tile of a stage is laid out [tap][row][channel] (one box after the other), so a fan-in tile is made of

@@ -592,7 +592,7 @@ snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nva
 int key_stride(const Geometry& g) { return (g.I + 3) & ~3; }  // a multiple of four entries: rows of keys start 32-byte aligned
 
 size_t keys_bytes(const Geometry& g) { return (size_t)g.R * key_stride(g) * sizeof(u64); }
-// list lengths, then 256 bytes that hold the weight bound of the walk (one float)
+// list lengths, then 256 bytes that hold the weight bound of the walk (up to 32 partial sums)
 size_t nvalid_only_bytes(const Geometry& g) { return ((size_t)g.R * sizeof(int) + 255) & ~(size_t)255; }
 size_t nvalid_bytes(const Geometry& g) { return nvalid_only_bytes(g) + 256; }
 
@@ -745,7 +745,8 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     const bool in_l1 = (size_t)(g.I + 1) * g.J * sizeof(float) <= (size_t)128 << 10;
     rows = warps_per_sm >= (lanes == 16 ? 48 : (lanes == 8 ? 14 : (in_l1 ? 6 : 10)));
     // (65 536 rows of 576 x 64: 364 us with the pairs walk and its weights in shared memory, 380 so, but 16 384 rows 130 and 113;
-    // 262 144 of 27 x 64: 222, 208, but 59 400 of 64 x 64 75, 83)
+    // 262 144 of 27 x 64: 222, 208, but 59 400 of 64 x 64 75, 83; where the weights do not fit shared memory the pairs walk from
+    // global memory is ahead too: 65 536 of 900 x 64 649, 672)
     if (g.jout == 64 && g.I >= 64 && g.R >= 32768) rows = false;
   }
   if ((fparts & 2) && (!ring || pad)) {   // the walk's bound on the weight sums (see walk_tolerance_base)

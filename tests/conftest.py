@@ -33,13 +33,11 @@ def _built_oracle():
 
 
 def pytest_sessionfinish(session, exitstatus):
-    """How much of every forward tensor was held to which bound (oracle/parity.py) goes to a report beside the
-    other outputs of a GPU run and, in short, to the terminal."""
+    """How much of every forward tensor was held to which bound (oracle/parity.py) goes to the terminal in short and, where
+    SNNTC_REPORT_DIR names a folder, to a report in it."""
     from oracle import parity
     if not parity.REPORT:
         return
-    try:
-        parity.dump_report(os.path.join(ROOT, os.environ.get("SNNTC_REPORT_DIR", "gpurun_out"), "parity_report.json"))
-    except OSError:
-        pass
+    if os.environ.get("SNNTC_REPORT_DIR"):
+        parity.dump_report(os.path.join(ROOT, os.environ["SNNTC_REPORT_DIR"], "parity_report.json"))
     print("\nparity summary: %s" % (parity.summary(),))
