@@ -649,7 +649,7 @@ int launch_walk2_smemw(const Geometry& g, const WalkEntry* keys_g, const int* nv
 // What a walk from global memory takes with n warps to an SM, in microseconds for rows of 500 inputs of which half spike: 32 warps
 // run at once, each full wave of them takes `wave`, the last one first + n * warp. Fitted to 100 to 16 000 rows x fan-outs
 // 68 to 1000 (n = 2 to 3500; within 5 % from n = 8 on). What counts is where two of them cross: at 300 to 4096 inputs, half or all
-// of them spiking, 33 to 70 warps of 64 outputs per SM, pairs against quads were 1.15 times as slow on average (700 rows of
+// of them spiking, 33 to 70 warps of 64 outputs per SM, pairs took 1.11 times the quads' time on average, in 15 of 180 sizes less (700 rows of
 // 784 -> 512: 128 against 103 us all spiking, 74 against 78 half; 1024 of 784 -> 400: 144 against 126), below 32 the quads
 // (300 rows of 500 -> 400: 29 against 35 us). What the rule cannot know is whether an output never fires, for which a warp walks
 // to the end of its list: with one such output in the layer the pairs lose less of the fan-out to it (2450 of 2305 -> 128: 179
