@@ -11,9 +11,9 @@
 //      registers, in sorted order, bias first, with the arithmetic of the reference kernel
 //      (snntc/snnfc_kernels.cu.cc:33-69); the causality test is the sign of q = ysum - x*wsum per step -- one FMA
 //      per output, the lane's smallest q as an integer, one warp vote -- backed by the reference's exact
-//      division-free comparisons whenever it turns non-positive in any lane (see walk_row). Three layouts of a
-//      lane's outputs: a pair in one 64-bit register (walk_row2), four consecutive outputs read by one 16-byte load, or
-//      outputs lane + 32*m (odd fan-out, unaligned weights).
+//      division-free comparisons wherever the sign is not certain (PairWalk in snntc_walk.cuh, walk_row). Three layouts of
+//      a lane's outputs: one pair or two pairs of neighbours in 64-bit registers (walk_pairs), or outputs lane + 32*m
+//      (odd fan-out, unaligned weights).
 #include "snntc_common.cuh"
 #include "snntc_walk.cuh"
 
@@ -21,6 +21,7 @@
 #include <limits.h>
 #include <math.h>
 #include <math_constants.h>
+#include <type_traits>
 
 namespace snntc {
 
@@ -124,7 +125,7 @@ snn_wbound_kernel(const float* w, int rows, int J, int rows_per_cta, float* __re
 // ulp of zero, or a NEGATIVE denominator, which inputs below the bias input can produce and for which the
 // reference fires on the way back up through zero -- makes the lane "sticky": the exact tests run again at
 // the next step whatever q is, until no live output of the lane is in that state any more.
-template <int JPT, int CH, bool FULL, bool VECW>
+template <int JPT, int CH, bool FULL>
 __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ents, int nvalid,
                                          const float* w, int jbase, int lane,
                                          float* __restrict__ y_row, float* __restrict__ inv_row,
@@ -136,11 +137,9 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
   int livemask[JPT];
 #pragma unroll
   for (int m = 0; m < JPT; ++m) {
-    // VECW: a lane owns four consecutive outputs and reads them with one 16-byte load (J % 4 == 0, so a lane is wholly
-    // inside or wholly outside the row); otherwise outputs lane + 32*m, 4-byte loads
-    const int j = VECW ? jbase + JPT * lane + m : jbase + lane + 32 * m;
+    const int j = jbase + lane + 32 * m;
     jok[m] = FULL || j < g.jout;
-    jl[m] = jok[m] ? j : (VECW ? J - JPT + m : J - 1);   // (padding behind jout: weights of zero, never stored)
+    jl[m] = jok[m] ? j : J - 1;   // (padding behind jout: weights of zero, never stored)
     wsum[m] = -g.theta;
     ysum[m] = 0.f;
     if (g.has_bias) {  // the bias input (value biasvolt, weight row I) is always consumed first
@@ -163,20 +162,11 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
   const float tolbase = walk_tolerance_base(g);
   int qlim = 0;           // bits of the largest q that still goes to the exact tests (see walk_tolerance_base)
 
-  const float* wl = w + (VECW ? jl[0] : (FULL ? jbase + lane : 0));
-  // VECW: addressed by a 32-bit element offset from the (uniform) weight base, widened before the scaling to
-  // bytes -- measured faster than a 64-bit per-lane pointer plus the entry's offset
-  const unsigned lane_off = (unsigned)jl[0];
-  const char* wbase = reinterpret_cast<const char*>(w);
+  const float* wl = w + (FULL ? jbase + lane : 0);
   auto load_weights = [&](unsigned eoff, float (&wv)[JPT]) {
     const float* wrow = wl + eoff;
-    if constexpr (VECW) {
-      const float4 v = ld_plain(reinterpret_cast<const float4*>(wbase + (size_t)(eoff + lane_off) * 4u));
-      wv[0] = v.x; wv[1] = v.y; wv[2] = v.z; wv[3] = v.w;
-    } else {
 #pragma unroll
-      for (int m = 0; m < JPT; ++m) wv[m] = FULL ? ld_plain(wrow + 32 * m) : ld_plain(wrow + jl[m]);
-    }
+    for (int m = 0; m < JPT; ++m) wv[m] = FULL ? ld_plain(wrow + 32 * m) : ld_plain(wrow + jl[m]);
   };
 
   // one step for all JPT outputs of this lane: sign test, (rarely) exact test, then consume
@@ -283,7 +273,7 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
       if (yv >= g.maxv) { yv = g.maxv; iv = 0.f; }
     }
     if (jok[m]) {
-      const int j = VECW ? jbase + JPT * lane + m : jbase + lane + 32 * m;
+      const int j = jbase + lane + 32 * m;
       y_row[j] = yv;
       if (inv_row != nullptr) inv_row[j] = iv;
       if (g.khist != nullptr) atomicAdd(g.khist + (yv < g.maxv ? entries_below(ents, nvalid, yv) : g.I + 1), 1);
@@ -291,166 +281,114 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
   }
 }
 
-// ---- two outputs per 64-bit register ---------------------------------------------------------------
-// sm_100 has two-lane FP32 add / sub / fma on 64-bit register pairs: one issue slot, two results, each
-// rounded exactly like the scalar instruction. A pair holds outputs (j, j+1) of one lane.
-// walk_row with the outputs of a lane held as one pair (j, j+1), j = jbase + 2*lane: the three FP32 operations of a step (q, the
-// weight sum, the weighted sum) are one packed instruction and a weight-row read is one 8-byte load. The weight sum is carried
-// NEGATED (nws = theta - sum w), so that q = fma(x, nws, ysum) needs no negated copy of x; negation is exact, so every value is
-// bit for bit the scalar walk's -- except the sign of an exactly cancelled sum (+0 on both sides), which is why the sum is
-// read back as 0 - nws: 1/(+0) = +inf clamps to "no spike", 1/(-0) would not. Requires J even and the
-// weights 8-byte aligned.
+// ---- outputs in pairs, two to a 64-bit register (PairWalk in snntc_walk.cuh): one pair of neighbouring outputs per lane (P = 1, 64 per
+// warp) or two (P = 2, 128 per warp). Requires J a multiple of 2 * P and the weights aligned to 8 * P bytes.
 // WS: the weights of this warp's 64 outputs sit in shared memory as [fan-in row][64] (see snn_walk2_smemw_kernel);
 // `ws_lane` is the shared-memory byte address of this lane's pair in row 0 and `wmul` = 256 / J (J = 64, 128 or 256): a
 // list entry's element offset (source index * J) times wmul is the row's byte offset in the slice -- one integer
 // multiply-add on the FMA pipe per weight read.
-template <int CH, bool FULL, bool WS = false>
-__device__ __forceinline__ void walk_row2(const Geometry& g, const WalkEntry* ents, int nvalid,
-                                          const float* w, int jbase, int lane,
-                                          float* __restrict__ y_row, float* __restrict__ inv_row,
-                                          WalkEntry* __restrict__ sbuf, unsigned ws_lane = 0u, unsigned wmul = 0u) {
-  const int J = g.J;
-  const int j0 = jbase + 2 * lane;                        // this lane's outputs: j0, j0 + 1
-  const int jl = FULL || j0 < g.jout ? j0 : J - 2;
-  uint64_t nws, ys;
-  float wfin[2], yfin[2];
-  int live[2] = {-1, -1};
-  {
-    float n0 = g.theta, n1 = g.theta, y0 = 0.f, y1 = 0.f;
-    if (g.has_bias) {  // the bias input (value biasvolt, weight row I) is always consumed first
-      const float2 wb = ld_plain(reinterpret_cast<const float2*>(w + (size_t)g.I * J + jl));
-      n0 -= wb.x; n1 -= wb.y;
-      y0 = g.biasvolt * wb.x; y1 = g.biasvolt * wb.y;
-    }
-    wfin[0] = 0.f - n0; wfin[1] = 0.f - n1;
-    yfin[0] = y0; yfin[1] = y1;
-    if (!FULL) {     // no output: parked from the start like one that has fired, or the walk would wait for it
-      if (j0 >= g.jout) { live[0] = 0; n0 = CUDART_INF_F; }
-      if (j0 + 1 >= g.jout) { live[1] = 0; n1 = CUDART_INF_F; }
-    }
-    nws = pack2(n0, n1);
-    ys = pack2(y0, y1);
-  }
-  float xprev = g.has_bias ? g.biasvolt : 0.f;
-
-  int sticky = INT_MAX;   // INT_MIN while some live output of this lane must be tested exactly at the next step
-  const float tolbase = walk_tolerance_base(g);
-  int qlim = 0;           // bits of the largest q that still goes to the exact tests (see walk_tolerance_base)
-  auto step = [&](const float x, const float xprev, const uint64_t wv) {
-    const uint64_t x2 = pack2(x, x);
-    int q[2];
-    unpack2i(fma2(x2, nws, ys), q[0], q[1]);
-    if (__builtin_expect(__any_sync(0xffffffffu, imin3(q[0], q[1], sticky) <= qlim), 0)) {
-      // rare path: the reference's own rounded comparisons for the live outputs (see walk_row)
-      bool again = false;
-      float n[2], y[2];
-      unpack2(nws, n[0], n[1]);
-      unpack2(ys, y[0], y[1]);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        // usually one output of one lane is concerned: skip the other half with a warp-uniform test
-        if (!__any_sync(0xffffffffu, (q[h] <= qlim) | (sticky < 0))) continue;
-        const float wsum = 0.f - n[h];   // not -n: an exactly cancelled sum must read +0 as in the scalar walk
-        const bool lv = live[h] != 0;
-        const bool fire = lv & ratio_gt(y[h], wsum, xprev) & ratio_le(y[h], wsum, x);
-        if (fire) {
-          live[h] = 0;           // spike lies in (previous input, x]: keep the sums aside ...
-          wfin[h] = wsum;
-          yfin[h] = y[h];
-          n[h] = CUDART_INF_F;   // ... and park the running weight sum where q stays +inf
-        }
-        again |= lv & !fire & (q[h] <= qlim);
-      }
-      nws = pack2(n[0], n[1]);
-      sticky = again ? INT_MIN : INT_MAX;
-    }
-    nws = sub2(nws, wv);
-    ys = fma2(x2, wv, ys);
-  };
-  const unsigned lane_off = (unsigned)jl;   // element offset of this lane's pair within a weight row
-  bool all_done = false;
-  auto load_row = [&](unsigned eoff) -> uint64_t {
+// The list goes through shared memory 32 entries at a time (sbuf: two blocks), one coalesced read per lane issued a block ahead
+// instead of an L2 round trip per step. CH entries and their weight rows are read together.
+template <int P, int CH, bool FULL, bool WS = false>
+__device__ __forceinline__ void walk_pairs(const Geometry& g, const WalkEntry* ents, int nvalid, const float* w, int jbase, int lane,
+                                           float* __restrict__ y_row, float* __restrict__ inv_row, WalkEntry* __restrict__ sbuf,
+                                           float* __restrict__ fin, unsigned ws_lane = 0u, unsigned wmul = 0u) {
+  const int j0 = jbase + 2 * P * lane;                    // this lane's outputs: 2 * P from j0 on
+  const unsigned lane_off = (unsigned)(FULL || j0 < g.J ? j0 : g.J - 2 * P);
+  const char* wbase = reinterpret_cast<const char*>(w);
+  // a 32-bit element offset from the (uniform) weight base, widened before the scaling to bytes: a 64-bit pointer per lane plus the
+  // entry's offset takes two instructions more per step
+  auto load_row = [&](unsigned eoff, uint64_t (&wv)[P]) {
     if constexpr (WS) {
-      uint64_t v;
-      asm("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(eoff * wmul + ws_lane));
-      return v;
+      static_assert(P == 1, "slices of 64 outputs");
+      asm("ld.shared.b64 %0, [%1];" : "=l"(wv[0]) : "r"(eoff * wmul + ws_lane));
+    } else if constexpr (P == 1) {
+      wv[0] = ld_plain(reinterpret_cast<const unsigned long long*>(wbase + (size_t)(eoff + lane_off) * 4u));
     } else {
-      // a 32-bit element offset from the (uniform) weight base measured faster than a 64-bit per-lane pointer plus the
-      // entry's offset
-      return ld_plain(reinterpret_cast<const unsigned long long*>(
-          reinterpret_cast<const char*>(w) + (size_t)(eoff + lane_off) * 4u));
+      const ulonglong2 v = ld_plain(reinterpret_cast<const ulonglong2*>(wbase + (size_t)(eoff + lane_off) * 4u));
+      wv[0] = v.x; wv[1] = v.y;
     }
   };
-  static_assert(CH % 2 == 0, "entries are fetched two at a time");
-  auto chunk = [&](const WalkEntry* cur) {
-    float xs[CH];
-    uint64_t wv[CH];
+  PairWalk<P> pw;
+  pw.fin = fin + lane;
+  {
+    float wb[2 * P];
+    bool ok[2 * P];
 #pragma unroll
-    for (int u = 0; u < CH; u += 2) {
-      const uint4 e2 = *reinterpret_cast<const uint4*>(cur + u);
-      xs[u] = __uint_as_float(e2.x);
-      wv[u] = load_row(e2.y);
-      xs[u + 1] = __uint_as_float(e2.z);
-      wv[u + 1] = load_row(e2.w);
+    for (int m = 0; m < 2 * P; ++m) {   // the bias input (value biasvolt, weight row I) is always consumed first
+      wb[m] = g.has_bias ? ld_plain(w + (size_t)g.I * g.J + lane_off + m) : 0.f;
+      ok[m] = FULL || j0 + m < g.jout;
     }
-    qlim = __float_as_int(tolbase * fmaxf(fabsf(xs[0]), fabsf(xs[CH - 1])));   // inputs ascend: |x| peaks at an end
-#pragma unroll
-    for (int u = 0; u < CH; ++u) step(xs[u], u == 0 ? xprev : xs[u > 0 ? u - 1 : 0], wv[u]);
-    xprev = xs[CH - 1];
-  };
-  auto single = [&](const WalkEntry e) {
-    const uint64_t wv = load_row(e.y);
-    qlim = __float_as_int(tolbase * fabsf(__uint_as_float(e.x)));
-    step(__uint_as_float(e.x), xprev, wv);
-    xprev = __uint_as_float(e.x);
-  };
-  // the list through shared memory, 32 entries at a time, read a block ahead (see walk_row)
+    // (the smallest input is read by all lanes from one address: taken out of lane 0's entry below it cost a divergence check in
+    // front of every vote)
+    pw.start(g, walk_tolerance_base(g), nvalid > 0 ? __uint_as_float(ld_l2(ents).x) : 0.f, wb, ok);
+  }
   WalkEntry pre = make_uint2(0u, 0u);
   if (lane < nvalid) pre = ld_l2(ents + lane);
-  int b = 0;
-  for (int base = 0; base < nvalid && !all_done; base += 32, b ^= 32) {
-    sbuf[b + lane] = pre;
-    __syncwarp();
-    if (base + 32 + lane < nvalid) pre = ld_l2(ents + base + 32 + lane);
-    const int nb = min(32, nvalid - base);
-    const WalkEntry* cur = sbuf + b;
+  // entry k of the list is staged at k % 64, the input in front of the first one at 63
+  if (lane == 0) sbuf[63] = make_uint2(__float_as_uint(g.has_bias ? g.biasvolt : 0.f), 0u);
+  auto inputs = [&](int at) { return make_float2(__uint_as_float(sbuf[at].x), __uint_as_float(sbuf[(at + 63) & 63].x)); };
+  bool flipped = false;
+  auto block = [&](int base, auto flip_c) {
+    constexpr bool FLIP = decltype(flip_c)::value;
+    constexpr int N = FLIP ? 2 : CH;                      // (FLIP with four: the walk spills more, 4 % slower)
+    const int b = base & 32, nb = min(32, nvalid - base);
+    pw.margin(__uint_as_float(sbuf[b].x), __uint_as_float(sbuf[b + nb - 1].x));   // inputs ascend: |x| peaks at an end
     int kk = 0;
 #pragma unroll 1
-    for (; kk + CH <= nb; kk += CH) chunk(cur + kk);
-    for (; kk < nb; ++kk) single(cur[kk]);
-    all_done = !__any_sync(0xffffffffu, (live[0] | live[1]) != 0);   // one "has every output fired" vote per block
-  }
-
-  float n[2], y[2];
-  unpack2(nws, n[0], n[1]);
-  unpack2(ys, y[0], y[1]);
+    for (; kk + N <= nb; kk += N) {
+      const int at = b + kk;
+      uint64_t x2[N], wv[N][P];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    // an output that stopped has fired; one that consumed every input fires iff it is armed
-    bool fired = true;
-    float ws = wfin[h], yy = yfin[h];
-    if (live[h]) {
-      ws = 0.f - n[h]; yy = y[h];
-      fired = ratio_gt(yy, ws, xprev);
+      for (int u = 0; u < N; u += 2) {
+        const uint4 e2 = *reinterpret_cast<const uint4*>(sbuf + at + u);
+        x2[u] = pack2(__uint_as_float(e2.x), __uint_as_float(e2.x));
+        load_row(e2.y, wv[u]);
+        x2[u + 1] = pack2(__uint_as_float(e2.z), __uint_as_float(e2.z));
+        load_row(e2.w, wv[u + 1]);
+      }
+      if constexpr (FLIP) {
+#pragma unroll
+        for (int u = 0; u < N; ++u) pw.template step<true>(x2[u], wv[u], [&] { return inputs(at + u); });
+      } else {
+#pragma unroll
+        for (int u = 0; u < N; u += 2)
+          pw.step2(x2[u], wv[u], x2[u + 1], wv[u + 1], [&] { return inputs(at + u); }, [&] { return inputs(at + u + 1); });
+      }
     }
-    float yv = g.maxv, iv = 0.f;
-    if (fired) {
-      iv = __fdividef(1.0f, ws);
-      yv = yy * iv;
-      if (yv >= g.maxv) { yv = g.maxv; iv = 0.f; }
+#pragma unroll 1
+    for (; kk < nb; ++kk) {
+      const WalkEntry e = sbuf[b + kk];
+      uint64_t wv[P];
+      load_row(e.y, wv);
+      pw.template step<FLIP>(pack2(__uint_as_float(e.x), __uint_as_float(e.x)), wv, [&] { return inputs(b + kk); });
     }
-    const int j = j0 + h;
-    if (FULL || j < g.jout) {
-      y_row[j] = yv;
-      if (inv_row != nullptr) inv_row[j] = iv;
-      if (g.khist != nullptr) atomicAdd(g.khist + (yv < g.maxv ? entries_below(ents, nvalid, yv) : g.I + 1), 1);
-    }
+    flipped = pw.template flip<FLIP>(__uint_as_float(sbuf[b + nb - 1].x));
+  };
+  for (int base = 0; base < nvalid; base += 32) {
+    sbuf[(base & 32) + lane] = pre;
+    __syncwarp();
+    if (base + 32 + lane < nvalid) pre = ld_l2(ents + base + 32 + lane);
+    if (__builtin_expect(flipped, 0)) block(base, std::true_type{});
+    else block(base, std::false_type{});
+    if (!__any_sync(0xffffffffu, pw.any_live())) break;   // every output has fired
+  }
+  const float xprev = __uint_as_float(sbuf[(nvalid + 63) & 63].x);
+#pragma unroll
+  for (int m = 0; m < 2 * P; ++m) {
+    const int j = j0 + m;
+    if (!FULL && j >= g.jout) continue;
+    float y, inv;
+    pw.finish(g, m, xprev, y, inv);
+    y_row[j] = y;
+    if (inv_row != nullptr) inv_row[j] = inv;
+    if (g.khist != nullptr) atomicAdd(g.khist + (y < g.maxv ? entries_below(ents, nvalid, y) : g.I + 1), 1);
   }
 }
 
 // ------------------------------------------------------------------------------------------- kernels
 // Walk kernel: every warp takes (row, block of 32*JPT outputs) items, adjacent warps share a row.
-template <int JPT, bool VECW>
+template <int JPT>
 __global__ void __launch_bounds__(kFwdThreads, 1024 / kFwdThreads)   // 64 registers, 32 warps per SM
 snn_walk_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, int istride,
                 const float* w, float* __restrict__ out) {
@@ -472,25 +410,29 @@ snn_walk_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, 
     const WalkEntry* krow = keys_g + (size_t)r * istride;
     const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     if (full_j)
-      walk_row<JPT, CH, true, VECW>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * g.jout, (inv_out ? inv_out + (size_t)r * g.jout : nullptr), sbuf);
+      walk_row<JPT, CH, true>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * g.jout, (inv_out ? inv_out + (size_t)r * g.jout : nullptr), sbuf);
     else
-      walk_row<JPT, CH, false, VECW>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * g.jout, (inv_out ? inv_out + (size_t)r * g.jout : nullptr), sbuf);
+      walk_row<JPT, CH, false>(g, krow, n, w, jc * 32 * JPT, lane, y_out + (size_t)r * g.jout, (inv_out ? inv_out + (size_t)r * g.jout : nullptr), sbuf);
     __syncwarp();   // the next row's first block goes into the buffer this row may have read last
   }
 }
 
-// The same items with the outputs of a lane held as a pair (walk_row2): a warp covers 64 outputs.
+// The same items with the outputs of a lane held in pairs (walk_pairs): a warp covers 64 * P outputs.
+template <int P>
 __global__ void __launch_bounds__(kFwdThreads, 1024 / kFwdThreads)
-snn_walk2_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, int istride,
-                 const float* w, float* __restrict__ out) {
+snn_walk_pairs_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, int istride, const float* w,
+                      float* __restrict__ out) {
   chain_wait();
   chain_next();
   __shared__ __align__(16) WalkEntry stage[kFwdWarps * 64];   // two blocks of 32 list entries per warp
+  __shared__ float fins[kFwdWarps * PairWalk<P>::kFloats];
+  constexpr int CH = P == 2 ? 4 : 8;
   WalkEntry* sbuf = stage + (threadIdx.x >> 5) * 64;
+  float* fin = fins + (threadIdx.x >> 5) * PairWalk<P>::kFloats;
   const int J = g.jout, R = g.R;
   const int lane = threadIdx.x & 31;
-  const int jchunks = (J + 63) / 64;
-  const bool full_j = (J % 64) == 0;
+  const int jchunks = (J + 64 * P - 1) / (64 * P);
+  const bool full_j = (J % (64 * P)) == 0;
   float* __restrict__ y_out = out;
   float* __restrict__ inv_out = g.infer ? nullptr : out + (size_t)R * J;
   const long items = (long)R * jchunks;
@@ -499,11 +441,11 @@ snn_walk2_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g,
     const int r = (int)(item / jchunks), jc = (int)(item - (long)r * jchunks);
     const WalkEntry* krow = keys_g + (size_t)r * istride;
     const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
-    if (full_j)
-      walk_row2<8, true>(g, krow, n, w, jc * 64, lane, y_out + (size_t)r * J, (inv_out ? inv_out + (size_t)r * J : nullptr), sbuf);
-    else
-      walk_row2<8, false>(g, krow, n, w, jc * 64, lane, y_out + (size_t)r * J, (inv_out ? inv_out + (size_t)r * J : nullptr), sbuf);
-    __syncwarp();
+    float* yr = y_out + (size_t)r * J;
+    float* ir = inv_out ? inv_out + (size_t)r * J : nullptr;
+    if (full_j) walk_pairs<P, CH, true>(g, krow, n, w, jc * 64 * P, lane, yr, ir, sbuf, fin);
+    else walk_pairs<P, CH, false>(g, krow, n, w, jc * 64 * P, lane, yr, ir, sbuf, fin);
+    __syncwarp();   // the next row's first block goes into the buffer this row may have read last
   }
 }
 
@@ -529,6 +471,7 @@ snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nva
   const int rows_w = g.I + g.has_bias;
   float* ws = reinterpret_cast<float*>(smem_raw);                                        // [rows_w][64]
   WalkEntry* stage = reinterpret_cast<WalkEntry*>(smem_raw + (size_t)rows_w * 256);      // [32 warps][64 entries]
+  float* fins = reinterpret_cast<float*>(stage + kSmemwWarps * 64);                      // [32 warps][PairWalk<1>::kFloats]
   const int lane = threadIdx.x & 31;
   const int warp = uniform_warp_index();
   const int slices = J >> 6;
@@ -552,7 +495,7 @@ snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nva
   }
   // Every thread waits for the copies itself (phase 0 of the barrier), for at most about a second of SM clocks. If
   // they have not arrived by then the CTA counts a timeout and walks with the weights read from global memory, like
-  // snn_walk2_kernel; before it leaves it gives the copies the same time once more, so that none is in flight into
+  // snn_walk_pairs_kernel; before it leaves it gives the copies the same time once more, so that none is in flight into
   // shared memory that the next CTA on this SM owns.
   auto copies_arrived = [&]() {
     const long long t0 = clock64();
@@ -569,6 +512,7 @@ snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nva
   if (!staged && threadIdx.x == 0) atomicAdd(&g_walk_copy_timeouts, 1u);
 
   WalkEntry* sbuf = stage + warp * 64;
+  float* fin = fins + warp * PairWalk<1>::kFloats;
   float* __restrict__ y_out = out;
   float* __restrict__ inv_out = g.infer ? nullptr : out + (size_t)R * J;
   const unsigned ws_lane = smem_u32(ws) + 8u * (unsigned)lane;
@@ -579,8 +523,8 @@ snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nva
     const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     float* yr = y_out + (size_t)r * J;
     float* ir = inv_out ? inv_out + (size_t)r * J : nullptr;
-    if (staged) walk_row2<8, true, true>(g, krow, n, w, j0, lane, yr, ir, sbuf, ws_lane, wmul);
-    else walk_row2<8, true, false>(g, krow, n, w, j0, lane, yr, ir, sbuf);
+    if (staged) walk_pairs<1, 8, true, true>(g, krow, n, w, j0, lane, yr, ir, sbuf, fin, ws_lane, wmul);
+    else walk_pairs<1, 8, true, false>(g, krow, n, w, j0, lane, yr, ir, sbuf, fin);
     __syncwarp();
   }
   if (!staged) {
@@ -596,24 +540,24 @@ size_t keys_bytes(const Geometry& g) { return (size_t)g.R * key_stride(g) * size
 size_t nvalid_only_bytes(const Geometry& g) { return ((size_t)g.R * sizeof(int) + 255) & ~(size_t)255; }
 size_t nvalid_bytes(const Geometry& g) { return nvalid_only_bytes(g) + 256; }
 
-template <int JPT, bool VECW>
+template <int JPT>
 int launch_walk(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g, const float* w, float* out,
                 cudaStream_t s) {
   const int jchunks = (g.jout + 32 * JPT - 1) / (32 * JPT);
   const long items = (long)g.R * jchunks;
   long grid = (items + kFwdWarps - 1) / kFwdWarps;
   if (grid > 0x7fffffffL) grid = 0x7fffffffL;      // (a warp goes on to item + warps of the grid)
-  (void)launch_chained(snn_walk_kernel<JPT, VECW>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
+  (void)launch_chained(snn_walk_kernel<JPT>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
 
-int launch_walk2(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g, const float* w, float* out, cudaStream_t s) {
-  const int jchunks = (g.J + 63) / 64;
-  const long items = (long)g.R * jchunks;
+template <int P>
+int launch_walk_pairs(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g, const float* w, float* out, cudaStream_t s) {
+  const long items = (long)g.R * ((g.jout + 64 * P - 1) / (64 * P));
   long grid = (items + kFwdWarps - 1) / kFwdWarps;
   if (grid > 0x7fffffffL) grid = 0x7fffffffL;      // (a warp goes on to item + warps of the grid)
-  (void)launch_chained(snn_walk2_kernel, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
+  (void)launch_chained(snn_walk_pairs_kernel<P>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -624,7 +568,7 @@ bool walk_smemw_ok(const Geometry& g, const float* w, const LaunchInfo& li, size
   if ((g.J != 64 && g.J != 128 && g.J != 256) || (reinterpret_cast<uintptr_t>(w) & 15) != 0) return false;
   if (g.jout != g.J) return false;      // J is the kernel's output stride too
   const size_t rows_w = (size_t)g.I + g.has_bias;
-  const size_t smem = rows_w * 256 + (size_t)kSmemwWarps * 64 * sizeof(WalkEntry);
+  const size_t smem = rows_w * 256 + (size_t)kSmemwWarps * (64 * sizeof(WalkEntry) + PairWalk<1>::kFloats * sizeof(float));
   if (smem + 2048 > (size_t)li.max_smem_optin || rows_w * 256 >= (1u << 20)) return false;
   if ((g.J >> 6) > li.num_sms) return false;
   *smem_bytes = smem;
@@ -787,11 +731,11 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, li, s);
     if (rows) return launch_walk_rows(g, keys_g, nvalid_g, key_stride(g), w, out, own ? g.J > 32 && g.R >= 32768 : (opt.walk_layout & 64) != 0, li, s);
     if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, s, smemw_bytes, smemw_shift);
-    if (variant == 1) return launch_walk2(g, keys_g, nvalid_g, w, out, s);
-    if (variant == 3) return launch_walk<4, true>(g, keys_g, nvalid_g, w, out, s);
-    if (lanes == 0) return launch_walk<1, false>(g, keys_g, nvalid_g, w, out, s);
-    if (lanes == 1) return launch_walk<2, false>(g, keys_g, nvalid_g, w, out, s);
-    return launch_walk<4, false>(g, keys_g, nvalid_g, w, out, s);
+    if (variant == 1) return launch_walk_pairs<1>(g, keys_g, nvalid_g, w, out, s);
+    if (variant == 3) return launch_walk_pairs<2>(g, keys_g, nvalid_g, w, out, s);
+    if (lanes == 0) return launch_walk<1>(g, keys_g, nvalid_g, w, out, s);
+    if (lanes == 1) return launch_walk<2>(g, keys_g, nvalid_g, w, out, s);
+    return launch_walk<4>(g, keys_g, nvalid_g, w, out, s);
   };
 
   if (use_merge_lists(g, opt, li)) {

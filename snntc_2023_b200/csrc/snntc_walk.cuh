@@ -3,6 +3,9 @@
 #include "snntc_common.cuh"
 #include "snntc_ptx.cuh"
 
+#include <limits.h>
+#include <math_constants.h>
+
 namespace snntc {
 
 // "ysum/wsum > c" without a division, as the reference evaluates it after consuming input c
@@ -34,5 +37,260 @@ __device__ __forceinline__ int entries_below(const WalkEntry* ents, int n, float
 // the result is <= 0 exactly when one of the floats is negative, -0 or +0 (negative floats are negative integers, +0 is 0,
 // positive floats and NaN patterns with a clear sign bit are positive integers).
 __device__ __forceinline__ int imin3(int a, int b, int c) { return min(min(a, b), c); }
+
+// The outputs of one lane as P pairs in 64-bit registers, walked with the two-lane FP32 instructions: q, the weight sum and the
+// weighted sum of two outputs are one instruction each. The weight sum is carried NEGATED (n = theta - sum w), so that
+// q = fma(x, n, ysum) needs no negated copy of x; negation is exact, so every value is bit for bit the scalar walk's -- except the
+// sign of an exactly cancelled sum, which is why it is read back as 0 - n: 1/(+0) = +inf clamps to "no spike", 1/(-0) would not.
+//
+// Two steps share a vote. Where it finds some q at or below the margin tol, nearly always an output has q < -tol, and that output
+// has fired, without the reference's comparisons: let X bound the inputs consumed so far (0 <= inputs, ascending; |biasvolt|),
+// tol = 8 * 2^-24 * X * (|theta| + B) with |sum w - theta| <= |theta| + B and |ysum| <= X * B.
+//   - the step before left q > tol (an output that did not is `again`, below), i.e. ysum' - x' wsum' > tol. Consuming x' rounds
+//     ysum and wsum once each and the reference rounds x' * wsum: together at most 3 * 2^-24 * X * (|theta| + B), so the
+//     reference sees ysum > x' * wsum;
+//   - q < -tol leaves ysum <= x * wsum whatever way that product is rounded;
+//   - q fell from above tol to below -tol with x' <= x: wsum > 0.
+// So "armed" and "fire" both hold. An output within tol of zero, of either sign, is taken through the reference's rounded
+// comparisons (exact()); if it does not fire there, so is every output of the lane at the next step (`again`), and so is the first
+// step of a row. Rows for which X is no bound (an input below zero, a NaN, or sums that may overflow: `careful`) take the
+// comparisons whenever q <= tol. An output that has fired is parked at n = +inf: q = +inf (x > 0) or a positive NaN (x = 0) from
+// then on. Its sums wait in shared memory: as registers they made the walk spill.
+//
+// An output may also cross zero without firing (the two rounded comparisons of the reference can both miss it, about once in 10^5
+// spikes) and then stays below, taking its row through the comparisons at every step: twice the time of its neighbours, and where
+// the rows are one wave, of the whole launch. So between two blocks such an output changes the sign of its sums (flip()). Its q is
+// positive again, and below -tol it fires again: q rose through zero, the denominator is NEGATIVE, and the proof above holds with
+// both signs turned. From then on the row is walked by the FLIP steps, which give the weights each output's sign.
+// Measured (B200, four outputs per lane from global memory, before -> now): 1024 rows of 784 -> 400 172 -> 133 us (145 with the FLIP
+// steps not unrolled, 202 without them), 65 536 of 576 -> 128 690 -> 634, 16 384 of 2304 -> 256 993 -> 890; instructions per step
+// of 128 outputs 24.5 -> 17.4 where nothing fires. One pair per lane: 262 144 of 576 -> 64 1385 -> 1291, with the weights in shared
+// memory 1260 -> 1104. What bounds it: the chain q - minimum - vote - branch at 32 warps per SM (issue slots 55 % busy) and the FMA
+// pipe that takes the packed instructions.
+template <int P>
+struct PairWalk {
+  static constexpr int kFloats = 128 * P;   // of shared memory per warp
+  uint64_t n[P], ys[P];
+  float* fin;       // this lane's column of [2 * P][2][32] floats: an output's sums once it has fired; until then the sign that its
+                    // running sums carry, and -inf (an n that overflows to +inf reads as fired at y = +inf, which is no spike)
+  float tolbase, xmag;
+  int qlim;         // bits of tol, or INT_MAX: every output of this lane goes to the comparisons at the next step
+  int qtol;         // bits of tol
+  bool careful;     // q < -tol is no proof in this row
+
+  // sums with the bias input consumed (value biasvolt, weight wb), which is always the first; first: the row's smallest input
+  __device__ __forceinline__ void start(const Geometry& g, float tolerance_base, float first, const float (&wb)[2 * P],
+                                        const bool (&ok)[2 * P]) {
+    tolbase = tolerance_base;
+    xmag = g.has_bias ? fabsf(g.biasvolt) : 0.f;
+    careful = !(first >= 0.f) | !(tolbase * 4194304.f * fmaxf(xmag, fabsf(g.maxv)) < CUDART_INF_F);   // 2^22 tolbase = 2 (|theta| + B)
+    qlim = INT_MAX;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      float nn[2], yy[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int m = 2 * p + h;
+        nn[h] = ok[m] ? g.theta - wb[m] : CUDART_INF_F;   // (no output: parked, or the walk would wait for it)
+        yy[h] = g.has_bias ? g.biasvolt * wb[m] : 0.f;
+        fin[64 * m] = 1.f; fin[64 * m + 32] = -CUDART_INF_F;
+      }
+      n[p] = pack2(nn[0], nn[1]);
+      ys[p] = pack2(yy[0], yy[1]);
+    }
+  }
+  // the margin of steps whose inputs lie in [x0, x1]
+  __device__ __forceinline__ void margin(float x0, float x1) {
+    const float a = fmaxf(xmag, fabsf(x0)), b = fabsf(x1);
+    qtol = __float_as_int(tolbase * (b <= a ? a : b));     // (a NaN for a NaN at the end of the list)
+    if (qlim != INT_MAX) qlim = qtol;
+  }
+  __device__ __forceinline__ bool any_live() const {
+    bool live = false;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      float a, b;
+      unpack2(n[p], a, b);
+      live |= (a != CUDART_INF_F) | (b != CUDART_INF_F);
+    }
+    return live;
+  }
+
+  // ---- one or two steps. x2: the input twice; inputs() gives the input and the one in front of it, for the comparisons
+  template <bool FLIP, typename Inputs>
+  __device__ __forceinline__ void step(uint64_t x2, const uint64_t (&w)[P], Inputs&& inputs) {
+    int q[2 * P];
+    form_q(x2, n, ys, q);
+    if (__builtin_expect(__any_sync(0xffffffffu, smallest(q) <= qlim), 0)) {
+      uint64_t n0[P];
+#pragma unroll
+      for (int p = 0; p < P; ++p) n0[p] = n[p];
+      hit<FLIP>(q, n0, ys, n, inputs);
+    }
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      const uint64_t ws = FLIP ? mul2(w[p], signs(p)) : w[p];
+      n[p] = sub2(n[p], ws);
+      ys[p] = fma2(x2, ws, ys[p]);
+    }
+  }
+  template <typename InputsA, typename InputsB>
+  __device__ __forceinline__ void step2(uint64_t xa, const uint64_t (&wa)[P], uint64_t xb, const uint64_t (&wb)[P], InputsA&& ia,
+                                        InputsB&& ib) {
+    int qa[2 * P], qb[2 * P];
+    uint64_t n1[P], ys1[P];
+    form_q(xa, n, ys, qa);
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      n1[p] = sub2(n[p], wa[p]);
+      ys1[p] = fma2(xa, wa[p], ys[p]);
+    }
+    form_q(xb, n1, ys1, qb);
+    int m;
+    if constexpr (P == 1) m = min(imin3(qa[0], qa[1], qb[0]), qb[1]);
+    else m = min(imin3(qa[0], qa[1], qa[2]), imin3(imin3(qa[3], qb[0], qb[1]), qb[2], qb[3]));
+    if (__builtin_expect(__any_sync(0xffffffffu, m <= qlim), 0)) {
+      if (__any_sync(0xffffffffu, smallest(qa) <= qlim)) {
+        hit<false>(qa, n, ys, n1, ia);
+        form_q(xb, n1, ys1, qb);
+      }
+      if (__any_sync(0xffffffffu, smallest(qb) <= qlim)) {
+        uint64_t n0[P];
+#pragma unroll
+        for (int p = 0; p < P; ++p) n0[p] = n1[p];
+        hit<false>(qb, n0, ys1, n1, ib);
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      n[p] = sub2(n1[p], wb[p]);
+      ys[p] = fma2(xb, wb[p], ys1[p]);
+    }
+  }
+
+  // Between two blocks: outputs below zero that have not fired change their sign. xprev: the last input consumed. FLIP: the warp
+  // has such outputs already. Returns whether it has any.
+  template <bool FLIP>
+  __device__ __forceinline__ bool flip(float xprev) {
+    const bool look = (qlim == INT_MAX) & !careful;
+    if (__builtin_expect(!__any_sync(0xffffffffu, look), 1)) return FLIP;
+    const float tol = __int_as_float(qtol);
+    bool any = false, sure = look;                        // sure: no live output of this lane is within the margin any more
+    int q[2 * P];
+    form_q(pack2(xprev, xprev), n, ys, q);
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      float nn[2], s[2];
+      unpack2(n[p], nn[0], nn[1]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float qm = __int_as_float(q[2 * p + h]);
+        const bool live = nn[h] != CUDART_INF_F, below = look & live & (qm < -tol);
+        s[h] = below ? -1.f : 1.f;
+        if (below) fin[64 * (2 * p + h)] *= -1.f;
+        any |= below;
+        sure &= !live | (fabsf(qm) > tol);
+      }
+      n[p] = mul2(n[p], pack2(s[0], s[1]));
+      ys[p] = mul2(ys[p], pack2(s[0], s[1]));
+    }
+    __syncwarp();
+    if (sure) qlim = qtol;
+    return FLIP | (bool)__any_sync(0xffffffffu, any);
+  }
+
+  // spike value and 1/(sum w - theta) of output m once the list is consumed: an output that stopped has fired; one that consumed
+  // every input fires iff it is armed
+  __device__ __forceinline__ void finish(const Geometry& g, int m, float xprev, float& y, float& inv) const {
+    float nn[2], yy[2];
+    unpack2(n[m / 2], nn[0], nn[1]);
+    unpack2(ys[m / 2], yy[0], yy[1]);
+    float a = fin[64 * m], ws = 0.f - a, yv = fin[64 * m + 32];
+    bool fired = true;
+    if (nn[m & 1] != CUDART_INF_F) {
+      ws = 0.f - a * nn[m & 1]; yv = a * yy[m & 1];
+      fired = ratio_gt(yv, ws, xprev);
+    }
+    y = g.maxv; inv = 0.f;
+    if (fired) {
+      inv = __fdividef(1.0f, ws);
+      y = yv * inv;
+      if (y >= g.maxv) { y = g.maxv; inv = 0.f; }
+    }
+  }
+
+ private:
+  static __device__ __forceinline__ void form_q(uint64_t x2, const uint64_t (&n)[P], const uint64_t (&ys)[P], int (&q)[2 * P]) {
+#pragma unroll
+    for (int p = 0; p < P; ++p) unpack2i(fma2(x2, n[p], ys[p]), q[2 * p], q[2 * p + 1]);
+  }
+  static __device__ __forceinline__ int smallest(const int (&q)[2 * P]) {
+    return P == 1 ? min(q[0], q[1]) : min(imin3(q[0], q[1], q[2 * P - 2]), q[2 * P - 1]);
+  }
+  // signs of a pair (of an output that has fired: the sign of a sum, which its parked n does not feel)
+  __device__ __forceinline__ uint64_t signs(int p) const { return pack2(copysignf(1.f, fin[128 * p]), copysignf(1.f, fin[128 * p + 64])); }
+  // true sums of a pair
+  template <bool FLIP>
+  __device__ __forceinline__ void sums(const uint64_t (&n)[P], const uint64_t (&ys)[P], int p, float (&nn)[2], float (&yy)[2]) const {
+    unpack2(FLIP ? mul2(n[p], signs(p)) : n[p], nn[0], nn[1]);
+    unpack2(FLIP ? mul2(ys[p], signs(p)) : ys[p], yy[0], yy[1]);
+  }
+  // both sums of an output that fires. Predicated, and with the park added to n instead of put in its place: a branch here, or halves
+  // of n that are written alone, cost a divergence check per vote and copies of all sums per step
+  static __device__ __forceinline__ void store_if(bool fire, float* to, float a, float b) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.shared.f32 [%1], %2;\n\t@p st.shared.f32 [%1 + 128], %3;\n\t}"
+                 ::"r"((unsigned)fire), "r"(smem_u32(to)), "f"(a), "f"(b) : "memory");
+  }
+  // a step whose vote has passed. n0, ys0: the sums in front of it; what fires is parked in n1
+  template <bool FLIP, typename Inputs>
+  __device__ __forceinline__ void hit(const int (&q)[2 * P], const uint64_t (&n0)[P], const uint64_t (&ys0)[P], uint64_t (&n1)[P],
+                                      Inputs&& inputs) {
+    const float tol = __int_as_float(qlim);                // (INT_MAX: a NaN, nothing below fires)
+    float near = CUDART_INF_F;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      float nn[2], yy[2], park[2];
+      sums<FLIP>(n0, ys0, p, nn, yy);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int m = 2 * p + h;
+        const float qm = __int_as_float(q[m]);
+        park[h] = qm < -tol ? CUDART_INF_F : 0.f;
+        store_if(qm < -tol, fin + 64 * m, nn[h], yy[h]);
+        near = fminf(near, fabsf(qm));
+      }
+      n1[p] = add2(n1[p], pack2(park[0], park[1]));
+    }
+    if (__any_sync(0xffffffffu, !(near > tol))) {
+      const float2 xx = inputs();
+      exact<FLIP>(q, n0, ys0, n1, xx.x, xx.y);
+    }
+  }
+  // the reference's own comparisons, for all outputs of the lanes concerned
+  template <bool FLIP>
+  __device__ __forceinline__ void exact(const int (&q)[2 * P], const uint64_t (&n0)[P], const uint64_t (&ys0)[P], uint64_t (&n1)[P],
+                                        float x, float xp) {
+    bool again = false;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      float nn[2], yy[2], after[2], park[2] = {0.f, 0.f};
+      sums<FLIP>(n0, ys0, p, nn, yy);
+      unpack2(n1[p], after[0], after[1]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int m = 2 * p + h;
+        if (!__any_sync(0xffffffffu, q[m] <= qlim)) continue;
+        const bool live = after[h] != CUDART_INF_F;
+        const float wsum = 0.f - nn[h];
+        const bool fire = live & ratio_gt(yy[h], wsum, xp) & ratio_le(yy[h], wsum, x);
+        park[h] = fire ? CUDART_INF_F : 0.f;
+        store_if(fire, fin + 64 * m, nn[h], yy[h]);
+        again |= live & !fire & (q[m] <= qtol);
+      }
+      n1[p] = add2(n1[p], pack2(park[0], park[1]));
+    }
+    qlim = again | careful ? INT_MAX : qtol;
+  }
+};
 
 }  // namespace snntc

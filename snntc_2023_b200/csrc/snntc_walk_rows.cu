@@ -2,16 +2,16 @@
 //
 // A walk that gives a warp to each (row, 64 outputs) leaves three quarters of it idle at fan-out 16 and pays a step's list entry,
 // vote and branch for 64 outputs at best. Here 16, 8 or 4 lanes (for fan-out up to 64, 32, 16) take a row with its own list, so a
-// warp's step advances 128 outputs whatever the fan-out. Per step and lane: q of four outputs, their smallest as an integer,
-// one vote, and the reference's own comparisons (snntc/snnfc_kernels.cu.cc:46-55) where some q is at or near zero -- the
-// arithmetic, order and decisions of walk_row in snntc_forward.cu: the same bits. Rows of one warp are neighbours (receptive
+// warp's step advances 128 outputs whatever the fan-out. The steps are those of PairWalk (snntc_walk.cuh) with two pairs per lane:
+// the same bits as every other walk. Rows of one warp are neighbours (receptive
 // fields next to each other), so their lists are about equally long; behind the end of its list a row repeats its last input
 // with weight zero, which changes no sum and can fire nothing.
 // WS: all weights fit one CTA's shared memory (up to 200 KB: 780 rows of 64, 3 100 of 16): a persistent CTA of 32 warps per SM
 // holds them, since rows of 64 to 256 bytes picked at random miss the L1 cache beside everything else that goes through it.
-// What bounds it: instruction issue, about 26 instructions per step of 128 outputs.
-// Measured (B200, walk alone, before -> now): 65 536 rows of 144 -> 16 inputs 123 -> 51 us, of 288 -> 32: 223 -> 131; 61 440 of 576 ->
-// 48: 401 -> 346; 18 000 of 3136 -> 32: 1219 -> 743. The weights in shared memory pay from fan-out 33 and 32 768 rows on.
+// What bounds it: instruction issue and the latency of a step's chain.
+// Measured (B200, walk alone): against the pairs walk 65 536 rows of 144 -> 16 inputs 123 -> 51 us, of 288 -> 32: 223 -> 131; 61 440
+// of 576 -> 48: 401 -> 346; 18 000 of 3136 -> 32: 1219 -> 743, all with scalar steps; with PairWalk 262 144 of 27 -> 64 265 -> 235 and
+// 16 384 of 576 -> 64 109 -> 101. The weights in shared memory pay from fan-out 33 and 32 768 rows on.
 #include "snntc_common.cuh"
 #include "snntc_walk.cuh"
 
@@ -42,7 +42,8 @@ snn_walk_rows_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
   constexpr int WARPS = (WS ? 1024 : 256) / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WalkEntry* stage_all = reinterpret_cast<WalkEntry*>(smem_raw);              // [warps][rows][BLK]
-  float* ws_smem = reinterpret_cast<float*>(smem_raw + (size_t)WARPS * RPW * BLK * sizeof(WalkEntry));   // [I + bias][J]
+  float* fins = reinterpret_cast<float*>(smem_raw + (size_t)WARPS * RPW * BLK * sizeof(WalkEntry));       // [warps][kFloats]
+  float* ws_smem = fins + WARPS * PairWalk<2>::kFloats;                                                    // [I + bias][J]
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int sub = lane / LPR, gl = lane % LPR;
   const int J = g.J, jout = g.jout;
@@ -66,15 +67,16 @@ snn_walk_rows_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
   const unsigned lane_off = in_row ? (unsigned)j : 0u;
   const char* wbytes = reinterpret_cast<const char*>(w);
   const unsigned ws_lane = smem_u32(ws_smem) + 4u * lane_off;
-  auto load_weights = [&](unsigned eoff) -> float4 {
+  auto load_weights = [&](unsigned eoff, uint64_t (&wv)[2]) {
     if constexpr (WS) {
-      float4 v;
-      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(4u * eoff + ws_lane));
-      return v;
+      asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(wv[0]), "=l"(wv[1]) : "r"(4u * eoff + ws_lane));
     } else {
-      return ld_plain(reinterpret_cast<const float4*>(wbytes + (size_t)(eoff + lane_off) * 4u));
+      const ulonglong2 v = ld_plain(reinterpret_cast<const ulonglong2*>(wbytes + (size_t)(eoff + lane_off) * 4u));
+      wv[0] = v.x; wv[1] = v.y;
     }
   };
+  PairWalk<2> pw;
+  pw.fin = fins + warp * PairWalk<2>::kFloats + lane;
 
   const int groups = (g.R + RPW - 1) / RPW;
   for (int grp = blockIdx.x * WARPS + warp; grp < groups; grp += gridDim.x * WARPS) {
@@ -85,57 +87,26 @@ snn_walk_rows_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
     const int nmin = (int)__reduce_min_sync(0xffffffffu, (unsigned)n);
     const WalkEntry* ents = lists + (size_t)(row_ok ? r : 0) * istride;
     // the bias input (value biasvolt, weight row I) is always consumed first
-    float wsum[4] = {-g.theta, -g.theta, -g.theta, -g.theta}, ysum[4] = {0.f, 0.f, 0.f, 0.f};
-    if (g.has_bias) {
-      const float4 wb = load_weights((unsigned)g.I * (unsigned)J);
-      wsum[0] += wb.x; wsum[1] += wb.y; wsum[2] += wb.z; wsum[3] += wb.w;
-      ysum[0] = g.biasvolt * wb.x; ysum[1] = g.biasvolt * wb.y; ysum[2] = g.biasvolt * wb.z; ysum[3] = g.biasvolt * wb.w;
-    }
-    float wfin[4], yfin[4];
-    int live[4];
+    {
+      uint64_t b2[2] = {0, 0};
+      if (g.has_bias) load_weights((unsigned)g.I * (unsigned)J, b2);
+      float wb[4];
+      unpack2(b2[0], wb[0], wb[1]);
+      unpack2(b2[1], wb[2], wb[3]);
+      bool ok[4];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      wfin[m] = 0.f; yfin[m] = 0.f;
-      live[m] = row_ok && j + m < jout ? -1 : 0;   // (padding behind jout never fires: the walk would wait for it)
-      if (live[m] == 0) wsum[m] = -CUDART_INF_F;
+      for (int m = 0; m < 4; ++m) ok[m] = row_ok & (j + m < jout);   // (padding behind jout never fires: the walk would wait for it)
+      const WalkEntry head = ld_l2(ents);
+      pw.start(g, tolbase, n > 0 ? __uint_as_float(head.x) : 0.f, wb, ok);
     }
     float xprev = g.has_bias ? g.biasvolt : 0.f;
-    int sticky = INT_MAX, qlim = 0;
 
-    auto step = [&](const float x, const float xp, const float4& w4) {
-      const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
-      int q[4];
-#pragma unroll
-      for (int m = 0; m < 4; ++m) q[m] = __float_as_int(fmaf(-x, wsum[m], ysum[m]));
-      const int qmin = imin3(imin3(q[0], q[1], q[2]), q[3], sticky);
-      if (__builtin_expect(__any_sync(0xffffffffu, qmin <= qlim), 0)) {
-        bool again = false;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          if (!__any_sync(0xffffffffu, (q[m] <= qlim) | (sticky < 0))) continue;
-          const bool lv = live[m] != 0;
-          const bool fire = lv & ratio_gt(ysum[m], wsum[m], xp) & ratio_le(ysum[m], wsum[m], x);
-          if (fire) {
-            live[m] = 0;                          // spike lies in (previous input, x]: keep the sums aside and park the running ones
-            wfin[m] = wsum[m];
-            yfin[m] = ysum[m];
-            wsum[m] = -CUDART_INF_F;
-          }
-          again |= lv & !fire & (q[m] <= qlim);
-        }
-        sticky = again ? INT_MIN : INT_MAX;
-      }
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        wsum[m] += wv[m];
-        ysum[m] = fmaf(x, wv[m], ysum[m]);
-      }
-    };
-    // entries c .. c + 3 of the staged block; LAST: some row's list ends among them (`left` entries of this row are valid)
-    auto chunk = [&](int c, int left, auto last_c) {
-      constexpr bool LAST = decltype(last_c)::value;
+    // entries c .. c + 3 of the staged block; LAST: some row's list ends among them (`left` entries of this row are valid): behind its
+    // end a row repeats its last input with weight zero
+    auto chunk = [&](int c, int left, auto last_c, auto flip_c) {
+      constexpr bool LAST = decltype(last_c)::value, FLIP = decltype(flip_c)::value;
       float xs[kChunk];
-      float4 wv[kChunk];
+      uint64_t wv[kChunk][2];
 #pragma unroll
       for (int u = 0; u < kChunk; u += 2) {
         const uint4 e2 = *reinterpret_cast<const uint4*>(stage + c + u);
@@ -146,16 +117,25 @@ snn_walk_rows_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
           if (u >= left) { xs[u] = u > 0 ? xs[u > 0 ? u - 1 : 0] : xprev; o0 = 0u; }
           if (u + 1 >= left) { xs[u + 1] = xs[u]; o1 = 0u; }
         }
-        wv[u] = load_weights(o0);
-        wv[u + 1] = load_weights(o1);
+        load_weights(o0, wv[u]);
+        load_weights(o1, wv[u + 1]);
         if (LAST) {
-          if (u >= left) wv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (u + 1 >= left) wv[u + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (u >= left) wv[u][0] = wv[u][1] = 0;
+          if (u + 1 >= left) wv[u + 1][0] = wv[u + 1][1] = 0;
         }
       }
-      qlim = __float_as_int(tolbase * fmaxf(fabsf(xs[0]), fabsf(xs[kChunk - 1])));   // inputs ascend: |x| peaks at an end
+      auto inputs = [&](int u) { return make_float2(xs[u], u == 0 ? xprev : xs[u > 0 ? u - 1 : 0]); };
+      pw.margin(xs[0], xs[kChunk - 1]);           // inputs ascend: |x| peaks at an end
 #pragma unroll
-      for (int u = 0; u < kChunk; ++u) step(xs[u], u == 0 ? xprev : xs[u > 0 ? u - 1 : 0], wv[u]);
+      for (int u = 0; u < kChunk; u += 2) {
+        const uint64_t xa = pack2(xs[u], xs[u]), xb = pack2(xs[u + 1], xs[u + 1]);
+        if constexpr (FLIP) {
+          pw.step<true>(xa, wv[u], [&] { return inputs(u); });
+          pw.step<true>(xb, wv[u + 1], [&] { return inputs(u + 1); });
+        } else {
+          pw.step2(xa, wv[u], xb, wv[u + 1], [&] { return inputs(u); }, [&] { return inputs(u + 1); });
+        }
+      }
       xprev = xs[kChunk - 1];
     };
 
@@ -169,37 +149,31 @@ snn_walk_rows_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
       }
     };
     read_block(0);
+    bool flipped = false;
     for (int base = 0; base < nmax; base += BLK) {
       __syncwarp();
 #pragma unroll
       for (int q = 0; q < PER; ++q) stage[gl + q * LPR] = pre[q];
       __syncwarp();
       if (base + BLK < nmax) read_block(base + BLK);
+      if (__builtin_expect(flipped, 0)) {
 #pragma unroll 1
-      for (int c = 0; c < BLK && base + c < nmax; c += kChunk) {
-        if (base + c + kChunk <= nmin) chunk(c, kChunk, std::false_type{});
-        else chunk(c, n - base - c, std::true_type{});
+        for (int c = 0; c < BLK && base + c < nmax; c += kChunk) chunk(c, n - base - c, std::true_type{}, std::true_type{});
+        pw.flip<true>(xprev);
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < BLK && base + c < nmax; c += kChunk) {
+          if (base + c + kChunk <= nmin) chunk(c, kChunk, std::false_type{}, std::false_type{});
+          else chunk(c, n - base - c, std::true_type{}, std::false_type{});
+        }
+        flipped = pw.flip<false>(xprev);
       }
-      if (!__any_sync(0xffffffffu, (live[0] | live[1] | live[2] | live[3]) != 0)) break;   // every output has fired
+      if (!__any_sync(0xffffffffu, pw.any_live())) break;   // every output has fired
     }
 
     float yo[4], io[4];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      // an output that stopped has fired; one that consumed every input fires iff it is armed
-      bool fired = true;
-      float ws = wfin[m], yy = yfin[m];
-      if (live[m]) {
-        ws = wsum[m]; yy = ysum[m];
-        fired = ratio_gt(yy, ws, xprev);
-      }
-      yo[m] = g.maxv; io[m] = 0.f;
-      if (fired) {
-        io[m] = __fdividef(1.0f, ws);
-        yo[m] = yy * io[m];
-        if (yo[m] >= g.maxv) { yo[m] = g.maxv; io[m] = 0.f; }
-      }
-    }
+    for (int m = 0; m < 4; ++m) pw.finish(g, m, xprev, yo[m], io[m]);
     if (row_ok && in_row) {
       float* yr = out + (size_t)r * jout + j;
       float* ir = yr + (size_t)g.R * jout;
@@ -228,7 +202,7 @@ template <int LPR, bool WS>
 int launch(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
            const LaunchInfo& li, cudaStream_t s) {
   constexpr int threads = WS ? 1024 : 256, warps = threads / 32;
-  const size_t smem = (size_t)warps * Shape<LPR>::rows * Shape<LPR>::block * sizeof(WalkEntry) +
+  const size_t smem = (size_t)warps * (Shape<LPR>::rows * Shape<LPR>::block * sizeof(WalkEntry) + PairWalk<2>::kFloats * sizeof(float)) +
                       (WS ? (size_t)(g.I + g.has_bias) * g.J * sizeof(float) : 0);
   if (allow_smem<snn_walk_rows_kernel<LPR, WS>>(smem) != cudaSuccess) return E_CUDA;
   const long groups = ((long)g.R + Shape<LPR>::rows - 1) / Shape<LPR>::rows;
@@ -243,7 +217,8 @@ int launch(const Geometry& g, const WalkEntry* lists, const int* nvalid, int ist
 template <int LPR>
 int launch_lanes(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
                  bool resident, const LaunchInfo& li, cudaStream_t s) {
-  const size_t need = (size_t)32 * Shape<LPR>::rows * Shape<LPR>::block * sizeof(WalkEntry) + (size_t)(g.I + g.has_bias) * g.J * sizeof(float);
+  const size_t need = (size_t)32 * (Shape<LPR>::rows * Shape<LPR>::block * sizeof(WalkEntry) + PairWalk<2>::kFloats * sizeof(float)) +
+                      (size_t)(g.I + g.has_bias) * g.J * sizeof(float);
   if (resident && need + 2048 <= (size_t)li.max_smem_optin) return launch<LPR, true>(g, lists, nvalid, istride, w, out, li, s);
   return launch<LPR, false>(g, lists, nvalid, istride, w, out, li, s);
 }

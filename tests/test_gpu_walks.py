@@ -108,3 +108,28 @@ def test_choice_among_the_walks_from_global_memory(R, I, J, offset):
     ref = ops.snn_fc(xd, torch.from_numpy(w).cuda(), params, opts=_lib.options(walk_layout=2, walk_outputs=1))
     assert torch.equal(out, ref)
     assert torch.equal(ops.snn_fc_infer(xd, wd, params), out[:R])
+
+
+@pytest.mark.parametrize("J", [16, 64, 96, 132])
+@pytest.mark.parametrize("band,scale", [(1e-4, 3e4), (1e-3, 3e3), (3e-3, 1e3)])
+def test_spikes_that_rounding_hides_and_negative_denominators(J, band, scale):
+    """Inputs so close together that rounding decides many steps: outputs cross their threshold without a spike, stay behind it
+    (the walks turn their sums' sign), and some spike on the way back, with a negative denominator. Every layout: the bits of one
+    output per lane, which takes every such step through the reference's comparisons."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    rng = np.random.default_rng(J)
+    I, R = 300, 600
+    x = np.exp(band * rng.random((R, I))).astype(np.float32)
+    w = (rng.standard_normal((I + 1, J)) * np.sqrt(15.0 / I) * scale).astype(np.float32)
+    w[I] = 0.0
+    params = O.fc_params(biasvolt=1.0)
+    o32, o64 = O.fc_forward(x[:64], w, params, "f32"), O.fc_forward(x[:64], w, params, "f64")
+    assert ((o32["y"] < 9e4) != (o64["y"] < 9e4)).sum() > 0 or J == 16
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
+    assert band > 1e-4 or int((ref[R:] < 0).sum()) > 0
+    for layout in (0, 1, 3, 8, 16, 32, 64):
+        assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=layout)), ref), "layout %d" % layout
+    got = ref[:64].cpu().numpy()
+    assert np.array_equal(got < 9e4, o32["y"] < 9e4)
