@@ -659,9 +659,12 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   const int istride = key_stride(g);
 
   const int fparts = opt.forward_parts;
-  // The walk that copies its weight rows ahead, up to about 24 items of 32 outputs per SM (8 where the rows have to be copied
-  // 4 bytes at a time): with few warps on an SM latency is what counts, with many the instructions per output. Measured lines:
-  // 784 -> 400 crosses at 3 300 items, 4096 -> 512 behind 4 100, 3x3 convolutions of 128 and 256 channels between 2 000 and 4 100.
+  // The walk that copies its weight rows ahead, up to two waves of its CTAs of 64 outputs (six to an SM; eight items of 32 outputs per
+  // SM for fan-out up to 32, where a copying warp serves a single one, and where the rows have to be copied 4 bytes at a time): with
+  // few warps on an SM latency is what counts, with many the instructions per output. Against the pairs walk, us: 784 -> 400 200 rows
+  // 29, 35, 300 rows 41, 37; 1000 -> 1000 80 rows 33, 43, 120 rows 46, 45; 576 -> 128 1000 rows (13.5 CTAs per SM) 33, 31; 1152 ->
+  // 128 700 rows 37, 47, 1500 72, 67; 4096 -> 512 still 172, 199 at 300 rows (16 per SM); 576 -> 32 1000 rows 23, 25, 2000 40, 27;
+  // 1500 -> 16 1000 rows 47, 53, 2000 83, 50.
   g.jout = g.J;
   const bool own = opt.walk_layout == 0 && opt.walk_outputs == 0;    // the library's own choice
   const long ring_items = (long)g.R * ((g.J + 31) / 32);
@@ -678,7 +681,8 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     g.J = jp;
   }
   const bool copies16 = (g.J & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
-  const bool ring = (opt.walk_layout & 16) != 0 || (own && ring_items <= (copies16 ? 24L : 8L) * li.num_sms);
+  const bool few = copies16 && g.J > 32 ? (long)g.R * ((g.J + 63) / 64) <= 12L * li.num_sms : ring_items <= 8L * li.num_sms;
+  const bool ring = (opt.walk_layout & 16) != 0 || (own && few);
   // Several rows per warp for fan-out up to 64, where that leaves enough warps: 6 per SM at eight rows to a warp (fan-out 16;
   // 10 where the weights miss the L1 cache), 14 at four (32), 48 at two (64). With fewer the pairs walk, a warp per row, hides
   // its latencies better (5 880 rows of 6400 x 16: 540 against 770 us; 8 064 of 576 x 16: 107 against 61).

@@ -1,21 +1,23 @@
-// The sorted walk for layers with few (row, output) pairs: a warp walks one row for 32 outputs, one per lane, and copies the
-// weight rows its list names into shared memory ahead of itself.
+// The sorted walk for layers with few (row, output) pairs: a warp walks one row for 32 outputs, one per lane, and a warp beside it
+// copies the weight rows that the list names into shared memory ahead of it.
 //
 // With few warps on an SM a walk is bound by latency: the walk from global memory (snntc_forward.cu) waits an L2 round trip for
-// every four to eight weight rows and a vote with its branch at every step, 75 to 130 cycles a step. Here
-//   - weight rows arrive by asynchronous copies, 32 (or 16) entries to a block, two blocks ahead of the one that is consumed;
-//   - the sums and sign tests of 16 (or 8) steps are formed before one vote, from operands that were read a group ahead. The
-//     sums in front of every step of the group stay in registers, so where the vote finds an output at or near zero, only the
-//     steps concerned are taken through the reference's own comparisons (snntc/snnfc_kernels.cu.cc:46-55) and nothing is
-//     replayed (groups of four without the read ahead: 30 % slower at one row of 25 088 inputs);
+// every four to eight weight rows and a vote with its branch per step or two, 75 to 130 cycles a step. Here
+//   - a warp of its own copies the list and, from it, the weight rows, 32 entries to a block, two blocks ahead of the one that is
+//     walked; one barrier per block. A warp that does both spends 38 cycles an entry (one row of 4096 -> 512, 51 us), one that only
+//     walks 25 (36 us). Two warps that walk the same row share the copies: 25 088 -> 1024 at 64 samples 804 us with each copying for
+//     itself, 463 so (copies past L1: 531 through it);
+//   - the sums and sign tests of 16 steps are formed before one vote. The sums in front of every step of the group stay in registers,
+//     so where the vote finds an output at or near zero, only the steps concerned are taken through the reference's own
+//     comparisons (snntc/snnfc_kernels.cu.cc:46-55) and nothing is replayed;
 //   - one output per lane: with a warp per scheduler every instruction of the dependent chain costs its latency, so the fewest
 //     instructions per step win (two outputs per lane, as pairs in 64-bit registers, took 82 cycles a step).
 // Arithmetic, order and decisions are those of walk_row: the same bits. The margin of a sign test is 2^-22 |x * sum w|, formed
 // from the output's own sum -- four times the rounding error of the reference's product x * sum w, so every step that
 // rounding could decide goes to the reference's comparisons, and no bound over the weight matrix has to be computed first.
-// Measured (B200, walk alone, before -> now): 784 -> 400 at 32 samples 58 -> 22 us; 4096 -> 512 at 32: 150 -> 47 us; 25 088 ->
-// 1024 at 64: 1918 -> 771 us; 3x3 convolution 256 -> 256 on 64 fields 85 -> 35 us. From about 24 items (row, 32 outputs) per
-// SM on the walk from global memory is the faster one: it spends fewer instructions per output.
+// Measured (B200, walk alone, each warp copying for itself -> now): one row of 784 -> 400 18.6 -> 14.3 us, 64 of 2304 -> 256 30 -> 25,
+// 128 of 2000 -> 512 76 -> 43, 100 of 6000 -> 1000 219 -> 164, 64 of 25 088 -> 1024 802 -> 424 (of which the outputs that rounding
+// keeps from firing, turn() below, 150).
 #include "snntc_common.cuh"
 #include "snntc_walk.cuh"
 
@@ -26,33 +28,34 @@ namespace snntc {
 
 namespace {
 
-constexpr int kWarps = 2;                          // per CTA, each on an item of its own
-constexpr int kRing = 3;                           // weight blocks per warp: one consumed, two on their way
-constexpr int kListRing = 4;                       // list blocks per warp
-
-template <int kBlock>
-struct RingWarp {
-  float w[kRing][kBlock][32];
-  float x[kListRing][kBlock];
-  unsigned off[kListRing][kBlock];                 // element offset of the weight row
-};
+constexpr int kBlock = 32;                         // list entries
+constexpr int kGroup = 16;                         // steps per vote
+constexpr int kRing = 3;                           // blocks of weights: one consumed, two on their way
+constexpr int kListAhead = 2;                      // blocks that the list is copied ahead of the weights it names
 
 template <int BYTES>
-__device__ __forceinline__ void copy_async(unsigned dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+__device__ __forceinline__ void copy_async(unsigned dst, const void* src, bool valid) {   // not valid: zeros
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? BYTES : 0) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(BYTES), "r"(valid ? BYTES : 0) : "memory");
 }
 
 // One output of one lane. wsum = sum w - theta and ysum = sum w*x run on; an output that has fired keeps its sums in fin and
 // its running weight sum at -inf, where q stays +inf.
 struct Walk {
-  float wsum, ysum;
+  float wsum, ysum;       // times sign
   float2 fin;
   bool live;
   int sticky;             // INT_MIN: the output was at or near zero at the last entry without firing, else INT_MAX
   float xprev;
+  float sign;             // -1: the output has crossed zero without firing (turn)
 
-  template <bool FIRST, int G>
-  __device__ __forceinline__ void steps(const float (&x)[G], const float (&w)[G]) {
+  __device__ __forceinline__ float plain(float v) const { return sign < 0.f ? 0.f - v : v; }   // (an exactly cancelled sum stays +0)
+
+  // lim: bits of the q beyond the margin that still goes to the comparisons, 0 unless the output has been turned
+  __device__ __forceinline__ void steps(const float (&x)[kGroup], const float (&w)[kGroup], const int lim) {
+    constexpr int G = kGroup;
     float sw[G], sy[G];
     int p[G];
     const float z = -2.384185791015625e-7f * fmaxf(fabsf(x[0]), fabsf(x[G - 1]));   // inputs ascend: |x| peaks at an end
@@ -61,23 +64,22 @@ struct Walk {
     for (int u = 0; u < G; ++u) {
       sw[u] = wsum; sy[u] = ysum;
       p[u] = __float_as_int(fmaf(z, fabsf(wsum), fmaf(-x[u], wsum, ysum)));   // (an output set aside: NaN, a positive integer)
-      m = min(m, p[u]);
+      if (u & 1) m = imin3(m, p[u - (u > 0)], p[u]);
       wsum += w[u];
       ysum = fmaf(x[u], w[u], ysum);
     }
-    if (__builtin_expect(__any_sync(0xffffffffu, m <= 0), 0)) {
-      // FIRST: every lane takes its own first step at or near zero through the comparisons, all lanes at once. Nearly always
-      // that step fires; where one does not, or was waited for from the group before, the steps are gone through one by one.
-      // (784 -> 400 at 32 samples with its sort 19.9 -> 17.3 us; where bandwidth counts the one by one code is the better one:
-      // 25 088 -> 1024 at 64 samples 819 us, 882 with FIRST)
-      if constexpr (FIRST) {
+    if (__builtin_expect(__any_sync(0xffffffffu, m <= lim), 0)) {
+      // Every lane takes its own first step at or near zero through the comparisons, all lanes at once. Nearly always that step
+      // fires; where one does not, or was waited for from the group before, the steps are gone through one by one.
+      {
         float tw = 0.f, ty = 0.f, tx = 0.f, txp = 0.f;
         bool at = false;
 #pragma unroll
         for (int u = G - 1; u >= 0; --u) {
-          if (p[u] <= 0) { tw = sw[u]; ty = sy[u]; tx = x[u]; txp = u == 0 ? xprev : x[u > 0 ? u - 1 : 0]; at = true; }
+          if (p[u] <= lim) { tw = sw[u]; ty = sy[u]; tx = x[u]; txp = u == 0 ? xprev : x[u > 0 ? u - 1 : 0]; at = true; }
         }
         at &= live;
+        tw = plain(tw); ty = plain(ty);
         const bool hit = at & ratio_gt(ty, tw, txp) & ratio_le(ty, tw, tx);
         if (!__any_sync(0xffffffffu, (at & !hit) | (sticky < 0))) {
           if (hit) {
@@ -91,11 +93,11 @@ struct Walk {
       }
 #pragma unroll
       for (int u = 0; u < G; ++u) {
-        const bool near = live & (p[u] <= 0);
+        const bool near = live & (p[u] <= lim);
         if (!__any_sync(0xffffffffu, near | (sticky < 0))) continue;
-        const float xp = u == 0 ? xprev : x[u > 0 ? u - 1 : 0];
-        const bool fire = live & ratio_gt(sy[u], sw[u], xp) & ratio_le(sy[u], sw[u], x[u]);
-        if (fire) fin = make_float2(sw[u], sy[u]);
+        const float xp = u == 0 ? xprev : x[u > 0 ? u - 1 : 0], tw = plain(sw[u]), ty = plain(sy[u]);
+        const bool fire = live & ratio_gt(ty, tw, xp) & ratio_le(ty, tw, x[u]);
+        if (fire) fin = make_float2(tw, ty);
         live = live & !fire;
         sticky = (near & !fire) ? INT_MIN : INT_MAX;
       }
@@ -103,70 +105,118 @@ struct Walk {
     }
     xprev = x[G - 1];
   }
+
+  // Between two groups. An output may cross zero without firing (both rounded comparisons of the reference can miss it: about once
+  // in 10^5 spikes at some hundred inputs, once in some hundred at 25 000) and would take its warp through the steps one by one to the
+  // end of the list. Beyond the margin its sums change their sign, and with them its q: it cannot fire before q comes back to zero.
+  // (A positive sum: not armed, if the present sums, too, see the last input beyond zero -- guard() widens the margin by what the
+  // step between may have added. A negative sum: not yet back.) Returns whether the warp has any such output.
+  __device__ __forceinline__ bool turn(bool turned) {
+    if (__builtin_expect(__any_sync(0xffffffffu, sticky < 0), 0)) {
+      const float q = fmaf(-xprev, wsum, ysum);
+      if (sticky < 0 && live && fabsf(q) > 2.384185791015625e-7f * fabsf(xprev * wsum)) {
+        sticky = INT_MAX;
+        if (q < 0.f) { sign = -sign; wsum = 0.f - wsum; ysum = 0.f - ysum; }
+      }
+      turned |= (bool)__any_sync(0xffffffffu, sign < 0.f);
+    }
+    return turned;
+  }
+  // weights of a group in a warp with turned outputs: their sign, and the limit for steps()
+  __device__ __forceinline__ int guard(const float (&x)[kGroup], float (&w)[kGroup]) const {
+    constexpr int G = kGroup;
+    float most = 0.f;
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      most = fmaxf(most, fabsf(w[u]));
+      w[u] *= sign;
+    }
+    return sign < 0.f ? __float_as_int(2.384185791015625e-7f * most * fmaxf(fabsf(x[0]), fabsf(x[G - 1]))) : 0;
+  }
 };
 
-// VEC: J is a multiple of 4 and w 16-byte aligned: 16-byte weight copies, else 4-byte ones. kBlock: list entries per block, 32,
-// or 16 where there are warps to fill the SMs (half the shared memory per warp: 58 against 68 us for 784 -> 400 at 256 samples).
-template <bool VEC, int kBlock>
-__global__ void __launch_bounds__(32 * kWarps)
-snn_walk_ring_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid, int istride,
-                     const float* w, float* __restrict__ out, int slices) {
+// A CTA takes a row and 32 * C outputs: C warps walk 32 outputs each, one more warp copies for them. VEC: J is a multiple of 4 and w
+// 16-byte aligned: 16-byte weight copies, else 4-byte ones (C = 1).
+template <int C>
+struct RingShared {
+  float w[kRing][kBlock][32 * C];
+  float x[kRing][kBlock];
+  WalkEntry list[2 * kListAhead][kBlock];
+};
+
+template <bool VEC, int C>
+__global__ void __launch_bounds__(32 * (C + 1))
+snn_walk_ring_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid, int istride, const float* w,
+                     float* __restrict__ out) {
   chain_wait();
   chain_next();
-  __shared__ __align__(16) RingWarp<kBlock> ring[kWarps];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  RingShared<C>& sm = *reinterpret_cast<RingShared<C>*>(smem_raw);
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
-  RingWarp<kBlock>& sm = ring[warp];
   const int J = g.J;
-  // neighbouring items are rows of the same output slice: the slice's weights stay in L2 while they run
-  const long item = (long)blockIdx.x * kWarps + warp;
-  if (item >= (long)g.R * slices) return;
-  const int r = (int)(item % g.R), j0 = (int)(item / g.R) * 32;
+  // neighbouring CTAs are rows of the same output slice: the slice's weights stay in L2 while they run
+  const int r = (int)(blockIdx.x % (unsigned)g.R), j0 = (int)(blockIdx.x / (unsigned)g.R) * 32 * C;
   const WalkEntry* ents = lists + (size_t)r * istride;
   const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid + r), 0);
   const int blocks = (n + kBlock - 1) / kBlock;
 
-  // list block b: read a block ahead into a register, then put into shared memory. Behind the end of the list: offset 0 (a
-  // row is copied that nothing consumes)
-  WalkEntry pre = make_uint2(0u, 0u);
-  auto read_list = [&](int b) {
-    pre = make_uint2(0u, 0u);
-    if ((kBlock == 32 || lane < kBlock) && b * kBlock + lane < n) pre = ld_l2(ents + b * kBlock + lane);
-  };
-  auto put_list = [&](int b) {
-    if (kBlock == 32 || lane < kBlock) {
-      sm.x[b % kListRing][lane] = __uint_as_float(pre.x);
-      sm.off[b % kListRing][lane] = pre.y;
-    }
-  };
-  // weight block b. VEC: a copy brings four rows of 32 outputs, 16 bytes per lane (columns outside the row: column 0 again)
-  // Else 4 bytes per lane, 32 / columns rows at a time.
-  const int cols = J - j0 < 32 ? J - j0 : 32;
-  const int per = VEC ? 4 : 32 / cols, sub = VEC ? lane >> 3 : min(lane / cols, per - 1);
-  const int col = VEC ? (4 * (lane & 7) < cols ? 4 * (lane & 7) : 0) : lane % cols;
-  const float* wj = w + j0 + col;
-  auto copy_weights = [&](int b) {
-    const unsigned* off = sm.off[b % kListRing];
-    const unsigned to = smem_u32(&sm.w[b % kRing][0][0]);
-    if constexpr (VEC) {
+  if (warp == C) {
+    // list block b: a lane per entry. Behind the end of the list: the last input again with weights of zero, which change no sum and
+    // can fire nothing
+    auto copy_list = [&](int b) {
+      if (b < blocks)
+        copy_async<8>(smem_u32(&sm.list[b % (2 * kListAhead)][lane]), ents + min(b * kBlock + lane, n - 1), true);
+    };
+    // VEC: a copy instruction brings 4 / C rows of 32 * C outputs, 16 bytes per lane. Else 4 bytes per lane, 32 / columns rows at a time.
+    // (Lanes behind the row copy nothing: with the row's first column once more 1024 rows of 400 -> 10 took 47 us, 15 so.)
+    const int cols = J - j0 < 32 * C ? J - j0 : 32 * C;
+    const int per = VEC ? 4 / C : 32 / cols, sub = VEC ? lane / (8 * C) : min(lane / cols, per - 1);
+    const int at = VEC ? 4 * (lane % (8 * C)) : lane % cols;
+    const float* wj = w + j0 + at;
+    const bool mine = !VEC || at < cols;
+    int s = 0;                                     // buffer of the block that is filled next
+    auto fill = [&](int b) {
+      if (b >= blocks) return;
+      const WalkEntry e = sm.list[b % (2 * kListAhead)][lane];
+      sm.x[s][lane] = __uint_as_float(e.x);
+      const unsigned to = smem_u32(&sm.w[s][0][at]);
+      // (the offsets of eight copies are shuffled together: one by one each waits for its own, 28 cycles a copy)
+#pragma unroll 1
+      for (int q = 0; q < kBlock; q += 8 * per) {
+        unsigned off[8];
 #pragma unroll
-      for (int q = 0; q < kBlock / 4; ++q) copy_async<16>(to + 512u * q + 16u * lane, wj + off[4 * q + sub]);
-    } else {
-#pragma unroll 4
-      for (int e = sub; e < kBlock; e += per) copy_async<4>(to + 128u * e + 4u * col, wj + off[e]);
-    }
-  };
-
-  const int j = j0 + lane;
-  const bool ok = j < g.jout;
+        for (int i = 0; i < 8; ++i) off[i] = __shfl_sync(0xffffffffu, e.y, (q + i * per + sub) & 31);
 #pragma unroll
-  for (int b = 0; b < kRing - 1; ++b) {
-    read_list(b);
-    put_list(b);
-    __syncwarp();
-    if (b < blocks) copy_weights(b);
+        for (int i = 0; i < 8; ++i) {
+          const int k = q + i * per + sub;
+          if (VEC ? mine : k < kBlock) copy_async<VEC ? 16 : 4>(to + 128u * C * k, wj + off[i], b * kBlock + k < n);
+        }
+      }
+      s = s + 1 == kRing ? 0 : s + 1;
+    };
+#pragma unroll
+    for (int b = 0; b < kRing - 1 + kListAhead; ++b) copy_list(b);
     copies_commit();
+    copies_wait<0>();
+    __syncwarp();
+#pragma unroll 1
+    for (int b = 0; b < kRing - 1; ++b) {
+      fill(b);
+      copies_commit();
+    }
+    for (int b = 0; b < blocks; ++b) {
+      copies_wait<kRing - 2>();                    // block b, and the list of block b + kListAhead
+      if (!__syncthreads_or(0)) break;             // (and every warp has read block b - 1, whose buffer is refilled)
+      fill(b + kRing - 1);
+      copy_list(b + kRing - 1 + kListAhead);
+      copies_commit();
+    }
+    copies_wait<0>();
+    return;
   }
-  read_list(kRing - 1);
+
+  const int j = j0 + 32 * warp + lane;
+  const bool ok = j < g.jout;
   Walk wk;
   wk.wsum = -g.theta;
   wk.ysum = 0.f;
@@ -180,63 +230,39 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
   wk.fin = make_float2(0.f, 0.f);
   wk.sticky = INT_MAX;
   wk.xprev = g.has_bias ? g.biasvolt : 0.f;
-  for (int b = 0; b < blocks; ++b) {
-    put_list(b + kRing - 1);
-    __syncwarp();                                  // (and every lane is through with block b - 1, whose buffer is refilled)
-    read_list(b + kRing);
-    if (b + kRing - 1 < blocks) copy_weights(b + kRing - 1);
-    copies_commit();
-    copies_wait<kRing - 1>();                      // weight block b
-    __syncwarp();
-    const float* xb = sm.x[b % kListRing];
-    const float* wb = &sm.w[b % kRing][0][lane];
-    constexpr int kGroup = kBlock / 2;             // steps per vote
-    const int nb = min(kBlock, n - b * kBlock);
-    int k = 0;
-    // the next group's operands are read while this one's vote is on its way
-    float x[2][kGroup], wv[2][kGroup];
-    auto read = [&](int at, float (&xs)[kGroup], float (&ws)[kGroup]) {
+  wk.sign = 1.f;
+  if (blocks > 0 && __syncthreads_or(wk.live)) {
+    bool more = true, turned = false;
+    // (one copy of the steps: reading the next group ahead of a vote takes two, and costs more in instructions that have to be
+    // fetched than it hides)
+    int half = 0;                                  // of the 2 * kRing halves of the buffers
+#pragma unroll 1
+    for (int h = 0; more; ++h) {
+      float x[kGroup], wv[kGroup];
+      const float* xb = &sm.x[0][0] + half * kGroup;
+      const float* wb = &sm.w[0][0][32 * warp + lane] + half * (kGroup * 32 * C);
+      half = half + 1 == 2 * kRing ? 0 : half + 1;
 #pragma unroll
       for (int u = 0; u < kGroup; u += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(xb + at + u);
-        xs[u] = v.x; xs[u + 1] = v.y; xs[u + 2] = v.z; xs[u + 3] = v.w;
+        const float4 v = *reinterpret_cast<const float4*>(xb + u);
+        x[u] = v.x; x[u + 1] = v.y; x[u + 2] = v.z; x[u + 3] = v.w;
       }
 #pragma unroll
-      for (int u = 0; u < kGroup; ++u) ws[u] = wb[(at + u) * 32];
-    };
-    read(0, x[0], wv[0]);
-#pragma unroll 1
-    for (; k + 2 * kGroup <= nb; k += 2 * kGroup) {
-      read(k + kGroup, x[1], wv[1]);
-      wk.steps<kBlock == 32, kGroup>(x[0], wv[0]);
-      read(k + 2 * kGroup < kBlock ? k + 2 * kGroup : 0, x[0], wv[0]);
-      wk.steps<kBlock == 32, kGroup>(x[1], wv[1]);
+      for (int u = 0; u < kGroup; ++u) wv[u] = wb[u * 32 * C];
+      // a block's barrier lies behind the reads of the block in front of it, not behind its steps
+      if (h & 1) more = (h >> 1) + 1 < blocks && __syncthreads_or(wk.live);
+      int lim = 0;
+      if (__builtin_expect(turned, 0)) lim = wk.guard(x, wv);
+      wk.steps(x, wv, lim);
+      turned = wk.turn(turned);
     }
-    if (k + kGroup <= nb) {
-      wk.steps<kBlock == 32, kGroup>(x[0], wv[0]);
-      k += kGroup;
-    }
-    if (kGroup > 8 && k + 8 <= nb) {
-      float x8[8], w8[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) { x8[u] = xb[k + u]; w8[u] = wb[(k + u) * 32]; }
-      wk.steps<kBlock == 32, 8>(x8, w8);
-      k += 8;
-    }
-#pragma unroll 1
-    for (; k < nb; ++k) {
-      const float x1[1] = {xb[k]}, w1[1] = {wb[k * 32]};
-      wk.steps<false, 1>(x1, w1);
-    }
-    if (!__any_sync(0xffffffffu, wk.live)) break;  // every output has fired
   }
-  copies_wait<0>();
 
   // an output that stopped has fired; one that consumed every input fires iff it is armed
   float ws = wk.fin.x, ys = wk.fin.y;
   bool fired = true;
   if (wk.live) {
-    ws = wk.wsum; ys = wk.ysum;
+    ws = wk.plain(wk.wsum); ys = wk.plain(wk.ysum);
     fired = ratio_gt(ys, ws, wk.xprev);
   }
   float yv = g.maxv, iv = 0.f;
@@ -252,20 +278,31 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
   }
 }
 
+template <bool VEC, int C>
+int launch(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out, cudaStream_t s) {
+  const long grid = (long)g.R * ((g.J + 32 * C - 1) / (32 * C));
+  if (grid > 0x7fffffffL) return E_UNSUPPORTED;
+  constexpr size_t smem = sizeof(RingShared<C>);
+  if (allow_smem<snn_walk_ring_kernel<VEC, C>>(smem) != cudaSuccess) return E_CUDA;
+  const cudaError_t e = launch_chained(snn_walk_ring_kernel<VEC, C>, (unsigned)grid, 32 * (C + 1), smem, s, 0, g, lists, nvalid, istride, w, out);
+  count_launch();
+  return e == cudaSuccess ? OK : E_CUDA;
+}
+
 }  // namespace
 
+// How many warps of 32 outputs share a list and a copying warp: one while every CTA has an SM to itself (one row of 4096 -> 512 36 us,
+// 38 with two), two up to six CTAs per SM, which is what the registers hold. Beyond, four where that makes it one wave again (25 088 ->
+// 1024 at 64 samples 424 us, 515 with two; 2000 -> 512 at 128 43, 53): the copying warp, 28 cycles an entry, holds four back (9000 ->
+// 700 at 30 samples 115 us, 89 with two).
 int launch_walk_ring(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
                      const LaunchInfo& li, cudaStream_t s) {
-  const int slices = (g.J + 31) / 32;
-  const long grid = ((long)g.R * slices + kWarps - 1) / kWarps;
-  if (grid > 0x7fffffffL) return E_UNSUPPORTED;
   const bool vec = (g.J & 3) == 0 && ((uintptr_t)w & 15) == 0;
-  const bool small = grid * kWarps > 8L * li.num_sms;
-  auto go = [&](auto kernel) { (void)launch_chained(kernel, (unsigned)grid, 32 * kWarps, 0, s, 0, g, lists, nvalid, istride, w, out, slices); };
-  if (vec) small ? go(snn_walk_ring_kernel<true, 16>) : go(snn_walk_ring_kernel<true, 32>);
-  else small ? go(snn_walk_ring_kernel<false, 16>) : go(snn_walk_ring_kernel<false, 32>);
-  count_launch();
-  return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
+  if (!vec) return launch<false, 1>(g, lists, nvalid, istride, w, out, s);
+  auto ctas = [&](int c) { return (long)g.R * ((g.J + 32 * c - 1) / (32 * c)); };
+  if (ctas(1) <= li.num_sms) return launch<true, 1>(g, lists, nvalid, istride, w, out, s);
+  if (ctas(2) > 6L * li.num_sms && ctas(4) <= 4L * li.num_sms) return launch<true, 4>(g, lists, nvalid, istride, w, out, s);
+  return launch<true, 2>(g, lists, nvalid, istride, w, out, s);
 }
 
 }  // namespace snntc

@@ -133,3 +133,21 @@ def test_spikes_that_rounding_hides_and_negative_denominators(J, band, scale):
         assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=layout)), ref), "layout %d" % layout
     got = ref[:64].cpu().numpy()
     assert np.array_equal(got < 9e4, o32["y"] < 9e4)
+
+
+@pytest.mark.parametrize("R,I,J", [(37, 33, 100), (37, 64, 128), (75, 97, 36), (290, 70, 256), (290, 31, 200), (148, 65, 500), (900, 40, 64),
+                                   (600, 200, 12)])
+@pytest.mark.parametrize("bv", [0.0, 1.0])
+def test_walk_with_a_copying_warp(R, I, J, bv):
+    """One, two and four warps beside the one that copies (chosen by the number of CTAs), ragged slices, lists that end anywhere in a
+    block, an empty row, a row of ties: the bits of one output per lane from global memory."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    x, w = P.make_inputs(R + I + J, (R, I), (I + (bv > 0), J), "ref", bias=bv > 0)
+    x[3] = 1e5
+    x[5] = 2.0
+    params = O.fc_params(biasvolt=bv)
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
+    assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=16)), ref)
+    assert torch.equal(ops.snn_fc(xd, wd, params), ref)
