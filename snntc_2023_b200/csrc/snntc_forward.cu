@@ -683,15 +683,16 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   const bool copies16 = (g.J & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
   const bool few = copies16 && g.J > 32 ? (long)g.R * ((g.J + 63) / 64) <= 12L * li.num_sms : ring_items <= 8L * li.num_sms;
   const bool ring = (opt.walk_layout & 16) != 0 || (own && few);
-  // Several rows per warp for fan-out up to 64, where that leaves enough warps: 6 per SM at eight rows to a warp (fan-out 16;
-  // 10 where the weights miss the L1 cache), 14 at four (32), 48 at two (64). With fewer the pairs walk, a warp per row, hides
-  // its latencies better (5 880 rows of 6400 x 16: 540 against 770 us; 8 064 of 576 x 16: 107 against 61).
+  // Several rows per warp for fan-out up to 64, where that leaves enough warps: 5 per SM at eight rows to a warp (fan-out 16;
+  // 10 where the weights miss the L1 cache), 11 at four (32), 40 at two (64). With fewer the pairs walk, a warp per row, hides
+  // its latencies better. Pairs against rows, us: 576 -> 16 4000 rows 35, 39, 7000 rows 53, 39; 576 -> 32 35, 37 and 54, 43; 147 -> 64 8000
+  // rows 25, 27, 14 000 37, 35; 500 -> 64 8000 54, 61, 14 000 85, 85, -> 36 80, 76.
   bool rows = !ring && walk_rows_ok(g, w) && (own || (opt.walk_layout & 96) != 0);
   if (rows && own) {
     const int lanes = g.J > 32 ? 16 : (g.J > 16 ? 8 : 4);
     const long warps_per_sm = (long)g.R * lanes / 32 / li.num_sms;
     const bool in_l1 = (size_t)(g.I + 1) * g.J * sizeof(float) <= (size_t)128 << 10;
-    rows = warps_per_sm >= (lanes == 16 ? 48 : (lanes == 8 ? 14 : (in_l1 ? 6 : 10)));
+    rows = warps_per_sm >= (lanes == 16 ? 40 : (lanes == 8 ? 11 : (in_l1 ? 5 : 10)));
     // (65 536 rows of 576 x 64: 364 us with the pairs walk and its weights in shared memory, 380 so, but 16 384 rows 130 and 113;
     // 262 144 of 27 x 64: 222, 208, but 59 400 of 64 x 64 75, 83; where the weights do not fit shared memory the pairs walk from
     // global memory is ahead too: 65 536 of 900 x 64 649, 672)
