@@ -80,9 +80,16 @@ __global__ void snn_weight_transpose_kernel(const float* w, float* __restrict__ 
 //
 // The lists a pixel needs (one per tap that an output reads it through) are first copied into shared memory by
 // the pixel's own lanes, back to back and with the tap folded into the entry (its third word becomes the element
-// offset of weight row (tap, j) in Wt), kStage / PPW entries per pixel and round. The arithmetic then runs over
-// that flat sequence: one broadcast shared-memory read per entry instead of a global read in front of every
-// weight read, and one loop instead of one per tap.
+// offset of weight row (tap, j) in Wt), kStage / PPW entries per pixel and round. A lane looks up one tap, a scan over the lanes
+// gives where each tap's entries lie in the sequence, and every lane finds the taps of its entries by bisection: two round
+// trips to the L2 per round instead of two per tap. The arithmetic then runs over that flat sequence, whose last group is filled
+// up with entries that add nothing: one broadcast shared-memory read per entry, UN weight rows in flight.
+// What bounds it: the L1 cache, which hands every weight to a single FMA, and instruction issue (a compare at half rate and a
+// predicated FMA per channel are 8 of 13 instructions per entry at CPL = 4).
+// Measured (B200, the whole dX, with a lookup per tap, entries masked one by one and 64-bit weight pointers -> now): 256 images of
+// 32x32, 64 -> 64 channels, 13 % of the outputs with a gradient 543 -> 449 us; 16x16, 64 -> 128, 36 %: 493 -> 467; 37 of 45x39, 20 ->
+// 52, 5x5 stride 2: 115 -> 73; 16 of 8x8, 256 -> 256: 83 -> 70. Eight entries in flight at CPL = 4: the last but one 76, a small layer of
+// 128 -> 256 72 instead of 77.
 constexpr int kStage = 256;   // staged list entries per warp and round
 
 template <int CPL, int LPP>
@@ -95,7 +102,7 @@ snn_dx_sparse_kernel(const Geometry g, const float* x, const float* wt,
   if (gate.nz != nullptr && ld_plain(gate.nz) > gate.threshold) return;
   constexpr int PPW = 32 / LPP;                       // pixels per warp
   constexpr int SB = kStage / PPW;                    // staged entries per pixel and round
-  constexpr int UN = CPL <= 4 ? 4 : 2;                // entries whose weight reads are in flight together
+  constexpr int UN = CPL <= 8 ? 4 : 2;                // entries whose weight reads are in flight together
   __shared__ uint4 stage_all[(kThreads / 32) * kStage];
   const int lane = threadIdx.x & 31;
   const int sub = lane / LPP;                         // which of the warp's pixels
@@ -103,18 +110,22 @@ snn_dx_sparse_kernel(const Geometry g, const float* x, const float* wt,
   const int c0 = gl * CPL;                            // first channel of this lane
   uint4* stage = stage_all + (threadIdx.x >> 5) * kStage + sub * SB;
   const int C = g.C, J = g.J;
-  const bool lane_has_channels = c0 < C;              // C % 4 == 0 and CPL % 4 == 0: a lane's float4s are all in or all out
   const int P = g.B * g.H * g.W;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   const int taps = g.Kh * g.Kw;
-  const float* wlane = wt + c0;
-  for (int pw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; pw * PPW < P; pw += warps) {
+  // C % 4 == 0 and CPL % 4 == 0: a lane's float4s are all in or all out; one that is out reads the row's first channels, for inputs of
+  // +inf that no output reaches
+  unsigned coff[CPL / 4];
+#pragma unroll
+  for (int k = 0; k < CPL / 4; ++k) coff[k] = c0 + 4 * k < C ? (unsigned)(c0 + 4 * k) : 0u;
+  const char* wbytes = reinterpret_cast<const char*>(wt);
+  for (int pw = __shfl_sync(0xffffffffu, (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), 0); pw * PPW < P; pw += warps) {
     const int p = pw * PPW + sub;
     const bool pix_ok = p < P;
     float xr[CPL], acc[CPL];
 #pragma unroll
     for (int k = 0; k < CPL; ++k) { xr[k] = CUDART_INF_F; acc[k] = 0.f; }
-    if (pix_ok && lane_has_channels) {
+    if (pix_ok) {
 #pragma unroll
       for (int k4 = 0; k4 < CPL; k4 += 4) {
         if (c0 + k4 < C) {
@@ -130,60 +141,72 @@ snn_dx_sparse_kernel(const Geometry g, const float* x, const float* wt,
       ph = t % g.H;
       pb = t / g.H;
     }
-    // cursor of this pixel through its lists: tap, and the first entry of that tap's list not staged yet
-    int tap = pix_ok ? 0 : taps, e0 = 0;
-    for (;;) {
-      // ---- stage up to SB entries of this pixel, tap after tap (the terms keep their order: tap-major, j ascending)
-      int staged = 0;
-      while (tap < taps && staged < SB) {
+    for (int tap0 = 0; tap0 < taps; tap0 += LPP) {    // (the terms keep their order: tap-major, j ascending)
+      // ---- this lane's tap: the receptive field that reads the pixel through (kh, kw), if there is one
+      int n = 0, r = 0;
+      const int tap = tap0 + gl;
+      {
         const int kh = tap / g.Kw, kw = tap - kh * g.Kw;
-        // the receptive field that reads this pixel through tap (kh, kw), if there is one
         const int hh = ph + g.pad_top - kh, ww = pwid + g.pad_left - kw;
         int nh = hh, nw = ww;
-        bool ok = hh >= 0 && ww >= 0;
+        bool ok = pix_ok && tap < taps && hh >= 0 && ww >= 0;
         if (g.Sh != 1 || g.Sw != 1) {
           nh = hh / g.Sh; nw = ww / g.Sw;
           ok = ok && nh * g.Sh == hh && nw * g.Sw == ww;
         }
-        ok = ok && nh < g.Nh && nw < g.Nw;
-        int n = 0;
-        const uint4* src = list;
-        if (ok) {
-          const int r = (pb * g.Nh + nh) * g.Nw + nw;
+        if (ok && nh < g.Nh && nw < g.Nw) {
+          r = (pb * g.Nh + nh) * g.Nw + nw;
           n = ld_plain(count + r);
-          src = list + (size_t)r * J;
         }
-        const int take = min(n - e0, SB - staged);
-        const unsigned tapoff = (unsigned)tap * (unsigned)J;
-        for (int e = gl; e < take; e += LPP) {
-          uint4 en = ld_plain(src + e0 + e);
-          en.z = (tapoff + en.z) * (unsigned)C;
-          stage[staged + e] = en;
-        }
-        staged += take;
-        e0 += take;
-        if (e0 >= n) { ++tap; e0 = 0; }
       }
-      __syncwarp();
-      const int nmax = __reduce_max_sync(0xffffffffu, staged);
-      if (nmax == 0) break;   // every pixel of the warp is through its lists
-      // ---- the arithmetic over the staged entries. A slot past the end of this pixel's share holds
-      // (y = -inf, u = 0, offset 0): its compare is false for every input and its weight read stays inside the table.
-      for (int e = 0; e < nmax; e += UN) {
-        uint4 en[UN];
+      int end = n;                                    // entries up to and with this lane's tap
 #pragma unroll
-        for (int q = 0; q < UN; ++q) {
-          en[q] = make_uint4(0xff800000u, 0u, 0u, 0u);
-          if (e + q < staged) en[q] = stage[e + q];
+      for (int d = 1; d < LPP; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, end, d, LPP);
+        if (gl >= d) end += v;
+      }
+      const int total = __shfl_sync(0xffffffffu, end, LPP - 1, LPP);
+      const int most = __reduce_max_sync(0xffffffffu, total);
+      for (int first = 0; first < most; first += SB) {
+        const int nmax = min(most - first, SB);
+        // ---- stage entries first .. first + nmax - 1 of this pixel
+#pragma unroll 1
+        for (int i = 0; i < nmax; i += 4 * LPP) {
+          uint4 en[4];
+          unsigned at[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int e = first + i + q * LPP + gl;
+            int t = 0;                                // taps whose entries all lie in front of e
+#pragma unroll
+            for (int d = LPP / 2; d >= 1; d >>= 1)
+              if (__shfl_sync(0xffffffffu, end, t + d - 1, LPP) <= e) t += d;
+            const int start = __shfl_sync(0xffffffffu, end - n, t, LPP), row = __shfl_sync(0xffffffffu, r, t, LPP);
+            at[q] = (unsigned)(tap0 + t) * (unsigned)J;
+            en[q] = make_uint4(0xff800000u, 0u, 0u, 0u);   // behind the end: y = -inf, u = 0
+            if (e < total) en[q] = ld_plain(list + (size_t)row * J + (e - start));
+            else at[q] = 0u;
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int e = i + q * LPP + gl;
+            en[q].z = (at[q] + en[q].z) * (unsigned)C;
+            if (SB % (4 * LPP) == 0 || e < SB) stage[e] = en[q];
+          }
         }
-        if (lane_has_channels) {
+        __syncwarp();
+        // ---- the arithmetic over the staged entries
+#pragma unroll 1
+        for (int e = 0; e < nmax; e += UN) {
+          uint4 en[UN];
           float4 w4[UN][CPL / 4];
 #pragma unroll
-          for (int q = 0; q < UN; ++q) {
-            const float* wrow = wlane + en[q].z;
+          for (int q = 0; q < UN; ++q) en[q] = stage[e + q];
 #pragma unroll
-            for (int k4 = 0; k4 < CPL; k4 += 4)
-              w4[q][k4 / 4] = (c0 + k4 < C) ? ld_readonly(reinterpret_cast<const float4*>(wrow + k4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int q = 0; q < UN; ++q) {
+#pragma unroll
+            for (int k = 0; k < CPL / 4; ++k)
+              w4[q][k] = ld_readonly(reinterpret_cast<const float4*>(wbytes + (size_t)(en[q].z + coff[k]) * 4u));
           }
 #pragma unroll
           for (int q = 0; q < UN; ++q) {
@@ -197,10 +220,10 @@ snn_dx_sparse_kernel(const Geometry g, const float* x, const float* wt,
             }
           }
         }
+        __syncwarp();   // the buffer is rewritten by the next round
       }
-      __syncwarp();   // the buffer is rewritten by the next round
     }
-    if (pix_ok && lane_has_channels) {
+    if (pix_ok) {
 #pragma unroll
       for (int k4 = 0; k4 < CPL; k4 += 4)
         if (c0 + k4 < C)

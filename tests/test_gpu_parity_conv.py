@@ -281,3 +281,23 @@ def test_conv_inputs_that_never_spike_or_are_not_numbers():
     out = ops.snn_cv(xd, wd, params, 1, 1, H, W).cpu().numpy()
     P.check_forward(out[:B], out[B:], O.cv_forward(x, w, params, "f32"), O.cv_forward(x, w, params, "f64"),
                     rows=P.im2col_rows(x, 3, 3, 1, 1, "SAME"), what="conv with empty lists")
+
+
+@pytest.mark.parametrize("C", [16, 20, 40, 72, 136, 260, 512])
+@pytest.mark.parametrize("k,stride,J,density", [(1, 1, 37, 1.0), (3, 1, 150, 1.0), (3, 2, 64, 0.2), (5, 1, 24, 0.5), (7, 3, 33, 0.05), (3, 1, 8, 0.0)])
+def test_conv_dx_list_rounds(C, k, stride, J, density):
+    """The list-walking dX against the register tile, bit for bit, where its rounds and groups have edges: more taps than lanes per
+    pixel, lists of a pixel longer than a round and shorter than a group of entries, no entry at all, channels that fill no lane."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    rng = np.random.default_rng(C + 10 * k + J)
+    B, H, W = 2, 9, 7
+    x, w = P.make_inputs(C + k + J, (B, H, W, C), (k * k * C + 1, J), "ref", bias=True)
+    params = O.cv_params(k, k, stride, stride, "SAME")
+    pt, pl, Nh, Nw = ops.conv_geometry(H, W, k, k, stride, stride, "SAME")
+    gr = rng.standard_normal((B, Nh, Nw, J)).astype(np.float32) * (rng.random((B, Nh, Nw, J)) < density)
+    xd, wd, gd = (torch.from_numpy(a.astype(np.float32)).cuda() for a in (x, w, gr))
+    out = ops.snn_cv(xd, wd, params, pt, pl, Nh, Nw)
+    a, _, _ = ops.snn_cv_grad(gd, xd, wd, params, out, pt, pl, opts=_lib.options(dx_kernel=1))
+    b, _, _ = ops.snn_cv_grad(gd, xd, wd, params, out, pt, pl, opts=_lib.options(dx_kernel=2))
+    assert torch.equal(a, b)
