@@ -4,7 +4,7 @@
 //
 //   dW[i,j] = sum_r [x_ri <= y_rj] (x_ri - y_rj) u_rj,   u_rj = 0 wherever output (r,j) carries no gradient.
 //
-// As there, a warp owns FOUR output channels and every lane 4*QL fan-in rows, a CTA 32 channels, a slice of the
+// As there, a warp owns FOUR output channels and every lane 4*QL fan-in rows, a CTA 64 (or 32) channels, a slice of the
 // rows r (blockIdx.z) and a tile of the fan-in (blockIdx.y), and the rows of a stage of 16 whose four channels
 // carry no gradient are skipped by a warp-uniform branch. What differs is how a stage gets into shared memory. In
 // snn_dw_skip_kernel 160 threads issue sixteen 16-byte copies each per stage, with the tap arithmetic and the
@@ -22,10 +22,12 @@
 // holds the warps together stage by stage: how much a warp has to do depends on how many of its four channels carry
 // gradients, and with a barrier per stage every warp took the time of the busiest (the largest stall of the kernel).
 //
-// What bounds it: waiting for a stage's copies (65 536 rows of 577 x 64, 12 % of the gradients, 100 us: of the warps per issue 2.98 wait
-// for copies, 2.13 for fixed latencies, 1.31 for shared memory; L1 and shared memory 53 % busy, issue 40 %): the taps' boxes overlap,
-// so that a stage brings every pixel in up to nine times. With dW of 262 144 rows of 577 x 64, 12 % of the outputs carrying a gradient, 353 -> 256 us
-// against two stages, a CTA barrier per stage, 32 outputs per CTA and eight waves of CTAs; 200 704 x 1153 x 128 790 -> 658 us.
+// What bounds it: the latency of a row's chain (read, test, FMAs) at four warps per scheduler, and the warp with the most to do. Which
+// channels a warp owns is therefore dealt out by their activity (see `order`). With dW of 262 144 rows of 577 x 64, 12 % of the
+// outputs carrying a gradient, 353 -> 256 us against two stages, a CTA barrier per stage, 32 outputs per CTA and eight waves of CTAs; 200 704
+// x 1153 x 128 790 -> 658 us. Channels by activity instead of four neighbours (the whole dW, its u kernel and reduction with it): 262 144 x
+// 577 x 64, 13 % active, 438 -> 378 us; 65 536 x 577 x 128, 36 % 410 -> 341; 16 384 x 1153 x 256, 36 % 461 -> 338; 65 536 x 1153 x 128, 13 %
+// 360 -> 359 (the neighbours there are nearly even); 131 072 x 576 x 128, 79 % 1032 -> 1014.
 //
 // The x tile of a stage is laid out [tap][row][channel] (one box after the other), so a fan-in tile is made of
 // whole taps, taps_per_tile = 640 / C of them; the bias row (x = biasvolt for every r) is a sum per output channel
@@ -70,7 +72,10 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long full[kMaxDepth], empty[kMaxDepth];
   __shared__ int gave_up;
-  unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);   // boxes land on 128-byte boundaries
+  __shared__ __align__(16) int order[kJT];                         // output channels (of this CTA) by warp, four each
+  __shared__ int active[kJT];
+  __shared__ float4 own_all[NW][2][kRS];                           // a stage's u and y of each warp's four channels
+  unsigned char* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // swizzled boxes: 1024-byte boundaries
   const int C = g.C, J = g.J, I = g.I;
   const int Itot = I + g.has_bias;
   const int taps = g.Kh * g.Kw;
@@ -79,8 +84,8 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   const bool bias_here = g.has_bias && blockIdx.y == gridDim.y - 1;
   const int xfloats = taps_per_tile * kRS * C;                     // floats of one x buffer
   float* Xs = reinterpret_cast<float*>(base);                      // [depth][taps_per_tile][kRS][C]
-  float* Ys = Xs + depth * xfloats;                                // [depth][kRS][kJT]
-  float* Us = Ys + depth * kRS * kJT;                              // [depth][kRS][kJT]
+  float* Ys = Xs + ((depth * xfloats + 255) & ~255);               // [depth][kJT / 32][kRS][32], chunks swizzled (see at_field)
+  float* Us = Ys + depth * kRS * kJT;                              // the same
 
   const bool fast = scale != 1.0f && ld_plain(exact_flag) == 0;
   const float sc = fast ? scale : 1.0f;                 // s
@@ -120,16 +125,16 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
     }
     __syncwarp();
-    for (int tl = lane; tl < ntap + 2; tl += 32) {
+    for (int tl = lane; tl < ntap + 2 * (kJT / 32); tl += 32) {
       if (tl < ntap) {
         const int tap = tap0 + tl;
         const int kh = tap / g.Kw, kw = tap - kh * g.Kw;
         tma_load_4d(smem_u32(Xs + buf * xfloats + tl * kRS * C), &map_x, bar, 0, nw0 - g.pad_left + kw,
                     nh0 - g.pad_top + kh, b);
-      } else if (tl == ntap) {
-        tma_load_4d(smem_u32(Ys + buf * kRS * kJT), &map_y, bar, j0, nw0, nh0, b);
       } else {
-        tma_load_4d(smem_u32(Us + buf * kRS * kJT), &map_u, bar, j0, nw0, nh0, b);
+        const int part = (tl - ntap) >> 1;          // 32 output channels
+        float* to = ((tl - ntap) & 1 ? Us : Ys) + buf * kRS * kJT + part * kRS * 32;
+        tma_load_4d(smem_u32(to), (tl - ntap) & 1 ? &map_u : &map_y, bar, j0 + 32 * part, nw0, nh0, b);
       }
     }
     __syncwarp();
@@ -159,38 +164,44 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   // the same (what it reads lies inside the CTA's shared memory: the other x buffer or the y/u tiles) and its sums
   // are dropped at the end.
   const int lane_part = C256 ? 4 * lane : ((4 * lane) / C) * kRS * C + (4 * lane) % C;
-  int irow[QL];              // weight row of the chunk's first float; -1: the chunk lies behind the tile's taps
-#pragma unroll
-  for (int c = 0; c < QL; ++c) {
-    const int f = 4 * lane + 128 * c;
-    irow[c] = f < ntap * C ? tap0 * C + f : -1;
-  }
   // the bias row: x = biasvolt for every r, one sum per output channel, kept by every lane alike (it takes two
   // instructions per row and channel beside the thirty of a fan-in chunk)
   float accb[4] = {0.f, 0.f, 0.f, 0.f};
 
-  // acc[c][jj][h]: fan-in rows irow[c] + 2h, +1 (one 64-bit pair), output channel j0 + 4*warp + jj
+  // acc[c][jj][h]: fan-in floats 4*lane + 128*c + 2h, +1 of the tile (one 64-bit pair), the warp's channel jj
   uint64_t acc[QL][4][2];
 #pragma unroll
   for (int c = 0; c < QL; ++c)
 #pragma unroll
     for (int jj = 0; jj < 4; ++jj) acc[c][jj][0] = acc[c][jj][1] = pack2(0.f, 0.f);
 
+  // float of field `row` and channel c in a y or u buffer: rows of 32 channels, whose 16-byte chunks the copy swizzles by the row, so
+  // that a channel's 16 fields are read two at a time instead of one after the other
+  auto at_field = [](int row, int c) { return (c >> 5) * (kRS * 32) + row * 32 + ((((c >> 2) ^ row) & 7) << 2) + (c & 3); };
+
+  unsigned at01 = 0u, at23 = 0u;                  // where this lane's field of the warp's four channels lies in a buffer
+  const float* const own_from = lane < kRS ? Us : Ys;
+
   auto reduce_stage = [&](int buf, auto fast_c) {
     constexpr bool FAST = decltype(fast_c)::value;
     const float* xb = Xs + buf * xfloats + lane_part;
-    // which of the 16 rows carry a gradient for one of this warp's four channels: lane rl looks at row rl, one vote
+    // The warp's four channels of the stage, a field per lane (lanes from 16 on: y), put side by side for the loop below. Which of the
+    // 16 rows carry a gradient for one of the four: one vote.
+    float4* own = &own_all[warp][0][0];
     unsigned todo;
     {
-      const float4 uq = *reinterpret_cast<const float4*>(Us + (buf * kRS + (lane & (kRS - 1))) * kJT + 4 * warp);
-      todo = __ballot_sync(0xffffffffu, (uq.x != 0.f) | (uq.y != 0.f) | (uq.z != 0.f) | (uq.w != 0.f)) & ((1u << kRS) - 1u);
+      const float* from = own_from + buf * kRS * kJT;
+      const float4 v = make_float4(from[at01 & 0xffff], from[at01 >> 16], from[at23 & 0xffff], from[at23 >> 16]);
+      todo = __ballot_sync(0xffffffffu, (v.x != 0.f) | (v.y != 0.f) | (v.z != 0.f) | (v.w != 0.f)) & ((1u << kRS) - 1u);
+      if (todo != 0u) own[lane] = v;                       // (every lane is through with the stage before: the vote)
+      __syncwarp();
     }
 #pragma unroll 1
     while (todo != 0u) {
       const int rl = __ffs((int)todo) - 1;
       todo &= todo - 1u;
-      const float4 y4 = *reinterpret_cast<const float4*>(Ys + (buf * kRS + rl) * kJT + 4 * warp);
-      const float4 u4 = *reinterpret_cast<const float4*>(Us + (buf * kRS + rl) * kJT + 4 * warp);
+      const float4 u4 = own[rl], y4 = own[kRS + rl];
+      const float uu[4] = {u4.x, u4.y, u4.z, u4.w}, yv[4] = {y4.x, y4.y, y4.z, y4.w};
       float xr[QL][4];
       const float* xrow = xb + rl * C;
 #pragma unroll
@@ -198,8 +209,6 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         const float4 v = *reinterpret_cast<const float4*>(xrow + (C256 ? (c >> 1) * kRS * 256 + (c & 1) * 128 : 2048 * c));
         xr[c][0] = v.x; xr[c][1] = v.y; xr[c][2] = v.z; xr[c][3] = v.w;
       }
-      const float yv[4] = {y4.x, y4.y, y4.z, y4.w};
-      const float uu[4] = {u4.x, u4.y, u4.z, u4.w};
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) {
         if (uu[jj] == 0.f) continue;              // warp-uniform
@@ -222,12 +231,44 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   // The warps are not held together by a barrier per stage: a warp that is through with a stage says so on the buffer's `empty`
   // barrier and goes on, ahead of the slowest by what is in flight. In turn, warp k mod NW when it comes to stage k, they wait
   // until everyone is through with stage k - lag and queue stage k - lag + depth in its place.
-  for (int st = warp; st < min(depth, nstages); st += NW) issue(st, st);
+  const int first_stages = min(depth, nstages);
+  for (int st = warp; st < first_stages; st += NW) issue(st, st);
   const int lag = min(2, depth - 1);
   bool failed = false;
+
+  // Which four channels a warp takes. Channels differ in how often they carry a gradient (one in four never, one in four nearly
+  // always), and a stage lasts as long as the warp with the most to do: of four neighbouring channels 1.7 to 2.2 times the mean, with
+  // the channels dealt out in the order of their activity, forth and back, 1.05 to 1.2 times. The activity is counted over the first
+  // stages, by every CTA for itself: which warp adds up a channel changes no sum.
+  for (int d = 0; d < first_stages && !failed; ++d) failed = !passed(&full[d], 0u);
+  if (tid < kJT) {
+    int n = 0;
+    if (!failed)
+      for (int d = 0; d < first_stages; ++d)
+#pragma unroll
+        for (int row = 0; row < kRS; ++row) n += Us[d * kRS * kJT + at_field(row, tid)] != 0.f;
+    active[tid] = n;
+  }
+  __syncthreads();
+  if (tid < kJT) {
+    const int n = active[tid];
+    int rank = 0;
+#pragma unroll 8
+    for (int c = 0; c < kJT; ++c) rank += active[c] > n || (active[c] == n && c < tid);
+    const int k = rank / NW, w = rank % NW;
+    order[4 * (k & 1 ? NW - 1 - w : w) + k] = tid;
+  }
+  failed = __syncthreads_or(failed) != 0;
+  {
+    const int4 ch = *reinterpret_cast<const int4*>(order + 4 * warp);
+    const int row = lane & (kRS - 1);
+    at01 = (unsigned)at_field(row, ch.x) | (unsigned)at_field(row, ch.y) << 16;
+    at23 = (unsigned)at_field(row, ch.z) | (unsigned)at_field(row, ch.w) << 16;
+  }
+
   int buf = 0, rbuf = depth - lag;        // buffers of stages it and it - lag
   unsigned phase = 0u, rphase = 1u;       // and the parities of their phases
-  for (int it = 0; it < nstages; ++it) {
+  for (int it = 0; it < nstages && !failed; ++it) {
     if (it >= lag && it % NW == warp && it - lag + depth < nstages) {
       failed = !passed(&empty[rbuf], rphase);
       if (failed) break;
@@ -252,26 +293,42 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     __syncthreads();
   }
 
-  float* __restrict__ dst = partial + (size_t)blockIdx.z * Itot * J;
-  const int j = j0 + 4 * warp;
-  if (j < J) {
+  // The sums go out through shared memory (no copy is in flight any more), where they are turned so that a row's channels lie
+  // together: row (f % 4, f / 4) for fan-in float f of the tile, lanes on neighbouring rows.
+  constexpr int kPitch = kJT + 1;
+  float* turn = reinterpret_cast<float*>(base);
+  {
+    const int4 ch = *reinterpret_cast<const int4*>(order + 4 * warp);
+    const int chs[4] = {ch.x, ch.y, ch.z, ch.w};
 #pragma unroll
     for (int c = 0; c < QL; ++c) {
-      if (irow[c] < 0) continue;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        float v[2][4];
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) unpack2(acc[c][jj][h], v[0][jj], v[1][jj]);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i = irow[c] + 2 * h + e;
-          *reinterpret_cast<float4*>(dst + (size_t)i * J + j) = make_float4(v[e][0], v[e][1], v[e][2], v[e][3]);
+        for (int jj = 0; jj < 4; ++jj) {
+          float a, b;
+          unpack2(acc[c][jj][h], a, b);
+          turn[((2 * h) * 32 * QL + 32 * c + lane) * kPitch + chs[jj]] = a;
+          turn[((2 * h + 1) * 32 * QL + 32 * c + lane) * kPitch + chs[jj]] = b;
         }
       }
     }
-    if (bias_here && lane == 0)
-      *reinterpret_cast<float4*>(dst + (size_t)I * J + j) = make_float4(accb[0], accb[1], accb[2], accb[3]);
+    if (bias_here && lane == 0) {
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) turn[128 * QL * kPitch + chs[jj]] = accb[jj];
+    }
+  }
+  __syncthreads();
+  float* __restrict__ dst = partial + (size_t)blockIdx.z * Itot * J;
+  const int j = j0 + 4 * (tid % NW);
+  if (j < J) {
+    for (int f = tid / NW; f <= ntap * C; f += 32) {
+      const bool bias_row = f == ntap * C;
+      if (bias_row && !bias_here) break;
+      const float* from = turn + (bias_row ? 128 * QL : (f & 3) * 32 * QL + (f >> 2)) * kPitch + 4 * (tid % NW);
+      const int i = bias_row ? I : tap0 * C + f;
+      *reinterpret_cast<float4*>(dst + (size_t)i * J + j) = make_float4(from[0], from[1], from[2], from[3]);
+    }
   }
 }
 
@@ -290,9 +347,10 @@ TmaPlan plan(const Geometry& g) {
   // leave half of a last CTA without outputs, 32 and two CTAs per SM (96 outputs: 54 against 58 us)
   p.nw = (g.J & 63) == 0 || (g.J & 63) > 32 ? 16 : 8;
   const size_t stage = (size_t)kRS * (tpt * g.C + 8 * p.nw) * sizeof(float);
-  const size_t room = (p.nw == 16 ? 224 : 111) * 1024;
+  const size_t room = (p.nw == 16 ? 216 : 106) * 1024;
   p.depth = (int)std::min<size_t>(kMaxDepth, room / stage);
-  p.smem = p.depth * stage + 128;
+  // (the tile of sums that goes out through the same memory: 640 fan-in rows and the bias row of 65 or 33 floats at most)
+  p.smem = std::max(p.depth * stage, (size_t)(128 * p.ql + 1) * (4 * p.nw + 1) * sizeof(float)) + 2048;
   return p;
 }
 
@@ -379,7 +437,7 @@ int launch_dw_tma(const Geometry& g, const float* uv, const float* x, const floa
   const TmaPlan p = plan(g);
   const int lg = stage_wseg_log2(g);
   const cuuint32_t wseg = 1u << lg, hseg = (cuuint32_t)kRS >> lg;
-  const cuuint32_t jt = 4u * p.nw;
+  const cuuint32_t jt = 4u * p.nw;   // output channels per CTA, copied 32 at a time (128 bytes: a swizzle's width)
   const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
   CUtensorMap mx, my, mu;
   {
@@ -395,13 +453,13 @@ int launch_dw_tma(const Geometry& g, const float* uv, const float* x, const floa
     // the outputs as [image][row][column][channel]: fields past the edge of the map read as zero
     const cuuint64_t dims[4] = {(cuuint64_t)g.J, (cuuint64_t)g.Nw, (cuuint64_t)g.Nh, (cuuint64_t)g.B};
     const cuuint64_t strides[3] = {(cuuint64_t)g.J * 4, (cuuint64_t)g.Nw * g.J * 4, (cuuint64_t)g.Nh * g.Nw * g.J * 4};
-    const cuuint32_t box[4] = {jt, wseg, hseg, 1u};
+    const cuuint32_t box[4] = {32u, wseg, hseg, 1u};
     if (enc(&my, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(out), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return E_UNSUPPORTED;
     if (enc(&mu, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(uv), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return E_UNSUPPORTED;
   }

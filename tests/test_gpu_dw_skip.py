@@ -31,3 +31,33 @@ def test_conv_dw_with_single_column_copies(B, H, W, C, Kh, Kw, Sh, Sw, Kc, paddi
     for kernel in (2, 1, 0):
         _, dw, _ = ops.snn_cv_grad(gd, xd, wd, params, out, pt, pl, opts=_lib.options(dw_kernel=kernel))
         P.check_close(dw.cpu().numpy(), ref["dw"], "dW kernel %d" % kernel, abs_sum=ref["dw_abs"])
+
+
+@pytest.mark.parametrize("C,J,k", [(64, 64, 3), (32, 96, 3), (128, 52, 3), (16, 128, 1), (256, 40, 2), (8, 36, 5)])
+@pytest.mark.parametrize("pattern", ["hot", "late", "none", "all"])
+def test_channels_dealt_out_by_activity(C, J, k, pattern):
+    """dW through tensor maps with output channels that differ in how often they carry a gradient: a few always and the rest never, only
+    in images that the first stages do not see, none at all, all: against the register tile."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    rng = np.random.default_rng(C + J + k)
+    B, H, W = 5, 19, 17
+    x, w = P.make_inputs(C + J + k, (B, H, W, C), (k * k * C + 1, J), "ref", bias=True)
+    params = O.cv_params(k, k, 1, 1, "SAME")
+    pt, pl, Nh, Nw = ops.conv_geometry(H, W, k, k, 1, 1, "SAME")
+    gr = rng.standard_normal((B, Nh, Nw, J)).astype(np.float32)
+    if pattern == "hot":
+        gr[..., rng.permutation(J)[J // 8:]] = 0
+    elif pattern == "late":
+        gr[:3] = 0
+        gr[..., ::3] = 0
+    elif pattern == "none":
+        gr[:] = 0
+    xd, wd, gd = (torch.from_numpy(a).cuda() for a in (x, w, gr))
+    out = ops.snn_cv(xd, wd, params, pt, pl, Nh, Nw)
+    _, dw1, _ = ops.snn_cv_grad(gd, xd, wd, params, out, pt, pl, opts=_lib.options(dw_kernel=1))
+    _, dw4, _ = ops.snn_cv_grad(gd, xd, wd, params, out, pt, pl, opts=_lib.options(dw_kernel=4))
+    assert float((dw4 - dw1).norm()) <= 1e-5 * float(dw1.norm())     # sums of 32-bit floats in another order
+    _, dw5, _ = ops.snn_cv_grad(gd, xd, wd, params, out, pt, pl, opts=_lib.options(dw_kernel=4))
+    assert torch.equal(dw4, dw5)
+    assert _lib.load_measure().snntc_copy_timeouts() == 0
