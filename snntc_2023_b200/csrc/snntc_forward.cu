@@ -671,9 +671,9 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   // A fan-out that is no multiple of four: with more than a few items, or more inputs than the 4-byte copies of the walk below
   // take as long over as one more launch (2 rows of 6852 -> 135: 176 -> 82 us with the sort, 30 of 991 -> 126: 36 -> 22, 20 of
   // 200 -> 501: 14 -> 12), the weights are copied with padded rows (by the kernel that reads them for the bound), so that every
-  // walk reads them 16 bytes at a time.
+  // walk reads them 16 bytes at a time. Up to 16 outputs a 4-byte copy brings two rows or more, which keeps up with the walk.
   const int jp = (g.J + 3) & ~3;
-  const bool pad = own && jp != g.J && (ring_items > 8L * li.num_sms || g.I >= 200) && (long long)(g.I + 1) * jp <= INT_MAX;
+  const bool pad = own && jp != g.J && (ring_items > 8L * li.num_sms || (g.I >= 200 && g.J > 16)) && (long long)(g.I + 1) * jp <= INT_MAX;
   const float* const w_in = w;
   float* const w_padded = reinterpret_cast<float*>(static_cast<unsigned char*>(ws) + padded_weights_at(g_in));
   if (pad) {

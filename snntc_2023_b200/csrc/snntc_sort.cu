@@ -108,7 +108,7 @@ snn_bucket_sort_kernel(const Geometry g, const float* x, WalkEntry* __restrict__
   chain_wait();
   chain_next();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned tmp[33];
+  __shared__ unsigned tmp[33], tmp_max[TPR > 32 ? TPR / 32 : 1];
   constexpr int kMostBig = TPR == 32 ? 8 : 256;      // at most I / 129 buckets hold more than 128 keys
   __shared__ int big_count[TPR == 32 ? 8 : 1], big_list[TPR == 32 ? 8 : 1][kMostBig];
   const int I = g.I;
@@ -193,19 +193,10 @@ snn_bucket_sort_kernel(const Geometry g, const float* x, WalkEntry* __restrict__
     kmax = __reduce_max_sync(0xffffffffu, kmax);
     if constexpr (TPR > 32) {
       __syncthreads();
-      if ((t & 31) == 0) tmp[t >> 5] = kmin;
+      if ((t & 31) == 0) { tmp[t >> 5] = kmin; tmp_max[t >> 5] = kmax; }
       __syncthreads();
-      uint32_t lo = kNone;
 #pragma unroll
-      for (int k = 0; k < TPR / 32; ++k) lo = min(lo, tmp[k]);
-      __syncthreads();
-      if ((t & 31) == 0) tmp[t >> 5] = kmax;
-      __syncthreads();
-      uint32_t hi = 0u;
-#pragma unroll
-      for (int k = 0; k < TPR / 32; ++k) hi = max(hi, tmp[k]);
-      kmin = lo;
-      kmax = hi;
+      for (int k = 0; k < TPR / 32; ++k) { kmin = min(kmin, tmp[k]); kmax = max(kmax, tmp_max[k]); }
     }
     // bucket of a key: (key - kmin) >> shift < nb
     const int bits = kmax > kmin ? 32 - __clz(kmax - kmin) : 0;
@@ -323,6 +314,12 @@ int launch_row_sort(const Geometry& g, const float* x, WalkEntry* lists, int* nv
   if (g.I > 32768) return E_UNSUPPORTED;
   int lg = 5;
   while ((1 << lg) * 2 < g.I && lg < 13) ++lg;
+  if (g.R <= li.num_sms && g.I <= 4096) {          // a CTA per SM at most: the fewest keys one after the other
+    if (g.I <= 512) return launch<128, 4>(g, x, lists, nvalid, istride, lg < 7 ? 7 : lg, li, s);
+    if (g.I <= 1024) return launch<256, 4>(g, x, lists, nvalid, istride, lg < 8 ? 8 : lg, li, s);
+    if (g.I <= 2048) return launch<512, 4>(g, x, lists, nvalid, istride, lg < 9 ? 9 : lg, li, s);
+    return launch<1024, 4>(g, x, lists, nvalid, istride, lg < 10 ? 10 : lg, li, s);
+  }
   if (g.I <= 1024) {
     if (g.R >= 16 * li.num_sms && (g.is_conv || g.I <= 512)) return launch<32, 0>(g, x, lists, nvalid, istride, lg, li, s);
     return launch<128, 8>(g, x, lists, nvalid, istride, lg < 7 ? 7 : lg, li, s);
