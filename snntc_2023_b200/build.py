@@ -29,7 +29,7 @@ SOURCES = ["snntc_forward.cu", "snntc_sort.cu", "snntc_walk_ring.cu", "snntc_wal
 NATIVE = os.path.join(HERE, "_native" + sysconfig.get_config_var("EXT_SUFFIX"))
 NATIVE_SOURCE = os.path.join(CSRC, "snntc_torch.cpp")
 API_SOURCE = "snntc_api.cu"   # the only file that reads SNNTC_MEASURE
-HEADERS = [os.path.join(CSRC, "snntc_common.cuh"), os.path.join(CSRC, "snntc_merge.cuh"), os.path.join(CSRC, "snntc_walk.cuh"),
+HEADERS = [os.path.join(CSRC, "snntc_common.cuh"), os.path.join(CSRC, "snntc_bound.cuh"), os.path.join(CSRC, "snntc_merge.cuh"), os.path.join(CSRC, "snntc_walk.cuh"),
            os.path.join(CSRC, "snntc_launch.cuh"), os.path.join(CSRC, "snntc_ptx.cuh"),
            os.path.join(HERE, "..", "include", "snntc_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

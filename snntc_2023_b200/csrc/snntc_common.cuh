@@ -28,7 +28,7 @@ struct Geometry {
   // inference only, may be null: I+2 counters. khist[k] += 1 for every output that fired after consuming k inputs
   // (the bias input is not counted), khist[I+1] += 1 for every output that did not fire.
   int* khist;
-  // forward only, set by launch_forward: wbound_n (<= 32) floats whose sum is an upper bound on sum_i |w_ij| for
+  // forward only, set by launch_forward: wbound_n (<= 64) floats whose sum is an upper bound on sum_i |w_ij| for
   // every output j (the walk derives from it how close to zero its sign test must hand over to the reference's
   // rounded comparisons)
   const float* wbound;
@@ -98,6 +98,15 @@ unsigned long long walk_copy_timeouts();
 int launch_forward(const Geometry& g, const float* x, const float* w, float* out, void* ws, size_t ws_bytes,
                    const LaunchInfo& li, const Options& opt, cudaStream_t s);
 
+// The walks' bound on the weight sums (snntc_bound.cuh): the first `ctas` CTAs of the kernel that a list builder launches first form it.
+struct WeightBound {
+  const float* w;
+  int rows, J, Jp;        // weight rows (bias row included), their length, the length of the padded copy's rows
+  float* bound;           // one partial sum per CTA
+  float* padded;          // null: no padded copy
+  int ctas;               // 0: no bound wanted
+};
+
 // Sorted lists of a 3x3 (any Kh x Kw up to 3x3 here), stride-1 convolution by per-pixel sorting and two levels of
 // merging (snntc_lists.cu). merge_lists_supported says whether the geometry qualifies, merge_lists_shape_ok the same
 // without looking at the strides (what a workspace query knows); merge_lists_bytes is the scratch it needs beyond
@@ -107,7 +116,7 @@ bool merge_lists_supported(const Geometry& g);
 size_t merge_lists_bytes(const Geometry& g);
 // split_log2: pieces per merge as a power of two (0 .. 5), -1 = chosen from the number of merges
 int launch_merge_lists(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride,
-                       void* scratch, int split_log2, const LaunchInfo& li, cudaStream_t s);
+                       void* scratch, int split_log2, const WeightBound& wb, const LaunchInfo& li, cudaStream_t s);
 
 // The walk with one output per lane and weight rows copied ahead into shared memory (snntc_walk_ring.cu); any shape.
 int launch_walk_ring(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
@@ -120,12 +129,12 @@ int launch_walk_rows(const Geometry& g, const WalkEntry* lists, const int* nvali
                      bool resident, const LaunchInfo& li, cudaStream_t s);
 
 // Sorted lists of everything else by a bucket sort per row (snntc_sort.cu).
-int launch_row_sort(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride, const LaunchInfo& li,
-                    cudaStream_t s);
+int launch_row_sort(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride, const WeightBound& wb,
+                    const LaunchInfo& li, cudaStream_t s);
 
 // Sorted lists of rows of at most 64 inputs by a sorting network in registers, one warp per row (snntc_lists.cu).
 bool small_rows_supported(const Geometry& g);
-int launch_small_rows(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride,
+int launch_small_rows(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride, const WeightBound& wb,
                       const LaunchInfo& li, cudaStream_t s);
 
 // ---- backward --------------------------------------------------------------------------------

@@ -17,7 +17,6 @@
 #include "snntc_common.cuh"
 #include "snntc_walk.cuh"
 
-#include <cooperative_groups.h>
 #include <limits.h>
 #include <math.h>
 #include <math_constants.h>
@@ -53,64 +52,10 @@ __device__ __forceinline__ int uniform_warp_index() { return __shfl_sync(0xfffff
 __device__ __forceinline__ float walk_tolerance_base(const Geometry& g) {
   const int lane = threadIdx.x & 31;
   float b = lane < g.wbound_n ? ld_plain(g.wbound + lane) : 0.f;
+  if (lane + 32 < g.wbound_n) b += ld_plain(g.wbound + lane + 32);
 #pragma unroll
   for (int d = 16; d >= 1; d >>= 1) b += __shfl_xor_sync(0xffffffffu, b, d);
   return 4.76837158203125e-7f * (fabsf(g.theta) + b) * 1.0001f;   // (a little slack for the rounding of the sums)
-}
-
-// bound[cluster] = sum over the weight rows of this cluster's eight CTAs of max_j |w_ij|: summed over the clusters an upper
-// bound on every column's sum of magnitudes. rows = I + bias row; CTA c takes rows [c * rows_per_cta, (c + 1) * rows_per_cta).
-// `padded` (may be null): receives the weights with rows of Jp >= J floats, zeros behind column J.
-// Bound by memory: up to 256 CTAs, 16 bytes per lane and load (32 CTAs read the 103 MB of a 25 088 x 1024 layer in 300 us).
-constexpr int kBoundClusters = 32;
-constexpr int kBoundCtas = 8 * kBoundClusters;
-__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256)
-snn_wbound_kernel(const float* w, int rows, int J, int rows_per_cta, float* __restrict__ bound,
-                  float* __restrict__ padded, int Jp) {
-  chain_wait();
-  chain_next();
-  __shared__ float part[9];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r0 = blockIdx.x * rows_per_cta;
-  const bool v4 = padded == nullptr && (J & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
-  float acc = 0.f;                                     // lane 0: sum of the row maxima of this warp's rows
-  for (int r = r0 + warp; r < min(rows, r0 + rows_per_cta); r += 8) {
-    const float* wr = w + (size_t)r * J;
-    float m = 0.f;
-    if (v4) {
-#pragma unroll 4
-      for (int j = 4 * lane; j < J; j += 128) {
-        const float4 v = ld_plain(reinterpret_cast<const float4*>(wr + j));
-        m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
-      }
-    } else {
-      for (int j = lane; j < Jp; j += 32) {
-        const float v = j < J ? ld_plain(wr + j) : 0.f;
-        m = fmaxf(m, fabsf(v));
-        if (padded != nullptr) padded[(size_t)r * Jp + j] = v;
-      }
-    }
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-    acc += m;
-  }
-  if (lane == 0) part[warp] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) t += part[k];
-    part[8] = t;
-  }
-  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-  cl.sync();
-  if (threadIdx.x == 0 && cl.block_rank() == 0) {
-    float t = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) t += *cl.map_shared_rank(part + 8, k);
-    bound[blockIdx.x / 8] = t;
-  }
-  cl.sync();                                           // no CTA leaves while its sum may still be read
 }
 
 // One warp walks one row for 32*JPT outputs. Let q_k = ysum - x_k*wsum be taken just before input k is
@@ -536,7 +481,7 @@ snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nva
 int key_stride(const Geometry& g) { return (g.I + 3) & ~3; }  // a multiple of four entries: rows of keys start 32-byte aligned
 
 size_t keys_bytes(const Geometry& g) { return (size_t)g.R * key_stride(g) * sizeof(u64); }
-// list lengths, then 256 bytes that hold the weight bound of the walk (up to 32 partial sums)
+// list lengths, then 256 bytes that hold the weight bound of the walk (up to 64 partial sums)
 size_t nvalid_only_bytes(const Geometry& g) { return ((size_t)g.R * sizeof(int) + 255) & ~(size_t)255; }
 size_t nvalid_bytes(const Geometry& g) { return nvalid_only_bytes(g) + 256; }
 
@@ -698,14 +643,12 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     // global memory is ahead too: 65 536 of 900 x 64 649, 672)
     if (g.jout == 64 && g.I >= 64 && g.R >= 32768) rows = false;
   }
-  if ((fparts & 2) && (!ring || pad)) {   // the walk's bound on the weight sums (see walk_tolerance_base)
-    const int rows_w = g.I + g.has_bias;
-    int per = (rows_w + kBoundCtas - 1) / kBoundCtas;
-    per = (per + 7) & ~7;                                // whole rounds of the CTA's eight warps
-    g.wbound_n = (rows_w + 8 * per - 1) / (8 * per);     // clusters
-    (void)launch_chained(snn_wbound_kernel, 8 * g.wbound_n, 256, 0, s, 0, w_in, rows_w, g.jout, per, wbound, pad ? w_padded : nullptr, g.J);
-    count_launch();
-    if (cudaGetLastError() != cudaSuccess) return E_CUDA;
+  // the walk's bound on the weight sums (see walk_tolerance_base), by up to 64 CTAs of 8192 weights and more beside the lists
+  WeightBound wb = {w_in, g.I + g.has_bias, g.jout, g.J, wbound, pad ? w_padded : nullptr, 0};
+  if (!ring || pad) {
+    const long long n = (long long)wb.rows * g.J;
+    wb.ctas = (int)(n < 64 * 8192 ? (n + 8191) / 8192 : 64);
+    g.wbound_n = wb.ctas;
   }
   // Variants of the walk from global memory: 1 = output pairs in 64-bit registers, 64 outputs per warp; 3 = four consecutive outputs
   // per lane, 128 per warp; 2 = outputs lane + 32*m (odd fan-out, weights that are not even 8-byte aligned). More outputs per warp
@@ -745,21 +688,21 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
 
   if (use_merge_lists(g, opt, li)) {
     if (fparts & 1) {
-      const int rc = launch_merge_lists(g, x, keys_g, nvalid_g, istride, merge_scratch, (opt.list_builder >> 2) - 1, li, s);
+      const int rc = launch_merge_lists(g, x, keys_g, nvalid_g, istride, merge_scratch, (opt.list_builder >> 2) - 1, wb, li, s);
       if (rc != OK) return rc;
     }
     return walk();
   }
   if (use_small_rows(g, opt)) {
     if (fparts & 1) {
-      const int rc = launch_small_rows(g, x, keys_g, nvalid_g, istride, li, s);
+      const int rc = launch_small_rows(g, x, keys_g, nvalid_g, istride, wb, li, s);
       if (rc != OK) return rc;
     }
     return walk();
   }
 
   if (fparts & 1) {
-    const int rc = launch_row_sort(g, x, keys_g, nvalid_g, istride, li, s);
+    const int rc = launch_row_sort(g, x, keys_g, nvalid_g, istride, wb, li, s);
     if (rc != OK) return rc;
   }
   return walk();

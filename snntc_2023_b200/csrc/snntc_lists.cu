@@ -18,6 +18,7 @@
 // the merges read and write 32 bytes (four entries) at a time.
 // The order among equal input values differs from a per-field sort's; no output can spike between two equal
 // inputs, so the walk's result does not depend on it.
+#include "snntc_bound.cuh"
 #include "snntc_common.cuh"
 #include "snntc_merge.cuh"
 
@@ -109,13 +110,14 @@ __device__ __forceinline__ void sort_and_write_run(u64 (&v)[EPL], int n, int lan
 template <int EPL>
 __global__ void __launch_bounds__(kPixelWarps * 32)
 snn_pixel_runs_kernel(const float* x, int npix, int C, int J, float maxcomp,
-                      WalkEntry* __restrict__ runs, int* __restrict__ counts, int stride) {
+                      WalkEntry* __restrict__ runs, int* __restrict__ counts, int stride, const WeightBound wb) {
   chain_wait();
   chain_next();
+  if ((int)blockIdx.x < wb.ctas) return weight_bound(wb, blockIdx.x);
   __shared__ u64 compact[kPixelWarps][EPL >= 2 ? 16 * EPL : 1];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  for (int p = blockIdx.x * kPixelWarps + warp; p < npix; p += gridDim.x * kPixelWarps) {
+  for (int p = (blockIdx.x - wb.ctas) * kPixelWarps + warp; p < npix; p += (gridDim.x - wb.ctas) * kPixelWarps) {
     const float* xp = x + (size_t)p * C;
     u64 v[EPL];
     int n = 0;
@@ -144,9 +146,10 @@ snn_pixel_runs_kernel(const float* x, int npix, int C, int J, float maxcomp,
 template <int EPL>
 __global__ void __launch_bounds__(kPixelWarps * 32)
 snn_small_rows_kernel(const Geometry g, const float* x, WalkEntry* __restrict__ lists,
-                      int* __restrict__ nvalid, int istride) {
+                      int* __restrict__ nvalid, int istride, const WeightBound wb) {
   chain_wait();
   chain_next();
+  if ((int)blockIdx.x < wb.ctas) return weight_bound(wb, blockIdx.x);
   __shared__ int tap_off[32 * EPL];
   __shared__ unsigned short tap_khw[32 * EPL];
   const int I = g.I;
@@ -168,7 +171,7 @@ snn_small_rows_kernel(const Geometry g, const float* x, WalkEntry* __restrict__ 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const float maxcomp = g.maxv - 0.1f;
-  for (int r = blockIdx.x * kPixelWarps + warp; r < g.R; r += gridDim.x * kPixelWarps) {
+  for (int r = (blockIdx.x - wb.ctas) * kPixelWarps + warp; r < g.R; r += (gridDim.x - wb.ctas) * kPixelWarps) {
     const float* xr = x + (size_t)r * I;
     int h0 = 0, w0 = 0;
     if (g.is_conv) {
@@ -391,7 +394,7 @@ int merge_split_log2(int items, const LaunchInfo& li) {
 }
 
 int launch_merge_lists(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride,
-                       void* scratch, int split_log2, const LaunchInfo& li, cudaStream_t s) {
+                       void* scratch, int split_log2, const WeightBound& wb, const LaunchInfo& li, cudaStream_t s) {
   const MergeScratch m = merge_scratch(g);
   unsigned char* base = static_cast<unsigned char*>(scratch);
   WalkEntry* pix = reinterpret_cast<WalkEntry*>(base + m.pix);
@@ -406,11 +409,11 @@ int launch_merge_lists(const Geometry& g, const float* x, WalkEntry* lists, int*
   const long cap = (long)li.num_sms * 8;
   if (grid > cap) grid = cap;
   const int epl = (g.C + 31) / 32;
-  if (epl <= 1) (void)launch_chained(snn_pixel_runs_kernel<1>, (int)grid, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
-  else if (epl <= 2) (void)launch_chained(snn_pixel_runs_kernel<2>, (int)grid, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
-  else if (epl <= 4) (void)launch_chained(snn_pixel_runs_kernel<4>, (int)grid, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
-  else if (epl <= 8) (void)launch_chained(snn_pixel_runs_kernel<8>, (int)grid, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
-  else (void)launch_chained(snn_pixel_runs_kernel<16>, (int)grid, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps);
+  if (epl <= 1) (void)launch_chained(snn_pixel_runs_kernel<1>, (int)grid + wb.ctas, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps, wb);
+  else if (epl <= 2) (void)launch_chained(snn_pixel_runs_kernel<2>, (int)grid + wb.ctas, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps, wb);
+  else if (epl <= 4) (void)launch_chained(snn_pixel_runs_kernel<4>, (int)grid + wb.ctas, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps, wb);
+  else if (epl <= 8) (void)launch_chained(snn_pixel_runs_kernel<8>, (int)grid + wb.ctas, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps, wb);
+  else (void)launch_chained(snn_pixel_runs_kernel<16>, (int)grid + wb.ctas, kPixelWarps * 32, 0, s, 0, x, npix, g.C, g.J, maxcomp, pix, pix_n, ps, wb);
   count_launch();
   if (cudaGetLastError() != cudaSuccess) return E_CUDA;
 
@@ -442,13 +445,13 @@ bool small_rows_supported(const Geometry& g) {
   return true;
 }
 
-int launch_small_rows(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride,
+int launch_small_rows(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride, const WeightBound& wb,
                       const LaunchInfo& li, cudaStream_t s) {
   long grid = ((long)g.R + kPixelWarps - 1) / kPixelWarps;
   const long cap = (long)li.num_sms * 8;
   if (grid > cap) grid = cap;
-  if (g.I <= 32) (void)launch_chained(snn_small_rows_kernel<1>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride);
-  else (void)launch_chained(snn_small_rows_kernel<2>, (int)grid, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride);
+  if (g.I <= 32) (void)launch_chained(snn_small_rows_kernel<1>, (int)grid + wb.ctas, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride, wb);
+  else (void)launch_chained(snn_small_rows_kernel<2>, (int)grid + wb.ctas, kPixelWarps * 32, 0, s, 0, g, x, lists, nvalid, istride, wb);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }

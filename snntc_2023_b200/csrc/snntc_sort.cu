@@ -12,6 +12,7 @@
 // costs about a third of the instructions, and a row is shared by up to 1024 threads where there are few of them.
 // Measured (B200, half of the inputs spiking, before -> now): 784 inputs at 32 samples 19 -> 6 us, at 1024: 24 -> 7; 4096 at 32:
 // 65 -> 8; 25 088 at 64: 376 -> 31; 17 020 fields of 5x5x20 inputs 106 -> 58; 3136 fields of 3x3x128, stride 2: 60 -> 36.
+#include "snntc_bound.cuh"
 #include "snntc_common.cuh"
 
 namespace snntc {
@@ -104,9 +105,10 @@ __host__ __device__ __forceinline__ size_t row_bytes(int I, int nb_log2) {
 template <int TPR, int EPT>
 __global__ void __launch_bounds__(TPR == 32 ? 256 : TPR)
 snn_bucket_sort_kernel(const Geometry g, const float* x, WalkEntry* __restrict__ lists, int* __restrict__ nvalid,
-                       int istride, int nb_log2, int table) {
+                       int istride, int nb_log2, int table, const WeightBound wb) {
   chain_wait();
   chain_next();
+  if ((int)blockIdx.x < wb.ctas) return weight_bound(wb, blockIdx.x);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned tmp[33], tmp_max[TPR > 32 ? TPR / 32 : 1];
   constexpr int kMostBig = TPR == 32 ? 8 : 256;      // at most I / 129 buckets hold more than 128 keys
@@ -134,7 +136,7 @@ snn_bucket_sort_kernel(const Geometry g, const float* x, WalkEntry* __restrict__
   }
   const float maxcomp = g.maxv - 0.1f;
 
-  for (int r = blockIdx.x * groups + group; r < g.R; r += gridDim.x * groups) {
+  for (int r = (blockIdx.x - wb.ctas) * groups + group; r < g.R; r += (gridDim.x - wb.ctas) * groups) {
     const float* xr = x + (size_t)r * I;
     int h0 = 0, w0 = 0;
     if (g.is_conv) {
@@ -278,8 +280,8 @@ snn_bucket_sort_kernel(const Geometry g, const float* x, WalkEntry* __restrict__
 }
 
 template <int TPR, int EPT>
-int launch(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride, int nb_log2, const LaunchInfo& li,
-           cudaStream_t s) {
+int launch(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride, int nb_log2, const WeightBound& wb,
+           const LaunchInfo& li, cudaStream_t s) {
   const size_t row = row_bytes<TPR>(g.I, nb_log2);
   size_t table = g.is_conv && g.Kh <= 255 && g.Kw <= 255 ? tap_table_bytes(g) : 0;
   const size_t budget = (size_t)li.max_smem_optin - 12 * 1024;              // (static arrays, the per-CTA reserve)
@@ -298,7 +300,7 @@ int launch(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int
   if (resident < 1) resident = 1;
   long grid = ((long)g.R + rows_per_cta - 1) / rows_per_cta;
   if (grid > resident * li.num_sms) grid = resident * li.num_sms;
-  (void)launch_chained(snn_bucket_sort_kernel<TPR, EPT>, (int)grid, threads, smem, s, 0, g, x, lists, nvalid, istride, nb_log2, table > 0);
+  (void)launch_chained(snn_bucket_sort_kernel<TPR, EPT>, (int)grid + wb.ctas, threads, smem, s, 0, g, x, lists, nvalid, istride, nb_log2, table > 0, wb);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -309,25 +311,25 @@ int launch(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int
 // receptive fields up to 1024 (the tap arithmetic then hides what a warp loses on longer rows: 784 inputs at 10 000 rows are
 // 63 us by warps and 57 by CTAs when dense, 80 against 88 as fields). Else a CTA per row of as many threads as leave a
 // thread eight keys (32 in the longest rows). Buckets: about one per two inputs, at least one per thread.
-int launch_row_sort(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride, const LaunchInfo& li,
-                    cudaStream_t s) {
+int launch_row_sort(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride, const WeightBound& wb,
+                    const LaunchInfo& li, cudaStream_t s) {
   if (g.I > 32768) return E_UNSUPPORTED;
   int lg = 5;
   while ((1 << lg) * 2 < g.I && lg < 13) ++lg;
   if (g.R <= li.num_sms && g.I <= 4096) {          // a CTA per SM at most: the fewest keys one after the other
-    if (g.I <= 512) return launch<128, 4>(g, x, lists, nvalid, istride, lg < 7 ? 7 : lg, li, s);
-    if (g.I <= 1024) return launch<256, 4>(g, x, lists, nvalid, istride, lg < 8 ? 8 : lg, li, s);
-    if (g.I <= 2048) return launch<512, 4>(g, x, lists, nvalid, istride, lg < 9 ? 9 : lg, li, s);
-    return launch<1024, 4>(g, x, lists, nvalid, istride, lg < 10 ? 10 : lg, li, s);
+    if (g.I <= 512) return launch<128, 4>(g, x, lists, nvalid, istride, lg < 7 ? 7 : lg, wb, li, s);
+    if (g.I <= 1024) return launch<256, 4>(g, x, lists, nvalid, istride, lg < 8 ? 8 : lg, wb, li, s);
+    if (g.I <= 2048) return launch<512, 4>(g, x, lists, nvalid, istride, lg < 9 ? 9 : lg, wb, li, s);
+    return launch<1024, 4>(g, x, lists, nvalid, istride, lg < 10 ? 10 : lg, wb, li, s);
   }
   if (g.I <= 1024) {
-    if (g.R >= 16 * li.num_sms && (g.is_conv || g.I <= 512)) return launch<32, 0>(g, x, lists, nvalid, istride, lg, li, s);
-    return launch<128, 8>(g, x, lists, nvalid, istride, lg < 7 ? 7 : lg, li, s);
+    if (g.R >= 16 * li.num_sms && (g.is_conv || g.I <= 512)) return launch<32, 0>(g, x, lists, nvalid, istride, lg, wb, li, s);
+    return launch<128, 8>(g, x, lists, nvalid, istride, lg < 7 ? 7 : lg, wb, li, s);
   }
-  if (g.I <= 2048) return launch<256, 8>(g, x, lists, nvalid, istride, lg < 8 ? 8 : lg, li, s);
-  if (g.I <= 4096) return launch<512, 8>(g, x, lists, nvalid, istride, lg < 9 ? 9 : lg, li, s);
-  if (g.I <= 8192) return launch<1024, 8>(g, x, lists, nvalid, istride, lg < 10 ? 10 : lg, li, s);
-  return launch<1024, 32>(g, x, lists, nvalid, istride, lg, li, s);
+  if (g.I <= 2048) return launch<256, 8>(g, x, lists, nvalid, istride, lg < 8 ? 8 : lg, wb, li, s);
+  if (g.I <= 4096) return launch<512, 8>(g, x, lists, nvalid, istride, lg < 9 ? 9 : lg, wb, li, s);
+  if (g.I <= 8192) return launch<1024, 8>(g, x, lists, nvalid, istride, lg < 10 ? 10 : lg, wb, li, s);
+  return launch<1024, 32>(g, x, lists, nvalid, istride, lg, wb, li, s);
 }
 
 }  // namespace snntc

@@ -58,6 +58,7 @@ snn_walk_rows_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
   float tolbase;                                  // see walk_tolerance_base in snntc_forward.cu
   {
     float b = lane < g.wbound_n ? ld_plain(g.wbound + lane) : 0.f;
+    if (lane + 32 < g.wbound_n) b += ld_plain(g.wbound + lane + 32);
 #pragma unroll
     for (int d = 16; d >= 1; d >>= 1) b += __shfl_xor_sync(0xffffffffu, b, d);
     tolbase = 4.76837158203125e-7f * (fabsf(g.theta) + b) * 1.0001f;
