@@ -92,7 +92,8 @@ __global__ void snn_weight_transpose_kernel(const float* w, float* __restrict__ 
 // 128 -> 256 72 instead of 77.
 constexpr int kStage = 256;   // staged list entries per warp and round
 
-template <int CPL, int LPP>
+// ONE: a 1x1 window, where there is nothing to look up between the taps (201 images of 23x33, 256 -> 16: 219 us without, 176 so).
+template <int CPL, int LPP, bool ONE>
 __global__ void __launch_bounds__(kThreads)
 snn_dx_sparse_kernel(const Geometry g, const float* x, const float* wt,
                      const uint4* list, const int* count, float* __restrict__ dx,
@@ -102,7 +103,8 @@ snn_dx_sparse_kernel(const Geometry g, const float* x, const float* wt,
   if (gate.nz != nullptr && ld_plain(gate.nz) > gate.threshold) return;
   constexpr int PPW = 32 / LPP;                       // pixels per warp
   constexpr int SB = kStage / PPW;                    // staged entries per pixel and round
-  constexpr int UN = CPL <= 8 ? 4 : 2;                // entries whose weight reads are in flight together
+  constexpr int UN = CPL <= 8 && !(ONE && CPL == 8) ? 4 : 2;   // entries whose weight reads are in flight together
+  static_assert(SB % (4 * LPP) == 0 && LPP % UN == 0, "groups of entries are staged whole");
   __shared__ uint4 stage_all[(kThreads / 32) * kStage];
   const int lane = threadIdx.x & 31;
   const int sub = lane / LPP;                         // which of the warp's pixels
@@ -112,7 +114,7 @@ snn_dx_sparse_kernel(const Geometry g, const float* x, const float* wt,
   const int C = g.C, J = g.J;
   const int P = g.B * g.H * g.W;
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  const int taps = g.Kh * g.Kw;
+  const int taps = ONE ? 1 : g.Kh * g.Kw;
   // C % 4 == 0 and CPL % 4 == 0: a lane's float4s are all in or all out; one that is out reads the row's first channels, for inputs of
   // +inf that no output reaches
   unsigned coff[CPL / 4];
@@ -144,7 +146,7 @@ snn_dx_sparse_kernel(const Geometry g, const float* x, const float* wt,
     for (int tap0 = 0; tap0 < taps; tap0 += LPP) {    // (the terms keep their order: tap-major, j ascending)
       // ---- this lane's tap: the receptive field that reads the pixel through (kh, kw), if there is one
       int n = 0, r = 0;
-      const int tap = tap0 + gl;
+      const int tap = ONE ? 0 : tap0 + gl;
       {
         const int kh = tap / g.Kw, kw = tap - kh * g.Kw;
         const int hh = ph + g.pad_top - kh, ww = pwid + g.pad_left - kw;
@@ -160,38 +162,59 @@ snn_dx_sparse_kernel(const Geometry g, const float* x, const float* wt,
         }
       }
       int end = n;                                    // entries up to and with this lane's tap
+      if constexpr (!ONE) {
 #pragma unroll
-      for (int d = 1; d < LPP; d <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, end, d, LPP);
-        if (gl >= d) end += v;
+        for (int d = 1; d < LPP; d <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, end, d, LPP);
+          if (gl >= d) end += v;
+        }
       }
-      const int total = __shfl_sync(0xffffffffu, end, LPP - 1, LPP);
+      const int total = ONE ? n : __shfl_sync(0xffffffffu, end, LPP - 1, LPP);
       const int most = __reduce_max_sync(0xffffffffu, total);
       for (int first = 0; first < most; first += SB) {
         const int nmax = min(most - first, SB);
         // ---- stage entries first .. first + nmax - 1 of this pixel
+        if constexpr (ONE) {
+          constexpr int Q = LPP >= 16 ? 1 : 4;
 #pragma unroll 1
-        for (int i = 0; i < nmax; i += 4 * LPP) {
-          uint4 en[4];
-          unsigned at[4];
+          for (int i = 0; i < nmax; i += Q * LPP) {
+            uint4 en[Q];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int e = first + i + q * LPP + gl;
-            int t = 0;                                // taps whose entries all lie in front of e
+            for (int q = 0; q < Q; ++q) {
+              const int e = first + i + q * LPP + gl;
+              en[q] = make_uint4(0xff800000u, 0u, 0u, 0u);
+              if (e < total) en[q] = ld_plain(list + (size_t)r * J + e);
+            }
 #pragma unroll
-            for (int d = LPP / 2; d >= 1; d >>= 1)
-              if (__shfl_sync(0xffffffffu, end, t + d - 1, LPP) <= e) t += d;
-            const int start = __shfl_sync(0xffffffffu, end - n, t, LPP), row = __shfl_sync(0xffffffffu, r, t, LPP);
-            at[q] = (unsigned)(tap0 + t) * (unsigned)J;
-            en[q] = make_uint4(0xff800000u, 0u, 0u, 0u);   // behind the end: y = -inf, u = 0
-            if (e < total) en[q] = ld_plain(list + (size_t)row * J + (e - start));
-            else at[q] = 0u;
+            for (int q = 0; q < Q; ++q) {
+              en[q].z *= (unsigned)C;
+              stage[i + q * LPP + gl] = en[q];
+            }
           }
+        } else {
+#pragma unroll 1
+          for (int i = 0; i < nmax; i += 4 * LPP) {
+            uint4 en[4];
+            unsigned at[4];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int e = i + q * LPP + gl;
-            en[q].z = (at[q] + en[q].z) * (unsigned)C;
-            if (SB % (4 * LPP) == 0 || e < SB) stage[e] = en[q];
+            for (int q = 0; q < 4; ++q) {
+              const int e = first + i + q * LPP + gl;
+              int t = 0;                                // taps whose entries all lie in front of e
+#pragma unroll
+              for (int d = LPP / 2; d >= 1; d >>= 1)
+                if (__shfl_sync(0xffffffffu, end, t + d - 1, LPP) <= e) t += d;
+              const int start = __shfl_sync(0xffffffffu, end - n, t, LPP), row = __shfl_sync(0xffffffffu, r, t, LPP);
+              at[q] = (unsigned)(tap0 + t) * (unsigned)J;
+              en[q] = make_uint4(0xff800000u, 0u, 0u, 0u);   // behind the end: y = -inf, u = 0
+              if (e < total) en[q] = ld_plain(list + (size_t)row * J + (e - start));
+              else at[q] = 0u;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int e = i + q * LPP + gl;
+              en[q].z = (at[q] + en[q].z) * (unsigned)C;
+              stage[e] = en[q];
+            }
           }
         }
         __syncwarp();
@@ -244,7 +267,8 @@ int launch_one(const Geometry& g, const float* x, const float* wt, const uint4* 
   if (grid > cap) grid = cap;
   // (in plain order: the transposed weights are read through the read-only path -- 256 channels: 64 us so, 90 with ordinary loads;
   // 512: 246 and 268)
-  snn_dx_sparse_kernel<CPL, LPP><<<(int)grid, kThreads, 0, s>>>(g, x, wt, list, count, dx, gate);
+  if (g.Kh * g.Kw == 1) snn_dx_sparse_kernel<CPL, LPP, true><<<(int)grid, kThreads, 0, s>>>(g, x, wt, list, count, dx, gate);
+  else snn_dx_sparse_kernel<CPL, LPP, false><<<(int)grid, kThreads, 0, s>>>(g, x, wt, list, count, dx, gate);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
