@@ -7,7 +7,7 @@
 // What bounds a dense layer at these sizes is not arithmetic but how little of the GPU a call reaches: 256 samples of a
 // 784 -> 400 layer are 52 tiles of 64 x 64 for dX, each reducing 400 outputs one after the other. Here
 //   - the unit of work is a small tile per WARP. dX: 32 x 32 down to 8 x 8 (rows x inputs), the largest that still gives every
-//     SM six warps; the reduction over the outputs is one running sum per element, ascending, as in the other dX kernels.
+//     SM four warps; the reduction over the outputs is one running sum per element, ascending, as in the other dX kernels.
 //     dW: 32 x 32, its rows cut into the slices that plan_dw (snntc_backward.cu) gives the register-tile kernel, a warp per
 //     slice, and the slices added through the distributed shared memory of a cluster in the order snn_dw_reduce_kernel adds
 //     planes. So the sums are the register-tile kernels' bit for bit;
@@ -382,9 +382,10 @@ int launch_dense_bwd(const Geometry& g, const float* uv, const float* x, const f
   }
   const bool vx = (g.I & 3) == 0 && ((uintptr_t)x & 15) == 0;
   const bool vj = (g.J & 3) == 0 && (((uintptr_t)uv | (uintptr_t)out | (uintptr_t)w) & 15) == 0;
-  // the largest dX tile that leaves every SM six warps: a large one reads less per product, with few warps latency counts
+  // the largest dX tile that leaves every SM four warps (beside those of dW): a large one reads less per product, with few warps latency
+  // counts (both gradients, six warps and four, us: 400 x 400 at 1024 samples 62, 58, 784 x 400 at 512 55, 53)
   auto tiles = [&](int m, int n) { return (long)((g.R + m - 1) / m) * ((g.I + n - 1) / n); };
-  const long enough = 6L * li.num_sms;
+  const long enough = 4L * li.num_sms;
   if (!dx || tiles(32, 32) >= enough) return launch_tile<4, 8>(a, p, vx, vj, s);
   if (tiles(16, 32) >= enough) return launch_tile<2, 8>(a, p, vx, vj, s);
   if (tiles(16, 16) >= enough) return launch_tile<2, 4>(a, p, vx, vj, s);
