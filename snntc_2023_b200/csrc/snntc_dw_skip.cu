@@ -26,7 +26,8 @@
 // (each input copied once for twice the outputs), stages queued three ahead, one barrier a stage and one wave of CTAs against 32
 // outputs, two stages, two barriers and eight waves, dW of 131 072 rows of 829 x 128: all outputs that fired 1445 -> 1213 us, 12 %
 // of them 731 -> 506; 65 536 of 325 x 64 at stride 2: 201 -> 146, 135 -> 82. Without VEC, 131 072 of 820 x 128 against the dense
-// tile: 2012 -> 1469, 1998 -> 734.
+// tile: 2012 -> 1469, 1998 -> 734. Channels dealt out to the warps by their activity instead of four neighbours, the sums out through
+// shared memory (whole dW): 200 704 of 148 x 64 284 -> 266, 3136 of 4609 x 512 354 -> 330, 1600 of 3201 x 64, 5x5 stride 2 48 -> 39.
 #include "snntc_common.cuh"
 #include "snntc_ptx.cuh"
 
@@ -66,6 +67,12 @@ snn_dw_skip_kernel(const Geometry g, const float* uv, const float* x,
   float* Xs = reinterpret_cast<float*>(smem_raw);                 // [kDepth][kRS][kTI]
   float* Ys = Xs + kDepth * kRS * kTI;                            // [kDepth][kRS][kJT]
   float* Us = Ys + kDepth * kRS * kJT;                            // [kDepth][kRS][kJT]
+  __shared__ __align__(16) int order[kJT];          // output channels (of this CTA) by warp, four each
+  __shared__ int active[kJT];
+  __shared__ float4 own_all[NW][2][kRS];            // a stage's u and y of each warp's four channels
+  // float of row rl and channel c in a y or u buffer: the 16-byte chunks are swizzled by the row, so that a channel's 16 rows are read
+  // two at a time instead of one after the other
+  auto at_field = [](int rl, int c) { return rl * kJT + (((c >> 2) ^ (rl & 7)) << 2 | (c & 3)); };
   int4* rowinfo = reinterpret_cast<int4*>(Us + kDepth * kRS * kJT);    // [2][kRS]: .x element offset of the top-left pixel, .y its h, .z its w, .w row valid
 
   const int J = g.J, I = g.I, R = g.R;
@@ -159,7 +166,7 @@ snn_dw_skip_kernel(const Geometry g, const float* uv, const float* x,
 #pragma unroll
       for (int e = tid; e < 2 * kRS * kJT; e += kThreads) {
         const int which = e / (kRS * kJT), rl = e / kJT % kRS, jl = e % kJT;
-        float* dst = (which == 0 ? Ys : Us) + (buf * kRS + rl) * kJT + jl;
+        float* dst = (which == 0 ? Ys : Us) + buf * kRS * kJT + at_field(rl, jl);
         if (rb + rl < r_end && j0 + jl < J) cp_async4(dst, (which == 0 ? out : uv) + (size_t)(rb + rl) * J + j0 + jl);
         else *dst = 0.f;
       }
@@ -181,7 +188,7 @@ snn_dw_skip_kernel(const Geometry g, const float* uv, const float* x,
         const int rl = h / (kJT / 4), cq = h - rl * (kJT / 4);
         const int r = rb + rl, j = j0 + 4 * cq;
         const float* base = which == 0 ? out : uv;
-        float* dst = (which == 0 ? Ys : Us) + (buf * kRS + rl) * kJT + 4 * cq;
+        float* dst = (which == 0 ? Ys : Us) + buf * kRS * kJT + at_field(rl, 4 * cq);
         if (r < r_end && j < J) cp_async16(dst, base + (size_t)r * J + j);
         else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);   // no spike value, no gradient
       }
@@ -189,7 +196,7 @@ snn_dw_skip_kernel(const Geometry g, const float* uv, const float* x,
     copies_commit();
   };
 
-  // acc[c][jj][h]: fan-in rows i0 + CW*(lane + 32c) + 2h, +1 (one 64-bit pair), output channel j0 + 4*warp + jj
+  // acc[c][jj][h]: fan-in rows i0 + CW*(lane + 32c) + 2h, +1 (one 64-bit pair), the warp's channel jj
   uint64_t acc[QL][4][CW / 2];
 #pragma unroll
   for (int c = 0; c < QL; ++c)
@@ -198,21 +205,27 @@ snn_dw_skip_kernel(const Geometry g, const float* uv, const float* x,
 #pragma unroll
       for (int h = 0; h < CW / 2; ++h) acc[c][jj][h] = pack2(0.f, 0.f);
 
+  unsigned at01 = 0u, at23 = 0u;                  // where this lane's row of the warp's four channels lies in a buffer
+  const float* const own_from = lane < kRS ? Us : Ys;
   auto reduce_stage = [&](int buf, auto fast_c) {
     constexpr bool FAST = decltype(fast_c)::value;
     const float* xs = Xs + buf * kRS * kTI;
-    // which of the 16 rows carry a gradient for one of this warp's four channels: lane rl looks at row rl, one vote
+    // The warp's four channels of the stage, a row per lane (lanes from 16 on: y), put side by side for the loop below. Which of the 16
+    // rows carry a gradient for one of the four: one vote.
+    float4* own = &own_all[warp][0][0];
     unsigned todo;
     {
-      const float4 uq = *reinterpret_cast<const float4*>(Us + (buf * kRS + (lane & (kRS - 1))) * kJT + 4 * warp);
-      todo = __ballot_sync(0xffffffffu, (uq.x != 0.f) | (uq.y != 0.f) | (uq.z != 0.f) | (uq.w != 0.f)) & ((1u << kRS) - 1u);
+      const float* from = own_from + buf * kRS * kJT;
+      const float4 v = make_float4(from[at01 & 0xffff], from[at01 >> 16], from[at23 & 0xffff], from[at23 >> 16]);
+      todo = __ballot_sync(0xffffffffu, (v.x != 0.f) | (v.y != 0.f) | (v.z != 0.f) | (v.w != 0.f)) & ((1u << kRS) - 1u);
+      if (todo != 0u) own[lane] = v;                       // (every lane is through with the stage before: the vote)
+      __syncwarp();
     }
 #pragma unroll 1
     while (todo != 0u) {
       const int rl = __ffs((int)todo) - 1;
       todo &= todo - 1u;
-      const float4 y4 = *reinterpret_cast<const float4*>(Ys + (buf * kRS + rl) * kJT + 4 * warp);
-      const float4 u4 = *reinterpret_cast<const float4*>(Us + (buf * kRS + rl) * kJT + 4 * warp);
+      const float4 u4 = own[rl], y4 = own[kRS + rl];
       float xr[QL][CW];
 #pragma unroll
       for (int c = 0; c < QL; ++c) {
@@ -252,6 +265,33 @@ snn_dw_skip_kernel(const Geometry g, const float* uv, const float* x,
     issue(d, d & 1, r_begin + d * kRS);        // (rows from r_end on: an empty stage)
   }
   fill_rowinfo((kDepth - 1) & 1, r_begin + (kDepth - 1) * kRS);
+  // Which four channels a warp takes: dealt out in the order of their activity over the stages that are there first, forth and back
+  // (see snn_dw_tma_kernel)
+  copies_wait<0>();
+  __syncthreads();
+  if (tid < kJT) {
+    int n = 0;
+    for (int d = 0; d < kDepth - 1; ++d)
+#pragma unroll
+      for (int rl = 0; rl < kRS; ++rl) n += Us[d * kRS * kJT + at_field(rl, tid)] != 0.f;
+    active[tid] = n;
+  }
+  __syncthreads();
+  if (tid < kJT) {
+    const int n = active[tid];
+    int rank = 0;
+#pragma unroll 8
+    for (int c = 0; c < kJT; ++c) rank += active[c] > n || (active[c] == n && c < tid);
+    const int k = rank / NW, w = rank % NW;
+    order[4 * (k & 1 ? NW - 1 - w : w) + k] = tid;
+  }
+  __syncthreads();
+  {
+    const int4 ch = *reinterpret_cast<const int4*>(order + 4 * warp);
+    const int rl = lane & (kRS - 1);
+    at01 = (unsigned)at_field(rl, ch.x) | (unsigned)at_field(rl, ch.y) << 16;
+    at23 = (unsigned)at_field(rl, ch.z) | (unsigned)at_field(rl, ch.w) << 16;
+  }
   int it = 0;
   for (int rb = r_begin; rb < r_end; rb += kRS, ++it) {
     copies_wait<kDepth - 2>();
@@ -263,29 +303,42 @@ snn_dw_skip_kernel(const Geometry g, const float* uv, const float* x,
   }
   copies_wait<0>();
 
-  float* __restrict__ dst = partial + (size_t)blockIdx.z * Itot * J;
-  const int j = j0 + 4 * warp;
-  if (j < J) {
+  // The sums go out through shared memory, where they are turned so that a row's channels lie together: row (f % CW, f / CW) for fan-in
+  // row f of the tile, lanes on neighbouring rows.
+  __syncthreads();
+  constexpr int kPitch = kJT + 1;
+  static_assert((size_t)kTI * kPitch <= (size_t)kDepth * kRS * (kTI + 2 * kJT), "the tile of sums fits the stages");
+  float* turn = Xs;
+  {
+    const int4 ch = *reinterpret_cast<const int4*>(order + 4 * warp);
+    const int chs[4] = {ch.x, ch.y, ch.z, ch.w};
 #pragma unroll
     for (int c = 0; c < QL; ++c)
 #pragma unroll
-      for (int h = 0; h < CW / 2; ++h) {
-        float v[2][4];
+      for (int h = 0; h < CW / 2; ++h)
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) unpack2(acc[c][jj][h], v[0][jj], v[1][jj]);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i = i0 + CW * (lane + 32 * c) + 2 * h + e;
-          if (i >= Itot) continue;
-          if (VEC || (J & 3) == 0) {
-            *reinterpret_cast<float4*>(dst + (size_t)i * J + j) = make_float4(v[e][0], v[e][1], v[e][2], v[e][3]);
-          } else {
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj)
-              if (j + jj < J) dst[(size_t)i * J + j + jj] = v[e][jj];
-          }
+        for (int jj = 0; jj < 4; ++jj) {
+          float a, b;
+          unpack2(acc[c][jj][h], a, b);
+          turn[((2 * h) * 32 * QL + 32 * c + lane) * kPitch + chs[jj]] = a;
+          turn[((2 * h + 1) * 32 * QL + 32 * c + lane) * kPitch + chs[jj]] = b;
         }
+  }
+  __syncthreads();
+  float* __restrict__ dst = partial + (size_t)blockIdx.z * Itot * J;
+  const int j = j0 + 4 * (tid % NW);
+  if (j < J) {
+    for (int f = tid / NW; f < kTI && i0 + f < Itot; f += 32) {
+      const float* from = turn + ((f % CW) * 32 * QL + f / CW) * kPitch + 4 * (tid % NW);
+      float* to = dst + (size_t)(i0 + f) * J + j;
+      if (VEC || (J & 3) == 0) {
+        *reinterpret_cast<float4*>(to) = make_float4(from[0], from[1], from[2], from[3]);
+      } else {
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj)
+          if (j + jj < J) to[jj] = from[jj];
       }
+    }
   }
 }
 
