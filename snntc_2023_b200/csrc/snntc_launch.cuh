@@ -75,9 +75,10 @@ cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, siz
 }
 
 // Raises the kernel's limit of dynamic shared memory on the current device to at least `bytes`; a call into the runtime only
-// when it grows.
+// when it grows. What every kernel may have anyway (48 KB less its static arrays, which are below 16 KB everywhere) is not looked up.
 template <auto Kernel>
 cudaError_t allow_smem(size_t bytes) {
+  if (bytes <= 32 * 1024) return cudaSuccess;
   constexpr int kDevices = 64;
   static std::atomic<int> have[kDevices];
   static std::mutex mutex;
