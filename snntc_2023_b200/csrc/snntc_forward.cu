@@ -395,8 +395,8 @@ snn_walk_pairs_kernel(const Geometry g, const WalkEntry* keys_g, const int* nval
 }
 
 // ---- the pairs walk with its weights staged in shared memory ---------------------------------------------
-// Where all fan-in rows of 64 outputs fit into one CTA's shared memory ((I + bias) * 256 bytes: up to about 800
-// rows), a persistent CTA of 32 warps copies that slice of the weight matrix in once -- one asynchronous bulk copy
+// Where all fan-in rows of 64 outputs fit into one CTA's shared memory ((I + bias) * 256 bytes beside the lists and the sums of the
+// spikes: up to about 770 rows), a persistent CTA of 32 warps copies that slice of the weight matrix in once -- one asynchronous bulk copy
 // (cp.async.bulk) per weight row, all completing on one mbarrier -- and every step of every walk then reads its
 // weight pair with one shared-memory load instead of a global load through L1. CTA c takes output slice
 // c % (J/64) and every (gridDim.x / (J/64))-th row of that slice.
@@ -536,13 +536,10 @@ int launch_walk2_smemw(const Geometry& g, const WalkEntry* keys_g, const int* nv
 }
 
 // What a walk from global memory takes with n warps to an SM, in microseconds for rows of 500 inputs of which half spike: 32 warps
-// run at once, each full wave of them takes `wave`, the last one first + n * warp. Fitted to 100 to 16 000 rows x fan-outs
-// 68 to 1000 (n = 2 to 3500; within 5 % from n = 8 on). What counts is where two of them cross: at 300 to 4096 inputs, half or all
-// of them spiking, 33 to 70 warps of 64 outputs per SM, pairs took 1.11 times the quads' time on average, in 15 of 180 sizes less (700 rows of
-// 784 -> 512: 128 against 103 us all spiking, 74 against 78 half; 1024 of 784 -> 400: 144 against 126), below 32 the quads
-// (300 rows of 500 -> 400: 29 against 35 us). What the rule cannot know is whether an output never fires, for which a warp walks
-// to the end of its list: with one such output in the layer the pairs lose less of the fan-out to it (2450 of 2305 -> 128: 179
-// against 216 us; with none, or many, 337 against 273).
+// run at once, each full wave of them takes `wave`, the last one first + n * warp. Fitted on the scalar steps; with the packed ones
+// both sides became faster alike, and the choice between pairs and quads was measured again: at 300 to 2304 inputs, half or all of them
+// spiking, 400 to 20 000 rows and fan-outs 70 to 512, 89 sizes, the one it takes is never more than 4 % behind the other. They cross at about
+// 32 warps of 64 outputs per SM (500 rows of 2304 -> 256: 89 us with pairs, 112 with quads, 1200 rows 166, 130).
 struct WalkCost { double wave, first, warp; };
 constexpr WalkCost kCostPairs = {27, 20, 0.6};                                        // 64 outputs per warp
 constexpr WalkCost kCostQuads = {43, 29, 0.8};                                        // 128
