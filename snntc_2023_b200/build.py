@@ -21,7 +21,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libsnntc_b200.so")
 LIB_MEASURE = os.path.join(HERE, "libsnntc_b200_measure.so")
-SOURCES = ["snntc_forward.cu", "snntc_sort.cu", "snntc_walk_ring.cu", "snntc_walk_rows.cu",
+SOURCES = ["snntc_forward.cu", "snntc_sort.cu", "snntc_walk_ring.cu", "snntc_walk_alone.cu", "snntc_walk_rows.cu",
            "snntc_lists.cu", "snntc_backward.cu", "snntc_bwd_dense.cu",
            "snntc_dw_skip.cu", "snntc_dw_tma.cu", "snntc_dx_sparse.cu", "snntc_dx_few.cu",
            "snntc_pool.cu",

@@ -118,6 +118,9 @@ size_t merge_lists_bytes(const Geometry& g);
 int launch_merge_lists(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride,
                        void* scratch, int split_log2, const WeightBound& wb, const LaunchInfo& li, cudaStream_t s);
 
+// The walk of one row per warp that copies its own weight rows ahead (snntc_walk_alone.cu): J <= 32, J % 4 == 0, w 16-byte aligned.
+int launch_walk_alone(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
+                      cudaStream_t s);
 // The walk with one output per lane and weight rows copied ahead into shared memory (snntc_walk_ring.cu); any shape.
 int launch_walk_ring(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
                      const LaunchInfo& li, cudaStream_t s);

@@ -602,11 +602,14 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
 
   const int fparts = opt.forward_parts;
   // The walk that copies its weight rows ahead, up to two waves of its CTAs of 64 outputs (six to an SM; eight items of 32 outputs per
-  // SM for fan-out up to 32, where a copying warp serves a single one, and where the rows have to be copied 4 bytes at a time): with
+  // SM where the rows have to be copied 4 bytes at a time and for fan-out up to 16; one wave, ten items, for fan-out 17 to 32): with
   // few warps on an SM latency is what counts, with many the instructions per output. Against the pairs walk, us: 784 -> 400 200 rows
   // 29, 35, 300 rows 41, 37; 1000 -> 1000 80 rows 33, 43, 120 rows 46, 45; 576 -> 128 1000 rows (13.5 CTAs per SM) 33, 31; 1152 ->
   // 128 700 rows 37, 47, 1500 72, 67; 4096 -> 512 still 172, 199 at 300 rows (16 per SM); 576 -> 32 1000 rows 23, 25, 2000 40, 27;
   // 1500 -> 16 1000 rows 47, 53, 2000 83, 50.
+  // Fan-out 17 to 32 beyond that, up to one wave of it (24 rows per SM): the walk whose warps copy for themselves. Copying warp, each
+  // for itself, pairs walk, us: 2304 -> 32 1200 rows 40, 46, 69, 1500 rows 50, 48, 70, 3500 rows 98, 77, 91, 4500 rows 118, 116, 116;
+  // 576 -> 32 1200 rows 16, 18, 21, 2600 rows 28, 24, 25, 4500 rows 42, 37, 34; 2304 -> 20 2600 rows 75, 65, 81.
   g.jout = g.J;
   const bool own = opt.walk_layout == 0 && opt.walk_outputs == 0;    // the library's own choice
   const long ring_items = (long)g.R * ((g.J + 31) / 32);
@@ -623,13 +626,14 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     g.J = jp;
   }
   const bool copies16 = (g.J & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
-  const bool few = copies16 && g.J > 32 ? (long)g.R * ((g.J + 63) / 64) <= 12L * li.num_sms : ring_items <= 8L * li.num_sms;
+  const bool few = copies16 && g.J > 32 ? (long)g.R * ((g.J + 63) / 64) <= 12L * li.num_sms : ring_items <= (copies16 && g.J > 16 ? 10L : 8L) * li.num_sms;
   const bool ring = (opt.walk_layout & 16) != 0 || (own && few);
+  const bool alone = own && !ring && copies16 && g.J > 16 && g.J <= 32 && ring_items <= 24L * li.num_sms;
   // Several rows per warp for fan-out up to 64, where that leaves enough warps: 5 per SM at eight rows to a warp (fan-out 16;
   // 10 where the weights miss the L1 cache), 11 at four (32), 40 at two (64). With fewer the pairs walk, a warp per row, hides
   // its latencies better. Pairs against rows, us: 576 -> 16 4000 rows 35, 39, 7000 rows 53, 39; 576 -> 32 35, 37 and 54, 43; 147 -> 64 8000
   // rows 25, 27, 14 000 37, 35; 500 -> 64 8000 54, 61, 14 000 85, 85, -> 36 80, 76.
-  bool rows = !ring && walk_rows_ok(g, w) && (own || (opt.walk_layout & 96) != 0);
+  bool rows = !ring && !alone && walk_rows_ok(g, w) && (own || (opt.walk_layout & 96) != 0);
   if (rows && own) {
     const int lanes = g.J > 32 ? 16 : (g.J > 16 ? 8 : 4);
     const long warps_per_sm = (long)g.R * lanes / 32 / li.num_sms;
@@ -642,7 +646,7 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   }
   // the walk's bound on the weight sums (see walk_tolerance_base), by up to 64 CTAs of 8192 weights and more beside the lists
   WeightBound wb = {w_in, g.I + g.has_bias, g.jout, g.J, wbound, pad ? w_padded : nullptr, 0};
-  if (!ring || pad) {
+  if (!(ring || alone) || pad) {
     const long long n = (long long)wb.rows * g.J;
     wb.ctas = (int)(n < 64 * 8192 ? (n + 8191) / 8192 : 64);
     g.wbound_n = wb.ctas;
@@ -673,6 +677,7 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
                      ((opt.walk_layout & 8) != 0 || ((opt.walk_layout & 3) == 0 && g.J == 64 && g.R >= 32768));
   auto walk = [&]() -> int {
     if (!(fparts & 2)) return OK;
+    if (alone) return launch_walk_alone(g, keys_g, nvalid_g, key_stride(g), w, out, s);
     if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, li, s);
     if (rows) return launch_walk_rows(g, keys_g, nvalid_g, key_stride(g), w, out, own ? g.J > 32 && g.R >= 32768 : (opt.walk_layout & 64) != 0, li, s);
     if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, s, smemw_bytes, smemw_shift);

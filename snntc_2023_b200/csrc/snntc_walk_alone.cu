@@ -1,0 +1,213 @@
+// The sorted walk for fan-outs of 17 to 32 and a moderate number of rows: a warp walks one row, one output per lane, and copies the
+// weight rows its list names into shared memory ahead of itself.
+//
+// Between the walk with a copying warp (snntc_walk_ring.cu), which with a second warp per row is two waves here, and the pairs walk,
+// half of whose lanes would be idle. Weight rows arrive by asynchronous copies, 16 entries to a block, two blocks ahead of the one
+// that is consumed; the sums and sign tests of eight steps are formed before one vote, from operands that were read a group ahead.
+// Arithmetic, order, margin and decisions are those of the walk with a copying warp: the same bits. Bound by the
+// latency of the chain of sums up to about ten rows per SM and by issue beyond. Measured (B200, walk alone; copying warp, this, pairs walk): 2304 -> 32 at 2600
+// rows 77, 65, 83 us, 5400 -> 32 161, 139, 180, 576 -> 32 28, 24, 25.
+#include "snntc_common.cuh"
+#include "snntc_walk.cuh"
+
+#include <limits.h>
+#include <math_constants.h>
+
+namespace snntc {
+
+namespace {
+
+constexpr int kWarps = 2;                          // per CTA, each on a row of its own
+constexpr int kBlock = 16;                         // list entries
+constexpr int kGroup = 8;                          // steps per vote
+constexpr int kRing = 3;                           // weight blocks per warp: one consumed, two on their way
+constexpr int kListRing = 4;                       // list blocks per warp
+
+struct RingWarp {
+  float w[kRing][kBlock][32];
+  float x[kListRing][kBlock];
+  unsigned off[kListRing][kBlock];                 // element offset of the weight row
+};
+
+// (through L1: weights of 17 to 31 columns share lines, 576 -> 20 at 3500 rows 26 us, 32 past it; 32 columns 27 and 26)
+__device__ __forceinline__ void copy_async(unsigned dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// One output of one lane. wsum = sum w - theta and ysum = sum w*x run on; an output that has fired keeps its sums in fin and
+// its running weight sum at -inf, where q stays +inf.
+struct Walk {
+  float wsum, ysum;
+  float2 fin;
+  bool live;
+  int sticky;             // INT_MIN: the output was at or near zero at the last entry without firing, else INT_MAX
+  float xprev;
+
+  template <int G>
+  __device__ __forceinline__ void steps(const float (&x)[G], const float (&w)[G]) {
+    float sw[G], sy[G];
+    int p[G];
+    const float z = -2.384185791015625e-7f * fmaxf(fabsf(x[0]), fabsf(x[G - 1]));   // inputs ascend: |x| peaks at an end
+    int m = sticky;
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      sw[u] = wsum; sy[u] = ysum;
+      p[u] = __float_as_int(fmaf(z, fabsf(wsum), fmaf(-x[u], wsum, ysum)));   // (an output set aside: NaN, a positive integer)
+      m = min(m, p[u]);
+      wsum += w[u];
+      ysum = fmaf(x[u], w[u], ysum);
+    }
+    if (__builtin_expect(__any_sync(0xffffffffu, m <= 0), 0)) {
+#pragma unroll
+      for (int u = 0; u < G; ++u) {
+        const bool near = live & (p[u] <= 0);
+        if (!__any_sync(0xffffffffu, near | (sticky < 0))) continue;
+        const float xp = u == 0 ? xprev : x[u > 0 ? u - 1 : 0];
+        const bool fire = live & ratio_gt(sy[u], sw[u], xp) & ratio_le(sy[u], sw[u], x[u]);
+        if (fire) fin = make_float2(sw[u], sy[u]);
+        live = live & !fire;
+        sticky = (near & !fire) ? INT_MIN : INT_MAX;
+      }
+      if (!live) wsum = -CUDART_INF_F;
+    }
+    xprev = x[G - 1];
+  }
+};
+
+__global__ void __launch_bounds__(32 * kWarps)
+snn_walk_alone_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid, int istride, const float* w,
+                      float* __restrict__ out) {
+  chain_wait();
+  chain_next();
+  __shared__ __align__(16) RingWarp ring[kWarps];
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+  RingWarp& sm = ring[warp];
+  const int J = g.J;
+  const long item = (long)blockIdx.x * kWarps + warp;
+  if (item >= g.R) return;
+  const int r = (int)item;
+  const WalkEntry* ents = lists + (size_t)r * istride;
+  const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid + r), 0);
+  const int blocks = (n + kBlock - 1) / kBlock;
+
+  // list block b: read a block ahead into a register, then put into shared memory. Behind the end of the list: offset 0 (a
+  // row is copied that nothing consumes)
+  WalkEntry pre = make_uint2(0u, 0u);
+  auto read_list = [&](int b) {
+    pre = make_uint2(0u, 0u);
+    if (lane < kBlock && b * kBlock + lane < n) pre = ld_l2(ents + b * kBlock + lane);
+  };
+  auto put_list = [&](int b) {
+    if (lane < kBlock) {
+      sm.x[b % kListRing][lane] = __uint_as_float(pre.x);
+      sm.off[b % kListRing][lane] = pre.y;
+    }
+  };
+  // weight block b: a copy brings four rows, 16 bytes per lane (lanes behind the row copy nothing)
+  const int sub = lane >> 3, col = 4 * (lane & 7);
+  const bool mine = col < J;
+  const float* wj = w + col;
+  auto copy_weights = [&](int b) {
+    const unsigned* off = sm.off[b % kListRing];
+    const unsigned to = smem_u32(&sm.w[b % kRing][0][0]);
+#pragma unroll
+    for (int q = 0; q < kBlock / 4; ++q)
+      if (mine) copy_async(to + 512u * q + 16u * lane, wj + off[4 * q + sub]);
+  };
+
+  const bool ok = lane < g.jout;
+#pragma unroll
+  for (int b = 0; b < kRing - 1; ++b) {
+    read_list(b);
+    put_list(b);
+    __syncwarp();
+    if (b < blocks) copy_weights(b);
+    copies_commit();
+  }
+  read_list(kRing - 1);
+  Walk wk;
+  wk.wsum = -g.theta;
+  wk.ysum = 0.f;
+  if (g.has_bias) {   // the bias input (value biasvolt, weight row I) is always consumed first
+    const float wb = ok ? ld_plain(w + (size_t)g.I * J + lane) : 0.f;
+    wk.wsum += wb;
+    wk.ysum = g.biasvolt * wb;
+  }
+  if (!ok) wk.wsum = -CUDART_INF_F;
+  wk.live = ok;
+  wk.fin = make_float2(0.f, 0.f);
+  wk.sticky = INT_MAX;
+  wk.xprev = g.has_bias ? g.biasvolt : 0.f;
+  for (int b = 0; b < blocks; ++b) {
+    put_list(b + kRing - 1);
+    __syncwarp();                                  // (and every lane is through with block b - 1, whose buffer is refilled)
+    read_list(b + kRing);
+    if (b + kRing - 1 < blocks) copy_weights(b + kRing - 1);
+    copies_commit();
+    copies_wait<kRing - 1>();                      // weight block b
+    __syncwarp();
+    const float* xb = sm.x[b % kListRing];
+    const float* wb = &sm.w[b % kRing][0][lane];
+    const int nb = min(kBlock, n - b * kBlock);
+    int k = 0;
+    // the next group's operands are read while this one's vote is on its way
+    float x[2][kGroup], wv[2][kGroup];
+    auto read = [&](int at, float (&xs)[kGroup], float (&ws)[kGroup]) {
+#pragma unroll
+      for (int u = 0; u < kGroup; u += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(xb + at + u);
+        xs[u] = v.x; xs[u + 1] = v.y; xs[u + 2] = v.z; xs[u + 3] = v.w;
+      }
+#pragma unroll
+      for (int u = 0; u < kGroup; ++u) ws[u] = wb[(at + u) * 32];
+    };
+    read(0, x[0], wv[0]);
+    if (nb == kBlock) {
+      read(kGroup, x[1], wv[1]);
+      wk.steps(x[0], wv[0]);
+      wk.steps(x[1], wv[1]);
+      k = kBlock;
+    } else if (kGroup <= nb) {
+      wk.steps(x[0], wv[0]);
+      k = kGroup;
+    }
+#pragma unroll 1
+    for (; k < nb; ++k) {
+      const float x1[1] = {xb[k]}, w1[1] = {wb[k * 32]};
+      wk.steps(x1, w1);
+    }
+    if (!__any_sync(0xffffffffu, wk.live)) break;  // every output has fired
+  }
+  copies_wait<0>();
+
+  // an output that stopped has fired; one that consumed every input fires iff it is armed
+  float ws = wk.fin.x, ys = wk.fin.y;
+  bool fired = true;
+  if (wk.live) {
+    ws = wk.wsum; ys = wk.ysum;
+    fired = ratio_gt(ys, ws, wk.xprev);
+  }
+  float yv = g.maxv, iv = 0.f;
+  if (fired) {
+    iv = __fdividef(1.0f, ws);
+    yv = ys * iv;
+    if (yv >= g.maxv) { yv = g.maxv; iv = 0.f; }
+  }
+  if (ok) {
+    out[(size_t)r * g.jout + lane] = yv;
+    if (!g.infer) out[(size_t)(g.R + r) * g.jout + lane] = iv;
+    if (g.khist != nullptr) atomicAdd(g.khist + (yv < g.maxv ? entries_below(ents, n, yv) : g.I + 1), 1);
+  }
+}
+
+}  // namespace
+
+int launch_walk_alone(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
+                      cudaStream_t s) {
+  const cudaError_t e = launch_chained(snn_walk_alone_kernel, ((unsigned)g.R + kWarps - 1) / kWarps, 32 * kWarps, 0, s, 0, g, lists,
+                                       nvalid, istride, w, out);
+  count_launch();
+  return e == cudaSuccess ? OK : E_CUDA;
+}
+
+}  // namespace snntc

@@ -291,7 +291,8 @@ int launch(const Geometry& g, const WalkEntry* lists, const int* nvalid, int ist
 
 }  // namespace
 
-// How many warps of 32 outputs share a list and a copying warp: one while every CTA has an SM to itself (one row of 4096 -> 512 36 us,
+// How many warps of 32 outputs share a list and a copying warp: one for fan-outs up to 32 (with a second, idle one 64 us instead of 48
+// for 1430 rows of 2304 -> 32) and while every CTA has an SM to itself (one row of 4096 -> 512 36 us,
 // 38 with two), two up to six CTAs per SM, which is what the registers hold. Beyond, four where that makes it one wave again (25 088 ->
 // 1024 at 64 samples 424 us, 515 with two; 2000 -> 512 at 128 43, 53): the copying warp, 28 cycles an entry, holds four back (9000 ->
 // 700 at 30 samples 115 us, 89 with two).
@@ -300,7 +301,7 @@ int launch_walk_ring(const Geometry& g, const WalkEntry* lists, const int* nvali
   const bool vec = (g.J & 3) == 0 && ((uintptr_t)w & 15) == 0;
   if (!vec) return launch<false, 1>(g, lists, nvalid, istride, w, out, s);
   auto ctas = [&](int c) { return (long)g.R * ((g.J + 32 * c - 1) / (32 * c)); };
-  if (ctas(1) <= li.num_sms) return launch<true, 1>(g, lists, nvalid, istride, w, out, s);
+  if (g.J <= 32 || ctas(1) <= li.num_sms) return launch<true, 1>(g, lists, nvalid, istride, w, out, s);
   if (ctas(2) > 6L * li.num_sms && ctas(4) <= 4L * li.num_sms) return launch<true, 4>(g, lists, nvalid, istride, w, out, s);
   return launch<true, 2>(g, lists, nvalid, istride, w, out, s);
 }

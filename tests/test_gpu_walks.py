@@ -151,3 +151,21 @@ def test_walk_with_a_copying_warp(R, I, J, bv):
     ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
     assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=16)), ref)
     assert torch.equal(ops.snn_fc(xd, wd, params), ref)
+
+
+@pytest.mark.parametrize("R,I,J", [(1481, 15, 17), (1600, 16, 32), (2500, 47, 20), (3552, 70, 27), (3553, 40, 32), (1480, 300, 24)])
+@pytest.mark.parametrize("bv", [0.0, 1.0])
+def test_walk_whose_warps_copy_for_themselves(R, I, J, bv):
+    """Fan-outs of 17 to 32 at 10 to 24 rows per SM and one row either side, padded and whole, lists that end anywhere in a block of 16,
+    an empty row, a row of ties: the bits of one output per lane from global memory."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    x, w = P.make_inputs(R + I + J, (R, I), (I + (bv > 0), J), "ref", bias=bv > 0)
+    x[np.arange(R) % 7 == 0, :I // 2] = 1e5
+    x[3] = 1e5
+    x[5] = 2.0
+    params = O.fc_params(biasvolt=bv)
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
+    assert torch.equal(ops.snn_fc(xd, wd, params), ref)
+    assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=16)), ref)
