@@ -193,7 +193,8 @@ snn_dw_tma_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       const float* from = own_from + buf * kRS * kJT;
       const float4 v = make_float4(from[at01 & 0xffff], from[at01 >> 16], from[at23 & 0xffff], from[at23 >> 16]);
       todo = __ballot_sync(0xffffffffu, (v.x != 0.f) | (v.y != 0.f) | (v.z != 0.f) | (v.w != 0.f)) & ((1u << kRS) - 1u);
-      if (todo != 0u) own[lane] = v;                       // (every lane is through with the stage before: the vote)
+      __syncwarp();                                        // every lane is through with the stage before (a vote orders no memory)
+      if (todo != 0u) own[lane] = v;
       __syncwarp();
     }
 #pragma unroll 1

@@ -272,6 +272,7 @@ __device__ __forceinline__ void walk_pairs(const Geometry& g, const WalkEntry* e
   if (lane < nvalid) pre = ld_l2(ents + lane);
   // entry k of the list is staged at k % 64, the input in front of the first one at 63
   if (lane == 0) sbuf[63] = make_uint2(__float_as_uint(g.has_bias ? g.biasvolt : 0.f), 0u);
+  __syncwarp();                                           // (a row without spiking inputs goes straight on to reading it)
   auto inputs = [&](int at) { return make_float2(__uint_as_float(sbuf[at].x), __uint_as_float(sbuf[(at + 63) & 63].x)); };
   bool flipped = false;
   auto block = [&](int base, auto flip_c) {
@@ -311,6 +312,7 @@ __device__ __forceinline__ void walk_pairs(const Geometry& g, const WalkEntry* e
     flipped = pw.template flip<FLIP>(__uint_as_float(sbuf[b + nb - 1].x));
   };
   for (int base = 0; base < nvalid; base += 32) {
+    __syncwarp();                                         // (the block in front has read the last input of the one that goes)
     sbuf[(base & 32) + lane] = pre;
     __syncwarp();
     if (base + 32 + lane < nvalid) pre = ld_l2(ents + base + 32 + lane);

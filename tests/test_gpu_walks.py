@@ -169,3 +169,23 @@ def test_walk_whose_warps_copy_for_themselves(R, I, J, bv):
     ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
     assert torch.equal(ops.snn_fc(xd, wd, params), ref)
     assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=16)), ref)
+
+
+@pytest.mark.parametrize("J", [64, 128, 40])
+def test_rows_without_inputs_beside_long_ones(J):
+    """Every third row has no input that can spike, so that the bias input alone decides (weights above one: the spike, below: none);
+    the rows around it end at inputs above that spike, and with 6000 rows every warp of the staged walk takes several."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    rng = np.random.default_rng(J)
+    R, I = 6000, 100
+    x = np.exp(2 + rng.random((R, I))).astype(np.float32)
+    x[::3] = 1e5
+    w = (rng.standard_normal((I + 1, J)) * 0.3).astype(np.float32)
+    w[I] = np.where(np.arange(J) % 2 == 0, 2.0, 0.5)
+    params = O.fc_params(biasvolt=1.0)
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    want = np.where(np.arange(J) % 2 == 0, np.float32(2.0), np.float32(1e5))
+    for layout in (0, 1, 2, 3, 8, 16, 32, 64):
+        y = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=layout))[:R].cpu().numpy()
+        assert np.abs(y[::3] - want).max() == 0.0, "layout %d" % layout
