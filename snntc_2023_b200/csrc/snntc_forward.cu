@@ -318,7 +318,7 @@ __device__ __forceinline__ void walk_pairs(const Geometry& g, const WalkEntry* e
     if (base + 32 + lane < nvalid) pre = ld_l2(ents + base + 32 + lane);
     if (__builtin_expect(flipped, 0)) block(base, std::true_type{});
     else block(base, std::false_type{});
-    if (!__any_sync(0xffffffffu, pw.any_live())) break;   // every output has fired
+    if (pw.done()) break;   // every output has fired
   }
   const float xprev = __uint_as_float(sbuf[(nvalid + 63) & 63].x);
 #pragma unroll

@@ -55,7 +55,8 @@ __device__ __forceinline__ int imin3(int a, int b, int c) { return min(min(a, b)
 // comparisons (exact()); if it does not fire there, so is every output of the lane at the next step (`again`), and so is the first
 // step of a row. Rows for which X is no bound (an input below zero, a NaN, or sums that may overflow: `careful`) take the
 // comparisons whenever q <= tol. An output that has fired is parked at n = +inf: q = +inf (x > 0) or a positive NaN (x = 0) from
-// then on. Its sums wait in shared memory: as registers they made the walk spill.
+// then on, or a NaN of either sum behind a weight that is no number, which is no spike either. Its sums wait in shared memory: as
+// registers they took the walk beyond its 64.
 //
 // An output may also cross zero without firing (the two rounded comparisons of the reference can both miss it, about once in 10^5
 // spikes) and then stays below, taking its row through the comparisons at every step: twice the time of its neighbours, and where
@@ -72,7 +73,7 @@ struct PairWalk {
   static constexpr int kFloats = 128 * P;   // of shared memory per warp
   uint64_t n[P], ys[P];
   float* fin;       // this lane's column of [2 * P][2][32] floats: an output's sums once it has fired; until then the sign that its
-                    // running sums carry, and -inf (an n that overflows to +inf reads as fired at y = +inf, which is no spike)
+                    // running sums carry, and a NaN (see fired)
   float tolbase, xmag;
   int qlim;         // bits of tol, or INT_MAX: every output of this lane goes to the comparisons at the next step
   int qtol;         // bits of tol
@@ -93,7 +94,7 @@ struct PairWalk {
         const int m = 2 * p + h;
         nn[h] = ok[m] ? g.theta - wb[m] : CUDART_INF_F;   // (no output: parked, or the walk would wait for it)
         yy[h] = g.has_bias ? g.biasvolt * wb[m] : 0.f;
-        fin[64 * m] = 1.f; fin[64 * m + 32] = -CUDART_INF_F;
+        fin[64 * m] = 1.f; fin[64 * m + 32] = ok[m] ? CUDART_NAN_F : 0.f;
       }
       n[p] = pack2(nn[0], nn[1]);
       ys[p] = pack2(yy[0], yy[1]);
@@ -105,7 +106,11 @@ struct PairWalk {
     qtol = __float_as_int(tolbase * (b <= a ? a : b));     // (a NaN for a NaN at the end of the list)
     if (qlim != INT_MAX) qlim = qtol;
   }
-  __device__ __forceinline__ bool any_live() const {
+  // Whether output m has fired. The sums of a spike are numbers: one of the two ways to it has compared them. The parked n tells nothing:
+  // a weight that is infinite or NaN takes it from +inf to NaN, and a sum may overflow to +inf without a spike.
+  __device__ __forceinline__ bool fired(int m) const { return fin[64 * m + 32] == fin[64 * m + 32]; }
+  // Has every output of the warp fired? Asked once per block of entries: the parked n says no in passing, shared memory has the word.
+  __device__ __forceinline__ bool done() const {
     bool live = false;
 #pragma unroll
     for (int p = 0; p < P; ++p) {
@@ -113,7 +118,10 @@ struct PairWalk {
       unpack2(n[p], a, b);
       live |= (a != CUDART_INF_F) | (b != CUDART_INF_F);
     }
-    return live;
+    if (__any_sync(0xffffffffu, live)) return false;
+#pragma unroll
+    for (int m = 0; m < 2 * P; ++m) live |= !fired(m);
+    return !__any_sync(0xffffffffu, live);
   }
 
   // ---- one or two steps. x2: the input twice; inputs() gives the input and the one in front of it, for the comparisons
@@ -175,21 +183,20 @@ struct PairWalk {
     const bool look = (qlim == INT_MAX) & !careful;
     if (__builtin_expect(!__any_sync(0xffffffffu, look), 1)) return FLIP;
     const float tol = __int_as_float(qtol);
-    bool any = false, sure = look;                        // sure: no live output of this lane is within the margin any more
+    bool any = false, sure = look;                        // sure: no live output of this lane is within the margin any more (a NaN never fires)
     int q[2 * P];
     form_q(pack2(xprev, xprev), n, ys, q);
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-      float nn[2], s[2];
-      unpack2(n[p], nn[0], nn[1]);
+      float s[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const float qm = __int_as_float(q[2 * p + h]);
-        const bool live = nn[h] != CUDART_INF_F, below = look & live & (qm < -tol);
+        const bool live = !fired(2 * p + h), below = look & live & (qm < -tol);
         s[h] = below ? -1.f : 1.f;
         if (below) fin[64 * (2 * p + h)] *= -1.f;
         any |= below;
-        sure &= !live | (fabsf(qm) > tol);
+        sure &= !live | !(fabsf(qm) <= tol);
       }
       n[p] = mul2(n[p], pack2(s[0], s[1]));
       ys[p] = mul2(ys[p], pack2(s[0], s[1]));
@@ -206,13 +213,13 @@ struct PairWalk {
     unpack2(n[m / 2], nn[0], nn[1]);
     unpack2(ys[m / 2], yy[0], yy[1]);
     float a = fin[64 * m], ws = 0.f - a, yv = fin[64 * m + 32];
-    bool fired = true;
-    if (nn[m & 1] != CUDART_INF_F) {
+    bool spike = true;
+    if (!fired(m)) {
       ws = 0.f - a * nn[m & 1]; yv = a * yy[m & 1];
-      fired = ratio_gt(yv, ws, xprev);
+      spike = ratio_gt(yv, ws, xprev);
     }
     y = g.maxv; inv = 0.f;
-    if (fired) {
+    if (spike) {
       inv = __fdividef(1.0f, ws);
       y = yv * inv;
       if (y >= g.maxv) { y = g.maxv; inv = 0.f; }
@@ -273,14 +280,13 @@ struct PairWalk {
     bool again = false;
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-      float nn[2], yy[2], after[2], park[2] = {0.f, 0.f};
+      float nn[2], yy[2], park[2] = {0.f, 0.f};
       sums<FLIP>(n0, ys0, p, nn, yy);
-      unpack2(n1[p], after[0], after[1]);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int m = 2 * p + h;
         if (!__any_sync(0xffffffffu, q[m] <= qlim)) continue;
-        const bool live = after[h] != CUDART_INF_F;
+        const bool live = !fired(m);
         const float wsum = 0.f - nn[h];
         const bool fire = live & ratio_gt(yy[h], wsum, xp) & ratio_le(yy[h], wsum, x);
         park[h] = fire ? CUDART_INF_F : 0.f;

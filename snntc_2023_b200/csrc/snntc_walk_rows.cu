@@ -169,7 +169,7 @@ snn_walk_rows_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
         }
         flipped = pw.flip<false>(xprev);
       }
-      if (!__any_sync(0xffffffffu, pw.any_live())) break;   // every output has fired
+      if (pw.done()) break;   // every output has fired
     }
 
     float yo[4], io[4];

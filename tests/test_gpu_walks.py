@@ -189,3 +189,34 @@ def test_rows_without_inputs_beside_long_ones(J):
     for layout in (0, 1, 2, 3, 8, 16, 32, 64):
         y = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=layout))[:R].cpu().numpy()
         assert np.abs(y[::3] - want).max() == 0.0, "layout %d" % layout
+
+
+@pytest.mark.parametrize("J", [16, 64, 96, 128, 132])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("bv", [0.0, 1.0])
+def test_spikes_in_front_of_weights_that_are_no_numbers(J, bad, bv):
+    """One infinite or NaN weight in every column, anywhere from the first input to the last: an output that fired in front of it keeps
+    its spike, in every layout, and what had not fired by then stays without one. The bits of one output per lane, which keeps a
+    flag per output, and the oracle's spikes."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    rng = np.random.default_rng(J)
+    R, I = 400, 120
+    x = np.exp(1.5 * rng.random((R, I))).astype(np.float32)
+    w = (rng.standard_normal((I + (bv > 0), J)) * np.sqrt(15.0 / I)).astype(np.float32)
+    w[I:] = 0.0
+    w[rng.integers(0, I, J), np.arange(J)] = bad
+    x[0, :6] = [1.0, 1.1, 1.2, 1.3, 1.4, 1.5]      # fires at 1.21667 in column 0, then meets `bad`
+    x[0, 6:] = 1e5
+    w[:6, 0] = [5.0, 1.0, 1.0, 0.1, bad, 0.1]
+    w[6:I, 0] = 0.1
+    params = O.fc_params(biasvolt=bv)
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
+    for layout in (0, 1, 3, 8, 16, 32, 64):
+        assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=layout)), ref), "layout %d" % layout
+    o32 = O.fc_forward(x, w, params, "f32")
+    got = ref[:R].cpu().numpy()
+    assert np.array_equal(got < 9e4, o32["y"] < 9e4)
+    assert abs(got[0, 0] - 1.21667) < 1e-4 and 0.1 < (got < 9e4).mean() < 0.95
+    assert np.allclose(got, o32["y"], rtol=1e-5)
