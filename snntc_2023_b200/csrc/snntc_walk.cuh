@@ -252,7 +252,7 @@ struct PairWalk {
   template <bool FLIP, typename Inputs>
   __device__ __forceinline__ void hit(const int (&q)[2 * P], const uint64_t (&n0)[P], const uint64_t (&ys0)[P], uint64_t (&n1)[P],
                                       Inputs&& inputs) {
-    const float tol = __int_as_float(qlim);                // (INT_MAX: a NaN, nothing below fires)
+    const float tol = careful ? CUDART_NAN_F : __int_as_float(qlim);   // (INT_MAX is a NaN, too: nothing below fires)
     float near = CUDART_INF_F;
 #pragma unroll
     for (int p = 0; p < P; ++p) {
@@ -295,7 +295,7 @@ struct PairWalk {
       }
       n1[p] = add2(n1[p], pack2(park[0], park[1]));
     }
-    qlim = again | careful ? INT_MAX : qtol;
+    qlim = again ? INT_MAX : qtol;
   }
 };
 

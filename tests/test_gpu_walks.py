@@ -220,3 +220,40 @@ def test_spikes_in_front_of_weights_that_are_no_numbers(J, bad, bv):
     assert np.array_equal(got < 9e4, o32["y"] < 9e4)
     assert abs(got[0, 0] - 1.21667) < 1e-4 and 0.1 < (got < 9e4).mean() < 0.95
     assert np.allclose(got, o32["y"], rtol=1e-5)
+
+
+@pytest.mark.parametrize("J,layout", [(128, 3), (64, 1), (64, 8), (32, 32)])
+def test_rows_with_an_input_below_zero_are_walked_as_fast(J, layout):
+    """Where no proof holds that a sum below the margin has fired, the reference's comparisons are taken near zero, not at every step:
+    rows with one small negative input against the same rows without it (median of interleaved runs, graph replays of ten calls)."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    rng = np.random.default_rng(J)
+    R, I = 16384, 576
+    x = np.exp(1.5 * rng.random((R, I))).astype(np.float32)
+    x[rng.random((R, I)) < 0.5] = 1e5
+    w = (rng.standard_normal((I, J)) * np.sqrt(15.0 / I)).astype(np.float32)
+    w[0] = 0.0
+    params = O.fc_params(biasvolt=0.0)
+    opts = _lib.options(walk_layout=layout)
+    times, graphs, outs = ([], []), [], []
+    for first in (0.5, -0.5):
+        x[:, 0] = first                             # (weight zero: changes no sum)
+        xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+        outs.append(ops.snn_fc(xd, wd, params, opts=opts))
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for _ in range(10):
+                ops.snn_fc(xd, wd, params, opts=opts)
+        graphs.append((g, xd, wd))
+    assert torch.equal(outs[0], outs[1])
+    for _ in range(7):
+        for t, (g, _, _) in zip(times, graphs):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            g.replay()
+            b.record()
+            b.synchronize()
+            t.append(a.elapsed_time(b))
+    plain, below = (sorted(t)[3] for t in times)
+    assert below < 1.3 * plain, "%.3f ms against %.3f" % (below, plain)
