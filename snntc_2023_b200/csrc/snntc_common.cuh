@@ -49,7 +49,8 @@ struct Options {
                             // 8: output pairs with the weights staged in shared memory (where they fit)
                             // 16: one output per lane, the warp's weight rows copied ahead into shared memory
                             // 32, 64: several rows per warp (fan-out <= 64, a multiple of 4), weights from global memory /
-                            // in shared memory where they fit. A layout that the weights do not allow: auto
+                            // in shared memory where they fit. 128: a row per warp that copies its own weight rows
+                            // (fan-out <= 32). A layout that the weights do not allow: auto
   int walk_outputs = 0;     // outputs per lane of layout 2: 0 auto, 1..3: 1, 2, 4
   int list_builder = 0;     // 0 auto, 1 per-row bucket sort, 2 per-pixel sort + merges (3x3 stride-1 conv only),
                             // 3 per-row sorting network in registers (rows of at most 64 inputs);

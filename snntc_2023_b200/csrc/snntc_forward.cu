@@ -630,7 +630,8 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   const bool copies16 = (g.J & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
   const bool few = copies16 && g.J > 32 ? (long)g.R * ((g.J + 63) / 64) <= 12L * li.num_sms : ring_items <= (copies16 && g.J > 16 ? 10L : 8L) * li.num_sms;
   const bool ring = (opt.walk_layout & 16) != 0 || (own && few);
-  const bool alone = own && !ring && copies16 && g.J > 16 && g.J <= 32 && ring_items <= 24L * li.num_sms;
+  const bool alone = copies16 && g.J <= 32 && ((opt.walk_layout & 128) != 0 ||
+                                               (own && !ring && g.J > 16 && ring_items <= 24L * li.num_sms));
   // Several rows per warp for fan-out up to 64, where that leaves enough warps: 5 per SM at eight rows to a warp (fan-out 16;
   // 10 where the weights miss the L1 cache), 11 at four (32), 40 at two (64). With fewer the pairs walk, a warp per row, hides
   // its latencies better. Pairs against rows, us: 576 -> 16 4000 rows 35, 39, 7000 rows 53, 39; 576 -> 32 35, 37 and 54, 43; 147 -> 64 8000

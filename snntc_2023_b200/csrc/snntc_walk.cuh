@@ -1,4 +1,5 @@
-// What the walk kernels share: the reference's fire comparisons, the causal-set size, the integer minimum of a step's sign test.
+// What the walk kernels share: the reference's fire comparisons, the causal-set size, the integer minimum of a step's sign test, and the
+// steps of a walk with a lane's outputs in pairs (PairWalk) and with one output per lane (LaneWalk).
 #pragma once
 #include "snntc_common.cuh"
 #include "snntc_ptx.cuh"
@@ -296,6 +297,136 @@ struct PairWalk {
       n1[p] = add2(n1[p], pack2(park[0], park[1]));
     }
     qlim = again ? INT_MAX : qtol;
+  }
+};
+
+// One output of one lane, for walks that are bound by the latency of the chain of sums: the sums and sign tests of G steps are formed
+// before one vote. wsum = sum w - theta and ysum = sum w*x run on; an output that has fired keeps its sums in fin and its running
+// weight sum at -inf, where q stays +inf. The margin of a sign test is 2^-22 |x * sum w|, formed from the output's own sum -- four
+// times the rounding error of the reference's product x * sum w, so every step that rounding could decide goes to the
+// reference's comparisons, and no bound over the weight matrix is needed.
+struct LaneWalk {
+  float wsum, ysum;       // times sign
+  float2 fin;
+  bool live;
+  int sticky;             // INT_MIN: the output was at or near zero at the last entry without firing, else INT_MAX
+  float xprev;
+  float sign;             // -1: the output has crossed zero without firing (turn)
+
+  // sums with the bias input consumed (value biasvolt, weight wb), which is always the first; not ok: no output, nothing waits for it
+  __device__ __forceinline__ void start(const Geometry& g, bool ok, float wb) {
+    wsum = -g.theta;
+    ysum = 0.f;
+    if (g.has_bias) {
+      wsum += wb;
+      ysum = g.biasvolt * wb;
+    }
+    if (!ok) wsum = -CUDART_INF_F;
+    live = ok;
+    fin = make_float2(0.f, 0.f);
+    sticky = INT_MAX;
+    xprev = g.has_bias ? g.biasvolt : 0.f;
+    sign = 1.f;
+  }
+  // spike value and 1/(sum w - theta) once the list is consumed: an output that stopped has fired; one that consumed every input fires
+  // iff it is armed
+  __device__ __forceinline__ void finish(const Geometry& g, float& y, float& inv) const {
+    float ws = fin.x, ys = fin.y;
+    bool spike = true;
+    if (live) {
+      ws = plain(wsum); ys = plain(ysum);
+      spike = ratio_gt(ys, ws, xprev);
+    }
+    y = g.maxv; inv = 0.f;
+    if (spike) {
+      inv = __fdividef(1.0f, ws);
+      y = ys * inv;
+      if (y >= g.maxv) { y = g.maxv; inv = 0.f; }
+    }
+  }
+
+  __device__ __forceinline__ float plain(float v) const { return sign < 0.f ? 0.f - v : v; }   // (an exactly cancelled sum stays +0)
+
+  // lim: bits of the q beyond the margin that still goes to the comparisons, 0 unless the output has been turned
+  template <int G>
+  __device__ __forceinline__ void steps(const float (&x)[G], const float (&w)[G], const int lim) {
+    float sw[G], sy[G];
+    int p[G];
+    const float z = -2.384185791015625e-7f * fmaxf(fabsf(x[0]), fabsf(x[G - 1]));   // inputs ascend: |x| peaks at an end
+    int m = sticky;
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      sw[u] = wsum; sy[u] = ysum;
+      p[u] = __float_as_int(fmaf(z, fabsf(wsum), fmaf(-x[u], wsum, ysum)));   // (an output set aside: NaN, a positive integer)
+      if (u & 1) m = imin3(m, p[u - (u > 0)], p[u]);
+      else if (u == G - 1) m = min(m, p[u]);
+      wsum += w[u];
+      ysum = fmaf(x[u], w[u], ysum);
+    }
+    if (__builtin_expect(__any_sync(0xffffffffu, m <= lim), 0)) {
+      // Every lane takes its own first step at or near zero through the comparisons, all lanes at once. Nearly always that step
+      // fires; where one does not, or was waited for from the group before, the steps are gone through one by one.
+      {
+        float tw = 0.f, ty = 0.f, tx = 0.f, txp = 0.f;
+        bool at = false;
+#pragma unroll
+        for (int u = G - 1; u >= 0; --u) {
+          if (p[u] <= lim) { tw = sw[u]; ty = sy[u]; tx = x[u]; txp = u == 0 ? xprev : x[u > 0 ? u - 1 : 0]; at = true; }
+        }
+        at &= live;
+        tw = plain(tw); ty = plain(ty);
+        const bool hit = at & ratio_gt(ty, tw, txp) & ratio_le(ty, tw, tx);
+        if (!__any_sync(0xffffffffu, (at & !hit) | (sticky < 0))) {
+          if (hit) {
+            fin = make_float2(tw, ty);
+            wsum = -CUDART_INF_F;
+            live = false;
+          }
+          xprev = x[G - 1];
+          return;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < G; ++u) {
+        const bool near = live & (p[u] <= lim);
+        if (!__any_sync(0xffffffffu, near | (sticky < 0))) continue;
+        const float xp = u == 0 ? xprev : x[u > 0 ? u - 1 : 0], tw = plain(sw[u]), ty = plain(sy[u]);
+        const bool fire = live & ratio_gt(ty, tw, xp) & ratio_le(ty, tw, x[u]);
+        if (fire) fin = make_float2(tw, ty);
+        live = live & !fire;
+        sticky = (near & !fire) ? INT_MIN : INT_MAX;
+      }
+      if (!live) wsum = -CUDART_INF_F;
+    }
+    xprev = x[G - 1];
+  }
+
+  // Between two groups. An output may cross zero without firing (both rounded comparisons of the reference can miss it: about once
+  // in 10^5 spikes at some hundred inputs, once in some hundred at 25 000) and would take its warp through the steps one by one to the
+  // end of the list. Beyond the margin its sums change their sign, and with them its q: it cannot fire before q comes back to zero.
+  // (A positive sum: not armed, if the present sums, too, see the last input beyond zero -- guard() widens the margin by what the
+  // step between may have added. A negative sum: not yet back.) Returns whether the warp has any such output.
+  __device__ __forceinline__ bool turn(bool turned) {
+    if (__builtin_expect(__any_sync(0xffffffffu, sticky < 0), 0)) {
+      const float q = fmaf(-xprev, wsum, ysum);
+      if (sticky < 0 && live && fabsf(q) > 2.384185791015625e-7f * fabsf(xprev * wsum)) {
+        sticky = INT_MAX;
+        if (q < 0.f) { sign = -sign; wsum = 0.f - wsum; ysum = 0.f - ysum; }
+      }
+      turned |= (bool)__any_sync(0xffffffffu, sign < 0.f);
+    }
+    return turned;
+  }
+  // weights of a group in a warp with turned outputs: their sign, and the limit for steps()
+  template <int G>
+  __device__ __forceinline__ int guard(const float (&x)[G], float (&w)[G]) const {
+    float most = 0.f;
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      most = fmaxf(most, fabsf(w[u]));
+      w[u] *= sign;
+    }
+    return sign < 0.f ? __float_as_int(2.384185791015625e-7f * most * fmaxf(fabsf(x[0]), fabsf(x[G - 1]))) : 0;
   }
 };
 

@@ -4,9 +4,9 @@
 // Between the walk with a copying warp (snntc_walk_ring.cu), which with a second warp per row is two waves here, and the pairs walk,
 // half of whose lanes would be idle. Weight rows arrive by asynchronous copies, 16 entries to a block, two blocks ahead of the one
 // that is consumed; the sums and sign tests of eight steps are formed before one vote, from operands that were read a group ahead.
-// Arithmetic, order, margin and decisions are those of the walk with a copying warp: the same bits. Bound by the
-// latency of the chain of sums up to about ten rows per SM and by issue beyond. Measured (B200, walk alone; copying warp, this, pairs walk): 2304 -> 32 at 2600
-// rows 77, 65, 83 us, 5400 -> 32 161, 139, 180, 576 -> 32 28, 24, 25.
+// The steps are those of the walk with a copying warp (LaneWalk in snntc_walk.cuh): the same bits. Bound by the latency of the chain of sums
+// up to about ten rows per SM and by issue beyond. Measured (B200, walk alone; copying warp, this, pairs walk): 2304 -> 32 at 2600 rows
+// 77, 65, 83 us, 5400 -> 32 161, 139, 180, 576 -> 32 28, 24, 25.
 #include "snntc_common.cuh"
 #include "snntc_walk.cuh"
 
@@ -33,46 +33,6 @@ struct RingWarp {
 __device__ __forceinline__ void copy_async(unsigned dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-
-// One output of one lane. wsum = sum w - theta and ysum = sum w*x run on; an output that has fired keeps its sums in fin and
-// its running weight sum at -inf, where q stays +inf.
-struct Walk {
-  float wsum, ysum;
-  float2 fin;
-  bool live;
-  int sticky;             // INT_MIN: the output was at or near zero at the last entry without firing, else INT_MAX
-  float xprev;
-
-  template <int G>
-  __device__ __forceinline__ void steps(const float (&x)[G], const float (&w)[G]) {
-    float sw[G], sy[G];
-    int p[G];
-    const float z = -2.384185791015625e-7f * fmaxf(fabsf(x[0]), fabsf(x[G - 1]));   // inputs ascend: |x| peaks at an end
-    int m = sticky;
-#pragma unroll
-    for (int u = 0; u < G; ++u) {
-      sw[u] = wsum; sy[u] = ysum;
-      p[u] = __float_as_int(fmaf(z, fabsf(wsum), fmaf(-x[u], wsum, ysum)));   // (an output set aside: NaN, a positive integer)
-      m = min(m, p[u]);
-      wsum += w[u];
-      ysum = fmaf(x[u], w[u], ysum);
-    }
-    if (__builtin_expect(__any_sync(0xffffffffu, m <= 0), 0)) {
-#pragma unroll
-      for (int u = 0; u < G; ++u) {
-        const bool near = live & (p[u] <= 0);
-        if (!__any_sync(0xffffffffu, near | (sticky < 0))) continue;
-        const float xp = u == 0 ? xprev : x[u > 0 ? u - 1 : 0];
-        const bool fire = live & ratio_gt(sy[u], sw[u], xp) & ratio_le(sy[u], sw[u], x[u]);
-        if (fire) fin = make_float2(sw[u], sy[u]);
-        live = live & !fire;
-        sticky = (near & !fire) ? INT_MIN : INT_MAX;
-      }
-      if (!live) wsum = -CUDART_INF_F;
-    }
-    xprev = x[G - 1];
-  }
-};
 
 __global__ void __launch_bounds__(32 * kWarps)
 snn_walk_alone_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid, int istride, const float* w,
@@ -125,19 +85,9 @@ snn_walk_alone_kernel(const Geometry g, const WalkEntry* lists, const int* nvali
     copies_commit();
   }
   read_list(kRing - 1);
-  Walk wk;
-  wk.wsum = -g.theta;
-  wk.ysum = 0.f;
-  if (g.has_bias) {   // the bias input (value biasvolt, weight row I) is always consumed first
-    const float wb = ok ? ld_plain(w + (size_t)g.I * J + lane) : 0.f;
-    wk.wsum += wb;
-    wk.ysum = g.biasvolt * wb;
-  }
-  if (!ok) wk.wsum = -CUDART_INF_F;
-  wk.live = ok;
-  wk.fin = make_float2(0.f, 0.f);
-  wk.sticky = INT_MAX;
-  wk.xprev = g.has_bias ? g.biasvolt : 0.f;
+  LaneWalk wk;
+  wk.start(g, ok, g.has_bias && ok ? ld_plain(w + (size_t)g.I * J + lane) : 0.f);
+  bool turned = false;
   for (int b = 0; b < blocks; ++b) {
     put_list(b + kRing - 1);
     __syncwarp();                                  // (and every lane is through with block b - 1, whose buffer is refilled)
@@ -161,38 +111,34 @@ snn_walk_alone_kernel(const Geometry g, const WalkEntry* lists, const int* nvali
 #pragma unroll
       for (int u = 0; u < kGroup; ++u) ws[u] = wb[(at + u) * 32];
     };
+    auto group = [&](const auto& xs, auto& ws) {
+      int lim = 0;
+      if (__builtin_expect(turned, 0)) lim = wk.guard(xs, ws);
+      wk.steps(xs, ws, lim);
+    };
     read(0, x[0], wv[0]);
     if (nb == kBlock) {
       read(kGroup, x[1], wv[1]);
-      wk.steps(x[0], wv[0]);
-      wk.steps(x[1], wv[1]);
+      group(x[0], wv[0]);
+      group(x[1], wv[1]);
       k = kBlock;
     } else if (kGroup <= nb) {
-      wk.steps(x[0], wv[0]);
+      group(x[0], wv[0]);
       k = kGroup;
     }
 #pragma unroll 1
     for (; k < nb; ++k) {
-      const float x1[1] = {xb[k]}, w1[1] = {wb[k * 32]};
-      wk.steps(x1, w1);
+      const float x1[1] = {xb[k]};
+      float w1[1] = {wb[k * 32]};
+      group(x1, w1);
     }
+    turned = wk.turn(turned);
     if (!__any_sync(0xffffffffu, wk.live)) break;  // every output has fired
   }
   copies_wait<0>();
 
-  // an output that stopped has fired; one that consumed every input fires iff it is armed
-  float ws = wk.fin.x, ys = wk.fin.y;
-  bool fired = true;
-  if (wk.live) {
-    ws = wk.wsum; ys = wk.ysum;
-    fired = ratio_gt(ys, ws, wk.xprev);
-  }
-  float yv = g.maxv, iv = 0.f;
-  if (fired) {
-    iv = __fdividef(1.0f, ws);
-    yv = ys * iv;
-    if (yv >= g.maxv) { yv = g.maxv; iv = 0.f; }
-  }
+  float yv, iv;
+  wk.finish(g, yv, iv);
   if (ok) {
     out[(size_t)r * g.jout + lane] = yv;
     if (!g.infer) out[(size_t)(g.R + r) * g.jout + lane] = iv;

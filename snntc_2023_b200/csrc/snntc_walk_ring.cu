@@ -12,9 +12,7 @@
 //     comparisons (snntc/snnfc_kernels.cu.cc:46-55) and nothing is replayed;
 //   - one output per lane: with a warp per scheduler every instruction of the dependent chain costs its latency, so the fewest
 //     instructions per step win (two outputs per lane, as pairs in 64-bit registers, took 82 cycles a step).
-// Arithmetic, order and decisions are those of walk_row: the same bits. The margin of a sign test is 2^-22 |x * sum w|, formed
-// from the output's own sum -- four times the rounding error of the reference's product x * sum w, so every step that
-// rounding could decide goes to the reference's comparisons, and no bound over the weight matrix has to be computed first.
+// Arithmetic, order and decisions (LaneWalk in snntc_walk.cuh) are those of walk_row: the same bits.
 // Measured (B200, walk alone, each warp copying for itself -> now): one row of 784 -> 400 18.6 -> 14.3 us, 64 of 2304 -> 256 30 -> 25,
 // 128 of 2000 -> 512 76 -> 43, 100 of 6000 -> 1000 219 -> 164, 64 of 25 088 -> 1024 802 -> 424 (of which the outputs that rounding
 // keeps from firing, turn() below, 150).
@@ -40,100 +38,6 @@ __device__ __forceinline__ void copy_async(unsigned dst, const void* src, bool v
   else
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(BYTES), "r"(valid ? BYTES : 0) : "memory");
 }
-
-// One output of one lane. wsum = sum w - theta and ysum = sum w*x run on; an output that has fired keeps its sums in fin and
-// its running weight sum at -inf, where q stays +inf.
-struct Walk {
-  float wsum, ysum;       // times sign
-  float2 fin;
-  bool live;
-  int sticky;             // INT_MIN: the output was at or near zero at the last entry without firing, else INT_MAX
-  float xprev;
-  float sign;             // -1: the output has crossed zero without firing (turn)
-
-  __device__ __forceinline__ float plain(float v) const { return sign < 0.f ? 0.f - v : v; }   // (an exactly cancelled sum stays +0)
-
-  // lim: bits of the q beyond the margin that still goes to the comparisons, 0 unless the output has been turned
-  __device__ __forceinline__ void steps(const float (&x)[kGroup], const float (&w)[kGroup], const int lim) {
-    constexpr int G = kGroup;
-    float sw[G], sy[G];
-    int p[G];
-    const float z = -2.384185791015625e-7f * fmaxf(fabsf(x[0]), fabsf(x[G - 1]));   // inputs ascend: |x| peaks at an end
-    int m = sticky;
-#pragma unroll
-    for (int u = 0; u < G; ++u) {
-      sw[u] = wsum; sy[u] = ysum;
-      p[u] = __float_as_int(fmaf(z, fabsf(wsum), fmaf(-x[u], wsum, ysum)));   // (an output set aside: NaN, a positive integer)
-      if (u & 1) m = imin3(m, p[u - (u > 0)], p[u]);
-      wsum += w[u];
-      ysum = fmaf(x[u], w[u], ysum);
-    }
-    if (__builtin_expect(__any_sync(0xffffffffu, m <= lim), 0)) {
-      // Every lane takes its own first step at or near zero through the comparisons, all lanes at once. Nearly always that step
-      // fires; where one does not, or was waited for from the group before, the steps are gone through one by one.
-      {
-        float tw = 0.f, ty = 0.f, tx = 0.f, txp = 0.f;
-        bool at = false;
-#pragma unroll
-        for (int u = G - 1; u >= 0; --u) {
-          if (p[u] <= lim) { tw = sw[u]; ty = sy[u]; tx = x[u]; txp = u == 0 ? xprev : x[u > 0 ? u - 1 : 0]; at = true; }
-        }
-        at &= live;
-        tw = plain(tw); ty = plain(ty);
-        const bool hit = at & ratio_gt(ty, tw, txp) & ratio_le(ty, tw, tx);
-        if (!__any_sync(0xffffffffu, (at & !hit) | (sticky < 0))) {
-          if (hit) {
-            fin = make_float2(tw, ty);
-            wsum = -CUDART_INF_F;
-            live = false;
-          }
-          xprev = x[G - 1];
-          return;
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < G; ++u) {
-        const bool near = live & (p[u] <= lim);
-        if (!__any_sync(0xffffffffu, near | (sticky < 0))) continue;
-        const float xp = u == 0 ? xprev : x[u > 0 ? u - 1 : 0], tw = plain(sw[u]), ty = plain(sy[u]);
-        const bool fire = live & ratio_gt(ty, tw, xp) & ratio_le(ty, tw, x[u]);
-        if (fire) fin = make_float2(tw, ty);
-        live = live & !fire;
-        sticky = (near & !fire) ? INT_MIN : INT_MAX;
-      }
-      if (!live) wsum = -CUDART_INF_F;
-    }
-    xprev = x[G - 1];
-  }
-
-  // Between two groups. An output may cross zero without firing (both rounded comparisons of the reference can miss it: about once
-  // in 10^5 spikes at some hundred inputs, once in some hundred at 25 000) and would take its warp through the steps one by one to the
-  // end of the list. Beyond the margin its sums change their sign, and with them its q: it cannot fire before q comes back to zero.
-  // (A positive sum: not armed, if the present sums, too, see the last input beyond zero -- guard() widens the margin by what the
-  // step between may have added. A negative sum: not yet back.) Returns whether the warp has any such output.
-  __device__ __forceinline__ bool turn(bool turned) {
-    if (__builtin_expect(__any_sync(0xffffffffu, sticky < 0), 0)) {
-      const float q = fmaf(-xprev, wsum, ysum);
-      if (sticky < 0 && live && fabsf(q) > 2.384185791015625e-7f * fabsf(xprev * wsum)) {
-        sticky = INT_MAX;
-        if (q < 0.f) { sign = -sign; wsum = 0.f - wsum; ysum = 0.f - ysum; }
-      }
-      turned |= (bool)__any_sync(0xffffffffu, sign < 0.f);
-    }
-    return turned;
-  }
-  // weights of a group in a warp with turned outputs: their sign, and the limit for steps()
-  __device__ __forceinline__ int guard(const float (&x)[kGroup], float (&w)[kGroup]) const {
-    constexpr int G = kGroup;
-    float most = 0.f;
-#pragma unroll
-    for (int u = 0; u < G; ++u) {
-      most = fmaxf(most, fabsf(w[u]));
-      w[u] *= sign;
-    }
-    return sign < 0.f ? __float_as_int(2.384185791015625e-7f * most * fmaxf(fabsf(x[0]), fabsf(x[G - 1]))) : 0;
-  }
-};
 
 // A CTA takes a row and 32 * C outputs: C warps walk 32 outputs each, one more warp copies for them. VEC: J is a multiple of 4 and w
 // 16-byte aligned: 16-byte weight copies, else 4-byte ones (C = 1).
@@ -217,20 +121,8 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
 
   const int j = j0 + 32 * warp + lane;
   const bool ok = j < g.jout;
-  Walk wk;
-  wk.wsum = -g.theta;
-  wk.ysum = 0.f;
-  if (g.has_bias) {   // the bias input (value biasvolt, weight row I) is always consumed first
-    const float wb = ok ? ld_plain(w + (size_t)g.I * J + j) : 0.f;
-    wk.wsum += wb;
-    wk.ysum = g.biasvolt * wb;
-  }
-  if (!ok) wk.wsum = -CUDART_INF_F;
-  wk.live = ok;
-  wk.fin = make_float2(0.f, 0.f);
-  wk.sticky = INT_MAX;
-  wk.xprev = g.has_bias ? g.biasvolt : 0.f;
-  wk.sign = 1.f;
+  LaneWalk wk;
+  wk.start(g, ok, g.has_bias && ok ? ld_plain(w + (size_t)g.I * J + j) : 0.f);
   if (blocks > 0 && __syncthreads_or(wk.live)) {
     bool more = true, turned = false;
     // (one copy of the steps: reading the next group ahead of a vote takes two, and costs more in instructions that have to be
@@ -258,19 +150,8 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
     }
   }
 
-  // an output that stopped has fired; one that consumed every input fires iff it is armed
-  float ws = wk.fin.x, ys = wk.fin.y;
-  bool fired = true;
-  if (wk.live) {
-    ws = wk.plain(wk.wsum); ys = wk.plain(wk.ysum);
-    fired = ratio_gt(ys, ws, wk.xprev);
-  }
-  float yv = g.maxv, iv = 0.f;
-  if (fired) {
-    iv = __fdividef(1.0f, ws);
-    yv = ys * iv;
-    if (yv >= g.maxv) { yv = g.maxv; iv = 0.f; }
-  }
+  float yv, iv;
+  wk.finish(g, yv, iv);
   if (ok) {
     out[(size_t)r * g.jout + j] = yv;
     if (!g.infer) out[(size_t)(g.R + r) * g.jout + j] = iv;

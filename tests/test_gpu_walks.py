@@ -257,3 +257,42 @@ def test_rows_with_an_input_below_zero_are_walked_as_fast(J, layout):
             t.append(a.elapsed_time(b))
     plain, below = (sorted(t)[3] for t in times)
     assert below < 1.3 * plain, "%.3f ms against %.3f" % (below, plain)
+
+
+@pytest.mark.parametrize("J", [20, 32])
+@pytest.mark.parametrize("R", [600, 1600, 3500])
+@pytest.mark.parametrize("band,scale", [(1e-4, 3e4), (1e-3, 3e3), (3e-3, 1e3)])
+def test_hidden_spikes_in_the_walk_whose_warps_copy_for_themselves(R, J, band, scale):
+    """As above at fan-outs of 17 to 32: by name at any number of rows (128), and as the library chooses it at 1600 and 3500."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    rng = np.random.default_rng(R + J)
+    I = 300
+    x = np.exp(band * rng.random((R, I))).astype(np.float32)
+    w = (rng.standard_normal((I + 1, J)) * np.sqrt(15.0 / I) * scale).astype(np.float32)
+    w[I] = 0.0
+    params = O.fc_params(biasvolt=1.0)
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
+    assert band > 1e-4 or int((ref[R:] < 0).sum()) > 0
+    for layout in (0, 16, 128):
+        assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=layout)), ref), "layout %d" % layout
+
+
+@pytest.mark.parametrize("J", [4, 16, 20, 32])
+@pytest.mark.parametrize("I", [1, 7, 8, 9, 15, 16, 17, 33, 64, 300])
+def test_warps_that_copy_for_themselves_by_name(I, J):
+    """Lists that end at every edge of a group of 8 and a block of 16, inputs below zero and below the bias input, empty rows."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    rng = np.random.default_rng(40 * I + J)
+    x = np.exp(1.5 * rng.random((70, I))).astype(np.float32)
+    x[rng.random((70, I)) < 0.3] = 1e5
+    x[2] = 1e5
+    x[4, 0] = -0.25
+    x[6] = 0.5
+    w = (rng.standard_normal((I + 1, J)) * np.sqrt(15.0 / I)).astype(np.float32)
+    params = O.fc_params(biasvolt=1.0)
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
+    assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=128)), ref)
