@@ -61,3 +61,33 @@ def test_channels_dealt_out_by_activity(C, J, k, pattern):
     _, dw5, _ = ops.snn_cv_grad(gd, xd, wd, params, out, pt, pl, opts=_lib.options(dw_kernel=4))
     assert torch.equal(dw4, dw5)
     assert _lib.load_measure().snntc_copy_timeouts() == 0
+
+
+@pytest.mark.parametrize("C,J,k,stride", [(64, 64, 3, 1), (32, 96, 3, 2), (20, 52, 5, 2), (128, 40, 3, 1), (16, 24, 3, 2),   # 16-byte copies
+                                          (19, 64, 3, 1), (3, 33, 7, 2), (53, 70, 3, 2), (7, 30, 5, 1), (90, 9, 3, 1)])       # single columns
+@pytest.mark.parametrize("pattern", ["hot", "late", "none", "all"])
+def test_channels_dealt_out_by_activity_with_copies_per_thread(C, J, k, stride, pattern):
+    """The same patterns in the row-skipping kernel with copies per thread: strides, channel and output counts that are no multiple of
+    four, 32 and 64 outputs to a CTA with ragged last ones."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    rng = np.random.default_rng(C + J + k + stride)
+    B, H, W = 5, 19, 17
+    x, w = P.make_inputs(C + J + k, (B, H, W, C), (k * k * C + 1, J), "ref", bias=True)
+    params = O.cv_params(k, k, stride, stride, "SAME")
+    pt, pl, Nh, Nw = ops.conv_geometry(H, W, k, k, stride, stride, "SAME")
+    gr = rng.standard_normal((B, Nh, Nw, J)).astype(np.float32)
+    if pattern == "hot":
+        gr[..., rng.permutation(J)[max(1, J // 8):]] = 0
+    elif pattern == "late":
+        gr[:3] = 0
+        gr[..., ::3] = 0
+    elif pattern == "none":
+        gr[:] = 0
+    xd, wd, gd = (torch.from_numpy(a).cuda() for a in (x, w, gr))
+    out = ops.snn_cv(xd, wd, params, pt, pl, Nh, Nw)
+    _, dw1, _ = ops.snn_cv_grad(gd, xd, wd, params, out, pt, pl, opts=_lib.options(dw_kernel=1))
+    _, dw2, _ = ops.snn_cv_grad(gd, xd, wd, params, out, pt, pl, opts=_lib.options(dw_kernel=2))
+    assert float((dw2 - dw1).norm()) <= 1e-5 * float(dw1.norm())     # sums of 32-bit floats in another order
+    _, dw3, _ = ops.snn_cv_grad(gd, xd, wd, params, out, pt, pl, opts=_lib.options(dw_kernel=2))
+    assert torch.equal(dw2, dw3)
