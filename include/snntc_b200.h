@@ -248,7 +248,11 @@ SNNTC_API unsigned long long snntc_copy_timeouts(void);
  * not export these). The four operators with the kernel choice of THE CALL given explicitly, so that a
  * benchmark can time the kernels of an operator apart and a test can check the variants against each other:
  *   opts8 = { forward_parts   bit 0: build the sorted lists, bit 1: walk them (default 3; without bit 1 the
- *                             output is not written),
+ *                             output is not written). Bit 1 alone walks what a call with bit 0 alone has left in the
+ *                             same workspace: the lists, and beside them the bound on the weight sums that walks need
+ *                             and, for a fan-out that is no multiple of four, the weights with padded rows. So between
+ *                             the two calls the weights stay the same, and for such a fan-out walk_layout and
+ *                             walk_outputs, too (the lists name weight rows by their offsets),
  *             walk_layout     0 auto, 1 output pairs, 2 outputs lane+32m, 3 four consecutive outputs per lane, 8 output
  *                             pairs with the weights in shared memory, 16 weight rows copied ahead, 32 / 64 several rows
  *                             per warp (64: weights in shared memory), 128 a row per warp that copies its own weight rows

@@ -647,9 +647,10 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     // global memory is ahead too: 65 536 of 900 x 64 649, 672)
     if (g.jout == 64 && g.I >= 64 && g.R >= 32768) rows = false;
   }
-  // the walk's bound on the weight sums (see walk_tolerance_base), by up to 64 CTAs of 8192 weights and more beside the lists
+  // the walk's bound on the weight sums (see walk_tolerance_base), by up to 64 CTAs of 8192 weights and more beside the lists. (Lists
+  // without a walk: whatever walk the next call names may need it.)
   WeightBound wb = {w_in, g.I + g.has_bias, g.jout, g.J, wbound, pad ? w_padded : nullptr, 0};
-  if (!(ring || alone) || pad) {
+  if (!(ring || alone) || pad || !(fparts & 2)) {
     const long long n = (long long)wb.rows * g.J;
     wb.ctas = (int)(n < 64 * 8192 ? (n + 8191) / 8192 : 64);
     g.wbound_n = wb.ctas;

@@ -296,3 +296,26 @@ def test_warps_that_copy_for_themselves_by_name(I, J):
     xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
     ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
     assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=128)), ref)
+
+
+@pytest.mark.parametrize("J", [32, 64, 128])
+@pytest.mark.parametrize("first", [0, 16, 128])
+def test_lists_of_one_call_walked_by_the_next(J, first):
+    """Lists built without a walk (by a call whose own walk would need no bound on the weight sums), then walked in every layout from the
+    same workspace, with inputs so close together that many steps need the bound: the bits of both in one call."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    rng = np.random.default_rng(J)
+    R, I = 600, 300
+    x = np.exp(1e-3 * rng.random((R, I))).astype(np.float32)
+    w = (rng.standard_normal((I + 1, J)) * np.sqrt(15.0 / I) * 3e3).astype(np.float32)
+    w[I] = 0.0
+    params = O.fc_params(biasvolt=1.0)
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
+    ws = ops.fc_forward_workspace(R, I, J, xd.device)
+    ws.view(torch.int32).fill_(0)                     # a bound of zero, were none formed
+    ops.snn_fc(xd, wd, params, opts=_lib.options(forward_parts=1, walk_layout=first), workspace=ws)
+    for layout in (1, 2, 3, 8, 16, 32, 64, 128):
+        got = ops.snn_fc(xd, wd, params, opts=_lib.options(forward_parts=2, walk_layout=layout), workspace=ws)
+        assert torch.equal(got, ref), "layout %d" % layout
