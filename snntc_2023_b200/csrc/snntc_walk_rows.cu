@@ -6,8 +6,9 @@
 // the same bits as every other walk. Rows of one warp are neighbours (receptive
 // fields next to each other), so their lists are about equally long; behind the end of its list a row repeats its last input
 // with weight zero, which changes no sum and can fire nothing.
-// WS: all weights fit one CTA's shared memory (up to 180 KB: 700 rows of 64, 2 800 of 16): a persistent CTA of 32 warps per SM
-// holds them, since rows of 64 to 256 bytes picked at random miss the L1 cache beside everything else that goes through it.
+// WS: all weights fit one CTA's shared memory beside lists and sums (177 KB, 708 rows of 64; 161 KB, 2 576 of 16): a persistent CTA of
+// 32 warps per SM holds them, since rows of 64 to 256 bytes picked at random miss the L1 cache beside everything else that goes
+// through it.
 // What bounds it: instruction issue and the latency of a step's chain.
 // Measured (B200, walk alone): against the pairs walk 65 536 rows of 144 -> 16 inputs 123 -> 51 us, of 288 -> 32: 223 -> 131; 61 440
 // of 576 -> 48: 401 -> 346; 18 000 of 3136 -> 32: 1219 -> 743, all with scalar steps; with PairWalk 262 144 of 27 -> 64 265 -> 235 and
