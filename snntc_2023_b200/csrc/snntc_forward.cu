@@ -19,6 +19,7 @@
 
 #include <limits.h>
 #include <math.h>
+#include <algorithm>
 #include <math_constants.h>
 #include <type_traits>
 
@@ -232,14 +233,16 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
 // `ws_lane` is the shared-memory byte address of this lane's pair in row 0 and `wmul` = 256 / J (J = 64, 128 or 256): a
 // list entry's element offset (source index * J) times wmul is the row's byte offset in the slice -- one integer
 // multiply-add on the FMA pipe per weight read.
-// The list goes through shared memory 32 entries at a time (sbuf: two blocks), one coalesced read per lane issued a block ahead
-// instead of an L2 round trip per step. CH entries and their weight rows are read together.
-template <int P, int CH, bool FULL, bool WS = false>
+// The list goes through shared memory 32 entries at a time (sbuf: a block and the entry in front of it), one coalesced read per lane
+// issued a block ahead instead of an L2 round trip per step. CH entries and their weight rows are read together.
+constexpr int kPairsStage = 34;                   // entries staged per warp: 33, and to a multiple of 16 bytes
+
+template <int P, int CH, bool WS = false>
 __device__ __forceinline__ void walk_pairs(const Geometry& g, const WalkEntry* ents, int nvalid, const float* w, int jbase, int lane,
                                            float* __restrict__ y_row, float* __restrict__ inv_row, WalkEntry* __restrict__ sbuf,
                                            float* __restrict__ fin, unsigned ws_lane = 0u, unsigned wmul = 0u) {
   const int j0 = jbase + 2 * P * lane;                    // this lane's outputs: 2 * P from j0 on
-  const unsigned lane_off = (unsigned)(FULL || j0 < g.J ? j0 : g.J - 2 * P);
+  const unsigned lane_off = (unsigned)(jbase + 2 * P * (WS ? lane : min(lane, (g.J - jbase) / (2 * P) - 1)));   // (behind the row: its last)
   const char* wbase = reinterpret_cast<const char*>(w);
   // a 32-bit element offset from the (uniform) weight base, widened before the scaling to bytes: a 64-bit pointer per lane plus the
   // entry's offset takes two instructions more per step
@@ -262,7 +265,7 @@ __device__ __forceinline__ void walk_pairs(const Geometry& g, const WalkEntry* e
 #pragma unroll
     for (int m = 0; m < 2 * P; ++m) {   // the bias input (value biasvolt, weight row I) is always consumed first
       wb[m] = g.has_bias ? ld_plain(w + (size_t)g.I * g.J + lane_off + m) : 0.f;
-      ok[m] = FULL || j0 + m < g.jout;
+      ok[m] = WS || j0 + m < g.jout;
     }
     // (the smallest input is read by all lanes from one address: taken out of lane 0's entry below it cost a divergence check in
     // front of every vote)
@@ -270,24 +273,23 @@ __device__ __forceinline__ void walk_pairs(const Geometry& g, const WalkEntry* e
   }
   WalkEntry pre = make_uint2(0u, 0u);
   if (lane < nvalid) pre = ld_l2(ents + lane);
-  // entry k of the list is staged at k % 64, the input in front of the first one at 63
-  if (lane == 0) sbuf[63] = make_uint2(__float_as_uint(g.has_bias ? g.biasvolt : 0.f), 0u);
+  // entry k of the list is staged at k % 32, the one in front of the block at 32
+  if (lane == 0) sbuf[32] = make_uint2(__float_as_uint(g.has_bias ? g.biasvolt : 0.f), 0u);
   __syncwarp();                                           // (a row without spiking inputs goes straight on to reading it)
-  auto inputs = [&](int at) { return make_float2(__uint_as_float(sbuf[at].x), __uint_as_float(sbuf[(at + 63) & 63].x)); };
+  auto inputs = [&](int at) { return make_float2(__uint_as_float(sbuf[at].x), __uint_as_float(sbuf[at > 0 ? at - 1 : 32].x)); };
   bool flipped = false;
   auto block = [&](int base, auto flip_c) {
     constexpr bool FLIP = decltype(flip_c)::value;
     constexpr int N = FLIP ? 2 : CH;                      // (FLIP with four: the walk spills more, 4 % slower)
-    const int b = base & 32, nb = min(32, nvalid - base);
-    pw.margin(__uint_as_float(sbuf[b].x), __uint_as_float(sbuf[b + nb - 1].x));   // inputs ascend: |x| peaks at an end
+    const int nb = min(32, nvalid - base);
+    pw.margin(__uint_as_float(sbuf[0].x), __uint_as_float(sbuf[nb - 1].x));   // inputs ascend: |x| peaks at an end
     int kk = 0;
 #pragma unroll 1
     for (; kk + N <= nb; kk += N) {
-      const int at = b + kk;
       uint64_t x2[N], wv[N][P];
 #pragma unroll
       for (int u = 0; u < N; u += 2) {
-        const uint4 e2 = *reinterpret_cast<const uint4*>(sbuf + at + u);
+        const uint4 e2 = *reinterpret_cast<const uint4*>(sbuf + kk + u);
         x2[u] = pack2(__uint_as_float(e2.x), __uint_as_float(e2.x));
         load_row(e2.y, wv[u]);
         x2[u + 1] = pack2(__uint_as_float(e2.z), __uint_as_float(e2.z));
@@ -295,36 +297,37 @@ __device__ __forceinline__ void walk_pairs(const Geometry& g, const WalkEntry* e
       }
       if constexpr (FLIP) {
 #pragma unroll
-        for (int u = 0; u < N; ++u) pw.template step<true>(x2[u], wv[u], [&] { return inputs(at + u); });
+        for (int u = 0; u < N; ++u) pw.template step<true>(x2[u], wv[u], [&] { return inputs(kk + u); });
       } else {
 #pragma unroll
         for (int u = 0; u < N; u += 2)
-          pw.step2(x2[u], wv[u], x2[u + 1], wv[u + 1], [&] { return inputs(at + u); }, [&] { return inputs(at + u + 1); });
+          pw.step2(x2[u], wv[u], x2[u + 1], wv[u + 1], [&] { return inputs(kk + u); }, [&] { return inputs(kk + u + 1); });
       }
     }
 #pragma unroll 1
     for (; kk < nb; ++kk) {
-      const WalkEntry e = sbuf[b + kk];
+      const WalkEntry e = sbuf[kk];
       uint64_t wv[P];
       load_row(e.y, wv);
-      pw.template step<FLIP>(pack2(__uint_as_float(e.x), __uint_as_float(e.x)), wv, [&] { return inputs(b + kk); });
+      pw.template step<FLIP>(pack2(__uint_as_float(e.x), __uint_as_float(e.x)), wv, [&] { return inputs(kk); });
     }
-    flipped = pw.template flip<FLIP>(__uint_as_float(sbuf[b + nb - 1].x));
+    flipped = pw.template flip<FLIP>(__uint_as_float(sbuf[nb - 1].x));
   };
   for (int base = 0; base < nvalid; base += 32) {
-    __syncwarp();                                         // (the block in front has read the last input of the one that goes)
-    sbuf[(base & 32) + lane] = pre;
+    __syncwarp();                                         // (every lane is through with the block that goes)
+    if (lane == 31 && base > 0) sbuf[32] = sbuf[31];      // (that lane's own store)
+    sbuf[lane] = pre;
     __syncwarp();
     if (base + 32 + lane < nvalid) pre = ld_l2(ents + base + 32 + lane);
     if (__builtin_expect(flipped, 0)) block(base, std::true_type{});
     else block(base, std::false_type{});
     if (pw.done()) break;   // every output has fired
   }
-  const float xprev = __uint_as_float(sbuf[(nvalid + 63) & 63].x);
+  const float xprev = __uint_as_float(sbuf[nvalid > 0 ? (nvalid - 1) & 31 : 32].x);
 #pragma unroll
   for (int m = 0; m < 2 * P; ++m) {
     const int j = j0 + m;
-    if (!FULL && j >= g.jout) continue;
+    if (!WS && j >= g.jout) continue;
     float y, inv;
     pw.finish(g, m, xprev, y, inv);
     y_row[j] = y;
@@ -371,15 +374,14 @@ snn_walk_pairs_kernel(const Geometry g, const WalkEntry* keys_g, const int* nval
                       float* __restrict__ out) {
   chain_wait();
   chain_next();
-  __shared__ __align__(16) WalkEntry stage[kFwdWarps * 64];   // two blocks of 32 list entries per warp
+  __shared__ __align__(16) WalkEntry stage[kFwdWarps * kPairsStage];
   __shared__ float fins[kFwdWarps * PairWalk<P>::kFloats];
   constexpr int CH = P == 2 ? 4 : 8;
-  WalkEntry* sbuf = stage + (threadIdx.x >> 5) * 64;
+  WalkEntry* sbuf = stage + (threadIdx.x >> 5) * kPairsStage;
   float* fin = fins + (threadIdx.x >> 5) * PairWalk<P>::kFloats;
   const int J = g.jout, R = g.R;
   const int lane = threadIdx.x & 31;
   const int jchunks = (J + 64 * P - 1) / (64 * P);
-  const bool full_j = (J % (64 * P)) == 0;
   float* __restrict__ y_out = out;
   float* __restrict__ inv_out = g.infer ? nullptr : out + (size_t)R * J;
   const long items = (long)R * jchunks;
@@ -390,8 +392,7 @@ snn_walk_pairs_kernel(const Geometry g, const WalkEntry* keys_g, const int* nval
     const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     float* yr = y_out + (size_t)r * J;
     float* ir = inv_out ? inv_out + (size_t)r * J : nullptr;
-    if (full_j) walk_pairs<P, CH, true>(g, krow, n, w, jc * 64 * P, lane, yr, ir, sbuf, fin);
-    else walk_pairs<P, CH, false>(g, krow, n, w, jc * 64 * P, lane, yr, ir, sbuf, fin);
+    walk_pairs<P, CH>(g, krow, n, w, jc * 64 * P, lane, yr, ir, sbuf, fin);
     __syncwarp();   // the next row's first block goes into the buffer this row may have read last
   }
 }
@@ -402,8 +403,10 @@ snn_walk_pairs_kernel(const Geometry g, const WalkEntry* keys_g, const int* nval
 // (cp.async.bulk) per weight row, all completing on one mbarrier -- and every step of every walk then reads its
 // weight pair with one shared-memory load instead of a global load through L1. CTA c takes output slice
 // c % (J/64) and every (gridDim.x / (J/64))-th row of that slice.
+// Where that leaves less room than 32 warps need beside it (from 803 rows on), the CTA has fewer.
 constexpr int kSmemwThreads = 1024;
-constexpr int kSmemwWarps = kSmemwThreads / 32;
+constexpr size_t kSmemwFewest = 20;                    // warps
+constexpr size_t kSmemwWarpBytes = kPairsStage * sizeof(WalkEntry) + PairWalk<1>::kFloats * sizeof(float);
 constexpr long long kSmemwWaitClocks = 2000000000LL;   // SM clocks a CTA waits for its weight copies (about a second)
 __device__ unsigned g_walk_copy_timeouts = 0u;          // CTAs that gave up waiting since the library was loaded
 
@@ -417,8 +420,9 @@ snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nva
   const int J = g.J, R = g.R;
   const int rows_w = g.I + g.has_bias;
   float* ws = reinterpret_cast<float*>(smem_raw);                                        // [rows_w][64]
-  WalkEntry* stage = reinterpret_cast<WalkEntry*>(smem_raw + (size_t)rows_w * 256);      // [32 warps][64 entries]
-  float* fins = reinterpret_cast<float*>(stage + kSmemwWarps * 64);                      // [32 warps][PairWalk<1>::kFloats]
+  const int warps = blockDim.x >> 5;
+  WalkEntry* stage = reinterpret_cast<WalkEntry*>(smem_raw + (size_t)rows_w * 256);      // [warps][kPairsStage]
+  float* fins = reinterpret_cast<float*>(stage + warps * kPairsStage);                   // [warps][PairWalk<1>::kFloats]
   const int lane = threadIdx.x & 31;
   const int warp = uniform_warp_index();
   const int slices = J >> 6;
@@ -458,20 +462,20 @@ snn_walk2_smemw_kernel(const Geometry g, const WalkEntry* keys_g, const int* nva
   const bool staged = !__syncthreads_or(!copies_arrived());
   if (!staged && threadIdx.x == 0) atomicAdd(&g_walk_copy_timeouts, 1u);
 
-  WalkEntry* sbuf = stage + warp * 64;
+  WalkEntry* sbuf = stage + warp * kPairsStage;
   float* fin = fins + warp * PairWalk<1>::kFloats;
   float* __restrict__ y_out = out;
   float* __restrict__ inv_out = g.infer ? nullptr : out + (size_t)R * J;
   const unsigned ws_lane = smem_u32(ws) + 8u * (unsigned)lane;
   const int ctas = gridDim.x / slices;                 // CTAs that share this slice (the host makes gridDim.x a multiple)
   const int cta = blockIdx.x / slices;
-  for (int r = cta * kSmemwWarps + warp; r < R; r += ctas * kSmemwWarps) {
+  for (int r = cta * warps + warp; r < R; r += ctas * warps) {
     const WalkEntry* krow = keys_g + (size_t)r * istride;
     const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     float* yr = y_out + (size_t)r * J;
     float* ir = inv_out ? inv_out + (size_t)r * J : nullptr;
-    if (staged) walk_pairs<1, 8, true, true>(g, krow, n, w, j0, lane, yr, ir, sbuf, fin, ws_lane, wmul);
-    else walk_pairs<1, 8, true, false>(g, krow, n, w, j0, lane, yr, ir, sbuf, fin);
+    if (staged) walk_pairs<1, 8, true>(g, krow, n, w, j0, lane, yr, ir, sbuf, fin, ws_lane, wmul);
+    else walk_pairs<1, 8>(g, krow, n, w, j0, lane, yr, ir, sbuf, fin);
     __syncwarp();
   }
   if (!staged) {
@@ -511,28 +515,29 @@ int launch_walk_pairs(const Geometry& g, const WalkEntry* keys_g, const int* nva
 
 // The pairs walk with the weights staged in shared memory: fan-out a power-of-two multiple of 64, weights 16-byte
 // aligned, all (I + bias) rows of a 64-output slice plus the list staging buffers within one CTA's shared memory.
-bool walk_smemw_ok(const Geometry& g, const float* w, const LaunchInfo& li, size_t* smem_bytes, int* wmul) {
+bool walk_smemw_ok(const Geometry& g, const float* w, const LaunchInfo& li, int* warps, int* wmul) {
   if ((g.J != 64 && g.J != 128 && g.J != 256) || (reinterpret_cast<uintptr_t>(w) & 15) != 0) return false;
   if (g.jout != g.J) return false;      // J is the kernel's output stride too
   const size_t rows_w = (size_t)g.I + g.has_bias;
-  const size_t smem = rows_w * 256 + (size_t)kSmemwWarps * (64 * sizeof(WalkEntry) + PairWalk<1>::kFloats * sizeof(float));
-  if (smem + 2048 > (size_t)li.max_smem_optin || rows_w * 256 >= (1u << 20)) return false;
+  const size_t room = (size_t)li.max_smem_optin - 2048;
+  if (rows_w * 256 + kSmemwFewest * kSmemwWarpBytes > room) return false;
   if ((g.J >> 6) > li.num_sms) return false;
-  *smem_bytes = smem;
+  *warps = (int)std::min<size_t>(kSmemwThreads / 32, (room - rows_w * 256) / kSmemwWarpBytes);
   *wmul = 256 / g.J;
   return true;
 }
 
 int launch_walk2_smemw(const Geometry& g, const WalkEntry* keys_g, const int* nvalid_g, const float* w, float* out,
-                       const LaunchInfo& li, cudaStream_t s, size_t smem, int wmul) {
+                       const LaunchInfo& li, cudaStream_t s, int warps, int wmul) {
   const int slices = g.J >> 6;
   long per_slice = li.num_sms / slices;                       // persistent: one CTA per SM
-  const long need = ((long)g.R + kSmemwWarps - 1) / kSmemwWarps;
+  const long need = ((long)g.R + warps - 1) / warps;
   if (per_slice > need) per_slice = need;
   if (per_slice < 1) per_slice = 1;
   const int grid = (int)(per_slice * slices);
+  const size_t smem = ((size_t)g.I + g.has_bias) * 256 + warps * kSmemwWarpBytes;
   if (allow_smem<snn_walk2_smemw_kernel>(smem) != cudaSuccess) return E_CUDA;
-  (void)launch_chained(snn_walk2_smemw_kernel, grid, kSmemwThreads, smem, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, (unsigned)wmul);
+  (void)launch_chained(snn_walk2_smemw_kernel, grid, 32 * warps, smem, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out, (unsigned)wmul);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
@@ -671,20 +676,19 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   const int named = opt.walk_layout & 3;
   if (named == 2 || (named == 1 && al8) || (named == 3 && al16)) variant = named;
   if (opt.walk_outputs >= 1 && opt.walk_outputs <= 3) lanes = opt.walk_outputs - 1;
-  size_t smemw_bytes = 0;
-  int smemw_shift = 0;
+  int smemw_warps = 0, smemw_mul = 0;
   // weights staged in shared memory: where they fit, for fan-out 64 with enough rows to keep one CTA of 32 warps
   // per SM busy (measured 13-16 % faster than the global-memory pairs walk; at fan-out 128 four outputs per lane
   // from global memory are 5 % faster than two staged slices); walk_layout 8 asks for it wherever it fits, a named
   // layout switches it off
-  const bool smemw = walk_smemw_ok(g, w, li, &smemw_bytes, &smemw_shift) &&
+  const bool smemw = walk_smemw_ok(g, w, li, &smemw_warps, &smemw_mul) &&
                      ((opt.walk_layout & 8) != 0 || ((opt.walk_layout & 3) == 0 && g.J == 64 && g.R >= 32768));
   auto walk = [&]() -> int {
     if (!(fparts & 2)) return OK;
     if (alone) return launch_walk_alone(g, keys_g, nvalid_g, key_stride(g), w, out, s);
     if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, li, s);
     if (rows) return launch_walk_rows(g, keys_g, nvalid_g, key_stride(g), w, out, own ? g.J > 32 && g.R >= 32768 : (opt.walk_layout & 64) != 0, li, s);
-    if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, s, smemw_bytes, smemw_shift);
+    if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, s, smemw_warps, smemw_mul);
     if (variant == 1) return launch_walk_pairs<1>(g, keys_g, nvalid_g, w, out, s);
     if (variant == 3) return launch_walk_pairs<2>(g, keys_g, nvalid_g, w, out, s);
     if (lanes == 0) return launch_walk<1>(g, keys_g, nvalid_g, w, out, s);

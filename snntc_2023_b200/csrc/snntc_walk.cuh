@@ -56,8 +56,8 @@ __device__ __forceinline__ int imin3(int a, int b, int c) { return min(min(a, b)
 // comparisons (exact()); if it does not fire there, so is every output of the lane at the next step (`again`), and so is the first
 // step of a row. Rows for which X is no bound (an input below zero, a NaN, or sums that may overflow: `careful`) take the
 // comparisons whenever q <= tol. An output that has fired is parked at n = +inf: q = +inf (x > 0) or a positive NaN (x = 0) from
-// then on, or a NaN of either sum behind a weight that is no number, which is no spike either. Its sums wait in shared memory: as
-// registers they took the walk beyond its 64.
+// then on, or a NaN behind a weight that is infinite or NaN, where nothing fires again either. So n tells who need not be waited for,
+// and whether there is a spike to write is read beside its sums, in shared memory (as registers they took the walk beyond its 64).
 //
 // An output may also cross zero without firing (the two rounded comparisons of the reference can both miss it, about once in 10^5
 // spikes) and then stays below, taking its row through the comparisons at every step: twice the time of its neighbours, and where
@@ -74,7 +74,7 @@ struct PairWalk {
   static constexpr int kFloats = 128 * P;   // of shared memory per warp
   uint64_t n[P], ys[P];
   float* fin;       // this lane's column of [2 * P][2][32] floats: an output's sums once it has fired; until then the sign that its
-                    // running sums carry, and a NaN (see fired)
+                    // running sums carry, and a NaN (the sums of a spike are numbers: both ways to it have compared them)
   float tolbase, xmag;
   int qlim;         // bits of tol, or INT_MAX: every output of this lane goes to the comparisons at the next step
   int qtol;         // bits of tol
@@ -95,7 +95,7 @@ struct PairWalk {
         const int m = 2 * p + h;
         nn[h] = ok[m] ? g.theta - wb[m] : CUDART_INF_F;   // (no output: parked, or the walk would wait for it)
         yy[h] = g.has_bias ? g.biasvolt * wb[m] : 0.f;
-        fin[64 * m] = 1.f; fin[64 * m + 32] = ok[m] ? CUDART_NAN_F : 0.f;
+        fin[64 * m] = 1.f; fin[64 * m + 32] = CUDART_NAN_F;
       }
       n[p] = pack2(nn[0], nn[1]);
       ys[p] = pack2(yy[0], yy[1]);
@@ -107,10 +107,7 @@ struct PairWalk {
     qtol = __float_as_int(tolbase * (b <= a ? a : b));     // (a NaN for a NaN at the end of the list)
     if (qlim != INT_MAX) qlim = qtol;
   }
-  // Whether output m has fired. The sums of a spike are numbers: one of the two ways to it has compared them. The parked n tells nothing:
-  // a weight that is infinite or NaN takes it from +inf to NaN, and a sum may overflow to +inf without a spike.
-  __device__ __forceinline__ bool fired(int m) const { return fin[64 * m + 32] == fin[64 * m + 32]; }
-  // Has every output of the warp fired? Asked once per block of entries: the parked n says no in passing, shared memory has the word.
+  // no output of the warp may fire any more (one whose weight sum has overflowed to -inf cannot)
   __device__ __forceinline__ bool done() const {
     bool live = false;
 #pragma unroll
@@ -119,9 +116,6 @@ struct PairWalk {
       unpack2(n[p], a, b);
       live |= (a != CUDART_INF_F) | (b != CUDART_INF_F);
     }
-    if (__any_sync(0xffffffffu, live)) return false;
-#pragma unroll
-    for (int m = 0; m < 2 * P; ++m) live |= !fired(m);
     return !__any_sync(0xffffffffu, live);
   }
 
@@ -189,11 +183,12 @@ struct PairWalk {
     form_q(pack2(xprev, xprev), n, ys, q);
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-      float s[2];
+      float nn[2], s[2];
+      unpack2(n[p], nn[0], nn[1]);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const float qm = __int_as_float(q[2 * p + h]);
-        const bool live = !fired(2 * p + h), below = look & live & (qm < -tol);
+        const bool live = nn[h] != CUDART_INF_F, below = look & live & (qm < -tol);
         s[h] = below ? -1.f : 1.f;
         if (below) fin[64 * (2 * p + h)] *= -1.f;
         any |= below;
@@ -214,13 +209,13 @@ struct PairWalk {
     unpack2(n[m / 2], nn[0], nn[1]);
     unpack2(ys[m / 2], yy[0], yy[1]);
     float a = fin[64 * m], ws = 0.f - a, yv = fin[64 * m + 32];
-    bool spike = true;
-    if (!fired(m)) {
+    bool fired = true;
+    if (yv != yv) {
       ws = 0.f - a * nn[m & 1]; yv = a * yy[m & 1];
-      spike = ratio_gt(yv, ws, xprev);
+      fired = (nn[m & 1] != CUDART_INF_F) & ratio_gt(yv, ws, xprev);
     }
     y = g.maxv; inv = 0.f;
-    if (spike) {
+    if (fired) {
       inv = __fdividef(1.0f, ws);
       y = yv * inv;
       if (y >= g.maxv) { y = g.maxv; inv = 0.f; }
@@ -271,23 +266,24 @@ struct PairWalk {
     }
     if (__any_sync(0xffffffffu, !(near > tol))) {
       const float2 xx = inputs();
-      exact<FLIP>(q, n0, ys0, n1, xx.x, xx.y);
+      exact<FLIP>(q, tol, n0, ys0, n1, xx.x, xx.y);
     }
   }
-  // the reference's own comparisons, for all outputs of the lanes concerned
+  // the reference's own comparisons, for all outputs of the lanes concerned that have not fired
   template <bool FLIP>
-  __device__ __forceinline__ void exact(const int (&q)[2 * P], const uint64_t (&n0)[P], const uint64_t (&ys0)[P], uint64_t (&n1)[P],
+  __device__ __forceinline__ void exact(const int (&q)[2 * P], float tol, const uint64_t (&n0)[P], const uint64_t (&ys0)[P], uint64_t (&n1)[P],
                                         float x, float xp) {
     bool again = false;
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-      float nn[2], yy[2], park[2] = {0.f, 0.f};
+      float nn[2], yy[2], before[2], park[2] = {0.f, 0.f};
       sums<FLIP>(n0, ys0, p, nn, yy);
+      unpack2(n0[p], before[0], before[1]);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int m = 2 * p + h;
         if (!__any_sync(0xffffffffu, q[m] <= qlim)) continue;
-        const bool live = !fired(m);
+        const bool live = (before[h] != CUDART_INF_F) & !(__int_as_float(q[m]) < -tol);   // (below: parked by hit())
         const float wsum = 0.f - nn[h];
         const bool fire = live & ratio_gt(yy[h], wsum, xp) & ratio_le(yy[h], wsum, x);
         park[h] = fire ? CUDART_INF_F : 0.f;
