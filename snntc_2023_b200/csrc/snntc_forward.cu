@@ -657,7 +657,8 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   WeightBound wb = {w_in, g.I + g.has_bias, g.jout, g.J, wbound, pad ? w_padded : nullptr, 0};
   if (!(ring || alone) || pad || !(fparts & 2)) {
     const long long n = (long long)wb.rows * g.J;
-    wb.ctas = (int)(n < 64 * 8192 ? (n + 8191) / 8192 : 64);
+    const long long ctas = std::max((n + 8191) / 8192, (wb.rows + 31LL) / 32);    // (32 rows of a few weights are as long as 8192 weights)
+    wb.ctas = (int)std::min(ctas, 64LL);
     g.wbound_n = wb.ctas;
   }
   // Variants of the walk from global memory: 1 = output pairs in 64-bit registers, 64 outputs per warp; 3 = four consecutive outputs
