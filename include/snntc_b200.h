@@ -255,8 +255,8 @@ SNNTC_API unsigned long long snntc_copy_timeouts(void);
  *                             walk_outputs, too (the lists name weight rows by their offsets),
  *             walk_layout     0 auto, 1 output pairs, 2 outputs lane+32m, 3 four consecutive outputs per lane, 8 output
  *                             pairs with the weights in shared memory, 16 weight rows copied ahead, 32 / 64 several rows
- *                             per warp (64: weights in shared memory), 128 a row per warp that copies its own weight rows
- *                             (fan-out up to 32); a layout that the weights do not allow: auto,
+ *                             per warp (64: weights in shared memory), 128 / 256 weight rows copied ahead by every
+ *                             warp for itself, 16 / 32 entries to a block; a layout that the weights do not allow: auto,
  *             walk_outputs    outputs per lane of layout 2: 0 auto, 1..3: 1, 2, 4,
  *             list_builder    0 auto, 1 per-row bucket sort, 2 per-pixel sort + merges, 3 register network (up to 64
  *                             inputs); + 4*(k+1): merges cut into 2^k pieces,

@@ -49,8 +49,8 @@ struct Options {
                             // 8: output pairs with the weights staged in shared memory (where they fit)
                             // 16: one output per lane, the warp's weight rows copied ahead into shared memory
                             // 32, 64: several rows per warp (fan-out <= 64, a multiple of 4), weights from global memory /
-                            // in shared memory where they fit. 128: a row per warp that copies its own weight rows
-                            // (fan-out <= 32). A layout that the weights do not allow: auto
+                            // in shared memory where they fit. 128, 256: weight rows copied ahead by every
+                            // warp for itself, 16 / 32 entries to a block. A layout that the weights do not allow: auto
   int walk_outputs = 0;     // outputs per lane of layout 2: 0 auto, 1..3: 1, 2, 4
   int list_builder = 0;     // 0 auto, 1 per-row bucket sort, 2 per-pixel sort + merges (3x3 stride-1 conv only),
                             // 3 per-row sorting network in registers (rows of at most 64 inputs);
@@ -119,12 +119,21 @@ size_t merge_lists_bytes(const Geometry& g);
 int launch_merge_lists(const Geometry& g, const float* x, WalkEntry* lists, int* nvalid, int istride,
                        void* scratch, int split_log2, const WeightBound& wb, const LaunchInfo& li, cudaStream_t s);
 
-// The walk of one row per warp that copies its own weight rows ahead (snntc_walk_alone.cu): J <= 32, J % 4 == 0, w 16-byte aligned.
+// The walk of 32 outputs per warp that copies its own weight rows ahead (snntc_walk_alone.cu): J % 4 == 0, w 16-byte aligned. large:
+// blocks of 32 entries instead of 16. list_ctas, here and below: CTAs of the kernel in front (see walk_chains).
 int launch_walk_alone(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
-                      cudaStream_t s);
+                      bool large, int list_ctas, const LaunchInfo& li, cudaStream_t s);
 // The walk with one output per lane and weight rows copied ahead into shared memory (snntc_walk_ring.cu); any shape.
 int launch_walk_ring(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
-                     const LaunchInfo& li, cudaStream_t s);
+                     int list_ctas, const LaunchInfo& li, cudaStream_t s);
+// Whether a walk of few warps is launched as a dependent of the kernel that builds its lists: where most of its CTAs find an SM that
+// kernel does not use. Otherwise they wait for the first SMs to be free of it and crowd there, on few SMs, for the whole of their serial
+// chains. Us, dependent and in plain order, rows of 2000 inputs, CTAs beside those of the lists: CTAs of one walking and one copying warp,
+// 148 beside 148 44, 23, 148 beside 74 21.8, 22.9, 148 beside 37 21.3, 21.7; of two walking warps, 148 beside 74 26.6, 23.6; of two warps
+// that copy for themselves, 74 beside 148 82, 38, 37 beside 74 36, 37. small: CTAs of the first kind.
+inline bool walk_chains(long ctas, int list_ctas, bool small, const LaunchInfo& li) {
+  return 2 * (ctas + list_ctas) <= (small ? 3L : 2L) * li.num_sms;
+}
 
 // The walk with several rows per warp (snntc_walk_rows.cu): fan-out up to 64 and a multiple of four, weights 16-byte aligned;
 // reads g.wbound. resident: weights in shared memory where they fit.

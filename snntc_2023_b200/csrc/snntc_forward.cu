@@ -608,15 +608,6 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   const int istride = key_stride(g);
 
   const int fparts = opt.forward_parts;
-  // The walk that copies its weight rows ahead, up to two waves of its CTAs of 64 outputs (six to an SM; eight items of 32 outputs per
-  // SM where the rows have to be copied 4 bytes at a time and for fan-out up to 16; one wave, ten items, for fan-out 17 to 32): with
-  // few warps on an SM latency is what counts, with many the instructions per output. Against the pairs walk, us: 784 -> 400 200 rows
-  // 29, 35, 300 rows 41, 37; 1000 -> 1000 80 rows 33, 43, 120 rows 46, 45; 576 -> 128 1000 rows (13.5 CTAs per SM) 33, 31; 1152 ->
-  // 128 700 rows 37, 47, 1500 72, 67; 4096 -> 512 still 172, 199 at 300 rows (16 per SM); 576 -> 32 1000 rows 23, 25, 2000 40, 27;
-  // 1500 -> 16 1000 rows 47, 53, 2000 83, 50.
-  // Fan-out 17 to 32 beyond that, up to one wave of it (24 rows per SM): the walk whose warps copy for themselves. Copying warp, each
-  // for itself, pairs walk, us: 2304 -> 32 1200 rows 40, 46, 69, 1500 rows 50, 48, 70, 3500 rows 98, 77, 91, 4500 rows 118, 116, 116;
-  // 576 -> 32 1200 rows 16, 18, 21, 2600 rows 28, 24, 25, 4500 rows 42, 37, 34; 2304 -> 20 2600 rows 75, 65, 81.
   g.jout = g.J;
   const bool own = opt.walk_layout == 0 && opt.walk_outputs == 0;    // the library's own choice
   const long ring_items = (long)g.R * ((g.J + 31) / 32);
@@ -625,7 +616,10 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   // 200 -> 501: 14 -> 12), the weights are copied with padded rows (by the kernel that reads them for the bound), so that every
   // walk reads them 16 bytes at a time. Up to 16 outputs a 4-byte copy brings two rows or more, which keeps up with the walk.
   const int jp = (g.J + 3) & ~3;
-  const bool pad = own && jp != g.J && (ring_items > 8L * li.num_sms || (g.I >= 200 && g.J > 16)) && (long long)(g.I + 1) * jp <= INT_MAX;
+  // (from six items per SM on, four at up to 64 inputs: 800 to 1184 rows of 40 -> 10 6.2 to 6.3 us so, 6.5 to 7.1 by 4-byte copies, of
+  // 400 -> 10 14.7 to 15.7, 14.2 to 16.6)
+  const long pad_line = (g.J > 32 ? 8 : (g.I <= 64 ? 4 : 6)) * (long)li.num_sms;
+  const bool pad = own && jp != g.J && (ring_items > pad_line || (g.I >= 200 && g.J > 16)) && (long long)(g.I + 1) * jp <= INT_MAX;
   const float* const w_in = w;
   float* const w_padded = reinterpret_cast<float*>(static_cast<unsigned char*>(ws) + padded_weights_at(g_in));
   if (pad) {
@@ -633,10 +627,32 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
     g.J = jp;
   }
   const bool copies16 = (g.J & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
-  const bool few = copies16 && g.J > 32 ? (long)g.R * ((g.J + 63) / 64) <= 12L * li.num_sms : ring_items <= (copies16 && g.J > 16 ? 10L : 8L) * li.num_sms;
+  // With few warps on an SM latency is what counts, with many the instructions per output. In turn:
+  //   - the walk with a copying warp while its CTAs are one wave: six to an SM with two walking warps, four with four (784 -> 128, 592 rows
+  //     27.6 us, each warp copying for itself 29.8, pairs walk 39; 740 rows, beyond, 35.3, 33.6, 41), for long lists two waves (4096 -> 256, 370
+  //     rows 117, 123, 130; 2000 -> 256, 333 rows 64, 65, 70). For fan-outs up to 32, where a CTA is one walking warp and the copying one, up
+  //     to six items (rows) per SM (784 -> 32, 888 rows 20.9, 24.4 and in blocks of 32 entries 22.0; 1184 rows 24.8, 25.6, 23.8), fewer where
+  //     lists are short, for it takes longer to begin, and where rows are no whole sectors, since it copies past L1 (200 -> 24, 888 rows 12.2,
+  //     12.2, 11.4; 40 -> 12, 592 rows 6.8, 5.8, 5.5; 40 -> 128, 592 rows 7.8, 6.7). Eight items where rows have to be copied 4 bytes at a time.
+  //   - the walk whose warps copy for themselves, up to 24 items of 32 outputs per SM (21 at 300 to 1200 inputs; 784 -> 400 input spikes, 250
+  //     rows, 22 items, 65, pairs walk 51; 100 -> 400, 273 rows, 24 items, 12.4, 14.0, 319 rows 14.0, 14.3), in blocks of 32 entries up to one wave of
+  //     those (16 items) where lists are not short or the fan-out is not above 32 (2000 -> 64, 1036 rows 60, in blocks of 16 64; 400 -> 16, 1480 rows
+  //     19.5, 20.5, pairs walk 51, 2960 rows (20 items) 30.1, 25.8, 37; 40 -> 256, 296 rows 8.0, 6.7).
+  const long sms = li.num_sms;
+  long line = 6;                                       // rows per SM of the walk with a copying warp at fan-outs up to 32
+  if (g.I <= 64) line = (g.J & 7) ? 1 : 4;
+  else if (g.I <= 256) line = (g.J & 7) ? 3 : 5;
+  bool few = ring_items <= (copies16 ? line : 8) * sms;
+  if (copies16 && g.J > 32) {
+    const long pairs_of_warps = (long)g.R * ((g.J + 63) / 64);
+    few = pairs_of_warps <= 6 * sms || (long)g.R * ((g.J + 127) / 128) <= 4 * sms;
+    if (g.I <= 64) few = few && ring_items <= 10 * sms;
+    if (g.I > 1200) few = few || (ring_items > 16 * sms && pairs_of_warps <= 12 * sms);
+  }
   const bool ring = (opt.walk_layout & 16) != 0 || (own && few);
-  const bool alone = copies16 && g.J <= 32 && ((opt.walk_layout & 128) != 0 ||
-                                               (own && !ring && g.J > 16 && ring_items <= 24L * li.num_sms));
+  const long most = (g.J > 32 && g.I > 300 && g.I <= 1200 ? 21 : 24) * sms;
+  const bool alone = copies16 && ((opt.walk_layout & 384) != 0 || (own && !ring && ring_items <= most));
+  const bool large = own ? ring_items <= 16 * sms && (g.J <= 32 || g.I > 400) : (opt.walk_layout & 256) != 0;
   // Several rows per warp for fan-out up to 64, where that leaves enough warps: 5 per SM at eight rows to a warp (fan-out 16;
   // 10 where the weights miss the L1 cache), 11 at four (32), 40 at two (64). With fewer the pairs walk, a warp per row, hides
   // its latencies better. Pairs against rows, us: 576 -> 16 4000 rows 35, 39, 7000 rows 53, 39; 576 -> 32 35, 37 and 54, 43; 147 -> 64 8000
@@ -684,10 +700,12 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   // layout switches it off
   const bool smemw = walk_smemw_ok(g, w, li, &smemw_warps, &smemw_mul) &&
                      ((opt.walk_layout & 8) != 0 || ((opt.walk_layout & 3) == 0 && g.J == 64 && g.R >= 32768));
+  // CTAs of the last kernel that builds the lists: eight rows each (sorting network), one row each (bucket sort of few rows), many
+  const int list_ctas = use_merge_lists(g, opt, li) ? li.num_sms : (use_small_rows(g, opt) ? (g.R + 7) / 8 : g.R) + wb.ctas;
   auto walk = [&]() -> int {
     if (!(fparts & 2)) return OK;
-    if (alone) return launch_walk_alone(g, keys_g, nvalid_g, key_stride(g), w, out, s);
-    if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, li, s);
+    if (alone) return launch_walk_alone(g, keys_g, nvalid_g, key_stride(g), w, out, large, list_ctas, li, s);
+    if (ring) return launch_walk_ring(g, keys_g, nvalid_g, key_stride(g), w, out, list_ctas, li, s);
     if (rows) return launch_walk_rows(g, keys_g, nvalid_g, key_stride(g), w, out, own ? g.J > 32 && g.R >= 32768 : (opt.walk_layout & 64) != 0, li, s);
     if (smemw) return launch_walk2_smemw(g, keys_g, nvalid_g, w, out, li, s, smemw_warps, smemw_mul);
     if (variant == 1) return launch_walk_pairs<1>(g, keys_g, nvalid_g, w, out, s);

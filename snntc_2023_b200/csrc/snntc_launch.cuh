@@ -51,9 +51,18 @@ __device__ __forceinline__ float ld_stream(const float* p) {
   return v;
 }
 
+// A grid, and whether it may be launched as a dependent (the kernel is written for it either way).
+struct ChainGrid {
+  dim3 grid;
+  bool chain = true;
+  ChainGrid(dim3 d) : grid(d) {}
+  ChainGrid(unsigned x, bool may_chain = true) : grid(x), chain(may_chain) {}
+};
+
 template <typename... Params, typename... Args>
-cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, unsigned cluster,
+cudaError_t launch_chained(void (*kernel)(Params...), ChainGrid where, dim3 block, size_t smem, cudaStream_t s, unsigned cluster,
                            Args... args) {
+  const dim3 grid = where.grid;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -61,7 +70,7 @@ cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, siz
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
-  if ((long)grid.x * grid.y * grid.z * (long)(block.x * block.y * block.z) <= kChainThreads) {
+  if (where.chain && (long)grid.x * grid.y * grid.z * (long)(block.x * block.y * block.z) <= kChainThreads) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
   }

@@ -18,11 +18,10 @@ namespace snntc {
 namespace {
 
 constexpr int kWarps = 2;                          // per CTA, each on a row of its own
-constexpr int kBlock = 16;                         // list entries
-constexpr int kGroup = 8;                          // steps per vote
 constexpr int kRing = 3;                           // weight blocks per warp: one consumed, two on their way
 constexpr int kListRing = 4;                       // list blocks per warp
 
+template <int kBlock>                              // list entries
 struct RingWarp {
   float w[kRing][kBlock][32];
   float x[kListRing][kBlock];
@@ -34,18 +33,21 @@ __device__ __forceinline__ void copy_async(unsigned dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
+template <int kBlock>
 __global__ void __launch_bounds__(32 * kWarps)
 snn_walk_alone_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid, int istride, const float* w,
-                      float* __restrict__ out) {
+                      float* __restrict__ out, int slices) {
   chain_wait();
   chain_next();
-  __shared__ __align__(16) RingWarp ring[kWarps];
+  constexpr int kGroup = kBlock / 2;               // steps per vote
+  __shared__ __align__(16) RingWarp<kBlock> ring[kWarps];
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
-  RingWarp& sm = ring[warp];
+  RingWarp<kBlock>& sm = ring[warp];
   const int J = g.J;
+  // neighbouring items are rows of the same output slice: the slice's weights stay in L2 while they run
   const long item = (long)blockIdx.x * kWarps + warp;
-  if (item >= g.R) return;
-  const int r = (int)item;
+  if (item >= (long)g.R * slices) return;
+  const int r = (int)(item % g.R), j0 = (int)(item / g.R) * 32;
   const WalkEntry* ents = lists + (size_t)r * istride;
   const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid + r), 0);
   const int blocks = (n + kBlock - 1) / kBlock;
@@ -55,18 +57,18 @@ snn_walk_alone_kernel(const Geometry g, const WalkEntry* lists, const int* nvali
   WalkEntry pre = make_uint2(0u, 0u);
   auto read_list = [&](int b) {
     pre = make_uint2(0u, 0u);
-    if (lane < kBlock && b * kBlock + lane < n) pre = ld_l2(ents + b * kBlock + lane);
+    if ((kBlock == 32 || lane < kBlock) && b * kBlock + lane < n) pre = ld_l2(ents + b * kBlock + lane);
   };
   auto put_list = [&](int b) {
-    if (lane < kBlock) {
+    if (kBlock == 32 || lane < kBlock) {
       sm.x[b % kListRing][lane] = __uint_as_float(pre.x);
       sm.off[b % kListRing][lane] = pre.y;
     }
   };
   // weight block b: a copy brings four rows, 16 bytes per lane (lanes behind the row copy nothing)
   const int sub = lane >> 3, col = 4 * (lane & 7);
-  const bool mine = col < J;
-  const float* wj = w + col;
+  const bool mine = j0 + col < J;
+  const float* wj = w + j0 + col;
   auto copy_weights = [&](int b) {
     const unsigned* off = sm.off[b % kListRing];
     const unsigned to = smem_u32(&sm.w[b % kRing][0][0]);
@@ -75,7 +77,8 @@ snn_walk_alone_kernel(const Geometry g, const WalkEntry* lists, const int* nvali
       if (mine) copy_async(to + 512u * q + 16u * lane, wj + off[4 * q + sub]);
   };
 
-  const bool ok = lane < g.jout;
+  const int j = j0 + lane;
+  const bool ok = j < g.jout;
 #pragma unroll
   for (int b = 0; b < kRing - 1; ++b) {
     read_list(b);
@@ -86,7 +89,7 @@ snn_walk_alone_kernel(const Geometry g, const WalkEntry* lists, const int* nvali
   }
   read_list(kRing - 1);
   LaneWalk wk;
-  wk.start(g, ok, g.has_bias && ok ? ld_plain(w + (size_t)g.I * J + lane) : 0.f);
+  wk.start(g, ok, g.has_bias && ok ? ld_plain(w + (size_t)g.I * J + j) : 0.f);
   bool turned = false;
   for (int b = 0; b < blocks; ++b) {
     put_list(b + kRing - 1);
@@ -126,6 +129,13 @@ snn_walk_alone_kernel(const Geometry g, const WalkEntry* lists, const int* nvali
       group(x[0], wv[0]);
       k = kGroup;
     }
+    if (kGroup > 8 && k + 8 <= nb) {
+      float x8[8], w8[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) { x8[u] = xb[k + u]; w8[u] = wb[(k + u) * 32]; }
+      group(x8, w8);
+      k += 8;
+    }
 #pragma unroll 1
     for (; k < nb; ++k) {
       const float x1[1] = {xb[k]};
@@ -140,20 +150,30 @@ snn_walk_alone_kernel(const Geometry g, const WalkEntry* lists, const int* nvali
   float yv, iv;
   wk.finish(g, yv, iv);
   if (ok) {
-    out[(size_t)r * g.jout + lane] = yv;
-    if (!g.infer) out[(size_t)(g.R + r) * g.jout + lane] = iv;
+    out[(size_t)r * g.jout + j] = yv;
+    if (!g.infer) out[(size_t)(g.R + r) * g.jout + j] = iv;
     if (g.khist != nullptr) atomicAdd(g.khist + (yv < g.maxv ? entries_below(ents, n, yv) : g.I + 1), 1);
   }
+}
+
+template <int kBlock>
+int launch(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out, int list_ctas,
+           const LaunchInfo& li, cudaStream_t s) {
+  const int slices = (g.J + 31) / 32;
+  const long grid = ((long)g.R * slices + kWarps - 1) / kWarps;
+  if (grid > 0x7fffffffL) return E_UNSUPPORTED;
+  const cudaError_t e = launch_chained(snn_walk_alone_kernel<kBlock>, {(unsigned)grid, walk_chains(grid, list_ctas, false, li)}, 32 * kWarps, 0, s, 0, g,
+                                       lists, nvalid, istride, w, out, slices);
+  count_launch();
+  return e == cudaSuccess ? OK : E_CUDA;
 }
 
 }  // namespace
 
 int launch_walk_alone(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
-                      cudaStream_t s) {
-  const cudaError_t e = launch_chained(snn_walk_alone_kernel, ((unsigned)g.R + kWarps - 1) / kWarps, 32 * kWarps, 0, s, 0, g, lists,
-                                       nvalid, istride, w, out);
-  count_launch();
-  return e == cudaSuccess ? OK : E_CUDA;
+                      bool large, int list_ctas, const LaunchInfo& li, cudaStream_t s) {
+  return large ? launch<32>(g, lists, nvalid, istride, w, out, list_ctas, li, s)
+               : launch<16>(g, lists, nvalid, istride, w, out, list_ctas, li, s);
 }
 
 }  // namespace snntc

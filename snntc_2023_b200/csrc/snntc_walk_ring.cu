@@ -160,12 +160,14 @@ snn_walk_ring_kernel(const Geometry g, const WalkEntry* lists, const int* nvalid
 }
 
 template <bool VEC, int C>
-int launch(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out, cudaStream_t s) {
+int launch(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out, int list_ctas,
+           const LaunchInfo& li, cudaStream_t s) {
   const long grid = (long)g.R * ((g.J + 32 * C - 1) / (32 * C));
   if (grid > 0x7fffffffL) return E_UNSUPPORTED;
   constexpr size_t smem = sizeof(RingShared<C>);
   if (allow_smem<snn_walk_ring_kernel<VEC, C>>(smem) != cudaSuccess) return E_CUDA;
-  const cudaError_t e = launch_chained(snn_walk_ring_kernel<VEC, C>, (unsigned)grid, 32 * (C + 1), smem, s, 0, g, lists, nvalid, istride, w, out);
+  const cudaError_t e = launch_chained(snn_walk_ring_kernel<VEC, C>, {(unsigned)grid, walk_chains(grid, list_ctas, C == 1, li)}, 32 * (C + 1), smem, s, 0, g,
+                                       lists, nvalid, istride, w, out);
   count_launch();
   return e == cudaSuccess ? OK : E_CUDA;
 }
@@ -178,13 +180,13 @@ int launch(const Geometry& g, const WalkEntry* lists, const int* nvalid, int ist
 // 1024 at 64 samples 424 us, 515 with two; 2000 -> 512 at 128 43, 53): the copying warp, 28 cycles an entry, holds four back (9000 ->
 // 700 at 30 samples 115 us, 89 with two).
 int launch_walk_ring(const Geometry& g, const WalkEntry* lists, const int* nvalid, int istride, const float* w, float* out,
-                     const LaunchInfo& li, cudaStream_t s) {
+                     int list_ctas, const LaunchInfo& li, cudaStream_t s) {
   const bool vec = (g.J & 3) == 0 && ((uintptr_t)w & 15) == 0;
-  if (!vec) return launch<false, 1>(g, lists, nvalid, istride, w, out, s);
+  if (!vec) return launch<false, 1>(g, lists, nvalid, istride, w, out, list_ctas, li, s);
   auto ctas = [&](int c) { return (long)g.R * ((g.J + 32 * c - 1) / (32 * c)); };
-  if (g.J <= 32 || ctas(1) <= li.num_sms) return launch<true, 1>(g, lists, nvalid, istride, w, out, s);
-  if (ctas(2) > 6L * li.num_sms && ctas(4) <= 4L * li.num_sms) return launch<true, 4>(g, lists, nvalid, istride, w, out, s);
-  return launch<true, 2>(g, lists, nvalid, istride, w, out, s);
+  if (g.J <= 32 || ctas(1) <= li.num_sms) return launch<true, 1>(g, lists, nvalid, istride, w, out, list_ctas, li, s);
+  if (ctas(2) > 6L * li.num_sms && ctas(4) <= 4L * li.num_sms) return launch<true, 4>(g, lists, nvalid, istride, w, out, list_ctas, li, s);
+  return launch<true, 2>(g, lists, nvalid, istride, w, out, list_ctas, li, s);
 }
 
 }  // namespace snntc

@@ -278,14 +278,15 @@ def test_hidden_spikes_in_the_walk_whose_warps_copy_for_themselves(R, J, band, s
     xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
     ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
     assert band > 1e-4 or int((ref[R:] < 0).sum()) > 0
-    for layout in (0, 16, 128):
+    for layout in (0, 16, 128, 256):
         assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=layout)), ref), "layout %d" % layout
 
 
-@pytest.mark.parametrize("J", [4, 16, 20, 32])
-@pytest.mark.parametrize("I", [1, 7, 8, 9, 15, 16, 17, 33, 64, 300])
+@pytest.mark.parametrize("J", [4, 16, 20, 32, 36, 100, 256])
+@pytest.mark.parametrize("I", [1, 7, 8, 9, 15, 16, 17, 24, 31, 32, 33, 64, 65, 300])
 def test_warps_that_copy_for_themselves_by_name(I, J):
-    """Lists that end at every edge of a group of 8 and a block of 16, inputs below zero and below the bias input, empty rows."""
+    """Lists that end at every edge of a group of 8 or 16 and a block of 16 or 32, one and several slices of 32 outputs with ragged last ones,
+    inputs below zero and below the bias input, empty rows."""
     import torch
     from snntc_2023_b200 import _lib, ops
     rng = np.random.default_rng(40 * I + J)
@@ -298,7 +299,8 @@ def test_warps_that_copy_for_themselves_by_name(I, J):
     params = O.fc_params(biasvolt=1.0)
     xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
     ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
-    assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=128)), ref)
+    for layout in (128, 256):
+        assert torch.equal(ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=layout)), ref), "layout %d" % layout
 
 
 @pytest.mark.parametrize("J", [32, 64, 128])
@@ -319,9 +321,27 @@ def test_lists_of_one_call_walked_by_the_next(J, first):
     ws = ops.fc_forward_workspace(R, I, J, xd.device)
     ws.view(torch.int32).fill_(0)                     # a bound of zero, were none formed
     ops.snn_fc(xd, wd, params, opts=_lib.options(forward_parts=1, walk_layout=first), workspace=ws)
-    for layout in (1, 2, 3, 8, 16, 32, 64, 128):
+    for layout in (1, 2, 3, 8, 16, 32, 64, 128, 256):
         got = ops.snn_fc(xd, wd, params, opts=_lib.options(forward_parts=2, walk_layout=layout), workspace=ws)
         assert torch.equal(got, ref), "layout %d" % layout
+
+
+@pytest.mark.parametrize("R,I,J", [(590, 64, 12), (595, 64, 12), (889, 257, 24), (1700, 400, 10), (2372, 70, 9), (2400, 300, 16), (3552, 65, 12),
+                                   (3553, 65, 12), (886, 60, 10), (900, 70, 64), (890, 300, 96), (1000, 300, 64), (400, 90, 200), (300, 784, 200)])
+@pytest.mark.parametrize("bv", [0.0, 1.0])
+def test_lines_between_the_walks_that_copy(R, I, J, bv):
+    """Either side of the lines between the walk with a copying warp, those whose warps copy for themselves (blocks of 32 and 16 entries) and
+    the pairs walk, padded and whole rows: the bits of one output per lane, training and inference."""
+    import torch
+    from snntc_2023_b200 import _lib, ops
+    x, w = P.make_inputs(R + I + J, (R, I), (I + (bv > 0), J), "ref", bias=bv > 0)
+    x[np.arange(R) % 5 == 0, :I // 3] = 1e5
+    x[3] = 1e5
+    params = O.fc_params(biasvolt=bv)
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    ref = ops.snn_fc(xd, wd, params, opts=_lib.options(walk_layout=2, walk_outputs=1))
+    assert torch.equal(ops.snn_fc(xd, wd, params), ref)
+    assert torch.equal(ops.snn_fc_infer(xd, wd, params), ref[:R])
 
 
 @pytest.mark.parametrize("I", [768, 784, 801, 802, 810, 830, 836, 837, 850])
