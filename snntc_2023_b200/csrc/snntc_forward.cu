@@ -398,12 +398,13 @@ snn_walk_pairs_kernel(const Geometry g, const WalkEntry* keys_g, const int* nval
 }
 
 // ---- the pairs walk with its weights staged in shared memory ---------------------------------------------
-// Where all fan-in rows of 64 outputs fit into one CTA's shared memory ((I + bias) * 256 bytes beside the lists and the sums of the
-// spikes: up to about 770 rows), a persistent CTA of 32 warps copies that slice of the weight matrix in once -- one asynchronous bulk copy
+// Where all fan-in rows of 64 outputs fit into one CTA's shared memory ((I + bias) * 256 bytes beside 784 for each warp's list and the sums
+// of its spikes), a persistent CTA of 32 warps copies that slice of the weight matrix in once -- one asynchronous bulk copy
 // (cp.async.bulk) per weight row, all completing on one mbarrier -- and every step of every walk then reads its
 // weight pair with one shared-memory load instead of a global load through L1. CTA c takes output slice
 // c % (J/64) and every (gridDim.x / (J/64))-th row of that slice.
-// Where that leaves less room than 32 warps need beside it (from 803 rows on), the CTA has fewer.
+// Where that leaves less room than 32 warps need (from 803 rows on), the CTA has fewer, down to 21 at 835 rows: 65 536 rows of 821 -> 64, 26
+// warps, 880 us, of 831 -> 64, 22 warps, 928 (walk from global memory 1020, 1031; 32 768 rows of 831, half of the inputs spiking, 285, 287).
 constexpr int kSmemwThreads = 1024;
 constexpr size_t kSmemwFewest = 20;                    // warps
 constexpr size_t kSmemwWarpBytes = kPairsStage * sizeof(WalkEntry) + PairWalk<1>::kFloats * sizeof(float);
@@ -543,8 +544,8 @@ int launch_walk2_smemw(const Geometry& g, const WalkEntry* keys_g, const int* nv
 }
 
 // What a walk from global memory takes with n warps to an SM, in microseconds for rows of 500 inputs of which half spike: 32 warps
-// run at once, each full wave of them takes `wave`, the last one first + n * warp. Fitted on the scalar steps; with the packed ones
-// both sides became faster alike, and the choice between pairs and quads was measured again: at 300 to 2304 inputs, half or all of them
+// run at once, each full wave of them takes `wave`, the last one first + n * warp. Fitted on the scalar steps, which one, two and four outputs
+// lane + 32 m still take; with the packed ones pairs and quads became faster alike, and the choice between them was measured again: at 300 to 2304 inputs, half or all of them
 // spiking, 400 to 20 000 rows and fan-outs 70 to 512, 89 sizes, the one it takes is never more than 4 % behind the other. They cross at about
 // 32 warps of 64 outputs per SM (500 rows of 2304 -> 256: 89 us with pairs, 112 with quads, 1200 rows 166, 130).
 struct WalkCost { double wave, first, warp; };
@@ -694,10 +695,10 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   if (named == 2 || (named == 1 && al8) || (named == 3 && al16)) variant = named;
   if (opt.walk_outputs >= 1 && opt.walk_outputs <= 3) lanes = opt.walk_outputs - 1;
   int smemw_warps = 0, smemw_mul = 0;
-  // weights staged in shared memory: where they fit, for fan-out 64 with enough rows to keep one CTA of 32 warps
-  // per SM busy (measured 13-16 % faster than the global-memory pairs walk; at fan-out 128 four outputs per lane
-  // from global memory are 5 % faster than two staged slices); walk_layout 8 asks for it wherever it fits, a named
-  // layout switches it off
+  // weights staged in shared memory: where they fit, for fan-out 64 with enough rows to keep one CTA of 32 warps per SM busy (walk alone,
+  // 262 144 rows of 576 -> 64 1210 us, from global memory 1535). At fan-out 128 and 256 two and four staged slices are level with four
+  // outputs per lane from global memory: 65 536 of 576 -> 128 630, 629, 131 072 with every input spiking 2222, 2197, 16 384 of 576 -> 256 325,
+  // 320, of 768 -> 256 739, 738. walk_layout 8 asks for it wherever it fits, a named layout switches it off
   const bool smemw = walk_smemw_ok(g, w, li, &smemw_warps, &smemw_mul) &&
                      ((opt.walk_layout & 8) != 0 || ((opt.walk_layout & 3) == 0 && g.J == 64 && g.R >= 32768));
   // CTAs of the last kernel that builds the lists: eight rows each (sorting network), one row each (bucket sort of few rows), many

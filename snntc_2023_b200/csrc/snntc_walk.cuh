@@ -64,11 +64,14 @@ __device__ __forceinline__ int imin3(int a, int b, int c) { return min(min(a, b)
 // the rows are one wave, of the whole launch. So between two blocks such an output changes the sign of its sums (flip()). Its q is
 // positive again, and below -tol it fires again: q rose through zero, the denominator is NEGATIVE, and the proof above holds with
 // both signs turned. From then on the row is walked by the FLIP steps, which give the weights each output's sign.
-// Measured (B200, four outputs per lane from global memory, before -> now): 1024 rows of 784 -> 400 172 -> 133 us (145 with the FLIP
-// steps not unrolled, 202 without them), 65 536 of 576 -> 128 690 -> 634, 16 384 of 2304 -> 256 993 -> 890; instructions per step
-// of 128 outputs 24.5 -> 17.4 where nothing fires. One pair per lane: 262 144 of 576 -> 64 1385 -> 1291, with the weights in shared
-// memory 1260 -> 1104. What bounds it: the chain q - minimum - vote - branch at 32 warps per SM (issue slots 55 % busy) and the FMA
-// pipe that takes the packed instructions.
+// Measured (B200, walk alone, scalar steps with a vote each -> now), four outputs per lane from global memory: 1024 rows of 784 -> 400 130 -> 109
+// us, 65 536 of 576 -> 128 687 -> 629, 16 384 of 2304 -> 256 1243 -> 1107; instructions per step of 128 outputs 24.5 -> 17.4 where nothing
+// fires. One pair per lane: 262 144 of 576 -> 64 1632 -> 1535, 250 of 4096 -> 512 158 -> 127, with the weights in shared memory 262 144 of
+// 576 -> 64 1384 -> 1210. Rows with an input below zero, where every spike is compared: 16 384 of 576 -> 128 186 -> 220 (scalar 206).
+// Asking shared memory after every block which outputs have fired took 0.5 to 3 % more; a second copy of the walk in the kernel, for warps
+// without lanes behind the row, up to 20 % (784 -> 400 at 256 rows by pairs 62 us, 51 with one copy).
+// What bounds it: the chain q - minimum - vote - branch at 32 warps per SM (issue slots 64 % busy) and the FMA pipe that takes the packed
+// instructions.
 template <int P>
 struct PairWalk {
   static constexpr int kFloats = 128 * P;   // of shared memory per warp

@@ -1,12 +1,14 @@
-// The sorted walk for fan-outs of 17 to 32 and a moderate number of rows: a warp walks one row, one output per lane, and copies the
-// weight rows its list names into shared memory ahead of itself.
+// The sorted walk for a moderate number of (row, 32 outputs) items: a warp walks one, one output per lane, and copies the weight rows its list
+// names into shared memory ahead of itself.
 //
-// Between the walk with a copying warp (snntc_walk_ring.cu), which with a second warp per row is two waves here, and the pairs walk,
-// half of whose lanes would be idle. Weight rows arrive by asynchronous copies, 16 entries to a block, two blocks ahead of the one
-// that is consumed; the sums and sign tests of eight steps are formed before one vote, from operands that were read a group ahead.
+// Between the walk with a copying warp (snntc_walk_ring.cu), which with a second warp per item is two waves here, and the pairs walk, which
+// at fan-outs up to 32 leaves half of its lanes idle and beyond has too few warps to hide its latencies. Weight rows arrive by asynchronous
+// copies, kBlock entries to a block, two blocks ahead of the one that is consumed; the sums and sign tests of kBlock / 2 steps are
+// formed before one vote, from operands that were read a group ahead. Blocks of 32 entries halve the votes, and take twice the shared
+// memory: 16 warps to an SM instead of 32.
 // The steps are those of the walk with a copying warp (LaneWalk in snntc_walk.cuh): the same bits. Bound by the latency of the chain of sums
-// up to about ten rows per SM and by issue beyond. Measured (B200, walk alone; copying warp, this, pairs walk): 2304 -> 32 at 2600 rows
-// 77, 65, 83 us, 5400 -> 32 161, 139, 180, 576 -> 32 28, 24, 25.
+// up to about ten items per SM and by issue beyond. Measured (B200, walk alone; copying warp, this, pairs walk): 2304 -> 32 at 2600 rows
+// 77, 65, 83 us, 5400 -> 32 161, 139, 180, 576 -> 32 28, 24, 25; further figures where the choice is made (snntc_forward.cu).
 #include "snntc_common.cuh"
 #include "snntc_walk.cuh"
 
