@@ -674,7 +674,12 @@ int launch_forward(const Geometry& g_in, const float* x, const float* w, float* 
   WeightBound wb = {w_in, g.I + g.has_bias, g.jout, g.J, wbound, pad ? w_padded : nullptr, 0};
   if (!(ring || alone) || pad || !(fparts & 2)) {
     const long long n = (long long)wb.rows * g.J;
-    const long long ctas = std::max((n + 8191) / 8192, (wb.rows + 31LL) / 32);    // (32 rows of a few weights are as long as 8192 weights)
+    // With few rows to sort the bound may take longer than they do: no more than 32 weight rows to a CTA then (a few weights each are
+    // as long as 8192 weights; 401 x 10 by one CTA 40 us beside a sort of 5), and padded rows, which are copied by 4 bytes, count twice
+    // (800 x 302 at 317 rows 45.0 us with the walk, 42 so). In front of many rows the CTAs only take their places (13 986 rows of 501 -> 52,
+    // trained, 220 us with 4 CTAs, 222 with 16, 227 with 32).
+    const bool hurry = g.R <= 4096;
+    const long long ctas = std::max((n + 8191) / 8192 * (pad && hurry ? 2 : 1), wb.rows / (hurry ? 32LL : 128LL) + 1);
     wb.ctas = (int)std::min(ctas, 64LL);
     g.wbound_n = wb.ctas;
   }
