@@ -237,12 +237,12 @@ __device__ __forceinline__ void walk_row(const Geometry& g, const WalkEntry* ent
 // issued a block ahead instead of an L2 round trip per step. CH entries and their weight rows are read together.
 constexpr int kPairsStage = 34;                   // entries staged per warp: 33, and to a multiple of 16 bytes
 
-template <int P, int CH, bool WS = false>
+template <int P, int CH, bool WS = false, bool FULL = WS>
 __device__ __forceinline__ void walk_pairs(const Geometry& g, const WalkEntry* ents, int nvalid, const float* w, int jbase, int lane,
                                            float* __restrict__ y_row, float* __restrict__ inv_row, WalkEntry* __restrict__ sbuf,
                                            float* __restrict__ fin, unsigned ws_lane = 0u, unsigned wmul = 0u) {
   const int j0 = jbase + 2 * P * lane;                    // this lane's outputs: 2 * P from j0 on
-  const unsigned lane_off = (unsigned)(jbase + 2 * P * (WS ? lane : min(lane, (g.J - jbase) / (2 * P) - 1)));   // (behind the row: its last)
+  const unsigned lane_off = (unsigned)(jbase + 2 * P * (FULL ? lane : min(lane, (g.J - jbase) / (2 * P) - 1)));   // (behind the row: its last)
   const char* wbase = reinterpret_cast<const char*>(w);
   // a 32-bit element offset from the (uniform) weight base, widened before the scaling to bytes: a 64-bit pointer per lane plus the
   // entry's offset takes two instructions more per step
@@ -265,7 +265,7 @@ __device__ __forceinline__ void walk_pairs(const Geometry& g, const WalkEntry* e
 #pragma unroll
     for (int m = 0; m < 2 * P; ++m) {   // the bias input (value biasvolt, weight row I) is always consumed first
       wb[m] = g.has_bias ? ld_plain(w + (size_t)g.I * g.J + lane_off + m) : 0.f;
-      ok[m] = WS || j0 + m < g.jout;
+      ok[m] = FULL || j0 + m < g.jout;
     }
     // (the smallest input is read by all lanes from one address: taken out of lane 0's entry below it cost a divergence check in
     // front of every vote)
@@ -327,7 +327,7 @@ __device__ __forceinline__ void walk_pairs(const Geometry& g, const WalkEntry* e
 #pragma unroll
   for (int m = 0; m < 2 * P; ++m) {
     const int j = j0 + m;
-    if (!WS && j >= g.jout) continue;
+    if (!FULL && j >= g.jout) continue;
     float y, inv;
     pw.finish(g, m, xprev, y, inv);
     y_row[j] = y;
@@ -368,7 +368,7 @@ snn_walk_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, 
 }
 
 // The same items with the outputs of a lane held in pairs (walk_pairs): a warp covers 64 * P outputs.
-template <int P>
+template <int P, bool FULL>
 __global__ void __launch_bounds__(kFwdThreads, 1024 / kFwdThreads)
 snn_walk_pairs_kernel(const Geometry g, const WalkEntry* keys_g, const int* nvalid_g, int istride, const float* w,
                       float* __restrict__ out) {
@@ -392,7 +392,7 @@ snn_walk_pairs_kernel(const Geometry g, const WalkEntry* keys_g, const int* nval
     const int n = __shfl_sync(0xffffffffu, ld_plain(nvalid_g + r), 0);
     float* yr = y_out + (size_t)r * J;
     float* ir = inv_out ? inv_out + (size_t)r * J : nullptr;
-    walk_pairs<P, CH>(g, krow, n, w, jc * 64 * P, lane, yr, ir, sbuf, fin);
+    walk_pairs<P, CH, false, FULL>(g, krow, n, w, jc * 64 * P, lane, yr, ir, sbuf, fin);
     __syncwarp();   // the next row's first block goes into the buffer this row may have read last
   }
 }
@@ -509,7 +509,12 @@ int launch_walk_pairs(const Geometry& g, const WalkEntry* keys_g, const int* nva
   const long items = (long)g.R * ((g.jout + 64 * P - 1) / (64 * P));
   long grid = (items + kFwdWarps - 1) / kFwdWarps;
   if (grid > 0x7fffffffL) grid = 0x7fffffffL;      // (a warp goes on to item + warps of the grid)
-  (void)launch_chained(snn_walk_pairs_kernel<P>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
+  // FULL (no lane behind the row) for lists of at most 64 entries, where a row costs more to begin and to end than to walk: 94 248 rows of
+  // 9 -> 128 with their lists 120 -> 112 us, 31 958 of 27 -> 256 97.7 -> 92.0. Long lists run slower in it (65 536 of 576 -> 128 628 -> 632).
+  if (g.I <= 64 && g.jout % (64 * P) == 0)
+    (void)launch_chained(snn_walk_pairs_kernel<P, true>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
+  else
+    (void)launch_chained(snn_walk_pairs_kernel<P, false>, (int)grid, kFwdThreads, 0, s, 0, g, keys_g, nvalid_g, key_stride(g), w, out);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? OK : E_CUDA;
 }
